@@ -320,6 +320,8 @@ __global__ void __launch_bounds__(threads_for(EPQ), 1)
 assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmXl,
                    const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmCl,
                    const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmXc,
+                   const __grid_constant__ CUtensorMap tmXlc,
                    AssignArgs p, int stages, int xbufs, int mode) {
   constexpr int NUM_EPI_WARPS = 4 * EPQ;
   constexpr int EPI_PER_QUAD = EPQ;
@@ -357,6 +359,19 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const long long c = (long long)*p.n_dev - p.row0;
     n_rows = c < 0 ? 0 : (c < p.n ? c : p.n);
   }
+  // rows selected by their distance bounds: the compact copy of the listed rows, or all rows
+  // when more than its capacity are listed
+  constexpr bool kSel = !F8 && !XMAX;
+  bool compact = false;
+  if (kSel && p.sel) {
+    const int c = *p.sel;
+    compact = c <= p.sel_cap;
+    if (compact) n_rows = c;
+  }
+  if (n_rows <= 0) return;  // uniform over the grid, before any barrier or TMEM allocation
+  auto map_x = [&](int pl) {
+    return compact ? (pl ? &tmXlc : &tmXc) : (pl ? &tmXl : &tmX);
+  };
   const long long n_units = (n_rows + UNIT - 1) / UNIT;
   const bool cand_mode = p.thr_in != nullptr;
   const bool grouped = p.u_prob != nullptr;
@@ -430,9 +445,9 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       mbar_init(smem_u32(&bars.merge_empty[q]), 32);
     }
     fence_mbar_init();
-    prefetch_tmap(&tmX);
+    prefetch_tmap(map_x(0));
     prefetch_tmap(&tmC);
-    if (xplanes > 1) prefetch_tmap(&tmXl);
+    if (xplanes > 1) prefetch_tmap(map_x(1));
     if (cplanes > 1) prefetch_tmap(&tmCl);
     if (bias) prefetch_tmap(&tmB);
   }
@@ -471,14 +486,14 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         const int xrow = (int)(p.row0 + u * UNIT + rank * BM);
         for (int pl = 0; pl < xplanes; ++pl)
           for (int kb = 0; kb < nkb; ++kb)
-            tma_load_2d_pair(smem_u32(xs + (size_t)(pl * nkb + kb) * XKB_BYTES), pl ? &tmXl : &tmX,
+            tma_load_2d_pair(smem_u32(xs + (size_t)(pl * nkb + kb) * XKB_BYTES), map_x(pl),
                              xb, kb * bk, xrow);
         // the next unit's points come from HBM: start them towards L2 now, so that their TMA
         // load (queued behind the center stages) is an L2 hit
         if (u + npairs < n_units) {
           const int nrow = (int)(p.row0 + (u + npairs) * UNIT + rank * BM);
           for (int pl = 0; pl < xplanes; ++pl)
-            for (int kb = 0; kb < nkb; ++kb) tma_prefetch_2d(pl ? &tmXl : &tmX, kb * bk, nrow);
+            for (int kb = 0; kb < nkb; ++kb) tma_prefetch_2d(map_x(pl), kb * bk, nrow);
         }
         for (int c = 0; c < ui.nch && ok; ++c) {
           const int crow = ui.cbase + chunk_of(ui, c) * BN + (int)rank * BNH;
@@ -603,7 +618,9 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       // the point's norm bound is needed only after the last chunk: load it now so that its
       // HBM latency hides behind the unit's chunks
       const float xn_pt = ((p.certify || XMAX) && !cand_mode && h == 0 && prow < n_rows)
-                              ? __ldg(p.xnorm + p.out0 + prow) : 0.0f;
+                              ? __ldg(p.xnorm + (compact ? (long long)__ldg(p.row_map + prow)
+                                                         : p.out0 + prow))
+                              : 0.0f;
       // separation mode: the unit's rows (one group: groups fill whole 256-row units) skip the
       // chunks of their own group
       const int unit_group = XMAX ? __ldg(p.slot_group + u * UNIT) : 0;
@@ -780,7 +797,9 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         b1 = fmaxf(b1, ob1[o]);
         b2 = nb2;
       }
-      const long long pt = p.out0 + prow;  // row of the data set
+      // row of the data set
+      const long long pt = !compact ? p.out0 + prow
+                                    : (prow < n_rows ? (long long)__ldg(p.row_map + prow) : 0);
       if (XMAX) {  // an upper bound of the largest exact key over the other groups' centers
         if (prow < n_rows)
           p.xmax_out[pt] = b1 > -1.0e38f ? __fadd_ru(b1, bound_acc(xn_pt, cm, p.d, mode, bias))
@@ -797,7 +816,18 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           const float eb = (fp8 ? bound_fp8(xn_pt, cm, p.d, sx_pt, sc_all)
                                       : bound_acc(xn_pt, cm, p.d, mode, bias)) +
                            1.02f * p.pert * (xn_pt * cm * 1.01f + 0.5f * cm * cm);
-          if (none || !(b1 - b2 > 2.0f * eb)) {
+          const bool flagged = none || !(b1 - b2 > 2.0f * eb);
+          if (kSel && p.ub) {
+            // d^2 = ||x||^2 - 2 key, ||x||^2 in [xn^2 (1 - 2^-19), xn^2] (xn: point_norms_kernel,
+            // or prep_centers_kernel's ||c||), the label's key at least b1 - E, every other
+            // usable center's at most b2 + E
+            const float t1 = __fmaf_ru(-2.0f, __fsub_rd(b1, eb), __fmul_ru(xn_pt, xn_pt));
+            const float t2 = __fmaf_rd(-2.0f, __fadd_ru(b2, eb),
+                                       __fmul_rd(__fmul_rd(xn_pt, xn_pt), 1.0f - 0x1p-19f));
+            p.ub[pt] = flagged ? INFINITY : __fsqrt_ru(fmaxf(t1, 0.0f));
+            p.lb[pt] = flagged || !(t2 > 0.0f) ? 0.0f : __fsqrt_rd(t2);
+          }
+          if (flagged) {
             const int slot = atomicAdd(p.rerank_count, 1);
             p.rerank_list[slot] = (int)pt;
             // the FP64 arg-min's key is >= b1 - 2E (E bounds every key's error)
@@ -931,8 +961,8 @@ static cudaError_t launch_assign_fp8(const void* X8, long long ld8x, const void*
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<4, true, false>, tmX, tmX, tmC, tmC, tmC, a,
-                                   stages, xbufs, 4));
+  KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<4, true, false>, tmX, tmX, tmC, tmC, tmC, tmX,
+                                   tmX, a, stages, xbufs, 4));
   count_launches(1);
   return cudaSuccess;
 }
@@ -1000,6 +1030,20 @@ cudaError_t launch_assign_bf16(const void* Xb, const void* Xl, long long ldxb, c
   if (mode > 1)
     KMGB_CUDA_TRY(kmgb_make_tmap_2d(&tmCl, Cl, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                                     (uint64_t)a.d, (uint64_t)a.k, (uint64_t)ldcb * 2, BK, BNH));
+  CUtensorMap tmXc = tmX, tmXlc = tmXl;
+  if (a.sel) {  // the compact copy of the selected rows
+    if (!a.Xc || !a.row_map || a.sel_cap <= 0 || a.u_prob || a.thr_in || a.n_dev ||
+        (mode == 2 && !a.Xlc) || (reinterpret_cast<uintptr_t>(a.Xc) & 15) ||
+        (reinterpret_cast<uintptr_t>(a.Xlc) & 15))
+      return cudaErrorInvalidValue;
+    KMGB_CUDA_TRY(kmgb_make_tmap_2d(&tmXc, a.Xc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.d,
+                                    (uint64_t)a.sel_cap, (uint64_t)ldxb * 2, BK, BM));
+    tmXlc = tmXc;
+    if (mode == 2)
+      KMGB_CUDA_TRY(kmgb_make_tmap_2d(&tmXlc, a.Xlc, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                                      (uint64_t)a.d, (uint64_t)a.sel_cap, (uint64_t)ldxb * 2, BK,
+                                      BM));
+  }
   const long long n_units = (a.n + UNIT - 1) / UNIT;
   const long long pairs = n_units < vi.max_pairs ? n_units : vi.max_pairs;
   if (pairs <= 0) return cudaSuccess;
@@ -1024,10 +1068,10 @@ cudaError_t launch_assign_bf16(const void* Xb, const void* Xl, long long ldxb, c
     if (vx.smem_budget < smem || vx.max_pairs < pairs) return cudaErrorInvalidConfiguration;
     if (epq == 2)
       KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<2, false, true, true>, tmX, tmXl,
-                                       tmC, tmCl, tmB, ab, stages, xbufs, mode));
+                                       tmC, tmCl, tmB, tmXc, tmXlc, ab, stages, xbufs, mode));
     else
       KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<4, false, true, true>, tmX, tmXl,
-                                       tmC, tmCl, tmB, ab, stages, xbufs, mode));
+                                       tmC, tmCl, tmB, tmXc, tmXlc, ab, stages, xbufs, mode));
     count_launches(1);
     return cudaSuccess;
   }
@@ -1039,16 +1083,16 @@ cudaError_t launch_assign_bf16(const void* Xb, const void* Xl, long long ldxb, c
   }
   if (epq == 2 && bias)
     KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<2, false, true>, tmX, tmXl, tmC, tmCl,
-                                     tmB, ab, stages, xbufs, mode));
+                                     tmB, tmXc, tmXlc, ab, stages, xbufs, mode));
   else if (epq == 2)
     KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<2, false, false>, tmX, tmXl, tmC,
-                                     tmCl, tmB, ab, stages, xbufs, mode));
+                                     tmCl, tmB, tmXc, tmXlc, ab, stages, xbufs, mode));
   else if (bias)
     KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<4, false, true>, tmX, tmXl, tmC, tmCl,
-                                     tmB, ab, stages, xbufs, mode));
+                                     tmB, tmXc, tmXlc, ab, stages, xbufs, mode));
   else
     KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<4, false, false>, tmX, tmXl, tmC,
-                                     tmCl, tmB, ab, stages, xbufs, mode));
+                                     tmCl, tmB, tmXc, tmXlc, ab, stages, xbufs, mode));
   count_launches(1);
   return cudaSuccess;
 }

@@ -234,6 +234,10 @@ struct kmgb_handle {
   float* xnF = nullptr;
   void* XbF = nullptr;
   void* XlF = nullptr;
+  // distance bounds between the iterations of a run (n 0: off), their buffers in one allocation
+  PruneState pr;
+  void* prune_arena = nullptr;
+  int* crr_list = nullptr;  // scratch of the centers' own scan
   // k-means++ work space (allocated on first use): D^2, block weight sums, max/pick, picks
   float* kpp_d2 = nullptr;
   unsigned long long* kpp_blk = nullptr;
@@ -286,7 +290,8 @@ struct kmgb_handle {
     if (stream) {
       cudaStreamSynchronize(stream);
       // the fixed buffers live in the arena; these are allocated on their own
-      void* ptrs[] = {arena, sse_dev, kpp_d2, kpp_blk, kpp_sc, kpp_picks, fb_arena, shard_arena};
+      void* ptrs[] = {arena, sse_dev, kpp_d2, kpp_blk, kpp_sc, kpp_picks, fb_arena, shard_arena,
+                      prune_arena};
       for (void* p : ptrs) dev_free(p, stream);
       router_destroy(router, stream);
       cudaStreamSynchronize(stream);
@@ -315,6 +320,58 @@ int audit_rows_for(const kmgb_options& o, bool streaming, int k, int d) {
   rows = std::max(0LL, std::min<long long>(rows, kAuditMaxRows));
   const long long cap = std::max(1LL, (1LL << 30) / ((long long)k * d));
   return (int)std::min(rows, cap);
+}
+
+// Distance bounds (prune.cu) where an iteration's scan is long next to their cost: the scan of the
+// centers against themselves (k rows), the pass over the bounds (20 bytes a row) and three more
+// launches, ~25 us in all at 900,000 x 128, K=256, where the scan takes 80 us. On GB300, 10
+// iterations of 4M x 128, K=1024 from sampled centers: 25.9 -> 17.8 ms.
+constexpr long long kPruneMinWork = 1LL << 33;  // rows x centers (in chunks of 256) x dimensions
+constexpr long long kPruneMaxBytes = 8LL << 30;  // of the compact copy
+
+bool prune_wanted(const kmgb_options& o, bool mini, bool streaming, long long n, int d, int k) {
+  if (o.assign_tier != KMGB_ASSIGN_BF16 && o.assign_tier != KMGB_ASSIGN_BF16X3) return false;
+  if (!o.certify || mini || streaming || o.router || k < 2) return false;
+  return n * round_up(k, kCenterPad) >= kPruneMinWork / d && (long long)k * 32 <= n;
+}
+
+// The bounds' buffers, from the pool. They are an optimisation: where they do not fit, the handle
+// scans every row in every iteration.
+void alloc_prune(kmgb_handle* h, bool split) {
+  const long long row = h->ldb * 2 * (split ? 2 : 1);
+  PruneState p;
+  p.n = h->n;
+  p.k = h->k;
+  // at about 0.65 of the rows the copy and the scan of the listed rows take as long as the scan of
+  // all rows
+  p.cap = (int)std::min(h->n * 13 / 20, kPruneMaxBytes / row);
+  if (p.cap < 256) return;
+  auto carve = [&](Arena& a) {
+    a.take(&p.ub, p.n);
+    a.take(&p.lb, p.n);
+    a.take(&p.shift, p.k);
+    a.take(&p.cxn, p.k);
+    a.take(&p.cub, p.k);
+    a.take(&p.clb, p.k);
+    a.take(&p.clab, p.k);
+    a.take(&h->crr_list, p.k);
+    a.take(&p.list, p.cap);
+    a.take(&p.flags, 4);
+    a.take(&p.top, 2);
+    a.take_bytes(&p.Xc, (size_t)p.cap * h->ldb * 2);
+    if (split) a.take_bytes(&p.Xlc, (size_t)p.cap * h->ldb * 2);
+  };
+  Arena sizing;
+  carve(sizing);
+  if (dev_alloc(&h->prune_arena, sizing.off, h->stream) != cudaSuccess) {
+    cudaGetLastError();
+    h->prune_arena = nullptr;
+    return;
+  }
+  Arena cut;
+  cut.base = static_cast<char*>(h->prune_arena);
+  carve(cut);
+  h->pr = p;
 }
 
 int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_options* opt) {
@@ -518,6 +575,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   w.sse_indexed = h->streaming ? 0 : 1;  // host-streamed iterations write their own slot
   h->sse_cap = std::max(1, h->opt.max_iters);
   KM_TRY(dalloc(&h->sse_dev, h->sse_cap, h->stream), (delete h, code));
+  if (prune_wanted(h->opt, h->mini, h->streaming, n, d, k)) alloc_prune(h, split);
   *out = h;
   return 0;
 }
@@ -739,6 +797,8 @@ int rerank_flagged(kmgb_handle* h, const AssignArgs& a, const float* Xa, const v
     c2.labels = nullptr;
     c2.certify = 0;
     c2.thr_out = nullptr;
+    c2.ub = c2.lb = nullptr;
+    c2.sel = nullptr;
     c2.n_dev = h->rr_count;
     c2.row0 = 0;
     c2.thr_in = h->thr_c;
@@ -876,6 +936,30 @@ int router_step(kmgb_handle* h, AssignArgs a) {
   return 0;
 }
 
+// With distance bounds: the nearest other center of every center (the centers scanned against
+// themselves as rows), then the rows whose label the moved bounds do not prove, in h->pr's list and
+// compact copy.
+int prune_rows(kmgb_handle* h, const AssignArgs& a, const void* Xba, const void* Xla) {
+  cudaStream_t s = h->stream;
+  PruneState& p = h->pr;
+  AssignArgs c = a;
+  c.n = h->k;
+  c.n_dev = p.flags;  // no rows while there are no bounds to check
+  c.xnorm = p.cxn;
+  c.labels = p.clab;
+  c.rerank_list = h->crr_list;
+  c.rerank_count = p.flags + 2;
+  c.thr_out = nullptr;
+  c.ub = p.cub;
+  c.lb = p.clb;
+  c.gamma = assign_bf16_gamma(h->d);
+  KM_TRY(launch_assign_bf16(h->Cb, h->Cl, h->ldb, h->Cb, h->Cl, h->ldb, c, s),
+         KMEANS_ERROR_CLOSEST_CENTERS);
+  KM_TRY(launch_prune_filter(p, h->labels, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
+  KM_TRY(launch_prune_gather(p, Xba, Xla, h->ldb * 2, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
+  return 0;
+}
+
 // One Lloyd iteration on the handle's stream; SSE lands in sse_dev[slot]. upload (tensor tiers,
 // full batch): the host data set arrives during this iteration -- chunk by chunk, each copied on
 // the copy stream, then prepared and assigned on the handle's stream while the next one crosses
@@ -911,8 +995,10 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   // reset (kmeans.cpp:1142-1170): norms of the current centers, cleared counters
   KM_TRY(cudaMemsetAsync(h->cmax, 0, sizeof(float), s), KMEANS_ERROR_RESET);
   KM_TRY(cudaMemsetAsync(h->rr_count, 0, 3 * sizeof(int), s), KMEANS_ERROR_RESET);
+  const bool prune = h->pr.n > 0 && !assign_only;
   KM_TRY(launch_prep_centers(h->C, h->ldx, h->k, h->d, h->Cop, h->Cb, h->ldb, h->cn, h->cmax, s,
-                             h->stop, h->cinit, h->Cl, h->cbias),
+                             h->stop, h->cinit, h->Cl, h->cbias, prune ? h->pr.shift : nullptr,
+                             prune ? h->pr.cxn : nullptr),
          KMEANS_ERROR_RESET);
   if (h->C8)
     KM_TRY(launch_centers_fp8(h->Cop, h->ldx, h->k, h->d, h->cmax, h->C8, h->ld8, h->cscale, s,
@@ -944,6 +1030,11 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   } else if (tc && upload) {
     a.gamma = assign_bf16_gamma(h->d);
     a.thr_out = h->opt.certify ? h->thr_full : nullptr;
+    if (prune) {  // this iteration scans every row and leaves valid bounds
+      a.ub = h->pr.ub;
+      a.lb = h->pr.lb;
+      KM_TRY(cudaMemsetAsync(h->pr.flags, 1, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+    }
     if (h->Xb) KM_TRY(cudaMemsetAsync(h->xinexact, 0, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
     if (h->ldx != h->d)  // the copies write d of ldx columns: the padding stays zero
       KM_TRY(cudaMemsetAsync(h->X, 0, sizeof(float) * h->ldx * h->n, s), KMEANS_ERROR_COPY_TILE);
@@ -980,6 +1071,17 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   } else if (tc) {
     a.gamma = assign_bf16_gamma(h->d);
     a.thr_out = h->opt.certify ? h->thr_full : nullptr;
+    if (prune) {
+      const int rc = prune_rows(h, a, Xba, Xla);
+      if (rc) return rc;
+      a.ub = h->pr.ub;
+      a.lb = h->pr.lb;
+      a.sel = h->pr.flags + 1;
+      a.sel_cap = h->pr.cap;
+      a.row_map = h->pr.list;
+      a.Xc = h->pr.Xc;
+      a.Xlc = Xla ? h->pr.Xlc : nullptr;
+    }
     KM_TRY(launch_assign_bf16(Xba, Xla, h->ldb, h->Cb, h->Cl, h->ldb, a, s),
            KMEANS_ERROR_CLOSEST_CENTERS);
   } else {
@@ -1220,6 +1322,8 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
   KM_TRY(cudaMemcpyAsync(h->loopf, kLoopInit, 2 * sizeof(double), cudaMemcpyHostToDevice,
                          h->stream),
          KMEANS_ERROR_COMPUTE);
+  if (h->pr.n > 0)  // no bounds yet: the first iteration scans every row
+    KM_TRY(cudaMemsetAsync(h->pr.flags, 0, 4 * sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
   KM_TRY(cudaEventRecord(h->ev0, h->stream), KMEANS_ERROR_COMPUTE);
   int first = 0;
   if (upload && iters > 0) {

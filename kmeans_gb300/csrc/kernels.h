@@ -70,6 +70,18 @@ struct AssignArgs {
   int fp8;
   const float* xscale;
   const float* cscale;
+  // Distance bounds kept within one run (prune.cu; null otherwise): for every row whose label the
+  // certificate proves, ub receives an upper bound of its distance to that center and lb a lower
+  // bound of its distance to every other usable center; a flagged row gets (inf, 0). With sel (a
+  // device count), *sel <= sel_cap rows are scanned instead of all n: row i of the compact copy
+  // Xc / Xlc (launch_assign_bf16) or of the gathered rows stands for row row_map[i].
+  float* ub;
+  float* lb;
+  const int* sel;
+  int sel_cap;
+  const int* row_map;
+  const void* Xc;
+  const void* Xlc;
   // test hook of the FP32 tier (kmgb_debug_withhold_stage): the producer issues no TMA load for
   // pipeline steps >= test_withhold (0: every step), and every wait gives up after
   // test_wait_cycles SM cycles (0: KMGB_WAIT_CYCLES)
@@ -179,12 +191,42 @@ cudaError_t launch_count_stats(const int* counts, int full_idx, unsigned long lo
 // cinit (nullable, round_up(k,128) floats) receives -cn/2 per usable center and -3e38 for
 // unusable centers and padding; cbias (nullable, round_up(k,128) rows of kBiasCols BF16) the same
 // start values split exactly into three BF16 numbers (columns 0..2, the rest zero), the B
-// operand of the pair kernel's start-value MMA.
+// operand of the pair kernel's start-value MMA. shift (nullable): upper bound of the distance
+// from the row Cop holds (the previous centers) to the new one, +inf from an unusable row, -1 for
+// a center that is unusable now; cxn (nullable): upper bound of ||c_j|| (0 when unusable).
 constexpr int kBiasCols = 16;
 cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, float* Cop,
                                 void* Cb, long long ldcb, float* cn, float* cmax, cudaStream_t s,
                                 const int* stop = nullptr, float* cinit = nullptr,
-                                void* Cl = nullptr, void* cbias = nullptr);
+                                void* Cl = nullptr, void* cbias = nullptr,
+                                float* shift = nullptr, float* cxn = nullptr);
+
+// Distance bounds within one run (prune.cu): which rows an iteration has to scan again.
+struct PruneState {
+  long long n = 0;
+  int k = 0;
+  int cap = 0;             // rows of the compact copy; more rows to scan: the full scan
+  float* ub = nullptr;     // [n] upper bound of the distance to the label's center
+  float* lb = nullptr;     // [n] lower bound of the distance to every other usable center
+  float* shift = nullptr;  // [k] upper bound of the center's last move, -1: unusable center
+  float* cxn = nullptr;    // [k] upper bound of ||c_j||
+  float* cub = nullptr;    // [k] scratch of the centers' own scan
+  float* clb = nullptr;    // [k] lower bound of the distance to the nearest other usable center
+  int* clab = nullptr;     // [k] scratch of the centers' own scan
+  int* list = nullptr;     // [cap] rows to scan
+  int* flags = nullptr;    // [0] 0: no bounds yet, else >= k, [1] rows to scan, [2] scratch count, [3] index of
+                           // the center that moved most
+  float* top = nullptr;    // [2] the two largest moves
+  void* Xc = nullptr;      // [cap][ldb] compact rows (BF16), and their residual plane
+  void* Xlc = nullptr;
+};
+// Resets / reads the flags and the two largest moves; then every row's bounds are moved with the
+// centers and the rows whose label they no longer prove are listed (flags[1] > cap: all rows).
+cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
+                                cudaStream_t s);
+// The listed rows' BF16 planes into the compact copy (nothing when flags[1] > cap).
+cudaError_t launch_prune_gather(const PruneState& ps, const void* Xb, const void* Xl,
+                                long long row_bytes, const int* stop, cudaStream_t s);
 
 // Per-point norms, computed once per data set: qn = ||x||^2 (FP64), xn = upper bound ||x||.
 cudaError_t launch_point_norms(const float* X, long long ldx, long long n, int d, double* qn,

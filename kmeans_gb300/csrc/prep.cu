@@ -34,7 +34,8 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
                                     long long ldcb, float* __restrict__ cn, float* cmax,
                                     const int* stop, float* __restrict__ cinit, int kpad,
                                     __nv_bfloat16* __restrict__ Cl,
-                                    __nv_bfloat16* __restrict__ cbias) {
+                                    __nv_bfloat16* __restrict__ cbias, float* __restrict__ shift,
+                                    float* __restrict__ cxn) {
   if (stopped(stop)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -54,6 +55,29 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   bad = __any_sync(0xffffffffu, bad);
   float* op = Cop + (size_t)warp * ldc;
+  if (shift) {
+    // the move since the previous centers: FP32 sum of squared differences, widened by more than
+    // its roundings; where squares leave the normal range, sqrt(d) times the largest difference
+    float m2 = 0.0f, mx = 0.0f;
+    for (int t = lane; t < d; t += 32) {
+      const float df = fabsf(c[t] - op[t]);
+      m2 = fmaf(df, df, m2);
+      mx = fmaxf(mx, df);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (lane == 0) {
+      const bool was_bad = !(cn[warp] < INFINITY);
+      const float slack = 1.0f + (float)(d + 16) * 2.4e-7f;
+      const float mv = (mx == 0.0f || (m2 > 1e-28f && m2 < 1e37f))
+                           ? __fsqrt_ru(__fmul_ru(m2, slack))
+                           : __fmul_ru(__fmul_ru(mx, 1.000001f), __fsqrt_ru((float)d));
+      shift[warp] = bad ? -1.0f : (was_bad ? INFINITY : mv);
+    }
+    __syncwarp();
+  }
   for (int t = lane; t < (int)ldc; t += 32) op[t] = (bad || t >= d) ? 0.0f : c[t];
   if (Cb) {
     __nv_bfloat16* ob = Cb + (size_t)warp * ldcb;
@@ -71,6 +95,7 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
   if (lane == 0) {
     if (bad) {
       cn[warp] = INFINITY;
+      if (cxn) cxn[warp] = 0.0f;
       if (cinit) cinit[warp] = -3.0e38f;
     } else {
       cn[warp] = __double2float_rn(s);
@@ -78,6 +103,7 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
       // upper bound of ||c||: round the FP64 sqrt up and add a relative margin
       const float nrm = __double2float_ru(sqrt(s) * (1.0 + 1e-12));
       atomicMax(reinterpret_cast<int*>(cmax), __float_as_int(nrm));
+      if (cxn) cxn[warp] = nrm;
     }
   }
 }
@@ -274,7 +300,8 @@ cudaError_t launch_centers_fp8(const float* Cop, long long ldc, int k, int d, co
 
 cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, float* Cop, void* Cb,
                                 long long ldcb, float* cn, float* cmax, cudaStream_t s,
-                                const int* stop, float* cinit, void* Cl, void* cbias) {
+                                const int* stop, float* cinit, void* Cl, void* cbias,
+                                float* shift, float* cxn) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (k <= 0) return cudaSuccess;
   const int threads = 256;
@@ -284,7 +311,8 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
                                                  reinterpret_cast<__nv_bfloat16*>(Cb), ldcb, cn,
                                                  cmax, stop, cinit, kpad,
                                                  reinterpret_cast<__nv_bfloat16*>(Cl),
-                                                 reinterpret_cast<__nv_bfloat16*>(cbias));
+                                                 reinterpret_cast<__nv_bfloat16*>(cbias), shift,
+                                                 cxn);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }

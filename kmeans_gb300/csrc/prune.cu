@@ -1,0 +1,231 @@
+// Distance bounds kept from one iteration of a run to the next (Hamerly, "Making k-means even
+// faster", SDM 2010): rows whose label is proved without looking at the centers again.
+//
+// The assignment leaves, for every row whose label its certificate proves, an upper bound ub of the
+// distance to the label's center and a lower bound lb of the distance to every other usable center
+// (directed rounding, the tier's error bound included). When the centers move, ub grows by the
+// move of the row's own center and lb shrinks by the largest move of the others; half the distance
+// from a center to its nearest other center (from one scan of the centers against themselves) is a
+// second threshold. While ub stays below the larger of the two, every other center is strictly
+// farther, so the label is still the FP64 arg-min and the row is not scanned; the other rows are
+// copied to a compact matrix and scanned as ever. The reference scans every row in every iteration
+// (kmeans.cpp:910-1014). Nothing survives a run: its first iteration scans every row.
+//
+// prune_filter_kernel is bound by HBM: 12 bytes read and 8 written per row.
+#include "common.cuh"
+#include "kernels.h"
+
+namespace kmgb {
+namespace {
+
+constexpr int PF_THREADS = 256;
+constexpr int PF_ROWS = 4 * PF_THREADS;  // rows per block step, four consecutive ones per thread
+
+// The two largest moves and the center of the largest (unusable centers, -1, never count); starts
+// the list of rows to scan: empty when the bounds are valid, else past every capacity. One block.
+__global__ void __launch_bounds__(1024)
+prune_top_kernel(PruneState ps, const int* stop) {
+  if (stopped(stop)) return;
+  __shared__ float s1[32], s2[32];
+  __shared__ int si[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  float b1 = 0.0f, b2 = 0.0f;
+  int i1 = -1;
+  for (int j = threadIdx.x; j < ps.k; j += blockDim.x) {
+    const float v = ps.shift[j];
+    if (v > b1) {
+      b2 = b1;
+      b1 = v;
+      i1 = j;
+    } else {
+      b2 = fmaxf(b2, v);
+    }
+  }
+  auto merge = [&](float o1, float o2, int oi) {
+    b2 = fmaxf(fminf(b1, o1), fmaxf(b2, o2));
+    if (o1 > b1) {
+      b1 = o1;
+      i1 = oi;
+    }
+  };
+  for (int o = 16; o > 0; o >>= 1)
+    merge(__shfl_down_sync(0xffffffffu, b1, o), __shfl_down_sync(0xffffffffu, b2, o),
+          __shfl_down_sync(0xffffffffu, i1, o));
+  if (lane == 0) {
+    s1[w] = b1;
+    s2[w] = b2;
+    si[w] = i1;
+  }
+  __syncthreads();
+  if (w == 0) {
+    b1 = s1[lane];
+    b2 = s2[lane];
+    i1 = si[lane];
+    for (int o = 16; o > 0; o >>= 1)
+      merge(__shfl_down_sync(0xffffffffu, b1, o), __shfl_down_sync(0xffffffffu, b2, o),
+            __shfl_down_sync(0xffffffffu, i1, o));
+    if (lane == 0) {
+      ps.top[0] = b1;
+      ps.top[1] = b2;
+      ps.flags[3] = i1;
+      ps.flags[1] = ps.flags[0] ? 0 : 0x7fffffff;
+      ps.flags[0] = ps.k;
+      ps.flags[2] = 0;  // the next iteration's scan of the centers counts from zero
+    }
+  }
+}
+
+// Moves every row's bounds with the centers and lists the rows they no longer prove. Once more than
+// `cap` rows are listed every row will be scanned (and its bounds written anew): the blocks still
+// to come return.
+__global__ void __launch_bounds__(PF_THREADS)
+prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
+  if (stopped(stop)) return;
+  __shared__ int wsum[PF_THREADS / 32];
+  __shared__ int base_sh;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float top1 = ps.top[0], top2 = ps.top[1];
+  const int topi = ps.flags[3];
+  for (long long b0 = (long long)blockIdx.x * PF_ROWS; b0 < ps.n; b0 += (long long)gridDim.x * PF_ROWS) {
+    if (threadIdx.x == 0) base_sh = *(volatile int*)(ps.flags + 1);
+    __syncthreads();
+    if (base_sh > ps.cap) return;  // uniform over the block
+    const long long i0 = b0 + 4 * threadIdx.x;
+    float u[4], l[4];
+    int a[4];
+    if (i0 + 4 <= ps.n) {
+      const float4 uv = *reinterpret_cast<const float4*>(ps.ub + i0);
+      const float4 lv = *reinterpret_cast<const float4*>(ps.lb + i0);
+      const int4 av = *reinterpret_cast<const int4*>(labels + i0);
+      u[0] = uv.x, u[1] = uv.y, u[2] = uv.z, u[3] = uv.w;
+      l[0] = lv.x, l[1] = lv.y, l[2] = lv.z, l[3] = lv.w;
+      a[0] = av.x, a[1] = av.y, a[2] = av.z, a[3] = av.w;
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const bool in = i0 + r < ps.n;
+        u[r] = in ? ps.ub[i0 + r] : 0.0f;
+        l[r] = in ? ps.lb[i0 + r] : 0.0f;
+        a[r] = in ? labels[i0 + r] : 0;
+      }
+    }
+    unsigned fail = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (i0 + r >= ps.n) continue;
+      const bool lab_ok = a[r] >= 0 && a[r] < ps.k;  // always, but for an error upstream
+      const float sh = lab_ok ? __ldg(ps.shift + a[r]) : -1.0f;
+      const float near = lab_ok ? __ldg(ps.clb + a[r]) : 0.0f;
+      u[r] = sh < 0.0f ? INFINITY : __fadd_ru(u[r], sh);
+      l[r] = __fsub_rd(l[r], a[r] == topi ? top2 : top1);
+      // the nearest other center is at least `near` from this one, hence near - ub from the row;
+      // a NaN (inf - inf) fails the comparison below
+      const float l2 = __fsub_rd(near, u[r]);
+      l[r] = l2 > l[r] ? l2 : l[r];
+      // 2^-20 covers the rounding of the FP64 distances the label is defined by
+      if (!(__fmul_ru(u[r], 1.0f + 0x1p-20f) < l[r])) fail |= 1u << r;
+    }
+    if (i0 + 4 <= ps.n) {
+      *reinterpret_cast<float4*>(ps.ub + i0) = make_float4(u[0], u[1], u[2], u[3]);
+      *reinterpret_cast<float4*>(ps.lb + i0) = make_float4(l[0], l[1], l[2], l[3]);
+    } else {
+      for (int r = 0; r < 4; ++r)
+        if (i0 + r < ps.n) {
+          ps.ub[i0 + r] = u[r];
+          ps.lb[i0 + r] = l[r];
+        }
+    }
+    // one block-wide scan and one atomic per block step
+    const int c = __popc(fail);
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    if (lane == 31) wsum[w] = inc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int t = 0;
+      for (int v = 0; v < PF_THREADS / 32; ++v) {
+        const int x = wsum[v];
+        wsum[v] = t;
+        t += x;
+      }
+      base_sh = t ? atomicAdd(ps.flags + 1, t) : 0;
+    }
+    __syncthreads();
+    int at = base_sh + wsum[w] + inc - c;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (fail & (1u << r)) {
+        if (at < ps.cap) ps.list[at] = (int)(i0 + r);
+        ++at;
+      }
+    __syncthreads();
+  }
+}
+
+// One warp per listed row, 16-byte moves, both planes' loads of a row in flight together.
+__global__ void prune_gather_kernel(PruneState ps, const uint4* __restrict__ Xb,
+                                    const uint4* __restrict__ Xl, int row_vec, const int* stop) {
+  if (stopped(stop)) return;
+  const int cnt = ps.flags[1];
+  if (cnt > ps.cap) return;
+  const int lane = threadIdx.x & 31;
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  uint4* Xc = static_cast<uint4*>(ps.Xc);
+  uint4* Xlc = static_cast<uint4*>(ps.Xlc);
+  const int planes = Xl ? 2 : 1;
+  const int per = row_vec * planes;
+  // rows of both planes as one run of `per` vectors; 32 / per2 rows per warp step when they are short
+  if (per <= 32) {
+    const int rows = 32 / per;
+    const int rr = lane / per, v = lane % per;
+    const bool on = rr < rows;
+    for (long long s0 = w0 * rows; s0 < cnt; s0 += nw * rows) {
+      const long long slot = s0 + rr;
+      if (!on || slot >= cnt) continue;
+      const long long pt = __ldg(ps.list + slot);
+      if (v < row_vec) Xc[slot * row_vec + v] = __ldg(Xb + pt * row_vec + v);
+      else Xlc[slot * row_vec + v - row_vec] = __ldg(Xl + pt * row_vec + v - row_vec);
+    }
+    return;
+  }
+  for (long long slot = w0; slot < cnt; slot += nw) {
+    const long long pt = __ldg(ps.list + slot);
+    for (int v = lane; v < row_vec; v += 32) {
+      const uint4 hi = __ldg(Xb + pt * row_vec + v);
+      const uint4 lo = Xl ? __ldg(Xl + pt * row_vec + v) : make_uint4(0, 0, 0, 0);
+      Xc[slot * row_vec + v] = hi;
+      if (Xl) Xlc[slot * row_vec + v] = lo;
+    }
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
+                                cudaStream_t s) {
+  if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
+  prune_top_kernel<<<1, 1024, 0, s>>>(ps, stop);
+  const long long steps = (ps.n + PF_ROWS - 1) / PF_ROWS;
+  const long long most = kmgb::num_sms() * 8LL;
+  prune_filter_kernel<<<(unsigned)(steps < most ? steps : most), PF_THREADS, 0, s>>>(ps, labels,
+                                                                                     stop);
+  count_launches(2);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prune_gather(const PruneState& ps, const void* Xb, const void* Xl,
+                                long long row_bytes, const int* stop, cudaStream_t s) {
+  if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
+  if (row_bytes % 16 || (Xl && !ps.Xlc)) return cudaErrorInvalidValue;
+  prune_gather_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(
+      ps, static_cast<const uint4*>(Xb), static_cast<const uint4*>(Xl), (int)(row_bytes / 16), stop);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+}  // namespace kmgb

@@ -1,0 +1,80 @@
+"""Distance bounds kept between the iterations of a run: runs large enough to use them (rows x
+centers x dimensions at or above the handle's threshold) must equal the oracle's loop bit for bit
+in labels and centers, whatever share of the rows an iteration scans."""
+import numpy as np
+import pytest
+
+from kmeans_gb300.synthetic import mixture_numpy, sample_init
+
+pytestmark = pytest.mark.gpu
+
+
+def check(res, want, name=""):
+    st, c, lab, sse, it = want
+    assert res.iterations == it and res.status == st, name
+    assert np.array_equal(res.labels, lab), f"{name}: labels"
+    assert np.array_equal(res.centers, c, equal_nan=True), f"{name}: centers"
+    np.testing.assert_allclose(res.sse, sse, rtol=1e-10)
+    assert res.audit_violations == 0
+
+
+CASES = [
+    # n, d, k, components, mean span, std, tier, BF16-valued, policy
+    (70_001, 128, 1000, 1000, 20.0, (0.3, 3.0), "BF16X3", False, 1),  # separated: most rows skipped
+    (66_003, 129, 1024, 64, 2.0, (1.0, 1.0), "BF16X3", False, 1),     # overlapping: most rows scanned
+    (140_000, 256, 256, 200, 8.0, (0.5, 1.5), "BF16X3", True, 0),     # two products, NaN policy
+    (132_777, 130, 500, 500, 20.0, (1.0, 1.0), "BF16", False, 1),     # plain tier
+    (600_000, 60, 250, 240, 10.0, (1.0, 1.0), "BF16X3", False, 1),
+]
+
+
+@pytest.mark.parametrize("n,d,k,comps,span,std,tier,bf16,policy", CASES)
+def test_bounds_match_oracle(km, orc, torch_cuda, n, d, k, comps, span, std, tier, bf16, policy):
+    X, _, _ = mixture_numpy(n, d, comps, seed=n, mean_lo=-span, mean_hi=span, std=std)
+    if bf16:
+        X = torch_cuda.from_numpy(X).bfloat16().float().numpy()
+    X[100:140] = X[100]  # duplicate rows: exact ties between duplicate centers
+    init = X[sample_init(n, k, seed=3)].copy()
+    init[7] = init[2] = X[100]
+    want = orc.lloyd(X, init, 8, empty_policy=policy)
+    t = getattr(km, "ASSIGN_" + tier)
+    # host rows travel with the first iteration, device rows do not
+    check(km.lloyd(X, k, init=init, max_iters=8, assign_tier=t, empty_policy=policy), want, "host")
+    Xd = torch_cuda.from_numpy(X).cuda()
+    check(km.lloyd(Xd, k, init=init, max_iters=8, assign_tier=t, empty_policy=policy), want, "device")
+
+
+def test_bounds_end_with_the_run(km, orc, torch_cuda, monkeypatch):
+    """Other centers, other data and single-iteration runs on one handle start without bounds; a
+    run that converges stops in the oracle's iteration; kernel-by-kernel launches agree."""
+    n, d, k = 70_001, 128, 1000
+    X, _, _ = mixture_numpy(n, d, k, seed=11, mean_lo=-20, mean_hi=20, std=(0.3, 3.0))
+    Y, _, _ = mixture_numpy(n, d, k, seed=12, mean_lo=-20, mean_hi=20, std=(0.3, 3.0))
+    i1, i2 = X[sample_init(n, k, seed=1)], X[sample_init(n, k, seed=2)]
+    h = km.Handle(n, d, k, assign_tier=km.ASSIGN_BF16X3, empty_policy=1, max_iters=6)
+
+    def run(init, data, iters):
+        if init is not None:
+            h.set_centers(init)
+        h.run(iters)
+        h.synchronize()
+        return h.labels(), h.centers()
+
+    h.set_data(X, on_device=False)
+    for init in (i1, i2):
+        _, c, lab, _, _ = orc.lloyd(X, init, 5, empty_policy=1)
+        got = run(init, X, 5)
+        assert np.array_equal(got[0], lab) and np.array_equal(got[1], c)
+    _, c, lab, _, _ = orc.lloyd(X, c, 1, empty_policy=1)
+    got = run(None, X, 1)  # continues from its centers
+    assert np.array_equal(got[0], lab) and np.array_equal(got[1], c)
+    h.set_data(Y, on_device=False)
+    _, c, lab, _, _ = orc.lloyd(Y, i2, 4, empty_policy=1)
+    got = run(i2, Y, 4)
+    assert np.array_equal(got[0], lab) and np.array_equal(got[1], c)
+    h.close()
+    want = orc.lloyd(X, i1, 40, criterion=1e-3, empty_policy=1)
+    for graphs in ("1", "0"):
+        monkeypatch.setenv("KMGB_GRAPHS", graphs)
+        check(km.lloyd(X, k, init=i1, max_iters=40, criterion=1e-3, empty_policy=1,
+                       assign_tier=km.ASSIGN_BF16X3), want, "criterion")
