@@ -357,7 +357,8 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   long long n_rows = p.n;
   if (p.n_dev) {
     const long long c = (long long)*p.n_dev - p.row0;
-    n_rows = c < 0 ? 0 : (c < p.n ? c : p.n);
+    if (c <= 0) return;  // uniform over the grid, before any barrier or TMEM allocation
+    n_rows = c < p.n ? c : p.n;
   }
   // rows selected by their distance bounds: the compact copy of the listed rows, or all rows
   // when more than its capacity are listed
@@ -366,9 +367,9 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   if (kSel && p.sel) {
     const int c = *p.sel;
     compact = c <= p.sel_cap;
+    if (c == 0) return;
     if (compact) n_rows = c;
   }
-  if (n_rows <= 0) return;  // uniform over the grid, before any barrier or TMEM allocation
   auto map_x = [&](int pl) {
     return compact ? (pl ? &tmXlc : &tmXc) : (pl ? &tmXl : &tmX);
   };

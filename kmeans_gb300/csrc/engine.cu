@@ -356,6 +356,8 @@ void alloc_prune(kmgb_handle* h, bool split) {
     a.take(&p.clab, p.k);
     a.take(&h->crr_list, p.k);
     a.take(&p.list, p.cap);
+    a.take(&p.lab_old, p.n);
+    a.take(&p.dirty, p.k);
     a.take(&p.flags, 4);
     a.take(&p.top, 2);
     a.take_bytes(&p.Xc, (size_t)p.cap * h->ldb * 2);
@@ -1034,6 +1036,8 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
       a.ub = h->pr.ub;
       a.lb = h->pr.lb;
       KM_TRY(cudaMemsetAsync(h->pr.flags, 1, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      KM_TRY(cudaMemsetAsync(h->pr.flags + 1, 0x7f, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      KM_TRY(cudaMemsetAsync(h->pr.dirty, 1, sizeof(int) * h->k, s), KMEANS_ERROR_COPY_TILE);
     }
     if (h->Xb) KM_TRY(cudaMemsetAsync(h->xinexact, 0, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
     if (h->ldx != h->d)  // the copies write d of ldx columns: the padding stays zero
@@ -1105,7 +1109,12 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   if (assign_only) return 0;
   // cluster centers + compactness (kmeans.cpp:1018-1104)
   // the SSE lands in sse_dev[iteration of the run] (device-side index)
-  KM_TRY(launch_update(Xa, qna, h->labels, h->C, h->ldx, h->opt.empty_policy, h->uw,
+  UpdateWork uw = h->uw;
+  if (prune) {
+    KM_TRY(launch_prune_dirty(h->pr, h->labels, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
+    uw.dirty = h->pr.dirty;
+  }
+  KM_TRY(launch_update(Xa, qna, h->labels, h->C, h->ldx, h->opt.empty_policy, uw,
                        h->uw.sse_indexed ? h->sse_dev : h->sse_dev + slot, s),
          KMEANS_ERROR_CLUSTER_CENTERS);
   KM_TRY(h->pmark(4), KMEANS_ERROR_CLUSTER_CENTERS);

@@ -214,6 +214,8 @@ struct PruneState {
   float* clb = nullptr;    // [k] lower bound of the distance to the nearest other usable center
   int* clab = nullptr;     // [k] scratch of the centers' own scan
   int* list = nullptr;     // [cap] rows to scan
+  int* lab_old = nullptr;  // [n] labels of the last update
+  int* dirty = nullptr;    // [k] nonzero: the center's members may differ from the last update's
   int* flags = nullptr;    // [0] 0: no bounds yet, else >= k, [1] rows to scan, [2] scratch count, [3] index of
                            // the center that moved most
   float* top = nullptr;    // [2] the two largest moves
@@ -224,6 +226,9 @@ struct PruneState {
 // centers and the rows whose label they no longer prove are listed (flags[1] > cap: all rows).
 cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
                                 cudaStream_t s);
+// After the labels are settled: the centers that lost or won a row.
+cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const int* stop,
+                               cudaStream_t s);
 // The listed rows' BF16 planes into the compact copy (nothing when flags[1] > cap).
 cudaError_t launch_prune_gather(const PruneState& ps, const void* Xb, const void* Xl,
                                 long long row_bytes, const int* stop, cudaStream_t s);
@@ -262,6 +267,8 @@ struct UpdateWork {
   double* sse_k;        // [k][ceil(d/32)] SSE terms per (center, group of 32 dimensions)
   long long* counts;    // [k]
   int* err;
+  const int* dirty;     // nullable: [k] zero where the center has the members of the previous
+                        // update: its sums, center and SSE terms stay as they are
   // stop rule (kmeans.cpp:1194-1237), evaluated on the device by the SSE reduction
   int* stop;            // nullable
   double criterion;

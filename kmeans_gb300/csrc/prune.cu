@@ -8,7 +8,8 @@
 // from a center to its nearest other center (from one scan of the centers against themselves) is a
 // second threshold. While ub stays below the larger of the two, every other center is strictly
 // farther, so the label is still the FP64 arg-min and the row is not scanned; the other rows are
-// copied to a compact matrix and scanned as ever. The reference scans every row in every iteration
+// copied to a compact matrix and scanned as ever. A center none of whose rows changed keeps its
+// sums, its place and its SSE terms: the update is deterministic, so they would come out the same. The reference scans every row in every iteration
 // (kmeans.cpp:910-1014). Nothing survives a run: its first iteration scans every row.
 //
 // prune_filter_kernel is bound by HBM: 12 bytes read and 8 written per row.
@@ -22,13 +23,15 @@ constexpr int PF_THREADS = 256;
 constexpr int PF_ROWS = 4 * PF_THREADS;  // rows per block step, four consecutive ones per thread
 
 // The two largest moves and the center of the largest (unusable centers, -1, never count); starts
-// the list of rows to scan: empty when the bounds are valid, else past every capacity. One block.
+// the list of rows to scan: empty when the bounds are valid, else past every capacity (and every
+// center's members count as changed). One block.
 __global__ void __launch_bounds__(1024)
 prune_top_kernel(PruneState ps, const int* stop) {
   if (stopped(stop)) return;
   __shared__ float s1[32], s2[32];
   __shared__ int si[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int first = ps.flags[0] == 0;
   float b1 = 0.0f, b2 = 0.0f;
   int i1 = -1;
   for (int j = threadIdx.x; j < ps.k; j += blockDim.x) {
@@ -40,6 +43,7 @@ prune_top_kernel(PruneState ps, const int* stop) {
     } else {
       b2 = fmaxf(b2, v);
     }
+    ps.dirty[j] = first;
   }
   auto merge = [&](float o1, float o2, int oi) {
     b2 = fmaxf(fminf(b1, o1), fmaxf(b2, o2));
@@ -68,7 +72,7 @@ prune_top_kernel(PruneState ps, const int* stop) {
       ps.top[0] = b1;
       ps.top[1] = b2;
       ps.flags[3] = i1;
-      ps.flags[1] = ps.flags[0] ? 0 : 0x7fffffff;
+      ps.flags[1] = first ? 0x7fffffff : 0;
       ps.flags[0] = ps.k;
       ps.flags[2] = 0;  // the next iteration's scan of the centers counts from zero
     }
@@ -204,7 +208,34 @@ __global__ void prune_gather_kernel(PruneState ps, const uint4* __restrict__ Xb,
   }
 }
 
+// Marks the old and the new center of every scanned row whose label changed since the last update
+// (after a first iteration every center is marked already and lab_old takes all labels).
+__global__ void __launch_bounds__(256)
+prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
+  if (stopped(stop)) return;
+  const int cnt = ps.flags[1];
+  const bool all = cnt > ps.cap;
+  const long long total = all ? ps.n : cnt;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += (long long)gridDim.x * blockDim.x) {
+    const long long pt = all ? i : (long long)__ldg(ps.list + i);
+    const int a = ps.lab_old[pt], b = labels[pt];
+    if (a == b) continue;
+    ps.lab_old[pt] = b;
+    if (a >= 0 && a < ps.k) ps.dirty[a] = 1;
+    if (b >= 0 && b < ps.k) ps.dirty[b] = 1;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const int* stop,
+                               cudaStream_t s) {
+  if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
+  prune_dirty_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(ps, labels, stop);
+  count_launches(1);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
                                 cudaStream_t s) {

@@ -155,7 +155,8 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
 // of label j (piece_cnt[k] = 0, the scan turns it into the total); counts[j] = members.
 __global__ void label_offsets_kernel(const int* __restrict__ hist, long long n, int k, int ntiles,
                                      int* __restrict__ label_off, int* __restrict__ piece_cnt,
-                                     long long* __restrict__ counts, const int* stop) {
+                                     long long* __restrict__ counts, const int* __restrict__ dirty,
+                                     const int* stop) {
   if (stopped(stop)) return;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j > k) return;
@@ -167,13 +168,15 @@ __global__ void label_offsets_kernel(const int* __restrict__ hist, long long n, 
   const int a = hist[(size_t)j * ntiles];
   const int b = (j + 1 < k) ? hist[(size_t)(j + 1) * ntiles] : (int)n;
   label_off[j] = a;
-  piece_cnt[j] = (b - a + kSumPiece - 1) / kSumPiece;
+  // no pieces for a center that keeps its sums (UpdateWork::dirty)
+  piece_cnt[j] = dirty && !dirty[j] ? 0 : (b - a + kSumPiece - 1) / kSumPiece;
   if (counts) counts[j] = b - a;
 }
 
 template <bool SMEM>
 __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int k, int tile_pts,
-                               int ntiles, int* pos, int* __restrict__ sorted, const int* stop) {
+                               int ntiles, int* pos, int* __restrict__ sorted,
+                               const int* __restrict__ dirty, const int* stop) {
   if (stopped(stop)) return;
   extern __shared__ int cnt_s[];
   const int tile = blockIdx.x;
@@ -199,7 +202,7 @@ __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int 
     for (int u = 0; u < U; ++u) {
       const long long i = b + 32 * u + lane;
       int l = lv[u];
-      if (l < 0 || l >= k) l = -1;
+      if (l < 0 || l >= k || (dirty && !__ldg(dirty + l))) l = -1;
       const unsigned peers = warp_peers(l, nbits);
       const int leader = __ffs(peers) - 1;
       const int rank = __popc(peers & lanemask_lt());
@@ -226,7 +229,8 @@ constexpr int kScatterWarps = 8;
 
 __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n, int k,
                                      int tile_pts, int ntiles, const int* __restrict__ pos,
-                                     int* __restrict__ sorted, const int* stop) {
+                                     int* __restrict__ sorted, const int* __restrict__ dirty,
+                                     const int* stop) {
   if (stopped(stop)) return;
   extern __shared__ int wcnt[];  // [kScatterWarps][k]
   const int tile = blockIdx.x;
@@ -256,7 +260,8 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
   for (long long b = s0; b < s1; b += 32) {
     const long long i = b + lane;
     int l = i < s1 ? __ldg(labels + i) : -1;
-    if (l < 0 || l >= k) l = -1;
+    if (l < 0 || l >= k || (dirty && !__ldg(dirty + l))) l = -1;
+    if (!__any_sync(0xffffffffu, l >= 0)) continue;
     const unsigned peers = warp_peers(l, nbits);
     const int leader = __ffs(peers) - 1;
     const int rank = __popc(peers & lanemask_lt());
@@ -641,13 +646,15 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
 __global__ void finalize_kernel(const double* __restrict__ part, const double* __restrict__ partq,
                                 const int* __restrict__ label_off, const int* __restrict__ pstart,
                                 int k, int d, float* __restrict__ C, long long ldc,
-                                int empty_policy, double* __restrict__ sse_k, const int* stop) {
+                                int empty_policy, double* __restrict__ sse_k,
+                                const int* __restrict__ dirty, const int* stop) {
   if (stopped(stop)) return;
   const int groups = (d + 31) / 32;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= (long long)k * groups) return;
   const int j = (int)(wid / groups), g = (int)(wid - (long long)j * groups);
+  if (dirty && !dirty[j]) return;
   const int c = g * 32 + lane;
   const long long n = (long long)label_off[j + 1] - label_off[j];
   const int p0 = pstart[j], p1 = pstart[j + 1];
@@ -700,12 +707,13 @@ __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
                                  const int* __restrict__ pstart, int k, int d,
                                  const float* __restrict__ X, long long ldx,
                                  const int* __restrict__ sorted, const float* __restrict__ C,
-                                 long long ldc, const int* stop) {
+                                 long long ldc, const int* __restrict__ dirty, const int* stop) {
   if (stopped(stop)) return;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= k) return;
   const int j = (int)wid;
+  if (dirty && !dirty[j]) return;
   const int m0 = label_off[j], m1 = label_off[j + 1];
   if (m1 <= m0) return;
   double t = 0.0, q = 0.0;
@@ -814,7 +822,8 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.hist, hist_elems, w.scan_tmp, s, w.stop));
   label_offsets_kernel<<<(k + 1 + 255) / 256, 256, 0, s>>>(w.hist, n, k, w.ntiles, w.label_off,
-                                                          w.piece_cnt, w.counts, w.stop); kmgb::count_launches(1);
+                                                          w.piece_cnt, w.counts, w.dirty, w.stop);
+  kmgb::count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.piece_cnt, k + 1, w.scan_tmp, s, w.stop));
   const size_t msmem = sizeof(int) * (size_t)k * kScatterWarps;
@@ -826,7 +835,7 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
       multi_attr_k = k;
     }
     scatter_multi_kernel<<<w.ntiles, 32 * kScatterWarps, msmem, s>>>(
-        labels, n, k, w.tile_pts, w.ntiles, w.hist, w.sorted, w.stop);
+        labels, n, k, w.tile_pts, w.ntiles, w.hist, w.sorted, w.dirty, w.stop);
     kmgb::count_launches(1);
   } else if (smem <= 96 * 1024) {
     static int attr_k = -1;
@@ -836,10 +845,10 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
       attr_k = k;
     }
     scatter_kernel<true><<<w.ntiles, 32, smem, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist,
-                                                    w.sorted, w.stop); kmgb::count_launches(1);
+                                                    w.sorted, w.dirty, w.stop); kmgb::count_launches(1);
   } else {
     scatter_kernel<false><<<w.ntiles, 32, 0, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist,
-                                                  w.sorted, w.stop); kmgb::count_launches(1);
+                                                  w.sorted, w.dirty, w.stop); kmgb::count_launches(1);
   }
   return cudaGetLastError();
 }
@@ -856,12 +865,12 @@ cudaError_t launch_update(const float* X, const double* qn, const int* labels, f
   const long long fin_warps = (long long)k * ((w.d + 31) / 32);
   finalize_kernel<<<(unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s>>>(
       w.part, qn ? w.partq : nullptr, w.label_off, w.piece_cnt, k, w.d, C, ldc, empty_policy,
-      w.sse_k, w.stop); kmgb::count_launches(1);
+      w.sse_k, w.dirty, w.stop); kmgb::count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   if (qn) {
     sse_fixup_kernel<<<(unsigned)((k * 32LL + 255) / 256), 256, 0, s>>>(
         w.sse_k, (w.d + 31) / 32, w.partq, w.label_off, w.piece_cnt, k, w.d, X, w.ldx, w.sorted, C,
-        ldc, w.stop);
+        ldc, w.dirty, w.stop);
     kmgb::count_launches(1);
     KMGB_CUDA_TRY(cudaGetLastError());
   }
@@ -1188,12 +1197,13 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
   const int groups = (d + 31) / 32;
   const long long fin_warps = (long long)b.K * groups;
   finalize_kernel<<<(unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s>>>(
-      w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, nullptr);
+      w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, nullptr,
+      nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   sse_fixup_kernel<<<(unsigned)((b.K * 32LL + 255) / 256), 256, 0, s>>>(
       w.sse_k, groups, w.partq, w.label_off, w.piece_cnt, b.K, d, X, ldx, w.sorted, C, ldc,
-      nullptr);
+      nullptr, nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   sse_batched_kernel<<<(unsigned)((b.P * 32LL + 255) / 256), 256, 0, s>>>(w.sse_k, groups, b);
