@@ -42,10 +42,63 @@ __device__ __forceinline__ float bound_e(float xn, float cm, float gamma, int d)
   return e * 1.01f + 1e-30f;
 }
 
+// The products of four dimensions (16-byte column q of the swizzled tiles) of a thread's 8 points
+// and 8 centers.
+__device__ __forceinline__ void tile_step(const uint8_t* xs, const uint8_t* cs, int tx, int ty, int q,
+                                          float (&acc)[8][8]) {
+  float4 cv[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) cv[j] = *reinterpret_cast<const float4*>(cs + swz128(tx + 16 * j, q));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float4 xv = *reinterpret_cast<const float4*>(xs + swz128(ty + 16 * i, q));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      acc[i][j] = fmaf(xv.x, cv[j].x, acc[i][j]);
+      acc[i][j] = fmaf(xv.y, cv[j].y, acc[i][j]);
+      acc[i][j] = fmaf(xv.z, cv[j].z, acc[i][j]);
+      acc[i][j] = fmaf(xv.w, cv[j].w, acc[i][j]);
+    }
+  }
+}
+
+// One 32-dimension block. TAIL: a row's last block stops at its last 16-byte column (the columns
+// past it are zero; at D=324 seven of the last block's eight, 8% of the kernel's work). That second
+// loop leaves fewer registers for the first, which is then unrolled by four instead of eight.
+template <bool TAIL>
+__device__ __forceinline__ void tile_block(const uint8_t* xs, const uint8_t* cs, int tx, int ty,
+                                           int dims_left, float (&acc)[8][8]) {
+  if (!TAIL) {
+#pragma unroll
+    for (int q = 0; q < BKF / 4; ++q) tile_step(xs, cs, tx, ty, q, acc);
+  } else if (dims_left > BKF - 4) {
+#pragma unroll 4
+    for (int q = 0; q < BKF / 4; ++q) tile_step(xs, cs, tx, ty, q, acc);
+  } else {
+#pragma unroll 1
+    for (int q = 0; 4 * q < dims_left; ++q) tile_step(xs, cs, tx, ty, q, acc);
+  }
+}
+
+template <bool TAIL>
 __global__ void __launch_bounds__(NTHREADS, 1)
 assign_fp32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmC,
-                   AssignArgs p) {
+                   const __grid_constant__ CUtensorMap tmXc, AssignArgs p) {
   if (stopped(p.stop)) return;
+  // rows present: a device count, or the rows selected by their distance bounds (the compact copy
+  // of the listed rows, or all rows when more than its capacity are listed)
+  long long n_rows = p.n;
+  bool compact = false;
+  if (p.n_dev) {
+    const long long c = *p.n_dev;
+    n_rows = c < p.n ? c : p.n;
+  }
+  if (p.sel) {
+    const int c = *p.sel;
+    compact = c <= p.sel_cap;
+    if (compact) n_rows = c;
+  }
+  if ((long long)blockIdx.x * BM >= n_rows) return;  // uniform over the CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -71,7 +124,7 @@ assign_fp32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t dst = smem_u32(smem + stage * STAGE_BYTES);
     const uint32_t bar = smem_u32(&full_bar[stage]);
     mbar_arrive_expect_tx(bar, STAGE_BYTES);
-    tma_load_2d(dst, &tmX, bar, kb * BKF, (int)row0);
+    tma_load_2d(dst, compact ? &tmXc : &tmX, bar, kb * BKF, (int)row0);
     tma_load_2d(dst + TILE_BYTES, &tmC, bar, kb * BKF, chunk * BN);
   };
 
@@ -82,7 +135,7 @@ assign_fp32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       mbar_init(smem_u32(&empty_bar[s]), NTHREADS / 32);
     }
     fence_mbar_init();
-    prefetch_tmap(&tmX);
+    prefetch_tmap(compact ? &tmXc : &tmX);
     prefetch_tmap(&tmC);
   }
   __syncthreads();
@@ -123,24 +176,7 @@ assign_fp32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       }
       const uint8_t* xs = smem + stage * STAGE_BYTES;
       const uint8_t* cs = xs + TILE_BYTES;
-#pragma unroll
-      for (int q = 0; q < BKF / 4; ++q) {
-        float4 cv[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          cv[j] = *reinterpret_cast<const float4*>(cs + swz128(tx + 16 * j, q));
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float4 xv = *reinterpret_cast<const float4*>(xs + swz128(ty + 16 * i, q));
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            acc[i][j] = fmaf(xv.x, cv[j].x, acc[i][j]);
-            acc[i][j] = fmaf(xv.y, cv[j].y, acc[i][j]);
-            acc[i][j] = fmaf(xv.z, cv[j].z, acc[i][j]);
-            acc[i][j] = fmaf(xv.w, cv[j].w, acc[i][j]);
-          }
-        }
-      }
+      tile_block<TAIL>(xs, cs, tx, ty, p.d - kb * BKF, acc);
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&empty_bar[stage]));
       if (tid < 32) {  // warp 0: thread 0 refills the stage once every warp released it
@@ -200,13 +236,24 @@ assign_fp32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const float cm = p.certify ? __ldg(p.cmax) : 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const long long pt = row0 + ty + 16 * i;
-      if (pt < p.n) {
+      const long long row = row0 + ty + 16 * i;
+      if (row < n_rows) {
+        const long long pt = compact ? (long long)__ldg(p.row_map + row) : row;
         p.labels[pt] = i1[i] < 0 ? 0 : i1[i];
         if (p.certify) {
-          const float e = bound_e(__ldg(p.xnorm + pt), cm, p.gamma, p.d);
+          const float xn = __ldg(p.xnorm + pt);
+          const float e = bound_e(xn, cm, p.gamma, p.d);
           const float margin = b2[i] - b1[i];
-          if (!(margin > 2.0f * e)) {
+          const bool flagged = !(margin > 2.0f * e);
+          if (p.ub) {
+            // d^2 = ||x||^2 + value, ||x||^2 in [xn^2 (1 - 2^-19), xn^2], every value within e
+            const float t1 = __fadd_ru(__fadd_ru(b1[i], e), __fmul_ru(xn, xn));
+            const float t2 = __fadd_rd(__fsub_rd(b2[i], e),
+                                       __fmul_rd(__fmul_rd(xn, xn), 1.0f - 0x1p-19f));
+            p.ub[pt] = flagged ? INFINITY : __fsqrt_ru(fmaxf(t1, 0.0f));
+            p.lb[pt] = flagged || !(t2 > 0.0f) ? 0.0f : __fsqrt_rd(t2);
+          }
+          if (flagged) {
             const int slot = atomicAdd(p.rerank_count, 1);
             p.rerank_list[slot] = (int)pt;
           }
@@ -328,24 +375,7 @@ assign_fp32_grouped_kernel(const __grid_constant__ CUtensorMap tmX,
         }
         const uint8_t* xs = smem + stage * STAGE_BYTES;
         const uint8_t* cs = xs + TILE_BYTES;
-#pragma unroll
-        for (int q = 0; q < BKF / 4; ++q) {
-          float4 cv[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            cv[j] = *reinterpret_cast<const float4*>(cs + swz128(tx + 16 * j, q));
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 xv = *reinterpret_cast<const float4*>(xs + swz128(ty + 16 * i, q));
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              acc[i][j] = fmaf(xv.x, cv[j].x, acc[i][j]);
-              acc[i][j] = fmaf(xv.y, cv[j].y, acc[i][j]);
-              acc[i][j] = fmaf(xv.z, cv[j].z, acc[i][j]);
-              acc[i][j] = fmaf(xv.w, cv[j].w, acc[i][j]);
-            }
-          }
-        }
+        tile_block<false>(xs, cs, tx, ty, p.d - kb * BKF, acc);
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&empty_bar[stage]));
         if (tid < 32) {  // warp 0: thread 0 refills the stage once every warp released it
@@ -439,13 +469,23 @@ cudaError_t launch_assign_fp32(const float* X, long long ldx, const float* Cop, 
                                   (uint64_t)a.k, (uint64_t)ldc * 4, BKF, BN));
   static bool attr_set = false;
   if (!attr_set) {
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(assign_fp32_kernel,
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(assign_fp32_kernel<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)SMEM_BYTES));
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(assign_fp32_kernel<true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)SMEM_BYTES));
     KMGB_CUDA_TRY(cudaFuncSetAttribute(assign_fp32_grouped_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)SMEM_BYTES));
     attr_set = true;
+  }
+  CUtensorMap tmXc = tmX;
+  if (a.sel) {
+    if (grp || !a.Xc || !a.row_map || a.sel_cap <= 0 || (reinterpret_cast<uintptr_t>(a.Xc) & 15))
+      return cudaErrorInvalidValue;
+    KMGB_CUDA_TRY(kmgb_make_tmap_2d(&tmXc, a.Xc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)a.d,
+                                    (uint64_t)a.sel_cap, (uint64_t)ldx * 4, BKF, BM));
   }
   if (grp) {
     if (tiles <= 0) return cudaSuccess;
@@ -459,7 +499,11 @@ cudaError_t launch_assign_fp32(const float* X, long long ldx, const float* Cop, 
   } else {
     const long long grid = (a.n + BM - 1) / BM;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    assign_fp32_kernel<<<(unsigned)grid, NTHREADS, SMEM_BYTES, s>>>(tmX, tmC, a);
+    const int tail = a.d % BKF;
+    if (tail > 0 && tail <= BKF - 4)
+      assign_fp32_kernel<true><<<(unsigned)grid, NTHREADS, SMEM_BYTES, s>>>(tmX, tmC, tmXc, a);
+    else
+      assign_fp32_kernel<false><<<(unsigned)grid, NTHREADS, SMEM_BYTES, s>>>(tmX, tmC, tmXc, a);
   }
   kmgb::count_launches(1);
   return cudaGetLastError();

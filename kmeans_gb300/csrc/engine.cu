@@ -209,7 +209,9 @@ struct kmgb_handle {
   void* XlC = nullptr;
   int* cand = nullptr;
   int* cand_cnt = nullptr;
-  long long cand_cap = 0;  // rows of the compact buffers for the candidate pass
+  long long cand_cap = 0;  // rows of the compact buffers for the candidate pass; FP32 tier: slots
+                           // of the band's candidates (0: none, the exact stage takes every row)
+  float* rr_hi3 = nullptr;  // FP32 tier: band ends of the rows left in rr_over
   unsigned long long* rr_stats = nullptr;
   // audit of certified labels: sampled rows per iteration against the FP64 arg-min
   // (launch_audit_labels; 0 rows: off)
@@ -326,19 +328,23 @@ int audit_rows_for(const kmgb_options& o, bool streaming, int k, int d) {
 // centers against themselves (k rows), the pass over the bounds (20 bytes a row) and three more
 // launches, ~25 us in all at 900,000 x 128, K=256, where the scan takes 80 us. On GB300, 10
 // iterations of 4M x 128, K=1024 from sampled centers: 25.9 -> 17.8 ms.
+// The FP32 tier's scan takes some 20 times as long: 796,160 x 324, K=256, 10 iterations 49.9 -> XX ms.
 constexpr long long kPruneMinWork = 1LL << 33;  // rows x centers (in chunks of 256) x dimensions
+constexpr long long kPruneMinWorkFp32 = 1LL << 30;
 constexpr long long kPruneMaxBytes = 8LL << 30;  // of the compact copy
 
 bool prune_wanted(const kmgb_options& o, bool mini, bool streaming, long long n, int d, int k) {
-  if (o.assign_tier != KMGB_ASSIGN_BF16 && o.assign_tier != KMGB_ASSIGN_BF16X3) return false;
+  if (o.assign_tier == KMGB_ASSIGN_FP8) return false;
   if (!o.certify || mini || streaming || o.router || k < 2) return false;
-  return n * round_up(k, kCenterPad) >= kPruneMinWork / d && (long long)k * 32 <= n;
+  const long long least = o.assign_tier == KMGB_ASSIGN_FP32 ? kPruneMinWorkFp32 : kPruneMinWork;
+  return n * round_up(k, kCenterPad) >= least / d && (long long)k * 32 <= n;
 }
 
 // The bounds' buffers, from the pool. They are an optimisation: where they do not fit, the handle
 // scans every row in every iteration.
 void alloc_prune(kmgb_handle* h, bool split) {
-  const long long row = h->ldb * 2 * (split ? 2 : 1);
+  const bool tc = h->opt.assign_tier != KMGB_ASSIGN_FP32;
+  const long long row = tc ? h->ldb * 2 * (split ? 2 : 1) : h->ldx * 4;
   PruneState p;
   p.n = h->n;
   p.k = h->k;
@@ -360,7 +366,7 @@ void alloc_prune(kmgb_handle* h, bool split) {
     a.take(&p.dirty, p.k);
     a.take(&p.flags, 4);
     a.take(&p.top, 2);
-    a.take_bytes(&p.Xc, (size_t)p.cap * h->ldb * 2);
+    a.take_bytes(&p.Xc, (size_t)p.cap * (tc ? h->ldb * 2 : h->ldx * 4));
     if (split) a.take_bytes(&p.Xlc, (size_t)p.cap * h->ldb * 2);
   };
   Arena sizing;
@@ -468,6 +474,10 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     // a third of the points can miss the certificate after the first update.)
     h->cand_cap = std::min(na, std::min<long long>(8LL << 20, std::max<long long>(1024, na / 2)));
   }
+  // FP32 tier: where thousands of rows can miss its FP32 bounds, the band's centers are recorded as
+  // candidates; on smaller data sets the two more launches cost more than the few FP64 rows
+  const bool fp32_band = !tcore && !h->streaming && h->opt.certify && na >= (1 << 16);
+  if (fp32_band) h->cand_cap = std::max<long long>(1024, na / 32);
   h->audit_rows = audit_rows_for(h->opt, h->streaming, k, d);
   UpdateWork& w = h->uw;
   w.n = na;
@@ -515,7 +525,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     if (bf16) a.take_bytes(&h->cbias, (size_t)round_up(k, kCenterPad) * kBiasCols * 2);
     a.take(&h->labels, nl);
     a.take(&h->rr_list, na);
-    a.take(&h->rr_count, 3);
+    a.take(&h->rr_count, 4);
     a.take(&h->rr_list2, na);
     a.take(&h->rr_hi2, na);
     if (tcore) {
@@ -529,6 +539,12 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
       if (split) a.take_bytes(&h->XlC, (size_t)cc * h->ldb * 2);
       a.take(&h->cand, (size_t)cc * kMaxCand);
       a.take(&h->cand_cnt, cc);
+    }
+    if (fp32_band) {
+      a.take(&h->rr_over, na);
+      a.take(&h->rr_hi3, na);
+      a.take(&h->cand, (size_t)h->cand_cap * kMaxCand);
+      a.take(&h->cand_cnt, h->cand_cap);
     }
     a.take(&h->rr_stats, 2);
     if (h->audit_rows > 0) a.take(&h->audit, 4 + 2 * (size_t)kAuditMaxRows);
@@ -826,7 +842,21 @@ int rerank_flagged(kmgb_handle* h, const AssignArgs& a, const float* Xa, const v
   r.list = h->rr_list2;
   r.count = h->rr_count + 2;
   r.stats = nullptr;
-  KM_TRY(launch_rerank_exact(r, h->rr_hi2, s), KMEANS_ERROR_CLOSEST_CENTERS);
+  const float* hi = h->rr_hi2;
+  if (!tc && h->cand_cap > 0) {  // FP32 tier: the bands' candidates first, what is left exactly
+    KM_TRY(launch_rerank_band(r, hi, h->cand, h->cand_cnt, h->cand_cap, h->rr_over, h->rr_count + 3,
+                              h->rr_hi3, s),
+           KMEANS_ERROR_CLOSEST_CENTERS);
+    KM_TRY(launch_resolve_candidates(h->rr_list2, h->rr_count + 2, h->cand_cap, h->cand,
+                                     h->cand_cnt, Xa, h->ldx, h->Cop, h->ldx, h->cn, h->d, labels,
+                                     h->rr_over, h->rr_count + 3, h->stop, s, nullptr, hi,
+                                     h->rr_hi3),
+           KMEANS_ERROR_CLOSEST_CENTERS);
+    r.list = h->rr_over;
+    r.count = h->rr_count + 3;
+    hi = h->rr_hi3;
+  }
+  KM_TRY(launch_rerank_exact(r, hi, s), KMEANS_ERROR_CLOSEST_CENTERS);
   KM_TRY(launch_count_stats(h->rr_count, tc ? 1 : 0, h->rr_stats, h->stop, s),
          KMEANS_ERROR_CLOSEST_CENTERS);
   return 0;
@@ -941,7 +971,7 @@ int router_step(kmgb_handle* h, AssignArgs a) {
 // With distance bounds: the nearest other center of every center (the centers scanned against
 // themselves as rows), then the rows whose label the moved bounds do not prove, in h->pr's list and
 // compact copy.
-int prune_rows(kmgb_handle* h, const AssignArgs& a, const void* Xba, const void* Xla) {
+int prune_rows(kmgb_handle* h, AssignArgs& a, const void* Xba, const void* Xla, bool tc) {
   cudaStream_t s = h->stream;
   PruneState& p = h->pr;
   AssignArgs c = a;
@@ -954,11 +984,19 @@ int prune_rows(kmgb_handle* h, const AssignArgs& a, const void* Xba, const void*
   c.thr_out = nullptr;
   c.ub = p.cub;
   c.lb = p.clb;
-  c.gamma = assign_bf16_gamma(h->d);
-  KM_TRY(launch_assign_bf16(h->Cb, h->Cl, h->ldb, h->Cb, h->Cl, h->ldb, c, s),
+  KM_TRY(tc ? launch_assign_bf16(h->Cb, h->Cl, h->ldb, h->Cb, h->Cl, h->ldb, c, s)
+            : launch_assign_fp32(h->Cop, h->ldx, h->Cop, h->ldx, c, s),
          KMEANS_ERROR_CLOSEST_CENTERS);
   KM_TRY(launch_prune_filter(p, h->labels, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
-  KM_TRY(launch_prune_gather(p, Xba, Xla, h->ldb * 2, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
+  KM_TRY(launch_prune_gather(p, Xba, Xla, tc ? h->ldb * 2 : h->ldx * 4, h->stop, s),
+         KMEANS_ERROR_CLOSEST_CENTERS);
+  a.ub = p.ub;
+  a.lb = p.lb;
+  a.sel = p.flags + 1;
+  a.sel_cap = p.cap;
+  a.row_map = p.list;
+  a.Xc = p.Xc;
+  a.Xlc = Xla ? p.Xlc : nullptr;
   return 0;
 }
 
@@ -996,7 +1034,7 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   KM_TRY(h->pmark(0), KMEANS_ERROR_RESET);
   // reset (kmeans.cpp:1142-1170): norms of the current centers, cleared counters
   KM_TRY(cudaMemsetAsync(h->cmax, 0, sizeof(float), s), KMEANS_ERROR_RESET);
-  KM_TRY(cudaMemsetAsync(h->rr_count, 0, 3 * sizeof(int), s), KMEANS_ERROR_RESET);
+  KM_TRY(cudaMemsetAsync(h->rr_count, 0, 4 * sizeof(int), s), KMEANS_ERROR_RESET);
   const bool prune = h->pr.n > 0 && !assign_only;
   KM_TRY(launch_prep_centers(h->C, h->ldx, h->k, h->d, h->Cop, h->Cb, h->ldb, h->cn, h->cmax, s,
                              h->stop, h->cinit, h->Cl, h->cbias, prune ? h->pr.shift : nullptr,
@@ -1076,20 +1114,17 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
     a.gamma = assign_bf16_gamma(h->d);
     a.thr_out = h->opt.certify ? h->thr_full : nullptr;
     if (prune) {
-      const int rc = prune_rows(h, a, Xba, Xla);
+      const int rc = prune_rows(h, a, Xba, Xla, true);
       if (rc) return rc;
-      a.ub = h->pr.ub;
-      a.lb = h->pr.lb;
-      a.sel = h->pr.flags + 1;
-      a.sel_cap = h->pr.cap;
-      a.row_map = h->pr.list;
-      a.Xc = h->pr.Xc;
-      a.Xlc = Xla ? h->pr.Xlc : nullptr;
     }
     KM_TRY(launch_assign_bf16(Xba, Xla, h->ldb, h->Cb, h->Cl, h->ldb, a, s),
            KMEANS_ERROR_CLOSEST_CENTERS);
   } else {
     a.gamma = assign_fp32_gamma(h->d);
+    if (prune) {
+      const int rc = prune_rows(h, a, Xa, nullptr, false);
+      if (rc) return rc;
+    }
     KM_TRY(launch_assign_fp32(Xa, h->ldx, h->Cop, h->ldx, a, s), KMEANS_ERROR_CLOSEST_CENTERS);
   }
   if (!routed) {
@@ -1161,7 +1196,7 @@ int step_stream(kmgb_handle* h, int slot) {
     if (tc)
       KM_TRY(launch_to_bf16(Xt, h->ldx, nt, h->d, h->Xb, h->ldb, s, h->stop, h->Xl),
              KMEANS_ERROR_COPY_TILE);
-    KM_TRY(cudaMemsetAsync(h->rr_count, 0, 3 * sizeof(int), s), KMEANS_ERROR_CLOSEST_CENTERS);
+    KM_TRY(cudaMemsetAsync(h->rr_count, 0, 4 * sizeof(int), s), KMEANS_ERROR_CLOSEST_CENTERS);
     int* lab = h->labels + r0;
     AssignArgs a{};
     a.cn = h->cn;

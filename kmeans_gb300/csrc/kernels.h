@@ -153,10 +153,16 @@ cudaError_t launch_rerank_grouped(const RerankArgs& a, const GroupArgs& g, cudaS
                                   long long cand_cap = 0);
 // FP64 stage over list2 (one CTA per point), candidates bounded by hi2.
 cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStream_t s);
+// The same list's FP32 bands as candidates for launch_resolve_candidates: slot i < cand_cap of the
+// list records in cand[i * kMaxCand ..], later slots go to over / over_hi (launch_rerank_exact's).
+cudaError_t launch_rerank_band(const RerankArgs& a, const float* hi2, int* cand, int* cand_cnt,
+                               long long cand_cap, int* over, int* over_count, float* over_hi,
+                               cudaStream_t s);
 // Candidate re-rank of the BF16 tiers: compact copy of up to `cap` flagged rows (the rest go to
 // `over`), then FP64 resolution of their recorded candidates (overflowing points are appended
 // to `over`). With row_map (the router's routed scan), list entries are routed rows whose
 // candidates are stored per routed row and whose FP32 row is X[row_map[entry]].
+// With hi_in / over_hi, a point passed on to `over` takes its band's upper end along.
 // row_bytes: bytes per row of Xb / Xl (a multiple of 16); xs / xsC (nullable): per-row scales
 // of the FP8 tier copied along.
 cudaError_t launch_gather_flagged(const int* list, const int* count, long long cap,
@@ -169,7 +175,8 @@ cudaError_t launch_resolve_candidates(const int* list, const int* count, long lo
                                       long long ldx, const float* C, long long ldc, const float* cn,
                                       int d, int* labels, int* over, int* over_count,
                                       const int* stop, cudaStream_t s,
-                                      const int* row_map = nullptr);
+                                      const int* row_map = nullptr, const float* hi_in = nullptr,
+                                      float* over_hi = nullptr);
 // stats[0] += counts[0] (points flagged by the assignment), stats[1] += counts[full_idx]
 // (points that needed a full rescan of the centers).
 // Audit of certified labels (rerank.cu): `rows` sampled rows (at most kAuditMaxRows) against

@@ -149,14 +149,15 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
   if (stopped(a.stop)) return;
   extern __shared__ float4 sm4[];
   const int dq = (a.d + 3) >> 2;          // float4 per row
-  const int rs = dq + 1;                  // row stride in float4 (padded: conflict-free)
+  const int rs = (dq + 1) | 1;            // row stride in float4, odd: 8 consecutive rows' columns
+                                          // lie in distinct banks
   float4* xs = sm4;                       // [TP][rs]
   float4* cs = xs + TP * rs;              // [TC][rs]
   float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] 0 usable, +inf unusable
   __shared__ float mb1[8][TP], mb2[8][TP];
   __shared__ int mi1[8][TP];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int pq = tid & 7;                 // points pq*4 .. pq*4+3
+  const int pq = tid & 7;                 // points pq, pq + 8, pq + 16, pq + 24
   const int cq = tid >> 3;                // centers cq*2, cq*2+1 of the block
   const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
   const float u = 5.9604645e-8f;
@@ -211,7 +212,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
         const float4 c1 = cs[(cq * 2 + 1) * rs + q];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float4 x = xs[(pq * 4 + i) * rs + q];
+          const float4 x = xs[(pq + 8 * i) * rs + q];
           float t;
           t = x.x - c0.x; acc[i][0] = fmaf(t, t, acc[i][0]);
           t = x.y - c0.y; acc[i][0] = fmaf(t, t, acc[i][0]);
@@ -253,9 +254,9 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
         b2[i] = nb2;
       }
       if (lane < 8) {
-        mb1[w][pq * 4 + i] = b1[i];
-        mb2[w][pq * 4 + i] = b2[i];
-        mi1[w][pq * 4 + i] = i1[i];
+        mb1[w][pq + 8 * i] = b1[i];
+        mb2[w][pq + 8 * i] = b2[i];
+        mi1[w][pq + 8 * i] = i1[i];
       }
     }
     __syncthreads();
@@ -290,22 +291,40 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
 // stage) is evaluated in FP64 in the oracle's order (sequential fma over the dimensions); the
 // smallest value wins, lowest index on ties. Centers are read once per 32 points, so the cost
 // stays that of one tiled FP32 scan however many points reach this stage.
+//
+// RECORD: instead of evaluating the pairs inside the band in FP64 (where one thread's evaluation
+// holds its whole warp on the narrow FP64 pipe), the band's centers become the candidates of
+// resolve_candidates_kernel, whose float-float tier settles nearly all of them: 796,160 x 324,
+// K=256, FP32 tier, 1.05 ms per iteration before. Slots from cand_cap on go to over / over_hi.
+template <bool RECORD>
 __global__ void __launch_bounds__(256)
-rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2) {
+rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict__ cand,
+                    int* __restrict__ cand_cnt, long long cand_cap, int* __restrict__ over,
+                    int* __restrict__ over_count, float* __restrict__ over_hi) {
   if (stopped(a.stop)) return;
   extern __shared__ float4 sm4[];
   const int dq = (a.d + 3) >> 2;
-  const int rs = dq + 1;
+  const int rs = (dq + 1) | 1;
   float4* xs = sm4;                       // [TP][rs]
   float4* cs = xs + TP * rs;              // [TC][rs]
   float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] 0 usable, +inf unusable
   __shared__ double mb[8][TP];
   __shared__ int mi[8][TP];
   __shared__ float hs[TP];
+  __shared__ int ncand[TP];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int pq = tid & 7;                 // points pq*4 .. pq*4+3
+  const int pq = tid & 7;                 // points pq, pq + 8, pq + 16, pq + 24
   const int cq = tid >> 3;                // centers cq*2, cq*2+1 of the block
-  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  if (RECORD && cnt > cand_cap) {
+    for (long long slot = cand_cap + (long long)blockIdx.x * blockDim.x + tid; slot < cnt;
+         slot += (long long)gridDim.x * blockDim.x) {
+      const int o = atomicAdd(over_count, 1);
+      over[o] = a.list[slot];
+      over_hi[o] = hi2[slot];
+    }
+    cnt = cand_cap;
+  }
   const float u = 5.9604645e-8f;
   const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;
 
@@ -324,7 +343,10 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2) {
       }
       xs[r * rs + q] = v;
     }
-    if (tid < TP) hs[tid] = (g0 + tid < cnt) ? hi2[g0 + tid] : -INFINITY;
+    if (tid < TP) {
+      hs[tid] = (g0 + tid < cnt) ? hi2[g0 + tid] : -INFINITY;
+      ncand[tid] = 0;
+    }
     double be[4];
     int bi[4];
 #pragma unroll
@@ -353,7 +375,7 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2) {
         const float4 c1 = cs[(cq * 2 + 1) * rs + q];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float4 x = xs[(pq * 4 + i) * rs + q];
+          const float4 x = xs[(pq + 8 * i) * rs + q];
           float t;
           t = x.x - c0.x; acc[i][0] = fmaf(t, t, acc[i][0]);
           t = x.y - c0.y; acc[i][0] = fmaf(t, t, acc[i][0]);
@@ -371,10 +393,15 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2) {
         const int j = j0 + cl;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int pl = pq * 4 + i;
+          const int pl = pq + 8 * i;
           if (cflag[cl] != 0.0f) continue;  // unusable (empty-cluster) or padding center
           const float v = acc[i][jj];
           if (!(v * (1.0f - gam) - 1e-30f <= hs[pl])) continue;
+          if (RECORD) {
+            const int at = atomicAdd(&ncand[pl], 1);
+            if (at < kMaxCand) cand[(g0 + pl) * kMaxCand + at] = j;
+            continue;
+          }
           // FP64 in the oracle's order: dimensions 0 .. d-1 (padding dimensions are zero)
           double ex = 0.0;
           for (int q = 0; q < dq; ++q) {
@@ -393,6 +420,11 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2) {
         }
       }
     }
+    if (RECORD) {
+      __syncthreads();
+      if (tid < TP && g0 + tid < cnt) cand_cnt[g0 + tid] = ncand[tid] <= kMaxCand ? ncand[tid] : -1;
+      continue;
+    }
     // merge the 32 threads of each point: lanes pq, pq+8, pq+16, pq+24 of every warp
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -405,8 +437,8 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2) {
         bi[i] = take ? oi : bi[i];
       }
       if (lane < 8) {
-        mb[w][pq * 4 + i] = be[i];
-        mi[w][pq * 4 + i] = bi[i];
+        mb[w][pq + 8 * i] = be[i];
+        mi[w][pq + 8 * i] = bi[i];
       }
     }
     __syncthreads();
@@ -701,7 +733,9 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
                                           const float* __restrict__ cn, int d,
                                           int* __restrict__ labels, int* __restrict__ over,
                                           int* __restrict__ over_count, const int* stop,
-                                          const int* __restrict__ row_map) {
+                                          const int* __restrict__ row_map,
+                                          const float* __restrict__ hi_in,
+                                          float* __restrict__ over_hi) {
   if (stopped(stop)) return;
   const long long cnt = min((long long)*(volatile const int*)count, max_list);
   const int lane = threadIdx.x & 31;
@@ -716,6 +750,12 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
   const double m32 = (double)((d + kGroupLanes - 1) / kGroupLanes);
   const double rel32 = 1.1 * (m32 + 8.0) * 0x1p-24 + (double)(d + 2) * 0x1p-52;
   const double abs32 = (double)(d + 32) * (m32 + 8.0) * 0x1p-149;
+  // a point this kernel cannot settle, with its band's upper end where the list carries them
+  auto to_over = [&](int pt, long long slot) {
+    const int o = atomicAdd(over_count, 1);
+    over[o] = pt;
+    if (over_hi) over_hi[o] = hi_in[slot];
+  };
   for (long long slot = w0; slot < cnt; slot += nw) {
     const int pt = list[slot];
     // with row_map (routed scan) the candidates are kept per routed row pt, and the point's FP32
@@ -723,7 +763,7 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
     const long long ci = row_map ? (long long)pt : slot;
     const int nc = cand_cnt[ci];
     if (nc <= 0 || nc > kMaxCand) {
-      if (lane == 0) over[atomicAdd(over_count, 1)] = pt;
+      if (lane == 0) to_over(pt, slot);
       continue;
     }
     const float* x = X + (size_t)(row_map ? row_map[pt] : pt) * ldx;
@@ -755,7 +795,7 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
       }
     }
     if (i1 < 0) {  // no usable candidate
-      if (lane == 0) over[atomicAdd(over_count, 1)] = pt;
+      if (lane == 0) to_over(pt, slot);
       continue;
     }
     // one usable candidate (v2 infinite, its value finite) is the arg-min itself
@@ -789,7 +829,7 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
       }
     }
     if (i1 < 0) {  // no usable candidate
-      if (lane == 0) over[atomicAdd(over_count, 1)] = pt;
+      if (lane == 0) to_over(pt, slot);
       continue;
     }
     // one usable candidate (v2 infinite, every value finite) is the arg-min itself; the
@@ -825,7 +865,7 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
       bidx = take ? oi : bidx;
     }
     if (lane == 0) {
-      if (bidx < 0) over[atomicAdd(over_count, 1)] = pt;
+      if (bidx < 0) to_over(pt, slot);
       else labels[pt] = bidx;
     }
   }
@@ -1011,18 +1051,19 @@ cudaError_t launch_resolve_candidates(const int* list, const int* count, long lo
                                       const int* cand, const int* cand_cnt, const float* X,
                                       long long ldx, const float* C, long long ldc, const float* cn,
                                       int d, int* labels, int* over, int* over_count,
-                                      const int* stop, cudaStream_t s, const int* row_map) {
+                                      const int* stop, cudaStream_t s, const int* row_map,
+                                      const float* hi_in, float* over_hi) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   const bool vec = d % 4 == 0 && ldx % 4 == 0 && ldc % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(X) % 16 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
   if (vec)
     resolve_candidates_kernel<true><<<kmgb::num_sms() * 8, 256, 0, s>>>(list, count, max_list, cand, cand_cnt,
                                                             X, ldx, C, ldc, cn, d, labels, over,
-                                                            over_count, stop, row_map);
+                                                            over_count, stop, row_map, hi_in, over_hi);
   else
     resolve_candidates_kernel<false><<<kmgb::num_sms() * 8, 256, 0, s>>>(list, count, max_list, cand, cand_cnt,
                                                              X, ldx, C, ldc, cn, d, labels, over,
-                                                             over_count, stop, row_map);
+                                                             over_count, stop, row_map, hi_in, over_hi);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1038,12 +1079,30 @@ cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStrea
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const int dq = (a.d + 3) / 4;
-  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * (dq + 1) + sizeof(float) * TC;
+  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel,
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  rerank_exact_kernel<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2);
+  rerank_exact_kernel<false><<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2, nullptr, nullptr, 0,
+                                                                    nullptr, nullptr, nullptr);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_rerank_band(const RerankArgs& a, const float* hi2, int* cand, int* cand_cnt,
+                               long long cand_cap, int* over, int* over_count, float* over_hi,
+                               cudaStream_t s) {
+  if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
+  if (a.n <= 0 || a.k <= 0) return cudaSuccess;
+  const int dq = (a.d + 3) / 4;
+  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
+  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > 48 * 1024)
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<true>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  rerank_exact_kernel<true><<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2, cand, cand_cnt, cand_cap,
+                                                                   over, over_count, over_hi);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1053,7 +1112,7 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const int dq = (a.d + 3) / 4;
-  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * (dq + 1) + sizeof(float) * TC;
+  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_tiled_kernel,

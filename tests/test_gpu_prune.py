@@ -24,6 +24,8 @@ CASES = [
     (66_003, 129, 1024, 64, 2.0, (1.0, 1.0), "BF16X3", False, 1),     # overlapping: most rows scanned
     (140_000, 256, 256, 200, 8.0, (0.5, 1.5), "BF16X3", True, 0),     # two products, NaN policy
     (132_777, 130, 500, 500, 20.0, (1.0, 1.0), "BF16", False, 1),     # plain tier
+    (90_001, 324, 300, 300, 1.0, (0.1, 0.1), "FP32", False, 1),       # FP32 tier, wide rows
+    (100_003, 45, 700, 80, 2.0, (1.0, 1.0), "FP32", False, 0),
     (600_000, 60, 250, 240, 10.0, (1.0, 1.0), "BF16X3", False, 1),
 ]
 
