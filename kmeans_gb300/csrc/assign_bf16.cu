@@ -819,7 +819,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                            1.02f * p.pert * (xn_pt * cm * 1.01f + 0.5f * cm * cm);
           const bool flagged = none || !(b1 - b2 > 2.0f * eb);
           if (kSel && p.ub) {
-            // d^2 = ||x||^2 - 2 key, ||x||^2 in [xn^2 (1 - 2^-19), xn^2] (xn: point_norms_kernel,
+            // d^2 = ||x||^2 - 2 key, ||x||^2 in [xn^2 (1 - 2^-19), xn^2] (xn: prep_rows_kernel,
             // or prep_centers_kernel's ||c||), the label's key at least b1 - E, every other
             // usable center's at most b2 + E
             const float t1 = __fmaf_ru(-2.0f, __fsub_rd(b1, eb), __fmul_ru(xn_pt, xn_pt));

@@ -328,7 +328,7 @@ int audit_rows_for(const kmgb_options& o, bool streaming, int k, int d) {
 // centers against themselves (k rows), the pass over the bounds (20 bytes a row) and three more
 // launches, ~25 us in all at 900,000 x 128, K=256, where the scan takes 80 us. On GB300, 10
 // iterations of 4M x 128, K=1024 from sampled centers: 25.9 -> 17.8 ms.
-// The FP32 tier's scan takes some 20 times as long: 796,160 x 324, K=256, 10 iterations 49.9 -> XX ms.
+// The FP32 tier's scan takes some 20 times as long: 796,160 x 324, K=256, 10 iterations 49.5 -> 20.0 ms.
 constexpr long long kPruneMinWork = 1LL << 33;  // rows x centers (in chunks of 256) x dimensions
 constexpr long long kPruneMinWorkFp32 = 1LL << 30;
 constexpr long long kPruneMaxBytes = 8LL << 30;  // of the compact copy
@@ -660,16 +660,15 @@ cudaError_t copy_rows(kmgb_handle* h, const float* X, long long r0, long long r1
 // Norms and BF16 planes of rows [r0, r1), on the handle's stream.
 cudaError_t prepare_rows(kmgb_handle* h, long long r0, long long r1) {
   const size_t xo = (size_t)r0 * h->ldx, bo = (size_t)r0 * h->ldb * 2;
-  cudaError_t r = launch_point_norms(h->X + xo, h->ldx, r1 - r0, h->d, h->qn + r0, h->xn + r0,
-                                     h->stream);
+  cudaError_t r = launch_prep_rows(h->X + xo, h->ldx, r1 - r0, h->d, h->qn + r0, h->xn + r0,
+                                   h->Xb ? static_cast<char*>(h->Xb) + bo : nullptr,
+                                   h->Xl ? static_cast<char*>(h->Xl) + bo : nullptr, h->ldb,
+                                   h->Xb ? h->xinexact : nullptr, h->stream);
   if (r == cudaSuccess && h->X8)
-    return launch_to_fp8(h->X + xo, h->ldx, r1 - r0, h->d,
-                         static_cast<char*>(h->X8) + (size_t)r0 * h->ld8, h->ld8, h->sx + r0,
-                         h->stream);
-  if (r != cudaSuccess || !h->Xb) return r;
-  return launch_to_bf16(h->X + xo, h->ldx, r1 - r0, h->d, static_cast<char*>(h->Xb) + bo,
-                        h->ldb, h->stream, nullptr,
-                        h->Xl ? static_cast<char*>(h->Xl) + bo : nullptr, h->xinexact);
+    r = launch_to_fp8(h->X + xo, h->ldx, r1 - r0, h->d,
+                      static_cast<char*>(h->X8) + (size_t)r0 * h->ld8, h->ld8, h->sx + r0,
+                      h->stream);
+  return r;
 }
 
 // The copy stream and its event; the copies that follow overwrite X only after the work queued
@@ -1022,7 +1021,8 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
                              h->stop),
            KMEANS_ERROR_CONSTRUCT_MINIBATCH);
     if (h->Xbw)
-      KM_TRY(launch_to_bf16(h->Xw, h->ldx, h->m_mb, h->d, h->Xbw, h->ldb, s, h->stop, h->Xlw),
+      KM_TRY(launch_prep_rows(h->Xw, h->ldx, h->m_mb, h->d, nullptr, nullptr, h->Xbw, h->Xlw,
+                              h->ldb, nullptr, s, h->stop),
              KMEANS_ERROR_CONSTRUCT_MINIBATCH);
     Xa = h->Xw;
     Xba = h->Xbw;
@@ -1192,10 +1192,9 @@ int step_stream(kmgb_handle* h, int slot) {
              KMEANS_ERROR_COPY_TILE);
     KM_TRY(cudaEventRecord(h->ev_copied[b], cs), KMEANS_ERROR_COPY_TILE);
     KM_TRY(cudaStreamWaitEvent(s, h->ev_copied[b], 0), KMEANS_ERROR_COPY_TILE);
-    KM_TRY(launch_point_norms(Xt, h->ldx, nt, h->d, h->qn, h->xn, s), KMEANS_ERROR_COPY_TILE);
-    if (tc)
-      KM_TRY(launch_to_bf16(Xt, h->ldx, nt, h->d, h->Xb, h->ldb, s, h->stop, h->Xl),
-             KMEANS_ERROR_COPY_TILE);
+    KM_TRY(launch_prep_rows(Xt, h->ldx, nt, h->d, h->qn, h->xn, tc ? h->Xb : nullptr,
+                            tc ? h->Xl : nullptr, h->ldb, nullptr, s, h->stop),
+           KMEANS_ERROR_COPY_TILE);
     KM_TRY(cudaMemsetAsync(h->rr_count, 0, 4 * sizeof(int), s), KMEANS_ERROR_CLOSEST_CENTERS);
     int* lab = h->labels + r0;
     AssignArgs a{};

@@ -262,16 +262,13 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   const bool tc = !mini && bf16_tc_supported(n, 2) &&
                   !(tier_env && std::strcmp(tier_env, "fp32") == 0);
   const long long ldx = (n + 3) / 4 * 4, ldb = (n + 7) / 8 * 8;
-  float *Xf = nullptr, *xn = nullptr, *Cf = nullptr, *Cop = nullptr, *cn = nullptr,
+  float *xn = nullptr, *Cf = nullptr, *Cop = nullptr, *cn = nullptr,
         *cmax = nullptr, *cinit = nullptr;
-  double* qn = nullptr;
   uint16_t *Xb = nullptr, *Xl = nullptr, *Cb = nullptr, *Cl = nullptr;
   int *rr_list = nullptr, *rr_count = nullptr, *derr = nullptr;
   if (tc) {
     const kmeansErrorStatus EA = KMEANS_ERROR_CLOSEST_CENTERS;
-    KD_TRY(B.alloc(&Xf, (size_t)m * ldx), E);
     KD_TRY(B.alloc(&xn, m), E);
-    KD_TRY(B.alloc(&qn, m), E);
     KD_TRY(B.alloc(&Xb, (size_t)m * ldb), E);
     KD_TRY(B.alloc(&Xl, (size_t)m * ldb), E);
     KD_TRY(B.alloc(&Cf, (size_t)k * ldx), E);
@@ -285,10 +282,7 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
     KD_TRY(B.alloc(&rr_count, 3), E);
     KD_TRY(B.alloc(&derr, 1), E);
     KD_TRY(cudaMemsetAsync(derr, 0, sizeof(int), s), E);
-    d2f_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(X, m, n, Xf, ldx); kmgb::count_launches(1);
-    KD_TRY(cudaGetLastError(), E);
-    KD_TRY(launch_point_norms(Xf, ldx, m, n, qn, xn, s), E);
-    KD_TRY(launch_to_bf16(Xf, ldx, m, n, Xb, ldb, s, nullptr, Xl, nullptr), EA);
+    KD_TRY(launch_prep_rows(X, n, m, n, nullptr, xn, Xb, Xl, ldb, nullptr, s), EA);
   }
 
   const int threads = 256;

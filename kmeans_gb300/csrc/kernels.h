@@ -240,9 +240,14 @@ cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const in
 cudaError_t launch_prune_gather(const PruneState& ps, const void* Xb, const void* Xl,
                                 long long row_bytes, const int* stop, cudaStream_t s);
 
-// Per-point norms, computed once per data set: qn = ||x||^2 (FP64), xn = upper bound ||x||.
-cudaError_t launch_point_norms(const float* X, long long ldx, long long n, int d, double* qn,
-                               float* xn, cudaStream_t s);
+// Rows of a data set, once: qn = ||x||^2 (FP64), xn = upper bound of ||x||, Xb / Xl = BF16 value and
+// residual planes (zero padded to ldb columns); each nullable. inexact (nullable, zeroed by the
+// caller; needs Xb) is set to 1 when some value is not a BF16 number. T = double: of the rows'
+// FP32 roundings.
+template <typename T>
+cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
+                             void* Xb, void* Xl, long long ldb, int* inexact, cudaStream_t s,
+                             const int* stop = nullptr);
 // FP8 E4M3 copies (the FP8 tier): every row of X scaled by its own power of two sx[row], the
 // centers (from the operand copy) by one power of two *cscale derived from *cmax; rows zero
 // padded to ld8 bytes (a multiple of 16).
@@ -251,13 +256,6 @@ cudaError_t launch_to_fp8(const float* X, long long ldx, long long n, int d, voi
 cudaError_t launch_centers_fp8(const float* Cop, long long ldc, int k, int d, const float* cmax,
                                void* C8, long long ld8, float* cscale, cudaStream_t s,
                                const int* stop = nullptr);
-// BF16 copy of the data set (zero padded to ldb columns).
-// Xl (nullable) receives the residual plane bf16(x - bf16(x)); inexact (nullable, zeroed by the
-// caller) is set to 1 when some value is not a BF16 number.
-cudaError_t launch_to_bf16(const float* X, long long ldx, long long n, int d, void* Xb,
-                           long long ldb, cudaStream_t s, const int* stop = nullptr,
-                           void* Xl = nullptr, int* inexact = nullptr);
-
 // Deterministic update: stable counting sort by label, FP64 piece sums, finalize.
 struct UpdateWork {
   // sizes

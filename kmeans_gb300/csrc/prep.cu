@@ -10,6 +10,8 @@
 
 #include <cuda_fp8.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -114,77 +116,137 @@ __device__ __forceinline__ void ff_two_sum(float a, float b, float& s, float& e)
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
 }
 
-// One warp per point: qn = ||x||^2 (FP64), xn = FP32 upper bound of ||x||. GB300's FP64 pipe is
-// narrow, so the sum runs on the FP32 pipe as an error-free float-float value: exact squares
-// (p + e by FMA), TwoSum accumulation per lane, a float-float tree over the warp, and a single
-// FP64 addition per point. The float-float sum is within (d/32 + 8) 2^-46 of ||x||^2 relative;
-// xn adds 2^-20 before its upward-rounded square root. Rows whose squares leave the FP32 range
-// are summed in FP64 instead.
-__global__ void point_norms_kernel(const float* __restrict__ X, long long ldx, long long n, int d,
-                                   double* __restrict__ qn, float* __restrict__ xn) {
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= n) return;
-  const float* x = X + (size_t)warp * ldx;
-  float hi = 0.0f, lo = 0.0f;
-  for (int t = lane; t < d; t += 32) {
-    const float v = __ldg(x + t);
-    const float p = __fmul_rn(v, v);
-    const float e = __fmaf_rn(v, v, -p);  // v*v - p exactly
-    float s1, err;
-    ff_two_sum(hi, p, s1, err);
-    hi = s1;
-    lo = __fadd_rn(lo, __fadd_rn(err, e));
+// Everything an iteration needs of a row, from one read of it: qn = ||x||^2 (FP64), xn = FP32 upper
+// bound of ||x||, the BF16 value plane and its residual plane bf16(x - bf16(x)) (each nullable).
+// GB300's FP64 pipe is narrow, so the norm runs on the FP32 pipe as an error-free float-float value:
+// exact squares (p + e by FMA), TwoSum accumulation per lane, a float-float tree over the lanes, and
+// a single FP64 addition per row; it is within (d/32 + 8) 2^-46 of ||x||^2 relative, and xn adds
+// 2^-20 before its upward-rounded square root. Rows whose squares leave the FP32 range are summed
+// in FP64 instead. inexact (nullable): set to 1 when some value is not a BF16 number (v != bf16(v);
+// NaN included), i.e. when the residual plane carries information.
+//
+// Bound by HBM: 4 bytes read and 4 written per element. L lanes share a row, each with 16 bytes of
+// it at a time (L = 32 from 68 dimensions on, fewer below, so that a warp's lanes are all busy and
+// its loads contiguous), and a warp takes two row groups at a time. One pass per kind of output with
+// a warp and 4 bytes a lane per row took 153 + 69 us for 898,790 x 128 (norms, one plane pair);
+// T = double: the FP32 roundings of FP64 rows (row stride ldx doubles, read element by element
+// unless rows are 16-byte aligned).
+template <typename T>
+__device__ __forceinline__ float4 load_row4(const T* __restrict__ x, int c, int d, bool vec) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (sizeof(T) == 4) {
+    if (vec && c + 4 <= d) return __ldg(reinterpret_cast<const float4*>(x + c));
+  } else if (vec && c + 4 <= d) {
+    const double2 a = __ldg(reinterpret_cast<const double2*>(x + c));
+    const double2 b = __ldg(reinterpret_cast<const double2*>(x + c + 2));
+    return make_float4(__double2float_rn(a.x), __double2float_rn(a.y), __double2float_rn(b.x),
+                       __double2float_rn(b.y));
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
-    const float ol = __shfl_xor_sync(0xffffffffu, lo, o);
-    float s1, err;
-    ff_two_sum(hi, oh, s1, err);
-    hi = s1;
-    lo = __fadd_rn(lo, __fadd_rn(ol, err));
-  }
-  if (!(fabsf(hi) < 1.0e37f)) {  // overflow (or NaN input): FP64 sum, same for every lane
-    double sd = 0.0;
-    for (int t = lane; t < d; t += 32) {
-      const double v = (double)__ldg(x + t);
-      sd = fma(v, v, sd);
-    }
-    for (int o = 16; o > 0; o >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, o);
-    if (lane == 0) {
-      if (qn) qn[warp] = sd;
-      if (xn) xn[warp] = __double2float_ru(sqrt(sd) * (1.0 + 1e-12));
-    }
-    return;
-  }
-  if (lane == 0) {
-    if (qn) qn[warp] = (double)hi + (double)lo;
-    if (xn) xn[warp] = __fsqrt_ru(__fmul_ru(__fadd_ru(hi, fabsf(lo)), 1.0f + 0x1p-20f));
-  }
+  if (c < d) v.x = (float)__ldg(x + c);
+  if (c + 1 < d) v.y = (float)__ldg(x + c + 1);
+  if (c + 2 < d) v.z = (float)__ldg(x + c + 2);
+  if (c + 3 < d) v.w = (float)__ldg(x + c + 3);
+  return v;
 }
 
-// One warp per row (grid-stride over rows): BF16 value plane and, when requested, the BF16
-// residual plane bf16(x - bf16(x)).
-// inexact (nullable): set to 1 when some value of X is not a BF16 number (v != bf16(v); NaN
-// included), i.e. when the residual plane carries information.
-__global__ void to_bf16_kernel(const float* __restrict__ X, long long ldx, long long n, int d,
-                               __nv_bfloat16* __restrict__ Xb, long long ldb, const int* stop,
-                               __nv_bfloat16* __restrict__ Xl, int* inexact) {
+__device__ __forceinline__ void ff_square_add(float v, float& hi, float& lo) {
+  const float p = __fmul_rn(v, v);
+  const float e = __fmaf_rn(v, v, -p);  // v*v - p exactly
+  float s, err;
+  ff_two_sum(hi, p, s, err);
+  hi = s;
+  lo = __fadd_rn(lo, __fadd_rn(err, e));
+}
+
+__device__ __forceinline__ uint2 bf16x4(float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+// the values of the four BF16 numbers
+__device__ __forceinline__ float4 widen4(uint2 b) {
+  return make_float4(__uint_as_float(b.x << 16), __uint_as_float(b.x & 0xFFFF0000u),
+                     __uint_as_float(b.y << 16), __uint_as_float(b.y & 0xFFFF0000u));
+}
+
+template <typename T, int L>
+__global__ void __launch_bounds__(256)
+prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, bool vec,
+                 double* __restrict__ qn, float* __restrict__ xn, uint2* __restrict__ Xb,
+                 uint2* __restrict__ Xl, int ldb, int* inexact, const int* stop) {
   if (stopped(stop)) return;
-  const int lane = threadIdx.x & 31;
+  constexpr int G = 32 / L;  // rows per warp and step
+  constexpr int U = 2;       // steps in flight
+  const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int ldb4 = ldb / 4;
+  const int width = Xb ? ldb : d;  // planes are written with their zero padding
+  const bool norms = qn || xn;
   bool off = false;
-  for (long long r = w0; r < n; r += nw) {
-    const float* x = X + (size_t)r * ldx;
-    __nv_bfloat16* ob = Xb + (size_t)r * ldb;
-    __nv_bfloat16* ol = Xl ? Xl + (size_t)r * ldb : nullptr;
-    for (int c = lane; c < (int)ldb; c += 32) {
-      const float v = c < d ? __ldg(x + c) : 0.0f;
-      const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-      ob[c] = hi;
-      off |= !(v == __bfloat162float(hi));
-      if (ol) ol[c] = __float2bfloat16_rn(v - __bfloat162float(hi));
+  for (long long r0 = w0 * G * U; r0 < n; r0 += nw * G * U) {
+    float hi[U], lo[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) hi[u] = lo[u] = 0.0f;
+    for (int c = 4 * sub; c < width; c += 4 * L) {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long r = r0 + u * G + grp;
+        v[u] = r < n ? load_row4(X + (size_t)r * ldx, c, d, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long r = r0 + u * G + grp;
+        if (norms) {
+          ff_square_add(v[u].x, hi[u], lo[u]);
+          ff_square_add(v[u].y, hi[u], lo[u]);
+          ff_square_add(v[u].z, hi[u], lo[u]);
+          ff_square_add(v[u].w, hi[u], lo[u]);
+        }
+        if (Xb && r < n) {
+          const uint2 h = bf16x4(v[u]);
+          Xb[(size_t)r * ldb4 + c / 4] = h;
+          if (Xl || inexact) {
+            const float4 hv = widen4(h);
+            off |= !(v[u].x == hv.x && v[u].y == hv.y && v[u].z == hv.z && v[u].w == hv.w);
+            if (Xl)
+              Xl[(size_t)r * ldb4 + c / 4] = bf16x4(make_float4(v[u].x - hv.x, v[u].y - hv.y,
+                                                                v[u].z - hv.z, v[u].w - hv.w));
+          }
+        }
+      }
+    }
+    if (!norms) continue;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long r = r0 + u * G + grp;
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) {
+        const float oh = __shfl_xor_sync(0xffffffffu, hi[u], o);
+        const float ol = __shfl_xor_sync(0xffffffffu, lo[u], o);
+        float s1, err;
+        ff_two_sum(hi[u], oh, s1, err);
+        hi[u] = s1;
+        lo[u] = __fadd_rn(lo[u], __fadd_rn(ol, err));
+      }
+      const bool wide = !(fabsf(hi[u]) < 1.0e37f);  // overflow (or NaN input): FP64 sum
+      if (__any_sync(0xffffffffu, wide)) {
+        double sd = 0.0;
+        if (r < n)
+          for (int t = sub; t < d; t += L) {
+            const double x = (double)(float)__ldg(X + (size_t)r * ldx + t);
+            sd = fma(x, x, sd);
+          }
+        for (int o = L / 2; o > 0; o >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, o);
+        if (wide && sub == 0 && r < n) {
+          if (qn) qn[r] = sd;
+          if (xn) xn[r] = __double2float_ru(sqrt(sd) * (1.0 + 1e-12));
+        }
+      }
+      if (!wide && sub == 0 && r < n) {
+        if (qn) qn[r] = (double)hi[u] + (double)lo[u];
+        if (xn) xn[r] = __fsqrt_ru(__fmul_ru(__fadd_ru(hi[u], fabsf(lo[u])), 1.0f + 0x1p-20f));
+      }
     }
   }
   if (inexact && __any_sync(0xffffffffu, off) && lane == 0) atomicExch(inexact, 1);
@@ -317,26 +379,36 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
   return cudaGetLastError();
 }
 
-cudaError_t launch_point_norms(const float* X, long long ldx, long long n, int d, double* qn,
-                               float* xn, cudaStream_t s) {
+template <typename T>
+cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
+                             void* Xb, void* Xl, long long ldb, int* inexact, cudaStream_t s,
+                             const int* stop) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (n <= 0) return cudaSuccess;
-  const int threads = 256;
-  const long long blocks = (n * 32 + threads - 1) / threads;
-  point_norms_kernel<<<(unsigned)blocks, threads, 0, s>>>(X, ldx, n, d, qn, xn); kmgb::count_launches(1);
+  if (Xb && (ldb % 8 || ldb < d)) return cudaErrorInvalidValue;
+  const bool vec = (ldx * sizeof(T)) % 16 == 0 && reinterpret_cast<uintptr_t>(X) % 16 == 0;
+  const int lanes = d <= 16 ? 4 : (d <= 32 ? 8 : (d <= 64 ? 16 : 32));
+  const long long steps = (n + 2 * (32 / lanes) - 1) / (2 * (32 / lanes));  // warps' worth of rows
+  const long long most = kmgb::num_sms() * 64LL;
+  const unsigned blocks = (unsigned)((steps < most ? steps : most) + 7) / 8;
+  uint2* b = static_cast<uint2*>(Xb);
+  uint2* l = static_cast<uint2*>(Xl);
+  auto go = [&](auto tag) {
+    prep_rows_kernel<T, decltype(tag)::value><<<blocks, 256, 0, s>>>(X, ldx, n, d, vec, qn, xn, b, l,
+                                                                     (int)ldb, inexact, stop);
+  };
+  if (lanes == 4) go(std::integral_constant<int, 4>{});
+  else if (lanes == 8) go(std::integral_constant<int, 8>{});
+  else if (lanes == 16) go(std::integral_constant<int, 16>{});
+  else go(std::integral_constant<int, 32>{});
+  kmgb::count_launches(1);
   return cudaGetLastError();
 }
-
-cudaError_t launch_to_bf16(const float* X, long long ldx, long long n, int d, void* Xb,
-                           long long ldb, cudaStream_t s, const int* stop, void* Xl,
-                           int* inexact) {
-  if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
-  if (n <= 0) return cudaSuccess;
-  to_bf16_kernel<<<kmgb::num_sms() * 16, 256, 0, s>>>(X, ldx, n, d, reinterpret_cast<__nv_bfloat16*>(Xb),
-                                          ldb, stop, reinterpret_cast<__nv_bfloat16*>(Xl),
-                                          inexact); kmgb::count_launches(1);
-  return cudaGetLastError();
-}
+template cudaError_t launch_prep_rows<float>(const float*, long long, long long, int, double*, float*,
+                                             void*, void*, long long, int*, cudaStream_t, const int*);
+template cudaError_t launch_prep_rows<double>(const double*, long long, long long, int, double*,
+                                              float*, void*, void*, long long, int*, cudaStream_t,
+                                              const int*);
 
 cudaError_t launch_gather_rows(const float* Xsrc, long long ldx, const int* perm, long long m,
                                long long start, long long m_mb, int d, float* Xdst, long long ldd,

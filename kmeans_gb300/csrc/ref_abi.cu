@@ -363,7 +363,7 @@ kmeansCudaErrorStatus ClosestCentersF(const int m0, const int nRowsA, const int 
     transpose_centers_kernel<float><<<kmgb::num_sms() * 4, 256, 0, kDefault>>>(B, d, k, Bt, ld); kmgb::count_launches(1);
     e = cudaGetLastError();
   }
-  if (!e) e = launch_point_norms(Xa, ld, nRowsA, d, nullptr, xn, kDefault);
+  if (!e) e = launch_prep_rows(Xa, ld, nRowsA, d, nullptr, xn, nullptr, nullptr, 0, nullptr, kDefault);
   if (!e) {
     cmax_expansion_kernel<<<(k * 32 + 255) / 256, 256, 0, kDefault>>>(Bt, ld, k, d,
                                                                      normColsOfB_squared, cmax); kmgb::count_launches(1);
