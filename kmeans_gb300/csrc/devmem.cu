@@ -96,7 +96,7 @@ int num_sms() {
   return v;
 }
 
-cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s) {
+cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
   if (inject_fault(kFaultAlloc)) return cudaErrorMemoryAllocation;
   if (bytes == 0) bytes = 1;
@@ -111,10 +111,13 @@ cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s) {
     cudaMemPoolTrimTo(pool, 0);
     r = cudaMallocFromPoolAsync(p, bytes, pool, s);
   }
-  if (r != cudaSuccess) {
-    *p = nullptr;
-    return r;
-  }
+  if (r != cudaSuccess) *p = nullptr;
+  return r;
+}
+
+cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s) {
+  const cudaError_t r = dev_alloc_async(p, bytes, s);
+  if (r != cudaSuccess) return r;
   // usable from every stream (copies on the legacy stream, a handle's copy stream) at once
   return cudaStreamSynchronize(s);
 }

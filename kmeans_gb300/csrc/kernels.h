@@ -138,8 +138,11 @@ struct RerankArgs {
   long long max_list;
   const int* stop;
 };
+// Any dimension; one warp per point, both modes.
 cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t s);
-// FP32 stage of the Lloyd re-rank (mode 0): certifies what FP32 can, passes the rest to list2.
+// Whether the tiled stages below take this dimension (their tiles stay in shared memory).
+bool rerank_tiled_supported(int d);
+// FP32 stage of the re-rank, both modes: certifies what FP32 can, passes the rest to list2.
 // hi2[slot] receives the FP32 upper end of the best center of every point passed on.
 cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, float* hi2,
                                 cudaStream_t s);
@@ -192,6 +195,25 @@ cudaError_t launch_audit_labels(const float* X, long long ldx, long long n, int 
 cudaError_t launch_count_stats(const int* counts, int full_idx, unsigned long long* stats,
                                const int* stop, cudaStream_t s);
 
+// Settles flagged points of the expansion form (value nb_j - 2 x.c_j, FP64 arg-min, lowest index on
+// ties) from their recorded candidates: float-float dot products, exact FP64 where they cannot
+// separate the two best; points without a usable record go to `over`.
+cudaError_t launch_resolve_expansion(const RerankArgs& a, const int* cand, const int* cand_cnt,
+                                     int* over, int* over_count, cudaStream_t s);
+// The same for FP64 data, always exactly: mode 0 sum_t (x_t - c_t)^2, mode 1 nb_j - 2 x.c_j, each
+// one sequential FMA chain; element t of center j is C[t * c_dim + j * c_row].
+struct ResolveD {
+  const double* X; long long ldx;
+  const double* C; long long c_dim; long long c_row;
+  const double* nb;
+  int d; int k; int mode;
+  const int* list; const int* count; long long max_list;
+  const int* cand; const int* cand_cnt;
+  int* labels;
+  int* over; int* over_count;
+};
+cudaError_t launch_resolve_fp64(const ResolveD& a, cudaStream_t s);
+
 // Center preparation: from the official centers C[k][ldc] write the operand copy Cop (NaN
 // rows -> 0), optional BF16 copy Cb[k][ldcb], cn (+inf for NaN rows) and atomically raise
 // *cmax (must be zeroed before).
@@ -240,14 +262,34 @@ cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const in
 cudaError_t launch_prune_gather(const PruneState& ps, const void* Xb, const void* Xl,
                                 long long row_bytes, const int* stop, cudaStream_t s);
 
+// Centers of the expansion form: B is d x k (centers are columns), nb their norms. See
+// prep_expansion_kernel; Cb, Cl, cinit and cbias together or null.
+template <typename T>
+cudaError_t launch_prep_expansion(const T* B, int d, int k, const T* nb, float* Bt, long long ld,
+                                  float* nbx, void* Cb, void* Cl, long long ldb, float* cinit,
+                                  void* cbias, float* cmax, cudaStream_t s);
+
 // Rows of a data set, once: qn = ||x||^2 (FP64), xn = upper bound of ||x||, Xb / Xl = BF16 value and
 // residual planes (zero padded to ldb columns); each nullable. inexact (nullable, zeroed by the
 // caller; needs Xb) is set to 1 when some value is not a BF16 number. T = double: of the rows'
 // FP32 roundings.
+// With rl: the rows X[rl.list[i]], i < min(*rl.count, n), into output row i, with their floors
+// thr_out[i] = thr[list[i]]; entries from n on are appended to rl.over.
+struct RowList {
+  const int* list;
+  const int* count;
+  const float* thr;
+  float* thr_out;
+  int* over;
+  int* over_count;
+};
 template <typename T>
 cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
                              void* Xb, void* Xl, long long ldb, int* inexact, cudaStream_t s,
-                             const int* stop = nullptr);
+                             const int* stop = nullptr, const RowList* rl = nullptr);
+// ||x||^2 of every row, rounded once to FP32.
+cudaError_t launch_row_norms(const float* X, long long ldx, long long n, int d, float* out,
+                             cudaStream_t s);
 // FP8 E4M3 copies (the FP8 tier): every row of X scaled by its own power of two sx[row], the
 // centers (from the operand copy) by one power of two *cscale derived from *cmax; rows zero
 // padded to ld8 bytes (a multiple of 16).
@@ -393,6 +435,8 @@ void test_wait_hook(long long* withhold, unsigned long long* wait_cycles);
 // Device memory from the library's stream-ordered pool of the current device (devmem.cu):
 // dev_alloc returns memory usable from every stream; dev_free gives it back in the order of s.
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s);
+// The same without waiting for s: memory for work queued on s after the call.
+cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
 cudaError_t dev_release_cached();
 

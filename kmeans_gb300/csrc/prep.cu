@@ -168,12 +168,28 @@ __device__ __forceinline__ float4 widen4(uint2 b) {
                      __uint_as_float(b.y << 16), __uint_as_float(b.y & 0xFFFF0000u));
 }
 
-template <typename T, int L>
+//
+// IDX 1: the rows of a device list (RowList): output row i is row list[i]; entries past the capacity
+// go to over.
+template <typename T, int L, int IDX>
 __global__ void __launch_bounds__(256)
 prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, bool vec,
                  double* __restrict__ qn, float* __restrict__ xn, uint2* __restrict__ Xb,
-                 uint2* __restrict__ Xl, int ldb, int* inexact, const int* stop) {
+                 uint2* __restrict__ Xl, int ldb, int* inexact, float* __restrict__ nf, RowList rl,
+                 const int* stop) {
   if (stopped(stop)) return;
+  if (IDX == 1) {
+    const long long total = *reinterpret_cast<volatile const int*>(rl.count);
+    const long long cap = n;
+    n = total < cap ? total : cap;
+    for (long long i = cap + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x)
+      rl.over[atomicAdd(rl.over_count, 1)] = rl.list[i];
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long long)gridDim.x * blockDim.x)
+      rl.thr_out[i] = rl.thr[rl.list[i]];
+  }
+  auto source = [&](long long r) { return IDX == 1 ? (long long)__ldg(rl.list + r) : r; };
   constexpr int G = 32 / L;  // rows per warp and step
   constexpr int U = 2;       // steps in flight
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
@@ -181,7 +197,7 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
   const int ldb4 = ldb / 4;
   const int width = Xb ? ldb : d;  // planes are written with their zero padding
-  const bool norms = qn || xn;
+  const bool norms = qn || xn || nf;
   bool off = false;
   for (long long r0 = w0 * G * U; r0 < n; r0 += nw * G * U) {
     float hi[U], lo[U];
@@ -192,7 +208,7 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const long long r = r0 + u * G + grp;
-        v[u] = r < n ? load_row4(X + (size_t)r * ldx, c, d, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[u] = r < n ? load_row4(X + (size_t)source(r) * ldx, c, d, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -229,27 +245,86 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
         hi[u] = s1;
         lo[u] = __fadd_rn(lo[u], __fadd_rn(ol, err));
       }
-      const bool wide = !(fabsf(hi[u]) < 1.0e37f);  // overflow (or NaN input): FP64 sum
+      // overflow (or NaN input): FP64 sum; for the rounded norm also where squares near the
+      // subnormals lose their low parts
+      const bool wide = !(fabsf(hi[u]) < 1.0e37f) || (nf && hi[u] < 1.0e-24f);
       if (__any_sync(0xffffffffu, wide)) {
         double sd = 0.0;
         if (r < n)
           for (int t = sub; t < d; t += L) {
-            const double x = (double)(float)__ldg(X + (size_t)r * ldx + t);
+            const double x = (double)(float)__ldg(X + (size_t)source(r) * ldx + t);
             sd = fma(x, x, sd);
           }
         for (int o = L / 2; o > 0; o >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, o);
         if (wide && sub == 0 && r < n) {
           if (qn) qn[r] = sd;
+          if (nf) nf[r] = __double2float_rn(sd);
           if (xn) xn[r] = __double2float_ru(sqrt(sd) * (1.0 + 1e-12));
         }
       }
       if (!wide && sub == 0 && r < n) {
         if (qn) qn[r] = (double)hi[u] + (double)lo[u];
+        if (nf) nf[r] = __fadd_rn(hi[u], lo[u]);
         if (xn) xn[r] = __fsqrt_ru(__fmul_ru(__fadd_ru(hi[u], fabsf(lo[u])), 1.0f + 0x1p-20f));
       }
     }
   }
   if (inexact && __any_sync(0xffffffffu, off) && lane == 0) atomicExch(inexact, 1);
+}
+
+// Centers of the expansion form (per-kernel ABI: B is d x k, centers are columns, with the caller's
+// norms nb): one warp per center writes the row-major FP32 copy Bt, nbx = the norm or +inf where the
+// center can never win (a NaN anywhere, a norm of +inf), the BF16 planes and the start values -nb/2
+// (nullable), and raises *cmax >= max(||c||, sqrt|nb|). A center whose value no bound covers
+// (infinite elements, a norm of -inf, magnitudes beyond 1e18) raises it to 3e38: every row then
+// misses its certificate and is settled exactly.
+template <typename T>
+__global__ void prep_expansion_kernel(const T* __restrict__ B, int d, int k, const T* __restrict__ nb,
+                                      float* __restrict__ Bt, long long ld, float* __restrict__ nbx,
+                                      __nv_bfloat16* __restrict__ Cb, __nv_bfloat16* __restrict__ Cl,
+                                      long long ldb, float* __restrict__ cinit,
+                                      __nv_bfloat16* __restrict__ cbias, int kpad, float* cmax) {
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (j >= kpad) return;
+  float start = -3.0e38f;
+  if (j < k) {
+    double s = 0.0;
+    bool nan = false, wide = false;
+    for (int t = lane; t < d; t += 32) {
+      const T v = B[(size_t)t * k + j];
+      nan |= v != v;
+      wide |= !(fabs((double)v) < 1e18);
+      s = fma((double)v, (double)v, s);
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const T n = nb[j];
+    nan = __any_sync(0xffffffffu, nan) || n != n;
+    wide = __any_sync(0xffffffffu, wide);
+    const bool never = nan || (!wide && n > T(0) && !(n < (T)INFINITY));
+    const bool force = !never && (wide || !(fabs((double)n) < 1e36));
+    const bool zero = never || force;
+    for (int t = lane; t < (int)ld; t += 32)
+      Bt[(size_t)j * ld + t] = (never || t >= d) ? 0.0f : (float)B[(size_t)t * k + j];
+    if (Cb)
+      for (int t = lane; t < (int)ldb; t += 32) {
+        const float v = (zero || t >= d) ? 0.0f : (float)B[(size_t)t * k + j];
+        const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+        Cb[(size_t)j * ldb + t] = hi;
+        Cl[(size_t)j * ldb + t] = __float2bfloat16_rn(v - __bfloat162float(hi));
+      }
+    if (!zero) start = -0.5f * (float)n;
+    if (lane == 0) {
+      nbx[j] = never ? INFINITY : (float)n;
+      if (!never) {
+        const float up = force ? 3.0e38f
+                               : __double2float_ru(sqrt(fmax(s, fabs((double)n))) * (1.0 + 1e-12));
+        atomicMax(reinterpret_cast<int*>(cmax), __float_as_int(up));
+      }
+    }
+  }
+  if (cinit && lane == 0) cinit[j] = start;
+  if (cbias) write_bias_row(cbias + (size_t)j * kBiasCols, start, lane);
 }
 
 __global__ void gather_rows_kernel(const float* __restrict__ Xs, long long ldx,
@@ -380,9 +455,9 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
 }
 
 template <typename T>
-cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
-                             void* Xb, void* Xl, long long ldb, int* inexact, cudaStream_t s,
-                             const int* stop) {
+static cudaError_t prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
+                             void* Xb, void* Xl, long long ldb, int* inexact, float* nf,
+                             cudaStream_t s, const int* stop, const RowList* rl) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (n <= 0) return cudaSuccess;
   if (Xb && (ldb % 8 || ldb < d)) return cudaErrorInvalidValue;
@@ -394,8 +469,12 @@ cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, doub
   uint2* b = static_cast<uint2*>(Xb);
   uint2* l = static_cast<uint2*>(Xl);
   auto go = [&](auto tag) {
-    prep_rows_kernel<T, decltype(tag)::value><<<blocks, 256, 0, s>>>(X, ldx, n, d, vec, qn, xn, b, l,
-                                                                     (int)ldb, inexact, stop);
+    if (rl)
+      prep_rows_kernel<T, decltype(tag)::value, 1><<<blocks, 256, 0, s>>>(
+          X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nullptr, *rl, stop);
+    else
+      prep_rows_kernel<T, decltype(tag)::value, 0><<<blocks, 256, 0, s>>>(
+          X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nf, RowList{}, stop);
   };
   if (lanes == 4) go(std::integral_constant<int, 4>{});
   else if (lanes == 8) go(std::integral_constant<int, 8>{});
@@ -404,11 +483,43 @@ cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, doub
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
+template <typename T>
+cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
+                             void* Xb, void* Xl, long long ldb, int* inexact, cudaStream_t s,
+                             const int* stop, const RowList* rl) {
+  return prep_rows<T>(X, ldx, n, d, qn, xn, Xb, Xl, ldb, inexact, nullptr, s, stop, rl);
+}
+
+cudaError_t launch_row_norms(const float* X, long long ldx, long long n, int d, float* out,
+                             cudaStream_t s) {
+  return prep_rows<float>(X, ldx, n, d, nullptr, nullptr, nullptr, nullptr, 0, nullptr, out, s, nullptr,
+                          nullptr);
+}
+
 template cudaError_t launch_prep_rows<float>(const float*, long long, long long, int, double*, float*,
-                                             void*, void*, long long, int*, cudaStream_t, const int*);
+                                             void*, void*, long long, int*, cudaStream_t, const int*,
+                                             const RowList*);
 template cudaError_t launch_prep_rows<double>(const double*, long long, long long, int, double*,
                                               float*, void*, void*, long long, int*, cudaStream_t,
-                                              const int*);
+                                              const int*, const RowList*);
+
+template <typename T>
+cudaError_t launch_prep_expansion(const T* B, int d, int k, const T* nb, float* Bt, long long ld,
+                                  float* nbx, void* Cb, void* Cl, long long ldb, float* cinit,
+                                  void* cbias, float* cmax, cudaStream_t s) {
+  const int kpad = cinit ? (k + kCenterPad - 1) / kCenterPad * kCenterPad : k;
+  prep_expansion_kernel<T><<<(unsigned)(((long long)kpad * 32 + 255) / 256), 256, 0, s>>>(
+      B, d, k, nb, Bt, ld, nbx, static_cast<__nv_bfloat16*>(Cb), static_cast<__nv_bfloat16*>(Cl), ldb,
+      cinit, static_cast<__nv_bfloat16*>(cbias), kpad, cmax);
+  kmgb::count_launches(1);
+  return cudaGetLastError();
+}
+template cudaError_t launch_prep_expansion<float>(const float*, int, int, const float*, float*,
+                                                  long long, float*, void*, void*, long long, float*,
+                                                  void*, float*, cudaStream_t);
+template cudaError_t launch_prep_expansion<double>(const double*, int, int, const double*, float*,
+                                                   long long, float*, void*, void*, long long, float*,
+                                                   void*, float*, cudaStream_t);
 
 cudaError_t launch_gather_rows(const float* Xsrc, long long ldx, const int* perm, long long m,
                                long long start, long long m_mb, int d, float* Xdst, long long ldd,

@@ -2,7 +2,9 @@
 // kernels. Same names, argument meaning and kmeansCudaErrorStatus codes; asynchronous on the
 // default stream like the reference; the reference's scratch arguments (Bpadded, C, Cindices,
 // normRowsOfA_squared in ClosestCenters) are accepted and not needed. Temporary buffers are
-// stream-ordered (cudaMallocAsync on the default stream).
+// stream-ordered on the default stream: cudaMallocAsync, and for ClosestCenters one allocation from
+// the library's pool (devmem.cu), bounded by working through the rows in chunks.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -24,18 +26,6 @@ void tmp_free(void* p) {
   if (p) cudaFreeAsync(p, kDefault);
 }
 
-// Bt[j][t] = B[t * k + j] (t < d), zero padding to ldc.
-template <typename T>
-__global__ void transpose_centers_kernel(const T* __restrict__ B, int d, int k, float* __restrict__ Bt,
-                                         long long ldc) {
-  const long long total = (long long)k * ldc;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(e / ldc), t = (int)(e % ldc);
-    Bt[e] = t < d ? (float)B[(size_t)t * k + j] : 0.0f;
-  }
-}
-
 __global__ void copy_pad_kernel(const float* __restrict__ A, long long m, int d, float* __restrict__ Ap,
                                 long long ld) {
   const long long total = m * ld;
@@ -47,34 +37,19 @@ __global__ void copy_pad_kernel(const float* __restrict__ A, long long m, int d,
   }
 }
 
-// cmax = max_j max(||Bt_j||, sqrt(|nb_j|)) (upper bound), for the expansion-mode bound.
-__global__ void cmax_expansion_kernel(const float* __restrict__ Bt, long long ldc, int k, int d,
-                                      const float* __restrict__ nb, float* cmax) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= k) return;
-  double s = 0.0;
-  for (int t = lane; t < d; t += 32) {
-    const double v = Bt[(size_t)warp * ldc + t];
-    s = fma(v, v, s);
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) {
-    double m = fmax(s, fabs((double)nb[warp]));
-    if (!(m < INFINITY)) m = 3.0e38;  // NaN / inf norms: make the bound huge (all re-ranked)
-    const float r = __double2float_ru(sqrt(m) * (1.0 + 1e-12));
-    atomicMax(reinterpret_cast<int*>(cmax), __float_as_int(r));
-  }
-}
-
-// FP64 arg-min of nb_j - 2 A_i.B_j (B is d x k, K fastest); one warp per row, lanes over j.
+// FP64 arg-min of nb_j - 2 A_i.B_j (B is d x k, K fastest); one warp per row, lanes over j. list
+// (nullable): only the rows list[0 .. *count).
 __global__ void closest_fp64_kernel(int m0, int m, int d, const double* __restrict__ A, int k,
                                     const double* __restrict__ B, const double* __restrict__ nb,
-                                    int* __restrict__ out) {
+                                    int* __restrict__ out, const int* __restrict__ list,
+                                    const int* __restrict__ count) {
   extern __shared__ double xs_all[];
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* xs = xs_all + (size_t)w * d;
-  for (long long i = (long long)blockIdx.x * warps + w; i < m; i += (long long)gridDim.x * warps) {
+  const long long todo = list ? (long long)*count : m;
+  for (long long slot = (long long)blockIdx.x * warps + w; slot < todo;
+       slot += (long long)gridDim.x * warps) {
+    const long long i = list ? (long long)list[slot] : slot;
     for (int t = lane; t < d; t += 32) xs[t] = A[(size_t)i * d + t];
     __syncwarp();
     double best = INFINITY;
@@ -134,39 +109,133 @@ __global__ void row_transform_min_kernel(int m0, int m, int n, const T* __restri
   }
 }
 
-// Squared distance of each row to its center, FP64, block partial sums.
-template <typename T>
-__global__ void compactness_partial_kernel(int m0, int m, int n, const T* __restrict__ data,
-                                           const int* __restrict__ idx, const T* __restrict__ centers,
-                                           double* __restrict__ partial) {
-  __shared__ double red[256];
-  double acc = 0.0;
-  const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (long long i = (long long)blockIdx.x * warps + w; i < m; i += (long long)gridDim.x * warps) {
-    const int l = idx[m0 + i];
-    double s = 0.0;
-    for (int t = lane; t < n; t += 32) {
-      const double u = (double)data[(size_t)i * n + t] - (double)centers[(size_t)l * n + t];
-      s = fma(u, u, s);
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    acc += s;  // identical in all lanes
-  }
-  red[threadIdx.x] = (lane == 0) ? acc : 0.0;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < (int)blockDim.x; i += 32) t += red[i];
-    partial[blockIdx.x] = t;
-  }
+__device__ __forceinline__ void ff_two_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float bp = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
 }
 
+// Sum over a block's threads (256), for thread 0.
+__device__ __forceinline__ double block_sum(double acc) {
+  __shared__ double red[8];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x == 0)
+    for (int i = 0; i < 8; ++i) t += red[i];
+  return t;
+}
+
+// Squared distances of the rows to their centers, block partial sums. Bound by HBM (every row once;
+// the centers come from L1/L2), with FP32 data also by GB300's narrow FP64 pipe as long as every
+// element is widened (898,790 x 128: 1.21 ms): there the terms run on the FP32 pipe as error-free
+// float-float values -- u = x - c exactly (TwoSum), u^2 = p + e (FMA), TwoSum accumulation -- and a
+// lane widens one pair per segment of kSegSteps rows. A segment whose sum leaves the range in which
+// that keeps 48 bits (overflow, squares near the subnormals, NaN) is evaluated in FP64.
+// L lanes share a row, 16 bytes each at a time where rows are aligned.
+constexpr int kSegSteps = 32;
+
+template <int L>
+__global__ void __launch_bounds__(256)
+compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const int* __restrict__ idx,
+                      const float* __restrict__ centers, bool vec, double* __restrict__ partial) {
+  constexpr int G = 32 / L;
+  const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  double acc = 0.0;
+  for (long long s0 = w0 * G * kSegSteps; s0 < m; s0 += nw * G * kSegSteps) {
+    float hi = 0.0f, lo = 0.0f, mx = 0.0f;
+    auto term = [&](float x, float c) {
+      float uh, ul, t, err;
+      ff_two_sum(x, -c, uh, ul);
+      const float p = __fmul_rn(uh, uh);
+      const float e = __fmaf_rn(uh, uh, -p);
+      const float r = __fmaf_rn(ul, ul, __fmaf_rn(__fadd_rn(uh, uh), ul, e));
+      ff_two_sum(hi, p, t, err);
+      hi = t;
+      lo = __fadd_rn(lo, __fadd_rn(err, r));
+      mx = fmaxf(mx, fabsf(uh));
+    };
+#pragma unroll 4
+    for (int i = 0; i < kSegSteps; ++i) {
+      const long long r = s0 + i * G + grp;
+      if (r >= m) continue;
+      const float* x = data + (size_t)r * n;
+      const float* c = centers + (size_t)__ldg(idx + r) * n;
+      if (vec) {
+        for (int t = 4 * sub; t < n; t += 4 * L) {
+          const float4 xv = __ldg(reinterpret_cast<const float4*>(x + t));
+          const float4 cv = __ldg(reinterpret_cast<const float4*>(c + t));
+          term(xv.x, cv.x);
+          term(xv.y, cv.y);
+          term(xv.z, cv.z);
+          term(xv.w, cv.w);
+        }
+      } else {
+        for (int t = sub; t < n; t += L) term(__ldg(x + t), __ldg(c + t));
+      }
+    }
+    if (hi < 1e37f && (hi > 1e-24f || mx == 0.0f)) {
+      acc += (double)hi + (double)lo;
+      continue;
+    }
+    for (int i = 0; i < kSegSteps; ++i) {
+      const long long r = s0 + i * G + grp;
+      if (r >= m) continue;
+      const float* x = data + (size_t)r * n;
+      const float* c = centers + (size_t)__ldg(idx + r) * n;
+      for (int t0 = vec ? 4 * sub : sub; t0 < n; t0 += vec ? 4 * L : L)
+        for (int t = t0; t < t0 + (vec ? 4 : 1); ++t) {
+          const double u = (double)x[t] - (double)c[t];
+          acc = fma(u, u, acc);
+        }
+    }
+  }
+  const double t = block_sum(acc);
+  if (threadIdx.x == 0) partial[blockIdx.x] = t;
+}
+
+// FP64 data: two FP64 operations per element (the lanes' sums meet once, at the end).
+__global__ void __launch_bounds__(256)
+compactness_d_kernel(long long m, int n, const double* __restrict__ data, const int* __restrict__ idx,
+                     const double* __restrict__ centers, double* __restrict__ partial) {
+  const int lane = threadIdx.x & 31;
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  double acc = 0.0;
+  constexpr int U = 4;  // rows in flight
+  for (long long r0 = w0 * U; r0 < m; r0 += nw * U) {
+    const double* x[U];
+    const double* c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long r = r0 + u < m ? r0 + u : m - 1;
+      x[u] = data + (size_t)r * n;
+      c[u] = centers + (size_t)__ldg(idx + r) * n;
+    }
+    for (int t = lane; t < n; t += 32) {
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = __ldg(x[u] + t) - __ldg(c[u] + t);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (r0 + u < m) acc = fma(v[u], v[u], acc);
+    }
+  }
+  const double t = block_sum(acc);
+  if (threadIdx.x == 0) partial[blockIdx.x] = t;
+}
+
+// One block: the partial sums, a strided chain per thread and a tree.
 template <typename T>
-__global__ void compactness_final_kernel(const double* __restrict__ partial, int nb, double* acc,
-                                         T* out, bool last) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < nb; ++i) t += partial[i];
+__global__ void __launch_bounds__(256)
+compactness_final_kernel(const double* __restrict__ partial, int nb, double* acc, T* out, bool last) {
+  double t = 0.0;
+  for (int i = threadIdx.x; i < nb; i += 256) t += partial[i];
+  t = block_sum(t);
+  if (threadIdx.x == 0) {
     *acc += t;
     if (last) out[0] = (T)*acc;
   }
@@ -183,12 +252,29 @@ __global__ void row_norm_kernel(int m0, int m, int n, const T* __restrict__ in, 
   }
 }
 
+// 32 columns per block (coalesced rows), 32 threads of a column taking every 32nd row; their FP64
+// sums are added in order. (One thread per column walked the rows alone: 128 x 256 took 23 us.)
 template <typename T>
-__global__ void col_norm_kernel(int m, int n, const T* __restrict__ in, T* __restrict__ out) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int i = 0; i < m; ++i) s = fma((double)in[(size_t)i * n + j], (double)in[(size_t)i * n + j], s);
-    out[j] = (T)s;
+__global__ void __launch_bounds__(1024)
+col_norm_kernel(int m, int n, const T* __restrict__ in, T* __restrict__ out) {
+  __shared__ double red[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long j = (long long)blockIdx.x * 32 + tx;
+  double s = 0.0;
+  if (j < n) {
+#pragma unroll 4
+    for (long long i = ty; i < m; i += 32) {
+      const double v = (double)__ldg(in + (size_t)i * n + j);
+      s = fma(v, v, s);
+    }
+  }
+  red[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && j < n) {
+    double t = 0.0;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) t += red[i][tx];
+    out[j] = (T)t;
   }
 }
 
@@ -262,6 +348,211 @@ kmeansCudaErrorStatus mat_mat_mult(int ra, int ca, const T* A, int cb, const T* 
   return cudaGetLastError() ? ERROR_MATMATMULT : NO_ERROR;
 }
 
+// Sizing (base null) or carving of one temporary allocation.
+struct Carver {
+  char* base = nullptr;
+  size_t off = 0;
+  template <typename T>
+  void take(T** p, size_t count) {
+    *p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+    off += (sizeof(T) * (count ? count : 1) + 255) / 256 * 256;
+  }
+};
+
+// ClosestCentersF/D. The rows' arg-min of nb_j - 2 A_i.B_j, equal to the FP64 evaluation.
+//
+// Split BF16 tensor cores where the dimension allows and the scan is long enough to pay for the
+// rows' BF16 planes (read once, written once) and some ten launches: FP32 from rows x centers (in
+// chunks of 128, the FP32 kernel's) x dimensions of 2^28 on, where the FP32 scan takes 12 us; FP64,
+// whose scan runs at 0.6 TFMA/s, from 2^24 on. The rows go through in chunks whose planes stay in L2
+// (and bound the workspace), whole waves of the pair kernel each. What the certificate leaves open
+// is settled from recorded candidates (float-float; FP64 data: FP64), the rest by the tiled stages
+// (FP64 data: a scan of the listed rows). FP32 scan: 898,790 x 128, K=256 took 1.52 ms, its re-rank
+// 0.28 ms; FP64 scan: 100,000 x 64, K=256 took 2.80 ms.
+template <typename T>
+cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const T* B, const T* nb,
+                            int* out) {
+  constexpr bool kF32 = sizeof(T) == 4;
+  const long long ld = (d + 3) / 4 * 4, ldb = (d + 7) / 8 * 8;
+  const bool direct = ld == d && !(reinterpret_cast<uintptr_t>(A) & 15);  // FP32 kernels' layout
+  const long long kp = (k + 127) / 128 * 128;
+  const bool tc = bf16_tc_supported(d, 2) && n >= 256 && n * kp >= (1LL << (kF32 ? 28 : 24)) / d;
+  const bool tiled = rerank_tiled_supported(d);
+  const int threads = 256;
+  const size_t smem = sizeof(double) * (size_t)d * (threads / 32);  // closest_fp64_kernel's
+  if (!kF32 && !tc) {
+    closest_fp64_kernel<<<kmgb::num_sms() * 8, threads, smem, kDefault>>>(
+        m0, (int)n, d, reinterpret_cast<const double*>(A), k, reinterpret_cast<const double*>(B),
+        reinterpret_cast<const double*>(nb), out, nullptr, nullptr);
+    count_launches(1);
+    return cudaGetLastError();
+  }
+  const bool copy = !tc && !direct;  // the FP32 scan reads 16-byte aligned rows
+  const long long wave = 256LL * (num_sms() / 2);
+  const long long chunk = std::min(n, wave * std::max(1LL, (96LL << 20) / (wave * ldb * 4)));
+  const long long cap = std::min(n, std::max(1024LL, n / 8));
+  float *Ap, *Bt, *nbx, *xn, *cmax, *cinit, *thr, *thrC, *hi2;
+  int *list, *list2, *over, *sc, *cand, *cand_cnt;
+  char *Xb, *Xl, *XbC, *XlC, *Cb, *Cl, *cbias;
+  const long long kpad = (k + kCenterPad - 1) / kCenterPad * kCenterPad;
+  auto carve = [&](Carver& c) {
+    c.take(&sc, 8);  // [0] cmax, [1] flagged, [2] left by the candidates, [3] left by FP32, [4] error
+    c.take(&Ap, copy ? n * ld : 0);
+    c.take(&Bt, k * ld);
+    c.take(&nbx, k);
+    c.take(&xn, n);
+    c.take(&list, n);
+    c.take(&over, tc ? n : 0);
+    c.take(&list2, kF32 ? n : 0);
+    c.take(&hi2, kF32 ? n : 0);
+    if (!tc) return;
+    c.take(&cinit, kpad);
+    c.take(&cbias, kpad * kBiasCols * 2);
+    c.take(&Cb, k * ldb * 2);
+    c.take(&Cl, k * ldb * 2);
+    c.take(&Xb, chunk * ldb * 2);
+    c.take(&Xl, chunk * ldb * 2);
+    c.take(&thr, n);
+    c.take(&XbC, cap * ldb * 2);
+    c.take(&XlC, cap * ldb * 2);
+    c.take(&thrC, cap);
+    c.take(&cand, cap * kMaxCand);
+    c.take(&cand_cnt, cap);
+  };
+  cinit = thr = thrC = nullptr;
+  Xb = Xl = XbC = XlC = Cb = Cl = cbias = nullptr;
+  cand = cand_cnt = nullptr;
+  Carver size;
+  carve(size);
+  void* mem = nullptr;
+  KMGB_CUDA_TRY(dev_alloc_async(&mem, size.off, kDefault));
+  Carver cut;
+  cut.base = static_cast<char*>(mem);
+  carve(cut);
+  cmax = reinterpret_cast<float*>(sc);
+  cudaError_t e = cudaMemsetAsync(sc, 0, 8 * sizeof(int), kDefault);
+  const T* Xa = A;
+  if (!e && copy) {
+    copy_pad_kernel<<<num_sms() * 8, 256, 0, kDefault>>>(reinterpret_cast<const float*>(A), n, d, Ap,
+                                                         ld);
+    count_launches(1);
+    e = cudaGetLastError();
+    Xa = reinterpret_cast<const T*>(Ap);
+  }
+  const long long ldx = copy ? ld : d;
+  if (!e)
+    e = launch_prep_expansion<T>(B, d, k, nb, Bt, ld, nbx, tc ? Cb : nullptr, Cl, ldb,
+                                 tc ? cinit : nullptr, tc ? cbias : nullptr, cmax, kDefault);
+  AssignArgs a{};
+  a.cn = nbx;
+  a.xnorm = xn;
+  a.cmax = cmax;
+  a.labels = out + m0;
+  a.rerank_list = list;
+  a.rerank_count = sc + 1;
+  a.err = sc + 4;
+  a.n = n;
+  a.k = k;
+  a.d = d;
+  a.certify = 1;
+  if (tc) {
+    a.gamma = assign_bf16_gamma(d);
+    a.cinit = cinit;
+    a.cbias = cbias;
+    a.thr_out = thr;
+    if (!kF32) a.pert = 0x1p-22f;  // FP32 roundings of FP64 rows and centers (computeKmeansD's bound)
+    for (long long r0 = 0; r0 < n && !e; r0 += chunk) {
+      const long long nr = std::min(chunk, n - r0);
+      e = launch_prep_rows(Xa + (size_t)r0 * ldx, ldx, nr, d, nullptr, xn + r0, Xb, Xl, ldb, nullptr,
+                           kDefault);
+      AssignArgs ac = a;
+      ac.n = nr;
+      ac.out0 = r0;
+      if (!e) e = launch_assign_bf16(Xb, Xl, ldb, Cb, Cl, ldb, ac, kDefault);
+    }
+    // the flagged rows again, recording their candidates
+    RowList rl{list, sc + 1, thr, thrC, over, sc + 2};
+    if (!e)
+      e = launch_prep_rows(Xa, ldx, cap, d, nullptr, nullptr, XbC, XlC, ldb, nullptr, kDefault, nullptr,
+                           &rl);
+    AssignArgs c2 = a;
+    c2.n = cap;
+    c2.n_dev = sc + 1;
+    c2.labels = nullptr;
+    c2.certify = 0;
+    c2.thr_out = nullptr;
+    c2.thr_in = thrC;
+    c2.cand = cand;
+    c2.cand_cnt = cand_cnt;
+    if (!e) e = launch_assign_bf16(XbC, XlC, ldb, Cb, Cl, ldb, c2, kDefault);
+  } else {
+    a.gamma = assign_fp32_gamma(d);
+    if (!e)
+      e = launch_prep_rows(Xa, ldx, n, d, nullptr, xn, nullptr, nullptr, 0, nullptr, kDefault);
+    if (!e) e = launch_assign_fp32(reinterpret_cast<const float*>(Xa), ld, Bt, ld, a, kDefault);
+  }
+  if (kF32) {
+    RerankArgs r{};
+    r.X = reinterpret_cast<const float*>(Xa);
+    r.ldx = ldx;
+    r.C = Bt;
+    r.ldc = ld;
+    r.nb = nbx;
+    r.xnorm = xn;
+    r.cmax = cmax;
+    r.list = list;
+    r.count = sc + 1;
+    r.labels = out + m0;
+    r.n = n;
+    r.k = k;
+    r.d = d;
+    r.mode = 1;
+    r.max_list = tc ? cap : n;
+    if (!e && tc) e = launch_resolve_expansion(r, cand, cand_cnt, over, sc + 2, kDefault);
+    if (tc) {
+      r.list = over;
+      r.count = sc + 2;
+      r.max_list = n;
+    }
+    if (!e && tiled) {
+      e = launch_rerank_tiled(r, list2, sc + 3, hi2, kDefault);
+      r.list = list2;
+      r.count = sc + 3;
+      if (!e) e = launch_rerank_exact(r, hi2, kDefault);
+    } else if (!e) {
+      e = launch_rerank(r, kDefault);
+    }
+  } else {
+    ResolveD r{};
+    r.X = reinterpret_cast<const double*>(A);
+    r.ldx = d;
+    r.C = reinterpret_cast<const double*>(B);
+    r.c_dim = k;
+    r.c_row = 1;
+    r.nb = reinterpret_cast<const double*>(nb);
+    r.d = d;
+    r.k = k;
+    r.mode = 1;
+    r.list = list;
+    r.count = sc + 1;
+    r.max_list = cap;
+    r.cand = cand;
+    r.cand_cnt = cand_cnt;
+    r.labels = out + m0;
+    r.over = over;
+    r.over_count = sc + 2;
+    if (!e) e = launch_resolve_fp64(r, kDefault);
+    if (!e) {
+      closest_fp64_kernel<<<num_sms() * 8, threads, smem, kDefault>>>(
+          m0, (int)n, d, r.X, k, r.C, r.nb, out, over, sc + 2);
+      count_launches(1);
+      e = cudaGetLastError();
+    }
+  }
+  dev_free(mem, kDefault);
+  return e;
+}
+
 template <typename T>
 kmeansCudaErrorStatus cluster_centers(int m0, int m, int n, int k, bool lastTile, const T* data,
                                       const int* indices, T* centers_large, int* counts_large,
@@ -297,6 +588,23 @@ kmeansCudaErrorStatus cluster_centers(int m0, int m, int n, int k, bool lastTile
   return e ? ERROR_CLUSTERCENTERS : NO_ERROR;
 }
 
+void launch_compactness(long long m, int n, const float* data, const int* idx, const float* centers,
+                        double* part, int blocks) {
+  const bool vec = n % 4 == 0 && !(reinterpret_cast<uintptr_t>(data) & 15) &&
+                   !(reinterpret_cast<uintptr_t>(centers) & 15);
+  const int per = vec ? (n + 3) / 4 : n;  // lanes' worth of a row
+  if (per <= 4) compactness_ff_kernel<4><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
+  else if (per <= 8) compactness_ff_kernel<8><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
+  else if (per <= 16) compactness_ff_kernel<16><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
+  else compactness_ff_kernel<32><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
+  count_launches(1);
+}
+void launch_compactness(long long m, int n, const double* data, const int* idx, const double* centers,
+                        double* part, int blocks) {
+  compactness_d_kernel<<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, part);
+  count_launches(1);
+}
+
 template <typename T>
 kmeansCudaErrorStatus compactness(int m0, int m, bool lastTile, int n, int k, const T* data,
                                   const int* indices, const T* centers, T* out) {
@@ -304,15 +612,15 @@ kmeansCudaErrorStatus compactness(int m0, int m, bool lastTile, int n, int k, co
   if (m < 0 || n <= 0 || !out) return ERROR_COMPACTNESS;
   double* acc = (sizeof(T) == 4) ? reinterpret_cast<double*>(out + 2) : reinterpret_cast<double*>(out + 1);
   if (reinterpret_cast<uintptr_t>(acc) & 7) return ERROR_COMPACTNESS;
-  const int blocks = kmgb::num_sms() * 4;
+  const int blocks = kmgb::num_sms() * 8;
   double* part = nullptr;
   cudaError_t e = tmp_alloc(&part, blocks);
   if (!e) {
-    compactness_partial_kernel<T><<<blocks, 256, 0, kDefault>>>(m0, m, n, data, indices, centers, part); kmgb::count_launches(1);
+    launch_compactness(m, n, data, indices + m0, centers, part, blocks);
     e = cudaGetLastError();
   }
   if (!e) {
-    compactness_final_kernel<T><<<1, 32, 0, kDefault>>>(part, blocks, acc, out, lastTile); kmgb::count_launches(1);
+    compactness_final_kernel<T><<<1, 256, 0, kDefault>>>(part, blocks, acc, out, lastTile); kmgb::count_launches(1);
     e = cudaGetLastError();
   }
   tmp_free(part);
@@ -337,81 +645,9 @@ kmeansCudaErrorStatus ClosestCentersF(const int m0, const int nRowsA, const int 
       !CindicesFinal)
     return ERROR_CLOSESTCENTERS;
   if (nRowsA == 0) return NO_ERROR;
-  const int d = nColsA, k = nColsB;
-  const long long ld = (d + 3) / 4 * 4;
-  const bool direct = (ld == d) && !(reinterpret_cast<uintptr_t>(A) & 15);
-  float *Ap = nullptr, *Bt = nullptr, *xn = nullptr, *cmax = nullptr;
-  int *list = nullptr, *count = nullptr, *err = nullptr;
-  cudaError_t e = cudaSuccess;
-  if (!direct) e = tmp_alloc(&Ap, (size_t)nRowsA * ld);
-  if (!e) e = tmp_alloc(&Bt, (size_t)k * ld);
-  if (!e) e = tmp_alloc(&xn, nRowsA);
-  if (!e) e = tmp_alloc(&cmax, 1);
-  if (!e) e = tmp_alloc(&list, nRowsA);
-  if (!e) e = tmp_alloc(&count, 2);
-  if (!e) e = tmp_alloc(&err, 1);
-  if (!e) e = cudaMemsetAsync(cmax, 0, sizeof(float), kDefault);
-  if (!e) e = cudaMemsetAsync(count, 0, 2 * sizeof(int), kDefault);
-  if (!e) e = cudaMemsetAsync(err, 0, sizeof(int), kDefault);
-  const float* Xa = A;
-  if (!e && !direct) {
-    copy_pad_kernel<<<kmgb::num_sms() * 8, 256, 0, kDefault>>>(A, nRowsA, d, Ap, ld); kmgb::count_launches(1);
-    e = cudaGetLastError();
-    Xa = Ap;
-  }
-  if (!e) {
-    transpose_centers_kernel<float><<<kmgb::num_sms() * 4, 256, 0, kDefault>>>(B, d, k, Bt, ld); kmgb::count_launches(1);
-    e = cudaGetLastError();
-  }
-  if (!e) e = launch_prep_rows(Xa, ld, nRowsA, d, nullptr, xn, nullptr, nullptr, 0, nullptr, kDefault);
-  if (!e) {
-    cmax_expansion_kernel<<<(k * 32 + 255) / 256, 256, 0, kDefault>>>(Bt, ld, k, d,
-                                                                     normColsOfB_squared, cmax); kmgb::count_launches(1);
-    e = cudaGetLastError();
-  }
-  if (!e) {
-    AssignArgs a{};
-    a.cn = normColsOfB_squared;
-    a.xnorm = xn;
-    a.cmax = cmax;
-    a.labels = CindicesFinal + m0;
-    a.rerank_list = list;
-    a.rerank_count = count;
-    a.err = err;
-    a.n = nRowsA;
-    a.k = k;
-    a.d = d;
-    a.certify = 1;
-    a.gamma = assign_fp32_gamma(d);
-    e = launch_assign_fp32(Xa, ld, Bt, ld, a, kDefault);
-  }
-  if (!e) {
-    RerankArgs r{};
-    r.X = Xa;
-    r.ldx = ld;
-    r.C = Bt;
-    r.ldc = ld;
-    r.nb = normColsOfB_squared;
-    r.xnorm = xn;
-    r.cmax = cmax;
-    r.list = list;
-    r.count = count;
-    r.labels = CindicesFinal + m0;
-    r.n = nRowsA;
-    r.k = k;
-    r.d = d;
-    r.mode = 1;
-    r.max_list = nRowsA;
-    e = launch_rerank(r, kDefault);
-  }
-  tmp_free(Ap);
-  tmp_free(Bt);
-  tmp_free(xn);
-  tmp_free(cmax);
-  tmp_free(list);
-  tmp_free(count);
-  tmp_free(err);
-  return e ? ERROR_CLOSESTCENTERS : NO_ERROR;
+  return closest_centers<float>(m0, nRowsA, nColsA, A, nColsB, B, normColsOfB_squared, CindicesFinal)
+             ? ERROR_CLOSESTCENTERS
+             : NO_ERROR;
 }
 
 kmeansCudaErrorStatus ClosestCentersD(const int m0, const int nRowsA, const int nColsA,
@@ -435,9 +671,10 @@ kmeansCudaErrorStatus ClosestCentersD(const int m0, const int nRowsA, const int 
       cudaFuncSetAttribute(closest_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return ERROR_CLOSESTCENTERS;
-  closest_fp64_kernel<<<kmgb::num_sms() * 8, threads, smem, kDefault>>>(m0, nRowsA, nColsA, A, nColsB, B,
-                                                            normColsOfB_squared, CindicesFinal); kmgb::count_launches(1);
-  return cudaGetLastError() ? ERROR_CLOSESTCENTERS : NO_ERROR;
+  return closest_centers<double>(m0, nRowsA, nColsA, A, nColsB, B, normColsOfB_squared,
+                                 CindicesFinal)
+             ? ERROR_CLOSESTCENTERS
+             : NO_ERROR;
 }
 
 kmeansCudaErrorStatus rowTransformMinimumF(const int m0, const int m, const int n,
@@ -504,8 +741,7 @@ kmeansCudaErrorStatus rowNormalizeF(const int m0, const int m, const int n, cons
                                     float* output) {
   if (m < 0 || n <= 0) return ERROR_ROWNORMALIZE;
   if (m == 0) return NO_ERROR;
-  row_norm_kernel<float><<<kmgb::num_sms() * 8, 256, 0, kDefault>>>(m0, m, n, input, output); kmgb::count_launches(1);
-  return cudaGetLastError() ? ERROR_ROWNORMALIZE : NO_ERROR;
+  return launch_row_norms(input, n, m, n, output + m0, kDefault) ? ERROR_ROWNORMALIZE : NO_ERROR;
 }
 
 kmeansCudaErrorStatus rowNormalizeD(const int m0, const int m, const int n, const double* input,
@@ -518,14 +754,14 @@ kmeansCudaErrorStatus rowNormalizeD(const int m0, const int m, const int n, cons
 
 kmeansCudaErrorStatus colNormalizeF(const int m, const int n, const float* input, float* output) {
   if (m < 0 || n <= 0) return ERROR_COLNORMALIZE;
-  col_norm_kernel<float><<<(n + 127) / 128, 128, 0, kDefault>>>(m, n, input, output); kmgb::count_launches(1);
+  col_norm_kernel<float><<<(unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault>>>(m, n, input, output); kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_COLNORMALIZE : NO_ERROR;
 }
 
 kmeansCudaErrorStatus colNormalizeD(const int m, const int n, const double* input,
                                     double* output) {
   if (m < 0 || n <= 0) return ERROR_COLNORMALIZE;
-  col_norm_kernel<double><<<(n + 127) / 128, 128, 0, kDefault>>>(m, n, input, output); kmgb::count_launches(1);
+  col_norm_kernel<double><<<(unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault>>>(m, n, input, output); kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_COLNORMALIZE : NO_ERROR;
 }
 

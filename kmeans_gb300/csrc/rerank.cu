@@ -135,7 +135,7 @@ __global__ void rerank_kernel(RerankArgs a) {
   }
 }
 
-// Tiled FP32 stage of the Lloyd re-rank (mode 0): 32 flagged points per CTA iteration against
+// Tiled FP32 stage of the re-rank (described for mode 0): 32 flagged points per CTA iteration against
 // 64-center blocks staged in shared memory; each thread accumulates 4 points x 2 centers of
 // sum_d (x_d - c_d)^2 with float4 loads. Per point (best, index, second) is merged over the 32
 // threads that share it (lowest index on ties) and certified with the relative bound of the
@@ -143,6 +143,39 @@ __global__ void rerank_kernel(RerankArgs a) {
 constexpr int TP = 32;   // points per CTA iteration
 constexpr int TC = 64;   // centers per block
 
+// The tiled stages' two forms. A center's offset: MODE 0 zero, MODE 1 its norm; +inf for padding and
+// (MODE 0) unusable centers.
+template <int MODE>
+__device__ __forceinline__ float tile_offset(const RerankArgs& a, int j) {
+  if (j >= a.k) return INFINITY;
+  if (MODE == 1) return a.nb[j];
+  return a.cn[j] < INFINITY ? 0.0f : INFINITY;
+}
+template <int MODE>
+__device__ __forceinline__ void tile_acc(const float4 x, const float4 c, float& acc) {
+  if (MODE == 0) {
+    float t;
+    t = x.x - c.x; acc = fmaf(t, t, acc);
+    t = x.y - c.y; acc = fmaf(t, t, acc);
+    t = x.z - c.z; acc = fmaf(t, t, acc);
+    t = x.w - c.w; acc = fmaf(t, t, acc);
+  } else {
+    acc = fmaf(x.x, c.x, acc);
+    acc = fmaf(x.y, c.y, acc);
+    acc = fmaf(x.z, c.z, acc);
+    acc = fmaf(x.w, c.w, acc);
+  }
+}
+// MODE 1: bound of |fl(nb_j - 2 x.c_j) - the FP64 value| over every center (|nb_j| <= cmax^2).
+__device__ __forceinline__ float expansion_bound(const RerankArgs& a, int pt) {
+  const float u = 5.9604645e-8f;
+  const float xn = a.xnorm[pt], cm = *a.cmax;
+  const float gd = (float)a.d * u * 1.001f;
+  return (2.0f * gd * xn * cm + u * 2.01f * xn * cm + (float)(a.d + 2) * 2.3e-16f * xn * cm +
+          u * 1.01f * cm * cm) * 1.01f + 1e-30f;
+}
+
+template <int MODE>
 __global__ void __launch_bounds__(256)
 rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ count2,
                     float* __restrict__ hi2) {
@@ -153,7 +186,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
                                           // lie in distinct banks
   float4* xs = sm4;                       // [TP][rs]
   float4* cs = xs + TP * rs;              // [TC][rs]
-  float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] 0 usable, +inf unusable
+  float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] value offset (tile_offset)
   __shared__ float mb1[8][TP], mb2[8][TP];
   __shared__ int mi1[8][TP];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -201,7 +234,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
       }
       if (tid < TC) {
         const int j = j0 + tid;
-        cflag[tid] = (j < a.k && a.cn[j] < INFINITY) ? 0.0f : INFINITY;
+        cflag[tid] = tile_offset<MODE>(a, j);
       }
       __syncthreads();
       float acc[4][2];
@@ -213,15 +246,8 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float4 x = xs[(pq + 8 * i) * rs + q];
-          float t;
-          t = x.x - c0.x; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.y - c0.y; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.z - c0.z; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.w - c0.w; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.x - c1.x; acc[i][1] = fmaf(t, t, acc[i][1]);
-          t = x.y - c1.y; acc[i][1] = fmaf(t, t, acc[i][1]);
-          t = x.z - c1.z; acc[i][1] = fmaf(t, t, acc[i][1]);
-          t = x.w - c1.w; acc[i][1] = fmaf(t, t, acc[i][1]);
+          tile_acc<MODE>(x, c0, acc[i][0]);
+          tile_acc<MODE>(x, c1, acc[i][1]);
         }
       }
 #pragma unroll
@@ -230,7 +256,8 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
         const float f = cflag[cq * 2 + jj];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float v = acc[i][jj] + f;  // +inf for unusable / padding centers
+          // +inf for unusable / padding centers
+          const float v = MODE == 0 ? acc[i][jj] + f : fmaf(-2.0f, acc[i][jj], f);
           const float nb2 = fminf(b2[i], fmaxf(b1[i], v));
           const bool lt = v < b1[i];
           b1[i] = lt ? v : b1[i];
@@ -274,12 +301,22 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
       }
       const int pt = a.list[g0 + tid];
       // certified when every other center's lower end exceeds the best's upper end
-      if (fi >= 0 && f2 * (1.0f - gam) - 1e-30f > f1 * (1.0f + gam) + 1e-30f) {
+      float lo2, hi1;
+      if (MODE == 0) {
+        lo2 = f2 * (1.0f - gam) - 1e-30f;
+        hi1 = f1 * (1.0f + gam) + 1e-30f;  // no usable center: +inf
+      } else {
+        const float e = expansion_bound(a, pt);
+        lo2 = f2 - e;
+        hi1 = f1 + e;
+        if (!(hi1 == hi1)) hi1 = INFINITY;
+      }
+      if (fi >= 0 && lo2 > hi1) {
         a.labels[pt] = fi;
       } else {
         const int slot = atomicAdd(count2, 1);
         list2[slot] = pt;
-        hi2[slot] = f1 * (1.0f + gam) + 1e-30f;  // no usable center: +inf
+        hi2[slot] = hi1;
       }
     }
   }
@@ -296,7 +333,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
 // holds its whole warp on the narrow FP64 pipe), the band's centers become the candidates of
 // resolve_candidates_kernel, whose float-float tier settles nearly all of them: 796,160 x 324,
 // K=256, FP32 tier, 1.05 ms per iteration before. Slots from cand_cap on go to over / over_hi.
-template <bool RECORD>
+template <int MODE, bool RECORD>
 __global__ void __launch_bounds__(256)
 rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict__ cand,
                     int* __restrict__ cand_cnt, long long cand_cap, int* __restrict__ over,
@@ -307,11 +344,12 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
   const int rs = (dq + 1) | 1;
   float4* xs = sm4;                       // [TP][rs]
   float4* cs = xs + TP * rs;              // [TC][rs]
-  float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] 0 usable, +inf unusable
+  float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] value offset (tile_offset)
   __shared__ double mb[8][TP];
   __shared__ int mi[8][TP];
   __shared__ float hs[TP];
   __shared__ int ncand[TP];
+  __shared__ float es[TP];  // MODE 1: the point's bound
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int pq = tid & 7;                 // points pq, pq + 8, pq + 16, pq + 24
   const int cq = tid >> 3;                // centers cq*2, cq*2+1 of the block
@@ -346,6 +384,7 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
     if (tid < TP) {
       hs[tid] = (g0 + tid < cnt) ? hi2[g0 + tid] : -INFINITY;
       ncand[tid] = 0;
+      es[tid] = MODE == 1 && g0 + tid < cnt ? expansion_bound(a, a.list[g0 + tid]) : 0.0f;
     }
     double be[4];
     int bi[4];
@@ -364,7 +403,7 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
       }
       if (tid < TC) {
         const int j = j0 + tid;
-        cflag[tid] = (j < a.k && a.cn[j] < INFINITY) ? 0.0f : INFINITY;
+        cflag[tid] = tile_offset<MODE>(a, j);
       }
       __syncthreads();
       float acc[4][2];
@@ -376,15 +415,8 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float4 x = xs[(pq + 8 * i) * rs + q];
-          float t;
-          t = x.x - c0.x; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.y - c0.y; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.z - c0.z; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.w - c0.w; acc[i][0] = fmaf(t, t, acc[i][0]);
-          t = x.x - c1.x; acc[i][1] = fmaf(t, t, acc[i][1]);
-          t = x.y - c1.y; acc[i][1] = fmaf(t, t, acc[i][1]);
-          t = x.z - c1.z; acc[i][1] = fmaf(t, t, acc[i][1]);
-          t = x.w - c1.w; acc[i][1] = fmaf(t, t, acc[i][1]);
+          tile_acc<MODE>(x, c0, acc[i][0]);
+          tile_acc<MODE>(x, c1, acc[i][1]);
         }
       }
 #pragma unroll
@@ -394,9 +426,11 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int pl = pq + 8 * i;
-          if (cflag[cl] != 0.0f) continue;  // unusable (empty-cluster) or padding center
-          const float v = acc[i][jj];
-          if (!(v * (1.0f - gam) - 1e-30f <= hs[pl])) continue;
+          // unusable (empty-cluster) or padding center
+          if (MODE == 0 ? cflag[cl] != 0.0f : j >= a.k) continue;
+          const float lo = MODE == 0 ? acc[i][jj] * (1.0f - gam) - 1e-30f
+                                     : fmaf(-2.0f, acc[i][jj], cflag[cl]) - es[pl];
+          if (!(lo <= hs[pl])) continue;
           if (RECORD) {
             const int at = atomicAdd(&ncand[pl], 1);
             if (at < kMaxCand) cand[(g0 + pl) * kMaxCand + at] = j;
@@ -407,12 +441,20 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
           for (int q = 0; q < dq; ++q) {
             const float4 x = xs[pl * rs + q];
             const float4 c = cs[cl * rs + q];
-            double dd;
-            dd = (double)x.x - (double)c.x; ex = fma(dd, dd, ex);
-            dd = (double)x.y - (double)c.y; ex = fma(dd, dd, ex);
-            dd = (double)x.z - (double)c.z; ex = fma(dd, dd, ex);
-            dd = (double)x.w - (double)c.w; ex = fma(dd, dd, ex);
+            if (MODE == 0) {
+              double dd;
+              dd = (double)x.x - (double)c.x; ex = fma(dd, dd, ex);
+              dd = (double)x.y - (double)c.y; ex = fma(dd, dd, ex);
+              dd = (double)x.z - (double)c.z; ex = fma(dd, dd, ex);
+              dd = (double)x.w - (double)c.w; ex = fma(dd, dd, ex);
+            } else {
+              ex = fma((double)x.x, (double)c.x, ex);
+              ex = fma((double)x.y, (double)c.y, ex);
+              ex = fma((double)x.z, (double)c.z, ex);
+              ex = fma((double)x.w, (double)c.w, ex);
+            }
           }
+          if (MODE == 1) ex = fma(-2.0, ex, (double)cflag[cl]);
           if (ex < INFINITY && (ex < be[i] || (ex == be[i] && (unsigned)j < (unsigned)bi[i]))) {
             be[i] = ex;
             bi[i] = j;
@@ -871,6 +913,186 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
   }
 }
 
+// x.c over the first d dimensions as a float-float (hi, lo), summed over each group of 8 consecutive
+// lanes as in ff_dist8: exact products (p + e by FMA), TwoSum.
+__device__ __forceinline__ void ff_product(float x, float c, float& hi, float& lo) {
+  const float p = __fmul_rn(x, c);
+  const float e = __fmaf_rn(x, c, -p);
+  float s, err;
+  two_sum(hi, p, s, err);
+  hi = s;
+  lo = __fadd_rn(lo, __fadd_rn(err, e));
+}
+template <bool VEC>
+__device__ __forceinline__ void ff_dot8(const float* __restrict__ x, const float* __restrict__ c, int d,
+                                        int r, float& hi, float& lo) {
+  hi = 0.0f;
+  lo = 0.0f;
+  if (VEC) {
+    for (int t = 4 * r; t < d; t += 4 * kGroupLanes) {
+      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + t));
+      const float4 cv = __ldg(reinterpret_cast<const float4*>(c + t));
+      ff_product(xv.x, cv.x, hi, lo);
+      ff_product(xv.y, cv.y, hi, lo);
+      ff_product(xv.z, cv.z, hi, lo);
+      ff_product(xv.w, cv.w, hi, lo);
+    }
+  } else {
+    for (int t = r; t < d; t += kGroupLanes) ff_product(__ldg(x + t), __ldg(c + t), hi, lo);
+  }
+  for (int o = kGroupLanes / 2; o > 0; o >>= 1) {
+    const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+    const float ol = __shfl_xor_sync(0xffffffffu, lo, o);
+    float s, err;
+    two_sum(hi, oh, s, err);
+    hi = s;
+    lo = __fadd_rn(lo, __fadd_rn(ol, err));
+  }
+}
+
+// Expansion form (mode 1, value nb_j - 2 x.c_j): the recorded candidates of every flagged point in
+// float-float, eight lanes per candidate. Each dot product is within rel sum|x_t c_t| <= rel ||x||
+// cmax of the exact one (rel: resolve_candidates_kernel's, for products instead of squares) and the
+// FP64 value the label is defined by within (d + 4) 2^-52 (||x|| + cmax)^2; a best candidate ahead by
+// more than both, twice, is the arg-min. Other points (ties, non-finite values) take the sequential
+// FP64 evaluation, one lane per candidate, lowest index on ties.
+template <bool VEC>
+__global__ void resolve_expansion_kernel(RerankArgs a, const int* __restrict__ cand,
+                                         const int* __restrict__ cand_cnt, int* __restrict__ over,
+                                         int* __restrict__ over_count) {
+  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  const int lane = threadIdx.x & 31;
+  const int grp = lane / kGroupLanes, sub = lane % kGroupLanes;
+  constexpr int kGroups = 32 / kGroupLanes;
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int d = a.d;
+  const double m = 4.0 * (double)((d + 31) / 32);
+  const double rel = 8.0 * ((m + 1.0) * (m + 1.0) + 2.0 + 3.0 * (m + 6.0)) * 0x1p-47;
+  const double cm = (double)*a.cmax;
+  for (long long slot = w0; slot < cnt; slot += nw) {
+    const int pt = a.list[slot];
+    const int nc = cand_cnt[slot];
+    if (nc <= 0 || nc > kMaxCand) {
+      if (lane == 0) over[atomicAdd(over_count, 1)] = pt;
+      continue;
+    }
+    const float* x = a.X + (size_t)pt * a.ldx;
+    const int myj = lane < nc ? cand[slot * kMaxCand + lane] : -1;
+    const float mynb = myj >= 0 && myj < a.k ? a.nb[myj] : INFINITY;
+    const int myok = mynb < INFINITY ? 1 : 0;  // a NaN or infinite norm never wins
+    double v1 = INFINITY, v2 = INFINITY;
+    int i1 = -1;
+    bool finite = true;
+    for (int q0 = 0; q0 < nc; q0 += kGroups) {
+      const int q = q0 + grp;
+      const int j = __shfl_sync(0xffffffffu, myj, q);
+      const int ok = __shfl_sync(0xffffffffu, myok, q) && q < nc;
+      const float nbj = __shfl_sync(0xffffffffu, mynb, q);
+      float hi, lo;
+      ff_dot8<VEC>(x, ok ? a.C + (size_t)j * a.ldc : x, ok ? d : 0, sub, hi, lo);
+      const double v = fma(-2.0, (double)hi + (double)lo, (double)nbj);
+      for (int g = 0; g < kGroups; ++g) {
+        const double vg = __shfl_sync(0xffffffffu, v, g * kGroupLanes);
+        const int jg = __shfl_sync(0xffffffffu, j, g * kGroupLanes);
+        if (!__shfl_sync(0xffffffffu, ok, g * kGroupLanes)) continue;
+        if (!(fabs(vg) < 1.0e300)) finite = false;
+        if (vg < v1) {
+          v2 = v1;
+          v1 = vg;
+          i1 = jg;
+        } else if (vg < v2) {
+          v2 = vg;
+        }
+      }
+    }
+    const double xn = (double)a.xnorm[pt];
+    const double tol = 2.0 * (2.0 * rel * xn * cm + (double)(d + 32) * 0x1p-118) +
+                       2.0 * (double)(d + 4) * 0x1p-52 * (xn + cm) * (xn + cm);
+    if (i1 >= 0 && finite && (v2 == INFINITY || v2 - v1 > tol)) {
+      if (lane == 0) a.labels[pt] = i1;
+      continue;
+    }
+    double best = INFINITY;
+    int bidx = -1;
+    if (myok) {
+      const float* c = a.C + (size_t)myj * a.ldc;
+      const double ex = exact_value(1, x, c, d, mynb);
+      if (ex < best) {
+        best = ex;
+        bidx = myj;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+      const bool take = (ob < best) || (ob == best && (unsigned)oi < (unsigned)bidx);
+      best = take ? ob : best;
+      bidx = take ? oi : bidx;
+    }
+    if (lane == 0) {
+      if (bidx < 0) over[atomicAdd(over_count, 1)] = pt;
+      else a.labels[pt] = bidx;
+    }
+  }
+}
+
+// FP64 data: every candidate's exact value, eight lanes (candidates) per point, four points per
+// warp: the FP64 pipe takes a warp instruction in the same time whatever its active lanes.
+__global__ void resolve_fp64_kernel(ResolveD a) {
+  constexpr int L = 8;
+  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
+  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long s0 = w0 * (32 / L); s0 < cnt; s0 += nw * (32 / L)) {
+    const long long slot = s0 + grp;
+    const bool live = slot < cnt;
+    const int pt = live ? a.list[slot] : 0;
+    const int nc = live ? a.cand_cnt[slot] : 0;
+    const bool rec = nc > 0 && nc <= kMaxCand;
+    double best = INFINITY;
+    int bidx = -1;
+    if (rec) {
+      const double* x = a.X + (size_t)pt * a.ldx;
+      for (int q = sub; q < nc; q += L) {
+        const int j = a.cand[slot * kMaxCand + q];
+        if (j < 0 || j >= a.k) continue;
+        const double* c = a.C + (size_t)j * a.c_row;
+        double v = 0.0;
+        if (a.mode == 0) {
+#pragma unroll 8
+          for (int t = 0; t < a.d; ++t) {
+            const double u = __ldg(x + t) - __ldg(c + (size_t)t * a.c_dim);
+            v = fma(u, u, v);
+          }
+        } else {
+#pragma unroll 8
+          for (int t = 0; t < a.d; ++t) v = fma(__ldg(x + t), __ldg(c + (size_t)t * a.c_dim), v);
+          v = fma(-2.0, v, a.nb[j]);
+        }
+        // (a lane's candidates do not come in index order)
+        if (v < best || (v == best && bidx >= 0 && j < bidx)) {
+          best = v;
+          bidx = j;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+      const bool take = (ob < best) || (ob == best && (unsigned)oi < (unsigned)bidx);
+      best = take ? ob : best;
+      bidx = take ? oi : bidx;
+    }
+    if (live && sub == 0) {
+      if (bidx < 0) a.over[atomicAdd(a.over_count, 1)] = pt;
+      else a.labels[pt] = bidx;
+    }
+  }
+}
+
 // ------------------------------- audit of certified labels -------------------------------
 // A rotating sample of rows is checked against the FP64 arg-min over every center, so that a
 // failure of a rounding model the certificate relies on (the tensor tiers' accumulation bound,
@@ -1068,6 +1290,27 @@ cudaError_t launch_resolve_candidates(const int* list, const int* count, long lo
   return cudaGetLastError();
 }
 
+cudaError_t launch_resolve_expansion(const RerankArgs& a, const int* cand, const int* cand_cnt,
+                                     int* over, int* over_count, cudaStream_t s) {
+  const bool vec = a.d % 4 == 0 && a.ldx % 4 == 0 && a.ldc % 4 == 0 &&
+                   reinterpret_cast<uintptr_t>(a.X) % 16 == 0 &&
+                   reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
+  if (vec)
+    resolve_expansion_kernel<true><<<kmgb::num_sms() * 8, 256, 0, s>>>(a, cand, cand_cnt, over,
+                                                                       over_count);
+  else
+    resolve_expansion_kernel<false><<<kmgb::num_sms() * 8, 256, 0, s>>>(a, cand, cand_cnt, over,
+                                                                        over_count);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_resolve_fp64(const ResolveD& a, cudaStream_t s) {
+  resolve_fp64_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(a);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_count_stats(const int* counts, int full_idx, unsigned long long* stats,
                                const int* stop, cudaStream_t s) {
   count_stats_kernel<<<1, 1, 0, s>>>(counts, full_idx, stats, stop);
@@ -1075,17 +1318,22 @@ cudaError_t launch_count_stats(const int* counts, int full_idx, unsigned long lo
   return cudaGetLastError();
 }
 
+static size_t tiled_smem(int d) {
+  const int dq = (d + 3) / 4;
+  return sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
+}
+
+bool rerank_tiled_supported(int d) { return tiled_smem(d) <= 200 * 1024; }
+
 cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
-  const int dq = (a.d + 3) / 4;
-  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
+  const size_t smem = tiled_smem(a.d);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  auto kern = a.mode == 0 ? rerank_exact_kernel<0, false> : rerank_exact_kernel<1, false>;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  rerank_exact_kernel<false><<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2, nullptr, nullptr, 0,
-                                                                    nullptr, nullptr, nullptr);
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1095,14 +1343,13 @@ cudaError_t launch_rerank_band(const RerankArgs& a, const float* hi2, int* cand,
                                cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
-  const int dq = (a.d + 3) / 4;
-  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  const size_t smem = tiled_smem(a.d);
+  if (smem > 200 * 1024 || a.mode != 0) return cudaErrorInvalidValue;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<true>,
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<0, true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  rerank_exact_kernel<true><<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2, cand, cand_cnt, cand_cap,
-                                                                   over, over_count, over_hi);
+  rerank_exact_kernel<0, true><<<kmgb::num_sms() * 2, 256, smem, s>>>(
+      a, hi2, cand, cand_cnt, cand_cap, over, over_count, over_hi);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1111,13 +1358,12 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
                                 cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
-  const int dq = (a.d + 3) / 4;
-  const size_t smem = sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
+  const size_t smem = tiled_smem(a.d);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  auto kern = a.mode == 0 ? rerank_tiled_kernel<0> : rerank_tiled_kernel<1>;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_tiled_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  rerank_tiled_kernel<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, list2, count2, hi2);
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, list2, count2, hi2);
   count_launches(1);
   return cudaGetLastError();
 }

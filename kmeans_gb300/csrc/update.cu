@@ -276,13 +276,9 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
 
 // Piece accumulator. FP32 data: an error-free float-float sum (Knuth's TwoSum on the FP32
 // pipe: hi + lo carries ~48 significant bits), turned into one FP64 value per piece; FP64 data:
-// a plain FP64 sum. GB300 issues FP64 (and FP32->FP64 conversions) at a small fraction of the
+// a plain FP64 sum (piece_sums_d_kernel). GB300 issues FP64 (and FP32->FP64 conversions) at a small fraction of the
 // FP32 rate, so converting every element would bound the update.
-template <typename T>
-struct PieceAcc;
-
-template <>
-struct PieceAcc<float> {
+struct PieceAcc {
   float hi = 0.0f, lo = 0.0f;
   __device__ __forceinline__ void add(float x) {
     const float t = __fadd_rn(hi, x);
@@ -292,13 +288,6 @@ struct PieceAcc<float> {
     lo = __fadd_rn(lo, err);
   }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
-};
-
-template <>
-struct PieceAcc<double> {
-  double s = 0.0;
-  __device__ __forceinline__ void add(double x) { s += x; }
-  __device__ __forceinline__ double value() const { return s; }
 };
 
 __device__ __forceinline__ int find_label(const int* __restrict__ pstart, int k, int p) {
@@ -312,8 +301,7 @@ __device__ __forceinline__ int find_label(const int* __restrict__ pstart, int k,
 }
 
 // One warp per piece; dims lane + 32 r in chunks of 256.
-template <typename T>
-__global__ void piece_sums_kernel(const T* __restrict__ X, long long ldx,
+__global__ void piece_sums_kernel(const float* __restrict__ X, long long ldx,
                                   const double* __restrict__ qn, const int* __restrict__ sorted,
                                   const int* __restrict__ label_off, const int* __restrict__ pstart,
                                   int k, int d, double* __restrict__ part,
@@ -329,12 +317,12 @@ __global__ void piece_sums_kernel(const T* __restrict__ X, long long ldx,
     const int b = label_off[j] + q * kSumPiece;
     const int e = min(b + kSumPiece, label_off[j + 1]);
     for (int d0 = 0; d0 < d; d0 += 256) {
-      PieceAcc<T> acc[8];
+      PieceAcc acc[8];
       double qs = 0.0;
 #pragma unroll 4
       for (int t = b; t < e; ++t) {
         const int i = __ldg(sorted + t);
-        const T* x = X + (size_t)i * ldx + d0;
+        const float* x = X + (size_t)i * ldx + d0;
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
           const int c = lane + 32 * r;
@@ -485,7 +473,7 @@ piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double*
   ring_issue(q, ptot, nw, X, ldx, qn, sorted, label_off, pstart, k, d, partq, ring0, lane, p0, f0);
   ring_issue(q, ptot, nw, X, ldx, qn, sorted, label_off, pstart, k, d, partq, ring0 + kSlotBytes,
              lane, p1, f1);
-  PieceAcc<float> a0, a1, a2, a3;
+  PieceAcc a0, a1, a2, a3;
   int slot_sum = 0, slot_issue = 2;
   for (;;) {
     int p2, f2;
@@ -515,7 +503,7 @@ piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double*
         o[3] = a3.value();
       }
     }
-    if (f0 & 2) a0 = a1 = a2 = a3 = PieceAcc<float>{};
+    if (f0 & 2) a0 = a1 = a2 = a3 = PieceAcc{};
     p0 = p1;
     f0 = f1;
     p1 = p2;
@@ -573,7 +561,7 @@ __global__ void piece_sums_small_kernel(const float* __restrict__ X, long long l
     const int c = 4 * sub;
     const bool on = live && c < d;
     const int n = e - b;
-    PieceAcc<float> a0, a1, a2, a3;
+    PieceAcc a0, a1, a2, a3;
     for (int t = 0; t < n; t += 8) {  // eight rows in flight per lane group
       int idx[8];
 #pragma unroll
@@ -633,8 +621,77 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
     piece_sums_ring_kernel<<<(unsigned)((rw + kRingWarps - 1) / kRingWarps), kRingWarps * 32, 0,
                              s>>>(X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, stop);
   } else
-    piece_sums_kernel<float><<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
+    piece_sums_kernel<<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
                                                     part, partq, stop);
+  kmgb::count_launches(1);
+  return cudaGetLastError();
+}
+
+// FP64 rows: one warp per (piece, chunk of 64 dimensions), two dimensions per lane (16 bytes where
+// rows are aligned), 16 rows' loads in flight; the additions per (piece, dimension) are in row order.
+// (A warp per piece with 4 rows in flight took 258 us for 400,000 x 64, K=256.)
+__global__ void __launch_bounds__(128)
+piece_sums_d_kernel(const double* __restrict__ X, long long ldx, const int* __restrict__ sorted,
+                    const int* __restrict__ label_off, const int* __restrict__ pstart, int k, int d,
+                    bool vec, double* __restrict__ part, const int* stop) {
+  if (stopped(stop)) return;
+  const int chunks = (d + 63) / 64;
+  const long long total = (long long)pstart[k] * chunks;
+  const int lane = threadIdx.x & 31;
+  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  constexpr int U = 16;
+  for (long long it = gw; it < total; it += nw) {
+    const int p = (int)(it / chunks), ch = (int)(it - (long long)p * chunks);
+    const int j = find_label(pstart, k, p);
+    const int b = label_off[j] + (p - pstart[j]) * kSumPiece;
+    const int e = min(b + kSumPiece, label_off[j + 1]);
+    const int c = ch * 64 + 2 * lane;
+    const bool on0 = c < d, on1 = c + 1 < d;
+    double s0 = 0.0, s1 = 0.0;
+    for (int t0 = b; t0 < e; t0 += 32) {
+      const int ids = t0 + lane < e ? __ldg(sorted + t0 + lane) : 0;
+#pragma unroll
+      for (int h = 0; h < 32; h += U) {
+        double2 v[U];
+#pragma unroll
+        for (int r = 0; r < U; ++r) {
+          const int i = __shfl_sync(0xffffffffu, ids, h + r);
+          v[r] = make_double2(0.0, 0.0);
+          if (t0 + h + r < e) {
+            const double* x = X + (size_t)i * ldx + c;
+            if (vec && on1) {
+              v[r] = __ldg(reinterpret_cast<const double2*>(x));
+            } else {
+              if (on0) v[r].x = __ldg(x);
+              if (on1) v[r].y = __ldg(x + 1);
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < U; ++r)
+          if (t0 + h + r < e) {
+            s0 += v[r].x;
+            s1 += v[r].y;
+          }
+      }
+    }
+    if (on0) part[(size_t)p * d + c] = s0;
+    if (on1) part[(size_t)p * d + c + 1] = s1;
+  }
+}
+
+cudaError_t launch_piece_sums(const float* X, long long ldx, const UpdateWork& w, cudaStream_t s) {
+  return launch_piece_sums_f32(X, ldx, nullptr, w.sorted, w.label_off, w.piece_cnt, w.k, w.d, w.part,
+                               nullptr, w.stop, w.max_pieces, s);
+}
+cudaError_t launch_piece_sums(const double* X, long long ldx, const UpdateWork& w, cudaStream_t s) {
+  const bool vec = ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  const long long items = w.max_pieces * ((w.d + 63) / 64);
+  const long long most = kmgb::num_sms() * 16LL;
+  const long long warps = items < most ? items : most;
+  piece_sums_d_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(
+      X, ldx, w.sorted, w.label_off, w.piece_cnt, w.k, w.d, vec, w.part, w.stop);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
@@ -884,20 +941,32 @@ cudaError_t launch_update(const float* X, const double* qn, const int* labels, f
 
 namespace {
 
-// Per-kernel ABI: add this tile's canonical per-center sums to FP64 accumulators.
+// Per-kernel ABI: add this tile's canonical per-center sums to FP64 accumulators. One warp per
+// (center, group of 32 dimensions), eight loads in flight, additions in piece order.
 __global__ void accumulate_kernel(const double* __restrict__ part, const int* __restrict__ label_off,
                                   const int* __restrict__ pstart, int k, int d,
                                   double* __restrict__ acc, int* __restrict__ acc_counts) {
-  const int j = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int groups = (d + 31) / 32;
+  const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (j >= k) return;
+  if (wid >= (long long)k * groups) return;
+  const int j = (int)(wid / groups), g = (int)(wid - (long long)j * groups);
   const int p0 = pstart[j], p1 = pstart[j + 1];
-  for (int c = lane; c < d; c += 32) {
+  const int c = g * 32 + lane;
+  if (c < d) {
     double s = 0.0;
-    for (int p = p0; p < p1; ++p) s += part[(size_t)p * d + c];
+    int p = p0;
+    for (; p + 8 <= p1; p += 8) {
+      double v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = __ldg(part + (size_t)(p + i) * d + c);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += v[i];
+    }
+    for (; p < p1; ++p) s += __ldg(part + (size_t)p * d + c);
     acc[(size_t)j * d + c] += s;
   }
-  if (lane == 0) acc_counts[j] += label_off[j + 1] - label_off[j];
+  if (g == 0 && lane == 0) acc_counts[j] += label_off[j + 1] - label_off[j];
 }
 
 // Host-streamed tiles: add this tile's canonical per-center sums, member counts and sum of
@@ -987,11 +1056,9 @@ cudaError_t launch_tile_accumulate(const T* X, long long ldx, const int* labels,
                                    double* acc, int* acc_counts, cudaStream_t s) {
   if (w.n <= 0 || w.k <= 0) return cudaSuccess;
   KMGB_CUDA_TRY(sort_by_label(labels, w, s));
-  long long warps = w.max_pieces < kmgb::num_sms() * 64LL ? w.max_pieces : kmgb::num_sms() * 64LL;
-  piece_sums_kernel<T><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(
-      X, ldx, nullptr, w.sorted, w.label_off, w.piece_cnt, w.k, w.d, w.part, nullptr, w.stop); kmgb::count_launches(1);
-  KMGB_CUDA_TRY(cudaGetLastError());
-  accumulate_kernel<<<(unsigned)(((long long)w.k * 32 + 255) / 256), 256, 0, s>>>(
+  KMGB_CUDA_TRY(launch_piece_sums(X, ldx, w, s));
+  const long long acc_warps = (long long)w.k * ((w.d + 31) / 32);
+  accumulate_kernel<<<(unsigned)((acc_warps * 32 + 255) / 256), 256, 0, s>>>(
       w.part, w.label_off, w.piece_cnt, w.k, w.d, acc, acc_counts); kmgb::count_launches(1);
   return cudaGetLastError();
 }

@@ -1,0 +1,113 @@
+"""ClosestCentersF/D on the tensor-core filter, CompactnessF/D and the norms at the sizes where their
+paths change: labels equal the FP64 evaluation of nb_j - 2 a.b_j (lowest index on ties) whatever
+the norms, the sums FP64's within the FP32 rounding of the outputs."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def exact_labels(A, B, nb):
+    A, B, nb = (np.asarray(v, np.float64) for v in (A, B, nb))
+    out = np.empty(len(A), np.int32)
+    for s in range(0, len(A), 4096):
+        acc = np.zeros((len(A[s:s + 4096]), B.shape[1]))
+        for t in range(B.shape[0]):  # the entry's order: one chain over the dimensions
+            acc += A[s:s + 4096, t, None] * B[None, t]
+        v = nb[None] - 2.0 * acc
+        v[np.isnan(v)] = np.inf
+        out[s:s + 4096] = v.argmin(1)
+    return out
+
+
+def closest(km, torch, A, B, nb, m0=3):
+    dev = "cuda"
+    F = A.dtype == np.float32
+    a, b, n = (torch.from_numpy(np.ascontiguousarray(v)).to(dev) for v in (A, B, nb))
+    out = torch.full((len(A) + m0,), -7, dtype=torch.int32, device=dev)
+    fn = km.ClosestCentersF if F else km.ClosestCentersD
+    assert fn(m0, A.shape[0], A.shape[1], a, B.shape[1], b, None, None, n, 0, None, None, out) == 0
+    got = out.cpu().numpy()
+    assert (got[:m0] == -7).all()
+    return got[m0:]
+
+
+# values on a grid of 1/8: every product and sum is exact in FP64, so equal values are exact ties
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k", [(20_000, 128, 256), (40_001, 33, 300), (9_000, 320, 129),
+                                   (30_000, 321, 64), (600_000, 7, 65), (70_000, 5, 3)])
+def test_closest_centers_grid(km, torch_cuda, dtype, n, d, k):
+    rng = np.random.default_rng(n + d + k)
+    A = (rng.integers(-40, 41, (n, d)) / 8).astype(dtype)
+    B = (rng.integers(-40, 41, (d, k)) / 8).astype(dtype)
+    B[:, k - 1] = B[:, 0]  # duplicate centers: the lower index wins
+    nb = (B.astype(np.float64) ** 2).sum(0).astype(dtype)
+    A[:k] = B.T[: min(k, n)]
+    assert np.array_equal(closest(km, torch_cuda, A, B, nb), exact_labels(A, B, nb))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("case", ["nan center", "inf norm", "minus inf norm", "zero norms",
+                                  "huge center", "inf row", "nan row", "all equal"])
+def test_closest_centers_special(km, torch_cuda, dtype, case):
+    rng = np.random.default_rng(5)
+    n, d, k = 20_000, 64, 256
+    A = (rng.integers(-40, 41, (n, d)) / 8).astype(dtype)
+    B = (rng.integers(-40, 41, (d, k)) / 8).astype(dtype)
+    nb = (B.astype(np.float64) ** 2).sum(0).astype(dtype)
+    if case == "nan center":
+        B[3, 7] = np.nan
+        nb[7] = np.nan
+    elif case == "inf norm":
+        nb[::2] = np.inf
+    elif case == "minus inf norm":
+        nb[9] = -np.inf
+    elif case == "zero norms":
+        nb[:] = 0
+    elif case == "huge center":
+        B[:, 11] *= dtype(2.0 ** 70)
+        nb = (B.astype(np.float64) ** 2).sum(0).astype(dtype)  # overflows to inf in FP32
+    elif case == "inf row":
+        A[17, 5] = np.inf
+    elif case == "nan row":
+        A[17, 5] = np.nan
+    else:
+        B[:] = B[:, :1]
+        nb[:] = nb[0]
+    with np.errstate(all="ignore"):
+        want = exact_labels(A, B, nb)
+    got = closest(km, torch_cuda, A, B, nb)
+    keep = np.ones(n, bool)
+    if case == "inf row":
+        keep[17] = False  # infinite values: the entry's label is a tie among infinities
+    assert np.array_equal(got[keep], want[keep])
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("m,d,k,scale", [(1, 1, 1, 1.0), (70_001, 128, 40, 1.0), (5_000, 30, 7, 1.0),
+                                         (3_000, 12, 5, 1e-18), (3_000, 16, 5, 1e19), (999, 200, 3, 0.0),
+                                         (2_000, 77, 2, 1e4)])
+def test_compactness_and_norms(km, torch_cuda, dtype, m, d, k, scale):
+    torch = torch_cuda
+    rng = np.random.default_rng(m + d)
+    X = (rng.standard_normal((m, d)) * scale).astype(dtype)
+    C = (rng.standard_normal((k, d)) * scale).astype(dtype)
+    lab = rng.integers(0, k, m).astype(np.int32)
+    F = dtype == np.float32
+    x, c, l = (torch.from_numpy(v).cuda() for v in (X, C, lab))
+    out = torch.zeros(4, dtype=x.dtype, device="cuda")
+    fn = km.CompactnessF if F else km.CompactnessD
+    assert fn(0, m, True, d, k, x, l, c, out) == 0
+    with np.errstate(over="ignore"):
+        want = dtype(((X.astype(np.float64) - C.astype(np.float64)[lab]) ** 2).sum())
+        rows = (X.astype(np.float64) ** 2).sum(1)
+        cols = (X.astype(np.float64) ** 2).sum(0)
+        # FP32 outputs are one rounding of (nearly) FP64 values; subnormal results keep absolute steps
+        tol = dict(rtol=1.3e-7, atol=3e-45) if F else dict(rtol=1e-12, atol=0)
+        np.testing.assert_allclose(out.cpu().numpy()[0], want, **tol)
+        r = torch.zeros(m + 2, dtype=x.dtype, device="cuda")
+        q = torch.zeros(d, dtype=x.dtype, device="cuda")
+        assert (km.rowNormalizeF if F else km.rowNormalizeD)(2, m, d, x, r) == 0
+        assert (km.colNormalizeF if F else km.colNormalizeD)(m, d, x, q) == 0
+        np.testing.assert_allclose(r.cpu().numpy()[2:], rows.astype(dtype), **tol)
+        np.testing.assert_allclose(q.cpu().numpy(), cols.astype(dtype), **tol)
