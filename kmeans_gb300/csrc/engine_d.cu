@@ -5,8 +5,9 @@
 // (cublasDgemm + rowTransformMinimumD, kmeans.cpp:958-993) defines FP64 behaviour. This path
 // computes what that one intends, exactly: label = FP64 arg-min of sum_d (x_d - c_d)^2 (lowest
 // index on ties), centers = canonical FP64 sums / counts, SSE in FP64 against the new centers.
-// FP64 throughput on GB300 is low (about 1.25 TFLOP/s), so this is the correctness path, not a
-// fast one; every kernel is plain SIMT.
+// FP64 throughput on GB300 is low (about 1.25 TFLOP/s): full batches take the tensor cores as a
+// filter on FP32 roundings and settle the few open rows from recorded candidates in FP64, and the
+// update and the SSE, two FP64 operations per element, run over the clusters whose members changed.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -86,37 +87,76 @@ __global__ void d2f_kernel(const double* __restrict__ in, long long rows, int d,
   }
 }
 
-__global__ void sse_d_partial_kernel(const double* __restrict__ X, long long n, int d,
-                                     const int* __restrict__ lab, const double* __restrict__ C,
-                                     double* __restrict__ partial) {
-  __shared__ double red[8];
-  const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double acc = 0.0;
-  for (long long i = (long long)blockIdx.x * warps + w; i < n; i += (long long)gridDim.x * warps) {
-    const int l = lab[i];
-    double s = 0.0;
-    for (int t = lane; t < d; t += 32) {
-      const double u = X[(size_t)i * d + t] - C[(size_t)l * d + t];
-      s = fma(u, u, s);
+// SSE against the new centers, by the pieces of the label-sorted rows (kSumPiece rows of one cluster
+// each, as the canonical sums): one warp per piece, lanes over the dimensions, four rows in flight;
+// the lanes meet once per piece.
+__global__ void __launch_bounds__(128)
+sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ sorted,
+                  const int* __restrict__ label_off, const int* __restrict__ pstart, int k,
+                  const double* __restrict__ C, double* __restrict__ piece) {
+  const int total = pstart[k];
+  const int lane = threadIdx.x & 31;
+  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  constexpr int U = 4;
+  for (int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); p < total; p += nw) {
+    int lo = 0, hi = k - 1;  // the cluster of piece p
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(pstart + mid) <= p) lo = mid;
+      else hi = mid - 1;
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    acc += s;
-  }
-  if (lane == 0) red[w] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < warps; ++i) t += red[i];
-    partial[blockIdx.x] = t;
+    const int b = label_off[lo] + (p - pstart[lo]) * kSumPiece;
+    const int e = min(b + kSumPiece, label_off[lo + 1]);
+    const double* c = C + (size_t)lo * d;
+    double acc = 0.0;
+    for (int t0 = b; t0 < e; t0 += 32) {
+      const int ids = t0 + lane < e ? __ldg(sorted + t0 + lane) : 0;
+      const int cnt = min(32, e - t0);
+      for (int h = 0; h < cnt; h += U) {
+        const double* x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          x[u] = X + (size_t)__shfl_sync(0xffffffffu, ids, min(h + u, cnt - 1)) * d;
+        for (int t = lane; t < d; t += 32) {
+          const double cv = __ldg(c + t);
+          double v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) v[u] = __ldg(x[u] + t) - cv;
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (h + u < cnt) acc = fma(v[u], v[u], acc);
+        }
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) piece[p] = acc;
   }
 }
 
-__global__ void sse_d_final_kernel(const double* __restrict__ partial, int nb, double* out) {
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < nb; ++i) t += partial[i];
-    *out = t;
+// One block: every cluster's SSE from its pieces (in order; a cluster without pieces in this
+// iteration keeps its value), and their sum.
+__global__ void __launch_bounds__(1024)
+sse_d_final_kernel(const double* __restrict__ piece, const int* __restrict__ pstart, int k,
+                   const int* __restrict__ dirty, double* __restrict__ sse_k, double* out) {
+  __shared__ double red[1024];
+  double t = 0.0;
+  for (int j = threadIdx.x; j < k; j += 1024) {
+    if (!dirty || dirty[j]) {
+      double s = 0.0;
+      const int p1 = pstart[j + 1];
+#pragma unroll 4
+      for (int p = pstart[j]; p < p1; ++p) s += piece[p];
+      sse_k[j] = s;
+    }
+    t += sse_k[j];
   }
+  red[threadIdx.x] = t;
+  __syncthreads();
+  for (int w = 512; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *out = red[0];
 }
 
 __global__ void gather_d_kernel(const double* __restrict__ X, int d, const int* __restrict__ perm,
@@ -131,15 +171,20 @@ __global__ void gather_d_kernel(const double* __restrict__ X, int d, const int* 
   }
 }
 
+// Device buffers from the library's pool (a call's some twenty cudaMalloc and cudaFree, each of
+// which waits for the device, took about 2 ms), given back when the call ends.
 struct DevBufs {
   std::vector<void*> ptrs;
   ~DevBufs() {
-    for (void* p : ptrs) cudaFree(p);
+    cudaStreamSynchronize(0);
+    for (void* p : ptrs) dev_free(p, 0);
   }
   template <typename T>
   cudaError_t alloc(T** p, size_t count) {
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (count ? count : 1));
-    if (e == cudaSuccess) ptrs.push_back(*p);
+    void* v = nullptr;
+    const cudaError_t e = dev_alloc_async(&v, sizeof(T) * (count ? count : 1), 0);
+    *p = static_cast<T*>(v);
+    if (e == cudaSuccess) ptrs.push_back(v);
     return e;
   }
 };
@@ -148,6 +193,48 @@ struct DevBufs {
   do {                                    \
     if ((expr) != cudaSuccess) return (code); \
   } while (0)
+
+// Distance bounds: as the FP32-data engine's, but from a fifth of its work on, since here the FP64
+// sums and SSE of the unchanged clusters are saved as well (400,000 x 64, K=256).
+bool prune_worthwhile(long long m, int k, int d) {
+  const long long kp = (k + kCenterPad - 1) / kCenterPad * kCenterPad;
+  return k >= 2 && (long long)k * 32 <= m && m * kp >= (1LL << 31) / d;
+}
+
+// The bounds' buffers; where they do not fit, every iteration scans every row.
+void alloc_prune_d(DevBufs& B, PruneState* out, int** crr, long long m, int k, long long ldb) {
+  PruneState p;
+  p.n = m;
+  p.k = k;
+  p.cap = (int)std::min(m * 13 / 20, (8LL << 30) / (ldb * 4));
+  if (p.cap < 256) return;
+  bool ok = true;
+  auto take = [&](auto** q, size_t count) { ok = ok && B.alloc(q, count) == cudaSuccess; };
+  uint16_t *xc = nullptr, *xlc = nullptr;
+  take(&p.ub, m);
+  take(&p.lb, m);
+  take(&p.shift, k);
+  take(&p.cxn, k);
+  take(&p.cub, k);
+  take(&p.clb, k);
+  take(&p.clab, k);
+  take(crr, k);
+  take(&p.list, p.cap);
+  take(&p.lab_old, m);
+  take(&p.dirty, k);
+  take(&p.flags, 4);
+  take(&p.top, 2);
+  take(&xc, (size_t)p.cap * ldb);
+  take(&xlc, (size_t)p.cap * ldb);
+  ok = ok && cudaMemsetAsync(p.flags, 0, 4 * sizeof(int), 0) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    return;
+  }
+  p.Xc = xc;
+  p.Xlc = xlc;
+  *out = p;
+}
 
 // One FP64 run. kpp_seed < 0: the reference initialisation; else k-means++ with that seed (on the
 // device, from the uploaded data). result receives the initial then the final centers (D x K);
@@ -180,7 +267,7 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
 
   DevBufs B;
   double *X = nullptr, *Xw = nullptr, *Cd = nullptr, *CT = nullptr, *acc = nullptr, *part = nullptr,
-         *sse = nullptr;
+         *sse = nullptr, *sse_k = nullptr;
   int *lab = nullptr, *cnt = nullptr, *permd = nullptr;
   const cudaStream_t s = 0;
   const kmeansErrorStatus E = KMEANS_ERROR_BUILDDATA;
@@ -213,8 +300,6 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   KD_TRY(B.alloc(&acc, (size_t)k * n), E);
   KD_TRY(B.alloc(&cnt, k), E);
   KD_TRY(B.alloc(&lab, m_mb), E);
-  const int sse_blocks = kmgb::num_sms() * 4;
-  KD_TRY(B.alloc(&part, sse_blocks), E);
   KD_TRY(B.alloc(&sse, 1), E);
   if (kpp_seed < 0) {
     KD_TRY(cudaMemcpy(Cd, C.data(), sizeof(double) * C.size(), cudaMemcpyHostToDevice), E);
@@ -253,6 +338,8 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   KD_TRY(B.alloc(&w.piece_cnt, k + 1), E);
   KD_TRY(B.alloc(&w.sorted, m_mb), E);
   KD_TRY(B.alloc(&w.part, (size_t)w.max_pieces * n), E);
+  KD_TRY(B.alloc(&part, w.max_pieces), E);
+  KD_TRY(B.alloc(&sse_k, k), E);
 
   // Tensor path (full batches, D within the split tier's limit): X and the centers are rounded
   // to FP32, the split BF16 tier assigns every point under its bound widened by that rounding
@@ -264,8 +351,15 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   const long long ldx = (n + 3) / 4 * 4, ldb = (n + 7) / 8 * 8;
   float *xn = nullptr, *Cf = nullptr, *Cop = nullptr, *cn = nullptr,
         *cmax = nullptr, *cinit = nullptr;
-  uint16_t *Xb = nullptr, *Xl = nullptr, *Cb = nullptr, *Cl = nullptr;
-  int *rr_list = nullptr, *rr_count = nullptr, *derr = nullptr;
+  uint16_t *Xb = nullptr, *Xl = nullptr, *Cb = nullptr, *Cl = nullptr, *cbias = nullptr,
+           *XbC = nullptr, *XlC = nullptr;
+  float *thr = nullptr, *thrC = nullptr;
+  int *rr_list = nullptr, *rr_count = nullptr, *derr = nullptr, *over = nullptr, *cand = nullptr,
+      *cand_cnt = nullptr;
+  // rows of the candidate pass's compact copies; flagged rows past it take the FP64 scan
+  const long long cap = std::min<long long>(m, std::max<long long>(1024, m / 8));
+  PruneState pr;
+  int* crr_list = nullptr;
   if (tc) {
     const kmeansErrorStatus EA = KMEANS_ERROR_CLOSEST_CENTERS;
     KD_TRY(B.alloc(&xn, m), E);
@@ -278,6 +372,15 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
     KD_TRY(B.alloc(&cn, k), E);
     KD_TRY(B.alloc(&cmax, 1), E);
     KD_TRY(B.alloc(&cinit, (size_t)((k + kCenterPad - 1) / kCenterPad * kCenterPad)), E);
+    KD_TRY(B.alloc(&cbias, (size_t)((k + kCenterPad - 1) / kCenterPad * kCenterPad) * kBiasCols), E);
+    KD_TRY(B.alloc(&thr, m), E);
+    KD_TRY(B.alloc(&thrC, cap), E);
+    KD_TRY(B.alloc(&XbC, (size_t)cap * ldb), E);
+    KD_TRY(B.alloc(&XlC, (size_t)cap * ldb), E);
+    KD_TRY(B.alloc(&cand, (size_t)cap * kMaxCand), E);
+    KD_TRY(B.alloc(&cand_cnt, cap), E);
+    KD_TRY(B.alloc(&over, m), E);
+    if (maxIters > 1 && prune_worthwhile(m, k, n)) alloc_prune_d(B, &pr, &crr_list, m, k, ldb);
     KD_TRY(B.alloc(&rr_list, m), E);
     KD_TRY(B.alloc(&rr_count, 3), E);
     KD_TRY(B.alloc(&derr, 1), E);
@@ -307,12 +410,16 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
       d2f_kernel<<<kmgb::num_sms() * 4, 256, 0, s>>>(Cd, k, n, Cf, ldx); kmgb::count_launches(1);
       KD_TRY(cudaMemsetAsync(cmax, 0, sizeof(float), s), EA);
       KD_TRY(cudaMemsetAsync(rr_count, 0, 3 * sizeof(int), s), EA);
-      KD_TRY(launch_prep_centers(Cf, ldx, k, n, Cop, Cb, ldb, cn, cmax, s, nullptr, cinit, Cl), EA);
+      KD_TRY(launch_prep_centers(Cf, ldx, k, n, Cop, Cb, ldb, cn, cmax, s, nullptr, cinit, Cl, cbias,
+                                 pr.shift, pr.cxn, 0x1p-22f),
+             EA);
       AssignArgs a{};
       a.cn = cn;
       a.xnorm = xn;
       a.cmax = cmax;
       a.cinit = cinit;
+      a.cbias = cbias;
+      a.thr_out = thr;
       a.labels = lab;
       a.rerank_list = rr_list;
       a.rerank_count = rr_count;
@@ -323,9 +430,70 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
       a.certify = 1;
       a.gamma = assign_bf16_gamma(n);
       a.pert = 0x1p-22f;
-      KD_TRY(launch_assign_bf16(Xb, Xl, ldb, Cb, Cl, ldb, a, s), EA);
-      assign_d_kernel<<<kmgb::num_sms() * 8, threads, smem, s>>>(X, m, n, CT, k, lab, rr_list, rr_count);
+      AssignArgs af = a;
+      if (pr.n > 0) {  // distance bounds (prune.cu)
+        AssignArgs c = a;
+        c.n = k;
+        c.n_dev = pr.flags;
+        c.xnorm = pr.cxn;
+        c.labels = pr.clab;
+        c.rerank_list = crr_list;
+        c.rerank_count = pr.flags + 2;
+        c.thr_out = nullptr;
+        c.ub = pr.cub;
+        c.lb = pr.clb;
+        KD_TRY(launch_assign_bf16(Cb, Cl, ldb, Cb, Cl, ldb, c, s), EA);
+        KD_TRY(launch_prune_filter(pr, lab, nullptr, s), EA);
+        KD_TRY(launch_prune_gather(pr, Xb, Xl, ldb * 2, nullptr, s), EA);
+        af.ub = pr.ub;
+        af.lb = pr.lb;
+        af.sel = pr.flags + 1;
+        af.sel_cap = pr.cap;
+        af.row_map = pr.list;
+        af.Xc = pr.Xc;
+        af.Xlc = pr.Xlc;
+      }
+      KD_TRY(launch_assign_bf16(Xb, Xl, ldb, Cb, Cl, ldb, af, s), EA);
+      // flagged rows: their candidates from a second pass, settled in FP64; rows without a record
+      // take the FP64 scan (every flagged row scanned: 183 us an iteration at 400,000 x 64, K=256)
+      KD_TRY(launch_gather_flagged(rr_list, rr_count, cap, Xb, Xl, ldb * 2, thr, XbC, XlC, thrC, over,
+                                   rr_count + 1, nullptr, s),
+             EA);
+      AssignArgs c2 = a;
+      c2.n = cap;
+      c2.n_dev = rr_count;
+      c2.labels = nullptr;
+      c2.certify = 0;
+      c2.thr_out = nullptr;
+      c2.thr_in = thrC;
+      c2.cand = cand;
+      c2.cand_cnt = cand_cnt;
+      KD_TRY(launch_assign_bf16(XbC, XlC, ldb, Cb, Cl, ldb, c2, s), EA);
+      ResolveD rd{};
+      rd.X = X;
+      rd.ldx = n;
+      rd.C = Cd;
+      rd.c_dim = 1;
+      rd.c_row = n;
+      rd.d = n;
+      rd.k = k;
+      rd.mode = 0;
+      rd.list = rr_list;
+      rd.count = rr_count;
+      rd.max_list = cap;
+      rd.cand = cand;
+      rd.cand_cnt = cand_cnt;
+      rd.labels = lab;
+      rd.over = over;
+      rd.over_count = rr_count + 1;
+      KD_TRY(launch_resolve_fp64(rd, s), EA);
+      assign_d_kernel<<<kmgb::num_sms() * 8, threads, smem, s>>>(X, m, n, CT, k, lab, over,
+                                                                 rr_count + 1);
       kmgb::count_launches(1);
+      if (pr.n > 0) {
+        KD_TRY(launch_prune_dirty(pr, lab, nullptr, s), EA);
+        w.dirty = pr.dirty;
+      }
     } else {
       assign_d_kernel<<<kmgb::num_sms() * 8, threads, smem, s>>>(Xa, m_mb, n, CT, k, lab);
       kmgb::count_launches(1);
@@ -334,9 +502,12 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
     KD_TRY(cudaMemsetAsync(acc, 0, sizeof(double) * (size_t)k * n, s), KMEANS_ERROR_RESET);
     KD_TRY(cudaMemsetAsync(cnt, 0, sizeof(int) * k, s), KMEANS_ERROR_RESET);
     KD_TRY(launch_tile_accumulate<double>(Xa, n, lab, w, acc, cnt, s), KMEANS_ERROR_CLUSTER_CENTERS);
-    KD_TRY(launch_finalize_acc<double>(acc, cnt, k, n, Cd, nullptr, s), KMEANS_ERROR_CLUSTER_CENTERS);
-    sse_d_partial_kernel<<<sse_blocks, 256, 0, s>>>(Xa, m_mb, n, lab, Cd, part); kmgb::count_launches(1);
-    sse_d_final_kernel<<<1, 32, 0, s>>>(part, sse_blocks, sse); kmgb::count_launches(1);
+    KD_TRY(launch_finalize_acc<double>(acc, cnt, k, n, Cd, nullptr, s, w.dirty),
+           KMEANS_ERROR_CLUSTER_CENTERS);
+    sse_pieces_kernel<<<kmgb::num_sms() * 8, 128, 0, s>>>(Xa, n, w.sorted, w.label_off, w.piece_cnt, k,
+                                                          Cd, part);
+    sse_d_final_kernel<<<1, 1024, 0, s>>>(part, w.piece_cnt, k, w.dirty, sse_k, sse);
+    kmgb::count_launches(2);
     KD_TRY(cudaGetLastError(), KMEANS_ERROR_COMPACTNESS);
     double h = 0.0;
     KD_TRY(cudaMemcpy(&h, sse, sizeof(double), cudaMemcpyDeviceToHost), KMEANS_ERROR_COMPACTNESS);

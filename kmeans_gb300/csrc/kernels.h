@@ -222,13 +222,15 @@ cudaError_t launch_resolve_fp64(const ResolveD& a, cudaStream_t s);
 // start values split exactly into three BF16 numbers (columns 0..2, the rest zero), the B
 // operand of the pair kernel's start-value MMA. shift (nullable): upper bound of the distance
 // from the row Cop holds (the previous centers) to the new one, +inf from an unusable row, -1 for
-// a center that is unusable now; cxn (nullable): upper bound of ||c_j|| (0 when unusable).
+// a center that is unusable now; cxn (nullable): upper bound of ||c_j|| (0 when unusable);
+// shift_pert: relative rounding of C's rows (FP64 centers), added to the moves.
 constexpr int kBiasCols = 16;
 cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, float* Cop,
                                 void* Cb, long long ldcb, float* cn, float* cmax, cudaStream_t s,
                                 const int* stop = nullptr, float* cinit = nullptr,
                                 void* Cl = nullptr, void* cbias = nullptr,
-                                float* shift = nullptr, float* cxn = nullptr);
+                                float* shift = nullptr, float* cxn = nullptr,
+                                float shift_pert = 0.0f);
 
 // Distance bounds within one run (prune.cu): which rows an iteration has to scan again.
 struct PruneState {
@@ -337,7 +339,7 @@ cudaError_t launch_tile_accumulate(const T* X, long long ldx, const int* labels,
                                    double* acc, int* acc_counts, cudaStream_t s);
 template <typename T>
 cudaError_t launch_finalize_acc(const double* acc, const int* acc_counts, int k, int d, T* centers,
-                                int* counts, cudaStream_t s);
+                                int* counts, cudaStream_t s, const int* dirty = nullptr);
 void plan_update_tiles(long long n, int k, int* tile_pts, int* ntiles);
 // Host-streamed tiles: per tile, label sort + canonical piece sums (with sum of ||x||^2) added to
 // FP64 accumulators accS[k][d], accN[k], accQ[k]; after the last tile, centers, SSE and the stop

@@ -37,7 +37,7 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
                                     const int* stop, float* __restrict__ cinit, int kpad,
                                     __nv_bfloat16* __restrict__ Cl,
                                     __nv_bfloat16* __restrict__ cbias, float* __restrict__ shift,
-                                    float* __restrict__ cxn) {
+                                    float* __restrict__ cxn, float shift_pert) {
   if (stopped(stop)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -76,7 +76,10 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
       const float mv = (mx == 0.0f || (m2 > 1e-28f && m2 < 1e37f))
                            ? __fsqrt_ru(__fmul_ru(m2, slack))
                            : __fmul_ru(__fmul_ru(mx, 1.000001f), __fsqrt_ru((float)d));
-      shift[warp] = bad ? -1.0f : (was_bad ? INFINITY : mv);
+      // FP64 centers: each end of the move is a rounding away from its center
+      const float pt = shift_pert > 0.0f
+                           ? __fmul_ru(shift_pert, __fadd_ru(__double2float_ru(sqrt(s)), mv)) : 0.0f;
+      shift[warp] = bad ? -1.0f : (was_bad ? INFINITY : __fadd_ru(mv, pt));
     }
     __syncwarp();
   }
@@ -186,8 +189,10 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
          i += (long long)gridDim.x * blockDim.x)
       rl.over[atomicAdd(rl.over_count, 1)] = rl.list[i];
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-      rl.thr_out[i] = rl.thr[rl.list[i]];
+         i += (long long)gridDim.x * blockDim.x) {
+      const float fl = rl.thr[rl.list[i]];  // without a finite floor: no candidates
+      rl.thr_out[i] = fl > -3.0e38f ? fl : INFINITY;
+    }
   }
   auto source = [&](long long r) { return IDX == 1 ? (long long)__ldg(rl.list + r) : r; };
   constexpr int G = 32 / L;  // rows per warp and step
@@ -438,7 +443,7 @@ cudaError_t launch_centers_fp8(const float* Cop, long long ldc, int k, int d, co
 cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, float* Cop, void* Cb,
                                 long long ldcb, float* cn, float* cmax, cudaStream_t s,
                                 const int* stop, float* cinit, void* Cl, void* cbias,
-                                float* shift, float* cxn) {
+                                float* shift, float* cxn, float shift_pert) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (k <= 0) return cudaSuccess;
   const int threads = 256;
@@ -449,7 +454,7 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
                                                  cmax, stop, cinit, kpad,
                                                  reinterpret_cast<__nv_bfloat16*>(Cl),
                                                  reinterpret_cast<__nv_bfloat16*>(cbias), shift,
-                                                 cxn);
+                                                 cxn, shift_pert);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }

@@ -648,7 +648,10 @@ __global__ void gather_flagged_kernel(const int* __restrict__ list, const int* _
       if (Xl) XlC[slot * row_vec + v] = Xl[pt * row_vec + v];
     }
     if (lane == 0) {
-      thrC[slot] = thr[pt];
+      // without a finite floor (no usable center, an infinite bound) the keys say nothing: no
+      // candidates, hence the full rescan
+      const float fl = thr[pt];
+      thrC[slot] = fl > -3.0e38f ? fl : INFINITY;
       if (xs) xsC[slot] = xs[pt];
     }
   }

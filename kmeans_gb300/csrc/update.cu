@@ -1031,11 +1031,13 @@ __global__ void finalize_stream_kernel(const double* __restrict__ accS, const in
 
 template <typename T>
 __global__ void finalize_acc_kernel(const double* __restrict__ acc, const int* __restrict__ acc_counts,
-                                    int k, int d, T* __restrict__ centers, int* __restrict__ counts) {
+                                    int k, int d, T* __restrict__ centers, int* __restrict__ counts,
+                                    const int* __restrict__ dirty) {
   const long long total = (long long)k * d;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(e / d);
+    if (dirty && !dirty[j]) continue;
     const int n = acc_counts[j];
     T v;
     if (n > 0) {
@@ -1065,8 +1067,10 @@ cudaError_t launch_tile_accumulate(const T* X, long long ldx, const int* labels,
 
 template <typename T>
 cudaError_t launch_finalize_acc(const double* acc, const int* acc_counts, int k, int d, T* centers,
-                                int* counts, cudaStream_t s) {
-  finalize_acc_kernel<T><<<kmgb::num_sms() * 4, 256, 0, s>>>(acc, acc_counts, k, d, centers, counts); kmgb::count_launches(1);
+                                int* counts, cudaStream_t s, const int* dirty) {
+  finalize_acc_kernel<T><<<kmgb::num_sms() * 4, 256, 0, s>>>(acc, acc_counts, k, d, centers, counts,
+                                                             dirty);
+  kmgb::count_launches(1);
   return cudaGetLastError();
 }
 
@@ -1103,9 +1107,9 @@ template cudaError_t launch_tile_accumulate<float>(const float*, long long, cons
 template cudaError_t launch_tile_accumulate<double>(const double*, long long, const int*,
                                                     const UpdateWork&, double*, int*, cudaStream_t);
 template cudaError_t launch_finalize_acc<float>(const double*, const int*, int, int, float*, int*,
-                                                cudaStream_t);
+                                                cudaStream_t, const int*);
 template cudaError_t launch_finalize_acc<double>(const double*, const int*, int, int, double*, int*,
-                                                 cudaStream_t);
+                                                 cudaStream_t, const int*);
 
 // ---------------------------------------------------------------------------------------
 // Batched Lloyd: many problems of one dimension share X (problem p: rows row_beg[p] ..

@@ -80,3 +80,17 @@ def test_bounds_end_with_the_run(km, orc, torch_cuda, monkeypatch):
         monkeypatch.setenv("KMGB_GRAPHS", graphs)
         check(km.lloyd(X, k, init=i1, max_iters=40, criterion=1e-3, empty_policy=1,
                        assign_tier=km.ASSIGN_BF16X3), want, "criterion")
+
+
+@pytest.mark.parametrize("n,d,k,span", [(70_001, 128, 250, 20.0), (150_000, 66, 256, 2.0)])
+def test_fp64_driver(km, orc, torch_cuda, n, d, k, span):
+    """computeKmeansD with bounds: FP64-only digits in the rows, exact duplicates."""
+    X, _, _ = mixture_numpy(n, d, k, seed=n, mean_lo=-span, mean_hi=span, std=(0.5, 2.0))
+    X = X.astype(np.float64) + np.random.default_rng(1).uniform(0, 1e-9, X.shape)
+    X[50:90] = X[50]
+    _, perm, picks = km.reference_init(X.astype(np.float32), k)
+    init = X[perm[picks]]
+    result = np.empty(k * d)
+    assert km.computeKmeansD(X, n, d, k, -1.0, 6, 1, 0, 0, 0, result, 1.0) == 13
+    _, c, _, _, _ = orc.lloyd_d(X, init, 6)
+    assert np.array_equal(result.reshape(d, k).T, c, equal_nan=True)
