@@ -241,9 +241,7 @@ struct kmgb_handle {
   void* prune_arena = nullptr;
   int* crr_list = nullptr;  // scratch of the centers' own scan
   // k-means++ work space (allocated on first use): D^2, block weight sums, max/pick, picks
-  float* kpp_d2 = nullptr;
-  unsigned long long* kpp_blk = nullptr;
-  unsigned long long* kpp_sc = nullptr;
+  KppWork<float> kpp;
   int* kpp_picks = nullptr;
   // device-side loop state: stop flag, previous SSE, last relErr, iterations done
   int* stop = nullptr;
@@ -292,7 +290,7 @@ struct kmgb_handle {
     if (stream) {
       cudaStreamSynchronize(stream);
       // the fixed buffers live in the arena; these are allocated on their own
-      void* ptrs[] = {arena, sse_dev, kpp_d2, kpp_blk, kpp_sc, kpp_picks, fb_arena, shard_arena,
+      void* ptrs[] = {arena, sse_dev, kpp.d2, kpp.blocksum, kpp.scalars, kpp.near, kpp.cc, kpp_picks, fb_arena, shard_arena,
                       prune_arena};
       for (void* p : ptrs) dev_free(p, stream);
       router_destroy(router, stream);
@@ -1498,6 +1496,23 @@ int set_centers(kmgb_handle* h, const float* C, bool on_device) {
   return 0;
 }
 
+// k-means++ work space (what is there already stays); without room for the row-skipping test's
+// arrays every draw reads every row.
+template <typename T>
+cudaError_t alloc_kpp(KppWork<T>* w, long long n, int k, cudaStream_t s) {
+  cudaError_t r = w->d2 ? cudaSuccess : dalloc(&w->d2, (size_t)kmeanspp_d2_elems(n), s);
+  if (r == cudaSuccess && !w->blocksum) r = dalloc(&w->blocksum, (size_t)kmeanspp_blocks(n), s);
+  if (r == cudaSuccess && !w->scalars) r = dalloc(&w->scalars, kKppScalars, s);
+  if (r != cudaSuccess) return r;
+  if (!w->cc && (dalloc(&w->near, (size_t)n, s) != cudaSuccess ||
+                 dalloc(&w->cc, (size_t)k, s) != cudaSuccess)) {
+    cudaGetLastError();
+    dev_free(w->near, s);
+    w->near = nullptr;
+  }
+  return cudaSuccess;
+}
+
 // k-means++ centers from the resident data into h->C (launch_kmeanspp); picks_out: host, k.
 int init_kmeanspp(kmgb_handle* h, unsigned long long seed, int* picks_out) {
   const int code = KMEANS_ERROR_INITIALIZE;
@@ -1510,15 +1525,13 @@ int init_kmeanspp(kmgb_handle* h, unsigned long long seed, int* picks_out) {
     set_err("k-means++ needs 0 < k <= n");
     return code;
   }
-  if (!h->kpp_d2) {
-    KM_TRY(dalloc(&h->kpp_d2, (size_t)kmeanspp_d2_elems(h->n), h->stream), code);
-    KM_TRY(dalloc(&h->kpp_blk, (size_t)kmeanspp_blocks(h->n), h->stream), code);
-    KM_TRY(dalloc(&h->kpp_sc, 3, h->stream), code);
+  if (!h->kpp_picks) {
+    KM_TRY(alloc_kpp(&h->kpp, h->n, h->k, h->stream), code);
     KM_TRY(dalloc(&h->kpp_picks, (size_t)h->k, h->stream), code);
   }
   KM_TRY(cudaMemsetAsync(h->C, 0, sizeof(float) * h->ldx * h->k, h->stream), code);
   KM_TRY(launch_kmeanspp(h->X, h->ldx, h->n, h->d, h->k, seed, h->C, h->ldx, h->kpp_picks,
-                         h->kpp_d2, h->kpp_blk, h->kpp_sc, h->err, h->stream),
+                         h->kpp, h->err, h->stream),
          code);
   if (picks_out)
     KM_TRY(cudaMemcpyAsync(picks_out, h->kpp_picks, sizeof(int) * h->k, cudaMemcpyDeviceToHost,
@@ -1689,8 +1702,8 @@ int kmeanspp_oneshot(const T* X, long long n, int d, int k, unsigned long long s
     return code;
   }
   const bool x_dev = is_device_ptr(X);
-  T *Xd = nullptr, *Cd = nullptr, *d2 = nullptr;
-  unsigned long long *blk = nullptr, *sc = nullptr;
+  T *Xd = nullptr, *Cd = nullptr;
+  KppWork<T> w;
   int *kp = nullptr, *err = nullptr;
   int rc = 0;
   // host data is uploaded with 16-byte aligned rows (the bulk-copy D^2 kernel's layout)
@@ -1706,21 +1719,19 @@ int kmeanspp_oneshot(const T* X, long long n, int d, int k, unsigned long long s
   if (x_dev) {
     fail(cudaStreamSynchronize(nullptr), "k-means++ (legacy stream)");
   } else {
-    fail(dalloc(&Xd, (size_t)n * ldx), "k-means++ (data)");
+    fail(dalloc(&Xd, (size_t)n * ldx, s), "k-means++ (data)");
     if (!rc)
       fail(cudaMemcpy2DAsync(Xd, sizeof(T) * ldx, X, sizeof(T) * d, sizeof(T) * d, n,
                              cudaMemcpyHostToDevice, s),
            "k-means++ (upload)");
   }
-  if (!rc) fail(dalloc(&Cd, (size_t)k * d), "k-means++ (centers)");
-  if (!rc) fail(dalloc(&d2, (size_t)kmeanspp_d2_elems(n)), "k-means++ (D^2)");
-  if (!rc) fail(dalloc(&blk, (size_t)kmeanspp_blocks(n)), "k-means++ (sums)");
-  if (!rc) fail(dalloc(&sc, 3), "k-means++ (scalars)");
-  if (!rc) fail(dalloc(&kp, (size_t)k), "k-means++ (picks)");
-  if (!rc) fail(dalloc(&err, 1), "k-means++ (error word)");
+  if (!rc) fail(dalloc(&Cd, (size_t)k * d, s), "k-means++ (centers)");
+  if (!rc) fail(alloc_kpp(&w, n, k, s), "k-means++ (work space)");
+  if (!rc) fail(dalloc(&kp, (size_t)k, s), "k-means++ (picks)");
+  if (!rc) fail(dalloc(&err, 1, s), "k-means++ (error word)");
   if (!rc) fail(cudaMemsetAsync(err, 0, sizeof(int), s), "k-means++ (error word)");
   if (!rc)
-    fail(launch_kmeanspp(x_dev ? X : Xd, ldx, n, d, k, seed, Cd, d, kp, d2, blk, sc, err, s),
+    fail(launch_kmeanspp(x_dev ? X : Xd, ldx, n, d, k, seed, Cd, d, kp, w, err, s),
          "k-means++ (kernels)");
   if (!rc && centers)
     fail(cudaMemcpyAsync(centers, Cd, sizeof(T) * (size_t)k * d,
@@ -1737,9 +1748,10 @@ int kmeanspp_oneshot(const T* X, long long n, int d, int k, unsigned long long s
     set_err("k-means++: a bounded wait in the D^2 kernel gave up (device error word set)");
     rc = code;
   }
+  for (void* p : {(void*)Xd, (void*)Cd, (void*)w.d2, (void*)w.blocksum, (void*)w.scalars,
+                  (void*)w.near, (void*)w.cc, (void*)kp, (void*)err})
+    dev_free(p, s);
   cudaStreamSynchronize(s);
-  for (void* p : {(void*)Xd, (void*)Cd, (void*)d2, (void*)blk, (void*)sc, (void*)kp, (void*)err})
-    if (p) cudaFree(p);
   cudaStreamDestroy(s);
   return rc;
 }

@@ -304,18 +304,18 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   if (kpp_seed < 0) {
     KD_TRY(cudaMemcpy(Cd, C.data(), sizeof(double) * C.size(), cudaMemcpyHostToDevice), E);
   } else {
-    double* d2 = nullptr;
-    unsigned long long *blk = nullptr, *sc = nullptr;
+    KppWork<double> kw;
     int *kp = nullptr, *err = nullptr;
     const kmeansErrorStatus EI = KMEANS_ERROR_INITIALIZE;
-    KD_TRY(B.alloc(&d2, kmeanspp_d2_elems(m)), EI);
-    KD_TRY(B.alloc(&blk, kmeanspp_blocks(m)), EI);
-    KD_TRY(B.alloc(&sc, 3), EI);
+    KD_TRY(B.alloc(&kw.d2, kmeanspp_d2_elems(m)), EI);
+    KD_TRY(B.alloc(&kw.blocksum, kmeanspp_blocks(m)), EI);
+    KD_TRY(B.alloc(&kw.scalars, kKppScalars), EI);
+    KD_TRY(B.alloc(&kw.near, m), EI);
+    KD_TRY(B.alloc(&kw.cc, k), EI);
     KD_TRY(B.alloc(&kp, k), EI);
     KD_TRY(B.alloc(&err, 1), EI);
     KD_TRY(cudaMemset(err, 0, sizeof(int)), EI);
-    KD_TRY(launch_kmeanspp(X, n, m, n, k, (unsigned long long)kpp_seed, Cd, n, kp, d2, blk, sc, err,
-                           s),
+    KD_TRY(launch_kmeanspp(X, n, m, n, k, (unsigned long long)kpp_seed, Cd, n, kp, kw, err, s),
            EI);
     KD_TRY(cudaMemcpy(C.data(), Cd, sizeof(double) * C.size(), cudaMemcpyDeviceToHost), EI);
     int e = 0;

@@ -14,9 +14,10 @@
 //   * Draw r takes u = splitmix64(splitmix64(seed) + r) >> 11 (53 bits) and picks the point whose
 //     interval [prefix, prefix + q) of the running sum of q holds (u * total) >> 53 (128-bit
 //     product). Draw 0, and any draw whose total weight is 0, picks point (u * n) >> 53.
-// Per draw: one pass over X (D^2 update and maximum), one over D^2 (weights and their sums per
-// 1024 points) and one single-block pass (scan of the block sums, the draw, the pick). D^2 is
-// n elements of T; X is read once per draw, which bounds the whole initialisation by HBM.
+// Per draw: one pass over X (D^2 update and maximum) and one over D^2 (weights and their sums per
+// 1024 points; the last block to finish scans the block sums, draws and picks). D^2 is n elements
+// of T; reading X bounds the whole initialisation by HBM, so rows whose D^2 a new center cannot lower
+// are not read where that can be told (kpp_update_bulk_kernel).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -178,15 +179,153 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
       : "memory");
 }
 
+//
+// Rows that need not be read (KppNear, from draw 2 on): near[i] is the draw whose center gave D^2_i,
+// and cc[q] a lower bound of the squared distance from draw q's center to the new one. Where
+// cc[near[i]] >= 4 D^2_i (1 + slack), the triangle inequality puts the row at least as far from the new
+// center as from its own, by more than the rounding of both computed distances, so the minimum is
+// D^2_i again, bit for bit. A warp tests 32 rows at a time and gathers the others, eight rows'
+// loads in flight; each row's sum is formed as above. The share of rows read falls with the draws
+// where clusters lie apart. At 1M x 128 a draw streams every row in 83 us (96 us before the eight-row
+// reduction below: the consumers' shuffles held the ring back) and gathers every row in 103 us, so a
+// draw gathers only when the last gathering draw read at most kKppGatherShare of the rows, and every
+// 16th draw gathers to look again. 256 draws from 256 Gaussians: 28.3 ms reading every row, 19.4 ms so.
+constexpr double kKppGatherShare = 0.7;
+
+struct KppNear {
+  int* near;               // [n] draw of the nearest center; null: every row is read
+  const void* cc;          // [draw] lower bounds (T) of squared distances to the new center
+  unsigned int* active;    // rows read by the last gathering draw, [1] its running count
+  int draw;
+};
+
+template <typename T>
+__device__ __forceinline__ bool kpp_in_range(T v);
+template <>
+__device__ __forceinline__ bool kpp_in_range<float>(float v) { return v >= 1e-30f && v < 1e37f; }
+template <>
+__device__ __forceinline__ bool kpp_in_range<double>(double v) { return v >= 1e-290 && v < 1e300; }
+
+// Relative error of a computed squared distance: at most d / 32 + 7 roundings, the difference's twice.
+template <typename T>
+__device__ __forceinline__ T kpp_rel(int d) {
+  return (T)(d / 32 + 16) * (sizeof(T) == 4 ? (T)5.9604645e-8 : (T)1.1102230246251565e-16);
+}
+
+// Eight rows' lane partials to their butterfly sums: lanes 4r .. 4r+3 end with row r's. The first three
+// steps of the butterfly halve the rows a lane still carries, nine shuffles for the eight rows instead
+// of forty; every addition joins the same two partials (in either order), so the sums are
+// those of a full butterfly, bit for bit.
+template <typename T>
+__device__ __forceinline__ T kpp_reduce8(T (&s)[8], int lane) {
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1) {
+    const int o = 4 * h;
+    const bool up = lane & o;
+#pragma unroll
+    for (int r = 0; r < h; ++r) {
+      const T keep = up ? s[r + h] : s[r], send = up ? s[r] : s[r + h];
+      s[r] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  s[0] = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 2);
+  s[0] = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+  return s[0];
+}
+
+template <typename T>
+__device__ __forceinline__ T kpp_gather_rows(const T* __restrict__ X, long long ldx, long long n, int d,
+                                             const T* cs, T* __restrict__ d2, const KppNear& nr) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const T* cc = static_cast<const T*>(nr.cc);
+  const T slack = T(4) * (T(1) + T(16) * kpp_rel<T>(d));
+  T mx = T(0);
+  unsigned int read = 0;
+  const long long step = (long long)gridDim.x * warps * 32;
+  long long i0 = ((long long)blockIdx.x * warps + warp) * 32;
+  T v = T(0);
+  int a = 0;
+  if (i0 + lane < n) {
+    v = d2[i0 + lane];
+    a = nr.near[i0 + lane];
+  }
+  for (; i0 < n; i0 += step) {
+    const long long i = i0 + lane;
+    const bool in = i < n;
+    const T cur = v;
+    const int cura = a;
+    if (i + step < n) {  // the next group's values in flight
+      v = d2[i + step];
+      a = nr.near[i + step];
+    }
+    const bool skip = !in || cur == T(0) ||
+                      (kpp_in_range(cur) && __ldg(cc + cura) >= slack * cur);
+    unsigned todo = __ballot_sync(0xffffffffu, !skip);
+    read += __popc(todo);
+    if (in && skip) mx = fmax(mx, cur);
+    while (todo) {
+      int row[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        row[r] = todo ? __ffs(todo) - 1 : -1;
+        todo &= todo - 1;
+      }
+      T sv[8];
+      const T* x[8];
+      int own = row[0];  // the row whose sum this lane ends with
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        sv[r] = T(0);
+        x[r] = X + (size_t)(i0 + (row[r] >= 0 ? row[r] : row[0])) * ldx;
+        if ((lane >> 2) == r) own = row[r];
+      }
+      // 512 bytes of each of the eight rows in flight together (slots without a row re-read a row)
+      constexpr int kSteps = 16 / sizeof(T);
+      for (int t0 = lane; t0 < d; t0 += 32 * kSteps) {
+        T xv[kSteps][8];
+#pragma unroll
+        for (int q = 0; q < kSteps; ++q)
+#pragma unroll
+          for (int r = 0; r < 8; ++r) xv[q][r] = t0 + 32 * q < d ? __ldg(x[r] + t0 + 32 * q) : T(0);
+#pragma unroll
+        for (int q = 0; q < kSteps; ++q) {
+          if (t0 + 32 * q >= d) break;
+          const T cv = cs[t0 + 32 * q];
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            const T u = xv[q][r] - cv;
+            sv[r] = kpp_fma(u, u, sv[r]);
+          }
+        }
+      }
+      const T sum = kpp_reduce8(sv, lane);
+      const T old = __shfl_sync(0xffffffffu, cur, own >= 0 ? own : 0);
+      if ((lane & 3) == 0 && own >= 0) {
+        const T nv = fmin(old, sum);
+        if (nv != old && nv == nv) {
+          d2[i0 + own] = nv;
+          nr.near[i0 + own] = nr.draw;
+        }
+        mx = fmax(mx, nv);
+      }
+    }
+  }
+  // (one more, so that a draw that read nothing still counts as measured)
+  if (lane == 0 && blockIdx.x == 0 && warp == 0) ++read;
+  if (lane == 0 && read) atomicAdd(nr.active + 1, read);
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  return mx;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(KPP_BULK_THREADS)
 kpp_update_bulk_kernel(const T* __restrict__ X, long long ldx, long long n, int d,
                        const int* __restrict__ pick, T* __restrict__ d2, int first,
                        unsigned long long* __restrict__ max_key, int rows_per_stage, int stages,
-                       int* __restrict__ err) {
+                       int* __restrict__ err, KppNear nr) {
   extern __shared__ __align__(128) unsigned char kpp_smem[];
   __shared__ __align__(8) uint64_t full_bar[KPP_MAX_STAGES], empty_bar[KPP_MAX_STAGES];
-  __shared__ unsigned long long wmax[KPP_CONSUMERS];
+  __shared__ unsigned long long wmax[KPP_CONSUMERS + 1];
   __shared__ int abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row_elems = ldx;
@@ -208,8 +347,15 @@ kpp_update_bulk_kernel(const T* __restrict__ X, long long ldx, long long n, int 
     fence_mbar_init();
   }
   __syncthreads();
+  // the last gathering draw's count is final: it was written by an earlier launch
+  const bool gather = nr.near && !first &&
+                      (nr.draw % 16 == 0 ||
+                       (double)nr.active[0] <= kKppGatherShare * (double)n);
 
-  if (warp == KPP_CONSUMERS) {  // producer
+  if (gather) {
+    const T m = kpp_gather_rows<T>(X, ldx, n, d, cs, d2, nr);
+    if (lane == 0) wmax[warp] = kpp_key(m);
+  } else if (warp == KPP_CONSUMERS) {  // producer
     if (lane == 0) {
       long long it = 0;
       for (long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x, ++it) {
@@ -252,93 +398,116 @@ kpp_update_bulk_kernel(const T* __restrict__ X, long long ldx, long long n, int 
       const int rows = (int)min((long long)rows_per_stage, n - r0);
       const T* xs = reinterpret_cast<const T*>(ring + (size_t)sidx * xstage_bytes);
       const T* ds = dring + (size_t)sidx * rows_per_stage;
-      for (int g = warp * KPP_ROWS; g < rows; g += KPP_CONSUMERS * KPP_ROWS) {
-        T sv[KPP_ROWS];
+      for (int g = warp * 8; g < rows; g += KPP_CONSUMERS * 8) {
+        T sv[8];
+        const T* xr[8];
 #pragma unroll
-        for (int r = 0; r < KPP_ROWS; ++r) sv[r] = T(0);
-        const T* xr[KPP_ROWS];
-#pragma unroll
-        for (int r = 0; r < KPP_ROWS; ++r) xr[r] = xs + (size_t)min(g + r, rows - 1) * row_elems;
+        for (int r = 0; r < 8; ++r) {
+          sv[r] = T(0);
+          xr[r] = xs + (size_t)min(g + r, rows - 1) * row_elems;
+        }
 #pragma unroll 4
         for (int t = lane; t < d; t += 32) {
           const T cv = cs[t];
 #pragma unroll
-          for (int r = 0; r < KPP_ROWS; ++r) {
+          for (int r = 0; r < 8; ++r) {
             const T u = xr[r][t] - cv;
             sv[r] = kpp_fma(u, u, sv[r]);
           }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-          for (int r = 0; r < KPP_ROWS; ++r) sv[r] = sv[r] + __shfl_xor_sync(0xffffffffu, sv[r], o);
-        }
-#pragma unroll
-        for (int r = 0; r < KPP_ROWS; ++r) {
-          if (g + r < rows) {
-            const T v = first ? sv[r] : fmin(ds[g + r], sv[r]);
-            if (lane == 0) d2[r0 + g + r] = v;
-            mx = fmax(mx, v);
-          }
+        const T sum = kpp_reduce8(sv, lane);
+        const int row = g + (lane >> 2);
+        if ((lane & 3) == 0 && row < rows) {
+          const T old = first ? sum : ds[row];
+          const T v = first ? sum : fmin(old, sum);
+          d2[r0 + row] = v;
+          if (nr.near && (first || v != old)) nr.near[r0 + row] = first ? 0 : nr.draw;
+          mx = fmax(mx, v);
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&empty_bar[sidx]));
     }
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) wmax[warp] = kpp_key(mx);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long m = 0;
-    for (int w = 0; w < KPP_CONSUMERS; ++w) m = max(m, wmax[w]);
+    for (int w = 0; w < KPP_CONSUMERS + (gather ? 1 : 0); ++w) m = max(m, wmax[w]);
     atomicMax(max_key, m);
   }
 }
 
-// Weights q of one 1024-point block and their exact sum.
+// Lower bounds of the squared distances from the newest center (row *pick) to the centers of draws
+// 0 .. draw-1 (rows picks[q]), one warp each; block 0 closes the last gathering draw's count.
 template <typename T>
-__global__ void __launch_bounds__(KPP_THREADS)
-kpp_weight_kernel(const T* __restrict__ d2, long long n, const unsigned long long* __restrict__ max_key,
-                  unsigned long long* __restrict__ blocksum) {
-  __shared__ unsigned long long part[KPP_THREADS / 32];
-  const T scale = kpp_scale<T>(*max_key);
-  unsigned long long s = 0;
-  const long long p0 = (long long)blockIdx.x * KPP_BLOCK;
-  for (int i = threadIdx.x; i < KPP_BLOCK; i += KPP_THREADS) {
-    const long long pt = p0 + i;
-    if (pt < n) s += kpp_weight(d2[pt], scale);
+__global__ void kpp_center_dist_kernel(const T* __restrict__ X, long long ldx, int d,
+                                       const int* __restrict__ picks, int draw, T* __restrict__ cc,
+                                       unsigned int* __restrict__ active) {
+  const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (q == 0 && lane == 0 && active[1]) {
+    active[0] = active[1];
+    active[1] = 0;
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long t = 0;
-    for (int w = 0; w < KPP_THREADS / 32; ++w) t += part[w];
-    blocksum[blockIdx.x] = t;
+  if (q >= draw) return;
+  const T* c = X + (size_t)picks[draw] * ldx;
+  const T* o = X + (size_t)picks[q] * ldx;
+  T s = T(0);
+  for (int t = lane; t < d; t += 32) {
+    const T u = __ldg(c + t) - __ldg(o + t);
+    s = kpp_fma(u, u, s);
   }
+  for (int m = 16; m > 0; m >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, m);
+  if (lane == 0) cc[q] = s * (T(1) - T(4) * kpp_rel<T>(d));
 }
 
-// The draw of round `round`: scan of the block sums, the block holding the target, then the
-// point inside it (1024 threads, one point each). Writes *pick and picks[round].
+// The draw of round `round`. Every block adds the weights q of its 1024-point blocks (exact sums); the
+// last block to finish scans them, draws, finds the 1024-point block holding the target, then the
+// point inside it (1024 threads, one point each), and writes *pick and picks[round]. Without weights
+// (round 0) the sums are zero and the draw uniform.
 template <typename T>
 __global__ void __launch_bounds__(KPP_BLOCK)
-kpp_pick_kernel(long long n, const T* __restrict__ d2, const unsigned long long* __restrict__ blocksum,
-                long long nblocks, const unsigned long long* __restrict__ max_key,
-                unsigned long long* __restrict__ next_max_key, unsigned long long seed, int round,
-                int* __restrict__ pick, int* __restrict__ picks) {
+kpp_draw_kernel(long long n, const T* __restrict__ d2, unsigned long long* blocksum, long long nblocks,
+                bool weights, const unsigned long long* __restrict__ max_key,
+                unsigned long long* __restrict__ next_max_key, unsigned int* ticket,
+                unsigned long long seed, int round, int* __restrict__ pick, int* __restrict__ picks) {
   __shared__ unsigned long long warp_sh[32];
   __shared__ unsigned long long total_sh, off_sh, tot2_sh;
   __shared__ long long block_sh, chosen_sh;
-  const int tid = threadIdx.x;
+  __shared__ bool last_sh;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const T scale = weights ? kpp_scale<T>(*max_key) : T(0);
+  if (weights) {  // one warp per 1024-point block, its loads in flight together
+    for (long long b = blockIdx.x * 32LL + warp; b < nblocks; b += gridDim.x * 32LL) {
+      const long long p0 = b * (long long)KPP_BLOCK + lane;
+      T v[KPP_BLOCK / 32];
+#pragma unroll
+      for (int i = 0; i < KPP_BLOCK / 32; ++i) v[i] = p0 + 32 * i < n ? __ldg(d2 + p0 + 32 * i) : T(0);
+      unsigned long long q = 0;
+#pragma unroll
+      for (int i = 0; i < KPP_BLOCK / 32; ++i) q += kpp_weight(v[i], scale);
+      for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+      if (lane == 0) __stcg(blocksum + b, q);
+    }
+    __syncthreads();
+  }
   if (tid == 0) {
+    __threadfence();  // this block's sums before its ticket
+    last_sh = atomicAdd(ticket, 1u) == gridDim.x - 1;
     block_sh = -1;
     chosen_sh = -1;
   }
+  __syncthreads();
+  if (!last_sh) return;
+  __threadfence();
+  if (tid == 0) *ticket = 0;
   // each thread sums a contiguous run of blocks
   const long long per = (nblocks + KPP_BLOCK - 1) / KPP_BLOCK;
   const long long b0 = (long long)tid * per, b1 = min(nblocks, b0 + per);
   unsigned long long s = 0;
-  for (long long b = b0; b < b1; ++b) s += blocksum[b];
+  for (long long b = b0; b < b1; ++b) s += weights ? __ldcg(blocksum + b) : 0ull;
   unsigned long long off = block_exclusive_scan(s, warp_sh, &total_sh);
   const unsigned long long total = total_sh;
   const uint64_t u = draw53(seed, (uint64_t)round);
@@ -354,7 +523,7 @@ kpp_pick_kernel(long long n, const T* __restrict__ d2, const unsigned long long*
   const unsigned long long target = __umul64hi(u << 11, total);  // (u * total) >> 53 < total
   if (off <= target && target < off + s) {  // exactly one thread's run holds the target
     for (long long b = b0; b < b1; ++b) {
-      const unsigned long long nx = off + blocksum[b];
+      const unsigned long long nx = off + __ldcg(blocksum + b);
       if (nx > target) {
         block_sh = b;
         off_sh = off;
@@ -365,7 +534,6 @@ kpp_pick_kernel(long long n, const T* __restrict__ d2, const unsigned long long*
   }
   __syncthreads();
   const long long b = block_sh;  // >= 0: the runs partition [0, total)
-  const T scale = kpp_scale<T>(*max_key);
   const long long pt = b * (long long)KPP_BLOCK + tid;
   const unsigned long long q = (b >= 0 && pt < n) ? kpp_weight(d2[pt], scale) : 0ull;
   const unsigned long long ex = off_sh + block_exclusive_scan(q, warp_sh, &tot2_sh);
@@ -389,16 +557,19 @@ __global__ void kpp_gather_kernel(const T* __restrict__ X, long long ldx, int d,
   }
 }
 
-// Ring geometry of kpp_update_bulk_kernel for rows of `row_bytes`: rows per stage (a multiple
-// of 4, about 16 KB of rows) and stages (2..8) within a shared-memory budget that leaves room for
-// two CTAs per SM. Returns false when the rows are too wide (the register kernel is used then).
+// Ring geometry of kpp_update_bulk_kernel for rows of `row_bytes`: rows per stage (a multiple of 8, a
+// warp's step, about 32 KB of rows, whole rounds of the 8 consumer warps where more than one; 4 very
+// wide ones) and stages (2..8) within a shared-memory budget that leaves room for two CTAs per SM.
+// Returns false when the rows are too wide (the register kernel is used then).
 constexpr size_t KPP_SMEM_BUDGET = 100 * 1024;
 
 bool kpp_bulk_plan(long long row_bytes, int elem, int d, int* rows_per_stage, int* stages,
                    size_t* smem) {
-  long long rps = (16384 / row_bytes) & ~3LL;
-  if (rps < 4) rps = 4;
+  long long rps = (32768 / row_bytes) & ~7LL;
+  if (rps < 8) rps = 8;
+  if (rps > 64 && rps % 64) rps -= rps % 64;
   const long long center = ((long long)d * elem + 127) / 128 * 128;
+  if (2 * rps * (row_bytes + elem) + center > (long long)KPP_SMEM_BUDGET) rps = 4;
   const long long per_stage = rps * row_bytes + rps * elem;
   long long st = ((long long)KPP_SMEM_BUDGET - center) / per_stage;
   if (st > KPP_MAX_STAGES) st = KPP_MAX_STAGES;
@@ -409,11 +580,14 @@ bool kpp_bulk_plan(long long row_bytes, int elem, int d, int* rows_per_stage, in
   return true;
 }
 
+// Rows are skipped only where reading X costs more than the launch that prepares the test: from the
+// size of the L2 on, a draw's pass takes 24 us or more.
+constexpr long long KPP_NEAR_MIN_BYTES = 128LL << 20;
+
 template <typename T>
 cudaError_t kmeanspp_impl(const T* X, long long ldx, long long n, int d, int k,
-                          unsigned long long seed, T* C, long long ldc, int* picks, T* d2,
-                          unsigned long long* blocksum, unsigned long long* scalars, int* err,
-                          cudaStream_t s) {
+                          unsigned long long seed, T* C, long long ldc, int* picks, const KppWork<T>& w,
+                          int* err, cudaStream_t s) {
   if (n <= 0 || d <= 0 || k <= 0 || k > n || n > 0x7fffffffLL || ldx < d || ldc < d)
     return cudaErrorInvalidValue;
   const long long nb = (n + KPP_BLOCK - 1) / KPP_BLOCK;
@@ -421,40 +595,55 @@ cudaError_t kmeanspp_impl(const T* X, long long ldx, long long n, int d, int k,
   int rps = 0, stages = 0;
   size_t smem = 0;
   const bool bulk = (row_bytes % 16) == 0 && (reinterpret_cast<uintptr_t>(X) % 16) == 0 &&
-                    (reinterpret_cast<uintptr_t>(d2) % 16) == 0 &&
+                    (reinterpret_cast<uintptr_t>(w.d2) % 16) == 0 &&
                     kpp_bulk_plan(row_bytes, (int)sizeof(T), d, &rps, &stages, &smem);
   int grid = 0;
   if (bulk) {
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kpp_update_bulk_kernel<T>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int dev = 0, sms = 0, per_sm = 0;
-    KMGB_CUDA_TRY(cudaGetDevice(&dev));
-    KMGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int per_sm = 0;
     KMGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, kpp_update_bulk_kernel<T>, KPP_BULK_THREADS, smem));
     const long long chunks = (n + rps - 1) / rps;
-    grid = (int)min((long long)sms * max(per_sm, 1), chunks);
+    grid = (int)min((long long)kmgb::num_sms() * max(per_sm, 1), chunks);
   }
-  // scalars: [0], [1] the maxima of alternate draws (the pick kernel of draw r clears draw
-  // r+1's), [2] the newest center's row
-  unsigned long long* mx = scalars;
-  int* pick = reinterpret_cast<int*>(scalars + 2);
+  // scalars: [0], [1] the maxima of alternate draws (draw r clears draw r+1's), [2] the newest
+  // center's row, [3] the draw's block ticket, [4] rows read by the last gathering draw and the
+  // running count (all ones: none yet)
+  unsigned long long* mx = w.scalars;
+  int* pick = reinterpret_cast<int*>(w.scalars + 2);
+  unsigned int* ticket = reinterpret_cast<unsigned int*>(w.scalars + 3);
+  KppNear nr{};
+  if (bulk && w.near && w.cc && n * row_bytes >= KPP_NEAR_MIN_BYTES) {
+    nr.near = w.near;
+    nr.cc = w.cc;
+    nr.active = reinterpret_cast<unsigned int*>(w.scalars + 4);
+    KMGB_CUDA_TRY(cudaMemsetAsync(nr.active, 0xff, sizeof(unsigned int), s));
+    KMGB_CUDA_TRY(cudaMemsetAsync(nr.active + 1, 0, sizeof(unsigned int), s));
+  }
+  KMGB_CUDA_TRY(cudaMemsetAsync(mx, 0, 4 * sizeof(unsigned long long), s));
+  const long long dblocks = (nb + 31) / 32, most = kmgb::num_sms();  // a warp per 1024 points
+  const unsigned dgrid = (unsigned)(dblocks < most ? dblocks : most);
   // draw 0: zero total weight, so uniform
-  KMGB_CUDA_TRY(cudaMemsetAsync(blocksum, 0, sizeof(unsigned long long) * nb, s));
-  KMGB_CUDA_TRY(cudaMemsetAsync(mx, 0, 2 * sizeof(unsigned long long), s));
-  kpp_pick_kernel<T><<<1, KPP_BLOCK, 0, s>>>(n, d2, blocksum, nb, mx, mx + 1, seed, 0, pick, picks);
+  kpp_draw_kernel<T><<<1, KPP_BLOCK, 0, s>>>(n, w.d2, w.blocksum, nb, false, mx, mx + 1, ticket, seed, 0,
+                                             pick, picks);
   count_launches(1);
   for (int r = 1; r < k; ++r) {
     unsigned long long* m = mx + (r & 1);
+    nr.draw = r - 1;
+    if (nr.near && r > 1) {
+      kpp_center_dist_kernel<T><<<(unsigned)((nr.draw + 7) / 8), 256, 0, s>>>(
+          X, ldx, d, picks, nr.draw, static_cast<T*>(w.cc), nr.active);
+      count_launches(1);
+    }
     if (bulk)
-      kpp_update_bulk_kernel<T><<<grid, KPP_BULK_THREADS, smem, s>>>(X, ldx, n, d, pick, d2, r == 1,
-                                                                     m, rps, stages, err);
+      kpp_update_bulk_kernel<T><<<grid, KPP_BULK_THREADS, smem, s>>>(
+          X, ldx, n, d, pick, w.d2, r == 1, m, rps, stages, err, nr);
     else
-      kpp_update_kernel<T><<<(unsigned)nb, KPP_THREADS, 0, s>>>(X, ldx, n, d, pick, d2, r == 1, m);
-    kpp_weight_kernel<T><<<(unsigned)nb, KPP_THREADS, 0, s>>>(d2, n, m, blocksum);
-    kpp_pick_kernel<T><<<1, KPP_BLOCK, 0, s>>>(n, d2, blocksum, nb, m, mx + ((r + 1) & 1), seed, r,
-                                               pick, picks);
-    count_launches(3);
+      kpp_update_kernel<T><<<(unsigned)nb, KPP_THREADS, 0, s>>>(X, ldx, n, d, pick, w.d2, r == 1, m);
+    kpp_draw_kernel<T><<<dgrid, KPP_BLOCK, 0, s>>>(n, w.d2, w.blocksum, nb, true, m,
+                                                   mx + ((r + 1) & 1), ticket, seed, r, pick, picks);
+    count_launches(2);
   }
   kpp_gather_kernel<T><<<kmgb::num_sms() * 4, 256, 0, s>>>(X, ldx, d, picks, k, C, ldc);
   count_launches(1);
@@ -468,17 +657,14 @@ long long kmeanspp_d2_elems(long long n) { return (n + 3) / 4 * 4; }
 
 cudaError_t launch_kmeanspp(const float* X, long long ldx, long long n, int d, int k,
                             unsigned long long seed, float* C, long long ldc, int* picks,
-                            float* d2, unsigned long long* blocksum, unsigned long long* scalars,
-                            int* err, cudaStream_t s) {
-  return kmeanspp_impl<float>(X, ldx, n, d, k, seed, C, ldc, picks, d2, blocksum, scalars, err, s);
+                            const KppWork<float>& w, int* err, cudaStream_t s) {
+  return kmeanspp_impl<float>(X, ldx, n, d, k, seed, C, ldc, picks, w, err, s);
 }
 
 cudaError_t launch_kmeanspp(const double* X, long long ldx, long long n, int d, int k,
                             unsigned long long seed, double* C, long long ldc, int* picks,
-                            double* d2, unsigned long long* blocksum, unsigned long long* scalars,
-                            int* err, cudaStream_t s) {
-  return kmeanspp_impl<double>(X, ldx, n, d, k, seed, C, ldc, picks, d2, blocksum, scalars, err,
-                               s);
+                            const KppWork<double>& w, int* err, cudaStream_t s) {
+  return kmeanspp_impl<double>(X, ldx, n, d, k, seed, C, ldc, picks, w, err, s);
 }
 
 }  // namespace kmgb

@@ -140,3 +140,23 @@ def test_rejections(km, torch_cuda):
         km.kmeanspp(X, 2001, 0)
     with pytest.raises(km.KmeansError):  # host-streamed data is not resident
         km.lloyd(X, 4, max_iters=2, stream_tile_rows=500, init_algorithm=km.INIT_KMEANSPP)
+
+
+@pytest.mark.parametrize("n,d,k,comps,dtype", [(300_000, 128, 64, 12, np.float32),
+                                               (350_001, 100, 40, 400, np.float32),
+                                               (150_000, 128, 48, 9, np.float64),
+                                               (1_100_000, 32, 50, 20, np.float32)])
+def test_rows_skipped_by_the_triangle_inequality(km, orc, torch_cuda, n, d, k, comps, dtype):
+    """Data sets past the L2's size: draws that gather only the rows a new center can reach pick the
+    oracle's rows (clusters apart: most rows skipped; overlapping ones, duplicates and zeros: few)."""
+    span = 20.0 if comps < 100 else 1.0
+    X, _, _ = mixture_numpy(n, d, comps, seed=n, mean_lo=-span, mean_hi=span)
+    X = X.astype(dtype)
+    X[1000:1100] = X[1000]
+    X[5000:5050] = 0
+    if dtype == np.float64:
+        X *= 1 + 1e-9
+    want, wcen = orc.kmeanspp(X, k, 5)
+    cen, picks = km.kmeanspp(X, k, 5)
+    assert np.array_equal(picks, want)
+    assert np.array_equal(cen, wcen)
