@@ -346,8 +346,8 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
       f.set(m.alloc(&cand_cnt, cand_cap), E, "re-rank") ||
       f.set(m.alloc(&rr_over, cand_cap), E, "re-rank") ||
       f.set(m.alloc(&over_count, 1), E, "re-rank") ||
-      f.set(m.alloc(&audit_ws, 4 + 2 * (size_t)kAuditMaxRows), E, "audit") ||
-      f.set(cudaMemsetAsync(audit_ws, 0, sizeof(unsigned long long) * (4 + 2 * kAuditMaxRows), s),
+      f.set(m.alloc(&audit_ws, kAuditWords), E, "audit") ||
+      f.set(cudaMemsetAsync(audit_ws, 0, sizeof(unsigned long long) * kAuditWords, s),
             E, "audit") ||
       f.set(cudaMemsetAsync(rr_stats, 0, 2 * sizeof(unsigned long long), s), E, "re-rank") ||
       f.set(cudaMemsetAsync(err, 0, sizeof(int), s), E, "error word") ||
@@ -478,7 +478,8 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
       f.set(m.alloc(&w.part, (size_t)w.max_pieces * d), EU, "update") ||
       f.set(m.alloc(&w.partq, w.max_pieces), EU, "update") ||
       f.set(m.alloc(&w.sse_k, (size_t)K * ((d + 31) / 32)), EU, "update") ||
-      f.set(m.alloc(&w.counts, K), EU, "update"))
+      f.set(m.alloc(&w.counts, K), EU, "update") || f.set(m.alloc(&w.tickets, 1), EU, "update") ||
+      f.set(cudaMemsetAsync(w.tickets, 0, sizeof(int), s), EU, "update"))
     return f.code;
 
   AssignArgs a{};

@@ -197,7 +197,8 @@ struct kmgb_handle {
   int* labels = nullptr;
   int* rr_list = nullptr;
   // re-rank lists: [0] flagged by the assignment (rr_list), [1] BF16 tiers: candidates overflowed
-  // (rr_over), [2] left for the exact FP64 stage after the FP32 rescan (rr_list2, rr_hi2)
+  // (rr_over); FP32 tier on large data: [2] left by the FP32 rescan (rr_list2, rr_hi2), [3] left by
+  // their candidates (rr_over, rr_hi3). The counts follow cmax
   int* rr_count = nullptr;
   int* rr_over = nullptr;
   int* rr_list2 = nullptr;
@@ -362,7 +363,7 @@ void alloc_prune(kmgb_handle* h, bool split) {
     a.take(&p.list, p.cap);
     a.take(&p.lab_old, p.n);
     a.take(&p.dirty, p.k);
-    a.take(&p.flags, 4);
+    a.take(&p.flags, 8);
     a.take(&p.top, 2);
     a.take_bytes(&p.Xc, (size_t)p.cap * (tc ? h->ldb * 2 : h->ldx * 4));
     if (split) a.take_bytes(&p.Xlc, (size_t)p.cap * h->ldb * 2);
@@ -518,14 +519,12 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
       a.take(&h->cscale, 1);
     }
     a.take(&h->cn, k);
-    a.take(&h->cmax, 1);
+    a.take(&h->cmax, 8);  // and the counts below: cleared together
     if (tcore) a.take(&h->cinit, (size_t)round_up(k, kCenterPad));
     if (bf16) a.take_bytes(&h->cbias, (size_t)round_up(k, kCenterPad) * kBiasCols * 2);
     a.take(&h->labels, nl);
     a.take(&h->rr_list, na);
-    a.take(&h->rr_count, 4);
-    a.take(&h->rr_list2, na);
-    a.take(&h->rr_hi2, na);
+    h->rr_count = reinterpret_cast<int*>(h->cmax + 1);
     if (tcore) {
       const long long cc = h->cand_cap;
       a.take(&h->rr_over, na);
@@ -539,13 +538,15 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
       a.take(&h->cand_cnt, cc);
     }
     if (fp32_band) {
+      a.take(&h->rr_list2, na);
+      a.take(&h->rr_hi2, na);
       a.take(&h->rr_over, na);
       a.take(&h->rr_hi3, na);
       a.take(&h->cand, (size_t)h->cand_cap * kMaxCand);
       a.take(&h->cand_cnt, h->cand_cap);
     }
     a.take(&h->rr_stats, 2);
-    if (h->audit_rows > 0) a.take(&h->audit, 4 + 2 * (size_t)kAuditMaxRows);
+    if (h->audit_rows > 0) a.take(&h->audit, kAuditWords);
     a.take(&h->err, 1);
     a.take(&h->stop, 1);
     a.take(&h->loopf, 2);
@@ -560,6 +561,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     a.take(&w.partq, w.max_pieces);
     a.take(&w.sse_k, (size_t)k * ((d + 31) / 32));  // per (center, 32 dims)
     a.take(&w.counts, k);
+    a.take(&w.tickets, 1);
   };
   Arena sizing;
   carve(sizing);
@@ -580,9 +582,10 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   KM_TRY(cudaMemset(h->labels, 0, sizeof(int) * nl), (delete h, code));
   KM_TRY(cudaMemset(h->rr_stats, 0, sizeof(unsigned long long) * 2), (delete h, code));
   if (h->audit)
-    KM_TRY(cudaMemset(h->audit, 0, sizeof(unsigned long long) * (4 + 2 * kAuditMaxRows)),
+    KM_TRY(cudaMemset(h->audit, 0, sizeof(unsigned long long) * kAuditWords),
            (delete h, code));
   KM_TRY(cudaMemset(h->err, 0, sizeof(int)), (delete h, code));
+  KM_TRY(cudaMemset(w.tickets, 0, sizeof(int)), (delete h, code));
   w.err = h->err;
   w.stop = h->stop;
   w.sse_prev = h->loopf;
@@ -834,13 +837,16 @@ int rerank_flagged(kmgb_handle* h, const AssignArgs& a, const float* Xa, const v
     r.count = h->rr_count + 1;
   }
   // FP32 stage over the points still open, exact FP64 stage over what FP32 cannot separate
-  KM_TRY(launch_rerank_tiled(r, h->rr_list2, h->rr_count + 2, h->rr_hi2, s),
-         KMEANS_ERROR_CLOSEST_CENTERS);
-  r.list = h->rr_list2;
-  r.count = h->rr_count + 2;
-  r.stats = nullptr;
-  const float* hi = h->rr_hi2;
-  if (!tc && h->cand_cap > 0) {  // FP32 tier: the bands' candidates first, what is left exactly
+  r.counts = h->rr_count;
+  r.full_idx = tc ? 1 : 0;
+  if (tc || h->cand_cap == 0) {
+    KM_TRY(launch_rerank_settle(r, s), KMEANS_ERROR_CLOSEST_CENTERS);
+  } else {  // FP32 tier: what FP32 leaves open takes the bands' candidates first, the rest exactly
+    KM_TRY(launch_rerank_tiled(r, h->rr_list2, h->rr_count + 2, h->rr_hi2, s),
+           KMEANS_ERROR_CLOSEST_CENTERS);
+    r.list = h->rr_list2;
+    r.count = h->rr_count + 2;
+    const float* hi = h->rr_hi2;
     KM_TRY(launch_rerank_band(r, hi, h->cand, h->cand_cnt, h->cand_cap, h->rr_over, h->rr_count + 3,
                               h->rr_hi3, s),
            KMEANS_ERROR_CLOSEST_CENTERS);
@@ -851,11 +857,8 @@ int rerank_flagged(kmgb_handle* h, const AssignArgs& a, const float* Xa, const v
            KMEANS_ERROR_CLOSEST_CENTERS);
     r.list = h->rr_over;
     r.count = h->rr_count + 3;
-    hi = h->rr_hi3;
+    KM_TRY(launch_rerank_exact(r, h->rr_hi3, s), KMEANS_ERROR_CLOSEST_CENTERS);
   }
-  KM_TRY(launch_rerank_exact(r, hi, s), KMEANS_ERROR_CLOSEST_CENTERS);
-  KM_TRY(launch_count_stats(h->rr_count, tc ? 1 : 0, h->rr_stats, h->stop, s),
-         KMEANS_ERROR_CLOSEST_CENTERS);
   return 0;
 }
 
@@ -1031,8 +1034,7 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   const long long na = h->n_act;
   KM_TRY(h->pmark(0), KMEANS_ERROR_RESET);
   // reset (kmeans.cpp:1142-1170): norms of the current centers, cleared counters
-  KM_TRY(cudaMemsetAsync(h->cmax, 0, sizeof(float), s), KMEANS_ERROR_RESET);
-  KM_TRY(cudaMemsetAsync(h->rr_count, 0, 4 * sizeof(int), s), KMEANS_ERROR_RESET);
+  KM_TRY(cudaMemsetAsync(h->cmax, 0, sizeof(float) + 4 * sizeof(int), s), KMEANS_ERROR_RESET);
   const bool prune = h->pr.n > 0 && !assign_only;
   KM_TRY(launch_prep_centers(h->C, h->ldx, h->k, h->d, h->Cop, h->Cb, h->ldb, h->cn, h->cmax, s,
                              h->stop, h->cinit, h->Cl, h->cbias, prune ? h->pr.shift : nullptr,
@@ -1071,7 +1073,9 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
     if (prune) {  // this iteration scans every row and leaves valid bounds
       a.ub = h->pr.ub;
       a.lb = h->pr.lb;
-      KM_TRY(cudaMemsetAsync(h->pr.flags, 1, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      KM_TRY(cudaMemsetAsync(h->pr.flags, 1, 8 * sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      KM_TRY(cudaMemsetAsync(h->pr.flags + 2, 0, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      KM_TRY(cudaMemsetAsync(h->pr.flags + 5, 0, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
       KM_TRY(cudaMemsetAsync(h->pr.flags + 1, 0x7f, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
       KM_TRY(cudaMemsetAsync(h->pr.dirty, 1, sizeof(int) * h->k, s), KMEANS_ERROR_COPY_TILE);
     }
@@ -1146,6 +1150,7 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   if (prune) {
     KM_TRY(launch_prune_dirty(h->pr, h->labels, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
     uw.dirty = h->pr.dirty;
+    uw.any_dirty = h->pr.flags + 4;
   }
   KM_TRY(launch_update(Xa, qna, h->labels, h->C, h->ldx, h->opt.empty_policy, uw,
                        h->uw.sse_indexed ? h->sse_dev : h->sse_dev + slot, s),
@@ -1261,14 +1266,9 @@ int step_stream(kmgb_handle* h, int slot) {
         r.list = h->rr_over;
         r.count = h->rr_count + 1;
       }
-      KM_TRY(launch_rerank_tiled(r, h->rr_list2, h->rr_count + 2, h->rr_hi2, s),
-             KMEANS_ERROR_CLOSEST_CENTERS);
-      r.list = h->rr_list2;
-      r.count = h->rr_count + 2;
-      r.stats = nullptr;
-      KM_TRY(launch_rerank_exact(r, h->rr_hi2, s), KMEANS_ERROR_CLOSEST_CENTERS);
-      KM_TRY(launch_count_stats(h->rr_count, tc ? 1 : 0, h->rr_stats, h->stop, s),
-             KMEANS_ERROR_CLOSEST_CENTERS);
+      r.counts = h->rr_count;
+      r.full_idx = tc ? 1 : 0;
+      KM_TRY(launch_rerank_settle(r, s), KMEANS_ERROR_CLOSEST_CENTERS);
     }
     // this tile's canonical sums into the run's FP64 totals (tiles in order)
     UpdateWork w = h->uw;
@@ -1364,7 +1364,7 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
                          h->stream),
          KMEANS_ERROR_COMPUTE);
   if (h->pr.n > 0)  // no bounds yet: the first iteration scans every row
-    KM_TRY(cudaMemsetAsync(h->pr.flags, 0, 4 * sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
+    KM_TRY(cudaMemsetAsync(h->pr.flags, 0, 8 * sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
   KM_TRY(cudaEventRecord(h->ev0, h->stream), KMEANS_ERROR_COMPUTE);
   int first = 0;
   if (upload && iters > 0) {
@@ -1804,7 +1804,7 @@ int kmgb_debug_audit(const float* X, long long n, int d, long long ldx, const fl
     set_err("kmgb_debug_audit: invalid arguments");
     return KMEANS_ERROR_COMPUTE;
   }
-  const size_t words = 4 + 2 * (size_t)kAuditMaxRows;
+  const size_t words = kAuditWords;
   unsigned long long* ws = nullptr;
   KM_TRY(dalloc(&ws, words), KMEANS_ERROR_COMPUTE);
   cudaError_t r = cudaMemset(ws, 0, sizeof(unsigned long long) * words);

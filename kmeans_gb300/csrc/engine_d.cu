@@ -222,11 +222,11 @@ void alloc_prune_d(DevBufs& B, PruneState* out, int** crr, long long m, int k, l
   take(&p.list, p.cap);
   take(&p.lab_old, m);
   take(&p.dirty, k);
-  take(&p.flags, 4);
+  take(&p.flags, 8);
   take(&p.top, 2);
   take(&xc, (size_t)p.cap * ldb);
   take(&xlc, (size_t)p.cap * ldb);
-  ok = ok && cudaMemsetAsync(p.flags, 0, 4 * sizeof(int), 0) == cudaSuccess;
+  ok = ok && cudaMemsetAsync(p.flags, 0, 8 * sizeof(int), 0) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     return;
@@ -340,6 +340,8 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   KD_TRY(B.alloc(&w.part, (size_t)w.max_pieces * n), E);
   KD_TRY(B.alloc(&part, w.max_pieces), E);
   KD_TRY(B.alloc(&sse_k, k), E);
+  KD_TRY(B.alloc(&w.tickets, 1), E);
+  KD_TRY(cudaMemsetAsync(w.tickets, 0, sizeof(int), s), E);
 
   // Tensor path (full batches, D within the split tier's limit): X and the centers are rounded
   // to FP32, the split BF16 tier assigns every point under its bound widened by that rounding

@@ -137,6 +137,10 @@ struct RerankArgs {
   int mode;
   long long max_list;
   const int* stop;
+  // launch_rerank_tiled, launch_rerank_settle (nullable): stats[0] += counts[0] (points flagged by the
+  // assignment), stats[1] += counts[full_idx] (points that needed a full rescan of the centers)
+  const int* counts;
+  int full_idx;
 };
 // Any dimension; one warp per point, both modes.
 cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t s);
@@ -154,7 +158,10 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
 cudaError_t launch_rerank_grouped(const RerankArgs& a, const GroupArgs& g, cudaStream_t s,
                                   int* cand = nullptr, int* cand_cnt = nullptr,
                                   long long cand_cap = 0);
-// FP64 stage over list2 (one CTA per point), candidates bounded by hi2.
+// Both stages in one launch: every block takes the points its FP32 pass leaves open straight through
+// the exact pass.
+cudaError_t launch_rerank_settle(const RerankArgs& a, cudaStream_t s);
+// FP64 stage over list2, candidates bounded by hi2.
 cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStream_t s);
 // The same list's FP32 bands as candidates for launch_resolve_candidates: slot i < cand_cap of the
 // list records in cand[i * kMaxCand ..], later slots go to over / over_hi (launch_rerank_exact's).
@@ -180,20 +187,17 @@ cudaError_t launch_resolve_candidates(const int* list, const int* count, long lo
                                       const int* stop, cudaStream_t s,
                                       const int* row_map = nullptr, const float* hi_in = nullptr,
                                       float* over_hi = nullptr);
-// stats[0] += counts[0] (points flagged by the assignment), stats[1] += counts[full_idx]
-// (points that needed a full rescan of the centers).
 // Audit of certified labels (rerank.cu): `rows` sampled rows (at most kAuditMaxRows) against
-// the FP64 arg-min over all k centers; ws holds 4 + 2 * kAuditMaxRows words, zero before the
-// first audit ([0] rows audited, [1] violations, [3] 1 + the last violating row).
+// the FP64 arg-min over all k centers; ws holds kAuditWords words, zero before the first audit
+// ([0] rows audited, [1] violations, [3] 1 + the last violating row).
 constexpr int kAuditMaxRows = 256;
+constexpr int kAuditWords = 5 + 2 * kAuditMaxRows;  // of ws
 // With grp (batched problems): each sampled row against its own problem's centers; padding rows
 // and rows of stopped problems are skipped (not counted in ws[0]).
 cudaError_t launch_audit_labels(const float* X, long long ldx, long long n, int d, const float* C,
                                 long long ldc, int k, const int* labels, unsigned long long* ws,
                                 int rows, const int* stop, cudaStream_t s,
                                 const GroupArgs* grp = nullptr);
-cudaError_t launch_count_stats(const int* counts, int full_idx, unsigned long long* stats,
-                               const int* stop, cudaStream_t s);
 
 // Settles flagged points of the expansion form (value nb_j - 2 x.c_j, FP64 arg-min, lowest index on
 // ties) from their recorded candidates: float-float dot products, exact FP64 where they cannot
@@ -221,8 +225,8 @@ cudaError_t launch_resolve_fp64(const ResolveD& a, cudaStream_t s);
 // unusable centers and padding; cbias (nullable, round_up(k,128) rows of kBiasCols BF16) the same
 // start values split exactly into three BF16 numbers (columns 0..2, the rest zero), the B
 // operand of the pair kernel's start-value MMA. shift (nullable): upper bound of the distance
-// from the row Cop holds (the previous centers) to the new one, +inf from an unusable row, -1 for
-// a center that is unusable now; cxn (nullable): upper bound of ||c_j|| (0 when unusable);
+// from the row Cop holds (the previous centers) to the new one, +inf from or to an unusable row, -1
+// for a center that stays unusable; cxn (nullable): upper bound of ||c_j|| (0 when unusable);
 // shift_pert: relative rounding of C's rows (FP64 centers), added to the moves.
 constexpr int kBiasCols = 16;
 cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, float* Cop,
@@ -239,7 +243,7 @@ struct PruneState {
   int cap = 0;             // rows of the compact copy; more rows to scan: the full scan
   float* ub = nullptr;     // [n] upper bound of the distance to the label's center
   float* lb = nullptr;     // [n] lower bound of the distance to every other usable center
-  float* shift = nullptr;  // [k] upper bound of the center's last move, -1: unusable center
+  float* shift = nullptr;  // [k] upper bound of the center's last move, -1: it stays unusable
   float* cxn = nullptr;    // [k] upper bound of ||c_j||
   float* cub = nullptr;    // [k] scratch of the centers' own scan
   float* clb = nullptr;    // [k] lower bound of the distance to the nearest other usable center
@@ -247,8 +251,9 @@ struct PruneState {
   int* list = nullptr;     // [cap] rows to scan
   int* lab_old = nullptr;  // [n] labels of the last update
   int* dirty = nullptr;    // [k] nonzero: the center's members may differ from the last update's
-  int* flags = nullptr;    // [0] 0: no bounds yet, else >= k, [1] rows to scan, [2] scratch count, [3] index of
-                           // the center that moved most
+  int* flags = nullptr;    // [0] 0: no bounds yet, else >= k, [1] rows to scan, [2] scratch count,
+                           // [3] index of the center that moved most, [4] nonzero: some center is
+                           // dirty, [5] nonzero: no center moved
   float* top = nullptr;    // [2] the two largest moves
   void* Xc = nullptr;      // [cap][ldb] compact rows (BF16), and their residual plane
   void* Xlc = nullptr;
@@ -313,9 +318,12 @@ struct UpdateWork {
   int* sorted;          // [n]
   double* part;         // [max_pieces * d]
   double* partq;        // [max_pieces]
-  double* sse_k;        // [k][ceil(d/32)] SSE terms per (center, group of 32 dimensions)
+  double* sse_k;        // [k][ceil(d/32)] SSE terms per (center, group of 32 dimensions); launch_update:
+                        // [k] per center
   long long* counts;    // [k]
   int* err;
+  int* tickets;         // [1] zero between launches (last_block)
+  const int* any_dirty; // nullable: zero when no center's members changed
   const int* dirty;     // nullable: [k] zero where the center has the members of the previous
                         // update: its sums, center and SSE terms stay as they are
   // stop rule (kmeans.cpp:1194-1237), evaluated on the device by the SSE reduction

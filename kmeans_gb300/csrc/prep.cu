@@ -79,7 +79,7 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
       // FP64 centers: each end of the move is a rounding away from its center
       const float pt = shift_pert > 0.0f
                            ? __fmul_ru(shift_pert, __fadd_ru(__double2float_ru(sqrt(s)), mv)) : 0.0f;
-      shift[warp] = bad ? -1.0f : (was_bad ? INFINITY : __fadd_ru(mv, pt));
+      shift[warp] = bad && was_bad ? -1.0f : (bad || was_bad ? INFINITY : __fadd_ru(mv, pt));
     }
     __syncwarp();
   }

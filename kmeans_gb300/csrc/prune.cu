@@ -73,6 +73,10 @@ prune_top_kernel(PruneState ps, const int* stop) {
       ps.top[1] = b2;
       ps.flags[3] = i1;
       ps.flags[1] = first ? 0x7fffffff : 0;
+      // the last update found every center's members unchanged, so no center has moved: every label
+      // and bound stands and nothing is scanned
+      ps.flags[5] = !first && ps.flags[4] == 0;
+      ps.flags[4] = first;
       ps.flags[0] = ps.k;
       ps.flags[2] = 0;  // the next iteration's scan of the centers counts from zero
     }
@@ -88,6 +92,7 @@ prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* st
   __shared__ int wsum[PF_THREADS / 32];
   __shared__ int base_sh;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (ps.flags[5]) return;
   const float top1 = ps.top[0], top2 = ps.top[1];
   const int topi = ps.flags[3];
   for (long long b0 = (long long)blockIdx.x * PF_ROWS; b0 < ps.n; b0 += (long long)gridDim.x * PF_ROWS) {
@@ -216,15 +221,19 @@ prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* sto
   const int cnt = ps.flags[1];
   const bool all = cnt > ps.cap;
   const long long total = all ? ps.n : cnt;
+  bool changed = false;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long pt = all ? i : (long long)__ldg(ps.list + i);
     const int a = ps.lab_old[pt], b = labels[pt];
     if (a == b) continue;
     ps.lab_old[pt] = b;
-    if (a >= 0 && a < ps.k) ps.dirty[a] = 1;
-    if (b >= 0 && b < ps.k) ps.dirty[b] = 1;
+    changed = true;
+    // (looked at first: in early iterations thousands of rows mark the same few centers)
+    if (a >= 0 && a < ps.k && !*(volatile int*)(ps.dirty + a)) ps.dirty[a] = 1;
+    if (b >= 0 && b < ps.k && !*(volatile int*)(ps.dirty + b)) ps.dirty[b] = 1;
   }
+  if (__syncthreads_or(changed) && threadIdx.x == 0) ps.flags[4] = 1;
 }
 
 }  // namespace

@@ -391,20 +391,18 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   const long long wave = 256LL * (num_sms() / 2);
   const long long chunk = std::min(n, wave * std::max(1LL, (96LL << 20) / (wave * ldb * 4)));
   const long long cap = std::min(n, std::max(1024LL, n / 8));
-  float *Ap, *Bt, *nbx, *xn, *cmax, *cinit, *thr, *thrC, *hi2;
-  int *list, *list2, *over, *sc, *cand, *cand_cnt;
+  float *Ap, *Bt, *nbx, *xn, *cmax, *cinit, *thr, *thrC;
+  int *list, *over, *sc, *cand, *cand_cnt;
   char *Xb, *Xl, *XbC, *XlC, *Cb, *Cl, *cbias;
   const long long kpad = (k + kCenterPad - 1) / kCenterPad * kCenterPad;
   auto carve = [&](Carver& c) {
-    c.take(&sc, 8);  // [0] cmax, [1] flagged, [2] left by the candidates, [3] left by FP32, [4] error
+    c.take(&sc, 8);  // [0] cmax, [1] flagged, [2] left by the candidates, [4] error
     c.take(&Ap, copy ? n * ld : 0);
     c.take(&Bt, k * ld);
     c.take(&nbx, k);
     c.take(&xn, n);
     c.take(&list, n);
     c.take(&over, tc ? n : 0);
-    c.take(&list2, kF32 ? n : 0);
-    c.take(&hi2, kF32 ? n : 0);
     if (!tc) return;
     c.take(&cinit, kpad);
     c.take(&cbias, kpad * kBiasCols * 2);
@@ -515,10 +513,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
       r.max_list = n;
     }
     if (!e && tiled) {
-      e = launch_rerank_tiled(r, list2, sc + 3, hi2, kDefault);
-      r.list = list2;
-      r.count = sc + 3;
-      if (!e) e = launch_rerank_exact(r, hi2, kDefault);
+      e = launch_rerank_settle(r, kDefault);
     } else if (!e) {
       e = launch_rerank(r, kDefault);
     }
@@ -575,6 +570,8 @@ kmeansCudaErrorStatus cluster_centers(int m0, int m, int n, int k, bool lastTile
     if (!e) e = tmp_alloc(&w.label_off, k + 1);
     if (!e) e = tmp_alloc(&w.piece_cnt, k + 1);
     if (!e) e = tmp_alloc(&w.sorted, m);
+    if (!e) e = tmp_alloc(&w.tickets, 1);
+    if (!e) e = cudaMemsetAsync(w.tickets, 0, sizeof(int), kDefault);
     if (!e) e = tmp_alloc(&w.part, (size_t)w.max_pieces * n);
     if (!e) e = launch_tile_accumulate<T>(data, n, indices + m0, w, acc, counts_large, kDefault);
   }
@@ -584,6 +581,7 @@ kmeansCudaErrorStatus cluster_centers(int m0, int m, int n, int k, bool lastTile
   tmp_free(w.label_off);
   tmp_free(w.piece_cnt);
   tmp_free(w.sorted);
+  tmp_free(w.tickets);
   tmp_free(w.part);
   return e ? ERROR_CLUSTERCENTERS : NO_ERROR;
 }

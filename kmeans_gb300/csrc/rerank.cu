@@ -175,7 +175,134 @@ __device__ __forceinline__ float expansion_bound(const RerankArgs& a, int pt) {
           u * 1.01f * cm * cm) * 1.01f + 1e-30f;
 }
 
-template <int MODE>
+// The exact pass over the points g0 .. of a.list whose rows lie in xs (see rerank_exact_kernel): every
+// (point, center) pair whose lower end is within the point's best upper end hs (NaN: a settled point,
+// left alone).
+template <int MODE, bool RECORD>
+__device__ __forceinline__ void exact_pass(const RerankArgs& a, const float4* xs, float4* cs,
+                                           float* cflag, int rs, int dq, long long g0, long long cnt,
+                                           const float* hs, const float* es, int* __restrict__ cand,
+                                           int* __restrict__ cand_cnt) {
+  __shared__ double mb[8][TP];
+  __shared__ int mi[8][TP];
+  __shared__ int ncand[TP];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int pq = tid & 7;                 // points pq, pq + 8, pq + 16, pq + 24
+  const int cq = tid >> 3;                // centers cq*2, cq*2+1 of the block
+  const float u = 5.9604645e-8f;
+  const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;
+  if (RECORD && tid < TP) ncand[tid] = 0;
+  double be[4];
+  int bi[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    be[i] = INFINITY;
+    bi[i] = -1;
+  }
+  for (int j0 = 0; j0 < a.k; j0 += TC) {
+    __syncthreads();
+    for (int e = tid; e < TC * dq; e += blockDim.x) {
+      const int r = e / dq, q = e % dq;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j0 + r < a.k) v = *reinterpret_cast<const float4*>(a.C + (size_t)(j0 + r) * a.ldc + q * 4);
+      cs[r * rs + q] = v;
+    }
+    if (tid < TC) {
+      const int j = j0 + tid;
+      cflag[tid] = tile_offset<MODE>(a, j);
+    }
+    __syncthreads();
+    float acc[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0f;
+    for (int q = 0; q < dq; ++q) {
+      const float4 c0 = cs[(cq * 2) * rs + q];
+      const float4 c1 = cs[(cq * 2 + 1) * rs + q];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 x = xs[(pq + 8 * i) * rs + q];
+        tile_acc<MODE>(x, c0, acc[i][0]);
+        tile_acc<MODE>(x, c1, acc[i][1]);
+      }
+    }
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+      const int cl = cq * 2 + jj;
+      const int j = j0 + cl;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int pl = pq + 8 * i;
+        // unusable (empty-cluster) or padding center
+        if (MODE == 0 ? cflag[cl] != 0.0f : j >= a.k) continue;
+        const float lo = MODE == 0 ? acc[i][jj] * (1.0f - gam) - 1e-30f
+                                   : fmaf(-2.0f, acc[i][jj], cflag[cl]) - es[pl];
+        if (!(lo <= hs[pl])) continue;
+        if (RECORD) {
+          const int at = atomicAdd(&ncand[pl], 1);
+          if (at < kMaxCand) cand[(g0 + pl) * kMaxCand + at] = j;
+          continue;
+        }
+        // FP64 in the oracle's order: dimensions 0 .. d-1 (padding dimensions are zero)
+        double ex = 0.0;
+        for (int q = 0; q < dq; ++q) {
+          const float4 x = xs[pl * rs + q];
+          const float4 c = cs[cl * rs + q];
+          if (MODE == 0) {
+            double dd;
+            dd = (double)x.x - (double)c.x; ex = fma(dd, dd, ex);
+            dd = (double)x.y - (double)c.y; ex = fma(dd, dd, ex);
+            dd = (double)x.z - (double)c.z; ex = fma(dd, dd, ex);
+            dd = (double)x.w - (double)c.w; ex = fma(dd, dd, ex);
+          } else {
+            ex = fma((double)x.x, (double)c.x, ex);
+            ex = fma((double)x.y, (double)c.y, ex);
+            ex = fma((double)x.z, (double)c.z, ex);
+            ex = fma((double)x.w, (double)c.w, ex);
+          }
+        }
+        if (MODE == 1) ex = fma(-2.0, ex, (double)cflag[cl]);
+        if (ex < INFINITY && (ex < be[i] || (ex == be[i] && (unsigned)j < (unsigned)bi[i]))) {
+          be[i] = ex;
+          bi[i] = j;
+        }
+      }
+    }
+  }
+  if (RECORD) {
+    __syncthreads();
+    if (tid < TP && g0 + tid < cnt) cand_cnt[g0 + tid] = ncand[tid] <= kMaxCand ? ncand[tid] : -1;
+    return;
+  }
+  // merge the 32 threads of each point: lanes pq, pq+8, pq+16, pq+24 of every warp
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int off = 8; off < 32; off <<= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, be[i], off);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi[i], off);
+      const bool take = (ob < be[i]) || (ob == be[i] && (unsigned)oi < (unsigned)bi[i]);
+      be[i] = take ? ob : be[i];
+      bi[i] = take ? oi : bi[i];
+    }
+    if (lane < 8) {
+      mb[w][pq + 8 * i] = be[i];
+      mi[w][pq + 8 * i] = bi[i];
+    }
+  }
+  __syncthreads();
+  if (tid < TP && g0 + tid < cnt && hs[tid] == hs[tid]) {
+    double fb = mb[0][tid];
+    int fi = mi[0][tid];
+    for (int ww = 1; ww < 8; ++ww) {
+      const bool take = (mb[ww][tid] < fb) || (mb[ww][tid] == fb && (unsigned)mi[ww][tid] < (unsigned)fi);
+      fb = take ? mb[ww][tid] : fb;
+      fi = take ? mi[ww][tid] : fi;
+    }
+    a.labels[a.list[g0 + tid]] = fi < 0 ? 0 : fi;
+  }
+}
+
+template <int MODE, bool SETTLE>
 __global__ void __launch_bounds__(256)
 rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ count2,
                     float* __restrict__ hi2) {
@@ -189,10 +316,15 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
   float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] value offset (tile_offset)
   __shared__ float mb1[8][TP], mb2[8][TP];
   __shared__ int mi1[8][TP];
+  __shared__ float hs[TP], es[TP];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int pq = tid & 7;                 // points pq, pq + 8, pq + 16, pq + 24
   const int cq = tid >> 3;                // centers cq*2, cq*2+1 of the block
   const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  if (a.counts && a.stats && blockIdx.x == 0 && tid == 0) {
+    a.stats[0] += (unsigned long long)a.counts[0];
+    a.stats[1] += (unsigned long long)a.counts[a.full_idx];
+  }
   const float u = 5.9604645e-8f;
   const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;
 
@@ -311,14 +443,22 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
         hi1 = f1 + e;
         if (!(hi1 == hi1)) hi1 = INFINITY;
       }
-      if (fi >= 0 && lo2 > hi1) {
-        a.labels[pt] = fi;
-      } else {
+      const bool settled = fi >= 0 && lo2 > hi1;
+      if (settled) a.labels[pt] = fi;
+      if (SETTLE) {
+        hs[tid] = settled ? __int_as_float(0x7fc00000) : hi1;
+        es[tid] = MODE == 1 ? expansion_bound(a, pt) : 0.0f;
+      } else if (!settled) {
         const int slot = atomicAdd(count2, 1);
         list2[slot] = pt;
         hi2[slot] = hi1;
       }
+    } else if (SETTLE && tid < TP) {
+      hs[tid] = __int_as_float(0x7fc00000);
+      es[tid] = 0.0f;
     }
+    if (SETTLE && __syncthreads_or(tid < TP && hs[tid] == hs[tid]))
+      exact_pass<MODE, false>(a, xs, cs, cflag, rs, dq, g0, cnt, hs, es, nullptr, nullptr);
   }
 }
 
@@ -345,14 +485,9 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
   float4* xs = sm4;                       // [TP][rs]
   float4* cs = xs + TP * rs;              // [TC][rs]
   float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] value offset (tile_offset)
-  __shared__ double mb[8][TP];
-  __shared__ int mi[8][TP];
   __shared__ float hs[TP];
-  __shared__ int ncand[TP];
   __shared__ float es[TP];  // MODE 1: the point's bound
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int pq = tid & 7;                 // points pq, pq + 8, pq + 16, pq + 24
-  const int cq = tid >> 3;                // centers cq*2, cq*2+1 of the block
+  const int tid = threadIdx.x;
   long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
   if (RECORD && cnt > cand_cap) {
     for (long long slot = cand_cap + (long long)blockIdx.x * blockDim.x + tid; slot < cnt;
@@ -363,9 +498,6 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
     }
     cnt = cand_cap;
   }
-  const float u = 5.9604645e-8f;
-  const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;
-
   for (long long g0 = (long long)blockIdx.x * TP; g0 < cnt; g0 += (long long)gridDim.x * TP) {
     __syncthreads();
     for (int e = tid; e < TP * dq; e += blockDim.x) {
@@ -383,117 +515,10 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
     }
     if (tid < TP) {
       hs[tid] = (g0 + tid < cnt) ? hi2[g0 + tid] : -INFINITY;
-      ncand[tid] = 0;
       es[tid] = MODE == 1 && g0 + tid < cnt ? expansion_bound(a, a.list[g0 + tid]) : 0.0f;
     }
-    double be[4];
-    int bi[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      be[i] = INFINITY;
-      bi[i] = -1;
-    }
-    for (int j0 = 0; j0 < a.k; j0 += TC) {
-      __syncthreads();
-      for (int e = tid; e < TC * dq; e += blockDim.x) {
-        const int r = e / dq, q = e % dq;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (j0 + r < a.k) v = *reinterpret_cast<const float4*>(a.C + (size_t)(j0 + r) * a.ldc + q * 4);
-        cs[r * rs + q] = v;
-      }
-      if (tid < TC) {
-        const int j = j0 + tid;
-        cflag[tid] = tile_offset<MODE>(a, j);
-      }
-      __syncthreads();
-      float acc[4][2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0f;
-      for (int q = 0; q < dq; ++q) {
-        const float4 c0 = cs[(cq * 2) * rs + q];
-        const float4 c1 = cs[(cq * 2 + 1) * rs + q];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 x = xs[(pq + 8 * i) * rs + q];
-          tile_acc<MODE>(x, c0, acc[i][0]);
-          tile_acc<MODE>(x, c1, acc[i][1]);
-        }
-      }
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const int cl = cq * 2 + jj;
-        const int j = j0 + cl;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int pl = pq + 8 * i;
-          // unusable (empty-cluster) or padding center
-          if (MODE == 0 ? cflag[cl] != 0.0f : j >= a.k) continue;
-          const float lo = MODE == 0 ? acc[i][jj] * (1.0f - gam) - 1e-30f
-                                     : fmaf(-2.0f, acc[i][jj], cflag[cl]) - es[pl];
-          if (!(lo <= hs[pl])) continue;
-          if (RECORD) {
-            const int at = atomicAdd(&ncand[pl], 1);
-            if (at < kMaxCand) cand[(g0 + pl) * kMaxCand + at] = j;
-            continue;
-          }
-          // FP64 in the oracle's order: dimensions 0 .. d-1 (padding dimensions are zero)
-          double ex = 0.0;
-          for (int q = 0; q < dq; ++q) {
-            const float4 x = xs[pl * rs + q];
-            const float4 c = cs[cl * rs + q];
-            if (MODE == 0) {
-              double dd;
-              dd = (double)x.x - (double)c.x; ex = fma(dd, dd, ex);
-              dd = (double)x.y - (double)c.y; ex = fma(dd, dd, ex);
-              dd = (double)x.z - (double)c.z; ex = fma(dd, dd, ex);
-              dd = (double)x.w - (double)c.w; ex = fma(dd, dd, ex);
-            } else {
-              ex = fma((double)x.x, (double)c.x, ex);
-              ex = fma((double)x.y, (double)c.y, ex);
-              ex = fma((double)x.z, (double)c.z, ex);
-              ex = fma((double)x.w, (double)c.w, ex);
-            }
-          }
-          if (MODE == 1) ex = fma(-2.0, ex, (double)cflag[cl]);
-          if (ex < INFINITY && (ex < be[i] || (ex == be[i] && (unsigned)j < (unsigned)bi[i]))) {
-            be[i] = ex;
-            bi[i] = j;
-          }
-        }
-      }
-    }
-    if (RECORD) {
-      __syncthreads();
-      if (tid < TP && g0 + tid < cnt) cand_cnt[g0 + tid] = ncand[tid] <= kMaxCand ? ncand[tid] : -1;
-      continue;
-    }
-    // merge the 32 threads of each point: lanes pq, pq+8, pq+16, pq+24 of every warp
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-#pragma unroll
-      for (int off = 8; off < 32; off <<= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, be[i], off);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi[i], off);
-        const bool take = (ob < be[i]) || (ob == be[i] && (unsigned)oi < (unsigned)bi[i]);
-        be[i] = take ? ob : be[i];
-        bi[i] = take ? oi : bi[i];
-      }
-      if (lane < 8) {
-        mb[w][pq + 8 * i] = be[i];
-        mi[w][pq + 8 * i] = bi[i];
-      }
-    }
     __syncthreads();
-    if (tid < TP && g0 + tid < cnt) {
-      double fb = mb[0][tid];
-      int fi = mi[0][tid];
-      for (int ww = 1; ww < 8; ++ww) {
-        const bool take = (mb[ww][tid] < fb) || (mb[ww][tid] == fb && (unsigned)mi[ww][tid] < (unsigned)fi);
-        fb = take ? mb[ww][tid] : fb;
-        fi = take ? mi[ww][tid] : fi;
-      }
-      a.labels[a.list[g0 + tid]] = fi < 0 ? 0 : fi;
-    }
+    exact_pass<MODE, RECORD>(a, xs, cs, cflag, rs, dq, g0, cnt, hs, es, cand, cand_cnt);
   }
 }
 
@@ -614,13 +639,6 @@ rerank_grouped_kernel(RerankArgs a, GroupArgs g, int* __restrict__ cand, int* __
 }  // namespace
 
 namespace {
-__global__ void count_stats_kernel(const int* counts, int full_idx, unsigned long long* stats,
-                                   const int* stop) {
-  if (stopped(stop)) return;
-  stats[0] += (unsigned long long)counts[0];
-  stats[1] += (unsigned long long)counts[full_idx];
-}
-
 // Copies the BF16 rows (and residual rows) of the flagged points into a compact buffer, row
 // `slot` for list[slot], with the point's candidate floor. One warp per row, 16-byte moves. The
 // compact buffer holds `cap` rows; flagged points beyond it go straight to `over` (the full
@@ -1108,7 +1126,8 @@ __global__ void resolve_fp64_kernel(ResolveD a) {
 // interval lies below the label's is a violation; only overlapping intervals (near ties) are
 // decided in FP64, which keeps the narrow FP64 pipe of GB300 out of the scan.
 // ws: [0] rows audited, [1] violations, [2] sampling sequence, [3] 1 + the last violating row,
-// then per sampled row a violation flag [rows] and the row [rows].
+// then per sampled row a violation flag [rows] and the row [rows], and the scan's block ticket in the
+// last word.
 __device__ __forceinline__ unsigned long long audit_hash(unsigned long long z) {
   z += 0x9E3779B97F4A7C15ull;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -1155,6 +1174,41 @@ __device__ __forceinline__ void audit_dist32x4(const float* ax, const float* __r
   }
 }
 
+// The last block of the scan to finish adds up the flags and clears them for the next audit.
+__device__ void audit_close(unsigned long long* ws, int rows) {
+  __shared__ bool last_sh;
+  __shared__ int nviol, naud;
+  __shared__ unsigned long long last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(ws + 4 + 2 * kAuditMaxRows);
+    last_sh = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last_sh) *ticket = 0;
+    __threadfence();
+    nviol = 0;
+    naud = 0;
+    last = 0;
+  }
+  __syncthreads();
+  if (!last_sh) return;
+  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+    const unsigned long long row = __ldcg(ws + 4 + rows + r);
+    if (row != ~0ull) atomicAdd(&naud, 1);  // not a skipped row
+    if (__ldcg(ws + 4 + r)) {
+      atomicAdd(&nviol, 1);
+      atomicMax(&last, row + 1);
+    }
+    ws[4 + r] = 0;  // ready for the next audit
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ws[0] += (unsigned long long)naud;
+    ws[1] += (unsigned long long)nviol;
+    ws[2] += (unsigned long long)rows;
+    if (last) ws[3] = last;
+  }
+}
+
 __global__ void __launch_bounds__(256)
 audit_scan_kernel(const float* __restrict__ X, long long ldx, long long n, int d,
                   const float* __restrict__ C, long long ldc, int k,
@@ -1174,6 +1228,7 @@ audit_scan_kernel(const float* __restrict__ X, long long ldx, long long n, int d
     const int prob = g.tile_prob[row >> 7];
     if (row >= g.row_end[prob] || (g.done && g.done[prob])) {  // uniform over the block
       if (threadIdx.x == 0 && part == 0) ws[4 + rows + r] = ~0ull;
+      audit_close(ws, rows);
       return;
     }
     cbeg = g.c_off[prob];
@@ -1227,33 +1282,7 @@ audit_scan_kernel(const float* __restrict__ X, long long ldx, long long n, int d
     if (viol_sh) atomicOr(ws + 4 + r, 1ull);
     if (part == 0) ws[4 + rows + r] = (unsigned long long)row;
   }
-}
-
-__global__ void audit_finish_kernel(unsigned long long* ws, int rows, const int* stop) {
-  if (stopped(stop)) return;
-  __shared__ int nviol, naud;
-  __shared__ unsigned long long last;
-  if (threadIdx.x == 0) {
-    nviol = 0;
-    naud = 0;
-    last = 0;
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-    if (ws[4 + rows + r] != ~0ull) atomicAdd(&naud, 1);  // not a skipped row
-    if (ws[4 + r]) {
-      atomicAdd(&nviol, 1);
-      atomicMax(&last, ws[4 + rows + r] + 1);
-    }
-    ws[4 + r] = 0;  // ready for the next audit
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ws[0] += (unsigned long long)naud;
-    ws[1] += (unsigned long long)nviol;
-    ws[2] += (unsigned long long)rows;
-    if (last) ws[3] = last;
-  }
+  audit_close(ws, rows);
 }
 }  // namespace
 
@@ -1314,13 +1343,6 @@ cudaError_t launch_resolve_fp64(const ResolveD& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_count_stats(const int* counts, int full_idx, unsigned long long* stats,
-                               const int* stop, cudaStream_t s) {
-  count_stats_kernel<<<1, 1, 0, s>>>(counts, full_idx, stats, stop);
-  count_launches(1);
-  return cudaGetLastError();
-}
-
 static size_t tiled_smem(int d) {
   const int dq = (d + 3) / 4;
   return sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
@@ -1363,10 +1385,23 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
-  auto kern = a.mode == 0 ? rerank_tiled_kernel<0> : rerank_tiled_kernel<1>;
+  auto kern = a.mode == 0 ? rerank_tiled_kernel<0, false> : rerank_tiled_kernel<1, false>;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, list2, count2, hi2);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_rerank_settle(const RerankArgs& a, cudaStream_t s) {
+  if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
+  if (a.n <= 0 || a.k <= 0) return cudaSuccess;
+  const size_t smem = tiled_smem(a.d);
+  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  auto kern = a.mode == 0 ? rerank_tiled_kernel<0, true> : rerank_tiled_kernel<1, true>;
+  if (smem > 48 * 1024)
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, nullptr, nullptr, nullptr);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1415,8 +1450,7 @@ cudaError_t launch_audit_labels(const float* X, long long ldx, long long n, int 
   audit_scan_kernel<<<rows * parts, 256, sizeof(float) * (size_t)d, s>>>(X, ldx, n, d, C, ldc, k,
                                                                         labels, ws, rows, parts, g,
                                                                         stop);
-  audit_finish_kernel<<<1, 256, 0, s>>>(ws, rows, stop);
-  count_launches(2);
+  count_launches(1);
   return cudaGetLastError();
 }
 

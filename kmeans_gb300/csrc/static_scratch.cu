@@ -109,7 +109,8 @@ extern "C" kmeansCudaErrorStatus ClusterCentersF_noalloc(const int m0, const int
   const size_t o_pcnt = o_off + align256(sizeof(int) * (size_t)(k + 1));
   const size_t o_sorted = o_pcnt + align256(sizeof(int) * (size_t)(k + 1));
   const size_t o_part = o_sorted + align256(sizeof(int) * (size_t)(m > 0 ? m : 1));
-  const size_t total = o_part + align256(sizeof(double) * (size_t)w.max_pieces * n);
+  const size_t o_tick = o_part + align256(sizeof(double) * (size_t)w.max_pieces * n);
+  const size_t total = o_tick + align256(sizeof(int));
   const cudaStream_t stream = 0;  // the reference's per-kernel entries run on the default stream
   cudaError_t e = cudaSuccess;
   // only a call with rows uses the working memory: a finalize-only call (m == 0, lastTile) is
@@ -132,8 +133,9 @@ extern "C" kmeansCudaErrorStatus ClusterCentersF_noalloc(const int m0, const int
     w.piece_cnt = reinterpret_cast<int*>(s + o_pcnt);
     w.sorted = reinterpret_cast<int*>(s + o_sorted);
     w.part = reinterpret_cast<double*>(s + o_part);
-    // clears the histogram itself before counting
-    e = launch_tile_accumulate<float>(data, n, indices + m0, w, acc, counts_large, stream);
+    w.tickets = reinterpret_cast<int*>(s + o_tick);
+    e = cudaMemsetAsync(w.tickets, 0, sizeof(int), stream);
+    if (e == cudaSuccess) e = launch_tile_accumulate<float>(data, n, indices + m0, w, acc, counts_large, stream);
   }
   if (e == cudaSuccess && lastTile)
     e = launch_finalize_acc<float>(acc, counts_large, k, n, centers, counts, stream);

@@ -22,6 +22,7 @@
 //   6. sse      one block adds the K cluster SSEs in a fixed order.
 // No floating-point atomics: the result is bit-identical run to run and equals the oracle's
 // canonical FP64 order.
+#include <algorithm>
 #include <cfloat>
 
 #include "common.cuh"
@@ -61,9 +62,55 @@ __device__ int block_excl_scan(int v) {
   return res;
 }
 
+// Nothing to update: no center won or lost a row (UpdateWork::any_dirty).
+__device__ __forceinline__ bool idle(const int* any_dirty) {
+  return any_dirty != nullptr && *reinterpret_cast<volatile const int*>(any_dirty) == 0;
+}
+
+// True in every thread of the block that finishes last of the grid (every block calls it once, after
+// its writes); *ticket is back at zero afterwards.
+__device__ __forceinline__ bool last_block(int* ticket) {
+  __shared__ bool last_sh;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last_sh = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    if (last_sh) *ticket = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last_sh;
+}
+
+// In-place exclusive scan by one block of SCAN_T threads, of values that other blocks wrote.
+__device__ void block_scan_inplace(int* data, long long n) {
+  __shared__ int carry_sh;
+  int carry = 0;
+  for (long long b0 = 0; b0 < n; b0 += SCAN_SEG) {
+    const long long base = b0 + (long long)threadIdx.x * SCAN_V;
+    int vals[SCAN_V];
+    int s = 0;
+#pragma unroll
+    for (int v = 0; v < SCAN_V; ++v) vals[v] = base + v < n ? __ldcg(data + base + v) : 0;
+#pragma unroll
+    for (int v = 0; v < SCAN_V; ++v) s += vals[v];
+    int pre = block_excl_scan(s) + carry;
+#pragma unroll
+    for (int v = 0; v < SCAN_V; ++v) {
+      if (base + v < n) data[base + v] = pre;
+      pre += vals[v];
+    }
+    if (threadIdx.x == SCAN_T - 1) carry_sh = pre;
+    __syncthreads();
+    carry = carry_sh;
+    __syncthreads();
+  }
+}
+
+// Sums of the segments; the last block turns them into their exclusive scan.
 __global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int* __restrict__ sums,
-                                   const int* stop) {
-  if (stopped(stop)) return;
+                                   int* ticket, const int* any_dirty, const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int s = 0;
 #pragma unroll
@@ -78,12 +125,13 @@ __global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int*
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (threadIdx.x == 0) sums[blockIdx.x] = t;
   }
+  if (last_block(ticket)) block_scan_inplace(sums, gridDim.x);
 }
 
 // In-place exclusive scan of segment blockIdx.x, plus offset (*offsets)[blockIdx.x] if given.
 __global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* __restrict__ offsets,
-                                const int* stop) {
-  if (stopped(stop)) return;
+                                const int* any_dirty, const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int vals[SCAN_V];
   int s = 0;
@@ -101,12 +149,70 @@ __global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* 
   }
 }
 
-// hist[l * ntiles + tile] = members of label l in the tile. SMEM: the tile counts in shared
-// memory (k ints) and writes each nonzero count once; otherwise global atomics per warp group.
-template <bool SMEM>
+// label_off[j] = start of label j in the sorted order (label_off[k] = n), counts[j] = members, and
+// piece_cnt[j] = first piece of label j, piece_cnt[k] = pieces in all, from the scanned counters. One
+// block of SCAN_T threads. No pieces for a center that keeps its sums (UpdateWork::dirty).
+__device__ void block_label_offsets(const int* hist, long long n, int k, int ntiles, int* label_off,
+                                    int* piece_cnt, long long* counts, const int* dirty) {
+  __shared__ int carry_sh;
+  constexpr int V = 4;
+  int carry = 0;
+  for (int b0 = 0; b0 < k; b0 += SCAN_T * V) {
+    const int base = b0 + threadIdx.x * V;
+    int at[V + 1], pc[V];
+    int s = 0;
+#pragma unroll
+    for (int v = 0; v <= V; ++v)
+      at[v] = base + v < k ? __ldcg(hist + (size_t)(base + v) * ntiles) : (int)n;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      pc[v] = 0;
+      if (base + v < k) {
+        const int c = at[v + 1] - at[v];
+        label_off[base + v] = at[v];
+        if (counts) counts[base + v] = c;
+        pc[v] = dirty && !dirty[base + v] ? 0 : (c + kSumPiece - 1) / kSumPiece;
+        s += pc[v];
+      }
+    }
+    int pre = block_excl_scan(s) + carry;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      if (base + v < k) piece_cnt[base + v] = pre;
+      pre += pc[v];
+    }
+    if (threadIdx.x == SCAN_T - 1) carry_sh = pre;
+    __syncthreads();
+    carry = carry_sh;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    label_off[k] = (int)n;
+    piece_cnt[k] = carry;
+  }
+}
+
+__global__ void __launch_bounds__(SCAN_T)
+label_offsets_kernel(const int* __restrict__ hist, long long n, int k, int ntiles,
+                     int* __restrict__ label_off, int* __restrict__ piece_cnt,
+                     long long* __restrict__ counts, const int* __restrict__ dirty,
+                     const int* any_dirty, const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
+  block_label_offsets(hist, n, k, ntiles, label_off, piece_cnt, counts, dirty);
+}
+
+// hist[l * ntiles + tile] = members of label l in the tile. SMEM: the tile counts in shared memory (k
+// ints) and writes every count; otherwise global atomics per warp group (hist cleared before).
+// SMALL (SCAN_T threads): the last block scans the counters and derives the labels' offsets, where
+// they are few enough for one block (kSmallHist): one launch instead of three.
+constexpr long long kSmallHist = 4 * SCAN_SEG;
+
+template <bool SMEM, bool SMALL>
 __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, int tile_pts,
-                            int ntiles, int* __restrict__ hist, int* err, const int* stop) {
-  if (stopped(stop)) return;
+                            int ntiles, int* __restrict__ hist, int* err, int* label_off,
+                            int* piece_cnt, long long* counts, const int* dirty, int* ticket,
+                            const int* any_dirty, const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
   extern __shared__ int cnt_s[];
   const int tile = blockIdx.x;
   const long long i0 = (long long)tile * tile_pts;
@@ -117,7 +223,7 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
     __syncthreads();
   }
   const int nbits = label_bits(k);
-  constexpr int U = 8;  // labels loaded ahead per thread: one memory round trip per U steps
+  constexpr int U = SMALL ? 4 : 8;  // labels loaded ahead per thread: one round trip per U steps
   for (long long b = i0; b < i1; b += (long long)blockDim.x * U) {
     int lv[U];
 #pragma unroll
@@ -144,40 +250,20 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
   }
   if (SMEM) {
     __syncthreads();
-    for (int j = threadIdx.x; j < k; j += blockDim.x) {
-      const int c = cnt_s[j];
-      if (c) hist[(size_t)j * ntiles + tile] = c;
-    }
+    for (int j = threadIdx.x; j < k; j += blockDim.x) hist[(size_t)j * ntiles + tile] = cnt_s[j];
   }
-}
-
-// label_off[j] = start of label j in the sorted order, label_off[k] = n; piece_cnt[j] = pieces
-// of label j (piece_cnt[k] = 0, the scan turns it into the total); counts[j] = members.
-__global__ void label_offsets_kernel(const int* __restrict__ hist, long long n, int k, int ntiles,
-                                     int* __restrict__ label_off, int* __restrict__ piece_cnt,
-                                     long long* __restrict__ counts, const int* __restrict__ dirty,
-                                     const int* stop) {
-  if (stopped(stop)) return;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j > k) return;
-  if (j == k) {
-    label_off[k] = (int)n;
-    piece_cnt[k] = 0;
-    return;
+  if (SMALL && last_block(ticket)) {
+    block_scan_inplace(hist, (long long)k * ntiles);
+    block_label_offsets(hist, n, k, ntiles, label_off, piece_cnt, counts, dirty);
   }
-  const int a = hist[(size_t)j * ntiles];
-  const int b = (j + 1 < k) ? hist[(size_t)(j + 1) * ntiles] : (int)n;
-  label_off[j] = a;
-  // no pieces for a center that keeps its sums (UpdateWork::dirty)
-  piece_cnt[j] = dirty && !dirty[j] ? 0 : (b - a + kSumPiece - 1) / kSumPiece;
-  if (counts) counts[j] = b - a;
 }
 
 template <bool SMEM>
 __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int k, int tile_pts,
                                int ntiles, int* pos, int* __restrict__ sorted,
-                               const int* __restrict__ dirty, const int* stop) {
-  if (stopped(stop)) return;
+                               const int* __restrict__ dirty, const int* any_dirty,
+                               const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
   extern __shared__ int cnt_s[];
   const int tile = blockIdx.x;
   const int lane = threadIdx.x;
@@ -230,8 +316,8 @@ constexpr int kScatterWarps = 8;
 __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n, int k,
                                      int tile_pts, int ntiles, const int* __restrict__ pos,
                                      int* __restrict__ sorted, const int* __restrict__ dirty,
-                                     const int* stop) {
-  if (stopped(stop)) return;
+                                     const int* any_dirty, const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
   extern __shared__ int wcnt[];  // [kScatterWarps][k]
   const int tile = blockIdx.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -305,8 +391,9 @@ __global__ void piece_sums_kernel(const float* __restrict__ X, long long ldx,
                                   const double* __restrict__ qn, const int* __restrict__ sorted,
                                   const int* __restrict__ label_off, const int* __restrict__ pstart,
                                   int k, int d, double* __restrict__ part,
-                                  double* __restrict__ partq, const int* stop) {
-  if (stopped(stop)) return;
+                                  double* __restrict__ partq, const int* any_dirty,
+                                  const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
   const int ptot = pstart[k];
   const int lane = threadIdx.x & 31;
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -455,8 +542,8 @@ __global__ void __launch_bounds__(kRingWarps * 32, 4)
 piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double* __restrict__ qn,
                        const int* __restrict__ sorted, const int* __restrict__ label_off,
                        const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
-                       double* __restrict__ partq, const int* stop) {
-  if (stopped(stop)) return;
+                       double* __restrict__ partq, const int* any_dirty, const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
   __shared__ __align__(16) float4 ring[kRingWarps][kRingStages][kRingRows][32];
   const long long ptot = pstart[k];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -514,74 +601,87 @@ piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double*
   cp_async_wait<0>();
 }
 
-// Small D (a multiple of 4, at most 64): L lanes per piece, each owning 4 consecutive
-// dimensions, 32/L pieces per warp. Each lane group walks its own piece's rows in order, so every
-// (piece, dimension) float-float sum is the same sequence of additions as in the
-// one-piece-per-warp kernel, and the whole warp computes each piece's sum of ||x||^2 with that
-// kernel's 32-lane tree; the results are identical, with 32/L times the rows in flight.
+// Small D (a multiple of 4, at most 64): L lanes per piece, each owning 4 consecutive dimensions,
+// 32/L pieces per warp. Each lane group walks its own piece's rows in order, so every (piece, dimension)
+// float-float sum is the same sequence of additions as in the one-piece-per-warp kernel; the piece's
+// sum of ||x||^2 is that kernel's 32-row tree: row i L + sub of a 32-row window is in register i of lane
+// sub, so the tree's upper levels join registers and its lower ones lanes. Bound by latency where
+// pieces are few: the window's ids and norms are loaded together, the next window's ids ahead, and
+// 16 rows are in flight per lane group (6,000 x 32, K=16: 43 us with an id round trip before every 8
+// rows and the norms piece after piece).
 template <int L>
-__global__ void piece_sums_small_kernel(const float* __restrict__ X, long long ldx,
-                                        const double* __restrict__ qn, const int* __restrict__ sorted,
-                                        const int* __restrict__ label_off,
-                                        const int* __restrict__ pstart, int k, int d,
-                                        double* __restrict__ part, double* __restrict__ partq,
-                                        const int* stop) {
-  if (stopped(stop)) return;
-  constexpr int G = 32 / L;
+__global__ void __launch_bounds__(256)
+piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double* __restrict__ qn,
+                        const int* __restrict__ sorted, const int* __restrict__ label_off,
+                        const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
+                        double* __restrict__ partq, const int* any_dirty, const int* stop) {
+  if (stopped(stop) || idle(any_dirty)) return;
+  constexpr int G = 32 / L;  // pieces per warp; also ids per lane and window
+  constexpr int R = 16;      // rows in flight
   const int ptot = pstart[k];
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int c = 4 * sub;
   for (long long p0 = gw * G; p0 < ptot; p0 += nw * G) {
     const long long p = p0 + grp;
     const bool live = p < ptot;
-    int b = 0, e = 0;
+    int b = 0, n = 0;
     if (live) {
       const int j = find_label(pstart, k, (int)p);
       b = label_off[j] + ((int)p - pstart[j]) * kSumPiece;
-      e = min(b + kSumPiece, label_off[j + 1]);
+      n = min(kSumPiece, label_off[j + 1] - b);
     }
-    if (qn) {  // the members' sum of ||x||^2, piece by piece, as the one-piece-per-warp kernel
-      for (int g = 0; g < G; ++g) {
-        const int bg = __shfl_sync(0xffffffffu, b, g * L);
-        const int eg = __shfl_sync(0xffffffffu, e, g * L);
-        if (p0 + g >= ptot) break;
-        double qs = 0.0;
-        for (int t0 = bg; t0 < eg; t0 += 32) {
-          const int nt = min(32, eg - t0);
-          double qv = lane < nt ? __ldg(qn + __ldg(sorted + t0 + lane)) : 0.0;
-          for (int o = 16; o > 0; o >>= 1) qv += __shfl_xor_sync(0xffffffffu, qv, o);
-          qs += qv;
-        }
-        if (lane == 0 && partq) partq[p0 + g] = qs;
-      }
-    } else if (partq && lane < G && p0 + lane < ptot) {
-      partq[p0 + lane] = 0.0;
-    }
-    const int c = 4 * sub;
     const bool on = live && c < d;
-    const int n = e - b;
     PieceAcc a0, a1, a2, a3;
-    for (int t = 0; t < n; t += 8) {  // eight rows in flight per lane group
-      int idx[8];
+    double qs = 0.0;
+    int id[G];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) idx[r] = t + r < n ? __ldg(sorted + b + t + r) : -1;
-      float4 v[8];
+    for (int i = 0; i < G; ++i) id[i] = i * L + sub < n ? __ldg(sorted + b + i * L + sub) : -1;
+    // the groups' pieces end at different windows: the shuffles take whole warps
+    for (int t = 0; __any_sync(0xffffffffu, t < n); t += 32) {
+      double q[G];
+      if (qn) {
 #pragma unroll
-      for (int r = 0; r < 8; ++r)
-        v[r] = (on && idx[r] >= 0)
-                   ? __ldg(reinterpret_cast<const float4*>(X + (size_t)idx[r] * ldx + c))
-                   : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < G; ++i) q[i] = id[i] >= 0 ? __ldg(qn + id[i]) : 0.0;
+      }
+      int nx[G];
 #pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        if (t + r < n) {
-          a0.add(v[r].x);
-          a1.add(v[r].y);
-          a2.add(v[r].z);
-          a3.add(v[r].w);
+      for (int i = 0; i < G; ++i)
+        nx[i] = t + 32 + i * L + sub < n ? __ldg(sorted + b + t + 32 + i * L + sub) : -1;
+#pragma unroll
+      for (int h = 0; h < 32; h += R) {
+        float4 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int row = __shfl_sync(0xffffffffu, id[(h + r) / L], grp * L + (h + r) % L);
+          v[r] = (on && row >= 0) ? __ldg(reinterpret_cast<const float4*>(X + (size_t)row * ldx + c))
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (t + h + r < n) {
+            a0.add(v[r].x);
+            a1.add(v[r].y);
+            a2.add(v[r].z);
+            a3.add(v[r].w);
+          }
         }
       }
+      if (qn) {
+#pragma unroll
+        for (int h = G / 2; h > 0; h >>= 1) {
+#pragma unroll
+          for (int i = 0; i < h; ++i) q[i] += q[i + h];
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) q[0] += __shfl_xor_sync(0xffffffffu, q[0], o);
+        if (t < n) qs += q[0];
+      }
+#pragma unroll
+      for (int i = 0; i < G; ++i) id[i] = nx[i];
     }
+    if (live && sub == 0 && partq) partq[p] = qs;
     if (on) {
       double* o = part + (size_t)p * d + c;
       o[0] = a0.value();
@@ -596,8 +696,8 @@ __global__ void piece_sums_small_kernel(const float* __restrict__ X, long long l
 // for other 16-byte-aligned rows, the scalar kernel otherwise.
 cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* qn,
                                   const int* sorted, const int* label_off, const int* pstart, int k,
-                                  int d, double* part, double* partq, const int* stop,
-                                  long long max_pieces, cudaStream_t s) {
+                                  int d, double* part, double* partq, const int* any,
+                                  const int* stop, long long max_pieces, cudaStream_t s) {
   // (the ring kernel's stage descriptor holds the chunk offset in 23 bits)
   const bool vec = ldx % 4 == 0 && d % 4 == 0 && d < (1 << 23) &&
                    (reinterpret_cast<uintptr_t>(X) & 15) == 0;
@@ -607,22 +707,22 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
   const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
   if (vec && lanes == 4)
     piece_sums_small_kernel<4><<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
-                                                      part, partq, stop);
+                                                      part, partq, any, stop);
   else if (vec && lanes == 8)
     piece_sums_small_kernel<8><<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
-                                                      part, partq, stop);
+                                                      part, partq, any, stop);
   else if (vec && lanes == 16)
     piece_sums_small_kernel<16><<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k,
-                                                       d, part, partq, stop);
+                                                       d, part, partq, any, stop);
   else if (vec) {
     // four 4-warp blocks (48 KB of ring each) per SM
     const long long cap = kmgb::num_sms() * 4LL * kRingWarps;
     const long long rw = max_pieces < cap ? max_pieces : cap;
     piece_sums_ring_kernel<<<(unsigned)((rw + kRingWarps - 1) / kRingWarps), kRingWarps * 32, 0,
-                             s>>>(X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, stop);
+                             s>>>(X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, any, stop);
   } else
     piece_sums_kernel<<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
-                                                    part, partq, stop);
+                                                    part, partq, any, stop);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
@@ -683,7 +783,7 @@ piece_sums_d_kernel(const double* __restrict__ X, long long ldx, const int* __re
 
 cudaError_t launch_piece_sums(const float* X, long long ldx, const UpdateWork& w, cudaStream_t s) {
   return launch_piece_sums_f32(X, ldx, nullptr, w.sorted, w.label_off, w.piece_cnt, w.k, w.d, w.part,
-                               nullptr, w.stop, w.max_pieces, s);
+                               nullptr, nullptr, w.stop, w.max_pieces, s);
 }
 cudaError_t launch_piece_sums(const double* X, long long ldx, const UpdateWork& w, cudaStream_t s) {
   const bool vec = ldx % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
@@ -703,15 +803,13 @@ cudaError_t launch_piece_sums(const double* X, long long ldx, const UpdateWork& 
 __global__ void finalize_kernel(const double* __restrict__ part, const double* __restrict__ partq,
                                 const int* __restrict__ label_off, const int* __restrict__ pstart,
                                 int k, int d, float* __restrict__ C, long long ldc,
-                                int empty_policy, double* __restrict__ sse_k,
-                                const int* __restrict__ dirty, const int* stop) {
+                                int empty_policy, double* __restrict__ sse_k, const int* stop) {
   if (stopped(stop)) return;
   const int groups = (d + 31) / 32;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= (long long)k * groups) return;
   const int j = (int)(wid / groups), g = (int)(wid - (long long)j * groups);
-  if (dirty && !dirty[j]) return;
   const int c = g * 32 + lane;
   const long long n = (long long)label_off[j + 1] - label_off[j];
   const int p0 = pstart[j], p1 = pstart[j + 1];
@@ -764,13 +862,12 @@ __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
                                  const int* __restrict__ pstart, int k, int d,
                                  const float* __restrict__ X, long long ldx,
                                  const int* __restrict__ sorted, const float* __restrict__ C,
-                                 long long ldc, const int* __restrict__ dirty, const int* stop) {
+                                 long long ldc, const int* stop) {
   if (stopped(stop)) return;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= k) return;
   const int j = (int)wid;
-  if (dirty && !dirty[j]) return;
   const int m0 = label_off[j], m1 = label_off[j + 1];
   if (m1 <= m0) return;
   double t = 0.0, q = 0.0;
@@ -794,8 +891,112 @@ __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
   for (int g = lane; g < groups; g += 32) sse_k[(size_t)j * groups + g] = (g == 0) ? s : 0.0;
 }
 
-// Second level of the SSE reduction plus the loop's stop rule (kmeans.cpp:1234-1237,1194):
-// relErr = |SSE - SSE_old| / |SSE|; the run stops once !(relErr > criterion), NaN included.
+// The iteration's SSE and the loop's stop rule (kmeans.cpp:1234-1237,1194): relErr = |SSE - SSE_old| /
+// |SSE|; the run stops once !(relErr > criterion), NaN included.
+__device__ __forceinline__ void store_sse(double sse, double* out, int* stop, double criterion,
+                                          double* sse_prev, double* rel_out, int* iters_done,
+                                          int indexed) {
+  if (indexed && iters_done) out[*iters_done] = sse;
+  else *out = sse;
+  if (sse_prev) {
+    const double rel = fabs(sse - *sse_prev) / fabs(sse);
+    *sse_prev = sse;
+    *rel_out = rel;
+    *iters_done += 1;
+    if (stop && !(rel > criterion)) *stop = 1;
+  }
+}
+
+// The single-problem update's last step, one block per center, a warp per group of 32 dimensions: the
+// center and its SSE term as in finalize_kernel and sse_fixup_kernel (the center's groups added in
+// order), then the last block adds the centers' terms (strided chains, a tree) and evaluates the
+// stop rule as sse_reduce_kernel does: one launch instead of three.
+__global__ void __launch_bounds__(256)
+finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long long ldc,
+                       int empty_policy, UpdateWork w, double* __restrict__ sse_out) {
+  if (stopped(w.stop)) return;
+  __shared__ double red[8];
+  const int j = blockIdx.x;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int d = w.d;
+  if (!w.dirty || w.dirty[j]) {  // uniform over the block
+    const int groups = (d + 31) / 32;
+    const int m0 = w.label_off[j], m1 = w.label_off[j + 1];
+    const long long n = m1 - m0;
+    const int p0 = w.piece_cnt[j], p1 = w.piece_cnt[j + 1];
+    double tot = 0.0;
+    for (int g = wp; g < groups; g += warps) {
+      const int c = g * 32 + lane;
+      double sse = 0.0;
+      if (c < d) {
+        double s = 0.0;
+        int p = p0;
+        for (; p + 8 <= p1; p += 8) {  // eight loads in flight, additions in piece order
+          double v[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = __ldg(w.part + (size_t)(p + i) * d + c);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) s += v[i];
+        }
+        for (; p < p1; ++p) s += __ldg(w.part + (size_t)p * d + c);
+        float mu;
+        if (n > 0) {
+          mu = __double2float_rn(__ddiv_rn(s, (double)n));
+          const double m = (double)mu;
+          sse = fma((double)n * m, m, -2.0 * m * s);
+        } else if (empty_policy == 1) {
+          mu = C[(size_t)j * ldc + c];
+        } else {
+          mu = __int_as_float(0x7fc00000);
+        }
+        C[(size_t)j * ldc + c] = mu;
+      }
+      for (int o = 16; o > 0; o >>= 1) sse += __shfl_xor_sync(0xffffffffu, sse, o);
+      tot += sse;
+    }
+    // the members' sum of ||x||^2: the last warp, lanes over the pieces, a tree
+    double q = 0.0;
+    if (wp == warps - 1) {
+      for (int p = p0 + lane; p < p1; p += 32) q += __ldg(w.partq + p);
+      for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    }
+    if (lane == 0) red[wp] = tot;
+    __syncthreads();  // and the center's dimensions are written
+    if (wp == warps - 1) {
+      double t = q;
+      for (int i = 0; i < warps; ++i) t += red[i];
+      if (n > 0 && fabs(t) <= 1e-9 * q) {
+        // cancelled: the direct form (see sse_fixup_kernel)
+        const float* mu = C + (size_t)j * ldc;
+        t = 0.0;
+        for (int m = m0; m < m1; ++m) {
+          const float* x = X + (size_t)w.sorted[m] * w.ldx;
+          for (int c = lane; c < d; c += 32) {
+            const double u = (double)x[c] - (double)mu[c];
+            t = fma(u, u, t);
+          }
+        }
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      }
+      if (lane == 0) w.sse_k[j] = n > 0 ? t : 0.0;
+    }
+  }
+  if (!last_block(w.tickets)) return;
+  double s = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < w.k; i += blockDim.x) s += __ldcg(w.sse_k + i);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __syncthreads();
+  if (lane == 0) red[wp] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double sse = 0.0;
+    for (int i = 0; i < warps; ++i) sse += red[i];
+    store_sse(sse, sse_out, w.stop, w.criterion, w.sse_prev, w.rel_out, w.iters_done, w.sse_indexed);
+  }
+}
+
+// Second level of the SSE reduction plus the loop's stop rule (host-streamed tiles, shards).
 __global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, double* __restrict__ out,
                                   int* stop, double criterion, double* sse_prev, double* rel_out,
                                   int* iters_done, int indexed) {
@@ -810,31 +1011,21 @@ __global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, doubl
     if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    const double sse = red[0];
-    if (indexed && iters_done) out[*iters_done] = sse;
-    else *out = sse;
-    if (sse_prev) {
-      const double rel = fabs(sse - *sse_prev) / fabs(sse);
-      *sse_prev = sse;
-      *rel_out = rel;
-      *iters_done += 1;
-      if (stop && !(rel > criterion)) *stop = 1;
-    }
-  }
+  if (threadIdx.x == 0)
+    store_sse(red[0], out, stop, criterion, sse_prev, rel_out, iters_done, indexed);
 }
 
-cudaError_t excl_scan(int* data, long long n, int* tmp, cudaStream_t s, const int* stop) {
+cudaError_t excl_scan(int* data, long long n, int* tmp, int* ticket, cudaStream_t s,
+                      const int* any_dirty, const int* stop) {
   if (n <= 0) return cudaSuccess;
   const long long nb = (n + SCAN_SEG - 1) / SCAN_SEG;
   if (nb > SCAN_SEG) return cudaErrorInvalidValue;
-  if (nb == 1) {
-    scan_seg_kernel<<<1, SCAN_T, 0, s>>>(data, n, nullptr, stop); kmgb::count_launches(1);
-    return cudaGetLastError();
+  if (nb > 1) {
+    scan_reduce_kernel<<<(unsigned)nb, SCAN_T, 0, s>>>(data, n, tmp, ticket, any_dirty, stop);
+    kmgb::count_launches(1);
   }
-  scan_reduce_kernel<<<(unsigned)nb, SCAN_T, 0, s>>>(data, n, tmp, stop); kmgb::count_launches(1);
-  scan_seg_kernel<<<1, SCAN_T, 0, s>>>(tmp, nb, nullptr, stop); kmgb::count_launches(1);
-  scan_seg_kernel<<<(unsigned)nb, SCAN_T, 0, s>>>(data, n, tmp, stop); kmgb::count_launches(1);
+  scan_seg_kernel<<<(unsigned)nb, SCAN_T, 0, s>>>(data, n, nb > 1 ? tmp : nullptr, any_dirty, stop);
+  kmgb::count_launches(1);
   return cudaGetLastError();
 }
 
@@ -860,29 +1051,37 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
   const long long n = w.n;
   const int k = w.k;
   const long long hist_elems = (long long)k * w.ntiles;
-  KMGB_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(int) * hist_elems, s));
   const size_t smem = sizeof(int) * (size_t)k;
-  if (smem <= 96 * 1024) {
+  const bool small = hist_elems <= kSmallHist && smem <= 48 * 1024;
+  if (small) {
+    hist_kernel<true, true><<<w.ntiles, SCAN_T, smem, s>>>(
+        labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, w.label_off, w.piece_cnt, w.counts, w.dirty,
+        w.tickets, w.any_dirty, w.stop);
+  } else if (smem <= 96 * 1024) {
     static int hist_attr_k = -1;
     if (smem > 48 * 1024 && hist_attr_k < k) {
-      KMGB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<true>,
+      KMGB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<true, false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
       hist_attr_k = k;
     }
-    hist_kernel<true><<<w.ntiles, 256, smem, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err,
-                                                  w.stop);
+    hist_kernel<true, false><<<w.ntiles, 256, smem, s>>>(
+        labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, nullptr, nullptr, nullptr, nullptr, nullptr,
+        w.any_dirty, w.stop);
   } else {
-    hist_kernel<false><<<w.ntiles, 256, 0, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err,
-                                                w.stop);
+    KMGB_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(int) * hist_elems, s));
+    hist_kernel<false, false><<<w.ntiles, 256, 0, s>>>(
+        labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, nullptr, nullptr, nullptr, nullptr, nullptr,
+        w.any_dirty, w.stop);
   }
   kmgb::count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  KMGB_CUDA_TRY(excl_scan(w.hist, hist_elems, w.scan_tmp, s, w.stop));
-  label_offsets_kernel<<<(k + 1 + 255) / 256, 256, 0, s>>>(w.hist, n, k, w.ntiles, w.label_off,
-                                                          w.piece_cnt, w.counts, w.dirty, w.stop);
-  kmgb::count_launches(1);
-  KMGB_CUDA_TRY(cudaGetLastError());
-  KMGB_CUDA_TRY(excl_scan(w.piece_cnt, k + 1, w.scan_tmp, s, w.stop));
+  if (!small) {
+    KMGB_CUDA_TRY(excl_scan(w.hist, hist_elems, w.scan_tmp, w.tickets, s, w.any_dirty, w.stop));
+    label_offsets_kernel<<<1, SCAN_T, 0, s>>>(w.hist, n, k, w.ntiles, w.label_off, w.piece_cnt, w.counts,
+                                              w.dirty, w.any_dirty, w.stop);
+    kmgb::count_launches(1);
+    KMGB_CUDA_TRY(cudaGetLastError());
+  }
   const size_t msmem = sizeof(int) * (size_t)k * kScatterWarps;
   if (msmem <= 96 * 1024) {
     static int multi_attr_k = -1;
@@ -892,7 +1091,7 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
       multi_attr_k = k;
     }
     scatter_multi_kernel<<<w.ntiles, 32 * kScatterWarps, msmem, s>>>(
-        labels, n, k, w.tile_pts, w.ntiles, w.hist, w.sorted, w.dirty, w.stop);
+        labels, n, k, w.tile_pts, w.ntiles, w.hist, w.sorted, w.dirty, w.any_dirty, w.stop);
     kmgb::count_launches(1);
   } else if (smem <= 96 * 1024) {
     static int attr_k = -1;
@@ -902,10 +1101,10 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
       attr_k = k;
     }
     scatter_kernel<true><<<w.ntiles, 32, smem, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist,
-                                                    w.sorted, w.dirty, w.stop); kmgb::count_launches(1);
+                                                    w.sorted, w.dirty, w.any_dirty, w.stop); kmgb::count_launches(1);
   } else {
     scatter_kernel<false><<<w.ntiles, 32, 0, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist,
-                                                  w.sorted, w.dirty, w.stop); kmgb::count_launches(1);
+                                                  w.sorted, w.dirty, w.any_dirty, w.stop); kmgb::count_launches(1);
   }
   return cudaGetLastError();
 }
@@ -918,25 +1117,11 @@ cudaError_t launch_update(const float* X, const double* qn, const int* labels, f
   if (w.n <= 0 || k <= 0) return cudaSuccess;
   KMGB_CUDA_TRY(sort_by_label(labels, w, s));
   KMGB_CUDA_TRY(launch_piece_sums_f32(X, w.ldx, qn, w.sorted, w.label_off, w.piece_cnt, k, w.d,
-                                     w.part, w.partq, w.stop, w.max_pieces, s));
-  const long long fin_warps = (long long)k * ((w.d + 31) / 32);
-  finalize_kernel<<<(unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s>>>(
-      w.part, qn ? w.partq : nullptr, w.label_off, w.piece_cnt, k, w.d, C, ldc, empty_policy,
-      w.sse_k, w.dirty, w.stop); kmgb::count_launches(1);
-  KMGB_CUDA_TRY(cudaGetLastError());
-  if (qn) {
-    sse_fixup_kernel<<<(unsigned)((k * 32LL + 255) / 256), 256, 0, s>>>(
-        w.sse_k, (w.d + 31) / 32, w.partq, w.label_off, w.piece_cnt, k, w.d, X, w.ldx, w.sorted, C,
-        ldc, w.dirty, w.stop);
-    kmgb::count_launches(1);
-    KMGB_CUDA_TRY(cudaGetLastError());
-  }
-  if (sse_out) {
-    sse_reduce_kernel<<<1, 1024, 0, s>>>(w.sse_k, (int)fin_warps, sse_out, w.stop, w.criterion,
-                                         w.sse_prev, w.rel_out, w.iters_done, w.sse_indexed); kmgb::count_launches(1);
-    KMGB_CUDA_TRY(cudaGetLastError());
-  }
-  return cudaSuccess;
+                                     w.part, w.partq, w.any_dirty, w.stop, w.max_pieces, s));
+  const int warps = std::min(8, (w.d + 31) / 32);
+  finalize_update_kernel<<<(unsigned)k, 32 * warps, 0, s>>>(X, C, ldc, empty_policy, w, sse_out);
+  kmgb::count_launches(1);
+  return cudaGetLastError();
 }
 
 namespace {
@@ -1080,7 +1265,7 @@ cudaError_t launch_stream_accumulate(const float* X, long long ldx, const double
   if (w.n <= 0 || w.k <= 0) return cudaSuccess;
   KMGB_CUDA_TRY(sort_by_label(labels, w, s));
   KMGB_CUDA_TRY(launch_piece_sums_f32(X, w.ldx, qn, w.sorted, w.label_off, w.piece_cnt, w.k, w.d,
-                                     w.part, w.partq, w.stop, w.max_pieces, s));
+                                     w.part, w.partq, nullptr, w.stop, w.max_pieces, s));
   accumulate_stream_kernel<<<(unsigned)(((long long)w.k * 32 + 255) / 256), 256, 0, s>>>(
       w.part, w.partq, w.label_off, w.piece_cnt, w.k, w.d, accS, accN, accQ, w.stop);
   kmgb::count_launches(1);
@@ -1250,12 +1435,12 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
   hist_batched_kernel<<<(unsigned)b.stiles, 256, 0, s>>>(labels, b, w.hist, w.err);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  KMGB_CUDA_TRY(excl_scan(w.hist, b.hist_elems, w.scan_tmp, s, nullptr));
+  KMGB_CUDA_TRY(excl_scan(w.hist, b.hist_elems, w.scan_tmp, w.tickets, s, nullptr, nullptr));
   label_offsets_batched_kernel<<<(b.K + 1 + 255) / 256, 256, 0, s>>>(w.hist, b, w.label_off,
                                                                     w.piece_cnt, w.counts);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  KMGB_CUDA_TRY(excl_scan(w.piece_cnt, b.K + 1, w.scan_tmp, s, nullptr));
+  KMGB_CUDA_TRY(excl_scan(w.piece_cnt, b.K + 1, w.scan_tmp, w.tickets, s, nullptr, nullptr));
   if (b.kmax <= 12288)
     scatter_batched_kernel<true><<<(unsigned)b.stiles, 32, sizeof(int) * (size_t)b.kmax, s>>>(
         labels, b, w.hist, w.sorted);
@@ -1264,17 +1449,16 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(launch_piece_sums_f32(X, ldx, qn, w.sorted, w.label_off, w.piece_cnt, b.K, d,
-                                     w.part, w.partq, nullptr, w.max_pieces, s));
+                                     w.part, w.partq, nullptr, nullptr, w.max_pieces, s));
   const int groups = (d + 31) / 32;
   const long long fin_warps = (long long)b.K * groups;
   finalize_kernel<<<(unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s>>>(
-      w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, nullptr,
-      nullptr);
+      w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   sse_fixup_kernel<<<(unsigned)((b.K * 32LL + 255) / 256), 256, 0, s>>>(
       w.sse_k, groups, w.partq, w.label_off, w.piece_cnt, b.K, d, X, ldx, w.sorted, C, ldc,
-      nullptr, nullptr);
+      nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   sse_batched_kernel<<<(unsigned)((b.P * 32LL + 255) / 256), 256, 0, s>>>(w.sse_k, groups, b);
