@@ -355,7 +355,11 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   const long long pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   // rows of this launch: [row0, row0 + n_rows); a device count bounds them in candidate mode
   long long n_rows = p.n;
-  if (p.n_dev) {
+  if (p.n_units_dev) {
+    const int c = *p.n_units_dev;
+    if (c <= 0) return;  // uniform over the grid, before any barrier or TMEM allocation
+    n_rows = (long long)c * UNIT;
+  } else if (p.n_dev) {
     const long long c = (long long)*p.n_dev - p.row0;
     if (c <= 0) return;  // uniform over the grid, before any barrier or TMEM allocation
     n_rows = c < p.n ? c : p.n;
@@ -370,8 +374,15 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     if (c == 0) return;
     if (compact) n_rows = c;
   }
-  auto map_x = [&](int pl) {
-    return compact ? (pl ? &tmXlc : &tmXc) : (pl ? &tmXl : &tmX);
+  // where unit u's rows lie: their first row, and whether in the compact copy
+  auto unit_rows = [&](long long u, bool& comp) -> long long {
+    if (kSel && p.u_src) {
+      const int src = __ldg(p.u_src + u);
+      comp = src < 0;
+      return src & 0x7fffffff;
+    }
+    comp = compact;
+    return u * UNIT;
   };
   const long long n_units = (n_rows + UNIT - 1) / UNIT;
   const bool cand_mode = p.thr_in != nullptr;
@@ -396,7 +407,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       if (p.g_done && p.g_done[pr]) return false;
       ui.nch = (p.g_k[pr] + BN - 1) / BN;
       ui.cbase = p.g_coff[pr];
-      ui.rend = p.g_rend[pr];
+      ui.rend = kSel && p.u_cnt ? u * UNIT + __ldg(p.u_cnt + u) : p.g_rend[pr];
       ui.cend = ui.cbase + p.g_k[pr];
     }
     ui.rot = (int)(pair % ui.nch);
@@ -446,9 +457,9 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       mbar_init(smem_u32(&bars.merge_empty[q]), 32);
     }
     fence_mbar_init();
-    prefetch_tmap(map_x(0));
+    prefetch_tmap(&tmX);
     prefetch_tmap(&tmC);
-    if (xplanes > 1) prefetch_tmap(map_x(1));
+    if (xplanes > 1) prefetch_tmap(&tmXl);
     if (cplanes > 1) prefetch_tmap(&tmCl);
     if (bias) prefetch_tmap(&tmB);
   }
@@ -484,17 +495,19 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         if (rank == 0) mbar_arrive_expect_tx(xb_local, (uint32_t)(2 * xbuf_bytes));
         const uint32_t xb = map_to_rank(xb_local, 0);
         uint8_t* xs = smem + (size_t)xi * xbuf_bytes;
-        const int xrow = (int)(p.row0 + u * UNIT + rank * BM);
+        bool comp;
+        const int xrow = (int)(p.row0 + unit_rows(u, comp) + rank * BM);
         for (int pl = 0; pl < xplanes; ++pl)
           for (int kb = 0; kb < nkb; ++kb)
-            tma_load_2d_pair(smem_u32(xs + (size_t)(pl * nkb + kb) * XKB_BYTES), map_x(pl),
-                             xb, kb * bk, xrow);
+            tma_load_2d_pair(smem_u32(xs + (size_t)(pl * nkb + kb) * XKB_BYTES),
+                             comp ? (pl ? &tmXlc : &tmXc) : (pl ? &tmXl : &tmX), xb, kb * bk, xrow);
         // the next unit's points come from HBM: start them towards L2 now, so that their TMA
         // load (queued behind the center stages) is an L2 hit
         if (u + npairs < n_units) {
-          const int nrow = (int)(p.row0 + (u + npairs) * UNIT + rank * BM);
+          const int nrow = (int)(p.row0 + unit_rows(u + npairs, comp) + rank * BM);
           for (int pl = 0; pl < xplanes; ++pl)
-            for (int kb = 0; kb < nkb; ++kb) tma_prefetch_2d(map_x(pl), kb * bk, nrow);
+            for (int kb = 0; kb < nkb; ++kb)
+              tma_prefetch_2d(comp ? (pl ? &tmXlc : &tmXc) : (pl ? &tmXl : &tmX), kb * bk, nrow);
         }
         for (int c = 0; c < ui.nch && ok; ++c) {
           const int crow = ui.cbase + chunk_of(ui, c) * BN + (int)rank * BNH;
@@ -601,6 +614,12 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t acc_empty_leader0 = map_to_rank(smem_u32(&bars.acc_empty[0]), 0);
     const uint32_t acc_empty_leader1 = map_to_rank(smem_u32(&bars.acc_empty[1]), 0);
 
+    // the data set's row behind row prow of unit u
+    auto row_of = [&](long long u, long long prow) -> long long {
+      bool comp;
+      const long long r = unit_rows(u, comp) + (prow - u * UNIT);
+      return comp ? (long long)__ldg(p.row_map + r) : p.out0 + r;
+    };
     bool alive = true;
     for (long long g0 = 0; g0 < 2 && g0 < total_chunks; ++g0)  // both buffers start free
       if (lane == 0) mbar_arrive_remote(g0 ? acc_empty_leader1 : acc_empty_leader0);
@@ -619,9 +638,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       // the point's norm bound is needed only after the last chunk: load it now so that its
       // HBM latency hides behind the unit's chunks
       const float xn_pt = ((p.certify || XMAX) && !cand_mode && h == 0 && prow < n_rows)
-                              ? __ldg(p.xnorm + (compact ? (long long)__ldg(p.row_map + prow)
-                                                         : p.out0 + prow))
-                              : 0.0f;
+                              ? __ldg(p.xnorm + row_of(u, prow)) : 0.0f;
       // separation mode: the unit's rows (one group: groups fill whole 256-row units) skip the
       // chunks of their own group
       const int unit_group = XMAX ? __ldg(p.slot_group + u * UNIT) : 0;
@@ -798,9 +815,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         b1 = fmaxf(b1, ob1[o]);
         b2 = nb2;
       }
-      // row of the data set
-      const long long pt = !compact ? p.out0 + prow
-                                    : (prow < n_rows ? (long long)__ldg(p.row_map + prow) : 0);
+      const long long pt = prow < n_rows ? row_of(u, prow) : 0;
       if (XMAX) {  // an upper bound of the largest exact key over the other groups' centers
         if (prow < n_rows)
           p.xmax_out[pt] = b1 > -1.0e38f ? __fadd_ru(b1, bound_acc(xn_pt, cm, p.d, mode, bias))
@@ -1032,8 +1047,10 @@ cudaError_t launch_assign_bf16(const void* Xb, const void* Xl, long long ldxb, c
     KMGB_CUDA_TRY(kmgb_make_tmap_2d(&tmCl, Cl, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                                     (uint64_t)a.d, (uint64_t)a.k, (uint64_t)ldcb * 2, BK, BNH));
   CUtensorMap tmXc = tmX, tmXlc = tmXl;
-  if (a.sel) {  // the compact copy of the selected rows
-    if (!a.Xc || !a.row_map || a.sel_cap <= 0 || a.u_prob || a.thr_in || a.n_dev ||
+  if (a.n_units_dev && (!a.u_prob || !a.u_src || !a.u_cnt || a.sel || a.n_dev || a.row0 || a.out0))
+    return cudaErrorInvalidValue;
+  if (a.sel || a.n_units_dev) {  // the compact copy of the selected rows
+    if (!a.Xc || !a.row_map || a.sel_cap <= 0 || (a.sel && a.u_prob) || a.thr_in || a.n_dev ||
         (mode == 2 && !a.Xlc) || (reinterpret_cast<uintptr_t>(a.Xc) & 15) ||
         (reinterpret_cast<uintptr_t>(a.Xlc) & 15))
       return cudaErrorInvalidValue;

@@ -75,6 +75,9 @@ constexpr long long kMaxRows = 1LL << 30;
 constexpr long long kMaxHist = 60LL << 20;  // scan capacity of the counting sort
 constexpr long long kMaxXBytes = 32LL << 30;
 
+constexpr size_t kPoolKeep = 8ull << 30;  // of the groups' memory, for the next call
+constexpr double kPruneMinWork = 2147483648.0;  // rows x centers (chunks of 256) x dimensions
+
 long long rup(long long v, long long m) { return (v + m - 1) / m * m; }
 
 bool on_device(const void* p) {
@@ -87,16 +90,21 @@ bool on_device(const void* p) {
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// A group's device buffers, from the library's pool and ordered on its stream (some forty cudaMalloc
+// and cudaFree per group, each waiting for the device, took 2.5 ms).
 struct DevPool {
   std::vector<void*> ptrs;
+  cudaStream_t s;
+  explicit DevPool(cudaStream_t st) : s(st) {}
   ~DevPool() {
-    for (void* p : ptrs) cudaFree(p);
+    for (void* p : ptrs) dev_free(p, s);
   }
   template <typename T>
   cudaError_t alloc(T** p, size_t count) {
-    *p = nullptr;
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (count ? count : 1));
-    if (e == cudaSuccess) ptrs.push_back(*p);
+    void* v = nullptr;
+    const cudaError_t e = dev_alloc_async(&v, sizeof(T) * (count ? count : 1), s);
+    *p = static_cast<T*>(v);
+    if (e == cudaSuccess) ptrs.push_back(v);
     return e;
   }
   template <typename T>
@@ -314,7 +322,7 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
   std::vector<float> C0((size_t)K * d, std::numeric_limits<float>::quiet_NaN());
   if (!initial_centers(pr, ids, d, C0, coff, f)) return f.code;
 
-  DevPool m;
+  DevPool m(s);
   const int E = KMEANS_ERROR_BUILDDATA;
   float *X = nullptr, *xn = nullptr, *C = nullptr, *Cop = nullptr, *cn = nullptr, *cmax = nullptr;
   double* qn = nullptr;
@@ -524,6 +532,97 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
   rx.count = over_count;
   rx.max_list = cand_cap;
   rx.stats = nullptr;
+  // Distance bounds (prune.cu) of the tensor tiers: where a group's scan is long next to their launches.
+  PruneBatch pb;
+  int* crr_list = nullptr;
+  int *d_cuprob = nullptr;
+  long long* d_crend = nullptr;
+  double work = 0.0;
+  for (int i = 0; i < P; ++i) work += (double)(rend[i] - rbeg[i]) * (double)rup(kk[i], 256) * d;
+  if (tc && o.certify && max_iters > 1 && work >= kPruneMinWork) {
+    std::vector<int> wprob, wrow, cuprob(K / 256);
+    std::vector<long long> crend(P);
+    for (int i = 0; i < P; ++i) {
+      for (long long r = rbeg[i]; r < rend[i]; r += kPruneWindow) {
+        wprob.push_back(i);
+        wrow.push_back((int)r);
+      }
+      const long long c1 = (i + 1 < P) ? coff[i + 1] : K;
+      for (long long u = coff[i] / 256; u < c1 / 256; ++u) cuprob[u] = i;
+      crend[i] = coff[i] + kk[i];
+    }
+    const long long row_bytes = ldb * (split ? 4 : 2);
+    const long long units = rows / 256 + (long long)wprob.size();
+    PruneState& q = pb.ps;
+    q.n = rows;
+    q.k = (int)K;
+    q.cap = (int)std::min<long long>(rows * 3 / 5 / 256 * 256 + 256 * (long long)wprob.size(),
+                                     (8LL << 30) / row_bytes);
+    pb.windows = (long long)wprob.size();
+    int *wp = nullptr, *wr = nullptr;
+    uint16_t *xc = nullptr, *xlc = nullptr;
+    const bool ok =
+        m.upload(&wp, wprob, s) == cudaSuccess && m.upload(&wr, wrow, s) == cudaSuccess &&
+        m.upload(&d_cuprob, cuprob, s) == cudaSuccess && m.upload(&d_crend, crend, s) == cudaSuccess &&
+        m.alloc(&q.ub, rows) == cudaSuccess && m.alloc(&q.lb, rows) == cudaSuccess &&
+        m.alloc(&q.shift, K) == cudaSuccess && m.alloc(&q.cxn, K) == cudaSuccess &&
+        m.alloc(&q.cub, K) == cudaSuccess && m.alloc(&q.clb, K) == cudaSuccess &&
+        m.alloc(&q.clab, K) == cudaSuccess && m.alloc(&crr_list, K) == cudaSuccess &&
+        m.alloc(&q.list, q.cap) == cudaSuccess && m.alloc(&q.lab_old, rows) == cudaSuccess &&
+        m.alloc(&q.dirty, K) == cudaSuccess && m.alloc(&q.flags, 8) == cudaSuccess &&
+        m.alloc(&q.top, 2 * (size_t)P) == cudaSuccess && m.alloc(&pb.top_idx, P) == cudaSuccess &&
+        m.alloc(&pb.u_prob, units) == cudaSuccess && m.alloc(&pb.u_src, units) == cudaSuccess &&
+        m.alloc(&pb.u_cnt, units) == cudaSuccess && m.alloc(&xc, (size_t)q.cap * ldb) == cudaSuccess &&
+        (!split || m.alloc(&xlc, (size_t)q.cap * ldb) == cudaSuccess) &&
+        cudaMemsetAsync(q.flags, 0, 8 * sizeof(int), s) == cudaSuccess &&
+        cudaMemsetAsync(q.dirty, 0, sizeof(int) * K, s) == cudaSuccess &&
+        cudaStreamSynchronize(s) == cudaSuccess;  // the tables are host vectors
+    if (ok) {
+      q.Xc = xc;
+      q.Xlc = xlc;
+      pb.P = P;
+      pb.win_prob = wp;
+      pb.win_row = wr;
+      pb.c_off = d_coff;
+      pb.kp = d_k;
+      pb.row_end = d_rend;
+      pb.done = d_done;
+      w.dirty = q.dirty;
+    } else {  // no room: every iteration scans every row
+      cudaGetLastError();
+    }
+  }
+  const bool prune = pb.P > 0;
+  // the scan of the centers against themselves, then the rows to scan
+  auto issue_prune = [&]() -> cudaError_t {
+    AssignArgs c = a;
+    c.n = K;
+    c.n_dev = pb.ps.flags;
+    c.xnorm = pb.ps.cxn;
+    c.labels = pb.ps.clab;
+    c.rerank_list = crr_list;
+    c.rerank_count = pb.ps.flags + 2;
+    c.ub = pb.ps.cub;
+    c.lb = pb.ps.clb;
+    c.u_prob = d_cuprob;
+    c.g_rend = d_crend;
+    cudaError_t e = launch_assign_bf16(Cb, Cl, ldb, Cb, Cl, ldb, c, s);
+    if (e == cudaSuccess) e = launch_prune_batched(pb, labels, Xb, Xl, ldb * 2, s);
+    return e;
+  };
+  AssignArgs am = a;
+  if (prune) {
+    am.ub = pb.ps.ub;
+    am.lb = pb.ps.lb;
+    am.u_prob = pb.u_prob;
+    am.u_src = pb.u_src;
+    am.u_cnt = pb.u_cnt;
+    am.n_units_dev = pb.ps.flags + 3;
+    am.sel_cap = pb.ps.cap;
+    am.row_map = pb.ps.list;
+    am.Xc = pb.ps.Xc;
+    am.Xlc = Xl ? pb.ps.Xlc : nullptr;
+  }
   cudaEvent_t ev[2] = {nullptr, nullptr};
   if (f.set(cudaEventCreate(&ev[0]), EU, "events") || f.set(cudaEventCreate(&ev[1]), EU, "events") ||
       f.set(cudaEventRecord(ev[0], s), EU, "events")) {
@@ -559,12 +658,13 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
     auto mk = [&]() { return !marks || mark(); };
     return mk() && !f.set(cudaMemsetAsync(cmax, 0, sizeof(float), s), EU, "centers") &&
            !f.set(launch_prep_centers(C, ldx, (int)K, d, Cop, Cb, ldb, cn, cmax, s, nullptr,
-                                      cinit, Cl, cbias),
+                                      cinit, Cl, cbias, pb.ps.shift, pb.ps.cxn),
                   EU, "center preparation") &&
            !f.set(cudaMemsetAsync(rr_count, 0, sizeof(int), s), KMEANS_ERROR_CLOSEST_CENTERS,
                   "re-rank") &&
            mk() &&
-           !f.set(tc ? launch_assign_bf16(Xb, Xl, ldb, Cb, Cl, ldb, a, s)
+           !(prune && f.set(issue_prune(), KMEANS_ERROR_CLOSEST_CENTERS, "distance bounds")) &&
+           !f.set(tc ? launch_assign_bf16(Xb, Xl, ldb, Cb, Cl, ldb, am, s)
                      : launch_assign_fp32(X, ldx, Cop, ldx, a, s, &g, tiles),
                   KMEANS_ERROR_CLOSEST_CENTERS, "assignment") &&
            mk() &&
@@ -583,6 +683,7 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
                                        audit_rows, nullptr, s, &g),
                    KMEANS_ERROR_CLOSEST_CENTERS, "audit")) &&
            mk() &&
+           !(prune && f.set(launch_prune_dirty_batched(pb, labels, s), EU, "distance bounds")) &&
            !f.set(launch_update_batched(X, ldx, d, qn, labels, C, ldx, o.empty_policy, w, b, s),
                   EU, "update") &&
            mk();
@@ -783,6 +884,7 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
   }
   cudaStreamSynchronize(s);
   cudaStreamDestroy(s);
+  dev_trim(kPoolKeep);
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
     int it = 0;

@@ -132,6 +132,11 @@ void dev_free(void* p, cudaStream_t s) {
   }
 }
 
+void dev_trim(size_t keep) {
+  cudaMemPool_t pool = nullptr;
+  if (pool_of_current_device(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, keep);
+}
+
 cudaError_t dev_release_cached() {
   cudaError_t r = cudaDeviceSynchronize();
   std::lock_guard<std::mutex> g(g_mu);

@@ -82,6 +82,12 @@ struct AssignArgs {
   const int* row_map;
   const void* Xc;
   const void* Xlc;
+  // Grouped problems with bounds (null otherwise): the units to scan are a device table of *n_units_dev
+  // entries -- problem u_prob[u], rows u_src[u] .. + u_cnt[u] - 1 of X, or, with the top bit of u_src
+  // set, of the compact copy Xc / Xlc (sel_cap rows), whose row i stands for row row_map[i]
+  const int* n_units_dev;
+  const int* u_src;
+  const int* u_cnt;
   // test hook of the FP32 tier (kmgb_debug_withhold_stage): the producer issues no TMA load for
   // pipeline steps >= test_withhold (0: every step), and every wait gives up after
   // test_wait_cycles SM cycles (0: KMGB_WAIT_CYCLES)
@@ -262,6 +268,30 @@ struct PruneState {
 // centers and the rows whose label they no longer prove are listed (flags[1] > cap: all rows).
 cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
                                 cudaStream_t s);
+// The same for batched problems (rows and centers as in GroupArgs, centers padded to 256 per problem):
+// windows of up to kPruneWindow rows of one problem, each listing its rows to scan as units of 256
+// (AssignArgs::n_units_dev).
+constexpr int kPruneWindow = 4096;
+struct PruneBatch {
+  PruneState ps;           // n, k: all rows and centers; cap: compact rows; list: [cap]; flags: [0] 0: no
+                           // bounds yet, else k, [2] scratch count, [3] units, [4] compact rows; top:
+                           // [2 P]; the rest as there
+  int P = 0;
+  long long windows = 0;
+  const int* win_prob = nullptr;   // [windows]
+  const int* win_row = nullptr;    // [windows] first row
+  const int* c_off = nullptr;      // [P]
+  const int* kp = nullptr;         // [P]
+  const long long* row_end = nullptr;
+  const int* done = nullptr;
+  int* top_idx = nullptr;          // [P] the center that moved most
+  int* u_prob = nullptr;           // the unit table
+  int* u_src = nullptr;
+  int* u_cnt = nullptr;
+};
+cudaError_t launch_prune_batched(const PruneBatch& pb, const int* labels, const void* Xb,
+                                 const void* Xl, long long row_bytes, cudaStream_t s);
+cudaError_t launch_prune_dirty_batched(const PruneBatch& pb, const int* labels, cudaStream_t s);
 // After the labels are settled: the centers that lost or won a row.
 cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const int* stop,
                                cudaStream_t s);
@@ -390,7 +420,7 @@ struct BatchUpdate {
 cudaError_t launch_update_batched(const float* X, long long ldx, int d, const double* qn,
                                   const int* labels, float* C, long long ldc, int empty_policy,
                                   const UpdateWork& w, const BatchUpdate& b,
-                                  cudaStream_t s);
+                                  cudaStream_t s);  // (w.dirty as in launch_update)
 
 // Mini-batch gather: rows perm[(start + r) mod m] of Xsrc into Xdst (m_mb rows).
 cudaError_t launch_gather_rows(const float* Xsrc, long long ldx, const int* perm, long long m,
@@ -456,6 +486,8 @@ cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s);
 // The same without waiting for s: memory for work queued on s after the call.
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
+// Unused memory beyond `keep` bytes goes back to the device.
+void dev_trim(size_t keep);
 cudaError_t dev_release_cached();
 
 }  // namespace kmgb

@@ -214,14 +214,32 @@ __global__ void prune_gather_kernel(PruneState ps, const uint4* __restrict__ Xb,
 }
 
 // Marks the old and the new center of every scanned row whose label changed since the last update
-// (after a first iteration every center is marked already and lab_old takes all labels).
-__global__ void __launch_bounds__(256)
+// (after a first iteration every center is marked already and lab_old takes all labels). A block
+// collects its marks in shared memory where the centers fit: in early iterations hundreds of
+// thousands of rows mark the same few hundred centers (898,790 rows, K=256: 300 us through global
+// memory).
+constexpr int kDirtyShared = 32768;
+
+__global__ void __launch_bounds__(1024)
 prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
   if (stopped(stop)) return;
   const int cnt = ps.flags[1];
+  if (cnt == 0) return;
+  extern __shared__ unsigned char mark[];
+  const bool sh = ps.k <= kDirtyShared;
+  if (sh) {
+    for (int j = threadIdx.x; j < ps.k; j += blockDim.x) mark[j] = 0;
+    __syncthreads();
+  }
   const bool all = cnt > ps.cap;
   const long long total = all ? ps.n : cnt;
   bool changed = false;
+  auto set = [&](int j) {
+    if (j < 0 || j >= ps.k) return;
+    if (sh) mark[j] = 1;
+    else if (!*(volatile int*)(ps.dirty + j)) ps.dirty[j] = 1;
+  };
+#pragma unroll 4
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long pt = all ? i : (long long)__ldg(ps.list + i);
@@ -229,19 +247,216 @@ prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* sto
     if (a == b) continue;
     ps.lab_old[pt] = b;
     changed = true;
-    // (looked at first: in early iterations thousands of rows mark the same few centers)
+    set(a);
+    set(b);
+  }
+  if (!__syncthreads_or(changed)) return;
+  if (threadIdx.x == 0) ps.flags[4] = 1;
+  if (sh)
+    for (int j = threadIdx.x; j < ps.k; j += blockDim.x)
+      if (mark[j]) ps.dirty[j] = 1;
+}
+
+// ------------------------------------ batched problems ------------------------------------
+// One block per problem: its two largest moves, and its centers' dirty marks cleared (set in the first
+// iteration).
+__global__ void __launch_bounds__(256)
+prune_top_batched_kernel(PruneBatch pb) {
+  __shared__ float s1[8], s2[8];
+  __shared__ int si[8];
+  const PruneState& ps = pb.ps;
+  const int prob = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int first = ps.flags[0] == 0;
+  const int c0 = pb.c_off[prob], k = pb.kp[prob];
+  float b1 = 0.0f, b2 = 0.0f;
+  int i1 = -1;
+  auto merge = [&](float o1, float o2, int oi) {
+    b2 = fmaxf(fminf(b1, o1), fmaxf(b2, o2));
+    if (o1 > b1) {
+      b1 = o1;
+      i1 = oi;
+    }
+  };
+  for (int j = c0 + threadIdx.x; j < c0 + k; j += blockDim.x) {
+    merge(ps.shift[j], 0.0f, j);
+    ps.dirty[j] = first;
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    merge(__shfl_down_sync(0xffffffffu, b1, o), __shfl_down_sync(0xffffffffu, b2, o),
+          __shfl_down_sync(0xffffffffu, i1, o));
+  if (lane == 0) {
+    s1[w] = b1;
+    s2[w] = b2;
+    si[w] = i1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int v = 1; v < 8; ++v) merge(s1[v], s2[v], si[v]);
+    ps.top[2 * prob] = b1;
+    ps.top[2 * prob + 1] = b2;
+    pb.top_idx[prob] = i1;
+  }
+}
+
+// One block per window: moves the rows' bounds, then hands the rows they no longer prove to the
+// scan -- copied to the compact matrix as ceil(rows / 256) units of their own, or, where most of the
+// window fails (or the compact matrix is full), as the window's original units. Units come in any
+// order; a window's last one may be part full, which at 4,096 rows a window costs less than a scan
+// over all windows' counts would.
+__global__ void __launch_bounds__(PF_THREADS)
+prune_window_kernel(PruneBatch pb, const int* __restrict__ labels, const uint4* __restrict__ Xb,
+                    const uint4* __restrict__ Xl, int row_vec) {
+  constexpr int kPer = kPruneWindow / PF_THREADS;
+  __shared__ int rows_sh[kPruneWindow];
+  __shared__ int wsum[PF_THREADS / 32];
+  __shared__ int unit_sh, crow_sh, total_sh;
+  const PruneState& ps = pb.ps;
+  const int win = blockIdx.x;
+  const int prob = pb.win_prob[win];
+  if (pb.done[prob]) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r0 = pb.win_row[win];
+  const int n = (int)min((long long)kPruneWindow, pb.row_end[prob] - r0);
+  const bool first = ps.flags[0] == 0;
+  unsigned fail = 0;
+  if (!first) {
+    const float top1 = ps.top[2 * prob], top2 = ps.top[2 * prob + 1];
+    const int topi = pb.top_idx[prob];
+    const int c0 = pb.c_off[prob], c1 = c0 + pb.kp[prob];
+#pragma unroll 4
+    for (int i = 0; i < kPer; ++i) {
+      const int r = i * PF_THREADS + threadIdx.x;
+      if (r >= n) continue;
+      const long long pt = (long long)r0 + r;
+      const int a = __ldg(labels + pt);
+      const bool lab_ok = a >= c0 && a < c1;
+      const float sh = lab_ok ? __ldg(ps.shift + a) : -1.0f;
+      const float near = lab_ok ? __ldg(ps.clb + a) : 0.0f;
+      const float u = sh < 0.0f ? INFINITY : __fadd_ru(ps.ub[pt], sh);
+      float l = __fsub_rd(ps.lb[pt], a == topi ? top2 : top1);
+      const float l2 = __fsub_rd(near, u);
+      l = l2 > l ? l2 : l;
+      ps.ub[pt] = u;
+      ps.lb[pt] = l;
+      if (!(__fmul_ru(u, 1.0f + 0x1p-20f) < l)) fail |= 1u << i;
+    }
+  }
+  const int c = __popc(fail);
+  int inc = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) wsum[w] = inc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int t = 0;
+    for (int v = 0; v < PF_THREADS / 32; ++v) {
+      const int x = wsum[v];
+      wsum[v] = t;
+      t += x;
+    }
+    total_sh = first ? n : t;
+    crow_sh = -1;
+    if (total_sh > 0) {
+      int units = (total_sh + 255) / 256;
+      if (!first && total_sh * 5 <= n * 3) {
+        const int at = atomicAdd(ps.flags + 4, units * 256);
+        if (at + units * 256 <= ps.cap) crow_sh = at;
+      }
+      if (crow_sh < 0) units = (n + 255) / 256;
+      unit_sh = atomicAdd(ps.flags + 3, units);
+    }
+  }
+  __syncthreads();
+  const int total = total_sh, crow = crow_sh, unit = unit_sh;
+  if (total == 0) return;
+  if (crow < 0) {
+    for (int u = threadIdx.x; u < (n + 255) / 256; u += PF_THREADS) {
+      pb.u_prob[unit + u] = prob;
+      pb.u_src[unit + u] = r0 + 256 * u;
+      pb.u_cnt[unit + u] = min(256, n - 256 * u);
+    }
+    return;
+  }
+  for (int u = threadIdx.x; u < (total + 255) / 256; u += PF_THREADS) {
+    pb.u_prob[unit + u] = prob;
+    pb.u_src[unit + u] = (crow + 256 * u) | (int)0x80000000;
+    pb.u_cnt[unit + u] = min(256, total - 256 * u);
+  }
+  int at = wsum[w] + inc - c;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i)
+    if (fail & (1u << i)) {
+      const int row = r0 + i * PF_THREADS + threadIdx.x;
+      rows_sh[at] = row;
+      ps.list[crow + at] = row;
+      ++at;
+    }
+  __syncthreads();
+  // the rows' planes, 16 bytes per thread at a time
+  const int per = row_vec * (Xl ? 2 : 1);
+  uint4* Xc = static_cast<uint4*>(ps.Xc);
+  uint4* Xlc = static_cast<uint4*>(ps.Xlc);
+#pragma unroll 4
+  for (int e = threadIdx.x; e < total * per; e += PF_THREADS) {
+    const int i = e / per, v = e - i * per;
+    const size_t src = (size_t)rows_sh[i] * row_vec, dst = (size_t)(crow + i) * row_vec;
+    if (v < row_vec) Xc[dst + v] = __ldg(Xb + src + v);
+    else Xlc[dst + v - row_vec] = __ldg(Xl + src + v - row_vec);
+  }
+}
+
+// The centers that lost or won a row since the last update; one block per window. The scans of this
+// iteration are done: block 0 starts the next one's unit table.
+__global__ void __launch_bounds__(PF_THREADS)
+prune_dirty_batched_kernel(PruneBatch pb, const int* __restrict__ labels) {
+  const PruneState& ps = pb.ps;
+  const int win = blockIdx.x;
+  if (win == 0 && threadIdx.x == 0) {
+    ps.flags[0] = ps.k;
+    ps.flags[2] = ps.flags[3] = ps.flags[4] = 0;
+  }
+  const int prob = pb.win_prob[win];
+  if (pb.done[prob]) return;
+  const int r0 = pb.win_row[win];
+  const int n = (int)min((long long)kPruneWindow, pb.row_end[prob] - r0);
+#pragma unroll 4
+  for (int r = threadIdx.x; r < n; r += PF_THREADS) {
+    const long long pt = (long long)r0 + r;
+    const int a = ps.lab_old[pt], b = labels[pt];
+    if (a == b) continue;
+    ps.lab_old[pt] = b;
     if (a >= 0 && a < ps.k && !*(volatile int*)(ps.dirty + a)) ps.dirty[a] = 1;
     if (b >= 0 && b < ps.k && !*(volatile int*)(ps.dirty + b)) ps.dirty[b] = 1;
   }
-  if (__syncthreads_or(changed) && threadIdx.x == 0) ps.flags[4] = 1;
 }
 
 }  // namespace
 
+cudaError_t launch_prune_batched(const PruneBatch& pb, const int* labels, const void* Xb,
+                                 const void* Xl, long long row_bytes, cudaStream_t s) {
+  if (row_bytes % 16 || (Xl && !pb.ps.Xlc)) return cudaErrorInvalidValue;
+  prune_top_batched_kernel<<<(unsigned)pb.P, 256, 0, s>>>(pb);
+  prune_window_kernel<<<(unsigned)pb.windows, PF_THREADS, 0, s>>>(
+      pb, labels, static_cast<const uint4*>(Xb), static_cast<const uint4*>(Xl), (int)(row_bytes / 16));
+  count_launches(2);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_prune_dirty_batched(const PruneBatch& pb, const int* labels, cudaStream_t s) {
+  prune_dirty_batched_kernel<<<(unsigned)pb.windows, PF_THREADS, 0, s>>>(pb, labels);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const int* stop,
                                cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
-  prune_dirty_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(ps, labels, stop);
+  const long long blocks = (ps.n + 1023) / 1024, most = 2LL * kmgb::num_sms();
+  prune_dirty_kernel<<<(unsigned)(blocks < most ? blocks : most), 1024,
+                       ps.k <= kDirtyShared ? ps.k : 0, s>>>(ps, labels, stop);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -523,27 +523,33 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
 }
 
 // Grouped (batched Lloyd) re-rank, one warp per flagged row of any problem; the row's own
-// problem (tile_prob[row / 128]) gives its center range. Pass 1, FP32 direct form: the lanes
-// split the dimensions of four centers at a time (coalesced rows, a tree sum per center -- like
-// any order it stays within the (d+4) 2u relative bound of a sum of non-negative terms); the
-// values of up to RG_VCAP centers stay in shared memory. Pass 2: every usable center whose FP32
+// problem (tile_prob[row / 128]) gives its center range. Pass 1, FP32 direct form: L lanes split a
+// center's dimensions, 16 bytes each at a time, 32 / L centers side by side and four in turn (a tree
+// sum per center -- like any order it stays within the (d+4) 2u relative bound of a sum of
+// non-negative terms); the values of up to RG_VCAP centers stay in shared memory. (A whole warp per
+// center left 16 of 32 lanes idle at D = 16 and took four centers a step.) Pass 2: every usable center whose FP32
 // lower end is within the smallest upper end is evaluated in FP64 in the oracle's order
 // (sequential fma over the dimensions), the smallest value winning, lowest index on ties.
 // Labels are global center indices.
 constexpr int RG_VCAP = 512;
 constexpr int RG_WARPS = 8;
 
+template <int L>
 __global__ void __launch_bounds__(RG_WARPS * 32)
 rerank_grouped_kernel(RerankArgs a, GroupArgs g, int* __restrict__ cand, int* __restrict__ cand_cnt,
                       long long cand_cap) {
   if (stopped(a.stop)) return;
-  extern __shared__ float rg_smem[];  // [warps][RG_VCAP] values, then [warps][d] rows
+  extern __shared__ float rg_smem[];  // [warps][RG_VCAP] values, then [warps][ds] rows
+  constexpr int G = 32 / L;           // centers side by side
+  constexpr int U = 4;                // and in turn, their loads in flight together
   const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
   const float u = 5.9604645e-8f;
   const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int grp = lane / L, sub = lane % L;
+  const int ds = (a.d + 3) / 4 * 4;
   float* vals = rg_smem + (size_t)w * RG_VCAP;
-  float* xs = rg_smem + (size_t)RG_WARPS * RG_VCAP + (size_t)w * a.d;
+  float* xs = rg_smem + (size_t)RG_WARPS * RG_VCAP + (size_t)w * ds;
   for (long long slot = (long long)blockIdx.x * RG_WARPS + w; slot < cnt;
        slot += (long long)gridDim.x * RG_WARPS) {
     const int pt = a.list[slot];
@@ -552,38 +558,40 @@ rerank_grouped_kernel(RerankArgs a, GroupArgs g, int* __restrict__ cand, int* __
     const bool keep = kp <= RG_VCAP;
     const float* x = a.X + (size_t)pt * a.ldx;
     __syncwarp();
-    for (int t = lane; t < a.d; t += 32) xs[t] = x[t];
+    for (int t = lane; t < ds; t += 32) xs[t] = t < a.d ? x[t] : 0.0f;
     __syncwarp();
     float lo = INFINITY;
-    for (int j0 = 0; j0 < kp; j0 += 4) {
-      float sv[4] = {0.f, 0.f, 0.f, 0.f};
-      const float* cr[4];
+    for (int j0 = 0; j0 < kp; j0 += G * U) {
+      float sv[U];
+      const float* cr[U];
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        cr[r] = a.C + (size_t)(cbeg + min(j0 + r, kp - 1)) * a.ldc;
-      for (int t = lane; t < a.d; t += 32) {
-        const float xt = xs[t];
+      for (int r = 0; r < U; ++r) {
+        sv[r] = 0.0f;
+        cr[r] = a.C + (size_t)(cbeg + min(j0 + r * G + grp, kp - 1)) * a.ldc;
+      }
+      // rows are padded with zeros to ldc, a multiple of 4, as xs to ds
+      for (int t = 4 * sub; t < ds; t += 4 * L) {
+        const float4 xt = *reinterpret_cast<const float4*>(xs + t);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const float df = xt - __ldg(cr[r] + t);
-          sv[r] = fmaf(df, df, sv[r]);
-        }
+        for (int r = 0; r < U; ++r) tile_acc<0>(xt, __ldg(reinterpret_cast<const float4*>(cr[r] + t)), sv[r]);
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
+      for (int o = L / 2; o > 0; o >>= 1) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r) sv[r] += __shfl_xor_sync(0xffffffffu, sv[r], o);
+        for (int r = 0; r < U; ++r) sv[r] += __shfl_xor_sync(0xffffffffu, sv[r], o);
       }
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int j = j0 + r;
+      for (int r = 0; r < U; ++r) {
+        const int j = j0 + r * G + grp;
         if (j < kp) {
           const float v = (a.cn[cbeg + j] < INFINITY) ? sv[r] : INFINITY;  // unusable center
           lo = fminf(lo, v);
-          if (keep && lane == 0) vals[j] = v;
+          if (keep && sub == 0) vals[j] = v;
         }
       }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     __syncwarp();
     const float best_hi = lo * (1.0f + gam) + 1e-30f;
     if (cand && slot < cand_cap) {
@@ -1409,13 +1417,16 @@ cudaError_t launch_rerank_settle(const RerankArgs& a, cudaStream_t s) {
 cudaError_t launch_rerank_grouped(const RerankArgs& a, const GroupArgs& g, cudaStream_t s,
                                   int* cand, int* cand_cnt, long long cand_cap) {
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
-  const size_t smem = sizeof(float) * (size_t)RG_WARPS * (RG_VCAP + (size_t)a.d);
+  if (a.ldc % 4 || (reinterpret_cast<uintptr_t>(a.C) & 15)) return cudaErrorInvalidValue;
+  const size_t ds = ((size_t)a.d + 3) / 4 * 4;
+  const size_t smem = sizeof(float) * (size_t)RG_WARPS * (RG_VCAP + ds);
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  auto kern = a.d <= 16 ? rerank_grouped_kernel<4>
+                        : (a.d <= 32 ? rerank_grouped_kernel<8>
+                                     : (a.d <= 64 ? rerank_grouped_kernel<16> : rerank_grouped_kernel<32>));
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_grouped_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  rerank_grouped_kernel<<<kmgb::num_sms() * 4, RG_WARPS * 32, smem, s>>>(a, g, cand, cand_cnt,
-                                                                          cand_cap);
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<kmgb::num_sms() * 4, RG_WARPS * 32, smem, s>>>(a, g, cand, cand_cnt, cand_cap);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -803,13 +803,15 @@ cudaError_t launch_piece_sums(const double* X, long long ldx, const UpdateWork& 
 __global__ void finalize_kernel(const double* __restrict__ part, const double* __restrict__ partq,
                                 const int* __restrict__ label_off, const int* __restrict__ pstart,
                                 int k, int d, float* __restrict__ C, long long ldc,
-                                int empty_policy, double* __restrict__ sse_k, const int* stop) {
+                                int empty_policy, double* __restrict__ sse_k,
+                                const int* __restrict__ dirty, const int* stop) {
   if (stopped(stop)) return;
   const int groups = (d + 31) / 32;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= (long long)k * groups) return;
   const int j = (int)(wid / groups), g = (int)(wid - (long long)j * groups);
+  if (dirty && !dirty[j]) return;
   const int c = g * 32 + lane;
   const long long n = (long long)label_off[j + 1] - label_off[j];
   const int p0 = pstart[j], p1 = pstart[j + 1];
@@ -862,12 +864,13 @@ __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
                                  const int* __restrict__ pstart, int k, int d,
                                  const float* __restrict__ X, long long ldx,
                                  const int* __restrict__ sorted, const float* __restrict__ C,
-                                 long long ldc, const int* stop) {
+                                 long long ldc, const int* __restrict__ dirty, const int* stop) {
   if (stopped(stop)) return;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= k) return;
   const int j = (int)wid;
+  if (dirty && !dirty[j]) return;
   const int m0 = label_off[j], m1 = label_off[j + 1];
   if (m1 <= m0) return;
   double t = 0.0, q = 0.0;
@@ -1337,7 +1340,8 @@ __global__ void hist_batched_kernel(const int* __restrict__ labels, BatchUpdate 
 // and member counts, from the scanned counters.
 __global__ void label_offsets_batched_kernel(const int* __restrict__ hist, BatchUpdate b,
                                              int* __restrict__ label_off, int* __restrict__ piece_cnt,
-                                             long long* __restrict__ counts) {
+                                             long long* __restrict__ counts,
+                                             const int* __restrict__ dirty) {
   const int gc = blockIdx.x * blockDim.x + threadIdx.x;
   if (gc > b.K) return;
   auto start = [&](int c) -> int {
@@ -1352,14 +1356,14 @@ __global__ void label_offsets_batched_kernel(const int* __restrict__ hist, Batch
   }
   const int a0 = start(gc), a1 = start(gc + 1);
   label_off[gc] = a0;
-  piece_cnt[gc] = (a1 - a0 + kSumPiece - 1) / kSumPiece;
+  piece_cnt[gc] = dirty && !dirty[gc] ? 0 : (a1 - a0 + kSumPiece - 1) / kSumPiece;
   if (counts) counts[gc] = a1 - a0;
 }
 
 // One warp per sort tile. SMEM: the tile's k counters live in shared memory (k <= smem_k).
 template <bool SMEM>
 __global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpdate b, int* pos,
-                                       int* __restrict__ sorted) {
+                                       int* __restrict__ sorted, const int* __restrict__ dirty) {
   extern __shared__ int cnt_s[];
   const long long st = blockIdx.x;
   const int prob = b.stile_prob[st];
@@ -1380,9 +1384,10 @@ __global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpda
     int l = -1;
     if (i < i1) {
       l = lnext - cb;
-      if (l < 0 || l >= kp) l = -1;
+      if (l < 0 || l >= kp || (dirty && !__ldg(dirty + cb + l))) l = -1;
     }
     if (base + 32 + lane < i1) lnext = labels[base + 32 + lane];  // next batch in flight
+    if (!__any_sync(0xffffffffu, l >= 0)) continue;
     const unsigned peers = warp_peers(l, nbits);
     const int leader = __ffs(peers) - 1;
     const int rank = __popc(peers & lanemask_lt());
@@ -1437,15 +1442,16 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.hist, b.hist_elems, w.scan_tmp, w.tickets, s, nullptr, nullptr));
   label_offsets_batched_kernel<<<(b.K + 1 + 255) / 256, 256, 0, s>>>(w.hist, b, w.label_off,
-                                                                    w.piece_cnt, w.counts);
+                                                                    w.piece_cnt, w.counts, w.dirty);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.piece_cnt, b.K + 1, w.scan_tmp, w.tickets, s, nullptr, nullptr));
   if (b.kmax <= 12288)
     scatter_batched_kernel<true><<<(unsigned)b.stiles, 32, sizeof(int) * (size_t)b.kmax, s>>>(
-        labels, b, w.hist, w.sorted);
+        labels, b, w.hist, w.sorted, w.dirty);
   else
-    scatter_batched_kernel<false><<<(unsigned)b.stiles, 32, 0, s>>>(labels, b, w.hist, w.sorted);
+    scatter_batched_kernel<false><<<(unsigned)b.stiles, 32, 0, s>>>(labels, b, w.hist, w.sorted,
+                                                                    w.dirty);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(launch_piece_sums_f32(X, ldx, qn, w.sorted, w.label_off, w.piece_cnt, b.K, d,
@@ -1453,12 +1459,13 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
   const int groups = (d + 31) / 32;
   const long long fin_warps = (long long)b.K * groups;
   finalize_kernel<<<(unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s>>>(
-      w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, nullptr);
+      w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, w.dirty,
+      nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   sse_fixup_kernel<<<(unsigned)((b.K * 32LL + 255) / 256), 256, 0, s>>>(
       w.sse_k, groups, w.partq, w.label_off, w.piece_cnt, b.K, d, X, ldx, w.sorted, C, ldc,
-      nullptr);
+      w.dirty, nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   sse_batched_kernel<<<(unsigned)((b.P * 32LL + 255) / 256), 256, 0, s>>>(w.sse_k, groups, b);

@@ -162,3 +162,24 @@ def test_auto_tier_and_graph_replay_equal_oracle(km, orc, torch_cuda):
     for a, b in zip(res, res2):
         assert np.array_equal(a.labels, b.labels)
         assert np.array_equal(a.centers, b.centers, equal_nan=True)
+
+
+@pytest.mark.parametrize("tier", [1, 2])
+@pytest.mark.parametrize("policy,criterion", [(1, -1.0), (0, 1e-4)])
+def test_bounds_in_large_batches(km, orc, torch_cuda, tier, policy, criterion):
+    """Groups large enough for the distance bounds: problems from one row to several windows,
+    separated and overlapping clusters, duplicates, stop rules that fire at different iterations."""
+    probs = []
+    for i, (n, d, k) in enumerate([(1, 16, 1), (255, 16, 4), (4096, 16, 30), (4097, 16, 45),
+                                   (90_001, 16, 200), (60_000, 16, 300), (300_000, 16, 250),
+                                   (70_000, 40, 187), (120_500, 40, 240), (13_000, 40, 80)]):
+        X, _, _ = mixture_numpy(n, d, k, seed=50 + i, mean_lo=-10 if i % 2 else -2,
+                                mean_hi=10 if i % 2 else 2)
+        X[: n // 50] = X[0]
+        init = X[sample_init(n, k, seed=i)].copy()
+        probs.append((X, k, init))
+    res, st = km.lloyd_batched(probs, max_iters=9, criterion=criterion, empty_policy=policy,
+                               assign_tier=tier)
+    for (X, k, init), r in zip(probs, res):
+        check(r, orc.lloyd(X, init, 9, criterion=criterion, empty_policy=policy))
+    assert st.reserved[7] & 0xFFFFFF == 0
