@@ -31,6 +31,7 @@
 // other points go to the exact re-rank list, so labels equal the FP64 arg-min.
 // Every mbarrier wait is bounded (error word + CTA abort flag); TMEM is freed on every path.
 #include <cfloat>
+#include <mutex>
 #include <utility>
 
 #include "common.cuh"
@@ -879,6 +880,8 @@ int g_num_sms = 0;
 
 template <int EPQ, bool F8, bool BIAS, bool XMAX = false>
 cudaError_t prepare_variant(VariantInfo& vi) {
+  static std::mutex mu;  // several threads may launch their first scan together
+  std::lock_guard<std::mutex> lock(mu);
   if (vi.ready) return cudaSuccess;
   int dev = 0, optin = 0;
   KMGB_CUDA_TRY(cudaGetDevice(&dev));

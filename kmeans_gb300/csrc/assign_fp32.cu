@@ -15,6 +15,7 @@
 //   * a point is certified when second - best > 2E, E the rigorous rounding bound of the
 //     FP32 evaluation; other points are appended to a re-rank list that the exact (FP64)
 //     re-rank resolves, so labels equal the FP64 arg-min.
+#include <atomic>
 #include <cfloat>
 
 #include "common.cuh"
@@ -467,8 +468,8 @@ cudaError_t launch_assign_fp32(const float* X, long long ldx, const float* Cop, 
                                   (uint64_t)a.n, (uint64_t)ldx * 4, BKF, BM));
   KMGB_CUDA_TRY(kmgb_make_tmap_2d(&tmC, Cop, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)a.d,
                                   (uint64_t)a.k, (uint64_t)ldc * 4, BKF, BN));
-  static bool attr_set = false;
-  if (!attr_set) {
+  static std::atomic<bool> attr_set{false};
+  if (!attr_set.load(std::memory_order_acquire)) {
     KMGB_CUDA_TRY(cudaFuncSetAttribute(assign_fp32_kernel<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)SMEM_BYTES));
@@ -478,7 +479,7 @@ cudaError_t launch_assign_fp32(const float* X, long long ldx, const float* Cop, 
     KMGB_CUDA_TRY(cudaFuncSetAttribute(assign_fp32_grouped_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)SMEM_BYTES));
-    attr_set = true;
+    attr_set.store(true, std::memory_order_release);
   }
   CUtensorMap tmXc = tmX;
   if (a.sel) {

@@ -395,7 +395,7 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   if (smem > 200 * 1024) return KMEANS_ERROR_CLOSEST_CENTERS;
   if (smem > 48 * 1024)
     KD_TRY(cudaFuncSetAttribute(assign_d_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem),
+                                200 * 1024),
            KMEANS_ERROR_CLOSEST_CENTERS);
   double sse_old = 0.0, rel = 1.0;
   int it = 0;

@@ -600,7 +600,8 @@ cudaError_t kmeanspp_impl(const T* X, long long ldx, long long n, int d, int k,
   int grid = 0;
   if (bulk) {
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kpp_update_bulk_kernel<T>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)KPP_SMEM_BUDGET));
     int per_sm = 0;
     KMGB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, kpp_update_bulk_kernel<T>, KPP_BULK_THREADS, smem));

@@ -667,7 +667,7 @@ kmeansCudaErrorStatus ClosestCentersD(const int m0, const int nRowsA, const int 
   if (smem > 200 * 1024) return ERROR_CLOSESTCENTERS;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(closest_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+                           200 * 1024) != cudaSuccess)
     return ERROR_CLOSESTCENTERS;
   return closest_centers<double>(m0, nRowsA, nColsA, A, nColsB, B, normColsOfB_squared,
                                  CindicesFinal)

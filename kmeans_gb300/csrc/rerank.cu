@@ -140,6 +140,9 @@ __global__ void rerank_kernel(RerankArgs a) {
 // sum_d (x_d - c_d)^2 with float4 loads. Per point (best, index, second) is merged over the 32
 // threads that share it (lowest index on ties) and certified with the relative bound of the
 // direct form; uncertified points go to list2 for the exact FP64 stage.
+// The dynamic shared memory that launches here may ask for. Always this limit is set, not a launch's
+// own size: another thread's smaller one could arrive between the call and the launch.
+constexpr int kMaxTileSmem = 200 * 1024;
 constexpr int TP = 32;   // points per CTA iteration
 constexpr int TC = 64;   // centers per block
 
@@ -1356,16 +1359,16 @@ static size_t tiled_smem(int d) {
   return sizeof(float4) * (size_t)(TP + TC) * ((dq + 1) | 1) + sizeof(float) * TC;
 }
 
-bool rerank_tiled_supported(int d) { return tiled_smem(d) <= 200 * 1024; }
+bool rerank_tiled_supported(int d) { return tiled_smem(d) <= (size_t)kMaxTileSmem; }
 
 cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
   auto kern = a.mode == 0 ? rerank_exact_kernel<0, false> : rerank_exact_kernel<1, false>;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
   count_launches(1);
   return cudaGetLastError();
@@ -1377,10 +1380,10 @@ cudaError_t launch_rerank_band(const RerankArgs& a, const float* hi2, int* cand,
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
-  if (smem > 200 * 1024 || a.mode != 0) return cudaErrorInvalidValue;
+  if (smem > (size_t)kMaxTileSmem || a.mode != 0) return cudaErrorInvalidValue;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<0, true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   rerank_exact_kernel<0, true><<<kmgb::num_sms() * 2, 256, smem, s>>>(
       a, hi2, cand, cand_cnt, cand_cap, over, over_count, over_hi);
   count_launches(1);
@@ -1392,10 +1395,10 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
   auto kern = a.mode == 0 ? rerank_tiled_kernel<0, false> : rerank_tiled_kernel<1, false>;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, list2, count2, hi2);
   count_launches(1);
   return cudaGetLastError();
@@ -1405,10 +1408,10 @@ cudaError_t launch_rerank_settle(const RerankArgs& a, cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
   auto kern = a.mode == 0 ? rerank_tiled_kernel<0, true> : rerank_tiled_kernel<1, true>;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, nullptr, nullptr, nullptr);
   count_launches(1);
   return cudaGetLastError();
@@ -1420,12 +1423,12 @@ cudaError_t launch_rerank_grouped(const RerankArgs& a, const GroupArgs& g, cudaS
   if (a.ldc % 4 || (reinterpret_cast<uintptr_t>(a.C) & 15)) return cudaErrorInvalidValue;
   const size_t ds = ((size_t)a.d + 3) / 4 * 4;
   const size_t smem = sizeof(float) * (size_t)RG_WARPS * (RG_VCAP + ds);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
   auto kern = a.d <= 16 ? rerank_grouped_kernel<4>
                         : (a.d <= 32 ? rerank_grouped_kernel<8>
                                      : (a.d <= 64 ? rerank_grouped_kernel<16> : rerank_grouped_kernel<32>));
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   kern<<<kmgb::num_sms() * 4, RG_WARPS * 32, smem, s>>>(a, g, cand, cand_cnt, cand_cap);
   count_launches(1);
   return cudaGetLastError();
@@ -1435,10 +1438,10 @@ cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t s) {
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const int threads = 256;
   const size_t smem = sizeof(float) * (size_t)a.d * (threads / 32);
-  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
   if (smem > 48 * 1024) {
     KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+                                       kMaxTileSmem));
   }
   // Persistent grid: the flagged count lives on the device, so no host round trip is needed.
   rerank_kernel<<<kmgb::num_sms() * 4, threads, smem, s>>>(a); kmgb::count_launches(1);

@@ -1061,12 +1061,9 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, w.label_off, w.piece_cnt, w.counts, w.dirty,
         w.tickets, w.any_dirty, w.stop);
   } else if (smem <= 96 * 1024) {
-    static int hist_attr_k = -1;
-    if (smem > 48 * 1024 && hist_attr_k < k) {
+    if (smem > 48 * 1024)
       KMGB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<true, false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-      hist_attr_k = k;
-    }
     hist_kernel<true, false><<<w.ntiles, 256, smem, s>>>(
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, nullptr, nullptr, nullptr, nullptr, nullptr,
         w.any_dirty, w.stop);
@@ -1087,22 +1084,16 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
   }
   const size_t msmem = sizeof(int) * (size_t)k * kScatterWarps;
   if (msmem <= 96 * 1024) {
-    static int multi_attr_k = -1;
-    if (msmem > 48 * 1024 && multi_attr_k < k) {
+    if (msmem > 48 * 1024)
       KMGB_CUDA_TRY(cudaFuncSetAttribute(scatter_multi_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-      multi_attr_k = k;
-    }
     scatter_multi_kernel<<<w.ntiles, 32 * kScatterWarps, msmem, s>>>(
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.sorted, w.dirty, w.any_dirty, w.stop);
     kmgb::count_launches(1);
   } else if (smem <= 96 * 1024) {
-    static int attr_k = -1;
-    if (smem > 48 * 1024 && attr_k < k) {
+    if (smem > 48 * 1024)
       KMGB_CUDA_TRY(cudaFuncSetAttribute(scatter_kernel<true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-      attr_k = k;
-    }
     scatter_kernel<true><<<w.ntiles, 32, smem, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist,
                                                     w.sorted, w.dirty, w.any_dirty, w.stop); kmgb::count_launches(1);
   } else {
