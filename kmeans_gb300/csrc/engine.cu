@@ -40,6 +40,8 @@ long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 namespace {
 
+__global__ void set_int_kernel(int* p, int v) { *p = v; }
+
 thread_local std::string g_last_error;
 
 void set_err(const char* where, cudaError_t e) {
@@ -178,6 +180,7 @@ struct kmgb_handle {
   bool have_data = false;
   // mini-batch windows
   int* perm = nullptr;
+  int* win_base = nullptr;  // window index of the run's first iteration
   float* Xw = nullptr;
   void* Xbw = nullptr;
   void* Xlw = nullptr;
@@ -263,6 +266,9 @@ struct kmgb_handle {
   // one iteration captured as a CUDA graph (resident data, full batches, profiling off),
   // replayed for every iteration while the buffers it was captured with are in place
   cudaGraphExec_t gexec = nullptr;
+  bool fork = false;  // capturing: the audit goes to aux_stream
+  cudaStream_t aux_stream = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   const double* g_sse = nullptr;
   long long g_launches = 0;
   // phase profiling: 5 events per iteration
@@ -302,6 +308,9 @@ struct kmgb_handle {
       if (ev_free[b]) cudaEventDestroy(ev_free[b]);
     }
     if (copy_stream) cudaStreamDestroy(copy_stream);
+    if (aux_stream) cudaStreamDestroy(aux_stream);
+    if (ev_fork) cudaEventDestroy(ev_fork);
+    if (ev_join) cudaEventDestroy(ev_join);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (stream) cudaStreamDestroy(stream);
@@ -504,6 +513,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     }
     if (h->mini) {
       a.take(&h->perm, n);
+      a.take(&h->win_base, 1);
       a.take(&h->Xw, (size_t)h->m_mb * h->ldx);
       a.take(&h->qnw, h->m_mb);
       a.take(&h->xnw, h->m_mb);
@@ -1014,17 +1024,11 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   const double* qna = h->qn;
   const float* xna = h->xn;
   if (h->mini) {
-    const long long st = window_start(h->n, h->m_mb, h->run_base + slot);
-    KM_TRY(launch_gather_rows(h->X, h->ldx, h->perm, h->n, st, h->m_mb, h->d, h->Xw, h->ldx, s,
-                              h->stop),
+    RowWindow rw{h->perm, h->n, h->win_base, h->iters_done, h->Xw, h->ldx};
+    KM_TRY(launch_prep_window(h->X, h->ldx, h->m_mb, h->d, h->qnw, h->xnw, h->Xbw,
+                              h->x_exact ? nullptr : h->Xlw, h->ldb, rw,
+                              s, h->stop),
            KMEANS_ERROR_CONSTRUCT_MINIBATCH);
-    KM_TRY(launch_gather_vec(h->qn, h->xn, h->perm, h->n, st, h->m_mb, h->qnw, h->xnw, s,
-                             h->stop),
-           KMEANS_ERROR_CONSTRUCT_MINIBATCH);
-    if (h->Xbw)
-      KM_TRY(launch_prep_rows(h->Xw, h->ldx, h->m_mb, h->d, nullptr, nullptr, h->Xbw, h->Xlw,
-                              h->ldb, nullptr, s, h->stop),
-             KMEANS_ERROR_CONSTRUCT_MINIBATCH);
     Xa = h->Xw;
     Xba = h->Xbw;
     Xla = h->x_exact ? nullptr : h->Xlw;
@@ -1138,15 +1142,29 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   }
   // the audit reads the centers as they are (an empty cluster's NaN center has a NaN distance and
   // never counts as nearer), not the operand copy whose unusable rows are zero
-  if (h->audit_rows > 0)
+  UpdateWork uw = h->uw;
+  if (h->audit_rows > 0) {
+    // In a captured iteration the audit is a branch of its own: it reads the labels and the centers,
+    // so only the kernel that writes the new centers waits for it, and its chain of L2 round trips
+    // (11-14 us) runs beside the sort and the sums.
+    cudaStream_t as = s;
+    if (h->fork) {
+      as = h->aux_stream;
+      KM_TRY(cudaEventRecord(h->ev_fork, s), KMEANS_ERROR_CLOSEST_CENTERS);
+      KM_TRY(cudaStreamWaitEvent(as, h->ev_fork, 0), KMEANS_ERROR_CLOSEST_CENTERS);
+    }
     KM_TRY(launch_audit_labels(Xa, h->ldx, na, h->d, h->C, h->ldx, h->k, h->labels, h->audit,
-                               h->audit_rows, h->stop, s),
+                               h->audit_rows, h->stop, as),
            KMEANS_ERROR_CLOSEST_CENTERS);
+    if (h->fork) {
+      KM_TRY(cudaEventRecord(h->ev_join, as), KMEANS_ERROR_CLOSEST_CENTERS);
+      uw.centers_free = h->ev_join;
+    }
+  }
   KM_TRY(h->pmark(3), KMEANS_ERROR_CLOSEST_CENTERS);
   if (assign_only) return 0;
   // cluster centers + compactness (kmeans.cpp:1018-1104)
   // the SSE lands in sse_dev[iteration of the run] (device-side index)
-  UpdateWork uw = h->uw;
   if (prune) {
     KM_TRY(launch_prune_dirty(h->pr, h->labels, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
     uw.dirty = h->pr.dirty;
@@ -1290,22 +1308,30 @@ int step_stream(kmgb_handle* h, int slot) {
 }
 
 // Enqueues `iters` iterations as launches of one captured CUDA graph holding a whole iteration
-// (resident data, full batches): every iteration issues the same kernels with the same
-// parameters -- the SSE slot and the stop rule are indexed on the device -- so the graph is
-// captured once and replayed until a buffer it uses is replaced. Returns 0 when launched, -1 when
-// the iteration cannot be captured (it is then launched kernel by kernel), else an error code.
+// (resident data): every iteration issues the same kernels with the same parameters -- the SSE slot, the
+// stop rule and a mini-batch window are indexed on the device -- so the graph is captured once and
+// replayed until a buffer it uses is replaced. Returns 0 when launched, -1 when the iteration cannot be
+// captured (it is then launched kernel by kernel), else an error code.
 int run_graph(kmgb_handle* h, int iters) {
   if (!(h->gexec && h->g_sse == h->sse_dev)) {
     if (h->gexec) {
       cudaGraphExecDestroy(h->gexec);
       h->gexec = nullptr;
     }
+    bool forks = h->audit_rows > 0;  // (without its stream and events the audit stays in line)
+    if (forks && !h->ev_join)
+      forks = cudaStreamCreateWithFlags(&h->aux_stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
+              cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) == cudaSuccess;
+    if (!forks) cudaGetLastError();
     if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       return -1;
     }
     const long long l0 = launch_count();
+    h->fork = forks;
     const int rc = step(h, 0);
+    h->fork = false;
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     const long long captured = launch_count() - l0;
@@ -1363,6 +1389,11 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
   KM_TRY(cudaMemcpyAsync(h->loopf, kLoopInit, 2 * sizeof(double), cudaMemcpyHostToDevice,
                          h->stream),
          KMEANS_ERROR_COMPUTE);
+  if (h->mini) {
+    set_int_kernel<<<1, 1, 0, h->stream>>>(h->win_base, h->run_base);
+    count_launches(1);
+    KM_TRY(cudaGetLastError(), KMEANS_ERROR_CONSTRUCT_MINIBATCH);
+  }
   if (h->pr.n > 0)  // no bounds yet: the first iteration scans every row
     KM_TRY(cudaMemsetAsync(h->pr.flags, 0, 8 * sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
   KM_TRY(cudaEventRecord(h->ev0, h->stream), KMEANS_ERROR_COMPUTE);
@@ -1383,7 +1414,7 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
   // Every iteration is enqueued; the SSE reduction evaluates the stop rule on the device and
   // the kernels of later iterations return at once after it fires.
   int graph_rc = -1;
-  if (!h->streaming && !h->mini && !h->prof && !h->opt.router && iters - first > 0 &&
+  if (!h->streaming && !h->prof && !h->opt.router && iters - first > 0 &&
       graphs_enabled()) {
     graph_rc = run_graph(h, iters - first);
     if (graph_rc > 0) return graph_rc;

@@ -320,6 +320,20 @@ struct RowList {
   int* over;
   int* over_count;
 };
+// A mini-batch window (kmeans.cpp:426-447, 746-780): rows perm[(start + r) mod m], r < n, into X_out
+// (row stride ld_out, zero padded) as well; start = ((*base + *done) n) mod m, the iteration read on
+// the device so that one captured iteration serves every window.
+struct RowWindow {
+  const int* perm;
+  long long m;
+  const int* base;
+  const int* done;
+  float* X_out;
+  long long ld_out;
+};
+cudaError_t launch_prep_window(const float* X, long long ldx, long long n, int d, double* qn, float* xn,
+                               void* Xb, void* Xl, long long ldb, const RowWindow& rw, cudaStream_t s,
+                               const int* stop);
 template <typename T>
 cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
                              void* Xb, void* Xl, long long ldb, int* inexact, cudaStream_t s,
@@ -352,6 +366,7 @@ struct UpdateWork {
                         // [k] per center
   long long* counts;    // [k]
   int* err;
+  cudaEvent_t centers_free;  // nullable: launch_update waits for it before it writes the centers
   int* tickets;         // [1] zero between launches (last_block)
   const int* any_dirty; // nullable: zero when no center's members changed
   const int* dirty;     // nullable: [k] zero where the center has the members of the previous
@@ -421,14 +436,6 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
                                   const int* labels, float* C, long long ldc, int empty_policy,
                                   const UpdateWork& w, const BatchUpdate& b,
                                   cudaStream_t s);  // (w.dirty as in launch_update)
-
-// Mini-batch gather: rows perm[(start + r) mod m] of Xsrc into Xdst (m_mb rows).
-cudaError_t launch_gather_rows(const float* Xsrc, long long ldx, const int* perm, long long m,
-                               long long start, long long m_mb, int d, float* Xdst,
-                               long long ldd, cudaStream_t s, const int* stop = nullptr);
-cudaError_t launch_gather_vec(const double* qsrc, const float* xsrc, const int* perm,
-                              long long m, long long start, long long m_mb, double* qdst,
-                              float* xdst, cudaStream_t s, const int* stop = nullptr);
 
 // k-means++ (D^2-weighted draws, seeded): k centers from X (n x d, row stride ldx) into C (k x d,
 // row stride ldc); picks[k] receives the chosen rows. Work space: d2[kmeanspp_d2_elems(n)],

@@ -173,13 +173,14 @@ __device__ __forceinline__ float4 widen4(uint2 b) {
 
 //
 // IDX 1: the rows of a device list (RowList): output row i is row list[i]; entries past the capacity
-// go to over.
+// go to over. IDX 2: a mini-batch window (RowWindow), whose rows are copied on the way (gathering the
+// rows, their norms and their planes were three launches: 32 + 6 + 19 us for 89,879 x 128).
 template <typename T, int L, int IDX>
 __global__ void __launch_bounds__(256)
 prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, bool vec,
                  double* __restrict__ qn, float* __restrict__ xn, uint2* __restrict__ Xb,
                  uint2* __restrict__ Xl, int ldb, int* inexact, float* __restrict__ nf, RowList rl,
-                 const int* stop) {
+                 RowWindow rw, const int* stop) {
   if (stopped(stop)) return;
   if (IDX == 1) {
     const long long total = *reinterpret_cast<volatile const int*>(rl.count);
@@ -194,14 +195,24 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
       rl.thr_out[i] = fl > -3.0e38f ? fl : INFINITY;
     }
   }
-  auto source = [&](long long r) { return IDX == 1 ? (long long)__ldg(rl.list + r) : r; };
+  long long start = 0;
+  if (IDX == 2) start = (((long long)*rw.base + *rw.done) * n) % rw.m;
+  auto source = [&](long long r) -> long long {
+    if (IDX == 1) return __ldg(rl.list + r);
+    if (IDX == 2) {
+      const long long pos = start + r;
+      return __ldg(rw.perm + (pos >= rw.m ? pos - rw.m : pos));
+    }
+    return r;
+  };
   constexpr int G = 32 / L;  // rows per warp and step
   constexpr int U = 2;       // steps in flight
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
   const int ldb4 = ldb / 4;
-  const int width = Xb ? ldb : d;  // planes are written with their zero padding
+  int width = Xb ? ldb : d;  // planes are written with their zero padding
+  if (IDX == 2 && rw.ld_out > width) width = (int)rw.ld_out;
   const bool norms = qn || xn || nf;
   bool off = false;
   for (long long r0 = w0 * G * U; r0 < n; r0 += nw * G * U) {
@@ -224,7 +235,9 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
           ff_square_add(v[u].z, hi[u], lo[u]);
           ff_square_add(v[u].w, hi[u], lo[u]);
         }
-        if (Xb && r < n) {
+        if (IDX == 2 && r < n && c < rw.ld_out)
+          *reinterpret_cast<float4*>(rw.X_out + (size_t)r * rw.ld_out + c) = v[u];
+        if (Xb && r < n && c < ldb) {
           const uint2 h = bf16x4(v[u]);
           Xb[(size_t)r * ldb4 + c / 4] = h;
           if (Xl || inexact) {
@@ -332,36 +345,6 @@ __global__ void prep_expansion_kernel(const T* __restrict__ B, int d, int k, con
   if (cbias) write_bias_row(cbias + (size_t)j * kBiasCols, start, lane);
 }
 
-__global__ void gather_rows_kernel(const float* __restrict__ Xs, long long ldx,
-                                   const int* __restrict__ perm, long long m, long long start,
-                                   long long m_mb, int d, float* __restrict__ Xd, long long ldd,
-                                   const int* stop) {
-  if (stopped(stop)) return;
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= m_mb) return;
-  long long pos = start + warp;
-  if (pos >= m) pos -= m;
-  const float* src = Xs + (size_t)perm[pos] * ldx;
-  float* dst = Xd + (size_t)warp * ldd;
-  for (int t = lane; t < (int)ldd; t += 32) dst[t] = t < d ? src[t] : 0.0f;
-}
-
-__global__ void gather_vec_kernel(const double* __restrict__ qs, const float* __restrict__ xs,
-                                  const int* __restrict__ perm, long long m, long long start,
-                                  long long m_mb, double* __restrict__ qd, float* __restrict__ xd,
-                                  const int* stop) {
-  if (stopped(stop)) return;
-  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < m_mb;
-       r += (long long)gridDim.x * blockDim.x) {
-    long long pos = start + r;
-    if (pos >= m) pos -= m;
-    const int src = perm[pos];
-    qd[r] = qs[src];
-    xd[r] = xs[src];
-  }
-}
-
 // FP8 E4M3 operands with power-of-two scales: x = s * x8 + error, s = 2^(e - 8) where the scaled
 // quantity (a row's largest |x_i|, or for the centers the largest ||c||) is below 2^e, so every
 // scaled value is below 2^8 = 256 < 448 (the largest E4M3 number: no saturation) and the division
@@ -462,7 +445,8 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
 template <typename T>
 static cudaError_t prep_rows(const T* X, long long ldx, long long n, int d, double* qn, float* xn,
                              void* Xb, void* Xl, long long ldb, int* inexact, float* nf,
-                             cudaStream_t s, const int* stop, const RowList* rl) {
+                             cudaStream_t s, const int* stop, const RowList* rl,
+                             const RowWindow* rw = nullptr) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (n <= 0) return cudaSuccess;
   if (Xb && (ldb % 8 || ldb < d)) return cudaErrorInvalidValue;
@@ -476,10 +460,13 @@ static cudaError_t prep_rows(const T* X, long long ldx, long long n, int d, doub
   auto go = [&](auto tag) {
     if (rl)
       prep_rows_kernel<T, decltype(tag)::value, 1><<<blocks, 256, 0, s>>>(
-          X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nullptr, *rl, stop);
+          X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nullptr, *rl, RowWindow{}, stop);
+    else if (rw)
+      prep_rows_kernel<T, decltype(tag)::value, 2><<<blocks, 256, 0, s>>>(
+          X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nullptr, RowList{}, *rw, stop);
     else
       prep_rows_kernel<T, decltype(tag)::value, 0><<<blocks, 256, 0, s>>>(
-          X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nf, RowList{}, stop);
+          X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nf, RowList{}, RowWindow{}, stop);
   };
   if (lanes == 4) go(std::integral_constant<int, 4>{});
   else if (lanes == 8) go(std::integral_constant<int, 8>{});
@@ -493,6 +480,14 @@ cudaError_t launch_prep_rows(const T* X, long long ldx, long long n, int d, doub
                              void* Xb, void* Xl, long long ldb, int* inexact, cudaStream_t s,
                              const int* stop, const RowList* rl) {
   return prep_rows<T>(X, ldx, n, d, qn, xn, Xb, Xl, ldb, inexact, nullptr, s, stop, rl);
+}
+
+cudaError_t launch_prep_window(const float* X, long long ldx, long long n, int d, double* qn, float* xn,
+                               void* Xb, void* Xl, long long ldb, const RowWindow& rw, cudaStream_t s,
+                               const int* stop) {
+  if (rw.ld_out % 4 || rw.ld_out < d || (reinterpret_cast<uintptr_t>(rw.X_out) & 15) || n > rw.m)
+    return cudaErrorInvalidValue;
+  return prep_rows<float>(X, ldx, n, d, qn, xn, Xb, Xl, ldb, nullptr, nullptr, s, stop, nullptr, &rw);
 }
 
 cudaError_t launch_row_norms(const float* X, long long ldx, long long n, int d, float* out,
@@ -525,24 +520,5 @@ template cudaError_t launch_prep_expansion<float>(const float*, int, int, const 
 template cudaError_t launch_prep_expansion<double>(const double*, int, int, const double*, float*,
                                                    long long, float*, void*, void*, long long, float*,
                                                    void*, float*, cudaStream_t);
-
-cudaError_t launch_gather_rows(const float* Xsrc, long long ldx, const int* perm, long long m,
-                               long long start, long long m_mb, int d, float* Xdst, long long ldd,
-                               cudaStream_t s, const int* stop) {
-  if (m_mb <= 0) return cudaSuccess;
-  const int threads = 256;
-  const long long blocks = (m_mb * 32 + threads - 1) / threads;
-  gather_rows_kernel<<<(unsigned)blocks, threads, 0, s>>>(Xsrc, ldx, perm, m, start, m_mb, d,
-                                                          Xdst, ldd, stop); kmgb::count_launches(1);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gather_vec(const double* qsrc, const float* xsrc, const int* perm, long long m,
-                              long long start, long long m_mb, double* qdst, float* xdst,
-                              cudaStream_t s, const int* stop) {
-  if (m_mb <= 0) return cudaSuccess;
-  gather_vec_kernel<<<kmgb::num_sms() * 4, 256, 0, s>>>(qsrc, xsrc, perm, m, start, m_mb, qdst, xdst, stop); kmgb::count_launches(1);
-  return cudaGetLastError();
-}
 
 }  // namespace kmgb

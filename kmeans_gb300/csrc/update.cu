@@ -205,7 +205,7 @@ label_offsets_kernel(const int* __restrict__ hist, long long n, int k, int ntile
 // ints) and writes every count; otherwise global atomics per warp group (hist cleared before).
 // SMALL (SCAN_T threads): the last block scans the counters and derives the labels' offsets, where
 // they are few enough for one block (kSmallHist): one launch instead of three.
-constexpr long long kSmallHist = 4 * SCAN_SEG;
+constexpr long long kSmallHist = 2 * SCAN_SEG;
 
 template <bool SMEM, bool SMALL>
 __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, int tile_pts,
@@ -328,9 +328,15 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
   int* mine = wcnt + (size_t)w * k;
   for (int j = threadIdx.x; j < kScatterWarps * k; j += blockDim.x) wcnt[j] = 0;
   __syncthreads();
-  for (long long i = s0 + lane; i < s1; i += 32) {
-    const int l = __ldg(labels + i);
-    if (l >= 0 && l < k) atomicAdd(&mine[l], 1);
+  // labels loaded ahead: one memory round trip per U steps of 32 rows, in both passes
+  constexpr int U = 8;
+  for (long long b = s0; b < s1; b += 32 * U) {
+    int lv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) lv[u] = b + 32 * u + lane < s1 ? __ldg(labels + b + 32 * u + lane) : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (lv[u] >= 0 && lv[u] < k) atomicAdd(&mine[lv[u]], 1);
   }
   __syncthreads();
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
@@ -343,20 +349,30 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
   }
   __syncthreads();
   const int nbits = label_bits(k);
-  for (long long b = s0; b < s1; b += 32) {
-    const long long i = b + lane;
-    int l = i < s1 ? __ldg(labels + i) : -1;
-    if (l < 0 || l >= k || (dirty && !__ldg(dirty + l))) l = -1;
-    if (!__any_sync(0xffffffffu, l >= 0)) continue;
-    const unsigned peers = warp_peers(l, nbits);
-    const int leader = __ffs(peers) - 1;
-    const int rank = __popc(peers & lanemask_lt());
-    int base = 0;
-    if (l >= 0 && lane == leader) base = mine[l];
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (l >= 0) sorted[base + rank] = (int)i;
-    if (l >= 0 && lane == leader) mine[l] = base + __popc(peers);
-    __syncwarp();
+  for (long long b0 = s0; b0 < s1; b0 += 32 * U) {
+    int lv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) lv[u] = b0 + 32 * u + lane < s1 ? __ldg(labels + b0 + 32 * u + lane) : -1;
+    if (dirty) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (lv[u] >= 0 && lv[u] < k && !__ldg(dirty + lv[u])) lv[u] = -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = b0 + 32 * u + lane;
+      const int l = lv[u] >= 0 && lv[u] < k ? lv[u] : -1;
+      if (!__any_sync(0xffffffffu, l >= 0)) continue;
+      const unsigned peers = warp_peers(l, nbits);
+      const int leader = __ffs(peers) - 1;
+      const int rank = __popc(peers & lanemask_lt());
+      int base = 0;
+      if (l >= 0 && lane == leader) base = mine[l];
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (l >= 0) sorted[base + rank] = (int)i;
+      if (l >= 0 && lane == leader) mine[l] = base + __popc(peers);
+      __syncwarp();
+    }
   }
 }
 
@@ -375,6 +391,27 @@ struct PieceAcc {
   }
   __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
+
+// The label of piece p: the last j with pstart[j] <= p (pstart non-decreasing, pstart[0] = 0). The L
+// lanes of a group look together, L places at a time (two or three round trips to L2 where a binary
+// search takes eight to sixteen); every lane of the warp calls it, p the same within a group.
+template <int L>
+__device__ __forceinline__ int find_label_group(const int* __restrict__ pstart, int k, int p) {
+  const int lane = threadIdx.x & 31, sub = lane % L, shift = lane - sub;
+  int lo = 0, n = k;  // the answer lies in [lo, lo + n)
+  while (__any_sync(0xffffffffu, n > 1)) {
+    const int step = (n + L - 1) / L;
+    const int at = lo + sub * step;
+    const bool in = n > 1 && sub * step < n && __ldg(pstart + at) <= p;
+    const unsigned bal = (__ballot_sync(0xffffffffu, in) >> shift) & (L == 32 ? 0xffffffffu : (1u << L) - 1u);
+    if (n > 1) {
+      const int hit = 31 - __clz(bal | 1u);  // place 0 always holds
+      n = min(step, n - hit * step);
+      lo += hit * step;
+    }
+  }
+  return lo;
+}
 
 __device__ __forceinline__ int find_label(const int* __restrict__ pstart, int k, int p) {
   int lo = 0, hi = k - 1;
@@ -476,7 +513,7 @@ __device__ __forceinline__ void ring_start_piece(RingCursor& q, long long ptot,
   q.d0 = 0;
   q.qs = 0.0;
   if (q.p >= ptot) return;
-  const int j = find_label(pstart, k, (int)q.p);
+  const int j = find_label_group<32>(pstart, k, (int)q.p);
   q.b = label_off[j] + ((int)q.p - pstart[j]) * kSumPiece;
   q.e = min(q.b + kSumPiece, label_off[j + 1]);
   q.t = q.b;
@@ -606,18 +643,18 @@ piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double*
 // float-float sum is the same sequence of additions as in the one-piece-per-warp kernel; the piece's
 // sum of ||x||^2 is that kernel's 32-row tree: row i L + sub of a 32-row window is in register i of lane
 // sub, so the tree's upper levels join registers and its lower ones lanes. Bound by latency where
-// pieces are few: the window's ids and norms are loaded together, the next window's ids ahead, and
-// 16 rows are in flight per lane group (6,000 x 32, K=16: 43 us with an id round trip before every 8
-// rows and the norms piece after piece).
+// pieces are few (a round trip to L2 costs some 900 cycles): the window's norms and the next window's
+// ids are loaded with its rows, and 16 rows are in flight while 16 are summed (6,000 x 32, K=16: an id
+// round trip before every 8 rows, the norms piece after piece).
 template <int L>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double* __restrict__ qn,
                         const int* __restrict__ sorted, const int* __restrict__ label_off,
                         const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
                         double* __restrict__ partq, const int* any_dirty, const int* stop) {
   if (stopped(stop) || idle(any_dirty)) return;
   constexpr int G = 32 / L;  // pieces per warp; also ids per lane and window
-  constexpr int R = 16;      // rows in flight
+  constexpr int R = 16;      // rows per batch: one is summed while the next is in flight
   const int ptot = pstart[k];
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -626,48 +663,53 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
   for (long long p0 = gw * G; p0 < ptot; p0 += nw * G) {
     const long long p = p0 + grp;
     const bool live = p < ptot;
-    int b = 0, n = 0;
-    if (live) {
-      const int j = find_label(pstart, k, (int)p);
-      b = label_off[j] + ((int)p - pstart[j]) * kSumPiece;
-      n = min(kSumPiece, label_off[j + 1] - b);
-    }
+    const int j = find_label_group<L>(pstart, k, live ? (int)p : 0);
+    const int b = live ? __ldg(label_off + j) + ((int)p - __ldg(pstart + j)) * kSumPiece : 0;
+    const int n = live ? min(kSumPiece, __ldg(label_off + j + 1) - b) : 0;
     const bool on = live && c < d;
-    PieceAcc a0, a1, a2, a3;
-    double qs = 0.0;
-    int id[G];
+    const float* xc = X + c;
+    auto load_ids = [&](int t, int (&id)[G]) {
 #pragma unroll
-    for (int i = 0; i < G; ++i) id[i] = i * L + sub < n ? __ldg(sorted + b + i * L + sub) : -1;
+      for (int i = 0; i < G; ++i)
+        id[i] = t + i * L + sub < n ? __ldg(sorted + b + t + i * L + sub) : -1;
+    };
+    // rows h .. h + R - 1 of the window whose ids are id (zeros past the piece: adding them changes
+    // no float-float sum)
+    auto load_rows = [&](const int (&id)[G], int h, float4 (&v)[R]) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int row = __shfl_sync(0xffffffffu, id[(h + r) / L], grp * L + (h + r) % L);
+        v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (on && row >= 0) v[r] = __ldg(reinterpret_cast<const float4*>(xc + (size_t)row * ldx));
+      }
+    };
+    PieceAcc a0, a1, a2, a3;
+    auto add_rows = [&](const float4 (&v)[R]) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        a0.add(v[r].x);
+        a1.add(v[r].y);
+        a2.add(v[r].z);
+        a3.add(v[r].w);
+      }
+    };
+    double qs = 0.0;
+    int id[G], nx[G];
+    float4 va[R], vb[R];
+    load_ids(0, id);
+    load_rows(id, 0, va);
     // the groups' pieces end at different windows: the shuffles take whole warps
     for (int t = 0; __any_sync(0xffffffffu, t < n); t += 32) {
       double q[G];
+      load_ids(t + 32, nx);
+      load_rows(id, R, vb);
       if (qn) {
 #pragma unroll
         for (int i = 0; i < G; ++i) q[i] = id[i] >= 0 ? __ldg(qn + id[i]) : 0.0;
       }
-      int nx[G];
-#pragma unroll
-      for (int i = 0; i < G; ++i)
-        nx[i] = t + 32 + i * L + sub < n ? __ldg(sorted + b + t + 32 + i * L + sub) : -1;
-#pragma unroll
-      for (int h = 0; h < 32; h += R) {
-        float4 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int row = __shfl_sync(0xffffffffu, id[(h + r) / L], grp * L + (h + r) % L);
-          v[r] = (on && row >= 0) ? __ldg(reinterpret_cast<const float4*>(X + (size_t)row * ldx + c))
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (t + h + r < n) {
-            a0.add(v[r].x);
-            a1.add(v[r].y);
-            a2.add(v[r].z);
-            a3.add(v[r].w);
-          }
-        }
-      }
+      add_rows(va);
+      load_rows(nx, 0, va);
+      add_rows(vb);
       if (qn) {
 #pragma unroll
         for (int h = G / 2; h > 0; h >>= 1) {
@@ -705,14 +747,15 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
   long long warps = (max_pieces + 32 / lanes - 1) / (32 / lanes);
   if (warps > kmgb::num_sms() * 64LL) warps = kmgb::num_sms() * 64LL;
   const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
+  const unsigned sblocks = (unsigned)((warps * 32 + 127) / 128);
   if (vec && lanes == 4)
-    piece_sums_small_kernel<4><<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
+    piece_sums_small_kernel<4><<<sblocks, 128, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
                                                       part, partq, any, stop);
   else if (vec && lanes == 8)
-    piece_sums_small_kernel<8><<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
+    piece_sums_small_kernel<8><<<sblocks, 128, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
                                                       part, partq, any, stop);
   else if (vec && lanes == 16)
-    piece_sums_small_kernel<16><<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k,
+    piece_sums_small_kernel<16><<<sblocks, 128, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k,
                                                        d, part, partq, any, stop);
   else if (vec) {
     // four 4-warp blocks (48 KB of ring each) per SM
@@ -933,15 +976,13 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
       double sse = 0.0;
       if (c < d) {
         double s = 0.0;
-        int p = p0;
-        for (; p + 8 <= p1; p += 8) {  // eight loads in flight, additions in piece order
+        for (int p = p0; p < p1; p += 8) {  // eight loads in flight, additions in piece order
           double v[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = __ldg(w.part + (size_t)(p + i) * d + c);
+          for (int i = 0; i < 8; ++i) v[i] = p + i < p1 ? __ldg(w.part + (size_t)(p + i) * d + c) : 0.0;
 #pragma unroll
           for (int i = 0; i < 8; ++i) s += v[i];
         }
-        for (; p < p1; ++p) s += __ldg(w.part + (size_t)p * d + c);
         float mu;
         if (n > 0) {
           mu = __double2float_rn(__ddiv_rn(s, (double)n));
@@ -1113,6 +1154,7 @@ cudaError_t launch_update(const float* X, const double* qn, const int* labels, f
   KMGB_CUDA_TRY(launch_piece_sums_f32(X, w.ldx, qn, w.sorted, w.label_off, w.piece_cnt, k, w.d,
                                      w.part, w.partq, w.any_dirty, w.stop, w.max_pieces, s));
   const int warps = std::min(8, (w.d + 31) / 32);
+  if (w.centers_free) KMGB_CUDA_TRY(cudaStreamWaitEvent(s, w.centers_free, 0));
   finalize_update_kernel<<<(unsigned)k, 32 * warps, 0, s>>>(X, C, ldc, empty_policy, w, sse_out);
   kmgb::count_launches(1);
   return cudaGetLastError();

@@ -472,3 +472,22 @@ def test_compute_kmeans_d_fp64_near_ties(km, orc, torch_cuda):
     assert km.computeKmeansD(X, m, d, k, -1.0, 3, 1, 0, 0, 0, res, 1.0) == 13
     _, c, _, _, _ = orc.lloyd_d(X, X[rows], 3)
     assert np.array_equal(res.reshape(d, k), c.T, equal_nan=True)
+
+
+@pytest.mark.parametrize("m,d,frac", [(1000, 3, 0.02), (5001, 13, 0.37), (9000, 130, 0.999),
+                                      (30_011, 100, 0.21)])
+@pytest.mark.parametrize("tier", [0, 2])
+def test_minibatch_windows_resume(km, orc, torch_cuda, m, d, frac, tier):
+    """Windows of ragged widths, from a few rows to nearly all, that wrap around and go on where
+    the last run of the handle ended."""
+    k = 5
+    X, _, _ = mixture_numpy(m, d, 6, seed=d)
+    init = X[sample_init(m, k, seed=9)]
+    h = km.Handle(m, d, k, max_iters=8, mini_batch_fraction=frac, assign_tier=tier)
+    h.set_data(X, False)
+    h.set_centers(init, False)
+    for iters in (3, 1, 4):  # the windows go on from where a finished run ended
+        h.run(iters)
+        h.synchronize()
+    ref = orc.lloyd(X, init, 8, mb_fraction=frac)
+    assert np.array_equal(h.centers(), ref[1], equal_nan=True)
