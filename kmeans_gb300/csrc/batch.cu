@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <limits>
 #include <map>
 #include <string>
@@ -701,11 +702,11 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
   const char* gv = std::getenv("KMGB_GRAPHS");
   if (max_iters > 0 && !(gv && std::strcmp(gv, "0") == 0) &&
       cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-    const long long l0 = launch_count();
+    const long long l0 = thread_launch_count();
     const bool ok = issue(false);
     cudaGraph_t graph = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(s, &graph);
-    g_launches = launch_count() - l0;
+    g_launches = thread_launch_count() - l0;
     count_launches(-g_launches);  // recorded into the graph, not launched
     if (ok && ec == cudaSuccess && graph &&
         cudaGraphInstantiate(&gexec, graph, 0) == cudaSuccess) {
@@ -894,8 +895,13 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
       return;
     kmgb_options og = o;
     og.assign_tier = g.tier;
-    run_group(problems, g.ids, g.d, og, s, &g.reranked, &g.loop_ms, g.phase_ms, g.f, &g.graph_launches,
-              g.audit);
+    try {
+      run_group(problems, g.ids, g.d, og, s, &g.reranked, &g.loop_ms, g.phase_ms, g.f, &g.graph_launches,
+                g.audit);
+    } catch (const std::exception&) {  // host memory or threads: an exception must not leave a thread
+      g.f.code = KMEANS_ERROR_BUILDDATA;
+      g.f.msg = "kmgb_lloyd_batched_f32: out of host memory or threads";
+    }
     cudaStreamSynchronize(s);
     cudaStreamDestroy(s);
   };

@@ -156,6 +156,7 @@ cudaError_t kmgb_make_tmap_2d_swz(CUtensorMap* map, const void* base, CUtensorMa
 namespace kmgb {
 void count_launches(long long n);
 long long launch_count();
+long long thread_launch_count();  // of the calling thread: what its captured graph holds
 }  // namespace kmgb
 
 #define KMGB_CUDA_TRY(expr)                        \

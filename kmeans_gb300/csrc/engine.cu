@@ -33,7 +33,12 @@ using namespace kmgb;
 
 namespace kmgb {
 static std::atomic<long long> g_launches{0};
-void count_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+static thread_local long long t_launches = 0;
+void count_launches(long long n) {
+  g_launches.fetch_add(n, std::memory_order_relaxed);
+  t_launches += n;
+}
+long long thread_launch_count() { return t_launches; }
 void set_last_error(const char* msg);
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 }  // namespace kmgb
@@ -1334,13 +1339,13 @@ int run_graph(kmgb_handle* h, int iters) {
       cudaGetLastError();
       return -1;
     }
-    const long long l0 = launch_count();
+    const long long l0 = thread_launch_count();
     h->fork = forks;
     const int rc = step(h, 0);
     h->fork = false;
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-    const long long captured = launch_count() - l0;
+    const long long captured = thread_launch_count() - l0;
     count_launches(-captured);  // recorded into the graph, not launched
     if (rc || e != cudaSuccess || !g) {
       if (g) cudaGraphDestroy(g);
