@@ -30,7 +30,25 @@ __device__ __forceinline__ void write_bias_row(__nv_bfloat16* row, float v, int 
     row[lane] = lane == 0 ? hi : (lane == 1 ? mid : (lane == 2 ? lo : __float2bfloat16_rn(0.0f)));
 }
 
-// One warp per center.
+__device__ __forceinline__ void ff_two_sum(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float bp = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
+}
+
+__device__ __forceinline__ void ff_square_add(float v, float& hi, float& lo) {
+  const float p = __fmul_rn(v, v);
+  const float e = __fmaf_rn(v, v, -p);  // v*v - p exactly
+  float s, err;
+  ff_two_sum(hi, p, s, err);
+  hi = s;
+  lo = __fadd_rn(lo, __fadd_rn(err, e));
+}
+
+// One warp per center, one pass over its old operand copy and its new values, four dimensions a lane in
+// flight. The norm is an error-free float-float sum on the FP32 pipe as a row's (prep_rows_kernel): an
+// FP64 chain per lane, its tree and two FP64 square roots in passes of their own took 36.5 us for
+// 16,384 x 256 (now 16.9) and 6.6 us for 256 x 128 (4.0).
 __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, int k, int d,
                                     float* __restrict__ Cop, __nv_bfloat16* __restrict__ Cb,
                                     long long ldcb, float* __restrict__ cn, float* cmax,
@@ -47,76 +65,97 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
     return;
   }
   const float* c = C + (size_t)warp * ldc;
-  double s = 0.0;
-  bool bad = false;
-  for (int t = lane; t < d; t += 32) {
-    const float v = c[t];
-    bad |= !isfinite(v);
-    s = fma((double)v, (double)v, s);
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  bad = __any_sync(0xffffffffu, bad);
   float* op = Cop + (size_t)warp * ldc;
-  if (shift) {
-    // the move since the previous centers: FP32 sum of squared differences, widened by more than
-    // its roundings; where squares leave the normal range, sqrt(d) times the largest difference
-    float m2 = 0.0f, mx = 0.0f;
-    for (int t = lane; t < d; t += 32) {
-      const float df = fabsf(c[t] - op[t]);
-      m2 = fmaf(df, df, m2);
-      mx = fmaxf(mx, df);
+  __nv_bfloat16* ob = Cb ? Cb + (size_t)warp * ldcb : nullptr;
+  __nv_bfloat16* ol = Cb && Cl ? Cl + (size_t)warp * ldcb : nullptr;
+  const int width = ob && ldcb > ldc ? (int)ldcb : (int)ldc;
+  float hi = 0.0f, lo = 0.0f;
+  float m2 = 0.0f, mx = 0.0f;  // the move since the previous centers
+  bool bad = false;
+  constexpr int U = 4;
+  for (int t0 = lane; t0 < width; t0 += 32 * U) {
+    float v[U], o[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + 32 * u;
+      v[u] = t < d ? c[t] : 0.0f;
+      o[u] = shift && t < d ? op[t] : 0.0f;
     }
-    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + 32 * u;
+      bad |= !isfinite(v[u]);
+      ff_square_add(v[u], hi, lo);
+      if (shift) {
+        const float df = fabsf(v[u] - o[u]);
+        m2 = fmaf(df, df, m2);
+        mx = fmaxf(mx, df);
+      }
+      if (t < (int)ldc) op[t] = v[u];
+      if (ob && t < (int)ldcb) {
+        const __nv_bfloat16 h = __float2bfloat16_rn(v[u]);
+        ob[t] = h;
+        if (ol) ol[t] = __float2bfloat16_rn(v[u] - __bfloat162float(h));
+      }
+    }
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  if (bad) {  // unusable: zero operands
+    for (int t = lane; t < width; t += 32) {
+      if (t < (int)ldc) op[t] = 0.0f;
+      if (ob && t < (int)ldcb) {
+        ob[t] = __float2bfloat16_rn(0.0f);
+        if (ol) ol[t] = __float2bfloat16_rn(0.0f);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
+    const float olo = __shfl_xor_sync(0xffffffffu, lo, o);
+    float s1, err;
+    ff_two_sum(hi, oh, s1, err);
+    hi = s1;
+    lo = __fadd_rn(lo, __fadd_rn(olo, err));
+    if (shift) {
       m2 += __shfl_xor_sync(0xffffffffu, m2, o);
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
-    if (lane == 0) {
-      const bool was_bad = !(cn[warp] < INFINITY);
-      const float slack = 1.0f + (float)(d + 16) * 2.4e-7f;
-      const float mv = (mx == 0.0f || (m2 > 1e-28f && m2 < 1e37f))
-                           ? __fsqrt_ru(__fmul_ru(m2, slack))
-                           : __fmul_ru(__fmul_ru(mx, 1.000001f), __fsqrt_ru((float)d));
-      // FP64 centers: each end of the move is a rounding away from its center
-      const float pt = shift_pert > 0.0f
-                           ? __fmul_ru(shift_pert, __fadd_ru(__double2float_ru(sqrt(s)), mv)) : 0.0f;
-      shift[warp] = bad && was_bad ? -1.0f : (bad || was_bad ? INFINITY : __fadd_ru(mv, pt));
-    }
-    __syncwarp();
   }
-  for (int t = lane; t < (int)ldc; t += 32) op[t] = (bad || t >= d) ? 0.0f : c[t];
-  if (Cb) {
-    __nv_bfloat16* ob = Cb + (size_t)warp * ldcb;
-    __nv_bfloat16* ol = Cl ? Cl + (size_t)warp * ldcb : nullptr;
-    for (int t = lane; t < (int)ldcb; t += 32) {
-      const float v = (bad || t >= d) ? 0.0f : c[t];
-      const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-      ob[t] = hi;
-      if (ol) ol[t] = __float2bfloat16_rn(v - __bfloat162float(hi));
-    }
+  // the squared norm, and an upper bound of the norm
+  float nn = __fadd_rn(hi, lo);
+  float nrm = __fsqrt_ru(__fmul_ru(__fadd_ru(hi, fabsf(lo)), 1.0f + 0x1p-22f));
+  if (!bad && !(hi < 1.0e37f && hi >= 1.0e-24f)) {  // squares out of FP32's normal range (uniform)
+    double s = 0.0;
+    for (int t = lane; t < d; t += 32) s = fma((double)c[t], (double)c[t], s);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    nn = __double2float_rn(s);
+    nrm = __double2float_ru(sqrt(s) * (1.0 + 1e-12));
   }
-  if (cbias)
-    write_bias_row(cbias + (size_t)warp * kBiasCols,
-                   bad ? -3.0e38f : -0.5f * __double2float_rn(s), lane);
-  if (lane == 0) {
-    if (bad) {
-      cn[warp] = INFINITY;
-      if (cxn) cxn[warp] = 0.0f;
-      if (cinit) cinit[warp] = -3.0e38f;
-    } else {
-      cn[warp] = __double2float_rn(s);
-      if (cinit) cinit[warp] = -0.5f * __double2float_rn(s);
-      // upper bound of ||c||: round the FP64 sqrt up and add a relative margin
-      const float nrm = __double2float_ru(sqrt(s) * (1.0 + 1e-12));
-      atomicMax(reinterpret_cast<int*>(cmax), __float_as_int(nrm));
-      if (cxn) cxn[warp] = nrm;
-    }
+  if (cbias) write_bias_row(cbias + (size_t)warp * kBiasCols, bad ? -3.0e38f : -0.5f * nn, lane);
+  if (lane != 0) return;
+  if (shift) {
+    // FP32 sum of squared differences, widened by more than its roundings; where squares leave the
+    // normal range, sqrt(d) times the largest difference
+    const bool was_bad = !(cn[warp] < INFINITY);
+    const float slack = 1.0f + (float)(d + 16) * 2.4e-7f;
+    const float mv = (mx == 0.0f || (m2 > 1e-28f && m2 < 1e37f))
+                         ? __fsqrt_ru(__fmul_ru(m2, slack))
+                         : __fmul_ru(__fmul_ru(mx, 1.000001f), __fsqrt_ru((float)d));
+    // FP64 centers: each end of the move is a rounding away from its center
+    const float pt = shift_pert > 0.0f ? __fmul_ru(shift_pert, __fadd_ru(nrm, mv)) : 0.0f;
+    shift[warp] = bad && was_bad ? -1.0f : (bad || was_bad ? INFINITY : __fadd_ru(mv, pt));
   }
-}
-
-__device__ __forceinline__ void ff_two_sum(float a, float b, float& s, float& e) {
-  s = __fadd_rn(a, b);
-  const float bp = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
+  if (bad) {
+    cn[warp] = INFINITY;
+    if (cxn) cxn[warp] = 0.0f;
+    if (cinit) cinit[warp] = -3.0e38f;
+  } else {
+    cn[warp] = nn;
+    if (cinit) cinit[warp] = -0.5f * nn;
+    atomicMax(reinterpret_cast<int*>(cmax), __float_as_int(nrm));
+    if (cxn) cxn[warp] = nrm;
+  }
 }
 
 // Everything an iteration needs of a row, from one read of it: qn = ||x||^2 (FP64), xn = FP32 upper
@@ -150,15 +189,6 @@ __device__ __forceinline__ float4 load_row4(const T* __restrict__ x, int c, int 
   if (c + 2 < d) v.z = (float)__ldg(x + c + 2);
   if (c + 3 < d) v.w = (float)__ldg(x + c + 3);
   return v;
-}
-
-__device__ __forceinline__ void ff_square_add(float v, float& hi, float& lo) {
-  const float p = __fmul_rn(v, v);
-  const float e = __fmaf_rn(v, v, -p);  // v*v - p exactly
-  float s, err;
-  ff_two_sum(hi, p, s, err);
-  hi = s;
-  lo = __fadd_rn(lo, __fadd_rn(err, e));
 }
 
 __device__ __forceinline__ uint2 bf16x4(float4 v) {

@@ -491,3 +491,30 @@ def test_minibatch_windows_resume(km, orc, torch_cuda, m, d, frac, tier):
         h.synchronize()
     ref = orc.lloyd(X, init, 8, mb_fraction=frac)
     assert np.array_equal(h.centers(), ref[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [2, 3, 130, 4097])
+@pytest.mark.parametrize("batched", [False, True])
+def test_means_at_ties_zeros_and_subnormals(km, orc, torch_cuda, n, batched):
+    """Means that lie on the middle between two FP32 numbers, beside it, at zeros of either sign, among
+    the subnormals and at ordinary values: the FP64 quotient rounded once, as the oracle's."""
+    rng = np.random.default_rng(n)
+    X = np.zeros((2 * n, 9), np.float32)
+    X[:, 0] = 16777216.0
+    X[::2, 0] += 2.0                      # pairs: 16777217, a tie
+    X[:, 1] = 0.0
+    X[:, 2] = -0.0
+    X[:, 3] = rng.integers(1, 50, 2 * n) * np.float32(1e-45)
+    X[:, 4] = -X[:, 0]
+    X[:, 5] = rng.normal(size=2 * n)
+    X[:, 6] = np.where(np.arange(2 * n) % 3, 1.0, np.float32(1.0) + np.float32(2.0) ** -23)
+    X[:, 7] = rng.integers(-3, 4, 2 * n)
+    X[:, 8] = np.repeat([-100.0, 100.0], n)
+    init = np.stack([X[0], X[-1]])
+    ref = orc.lloyd(X, init, 3)
+    if batched:
+        res = km.lloyd_batched([(X, 2, init)], max_iters=3)[0][0]
+    else:
+        res = km.lloyd(X, 2, init=init, max_iters=3)
+    assert np.array_equal(res.labels, ref[2])
+    assert np.array_equal(res.centers.view(np.uint32), np.asarray(ref[1], np.float32).view(np.uint32))
