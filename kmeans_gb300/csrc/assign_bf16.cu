@@ -324,6 +324,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
                    const __grid_constant__ CUtensorMap tmXc,
                    const __grid_constant__ CUtensorMap tmXlc,
                    AssignArgs p, int stages, int xbufs, int mode) {
+  if (grid_enter()) return;
   constexpr int NUM_EPI_WARPS = 4 * EPQ;
   constexpr int EPI_PER_QUAD = EPQ;
   constexpr int COLS_PER_WARP = BN / EPQ;           // columns of a chunk per epilogue warp
@@ -973,13 +974,15 @@ static cudaError_t launch_assign_fp8(const void* X8, long long ld8x, const void*
   cfg.blockDim = dim3(threads_for(4));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch()
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap_allowed(s) ? 2 : 1;
   KMGB_CUDA_TRY(cudaLaunchKernelEx(&cfg, assign_bf16_kernel<4, true, false>, tmX, tmX, tmC, tmC, tmC, tmX,
                                    tmX, a, stages, xbufs, 4));
   count_launches(1);
@@ -1073,13 +1076,15 @@ cudaError_t launch_assign_bf16(const void* Xb, const void* Xl, long long ldxb, c
   cfg.blockDim = dim3(threads_for(epq));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch()
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap_allowed(s) ? 2 : 1;
   if (ab.xmax_out) {  // separation mode: start values by MMA, rows and chunks of whole groups
     if (!bias || !ab.slot_group || ab.u_prob || ab.thr_in || ab.certify)
       return cudaErrorInvalidValue;

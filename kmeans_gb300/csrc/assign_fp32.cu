@@ -85,6 +85,7 @@ template <bool TAIL>
 __global__ void __launch_bounds__(NTHREADS, 1)
 assign_fp32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmC,
                    const __grid_constant__ CUtensorMap tmXc, AssignArgs p) {
+  if (grid_enter()) return;
   if (stopped(p.stop)) return;
   // rows present: a device count, or the rows selected by their distance bounds (the compact copy
   // of the listed rows, or all rows when more than its capacity are listed)
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 assign_fp32_grouped_kernel(const __grid_constant__ CUtensorMap tmX,
                            const __grid_constant__ CUtensorMap tmC, AssignArgs p, GroupArgs g,
                            long long ntiles) {
+  if (grid_enter()) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -495,16 +497,16 @@ cudaError_t launch_assign_fp32(const float* X, long long ldx, const float* Cop, 
     KMGB_CUDA_TRY(cudaGetDevice(&dev));
     KMGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const long long grid = tiles < sms ? tiles : sms;
-    assign_fp32_grouped_kernel<<<(unsigned)grid, NTHREADS, SMEM_BYTES, s>>>(tmX, tmC, a, *grp,
+    launch(assign_fp32_grouped_kernel, (unsigned)grid, NTHREADS, SMEM_BYTES, s)(tmX, tmC, a, *grp,
                                                                            tiles);
   } else {
     const long long grid = (a.n + BM - 1) / BM;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const int tail = a.d % BKF;
     if (tail > 0 && tail <= BKF - 4)
-      assign_fp32_kernel<true><<<(unsigned)grid, NTHREADS, SMEM_BYTES, s>>>(tmX, tmC, tmXc, a);
+      launch(assign_fp32_kernel<true>, (unsigned)grid, NTHREADS, SMEM_BYTES, s)(tmX, tmC, tmXc, a);
     else
-      assign_fp32_kernel<false><<<(unsigned)grid, NTHREADS, SMEM_BYTES, s>>>(tmX, tmC, tmXc, a);
+      launch(assign_fp32_kernel<false>, (unsigned)grid, NTHREADS, SMEM_BYTES, s)(tmX, tmC, tmXc, a);
   }
   kmgb::count_launches(1);
   return cudaGetLastError();

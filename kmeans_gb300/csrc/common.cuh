@@ -13,6 +13,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <utility>
+
 #ifndef KMGB_WAIT_CYCLES
 #define KMGB_WAIT_CYCLES 4000000000ull  // about 2 s per wait at a 2 GHz SM clock
 #endif
@@ -109,6 +111,16 @@ __device__ __forceinline__ uint32_t swz128(uint32_t row, uint32_t chunk) {
   return row * 128u + ((chunk ^ (row & 7u)) << 4);
 }
 
+// First statement of every kernel that launch() starts: waits until the grids before it in its stream
+// are complete and their writes visible, then lets the next grid's blocks take their places. Returns
+// false; the compiler cannot know it, so that no load moves above the wait.
+__device__ __forceinline__ bool grid_enter() {
+  unsigned z;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(z) : : "memory");
+  asm volatile("griddepcontrol.launch_dependents;" : : : "memory");
+  return z != 0;
+}
+
 // Device-side stop rule of the Lloyd loop: once the flag is set every later kernel of the run
 // returns at once, so the host never has to synchronise to evaluate the criterion.
 __device__ __forceinline__ bool stopped(const int* stop) {
@@ -157,6 +169,45 @@ namespace kmgb {
 void count_launches(long long n);
 long long launch_count();
 long long thread_launch_count();  // of the calling thread: what its captured graph holds
+// Whether a launch may overlap the grid before it in its stream (programmatic dependent launch): its
+// blocks take their places while that grid still runs and wait in grid_enter() for its end. Launches
+// one by one gain by it -- five short kernels an entry of the per-kernel interface on 100,000 x 64,
+// K=256 (FP64): 0.78 -> 0.66 ms for nine calls; a draw of k-means++ on 1M x 128: 76 -> 72 us. The nodes
+// of a captured iteration do not: they follow each other within half a microsecond as they are, and
+// with programmatic edges 20 iterations of 100,000 x 32, K=64 took 2.02 instead of 1.87 ms.
+inline bool overlap_allowed(cudaStream_t s) {
+  if (s == nullptr) return true;  // the legacy stream is never captured
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+}
+
+// launch(kernel, grid, block, shared memory, stream)(arguments); the kernel begins with grid_enter().
+template <class... P>
+struct Launch {
+  void (*kernel)(P...);
+  cudaLaunchConfig_t cfg;
+  template <class... A>
+  cudaError_t operator()(A&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = overlap_allowed(cfg.stream) ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  }
+};
+template <class... P>
+Launch<P...> launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
+  Launch<P...> l;
+  l.kernel = kernel;
+  l.cfg = cudaLaunchConfig_t{};
+  l.cfg.gridDim = grid;
+  l.cfg.blockDim = block;
+  l.cfg.dynamicSmemBytes = smem;
+  l.cfg.stream = s;
+  return l;
+}
+
 }  // namespace kmgb
 
 #define KMGB_CUDA_TRY(expr)                        \

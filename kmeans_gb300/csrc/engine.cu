@@ -45,7 +45,9 @@ long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 namespace {
 
-__global__ void set_int_kernel(int* p, int v) { *p = v; }
+__global__ void set_int_kernel(int* p, int v) {
+  if (grid_enter()) return;
+  *p = v; }
 
 thread_local std::string g_last_error;
 
@@ -1401,7 +1403,7 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
                          h->stream),
          KMEANS_ERROR_COMPUTE);
   if (h->mini) {
-    set_int_kernel<<<1, 1, 0, h->stream>>>(h->win_base, h->run_base);
+    launch(set_int_kernel, 1, 1, 0, h->stream)(h->win_base, h->run_base);
     count_launches(1);
     KM_TRY(cudaGetLastError(), KMEANS_ERROR_CONSTRUCT_MINIBATCH);
   }

@@ -28,6 +28,7 @@ namespace {
 
 // CT[t][j] = C[j][t]
 __global__ void transpose_d_kernel(const double* __restrict__ C, int k, int d, double* __restrict__ CT) {
+  if (grid_enter()) return;
   const long long total = (long long)k * d;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -40,8 +41,9 @@ __global__ void transpose_d_kernel(const double* __restrict__ C, int k, int d, d
 // list (nullable): only the points list[0 .. *count) (the tensor pass's uncertified points).
 __global__ void assign_d_kernel(const double* __restrict__ X, long long n, int d,
                                 const double* __restrict__ CT, int k, int* __restrict__ labels,
-                                const int* __restrict__ list = nullptr,
-                                const int* __restrict__ count = nullptr) {
+                                const int* __restrict__ list,
+                                const int* __restrict__ count) {
+  if (grid_enter()) return;
   extern __shared__ double xs_all[];
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* xs = xs_all + (size_t)w * d;
@@ -79,6 +81,7 @@ __global__ void assign_d_kernel(const double* __restrict__ X, long long n, int d
 // out[r][c] = (float)in[r][c] (round to nearest) for c < d, 0 for d <= c < ldo.
 __global__ void d2f_kernel(const double* __restrict__ in, long long rows, int d,
                            float* __restrict__ out, long long ldo) {
+  if (grid_enter()) return;
   const long long total = rows * ldo;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -94,6 +97,7 @@ __global__ void __launch_bounds__(128)
 sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ sorted,
                   const int* __restrict__ label_off, const int* __restrict__ pstart, int k,
                   const double* __restrict__ C, double* __restrict__ piece) {
+  if (grid_enter()) return;
   const int total = pstart[k];
   const int lane = threadIdx.x & 31;
   const int nw = (int)((gridDim.x * blockDim.x) >> 5);
@@ -138,6 +142,7 @@ sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ s
 __global__ void __launch_bounds__(1024)
 sse_d_final_kernel(const double* __restrict__ piece, const int* __restrict__ pstart, int k,
                    const int* __restrict__ dirty, double* __restrict__ sse_k, double* out) {
+  if (grid_enter()) return;
   __shared__ double red[1024];
   double t = 0.0;
   for (int j = threadIdx.x; j < k; j += 1024) {
@@ -161,6 +166,7 @@ sse_d_final_kernel(const double* __restrict__ piece, const int* __restrict__ pst
 
 __global__ void gather_d_kernel(const double* __restrict__ X, int d, const int* __restrict__ perm,
                                 long long m, long long start, long long m_mb, double* __restrict__ Xw) {
+  if (grid_enter()) return;
   const long long total = m_mb * d;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -403,13 +409,13 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   while (it < maxIters && rel > criterion) {
     const double* Xa = X;
     if (mini) {
-      gather_d_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(X, n, permd, m, start, m_mb, Xw); kmgb::count_launches(1);
+      launch(gather_d_kernel, kmgb::num_sms() * 8, 256, 0, s)(X, n, permd, m, start, m_mb, Xw); kmgb::count_launches(1);
       Xa = Xw;
     }
-    transpose_d_kernel<<<kmgb::num_sms() * 4, 256, 0, s>>>(Cd, k, n, CT); kmgb::count_launches(1);
+    launch(transpose_d_kernel, kmgb::num_sms() * 4, 256, 0, s)(Cd, k, n, CT); kmgb::count_launches(1);
     if (tc) {
       const kmeansErrorStatus EA = KMEANS_ERROR_CLOSEST_CENTERS;
-      d2f_kernel<<<kmgb::num_sms() * 4, 256, 0, s>>>(Cd, k, n, Cf, ldx); kmgb::count_launches(1);
+      launch(d2f_kernel, kmgb::num_sms() * 4, 256, 0, s)(Cd, k, n, Cf, ldx); kmgb::count_launches(1);
       KD_TRY(cudaMemsetAsync(cmax, 0, sizeof(float), s), EA);
       KD_TRY(cudaMemsetAsync(rr_count, 0, 3 * sizeof(int), s), EA);
       KD_TRY(launch_prep_centers(Cf, ldx, k, n, Cop, Cb, ldb, cn, cmax, s, nullptr, cinit, Cl, cbias,
@@ -489,7 +495,7 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
       rd.over = over;
       rd.over_count = rr_count + 1;
       KD_TRY(launch_resolve_fp64(rd, s), EA);
-      assign_d_kernel<<<kmgb::num_sms() * 8, threads, smem, s>>>(X, m, n, CT, k, lab, over,
+      launch(assign_d_kernel, kmgb::num_sms() * 8, threads, smem, s)(X, m, n, CT, k, lab, over,
                                                                  rr_count + 1);
       kmgb::count_launches(1);
       if (pr.n > 0) {
@@ -497,7 +503,7 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
         w.dirty = pr.dirty;
       }
     } else {
-      assign_d_kernel<<<kmgb::num_sms() * 8, threads, smem, s>>>(Xa, m_mb, n, CT, k, lab);
+      launch(assign_d_kernel, kmgb::num_sms() * 8, threads, smem, s)(Xa, m_mb, n, CT, k, lab, nullptr, nullptr);
       kmgb::count_launches(1);
     }
     KD_TRY(cudaGetLastError(), KMEANS_ERROR_CLOSEST_CENTERS);
@@ -506,9 +512,9 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
     KD_TRY(launch_tile_accumulate<double>(Xa, n, lab, w, acc, cnt, s), KMEANS_ERROR_CLUSTER_CENTERS);
     KD_TRY(launch_finalize_acc<double>(acc, cnt, k, n, Cd, nullptr, s, w.dirty),
            KMEANS_ERROR_CLUSTER_CENTERS);
-    sse_pieces_kernel<<<kmgb::num_sms() * 8, 128, 0, s>>>(Xa, n, w.sorted, w.label_off, w.piece_cnt, k,
+    launch(sse_pieces_kernel, kmgb::num_sms() * 8, 128, 0, s)(Xa, n, w.sorted, w.label_off, w.piece_cnt, k,
                                                           Cd, part);
-    sse_d_final_kernel<<<1, 1024, 0, s>>>(part, w.piece_cnt, k, w.dirty, sse_k, sse);
+    launch(sse_d_final_kernel, 1, 1024, 0, s)(part, w.piece_cnt, k, w.dirty, sse_k, sse);
     kmgb::count_launches(2);
     KD_TRY(cudaGetLastError(), KMEANS_ERROR_COMPACTNESS);
     double h = 0.0;

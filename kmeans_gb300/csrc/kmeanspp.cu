@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(KPP_THREADS)
 kpp_update_kernel(const T* __restrict__ X, long long ldx, long long n, int d,
                   const int* __restrict__ pick, T* __restrict__ d2, int first,
                   unsigned long long* __restrict__ max_key) {
+  if (grid_enter()) return;
   __shared__ unsigned long long wmax[KPP_THREADS / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* c = X + (size_t)(*pick) * ldx;
@@ -323,6 +324,7 @@ kpp_update_bulk_kernel(const T* __restrict__ X, long long ldx, long long n, int 
                        const int* __restrict__ pick, T* __restrict__ d2, int first,
                        unsigned long long* __restrict__ max_key, int rows_per_stage, int stages,
                        int* __restrict__ err, KppNear nr) {
+  if (grid_enter()) return;
   extern __shared__ __align__(128) unsigned char kpp_smem[];
   __shared__ __align__(8) uint64_t full_bar[KPP_MAX_STAGES], empty_bar[KPP_MAX_STAGES];
   __shared__ unsigned long long wmax[KPP_CONSUMERS + 1];
@@ -445,6 +447,7 @@ template <typename T>
 __global__ void kpp_center_dist_kernel(const T* __restrict__ X, long long ldx, int d,
                                        const int* __restrict__ picks, int draw, T* __restrict__ cc,
                                        unsigned int* __restrict__ active) {
+  if (grid_enter()) return;
   const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (q == 0 && lane == 0 && active[1]) {
@@ -473,6 +476,7 @@ kpp_draw_kernel(long long n, const T* __restrict__ d2, unsigned long long* block
                 bool weights, const unsigned long long* __restrict__ max_key,
                 unsigned long long* __restrict__ next_max_key, unsigned int* ticket,
                 unsigned long long seed, int round, int* __restrict__ pick, int* __restrict__ picks) {
+  if (grid_enter()) return;
   __shared__ unsigned long long warp_sh[32];
   __shared__ unsigned long long total_sh, off_sh, tot2_sh;
   __shared__ long long block_sh, chosen_sh;
@@ -550,6 +554,7 @@ template <typename T>
 __global__ void kpp_gather_kernel(const T* __restrict__ X, long long ldx, int d,
                                   const int* __restrict__ picks, int k, T* __restrict__ C,
                                   long long ldc) {
+  if (grid_enter()) return;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < (long long)k * d;
        e += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(e / d), t = (int)(e - (long long)j * d);
@@ -626,27 +631,27 @@ cudaError_t kmeanspp_impl(const T* X, long long ldx, long long n, int d, int k,
   const long long dblocks = (nb + 31) / 32, most = kmgb::num_sms();  // a warp per 1024 points
   const unsigned dgrid = (unsigned)(dblocks < most ? dblocks : most);
   // draw 0: zero total weight, so uniform
-  kpp_draw_kernel<T><<<1, KPP_BLOCK, 0, s>>>(n, w.d2, w.blocksum, nb, false, mx, mx + 1, ticket, seed, 0,
+  launch(kpp_draw_kernel<T>, 1, KPP_BLOCK, 0, s)(n, w.d2, w.blocksum, nb, false, mx, mx + 1, ticket, seed, 0,
                                              pick, picks);
   count_launches(1);
   for (int r = 1; r < k; ++r) {
     unsigned long long* m = mx + (r & 1);
     nr.draw = r - 1;
     if (nr.near && r > 1) {
-      kpp_center_dist_kernel<T><<<(unsigned)((nr.draw + 7) / 8), 256, 0, s>>>(
+      launch(kpp_center_dist_kernel<T>, (unsigned)((nr.draw + 7) / 8), 256, 0, s)(
           X, ldx, d, picks, nr.draw, static_cast<T*>(w.cc), nr.active);
       count_launches(1);
     }
     if (bulk)
-      kpp_update_bulk_kernel<T><<<grid, KPP_BULK_THREADS, smem, s>>>(
+      launch(kpp_update_bulk_kernel<T>, grid, KPP_BULK_THREADS, smem, s)(
           X, ldx, n, d, pick, w.d2, r == 1, m, rps, stages, err, nr);
     else
-      kpp_update_kernel<T><<<(unsigned)nb, KPP_THREADS, 0, s>>>(X, ldx, n, d, pick, w.d2, r == 1, m);
-    kpp_draw_kernel<T><<<dgrid, KPP_BLOCK, 0, s>>>(n, w.d2, w.blocksum, nb, true, m,
+      launch(kpp_update_kernel<T>, (unsigned)nb, KPP_THREADS, 0, s)(X, ldx, n, d, pick, w.d2, r == 1, m);
+    launch(kpp_draw_kernel<T>, dgrid, KPP_BLOCK, 0, s)(n, w.d2, w.blocksum, nb, true, m,
                                                    mx + ((r + 1) & 1), ticket, seed, r, pick, picks);
     count_launches(2);
   }
-  kpp_gather_kernel<T><<<kmgb::num_sms() * 4, 256, 0, s>>>(X, ldx, d, picks, k, C, ldc);
+  launch(kpp_gather_kernel<T>, kmgb::num_sms() * 4, 256, 0, s)(X, ldx, d, picks, k, C, ldc);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -56,6 +56,7 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
                                     __nv_bfloat16* __restrict__ Cl,
                                     __nv_bfloat16* __restrict__ cbias, float* __restrict__ shift,
                                     float* __restrict__ cxn, float shift_pert) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -211,6 +212,7 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
                  double* __restrict__ qn, float* __restrict__ xn, uint2* __restrict__ Xb,
                  uint2* __restrict__ Xl, int ldb, int* inexact, float* __restrict__ nf, RowList rl,
                  RowWindow rw, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   if (IDX == 1) {
     const long long total = *reinterpret_cast<volatile const int*>(rl.count);
@@ -332,6 +334,7 @@ __global__ void prep_expansion_kernel(const T* __restrict__ B, int d, int k, con
                                       __nv_bfloat16* __restrict__ Cb, __nv_bfloat16* __restrict__ Cl,
                                       long long ldb, float* __restrict__ cinit,
                                       __nv_bfloat16* __restrict__ cbias, int kpad, float* cmax) {
+  if (grid_enter()) return;
   const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (j >= kpad) return;
@@ -391,6 +394,7 @@ __device__ __forceinline__ float pow2_scale_for(float mx) {
 __global__ void to_fp8_kernel(const float* __restrict__ X, long long ldx, long long n, int d,
                               uint8_t* __restrict__ X8, long long ld8, float* __restrict__ sx,
                               const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int lane = threadIdx.x & 31;
   for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n;
@@ -414,6 +418,7 @@ __global__ void to_fp8_kernel(const float* __restrict__ X, long long ldx, long l
 __global__ void centers_fp8_kernel(const float* __restrict__ Cop, long long ldc, int k, int d,
                                    const float* __restrict__ cmax, uint8_t* __restrict__ C8,
                                    long long ld8, float* __restrict__ cscale, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const float sc = pow2_scale_for(*cmax);
   const float inv = 1.0f / sc;
@@ -435,7 +440,7 @@ cudaError_t launch_to_fp8(const float* X, long long ldx, long long n, int d, voi
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (n <= 0) return cudaSuccess;
   if (ld8 % 16 || ld8 < d) return cudaErrorInvalidValue;
-  to_fp8_kernel<<<kmgb::num_sms() * 16, 256, 0, s>>>(X, ldx, n, d, static_cast<uint8_t*>(X8), ld8,
+  launch(to_fp8_kernel, kmgb::num_sms() * 16, 256, 0, s)(X, ldx, n, d, static_cast<uint8_t*>(X8), ld8,
                                                      sx, stop);
   kmgb::count_launches(1);
   return cudaGetLastError();
@@ -446,7 +451,7 @@ cudaError_t launch_centers_fp8(const float* Cop, long long ldc, int k, int d, co
                                const int* stop) {
   if (k <= 0) return cudaSuccess;
   if (ld8 % 16 || ld8 < d) return cudaErrorInvalidValue;
-  centers_fp8_kernel<<<kmgb::num_sms() * 4, 256, 0, s>>>(Cop, ldc, k, d, cmax,
+  launch(centers_fp8_kernel, kmgb::num_sms() * 4, 256, 0, s)(Cop, ldc, k, d, cmax,
                                                          static_cast<uint8_t*>(C8), ld8, cscale,
                                                          stop);
   kmgb::count_launches(1);
@@ -462,7 +467,7 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
   const int threads = 256;
   const int kpad = (k + kCenterPad - 1) / kCenterPad * kCenterPad;
   const int blocks = (int)(((long long)(cinit || cbias ? kpad : k) * 32 + threads - 1) / threads);
-  prep_centers_kernel<<<blocks, threads, 0, s>>>(C, ldc, k, d, Cop,
+  launch(prep_centers_kernel, blocks, threads, 0, s)(C, ldc, k, d, Cop,
                                                  reinterpret_cast<__nv_bfloat16*>(Cb), ldcb, cn,
                                                  cmax, stop, cinit, kpad,
                                                  reinterpret_cast<__nv_bfloat16*>(Cl),
@@ -489,13 +494,13 @@ static cudaError_t prep_rows(const T* X, long long ldx, long long n, int d, doub
   uint2* l = static_cast<uint2*>(Xl);
   auto go = [&](auto tag) {
     if (rl)
-      prep_rows_kernel<T, decltype(tag)::value, 1><<<blocks, 256, 0, s>>>(
+      launch(prep_rows_kernel<T, decltype(tag)::value, 1>, blocks, 256, 0, s)(
           X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nullptr, *rl, RowWindow{}, stop);
     else if (rw)
-      prep_rows_kernel<T, decltype(tag)::value, 2><<<blocks, 256, 0, s>>>(
+      launch(prep_rows_kernel<T, decltype(tag)::value, 2>, blocks, 256, 0, s)(
           X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nullptr, RowList{}, *rw, stop);
     else
-      prep_rows_kernel<T, decltype(tag)::value, 0><<<blocks, 256, 0, s>>>(
+      launch(prep_rows_kernel<T, decltype(tag)::value, 0>, blocks, 256, 0, s)(
           X, ldx, n, d, vec, qn, xn, b, l, (int)ldb, inexact, nf, RowList{}, RowWindow{}, stop);
   };
   if (lanes == 4) go(std::integral_constant<int, 4>{});
@@ -538,7 +543,7 @@ cudaError_t launch_prep_expansion(const T* B, int d, int k, const T* nb, float* 
                                   float* nbx, void* Cb, void* Cl, long long ldb, float* cinit,
                                   void* cbias, float* cmax, cudaStream_t s) {
   const int kpad = cinit ? (k + kCenterPad - 1) / kCenterPad * kCenterPad : k;
-  prep_expansion_kernel<T><<<(unsigned)(((long long)kpad * 32 + 255) / 256), 256, 0, s>>>(
+  launch(prep_expansion_kernel<T>, (unsigned)(((long long)kpad * 32 + 255) / 256), 256, 0, s)(
       B, d, k, nb, Bt, ld, nbx, static_cast<__nv_bfloat16*>(Cb), static_cast<__nv_bfloat16*>(Cl), ldb,
       cinit, static_cast<__nv_bfloat16*>(cbias), kpad, cmax);
   kmgb::count_launches(1);

@@ -27,6 +27,7 @@ constexpr int PF_ROWS = 4 * PF_THREADS;  // rows per block step, four consecutiv
 // center's members count as changed). One block.
 __global__ void __launch_bounds__(1024)
 prune_top_kernel(PruneState ps, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   __shared__ float s1[32], s2[32];
   __shared__ int si[32];
@@ -88,6 +89,7 @@ prune_top_kernel(PruneState ps, const int* stop) {
 // to come return.
 __global__ void __launch_bounds__(PF_THREADS)
 prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   __shared__ int wsum[PF_THREADS / 32];
   __shared__ int base_sh;
@@ -178,6 +180,7 @@ prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* st
 // One warp per listed row, 16-byte moves, both planes' loads of a row in flight together.
 __global__ void prune_gather_kernel(PruneState ps, const uint4* __restrict__ Xb,
                                     const uint4* __restrict__ Xl, int row_vec, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int cnt = ps.flags[1];
   if (cnt > ps.cap) return;
@@ -222,6 +225,7 @@ constexpr int kDirtyShared = 32768;
 
 __global__ void __launch_bounds__(1024)
 prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int cnt = ps.flags[1];
   if (cnt == 0) return;
@@ -262,6 +266,7 @@ prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* sto
 // iteration).
 __global__ void __launch_bounds__(256)
 prune_top_batched_kernel(PruneBatch pb) {
+  if (grid_enter()) return;
   __shared__ float s1[8], s2[8];
   __shared__ int si[8];
   const PruneState& ps = pb.ps;
@@ -306,6 +311,7 @@ prune_top_batched_kernel(PruneBatch pb) {
 __global__ void __launch_bounds__(PF_THREADS)
 prune_window_kernel(PruneBatch pb, const int* __restrict__ labels, const uint4* __restrict__ Xb,
                     const uint4* __restrict__ Xl, int row_vec) {
+  if (grid_enter()) return;
   constexpr int kPer = kPruneWindow / PF_THREADS;
   __shared__ int rows_sh[kPruneWindow];
   __shared__ int wsum[PF_THREADS / 32];
@@ -412,6 +418,7 @@ prune_window_kernel(PruneBatch pb, const int* __restrict__ labels, const uint4* 
 // iteration are done: block 0 starts the next one's unit table.
 __global__ void __launch_bounds__(PF_THREADS)
 prune_dirty_batched_kernel(PruneBatch pb, const int* __restrict__ labels) {
+  if (grid_enter()) return;
   const PruneState& ps = pb.ps;
   const int win = blockIdx.x;
   if (win == 0 && threadIdx.x == 0) {
@@ -438,15 +445,15 @@ prune_dirty_batched_kernel(PruneBatch pb, const int* __restrict__ labels) {
 cudaError_t launch_prune_batched(const PruneBatch& pb, const int* labels, const void* Xb,
                                  const void* Xl, long long row_bytes, cudaStream_t s) {
   if (row_bytes % 16 || (Xl && !pb.ps.Xlc)) return cudaErrorInvalidValue;
-  prune_top_batched_kernel<<<(unsigned)pb.P, 256, 0, s>>>(pb);
-  prune_window_kernel<<<(unsigned)pb.windows, PF_THREADS, 0, s>>>(
+  launch(prune_top_batched_kernel, (unsigned)pb.P, 256, 0, s)(pb);
+  launch(prune_window_kernel, (unsigned)pb.windows, PF_THREADS, 0, s)(
       pb, labels, static_cast<const uint4*>(Xb), static_cast<const uint4*>(Xl), (int)(row_bytes / 16));
   count_launches(2);
   return cudaGetLastError();
 }
 
 cudaError_t launch_prune_dirty_batched(const PruneBatch& pb, const int* labels, cudaStream_t s) {
-  prune_dirty_batched_kernel<<<(unsigned)pb.windows, PF_THREADS, 0, s>>>(pb, labels);
+  launch(prune_dirty_batched_kernel, (unsigned)pb.windows, PF_THREADS, 0, s)(pb, labels);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -455,8 +462,7 @@ cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const in
                                cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   const long long blocks = (ps.n + 1023) / 1024, most = 2LL * kmgb::num_sms();
-  prune_dirty_kernel<<<(unsigned)(blocks < most ? blocks : most), 1024,
-                       ps.k <= kDirtyShared ? ps.k : 0, s>>>(ps, labels, stop);
+  launch(prune_dirty_kernel, (unsigned)(blocks < most ? blocks : most), 1024, ps.k <= kDirtyShared ? ps.k : 0, s)(ps, labels, stop);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -464,10 +470,10 @@ cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const in
 cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
                                 cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
-  prune_top_kernel<<<1, 1024, 0, s>>>(ps, stop);
+  launch(prune_top_kernel, 1, 1024, 0, s)(ps, stop);
   const long long steps = (ps.n + PF_ROWS - 1) / PF_ROWS;
   const long long most = kmgb::num_sms() * 8LL;
-  prune_filter_kernel<<<(unsigned)(steps < most ? steps : most), PF_THREADS, 0, s>>>(ps, labels,
+  launch(prune_filter_kernel, (unsigned)(steps < most ? steps : most), PF_THREADS, 0, s)(ps, labels,
                                                                                      stop);
   count_launches(2);
   return cudaGetLastError();
@@ -477,7 +483,7 @@ cudaError_t launch_prune_gather(const PruneState& ps, const void* Xb, const void
                                 long long row_bytes, const int* stop, cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (row_bytes % 16 || (Xl && !ps.Xlc)) return cudaErrorInvalidValue;
-  prune_gather_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(
+  launch(prune_gather_kernel, kmgb::num_sms() * 8, 256, 0, s)(
       ps, static_cast<const uint4*>(Xb), static_cast<const uint4*>(Xl), (int)(row_bytes / 16), stop);
   count_launches(1);
   return cudaGetLastError();

@@ -28,6 +28,7 @@ void tmp_free(void* p) {
 
 __global__ void copy_pad_kernel(const float* __restrict__ A, long long m, int d, float* __restrict__ Ap,
                                 long long ld) {
+  if (grid_enter()) return;
   const long long total = m * ld;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -43,6 +44,7 @@ __global__ void closest_fp64_kernel(int m0, int m, int d, const double* __restri
                                     const double* __restrict__ B, const double* __restrict__ nb,
                                     int* __restrict__ out, const int* __restrict__ list,
                                     const int* __restrict__ count) {
+  if (grid_enter()) return;
   extern __shared__ double xs_all[];
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* xs = xs_all + (size_t)w * d;
@@ -80,6 +82,7 @@ template <typename T>
 __global__ void row_transform_min_kernel(int m0, int m, int n, const T* __restrict__ na,
                                          const T* __restrict__ nbv, const T* __restrict__ in,
                                          int* __restrict__ out) {
+  if (grid_enter()) return;
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (long long i = (long long)blockIdx.x * warps + w; i < m; i += (long long)gridDim.x * warps) {
     T best = (T)FLT_MAX;
@@ -140,6 +143,7 @@ template <int L>
 __global__ void __launch_bounds__(256)
 compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const int* __restrict__ idx,
                       const float* __restrict__ centers, bool vec, double* __restrict__ partial) {
+  if (grid_enter()) return;
   constexpr int G = 32 / L;
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -201,6 +205,7 @@ compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const 
 __global__ void __launch_bounds__(256)
 compactness_d_kernel(long long m, int n, const double* __restrict__ data, const int* __restrict__ idx,
                      const double* __restrict__ centers, double* __restrict__ partial) {
+  if (grid_enter()) return;
   const int lane = threadIdx.x & 31;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -232,6 +237,7 @@ compactness_d_kernel(long long m, int n, const double* __restrict__ data, const 
 template <typename T>
 __global__ void __launch_bounds__(256)
 compactness_final_kernel(const double* __restrict__ partial, int nb, double* acc, T* out, bool last) {
+  if (grid_enter()) return;
   double t = 0.0;
   for (int i = threadIdx.x; i < nb; i += 256) t += partial[i];
   t = block_sum(t);
@@ -243,6 +249,7 @@ compactness_final_kernel(const double* __restrict__ partial, int nb, double* acc
 
 template <typename T>
 __global__ void row_norm_kernel(int m0, int m, int n, const T* __restrict__ in, T* __restrict__ out) {
+  if (grid_enter()) return;
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (long long i = (long long)blockIdx.x * warps + w; i < m; i += (long long)gridDim.x * warps) {
     double s = 0.0;
@@ -257,6 +264,7 @@ __global__ void row_norm_kernel(int m0, int m, int n, const T* __restrict__ in, 
 template <typename T>
 __global__ void __launch_bounds__(1024)
 col_norm_kernel(int m, int n, const T* __restrict__ in, T* __restrict__ out) {
+  if (grid_enter()) return;
   __shared__ double red[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long long j = (long long)blockIdx.x * 32 + tx;
@@ -284,6 +292,7 @@ col_norm_kernel(int m, int n, const T* __restrict__ in, T* __restrict__ out) {
 template <typename T>
 __global__ void matmul_kernel(int ra, int ca, int cb, const T* __restrict__ A,
                               const T* __restrict__ B, T* __restrict__ C) {
+  if (grid_enter()) return;
   constexpr int TM = 64, TN = 64, TK = 16;
   __shared__ T As[TK][TM + 1];
   __shared__ T Bs[TK][TN];
@@ -343,7 +352,7 @@ kmeansCudaErrorStatus mat_mat_mult(int ra, int ca, const T* A, int cb, const T* 
   if (!C || (ca > 0 && (!A || !B))) return ERROR_MATMATMULT;
   const long long col_tiles = ((long long)cb + 63) / 64, row_tiles = ((long long)ra + 63) / 64;
   const dim3 grid((unsigned)col_tiles, (unsigned)(row_tiles < 65535 ? row_tiles : 65535));
-  matmul_kernel<T><<<grid, 256, 0, kDefault>>>(ra, ca, cb, A, B, C);
+  launch(matmul_kernel<T>, grid, 256, 0, kDefault)(ra, ca, cb, A, B, C);
   kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_MATMATMULT : NO_ERROR;
 }
@@ -381,7 +390,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   const int threads = 256;
   const size_t smem = sizeof(double) * (size_t)d * (threads / 32);  // closest_fp64_kernel's
   if (!kF32 && !tc) {
-    closest_fp64_kernel<<<kmgb::num_sms() * 8, threads, smem, kDefault>>>(
+    launch(closest_fp64_kernel, kmgb::num_sms() * 8, threads, smem, kDefault)(
         m0, (int)n, d, reinterpret_cast<const double*>(A), k, reinterpret_cast<const double*>(B),
         reinterpret_cast<const double*>(nb), out, nullptr, nullptr);
     count_launches(1);
@@ -431,7 +440,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   cudaError_t e = cudaMemsetAsync(sc, 0, 8 * sizeof(int), kDefault);
   const T* Xa = A;
   if (!e && copy) {
-    copy_pad_kernel<<<num_sms() * 8, 256, 0, kDefault>>>(reinterpret_cast<const float*>(A), n, d, Ap,
+    launch(copy_pad_kernel, num_sms() * 8, 256, 0, kDefault)(reinterpret_cast<const float*>(A), n, d, Ap,
                                                          ld);
     count_launches(1);
     e = cudaGetLastError();
@@ -538,7 +547,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
     r.over_count = sc + 2;
     if (!e) e = launch_resolve_fp64(r, kDefault);
     if (!e) {
-      closest_fp64_kernel<<<num_sms() * 8, threads, smem, kDefault>>>(
+      launch(closest_fp64_kernel, num_sms() * 8, threads, smem, kDefault)(
           m0, (int)n, d, r.X, k, r.C, r.nb, out, over, sc + 2);
       count_launches(1);
       e = cudaGetLastError();
@@ -591,15 +600,15 @@ void launch_compactness(long long m, int n, const float* data, const int* idx, c
   const bool vec = n % 4 == 0 && !(reinterpret_cast<uintptr_t>(data) & 15) &&
                    !(reinterpret_cast<uintptr_t>(centers) & 15);
   const int per = vec ? (n + 3) / 4 : n;  // lanes' worth of a row
-  if (per <= 4) compactness_ff_kernel<4><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
-  else if (per <= 8) compactness_ff_kernel<8><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
-  else if (per <= 16) compactness_ff_kernel<16><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
-  else compactness_ff_kernel<32><<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, vec, part);
+  if (per <= 4) launch(compactness_ff_kernel<4>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
+  else if (per <= 8) launch(compactness_ff_kernel<8>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
+  else if (per <= 16) launch(compactness_ff_kernel<16>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
+  else launch(compactness_ff_kernel<32>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
   count_launches(1);
 }
 void launch_compactness(long long m, int n, const double* data, const int* idx, const double* centers,
                         double* part, int blocks) {
-  compactness_d_kernel<<<blocks, 256, 0, kDefault>>>(m, n, data, idx, centers, part);
+  launch(compactness_d_kernel, blocks, 256, 0, kDefault)(m, n, data, idx, centers, part);
   count_launches(1);
 }
 
@@ -618,7 +627,7 @@ kmeansCudaErrorStatus compactness(int m0, int m, bool lastTile, int n, int k, co
     e = cudaGetLastError();
   }
   if (!e) {
-    compactness_final_kernel<T><<<1, 256, 0, kDefault>>>(part, blocks, acc, out, lastTile); kmgb::count_launches(1);
+    launch(compactness_final_kernel<T>, 1, 256, 0, kDefault)(part, blocks, acc, out, lastTile); kmgb::count_launches(1);
     e = cudaGetLastError();
   }
   tmp_free(part);
@@ -681,7 +690,7 @@ kmeansCudaErrorStatus rowTransformMinimumF(const int m0, const int m, const int 
                                            int* output) {
   if (m < 0 || n <= 0) return ERROR_ROWTRANSFORMMINIMUM;
   if (m == 0) return NO_ERROR;
-  row_transform_min_kernel<float><<<kmgb::num_sms() * 8, 256, 0, kDefault>>>(
+  launch(row_transform_min_kernel<float>, kmgb::num_sms() * 8, 256, 0, kDefault)(
       m0, m, n, normRowsOfA_squared, normColsOfB_squared, input, output); kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_ROWTRANSFORMMINIMUM : NO_ERROR;
 }
@@ -692,7 +701,7 @@ kmeansCudaErrorStatus rowTransformMinimumD(const int m0, const int m, const int 
                                            const double* input, int* output) {
   if (m < 0 || n <= 0) return ERROR_ROWTRANSFORMMINIMUM;
   if (m == 0) return NO_ERROR;
-  row_transform_min_kernel<double><<<kmgb::num_sms() * 8, 256, 0, kDefault>>>(
+  launch(row_transform_min_kernel<double>, kmgb::num_sms() * 8, 256, 0, kDefault)(
       m0, m, n, normRowsOfA_squared, normColsOfB_squared, input, output); kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_ROWTRANSFORMMINIMUM : NO_ERROR;
 }
@@ -746,20 +755,20 @@ kmeansCudaErrorStatus rowNormalizeD(const int m0, const int m, const int n, cons
                                     double* output) {
   if (m < 0 || n <= 0) return ERROR_ROWNORMALIZE;
   if (m == 0) return NO_ERROR;
-  row_norm_kernel<double><<<kmgb::num_sms() * 8, 256, 0, kDefault>>>(m0, m, n, input, output); kmgb::count_launches(1);
+  launch(row_norm_kernel<double>, kmgb::num_sms() * 8, 256, 0, kDefault)(m0, m, n, input, output); kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_ROWNORMALIZE : NO_ERROR;
 }
 
 kmeansCudaErrorStatus colNormalizeF(const int m, const int n, const float* input, float* output) {
   if (m < 0 || n <= 0) return ERROR_COLNORMALIZE;
-  col_norm_kernel<float><<<(unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault>>>(m, n, input, output); kmgb::count_launches(1);
+  launch(col_norm_kernel<float>, (unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault)(m, n, input, output); kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_COLNORMALIZE : NO_ERROR;
 }
 
 kmeansCudaErrorStatus colNormalizeD(const int m, const int n, const double* input,
                                     double* output) {
   if (m < 0 || n <= 0) return ERROR_COLNORMALIZE;
-  col_norm_kernel<double><<<(unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault>>>(m, n, input, output); kmgb::count_launches(1);
+  launch(col_norm_kernel<double>, (unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault)(m, n, input, output); kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_COLNORMALIZE : NO_ERROR;
 }
 

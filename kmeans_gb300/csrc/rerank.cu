@@ -55,6 +55,7 @@ __device__ __forceinline__ double exact_value(int mode, const float* __restrict_
 }
 
 __global__ void rerank_kernel(RerankArgs a) {
+  if (grid_enter()) return;
   if (stopped(a.stop)) return;
   extern __shared__ float xs_all[];
   const int warps = blockDim.x >> 5;
@@ -309,6 +310,7 @@ template <int MODE, bool SETTLE>
 __global__ void __launch_bounds__(256)
 rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ count2,
                     float* __restrict__ hi2) {
+  if (grid_enter()) return;
   if (stopped(a.stop)) return;
   extern __shared__ float4 sm4[];
   const int dq = (a.d + 3) >> 2;          // float4 per row
@@ -481,6 +483,7 @@ __global__ void __launch_bounds__(256)
 rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict__ cand,
                     int* __restrict__ cand_cnt, long long cand_cap, int* __restrict__ over,
                     int* __restrict__ over_count, float* __restrict__ over_hi) {
+  if (grid_enter()) return;
   if (stopped(a.stop)) return;
   extern __shared__ float4 sm4[];
   const int dq = (a.d + 3) >> 2;
@@ -541,6 +544,7 @@ template <int L>
 __global__ void __launch_bounds__(RG_WARPS * 32)
 rerank_grouped_kernel(RerankArgs a, GroupArgs g, int* __restrict__ cand, int* __restrict__ cand_cnt,
                       long long cand_cap) {
+  if (grid_enter()) return;
   if (stopped(a.stop)) return;
   extern __shared__ float rg_smem[];  // [warps][RG_VCAP] values, then [warps][ds] rows
   constexpr int G = 32 / L;           // centers side by side
@@ -662,6 +666,7 @@ __global__ void gather_flagged_kernel(const int* __restrict__ list, const int* _
                                       int* __restrict__ over, int* __restrict__ over_count,
                                       const int* stop, const float* __restrict__ xs,
                                       float* __restrict__ xsC) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const long long total = *(volatile const int*)count;
   const long long cnt = min(total, cap);
@@ -810,6 +815,7 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
                                           const int* __restrict__ row_map,
                                           const float* __restrict__ hi_in,
                                           float* __restrict__ over_hi) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const long long cnt = min((long long)*(volatile const int*)count, max_list);
   const int lane = threadIdx.x & 31;
@@ -992,6 +998,7 @@ template <bool VEC>
 __global__ void resolve_expansion_kernel(RerankArgs a, const int* __restrict__ cand,
                                          const int* __restrict__ cand_cnt, int* __restrict__ over,
                                          int* __restrict__ over_count) {
+  if (grid_enter()) return;
   const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
   const int lane = threadIdx.x & 31;
   const int grp = lane / kGroupLanes, sub = lane % kGroupLanes;
@@ -1072,6 +1079,7 @@ __global__ void resolve_expansion_kernel(RerankArgs a, const int* __restrict__ c
 // FP64 data: every candidate's exact value, eight lanes (candidates) per point, four points per
 // warp: the FP64 pipe takes a warp instruction in the same time whatever its active lanes.
 __global__ void resolve_fp64_kernel(ResolveD a) {
+  if (grid_enter()) return;
   constexpr int L = 8;
   const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
@@ -1225,6 +1233,7 @@ audit_scan_kernel(const float* __restrict__ X, long long ldx, long long n, int d
                   const float* __restrict__ C, long long ldc, int k,
                   const int* __restrict__ labels, unsigned long long* ws, int rows, int parts,
                   GroupArgs g, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   extern __shared__ float ax[];
   __shared__ int viol_sh;
@@ -1304,7 +1313,7 @@ cudaError_t launch_gather_flagged(const int* list, const int* count, long long c
                                   const float* xs, float* xsC) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (row_bytes % 16) return cudaErrorInvalidValue;
-  gather_flagged_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(
+  launch(gather_flagged_kernel, kmgb::num_sms() * 8, 256, 0, s)(
       list, count, cap, reinterpret_cast<const uint4*>(Xb), reinterpret_cast<const uint4*>(Xl),
       row_bytes / 16, thr, reinterpret_cast<uint4*>(XbC), reinterpret_cast<uint4*>(XlC), thrC, over,
       over_count, stop, xs, xsC);
@@ -1322,11 +1331,11 @@ cudaError_t launch_resolve_candidates(const int* list, const int* count, long lo
   const bool vec = d % 4 == 0 && ldx % 4 == 0 && ldc % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(X) % 16 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
   if (vec)
-    resolve_candidates_kernel<true><<<kmgb::num_sms() * 8, 256, 0, s>>>(list, count, max_list, cand, cand_cnt,
+    launch(resolve_candidates_kernel<true>, kmgb::num_sms() * 8, 256, 0, s)(list, count, max_list, cand, cand_cnt,
                                                             X, ldx, C, ldc, cn, d, labels, over,
                                                             over_count, stop, row_map, hi_in, over_hi);
   else
-    resolve_candidates_kernel<false><<<kmgb::num_sms() * 8, 256, 0, s>>>(list, count, max_list, cand, cand_cnt,
+    launch(resolve_candidates_kernel<false>, kmgb::num_sms() * 8, 256, 0, s)(list, count, max_list, cand, cand_cnt,
                                                              X, ldx, C, ldc, cn, d, labels, over,
                                                              over_count, stop, row_map, hi_in, over_hi);
   count_launches(1);
@@ -1339,17 +1348,17 @@ cudaError_t launch_resolve_expansion(const RerankArgs& a, const int* cand, const
                    reinterpret_cast<uintptr_t>(a.X) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(a.C) % 16 == 0;
   if (vec)
-    resolve_expansion_kernel<true><<<kmgb::num_sms() * 8, 256, 0, s>>>(a, cand, cand_cnt, over,
+    launch(resolve_expansion_kernel<true>, kmgb::num_sms() * 8, 256, 0, s)(a, cand, cand_cnt, over,
                                                                        over_count);
   else
-    resolve_expansion_kernel<false><<<kmgb::num_sms() * 8, 256, 0, s>>>(a, cand, cand_cnt, over,
+    launch(resolve_expansion_kernel<false>, kmgb::num_sms() * 8, 256, 0, s)(a, cand, cand_cnt, over,
                                                                         over_count);
   count_launches(1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_resolve_fp64(const ResolveD& a, cudaStream_t s) {
-  resolve_fp64_kernel<<<kmgb::num_sms() * 8, 256, 0, s>>>(a);
+  launch(resolve_fp64_kernel, kmgb::num_sms() * 8, 256, 0, s)(a);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1369,7 +1378,7 @@ cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStrea
   auto kern = a.mode == 0 ? rerank_exact_kernel<0, false> : rerank_exact_kernel<1, false>;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
-  kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, hi2, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
+  launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, hi2, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1384,7 +1393,7 @@ cudaError_t launch_rerank_band(const RerankArgs& a, const float* hi2, int* cand,
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<0, true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
-  rerank_exact_kernel<0, true><<<kmgb::num_sms() * 2, 256, smem, s>>>(
+  launch(rerank_exact_kernel<0, true>, kmgb::num_sms() * 2, 256, smem, s)(
       a, hi2, cand, cand_cnt, cand_cap, over, over_count, over_hi);
   count_launches(1);
   return cudaGetLastError();
@@ -1399,7 +1408,7 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
   auto kern = a.mode == 0 ? rerank_tiled_kernel<0, false> : rerank_tiled_kernel<1, false>;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
-  kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, list2, count2, hi2);
+  launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, list2, count2, hi2);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1412,7 +1421,7 @@ cudaError_t launch_rerank_settle(const RerankArgs& a, cudaStream_t s) {
   auto kern = a.mode == 0 ? rerank_tiled_kernel<0, true> : rerank_tiled_kernel<1, true>;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
-  kern<<<kmgb::num_sms() * 2, 256, smem, s>>>(a, nullptr, nullptr, nullptr);
+  launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, nullptr, nullptr, nullptr);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1429,7 +1438,7 @@ cudaError_t launch_rerank_grouped(const RerankArgs& a, const GroupArgs& g, cudaS
                                      : (a.d <= 64 ? rerank_grouped_kernel<16> : rerank_grouped_kernel<32>));
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
-  kern<<<kmgb::num_sms() * 4, RG_WARPS * 32, smem, s>>>(a, g, cand, cand_cnt, cand_cap);
+  launch(kern, kmgb::num_sms() * 4, RG_WARPS * 32, smem, s)(a, g, cand, cand_cnt, cand_cap);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1444,7 +1453,7 @@ cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t s) {
                                        kMaxTileSmem));
   }
   // Persistent grid: the flagged count lives on the device, so no host round trip is needed.
-  rerank_kernel<<<kmgb::num_sms() * 4, threads, smem, s>>>(a); kmgb::count_launches(1);
+  launch(rerank_kernel, kmgb::num_sms() * 4, threads, smem, s)(a); kmgb::count_launches(1);
   return cudaGetLastError();
 }
 
@@ -1461,7 +1470,7 @@ cudaError_t launch_audit_labels(const float* X, long long ldx, long long n, int 
   if (rows > kAuditMaxRows || (size_t)d * sizeof(float) > 48 * 1024) return cudaErrorInvalidValue;
   const int parts = audit_parts(rows);
   const GroupArgs g = grp ? *grp : GroupArgs{};
-  audit_scan_kernel<<<rows * parts, 256, sizeof(float) * (size_t)d, s>>>(X, ldx, n, d, C, ldc, k,
+  launch(audit_scan_kernel, rows * parts, 256, sizeof(float) * (size_t)d, s)(X, ldx, n, d, C, ldc, k,
                                                                         labels, ws, rows, parts, g,
                                                                         stop);
   count_launches(1);

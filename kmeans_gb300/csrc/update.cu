@@ -110,6 +110,7 @@ __device__ void block_scan_inplace(int* data, long long n) {
 // Sums of the segments; the last block turns them into their exclusive scan.
 __global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int* __restrict__ sums,
                                    int* ticket, const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int s = 0;
@@ -131,6 +132,7 @@ __global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int*
 // In-place exclusive scan of segment blockIdx.x, plus offset (*offsets)[blockIdx.x] if given.
 __global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* __restrict__ offsets,
                                 const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int vals[SCAN_V];
@@ -197,6 +199,7 @@ label_offsets_kernel(const int* __restrict__ hist, long long n, int k, int ntile
                      int* __restrict__ label_off, int* __restrict__ piece_cnt,
                      long long* __restrict__ counts, const int* __restrict__ dirty,
                      const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   block_label_offsets(hist, n, k, ntiles, label_off, piece_cnt, counts, dirty);
 }
@@ -212,6 +215,7 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
                             int ntiles, int* __restrict__ hist, int* err, int* label_off,
                             int* piece_cnt, long long* counts, const int* dirty, int* ticket,
                             const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   extern __shared__ int cnt_s[];
   const int tile = blockIdx.x;
@@ -263,6 +267,7 @@ __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int 
                                int ntiles, int* pos, int* __restrict__ sorted,
                                const int* __restrict__ dirty, const int* any_dirty,
                                const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   extern __shared__ int cnt_s[];
   const int tile = blockIdx.x;
@@ -317,6 +322,7 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
                                      int tile_pts, int ntiles, const int* __restrict__ pos,
                                      int* __restrict__ sorted, const int* __restrict__ dirty,
                                      const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   extern __shared__ int wcnt[];  // [kScatterWarps][k]
   const int tile = blockIdx.x;
@@ -430,6 +436,7 @@ __global__ void piece_sums_kernel(const float* __restrict__ X, long long ldx,
                                   int k, int d, double* __restrict__ part,
                                   double* __restrict__ partq, const int* any_dirty,
                                   const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   const int ptot = pstart[k];
   const int lane = threadIdx.x & 31;
@@ -580,6 +587,7 @@ piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double*
                        const int* __restrict__ sorted, const int* __restrict__ label_off,
                        const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
                        double* __restrict__ partq, const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   __shared__ __align__(16) float4 ring[kRingWarps][kRingStages][kRingRows][32];
   const long long ptot = pstart[k];
@@ -652,6 +660,7 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
                         const int* __restrict__ sorted, const int* __restrict__ label_off,
                         const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
                         double* __restrict__ partq, const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop) || idle(any_dirty)) return;
   constexpr int G = 32 / L;  // pieces per warp; also ids per lane and window
   constexpr int R = 16;      // rows per batch: one is summed while the next is in flight
@@ -749,22 +758,21 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
   const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
   const unsigned sblocks = (unsigned)((warps * 32 + 127) / 128);
   if (vec && lanes == 4)
-    piece_sums_small_kernel<4><<<sblocks, 128, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
+    launch(piece_sums_small_kernel<4>, sblocks, 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d,
                                                       part, partq, any, stop);
   else if (vec && lanes == 8)
-    piece_sums_small_kernel<8><<<sblocks, 128, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
+    launch(piece_sums_small_kernel<8>, sblocks, 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d,
                                                       part, partq, any, stop);
   else if (vec && lanes == 16)
-    piece_sums_small_kernel<16><<<sblocks, 128, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k,
+    launch(piece_sums_small_kernel<16>, sblocks, 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k,
                                                        d, part, partq, any, stop);
   else if (vec) {
     // four 4-warp blocks (48 KB of ring each) per SM
     const long long cap = kmgb::num_sms() * 4LL * kRingWarps;
     const long long rw = max_pieces < cap ? max_pieces : cap;
-    piece_sums_ring_kernel<<<(unsigned)((rw + kRingWarps - 1) / kRingWarps), kRingWarps * 32, 0,
-                             s>>>(X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, any, stop);
+    launch(piece_sums_ring_kernel, (unsigned)((rw + kRingWarps - 1) / kRingWarps), kRingWarps * 32, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, any, stop);
   } else
-    piece_sums_kernel<<<blocks, 256, 0, s>>>(X, ldx, qn, sorted, label_off, pstart, k, d,
+    launch(piece_sums_kernel, blocks, 256, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d,
                                                     part, partq, any, stop);
   kmgb::count_launches(1);
   return cudaGetLastError();
@@ -777,6 +785,7 @@ __global__ void __launch_bounds__(128)
 piece_sums_d_kernel(const double* __restrict__ X, long long ldx, const int* __restrict__ sorted,
                     const int* __restrict__ label_off, const int* __restrict__ pstart, int k, int d,
                     bool vec, double* __restrict__ part, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int chunks = (d + 63) / 64;
   const long long total = (long long)pstart[k] * chunks;
@@ -833,7 +842,7 @@ cudaError_t launch_piece_sums(const double* X, long long ldx, const UpdateWork& 
   const long long items = w.max_pieces * ((w.d + 63) / 64);
   const long long most = kmgb::num_sms() * 16LL;
   const long long warps = items < most ? items : most;
-  piece_sums_d_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(
+  launch(piece_sums_d_kernel, (unsigned)((warps + 3) / 4), 128, 0, s)(
       X, ldx, w.sorted, w.label_off, w.piece_cnt, w.k, w.d, vec, w.part, w.stop);
   kmgb::count_launches(1);
   return cudaGetLastError();
@@ -848,6 +857,7 @@ __global__ void finalize_kernel(const double* __restrict__ part, const double* _
                                 int k, int d, float* __restrict__ C, long long ldc,
                                 int empty_policy, double* __restrict__ sse_k,
                                 const int* __restrict__ dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int groups = (d + 31) / 32;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -908,6 +918,7 @@ __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
                                  const float* __restrict__ X, long long ldx,
                                  const int* __restrict__ sorted, const float* __restrict__ C,
                                  long long ldc, const int* __restrict__ dirty, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -960,6 +971,7 @@ __device__ __forceinline__ void store_sse(double sse, double* out, int* stop, do
 __global__ void __launch_bounds__(256)
 finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long long ldc,
                        int empty_policy, UpdateWork w, double* __restrict__ sse_out) {
+  if (grid_enter()) return;
   if (stopped(w.stop)) return;
   __shared__ double red[8];
   const int j = blockIdx.x;
@@ -1044,6 +1056,7 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
 __global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, double* __restrict__ out,
                                   int* stop, double criterion, double* sse_prev, double* rel_out,
                                   int* iters_done, int indexed) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   __shared__ double red[1024];
   const int per = (k + blockDim.x - 1) / blockDim.x;
@@ -1065,10 +1078,10 @@ cudaError_t excl_scan(int* data, long long n, int* tmp, int* ticket, cudaStream_
   const long long nb = (n + SCAN_SEG - 1) / SCAN_SEG;
   if (nb > SCAN_SEG) return cudaErrorInvalidValue;
   if (nb > 1) {
-    scan_reduce_kernel<<<(unsigned)nb, SCAN_T, 0, s>>>(data, n, tmp, ticket, any_dirty, stop);
+    launch(scan_reduce_kernel, (unsigned)nb, SCAN_T, 0, s)(data, n, tmp, ticket, any_dirty, stop);
     kmgb::count_launches(1);
   }
-  scan_seg_kernel<<<(unsigned)nb, SCAN_T, 0, s>>>(data, n, nb > 1 ? tmp : nullptr, any_dirty, stop);
+  launch(scan_seg_kernel, (unsigned)nb, SCAN_T, 0, s)(data, n, nb > 1 ? tmp : nullptr, any_dirty, stop);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
@@ -1098,19 +1111,19 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
   const size_t smem = sizeof(int) * (size_t)k;
   const bool small = hist_elems <= kSmallHist && smem <= 48 * 1024;
   if (small) {
-    hist_kernel<true, true><<<w.ntiles, SCAN_T, smem, s>>>(
+    launch(hist_kernel<true, true>, w.ntiles, SCAN_T, smem, s)(
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, w.label_off, w.piece_cnt, w.counts, w.dirty,
         w.tickets, w.any_dirty, w.stop);
   } else if (smem <= 96 * 1024) {
     if (smem > 48 * 1024)
       KMGB_CUDA_TRY(cudaFuncSetAttribute(hist_kernel<true, false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    hist_kernel<true, false><<<w.ntiles, 256, smem, s>>>(
+    launch(hist_kernel<true, false>, w.ntiles, 256, smem, s)(
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, nullptr, nullptr, nullptr, nullptr, nullptr,
         w.any_dirty, w.stop);
   } else {
     KMGB_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(int) * hist_elems, s));
-    hist_kernel<false, false><<<w.ntiles, 256, 0, s>>>(
+    launch(hist_kernel<false, false>, w.ntiles, 256, 0, s)(
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, nullptr, nullptr, nullptr, nullptr, nullptr,
         w.any_dirty, w.stop);
   }
@@ -1118,7 +1131,7 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
   KMGB_CUDA_TRY(cudaGetLastError());
   if (!small) {
     KMGB_CUDA_TRY(excl_scan(w.hist, hist_elems, w.scan_tmp, w.tickets, s, w.any_dirty, w.stop));
-    label_offsets_kernel<<<1, SCAN_T, 0, s>>>(w.hist, n, k, w.ntiles, w.label_off, w.piece_cnt, w.counts,
+    launch(label_offsets_kernel, 1, SCAN_T, 0, s)(w.hist, n, k, w.ntiles, w.label_off, w.piece_cnt, w.counts,
                                               w.dirty, w.any_dirty, w.stop);
     kmgb::count_launches(1);
     KMGB_CUDA_TRY(cudaGetLastError());
@@ -1128,17 +1141,17 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
     if (msmem > 48 * 1024)
       KMGB_CUDA_TRY(cudaFuncSetAttribute(scatter_multi_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    scatter_multi_kernel<<<w.ntiles, 32 * kScatterWarps, msmem, s>>>(
+    launch(scatter_multi_kernel, w.ntiles, 32 * kScatterWarps, msmem, s)(
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.sorted, w.dirty, w.any_dirty, w.stop);
     kmgb::count_launches(1);
   } else if (smem <= 96 * 1024) {
     if (smem > 48 * 1024)
       KMGB_CUDA_TRY(cudaFuncSetAttribute(scatter_kernel<true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    scatter_kernel<true><<<w.ntiles, 32, smem, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist,
+    launch(scatter_kernel<true>, w.ntiles, 32, smem, s)(labels, n, k, w.tile_pts, w.ntiles, w.hist,
                                                     w.sorted, w.dirty, w.any_dirty, w.stop); kmgb::count_launches(1);
   } else {
-    scatter_kernel<false><<<w.ntiles, 32, 0, s>>>(labels, n, k, w.tile_pts, w.ntiles, w.hist,
+    launch(scatter_kernel<false>, w.ntiles, 32, 0, s)(labels, n, k, w.tile_pts, w.ntiles, w.hist,
                                                   w.sorted, w.dirty, w.any_dirty, w.stop); kmgb::count_launches(1);
   }
   return cudaGetLastError();
@@ -1155,7 +1168,7 @@ cudaError_t launch_update(const float* X, const double* qn, const int* labels, f
                                      w.part, w.partq, w.any_dirty, w.stop, w.max_pieces, s));
   const int warps = std::min(8, (w.d + 31) / 32);
   if (w.centers_free) KMGB_CUDA_TRY(cudaStreamWaitEvent(s, w.centers_free, 0));
-  finalize_update_kernel<<<(unsigned)k, 32 * warps, 0, s>>>(X, C, ldc, empty_policy, w, sse_out);
+  launch(finalize_update_kernel, (unsigned)k, 32 * warps, 0, s)(X, C, ldc, empty_policy, w, sse_out);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
@@ -1167,6 +1180,7 @@ namespace {
 __global__ void accumulate_kernel(const double* __restrict__ part, const int* __restrict__ label_off,
                                   const int* __restrict__ pstart, int k, int d,
                                   double* __restrict__ acc, int* __restrict__ acc_counts) {
+  if (grid_enter()) return;
   const int groups = (d + 31) / 32;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -1199,6 +1213,7 @@ __global__ void accumulate_stream_kernel(const double* __restrict__ part,
                                          const int* __restrict__ pstart, int k, int d,
                                          double* __restrict__ accS, int* __restrict__ accN,
                                          double* __restrict__ accQ, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int j = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -1223,6 +1238,7 @@ __global__ void finalize_stream_kernel(const double* __restrict__ accS, const in
                                        const double* __restrict__ accQ, int k, int d,
                                        float* __restrict__ C, long long ldc, int empty_policy,
                                        double* __restrict__ sse_k, const int* stop) {
+  if (grid_enter()) return;
   if (stopped(stop)) return;
   const int groups = (d + 31) / 32;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1254,6 +1270,7 @@ template <typename T>
 __global__ void finalize_acc_kernel(const double* __restrict__ acc, const int* __restrict__ acc_counts,
                                     int k, int d, T* __restrict__ centers, int* __restrict__ counts,
                                     const int* __restrict__ dirty) {
+  if (grid_enter()) return;
   const long long total = (long long)k * d;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
@@ -1281,7 +1298,7 @@ cudaError_t launch_tile_accumulate(const T* X, long long ldx, const int* labels,
   KMGB_CUDA_TRY(sort_by_label(labels, w, s));
   KMGB_CUDA_TRY(launch_piece_sums(X, ldx, w, s));
   const long long acc_warps = (long long)w.k * ((w.d + 31) / 32);
-  accumulate_kernel<<<(unsigned)((acc_warps * 32 + 255) / 256), 256, 0, s>>>(
+  launch(accumulate_kernel, (unsigned)((acc_warps * 32 + 255) / 256), 256, 0, s)(
       w.part, w.label_off, w.piece_cnt, w.k, w.d, acc, acc_counts); kmgb::count_launches(1);
   return cudaGetLastError();
 }
@@ -1289,7 +1306,7 @@ cudaError_t launch_tile_accumulate(const T* X, long long ldx, const int* labels,
 template <typename T>
 cudaError_t launch_finalize_acc(const double* acc, const int* acc_counts, int k, int d, T* centers,
                                 int* counts, cudaStream_t s, const int* dirty) {
-  finalize_acc_kernel<T><<<kmgb::num_sms() * 4, 256, 0, s>>>(acc, acc_counts, k, d, centers, counts,
+  launch(finalize_acc_kernel<T>, kmgb::num_sms() * 4, 256, 0, s)(acc, acc_counts, k, d, centers, counts,
                                                              dirty);
   kmgb::count_launches(1);
   return cudaGetLastError();
@@ -1302,7 +1319,7 @@ cudaError_t launch_stream_accumulate(const float* X, long long ldx, const double
   KMGB_CUDA_TRY(sort_by_label(labels, w, s));
   KMGB_CUDA_TRY(launch_piece_sums_f32(X, w.ldx, qn, w.sorted, w.label_off, w.piece_cnt, w.k, w.d,
                                      w.part, w.partq, nullptr, w.stop, w.max_pieces, s));
-  accumulate_stream_kernel<<<(unsigned)(((long long)w.k * 32 + 255) / 256), 256, 0, s>>>(
+  launch(accumulate_stream_kernel, (unsigned)(((long long)w.k * 32 + 255) / 256), 256, 0, s)(
       w.part, w.partq, w.label_off, w.piece_cnt, w.k, w.d, accS, accN, accQ, w.stop);
   kmgb::count_launches(1);
   return cudaGetLastError();
@@ -1313,11 +1330,11 @@ cudaError_t launch_stream_finalize(const double* accS, const int* accN, const do
                                    double* sse_out, cudaStream_t s) {
   const int k = w.k;
   const long long fin_warps = (long long)k * ((w.d + 31) / 32);
-  finalize_stream_kernel<<<(unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s>>>(
+  launch(finalize_stream_kernel, (unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s)(
       accS, accN, accQ, k, w.d, C, ldc, empty_policy, w.sse_k, w.stop);
   kmgb::count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  sse_reduce_kernel<<<1, 1024, 0, s>>>(w.sse_k, (int)fin_warps, sse_out, w.stop, w.criterion,
+  launch(sse_reduce_kernel, 1, 1024, 0, s)(w.sse_k, (int)fin_warps, sse_out, w.stop, w.criterion,
                                        w.sse_prev, w.rel_out, w.iters_done, w.sse_indexed);
   kmgb::count_launches(1);
   return cudaGetLastError();
@@ -1344,6 +1361,7 @@ namespace {
 
 __global__ void hist_batched_kernel(const int* __restrict__ labels, BatchUpdate b,
                                     int* __restrict__ hist, int* err) {
+  if (grid_enter()) return;
   const long long st = blockIdx.x;
   const int prob = b.stile_prob[st];
   const int tl = b.stile_local[st];
@@ -1375,6 +1393,7 @@ __global__ void label_offsets_batched_kernel(const int* __restrict__ hist, Batch
                                              int* __restrict__ label_off, int* __restrict__ piece_cnt,
                                              long long* __restrict__ counts,
                                              const int* __restrict__ dirty) {
+  if (grid_enter()) return;
   const int gc = blockIdx.x * blockDim.x + threadIdx.x;
   if (gc > b.K) return;
   auto start = [&](int c) -> int {
@@ -1397,6 +1416,7 @@ __global__ void label_offsets_batched_kernel(const int* __restrict__ hist, Batch
 template <bool SMEM>
 __global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpdate b, int* pos,
                                        int* __restrict__ sorted, const int* __restrict__ dirty) {
+  if (grid_enter()) return;
   extern __shared__ int cnt_s[];
   const long long st = blockIdx.x;
   const int prob = b.stile_prob[st];
@@ -1442,6 +1462,7 @@ __global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpda
 // The problem's SSE history slot is its own count of recorded iterations (a stopped problem
 // records nothing more), so every iteration issues the same launch: a CUDA graph replays it.
 __global__ void sse_batched_kernel(const double* __restrict__ sse_k, int groups, BatchUpdate b) {
+  if (grid_enter()) return;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= b.P) return;
@@ -1470,20 +1491,20 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
                                   const UpdateWork& w, const BatchUpdate& b, cudaStream_t s) {
   if (b.P <= 0 || b.K <= 0 || b.n_valid <= 0) return cudaSuccess;
   KMGB_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(int) * b.hist_elems, s));
-  hist_batched_kernel<<<(unsigned)b.stiles, 256, 0, s>>>(labels, b, w.hist, w.err);
+  launch(hist_batched_kernel, (unsigned)b.stiles, 256, 0, s)(labels, b, w.hist, w.err);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.hist, b.hist_elems, w.scan_tmp, w.tickets, s, nullptr, nullptr));
-  label_offsets_batched_kernel<<<(b.K + 1 + 255) / 256, 256, 0, s>>>(w.hist, b, w.label_off,
+  launch(label_offsets_batched_kernel, (b.K + 1 + 255) / 256, 256, 0, s)(w.hist, b, w.label_off,
                                                                     w.piece_cnt, w.counts, w.dirty);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.piece_cnt, b.K + 1, w.scan_tmp, w.tickets, s, nullptr, nullptr));
   if (b.kmax <= 12288)
-    scatter_batched_kernel<true><<<(unsigned)b.stiles, 32, sizeof(int) * (size_t)b.kmax, s>>>(
+    launch(scatter_batched_kernel<true>, (unsigned)b.stiles, 32, sizeof(int) * (size_t)b.kmax, s)(
         labels, b, w.hist, w.sorted, w.dirty);
   else
-    scatter_batched_kernel<false><<<(unsigned)b.stiles, 32, 0, s>>>(labels, b, w.hist, w.sorted,
+    launch(scatter_batched_kernel<false>, (unsigned)b.stiles, 32, 0, s)(labels, b, w.hist, w.sorted,
                                                                     w.dirty);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
@@ -1491,17 +1512,17 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
                                      w.part, w.partq, nullptr, nullptr, w.max_pieces, s));
   const int groups = (d + 31) / 32;
   const long long fin_warps = (long long)b.K * groups;
-  finalize_kernel<<<(unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s>>>(
+  launch(finalize_kernel, (unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s)(
       w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, w.dirty,
       nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  sse_fixup_kernel<<<(unsigned)((b.K * 32LL + 255) / 256), 256, 0, s>>>(
+  launch(sse_fixup_kernel, (unsigned)((b.K * 32LL + 255) / 256), 256, 0, s)(
       w.sse_k, groups, w.partq, w.label_off, w.piece_cnt, b.K, d, X, ldx, w.sorted, C, ldc,
       w.dirty, nullptr);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  sse_batched_kernel<<<(unsigned)((b.P * 32LL + 255) / 256), 256, 0, s>>>(w.sse_k, groups, b);
+  launch(sse_batched_kernel, (unsigned)((b.P * 32LL + 255) / 256), 256, 0, s)(w.sse_k, groups, b);
   count_launches(1);
   return cudaGetLastError();
 }
