@@ -923,6 +923,68 @@ cudaError_t launch_piece_sums(const double* X, long long ldx, const UpdateWork& 
   return cudaGetLastError();
 }
 
+// (double)f from its bits: GB300's FP64 pipe, conversions included, takes a warp 16 cycles per
+// instruction. A subnormal, infinite or NaN f is converted there.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u && m != 0) return (double)f;
+  const unsigned h = m ? (m >> 3) + 0x38000000u : 0u;
+  return __hiloint2double((int)((u & 0x80000000u) | h), (int)(u << 29));
+}
+
+// 1 / n by Newton's iteration from the FP32 reciprocal (relative errors 2^-23, 2^-46, 2^-52).
+__device__ __forceinline__ double reciprocal_of_count(int n, double nd) {
+  double r = widen(__frcp_rn((float)n));
+  r = fma(r, fma(-nd, r, 1.0), r);
+  return fma(r, fma(-nd, r, 1.0), r);
+}
+
+// A center's coordinate: the FP64 quotient s / n rounded to FP32. s times the reciprocal is within 3
+// units in the last place of that quotient, so it rounds to the same FP32 number unless it lies within
+// 8 of the middle between two; only there, and outside FP32's normal range, the division itself (some
+// twenty FP64 instructions) runs.
+__device__ __forceinline__ float mean_rn(double s, double nd, double rn) {
+  const double q = s * rn;
+  const long long b = __double_as_longlong(q);
+  const unsigned ex = (unsigned)(b >> 52) & 0x7ffu, low = (unsigned)b & 0x1fffffffu;
+  if ((b << 1) == 0) return __int_as_float((int)(b >> 32));  // a zero of s's sign
+  if (ex - 897u > 252u || low - 0x0ffffff8u <= 16u) return __double2float_rn(__ddiv_rn(s, nd));
+  const unsigned m = (unsigned)(b >> 29);  // 23 bits of significand, the exponent above (modulo 512)
+  return __uint_as_float(((unsigned)(b >> 32) & 0x80000000u) |
+                         (m - (896u << 23) + (low > 0x10000000u ? 1u : 0u)));
+}
+
+// Half of a dimension's share n mu^2 - 2 mu s of the SSE identity.
+__device__ __forceinline__ double half_sse_share(float mu, double s, double nd) {
+  const double m = widen(mu);
+  return m * fma(0.5 * nd, m, -s);
+}
+
+// A center's piece sums of one dimension (part[p * d], p0 <= p < p1) added in piece order, U loads
+// in flight. An addition runs only where there is a piece (the empty statement keeps the compiler from
+// running all of them and selecting): the FP64 pipe is what bounds the kernels that call this.
+template <int U>
+__device__ __forceinline__ double sum_pieces_by(const double* __restrict__ part, int d, int p0, int p1) {
+  double s = 0.0;
+  for (int p = p0; p < p1; p += U) {
+    double v[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+      if (p + i < p1) v[i] = __ldg(part + (size_t)(p + i) * d);
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+      if (p + i >= p1) break;
+      asm volatile("" : "+d"(s));
+      s += v[i];
+    }
+  }
+  return s;
+}
+
+__device__ __forceinline__ double sum_pieces(const double* __restrict__ part, int d, int p0, int p1) {
+  return p1 - p0 <= 4 ? sum_pieces_by<4>(part, d, p0, p1) : sum_pieces_by<16>(part, d, p0, p1);
+}
+
 // One warp per (center j, group g of 32 dimensions): lane c of group g owns dimension
 // g*32 + c, adds the center's piece sums in piece order (the canonical order: centers are
 // unchanged by the split), divides in FP64 and rounds once. The group's SSE term
@@ -941,25 +1003,16 @@ __global__ void finalize_kernel(const double* __restrict__ part, const double* _
   const int j = (int)(wid / groups), g = (int)(wid - (long long)j * groups);
   if (dirty && !dirty[j]) return;
   const int c = g * 32 + lane;
-  const long long n = (long long)label_off[j + 1] - label_off[j];
+  const int n = label_off[j + 1] - label_off[j];
   const int p0 = pstart[j], p1 = pstart[j + 1];
   double sse = 0.0;
   if (c < d) {
-    double s = 0.0;
-    int p = p0;
-    for (; p + 8 <= p1; p += 8) {  // eight loads in flight, additions in piece order
-      double v[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = __ldg(part + (size_t)(p + i) * d + c);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s += v[i];
-    }
-    for (; p < p1; ++p) s += __ldg(part + (size_t)p * d + c);
+    const double s = sum_pieces(part + c, d, p0, p1);
     float mu;
     if (n > 0) {
-      mu = __double2float_rn(__ddiv_rn(s, (double)n));
-      const double m = (double)mu;
-      sse = fma((double)n * m, m, -2.0 * m * s);
+      const double nd = (double)n;
+      mu = mean_rn(s, nd, reciprocal_of_count(n, nd));
+      sse = 2.0 * half_sse_share(mu, s, nd);
     } else if (empty_policy == 1) {
       mu = C[(size_t)j * ldc + c];
     } else {
@@ -1025,77 +1078,90 @@ __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
 
 // The iteration's SSE and the loop's stop rule (kmeans.cpp:1234-1237,1194): relErr = |SSE - SSE_old| /
 // |SSE|; the run stops once !(relErr > criterion), NaN included.
-__device__ __forceinline__ void store_sse(double sse, double* out, int* stop, double criterion,
-                                          double* sse_prev, double* rel_out, int* iters_done,
-                                          int indexed) {
-  if (indexed && iters_done) out[*iters_done] = sse;
+// Its inputs are loaded with the caller's first loads (load_loop): one after the other between the
+// stores they cost three round trips.
+struct LoopIn {
+  int it = 0;
+  double prev = 0.0;
+};
+__device__ __forceinline__ LoopIn load_loop(const int* iters_done, const double* sse_prev) {
+  LoopIn l;
+  if (iters_done) l.it = *iters_done;
+  if (sse_prev) l.prev = *sse_prev;
+  return l;
+}
+__device__ __forceinline__ void store_sse(double sse, const LoopIn& l, double* out, int* stop,
+                                          double criterion, double* sse_prev, double* rel_out,
+                                          int* iters_done, int indexed) {
+  if (indexed && iters_done) out[l.it] = sse;
   else *out = sse;
   if (sse_prev) {
-    const double rel = fabs(sse - *sse_prev) / fabs(sse);
+    const double rel = fabs(sse - l.prev) / fabs(sse);
     *sse_prev = sse;
     *rel_out = rel;
-    *iters_done += 1;
+    *iters_done = l.it + 1;
     if (stop && !(rel > criterion)) *stop = 1;
   }
 }
 
-// The single-problem update's last step, one block per center, a warp per group of 32 dimensions: the
-// center and its SSE term as in finalize_kernel and sse_fixup_kernel (the center's groups added in
-// order), then the last block adds the centers' terms (strided chains, a tree) and evaluates the
-// stop rule as sse_reduce_kernel does: one launch instead of three.
+// The single-problem update's last step, a block per center and step, a warp per group of 32 dimensions:
+// the center as in finalize_kernel, and its SSE with the cancelled clusters' direct form as in
+// sse_fixup_kernel; then the last block adds the centers' terms (strided chains, a tree) and evaluates
+// the stop rule as sse_reduce_kernel does: one launch instead of three. Bound by the latency of its
+// chain of loads where centers are few, so what does not depend on each other is loaded together
+// (64 x 32: 12.0 -> 10.0 us; 256 x 128: 12.2 -> 10.4), and by the FP64 pipe (2 lanes a cycle) where they
+// are many, so the lanes' terms meet in shared memory, a block runs one tree for them and one for the
+// norms, quotients avoid the division and a block takes several centers before its fence and ticket
+// (16,384 x 256: 268 -> 192 us).
 __global__ void __launch_bounds__(256)
 finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long long ldc,
                        int empty_policy, UpdateWork w, double* __restrict__ sse_out) {
   if (grid_enter()) return;
   if (stopped(w.stop)) return;
-  __shared__ double red[8];
-  const int j = blockIdx.x;
+  __shared__ double red[256];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int d = w.d;
-  if (!w.dirty || w.dirty[j]) {  // uniform over the block
-    const int groups = (d + 31) / 32;
+  const int groups = (d + 31) / 32;
+  LoopIn loop;  // (written by the last block only, at its end)
+  if (threadIdx.x == 0) loop = load_loop(w.iters_done, w.sse_prev);
+  for (int j = blockIdx.x; j < w.k; j += gridDim.x) {
+    const int live = w.dirty ? w.dirty[j] : 1;  // uniform over the block
     const int m0 = w.label_off[j], m1 = w.label_off[j + 1];
-    const long long n = m1 - m0;
     const int p0 = w.piece_cnt[j], p1 = w.piece_cnt[j + 1];
-    double tot = 0.0;
+    if (!live) continue;
+    // the members' sum of ||x||^2: the last warp's lanes over the pieces, the first ones ahead
+    double q = 0.0;
+    if (wp == warps - 1 && p0 + lane < p1) q = __ldg(w.partq + p0 + lane);
+    const int n = m1 - m0;
+    const double nd = (double)n, rn = reciprocal_of_count(n > 0 ? n : 1, nd);
+    double half = 0.0;  // of the lane's share of n mu^2 - 2 mu s
     for (int g = wp; g < groups; g += warps) {
       const int c = g * 32 + lane;
-      double sse = 0.0;
-      if (c < d) {
-        double s = 0.0;
-        for (int p = p0; p < p1; p += 8) {  // eight loads in flight, additions in piece order
-          double v[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = p + i < p1 ? __ldg(w.part + (size_t)(p + i) * d + c) : 0.0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) s += v[i];
-        }
-        float mu;
-        if (n > 0) {
-          mu = __double2float_rn(__ddiv_rn(s, (double)n));
-          const double m = (double)mu;
-          sse = fma((double)n * m, m, -2.0 * m * s);
-        } else if (empty_policy == 1) {
-          mu = C[(size_t)j * ldc + c];
-        } else {
-          mu = __int_as_float(0x7fc00000);
-        }
-        C[(size_t)j * ldc + c] = mu;
+      if (c >= d) continue;
+      const double s = sum_pieces(w.part + c, d, p0, p1);
+      float mu;
+      if (n > 0) {
+        mu = mean_rn(s, nd, rn);
+        half += half_sse_share(mu, s, nd);
+      } else if (empty_policy == 1) {
+        mu = C[(size_t)j * ldc + c];
+      } else {
+        mu = __int_as_float(0x7fc00000);
       }
-      for (int o = 16; o > 0; o >>= 1) sse += __shfl_xor_sync(0xffffffffu, sse, o);
-      tot += sse;
+      C[(size_t)j * ldc + c] = mu;
     }
-    // the members' sum of ||x||^2: the last warp, lanes over the pieces, a tree
-    double q = 0.0;
-    if (wp == warps - 1) {
-      for (int p = p0 + lane; p < p1; p += 32) q += __ldg(w.partq + p);
-      for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-    }
-    if (lane == 0) red[wp] = tot;
+    red[threadIdx.x] = half;
+    if (wp == warps - 1)
+      for (int p = p0 + 32 + lane; p < p1; p += 32) q += __ldg(w.partq + p);
     __syncthreads();  // and the center's dimensions are written
     if (wp == warps - 1) {
-      double t = q;
-      for (int i = 0; i < warps; ++i) t += red[i];
+      double t = 0.0;
+      for (int i = 0; i < warps; ++i) t += red[32 * i + lane];
+      for (int o = 16; o > 0; o >>= 1) {
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+        q += __shfl_xor_sync(0xffffffffu, q, o);
+      }
+      t = fma(2.0, t, q);
       if (n > 0 && fabs(t) <= 1e-9 * q) {
         // cancelled: the direct form (see sse_fixup_kernel)
         const float* mu = C + (size_t)j * ldc;
@@ -1111,19 +1177,19 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
       }
       if (lane == 0) w.sse_k[j] = n > 0 ? t : 0.0;
     }
+    __syncthreads();  // red serves the next center
   }
   if (!last_block(w.tickets)) return;
   double s = 0.0;
 #pragma unroll 4
   for (int i = threadIdx.x; i < w.k; i += blockDim.x) s += __ldcg(w.sse_k + i);
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __syncthreads();
   if (lane == 0) red[wp] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     double sse = 0.0;
     for (int i = 0; i < warps; ++i) sse += red[i];
-    store_sse(sse, sse_out, w.stop, w.criterion, w.sse_prev, w.rel_out, w.iters_done, w.sse_indexed);
+    store_sse(sse, loop, sse_out, w.stop, w.criterion, w.sse_prev, w.rel_out, w.iters_done, w.sse_indexed);
   }
 }
 
@@ -1134,6 +1200,8 @@ __global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, doubl
   if (grid_enter()) return;
   if (stopped(stop)) return;
   __shared__ double red[1024];
+  LoopIn loop;
+  if (threadIdx.x == 0) loop = load_loop(iters_done, sse_prev);
   const int per = (k + blockDim.x - 1) / blockDim.x;
   double s = 0.0;
   for (int j = threadIdx.x * per; j < min(k, (int)(threadIdx.x + 1) * per); ++j) s += sse_k[j];
@@ -1144,7 +1212,7 @@ __global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, doubl
     __syncthreads();
   }
   if (threadIdx.x == 0)
-    store_sse(red[0], out, stop, criterion, sse_prev, rel_out, iters_done, indexed);
+    store_sse(red[0], loop, out, stop, criterion, sse_prev, rel_out, iters_done, indexed);
 }
 
 cudaError_t excl_scan(int* data, long long n, int* tmp, int* ticket, cudaStream_t s,
@@ -1244,7 +1312,8 @@ cudaError_t launch_update(const float* X, const double* qn, const int* labels, f
                                      w.part, w.partq, w.any_dirty, w.stop, w.max_pieces, s));
   const int warps = std::min(8, (w.d + 31) / 32);
   if (w.centers_free) KMGB_CUDA_TRY(cudaStreamWaitEvent(s, w.centers_free, 0));
-  launch(finalize_update_kernel, (unsigned)k, 32 * warps, 0, s)(X, C, ldc, empty_policy, w, sse_out);
+  const int most = kmgb::num_sms() * (64 / warps);  // blocks the SMs hold at a time
+  launch(finalize_update_kernel, (unsigned)std::min(k, most), 32 * warps, 0, s)(X, C, ldc, empty_policy, w, sse_out);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
