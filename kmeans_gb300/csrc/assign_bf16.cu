@@ -344,8 +344,13 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     if (tid == 0 && blockIdx.x == 0) set_error(p.err, KMGB_DEV_BAD_SHAPE);
     return;
   }
-  const bool stop_now = stopped(p.stop);  // uniform: every CTA of the grid sees the same flag
-  if (stop_now) return;
+  // uniform: every CTA of the grid sees the same flag and counts
+  constexpr bool kSel = !F8 && !XMAX;
+  const int halt = p.stop ? pinned(p.stop) : 0;
+  const int units_in = p.n_units_dev ? pinned(p.n_units_dev) : 1;
+  const int rows_in = p.n_dev ? pinned(p.n_dev) : 0;
+  const int sel_in = kSel && p.sel ? pinned(p.sel) : 0;
+  if (halt) return;
   // The two-plane variant (EPQ 2) runs the split modes 2 and 3 only; the plain BF16 tier, the FP8
   // tier and the store mode run with EPQ 4, so their code is compiled out of the split variant
   // (it kept the split epilogue from spilling).
@@ -358,20 +363,19 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   // rows of this launch: [row0, row0 + n_rows); a device count bounds them in candidate mode
   long long n_rows = p.n;
   if (p.n_units_dev) {
-    const int c = *p.n_units_dev;
+    const int c = units_in;
     if (c <= 0) return;  // uniform over the grid, before any barrier or TMEM allocation
     n_rows = (long long)c * UNIT;
   } else if (p.n_dev) {
-    const long long c = (long long)*p.n_dev - p.row0;
+    const long long c = (long long)rows_in - p.row0;
     if (c <= 0) return;  // uniform over the grid, before any barrier or TMEM allocation
     n_rows = c < p.n ? c : p.n;
   }
   // rows selected by their distance bounds: the compact copy of the listed rows, or all rows
   // when more than its capacity are listed
-  constexpr bool kSel = !F8 && !XMAX;
   bool compact = false;
   if (kSel && p.sel) {
-    const int c = *p.sel;
+    const int c = sel_in;
     compact = c <= p.sel_cap;
     if (c == 0) return;
     if (compact) n_rows = c;

@@ -215,7 +215,7 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
   if (grid_enter()) return;
   if (stopped(stop)) return;
   if (IDX == 1) {
-    const long long total = *reinterpret_cast<volatile const int*>(rl.count);
+    const long long total = pinned(rl.count);
     const long long cap = n;
     n = total < cap ? total : cap;
     for (long long i = cap + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;

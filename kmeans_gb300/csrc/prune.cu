@@ -181,8 +181,9 @@ prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* st
 __global__ void prune_gather_kernel(PruneState ps, const uint4* __restrict__ Xb,
                                     const uint4* __restrict__ Xl, int row_vec, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop)) return;
-  const int cnt = ps.flags[1];
+  const int halt = stop ? pinned(stop) : 0;
+  const int cnt = pinned(ps.flags + 1);
+  if (halt) return;
   if (cnt > ps.cap) return;
   const int lane = threadIdx.x & 31;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -226,8 +227,9 @@ constexpr int kDirtyShared = 32768;
 __global__ void __launch_bounds__(1024)
 prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop)) return;
-  const int cnt = ps.flags[1];
+  const int halt = stop ? pinned(stop) : 0;
+  const int cnt = pinned(ps.flags + 1);
+  if (halt) return;
   if (cnt == 0) return;
   extern __shared__ unsigned char mark[];
   const bool sh = ps.k <= kDirtyShared;

@@ -20,6 +20,8 @@
 #include <cfloat>
 #include <cstdint>
 
+#include <cmath>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -61,7 +63,7 @@ __global__ void rerank_kernel(RerankArgs a) {
   const int warps = blockDim.x >> 5;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* xs = xs_all + (size_t)w * a.d;
-  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  const long long cnt = min((long long)pinned(a.count), a.max_list);
   const float u = 5.9604645e-8f;
   const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;  // mode 0 relative bound (doubled)
   for (long long slot = (long long)blockIdx.x * warps + w; slot < cnt;
@@ -311,7 +313,9 @@ __global__ void __launch_bounds__(256)
 rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ count2,
                     float* __restrict__ hi2) {
   if (grid_enter()) return;
-  if (stopped(a.stop)) return;
+  const int halt = a.stop ? pinned(a.stop) : 0;
+  const long long cnt = min((long long)pinned(a.count), a.max_list);
+  if (halt) return;
   extern __shared__ float4 sm4[];
   const int dq = (a.d + 3) >> 2;          // float4 per row
   const int rs = (dq + 1) | 1;            // row stride in float4, odd: 8 consecutive rows' columns
@@ -325,7 +329,6 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int pq = tid & 7;                 // points pq, pq + 8, pq + 16, pq + 24
   const int cq = tid >> 3;                // centers cq*2, cq*2+1 of the block
-  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
   if (a.counts && a.stats && blockIdx.x == 0 && tid == 0) {
     a.stats[0] += (unsigned long long)a.counts[0];
     a.stats[1] += (unsigned long long)a.counts[a.full_idx];
@@ -494,7 +497,7 @@ rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict
   __shared__ float hs[TP];
   __shared__ float es[TP];  // MODE 1: the point's bound
   const int tid = threadIdx.x;
-  long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  long long cnt = min((long long)pinned(a.count), a.max_list);
   if (RECORD && cnt > cand_cap) {
     for (long long slot = cand_cap + (long long)blockIdx.x * blockDim.x + tid; slot < cnt;
          slot += (long long)gridDim.x * blockDim.x) {
@@ -549,7 +552,7 @@ rerank_grouped_kernel(RerankArgs a, GroupArgs g, int* __restrict__ cand, int* __
   extern __shared__ float rg_smem[];  // [warps][RG_VCAP] values, then [warps][ds] rows
   constexpr int G = 32 / L;           // centers side by side
   constexpr int U = 4;                // and in turn, their loads in flight together
-  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  const long long cnt = min((long long)pinned(a.count), a.max_list);
   const float u = 5.9604645e-8f;
   const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -667,8 +670,9 @@ __global__ void gather_flagged_kernel(const int* __restrict__ list, const int* _
                                       const int* stop, const float* __restrict__ xs,
                                       float* __restrict__ xsC) {
   if (grid_enter()) return;
-  if (stopped(stop)) return;
-  const long long total = *(volatile const int*)count;
+  const int halt = stop ? pinned(stop) : 0;
+  const long long total = pinned(count);
+  if (halt) return;
   const long long cnt = min(total, cap);
   const int lane = threadIdx.x & 31;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -803,6 +807,27 @@ __device__ __forceinline__ float f32_dist8(const float* __restrict__ x, const fl
 // values) the point's candidates are evaluated exactly as the oracle does, one lane per
 // candidate, in FP64. Points with more candidates than recorded (or none) go to `over` for the
 // full re-rank.
+// The tolerances, computed on the host, the first tier's as FP32 numbers rounded up: GB300's FP64 pipe
+// takes a warp 16 cycles an instruction. Twenty of them per warp of the grid, most of which find no
+// point, and as many per point in the first tier were the kernel's time (1M x 256, K=16,384: 172 us an
+// iteration).
+struct ResolveTol {
+  double rel, abs_tol;
+  float rel32, twice_abs32;
+};
+ResolveTol resolve_tolerances(int d) {
+  const double m = 4.0 * (double)((d + 31) / 32);
+  const double m32 = (double)((d + kGroupLanes - 1) / kGroupLanes);
+  ResolveTol t;
+  t.rel = 8.0 * ((m + 1.0) * (m + 1.0) + 2.0 + 3.0 * (m + 6.0)) * 0x1p-47 + (double)(d + 2) * 0x1p-52;
+  t.abs_tol = (double)(d + 32) * 0x1p-118;
+  const double rel32 = 1.1 * (m32 + 8.0) * 0x1p-24 + (double)(d + 2) * 0x1p-52;
+  const double abs32 = (double)(d + 32) * (m32 + 8.0) * 0x1p-149;
+  t.rel32 = std::nextafter((float)rel32, INFINITY);
+  t.twice_abs32 = std::nextafter((float)(2.0 * abs32), INFINITY);
+  return t;
+}
+
 template <bool VEC>
 __global__ void resolve_candidates_kernel(const int* __restrict__ list, const int* __restrict__ count,
                                           long long max_list, const int* __restrict__ cand,
@@ -814,22 +839,16 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
                                           int* __restrict__ over_count, const int* stop,
                                           const int* __restrict__ row_map,
                                           const float* __restrict__ hi_in,
-                                          float* __restrict__ over_hi) {
+                                          float* __restrict__ over_hi, ResolveTol tol) {
   if (grid_enter()) return;
-  if (stopped(stop)) return;
-  const long long cnt = min((long long)*(volatile const int*)count, max_list);
+  const int halt = stop ? pinned(stop) : 0;
+  const long long cnt = min((long long)pinned(count), max_list);
+  if (halt || cnt <= 0) return;
   const int lane = threadIdx.x & 31;
   const int grp = lane / kGroupLanes, sub = lane % kGroupLanes;
   constexpr int kGroups = 32 / kGroupLanes;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  const double m = 4.0 * (double)((d + 31) / 32);
-  const double rel = 8.0 * ((m + 1.0) * (m + 1.0) + 2.0 + 3.0 * (m + 6.0)) * 0x1p-47 +
-                     (double)(d + 2) * 0x1p-52;
-  const double abs_tol = (double)(d + 32) * 0x1p-118;
-  const double m32 = (double)((d + kGroupLanes - 1) / kGroupLanes);
-  const double rel32 = 1.1 * (m32 + 8.0) * 0x1p-24 + (double)(d + 2) * 0x1p-52;
-  const double abs32 = (double)(d + 32) * (m32 + 8.0) * 0x1p-149;
   // a point this kernel cannot settle, with its band's upper end where the list carries them
   auto to_over = [&](int pt, long long slot) {
     const int o = atomicAdd(over_count, 1);
@@ -851,41 +870,36 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
     const int myj = lane < nc ? cand[ci * kMaxCand + lane] : -1;
     const int myok = (myj >= 0 && cn[myj] < INFINITY) ? 1 : 0;
     // both fast tiers certify only a strict separation, so the list order (column slice by
-    // column slice) does not matter
-    double v1 = INFINITY, v2 = INFINITY;
-    int i1 = -1;
-    bool finite = true;
+    // column slice) does not matter. First tier: lane q ends with candidate q's value; values are
+    // non-negative, so their bits order as they do
+    float mv = INFINITY;
     for (int q0 = 0; q0 < nc; q0 += kGroups) {
       const int q = q0 + grp;  // <= 31: q0 is a multiple of 4 below nc <= kMaxCand = 32
       const int j = __shfl_sync(0xffffffffu, myj, q);
       const int ok = __shfl_sync(0xffffffffu, myok, q) && q < nc;
       const float v = f32_dist8<VEC>(x, ok ? C + (size_t)j * ldc : x, ok ? d : 0, sub);
-      for (int g = 0; g < kGroups; ++g) {
-        const double vg = (double)__shfl_sync(0xffffffffu, v, g * kGroupLanes);
-        const int jg = __shfl_sync(0xffffffffu, j, g * kGroupLanes);
-        if (!__shfl_sync(0xffffffffu, ok, g * kGroupLanes)) continue;
-        if (!(vg < 3.0e38)) finite = false;  // overflow, inf or NaN
-        if (vg < v1) {
-          v2 = v1;
-          v1 = vg;
-          i1 = jg;
-        } else if (vg < v2) {
-          v2 = vg;
-        }
-      }
+      const float vq = __shfl_sync(0xffffffffu, v, (lane - q0) % kGroups * kGroupLanes);
+      if (lane >= q0 && lane < q0 + kGroups) mv = vq;
     }
-    if (i1 < 0) {  // no usable candidate
+    if (!__any_sync(0xffffffffu, myok)) {  // no usable candidate
       if (lane == 0) to_over(pt, slot);
       continue;
     }
-    // one usable candidate (v2 infinite, its value finite) is the arg-min itself
-    if (finite && (v2 == INFINITY || v2 - v1 > (v1 + v2) * rel32 + 2.0 * abs32)) {
-      if (lane == 0) labels[pt] = i1;
+    bool finite = !__any_sync(0xffffffffu, myok && !(mv < 3.0e38f));  // overflow, inf or NaN
+    const unsigned bits = __float_as_uint(myok && finite ? mv : INFINITY);
+    const unsigned b1 = __reduce_min_sync(0xffffffffu, bits);
+    const int at = __ffs(__ballot_sync(0xffffffffu, bits == b1)) - 1;
+    const unsigned b2 = __reduce_min_sync(0xffffffffu, lane == at ? 0x7f800000u : bits);
+    // one usable candidate (the second infinite, its own value finite) is the arg-min itself
+    const float f1 = __uint_as_float(b1), f2 = __uint_as_float(b2);
+    if (finite &&
+        (f2 == INFINITY ||
+         __fsub_rd(f2, f1) > __fmaf_ru(__fadd_ru(f1, f2), tol.rel32, tol.twice_abs32))) {
+      if (lane == at) labels[pt] = myj;
       continue;
     }
-    v1 = INFINITY;
-    v2 = INFINITY;
-    i1 = -1;
+    double v1 = INFINITY, v2 = INFINITY;
+    int i1 = -1;
     finite = true;
     for (int q0 = 0; q0 < nc; q0 += kGroups) {
       const int q = q0 + grp;  // <= 31: q0 is a multiple of 4 below nc <= kMaxCand = 32
@@ -914,7 +928,7 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
     }
     // one usable candidate (v2 infinite, every value finite) is the arg-min itself; the
     // comparison below would read inf > inf
-    if (finite && (v2 == INFINITY || v2 - v1 > (v1 + v2) * rel + 2.0 * abs_tol)) {
+    if (finite && (v2 == INFINITY || v2 - v1 > (v1 + v2) * tol.rel + 2.0 * tol.abs_tol)) {
       if (lane == 0) labels[pt] = i1;
       continue;
     }
@@ -999,7 +1013,7 @@ __global__ void resolve_expansion_kernel(RerankArgs a, const int* __restrict__ c
                                          const int* __restrict__ cand_cnt, int* __restrict__ over,
                                          int* __restrict__ over_count) {
   if (grid_enter()) return;
-  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  const long long cnt = min((long long)pinned(a.count), a.max_list);
   const int lane = threadIdx.x & 31;
   const int grp = lane / kGroupLanes, sub = lane % kGroupLanes;
   constexpr int kGroups = 32 / kGroupLanes;
@@ -1081,7 +1095,7 @@ __global__ void resolve_expansion_kernel(RerankArgs a, const int* __restrict__ c
 __global__ void resolve_fp64_kernel(ResolveD a) {
   if (grid_enter()) return;
   constexpr int L = 8;
-  const long long cnt = min((long long)*(volatile const int*)a.count, a.max_list);
+  const long long cnt = min((long long)pinned(a.count), a.max_list);
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -1333,11 +1347,13 @@ cudaError_t launch_resolve_candidates(const int* list, const int* count, long lo
   if (vec)
     launch(resolve_candidates_kernel<true>, kmgb::num_sms() * 8, 256, 0, s)(list, count, max_list, cand, cand_cnt,
                                                             X, ldx, C, ldc, cn, d, labels, over,
-                                                            over_count, stop, row_map, hi_in, over_hi);
+                                                            over_count, stop, row_map, hi_in, over_hi,
+                                                            resolve_tolerances(d));
   else
     launch(resolve_candidates_kernel<false>, kmgb::num_sms() * 8, 256, 0, s)(list, count, max_list, cand, cand_cnt,
                                                              X, ldx, C, ldc, cn, d, labels, over,
-                                                             over_count, stop, row_map, hi_in, over_hi);
+                                                             over_count, stop, row_map, hi_in, over_hi,
+                                                            resolve_tolerances(d));
   count_launches(1);
   return cudaGetLastError();
 }
