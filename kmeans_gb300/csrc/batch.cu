@@ -654,6 +654,35 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
     pev.push_back(e);
     return !f.set(cudaEventRecord(e, s), EU, "events");
   };
+  // The label audit reads the labels and the centers: in a captured iteration it is a branch that only
+  // the kernel writing the new centers waits for (as in engine.cu).
+  struct Branch {
+    cudaStream_t s = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    ~Branch() {
+      if (s) cudaStreamDestroy(s);
+      if (fork) cudaEventDestroy(fork);
+      if (join) cudaEventDestroy(join);
+    }
+  } br;
+  const bool branch =
+      audit_rows > 0 && cudaStreamCreateWithFlags(&br.s, cudaStreamNonBlocking) == cudaSuccess &&
+      cudaEventCreateWithFlags(&br.fork, cudaEventDisableTiming) == cudaSuccess &&
+      cudaEventCreateWithFlags(&br.join, cudaEventDisableTiming) == cudaSuccess;
+  if (!branch) cudaGetLastError();  // without them it stays in line
+  bool capturing = false;
+  auto issue_audit = [&](bool may_fork) -> bool {
+    const int EA = KMEANS_ERROR_CLOSEST_CENTERS;
+    const bool fork = branch && capturing && may_fork;
+    cudaStream_t as = fork ? br.s : s;
+    w.centers_free = fork ? br.join : nullptr;
+    return !(fork && (f.set(cudaEventRecord(br.fork, s), EA, "audit") ||
+                      f.set(cudaStreamWaitEvent(as, br.fork, 0), EA, "audit"))) &&
+           !f.set(launch_audit_labels(X, ldx, rows, d, C, ldx, (int)K, labels, audit_ws, audit_rows,
+                                      nullptr, as, &g),
+                  EA, "audit") &&
+           !(fork && f.set(cudaEventRecord(br.join, as), EA, "audit"));
+  };
   // One iteration of the group. Its launches do not depend on the iteration index (every
   // problem's SSE slot is its own device-side count), so with graphs on it is captured once and
   // replayed; phase events (marks) are recorded only in kernel-by-kernel runs.
@@ -681,11 +710,7 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
                                               nullptr, s),
                     KMEANS_ERROR_CLOSEST_CENTERS, "re-rank") ||
               f.set(launch_rerank_grouped(rx, g, s), KMEANS_ERROR_CLOSEST_CENTERS, "re-rank"))) &&
-           !(audit_rows > 0 &&
-             f.set(launch_audit_labels(X, ldx, rows, d, C, ldx, (int)K, labels, audit_ws,
-                                       audit_rows, nullptr, s, &g),
-                   KMEANS_ERROR_CLOSEST_CENTERS, "audit")) &&
-           mk() &&
+           !(audit_rows > 0 && !issue_audit(!marks)) && mk() &&
            !(prune && f.set(launch_prune_dirty_batched(pb, labels, s), EU, "distance bounds")) &&
            !f.set(launch_update_batched(X, ldx, d, qn, labels, C, ldx, o.empty_policy, w, b, s),
                   EU, "update") &&
@@ -703,7 +728,10 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
   if (max_iters > 0 && !(gv && std::strcmp(gv, "0") == 0) &&
       cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
     const long long l0 = thread_launch_count();
+    capturing = true;
     const bool ok = issue(false);
+    capturing = false;
+    w.centers_free = nullptr;
     cudaGraph_t graph = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(s, &graph);
     g_launches = thread_launch_count() - l0;

@@ -505,7 +505,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   w.k = k;
   w.d = d;
   w.ldx = h->ldx;
-  plan_update_tiles(na, k, &w.tile_pts, &w.ntiles);
+  plan_update_tiles_fine(na, k, &w.tile_pts, &w.ntiles);
   w.max_pieces = na / kSumPiece + k + 1;
   const long long hist_elems = (long long)k * w.ntiles;
   auto carve = [&](Arena& a) {

@@ -335,7 +335,7 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   w.k = k;
   w.d = n;
   w.ldx = n;
-  plan_update_tiles(m_mb, k, &w.tile_pts, &w.ntiles);
+  plan_update_tiles_fine(m_mb, k, &w.tile_pts, &w.ntiles);
   w.max_pieces = m_mb / kSumPiece + k + 1;
   const long long hist_elems = (long long)k * w.ntiles;
   KD_TRY(B.alloc(&w.hist, hist_elems), E);

@@ -394,6 +394,7 @@ template <typename T>
 cudaError_t launch_finalize_acc(const double* acc, const int* acc_counts, int k, int d, T* centers,
                                 int* counts, cudaStream_t s, const int* dirty = nullptr);
 void plan_update_tiles(long long n, int k, int* tile_pts, int* ntiles);
+void plan_update_tiles_fine(long long n, int k, int* tile_pts, int* ntiles);
 // Host-streamed tiles: per tile, label sort + canonical piece sums (with sum of ||x||^2) added to
 // FP64 accumulators accS[k][d], accN[k], accQ[k]; after the last tile, centers, SSE and the stop
 // rule from the accumulators.

@@ -569,7 +569,7 @@ kmeansCudaErrorStatus cluster_centers(int m0, int m, int n, int k, bool lastTile
   w.k = k;
   w.d = n;
   w.ldx = n;
-  plan_update_tiles(m, k, &w.tile_pts, &w.ntiles);
+  plan_update_tiles_fine(m, k, &w.tile_pts, &w.ntiles);
   w.max_pieces = m / kSumPiece + k + 1;
   const long long hist_elems = (long long)k * w.ntiles;
   cudaError_t e = cudaSuccess;

@@ -62,9 +62,12 @@ __device__ int block_excl_scan(int v) {
   return res;
 }
 
-// Nothing to update: no center won or lost a row (UpdateWork::any_dirty).
-__device__ __forceinline__ bool idle(const int* any_dirty) {
-  return any_dirty != nullptr && *reinterpret_cast<volatile const int*>(any_dirty) == 0;
+// The run has stopped, or there is nothing to update: no center won or lost a row
+// (UpdateWork::any_dirty). Both flags are loaded together.
+__device__ __forceinline__ bool skip(const int* stop, const int* any_dirty) {
+  const int st = stop ? pinned(stop) : 0;
+  const int any = any_dirty ? pinned(any_dirty) : 1;
+  return st != 0 || any == 0;
 }
 
 // True in every thread of the block that finishes last of the grid (every block calls it once, after
@@ -111,7 +114,7 @@ __device__ void block_scan_inplace(int* data, long long n) {
 __global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int* __restrict__ sums,
                                    int* ticket, const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  if (skip(stop, any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int s = 0;
 #pragma unroll
@@ -133,7 +136,7 @@ __global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int*
 __global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* __restrict__ offsets,
                                 const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  if (skip(stop, any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int vals[SCAN_V];
   int s = 0;
@@ -222,7 +225,7 @@ label_rows_kernel(int* __restrict__ hist, long long n, int k, int ntiles, int* l
                   long long* __restrict__ counts, const int* __restrict__ dirty, int* ticket,
                   const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  if (skip(stop, any_dirty)) return;
   const int lane = threadIdx.x & 31;
   const int j = (int)blockIdx.x * (SCAN_T / 32) + (int)(threadIdx.x >> 5);
   if (j < k) {
@@ -283,7 +286,7 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
                             int* piece_cnt, long long* counts, const int* dirty, int* ticket,
                             const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  if (skip(stop, any_dirty)) return;
   extern __shared__ int cnt_s[];
   const int tile = blockIdx.x;
   const long long i0 = (long long)tile * tile_pts;
@@ -340,7 +343,7 @@ __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int 
                                int* __restrict__ sorted, const int* __restrict__ dirty,
                                const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  if (skip(stop, any_dirty)) return;
   extern __shared__ int cnt_s[];
   const int tile = blockIdx.x;
   const int lane = threadIdx.x;
@@ -398,7 +401,7 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
                                      const int* __restrict__ dirty,
                                      const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  if (skip(stop, any_dirty)) return;
   extern __shared__ int wcnt[];  // [kScatterWarps][k]
   const int tile = blockIdx.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -512,8 +515,8 @@ __global__ void piece_sums_kernel(const float* __restrict__ X, long long ldx,
                                   double* __restrict__ partq, const int* any_dirty,
                                   const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
-  const int ptot = pstart[k];
+  const int ptot = pinned(pstart + k);
+  if (skip(stop, any_dirty)) return;
   const int lane = threadIdx.x & 31;
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -663,9 +666,9 @@ piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double*
                        const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
                        double* __restrict__ partq, const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  const long long ptot = pinned(pstart + k);
+  if (skip(stop, any_dirty)) return;
   __shared__ __align__(16) float4 ring[kRingWarps][kRingStages][kRingRows][32];
-  const long long ptot = pstart[k];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long nw = (long long)gridDim.x * kRingWarps;
   const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(&ring[w][0][0][lane]);
@@ -736,10 +739,10 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
                         const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
                         double* __restrict__ partq, const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
-  if (stopped(stop) || idle(any_dirty)) return;
+  const int ptot = pinned(pstart + k);
+  if (skip(stop, any_dirty)) return;
   constexpr int G = 32 / L;  // pieces per warp; also ids per lane and window
   constexpr int R = 16;      // rows per batch: one is summed while the next is in flight
-  const int ptot = pstart[k];
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
   const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -751,7 +754,7 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
     const int b = live ? __ldg(label_off + j) + ((int)p - __ldg(pstart + j)) * kSumPiece : 0;
     const int n = live ? min(kSumPiece, __ldg(label_off + j + 1) - b) : 0;
     const bool on = live && c < d;
-    const float* xc = X + c;
+    const float* xc = X + (on ? c : 0);
     auto load_ids = [&](int t, int (&id)[G]) {
 #pragma unroll
       for (int i = 0; i < G; ++i)
@@ -763,8 +766,8 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int row = __shfl_sync(0xffffffffu, id[(h + r) / L], grp * L + (h + r) % L);
-        v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (on && row >= 0) v[r] = __ldg(reinterpret_cast<const float4*>(xc + (size_t)row * ldx));
+        v[r] = __ldg(reinterpret_cast<const float4*>(xc + (size_t)max(row, 0) * ldx));  // (no branch)
+        if (row < 0) v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     };
     PieceAcc a0, a1, a2, a3;
@@ -818,6 +821,73 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
   }
 }
 
+// The same sums where pieces are few: a warp per piece and 32 dimensions, one dimension a lane, every id
+// of the piece, then every row in flight at once. A piece is a serial chain of 128 additions, but its
+// loads need not be one: with 16 rows ahead a warp waits eight times for L2 (900 cycles each).
+__global__ void __launch_bounds__(128)
+piece_sums_few_kernel(const float* __restrict__ X, long long ldx, const double* __restrict__ qn,
+                      const int* __restrict__ sorted, const int* __restrict__ label_off,
+                      const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
+                      double* __restrict__ partq, const int* any_dirty, const int* stop) {
+  if (grid_enter()) return;
+  const int ptot = pinned(pstart + k);
+  if (skip(stop, any_dirty)) return;
+  constexpr int W = kSumPiece / 32;  // 32-row windows of a piece
+  const int groups = (d + 31) / 32;
+  const long long total = (long long)ptot * groups;
+  const int lane = threadIdx.x & 31;
+  const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long it = gw; it < total; it += nw) {
+    const int p = (int)(it / groups), g = (int)(it - (long long)p * groups);
+    const int j = find_label_group<32>(pstart, k, p);
+    const int b = __ldg(label_off + j) + (p - __ldg(pstart + j)) * kSumPiece;
+    const int n = min(kSumPiece, __ldg(label_off + j + 1) - b);
+    const int c = g * 32 + lane;
+    const bool on = c < d;
+    const float* xc = X + (on ? c : 0);
+    int id[W];
+    double q[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) id[w] = 32 * w + lane < n ? __ldg(sorted + b + 32 * w + lane) : -1;
+    float v[kSumPiece];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      q[w] = qn && g == 0 && id[w] >= 0 ? __ldg(qn + id[w]) : 0.0;
+#pragma unroll
+      for (int r = 0; r < 32; ++r) {
+        const int row = __shfl_sync(0xffffffffu, id[w], r);
+        v[32 * w + r] = __ldg(xc + (size_t)max(row, 0) * ldx);  // (no branch per load)
+      }
+    }
+    PieceAcc a;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      if (32 * w + 32 <= n) {
+#pragma unroll
+        for (int r = 0; r < 32; ++r) a.add(v[32 * w + r]);
+      } else {  // zeros past the piece: adding them changes no float-float sum
+#pragma unroll
+        for (int r = 0; r < 32; ++r) a.add(32 * w + r < n ? v[32 * w + r] : 0.0f);
+        break;
+      }
+    }
+    if (on) part[(size_t)p * d + c] = a.value();
+    if (g == 0 && partq) {
+      double qs = 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) q[w] += __shfl_xor_sync(0xffffffffu, q[w], o);
+      }
+#pragma unroll
+      for (int w = 0; w < W; ++w)
+        if (32 * w < n) qs += q[w];
+      if (lane == 0) partq[p] = qs;
+    }
+  }
+}
+
 // Canonical piece sums of FP32 rows: the small-D kernel where D <= 64, the cp.async ring kernel
 // for other 16-byte-aligned rows, the scalar kernel otherwise.
 cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* qn,
@@ -827,21 +897,26 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
   // (the ring kernel's stage descriptor holds the chunk offset in 23 bits)
   const bool vec = ldx % 4 == 0 && d % 4 == 0 && d < (1 << 23) &&
                    (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  // up to 8 warps of work an SM, what it holds of the kernel: the latency of a piece's loads is what
+  // counts (846 pieces of 32 dimensions 16.7 -> 11.2 us, 63 pieces 16.2 -> 8.9; 958 of 128 dimensions,
+  // 25 warps an SM, 20.9 -> 25.2)
+  const long long few = max_pieces * ((d + 31) / 32);
+  if (few <= kmgb::num_sms() * 8LL) {
+    launch(piece_sums_few_kernel, (unsigned)((few + 3) / 4), 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k,
+                                                                   d, part, partq, any, stop);
+    kmgb::count_launches(1);
+    return cudaGetLastError();
+  }
   const int lanes = !vec || d > 64 ? 32 : (d <= 16 ? 4 : (d <= 32 ? 8 : 16));
   long long warps = (max_pieces + 32 / lanes - 1) / (32 / lanes);
   if (warps > kmgb::num_sms() * 64LL) warps = kmgb::num_sms() * 64LL;
   const unsigned blocks = (unsigned)((warps * 32 + 255) / 256);
   const unsigned sblocks = (unsigned)((warps * 32 + 127) / 128);
-  if (vec && lanes == 4)
-    launch(piece_sums_small_kernel<4>, sblocks, 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d,
-                                                      part, partq, any, stop);
-  else if (vec && lanes == 8)
-    launch(piece_sums_small_kernel<8>, sblocks, 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d,
-                                                      part, partq, any, stop);
-  else if (vec && lanes == 16)
-    launch(piece_sums_small_kernel<16>, sblocks, 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k,
-                                                       d, part, partq, any, stop);
-  else if (vec) {
+  if (vec && lanes < 32) {
+    auto kern = lanes == 4 ? piece_sums_small_kernel<4>
+                           : (lanes == 8 ? piece_sums_small_kernel<8> : piece_sums_small_kernel<16>);
+    launch(kern, sblocks, 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, any, stop);
+  } else if (vec) {
     // four 4-warp blocks (48 KB of ring each) per SM
     const long long cap = kmgb::num_sms() * 4LL * kRingWarps;
     const long long rw = max_pieces < cap ? max_pieces : cap;
@@ -1117,7 +1192,7 @@ __global__ void __launch_bounds__(256)
 finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long long ldc,
                        int empty_policy, UpdateWork w, double* __restrict__ sse_out) {
   if (grid_enter()) return;
-  if (stopped(w.stop)) return;
+  const int halt = w.stop ? pinned(w.stop) : 0;
   __shared__ double red[256];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int d = w.d;
@@ -1125,9 +1200,10 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
   LoopIn loop;  // (written by the last block only, at its end)
   if (threadIdx.x == 0) loop = load_loop(w.iters_done, w.sse_prev);
   for (int j = blockIdx.x; j < w.k; j += gridDim.x) {
-    const int live = w.dirty ? w.dirty[j] : 1;  // uniform over the block
-    const int m0 = w.label_off[j], m1 = w.label_off[j + 1];
-    const int p0 = w.piece_cnt[j], p1 = w.piece_cnt[j + 1];
+    const int live = w.dirty ? pinned(w.dirty + j) : 1;  // uniform over the block
+    const int m0 = pinned(w.label_off + j), m1 = pinned(w.label_off + j + 1);
+    const int p0 = pinned(w.piece_cnt + j), p1 = pinned(w.piece_cnt + j + 1);
+    if (halt) return;
     if (!live) continue;
     // the members' sum of ||x||^2: the last warp's lanes over the pieces, the first ones ahead
     double q = 0.0;
@@ -1240,6 +1316,16 @@ void plan_update_tiles(long long n, int k, int* tile_pts, int* ntiles) {
   if (tp > (1LL << 30)) tp = 1LL << 30;
   *tile_pts = (int)tp;
   *ntiles = (int)((n + tp - 1) / tp);
+}
+
+// The same, with smaller tiles where the counters still fit one step of the single-block scan
+// (SCAN_SEG): a small data set's histogram and scatter otherwise run on a few SMs (100,000 rows, K=64:
+// 25 blocks; scatter 8.2 us). Only for callers whose buffers are sized by this plan.
+void plan_update_tiles_fine(long long n, int k, int* tile_pts, int* ntiles) {
+  plan_update_tiles(n, k, tile_pts, ntiles);
+  while (*tile_pts > 512 && *ntiles < 2 * kmgb::num_sms() &&
+         (long long)k * ((n + *tile_pts / 2 - 1) / (*tile_pts / 2)) <= SCAN_SEG)
+    *tile_pts /= 2, *ntiles = (int)((n + *tile_pts - 1) / *tile_pts);
 }
 
 size_t update_scan_tmp_elems(long long elems) {
@@ -1504,9 +1590,13 @@ template cudaError_t launch_finalize_acc<double>(const double*, const int*, int,
 // are the single-problem kernels over all K centers.
 namespace {
 
+// SMEM: the tile's counters in shared memory (one global atomic per peer group, label by label, took
+// 14.7 us for 1.5M rows in 775 tiles).
+template <bool SMEM>
 __global__ void hist_batched_kernel(const int* __restrict__ labels, BatchUpdate b,
                                     int* __restrict__ hist, int* err) {
   if (grid_enter()) return;
+  extern __shared__ int cnt_s[];
   const long long st = blockIdx.x;
   const int prob = b.stile_prob[st];
   const int tl = b.stile_local[st];
@@ -1516,19 +1606,36 @@ __global__ void hist_batched_kernel(const int* __restrict__ labels, BatchUpdate 
   int* h = hist + b.hoff[prob];
   const int lane = threadIdx.x & 31;
   const int nbits = label_bits(kp);
-  for (long long base = i0; base < i1; base += blockDim.x) {
-    const long long i = base + threadIdx.x;
-    int l = -1;
-    if (i < i1) {
-      l = labels[i] - cb;
-      if (l < 0 || l >= kp) {
+  constexpr int U = 8;  // labels in flight per thread
+  if (SMEM) {
+    for (int j = threadIdx.x; j < kp; j += blockDim.x) cnt_s[j] = 0;
+    __syncthreads();
+  }
+  for (long long base = i0; base < i1; base += (long long)blockDim.x * U) {
+    int lv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = base + (long long)u * blockDim.x + threadIdx.x;
+      lv[u] = i < i1 ? __ldg(labels + i) - cb : -1;
+      if (i < i1 && (lv[u] < 0 || lv[u] >= kp)) {
         set_error(err, KMGB_DEV_BAD_LABEL);
-        l = -1;
+        lv[u] = -1;
       }
     }
-    const unsigned peers = warp_peers(l, nbits);
-    const int leader = __ffs(peers) - 1;
-    if (l >= 0 && lane == leader) atomicAdd(&h[(size_t)l * nt + tl], __popc(peers));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int l = lv[u];
+      if (SMEM) {
+        if (l >= 0) atomicAdd(&cnt_s[l], 1);
+      } else {
+        const unsigned peers = warp_peers(l, nbits);
+        if (l >= 0 && lane == __ffs(peers) - 1) atomicAdd(&h[(size_t)l * nt + tl], __popc(peers));
+      }
+    }
+  }
+  if (SMEM) {
+    __syncthreads();
+    for (int j = threadIdx.x; j < kp; j += blockDim.x) h[(size_t)j * nt + tl] = cnt_s[j];
   }
 }
 
@@ -1601,6 +1708,80 @@ __global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpda
   }
 }
 
+// The same by kScatterWarps warps, as scatter_multi_kernel, where their counters fit (kmax <=
+// kScatterMultiK): one warp's chain of steps took 29.5 us for 775 tiles of 2048 rows.
+constexpr int kScatterMultiK = 48 * 1024 / 4 / kScatterWarps;
+
+__global__ void scatter_batched_multi_kernel(const int* __restrict__ labels, BatchUpdate b,
+                                             const int* __restrict__ pos, int* __restrict__ sorted,
+                                             const int* __restrict__ dirty) {
+  if (grid_enter()) return;
+  extern __shared__ int wcnt[];  // [kScatterWarps][kp]
+  const long long st = blockIdx.x;
+  const int prob = b.stile_prob[st];
+  const int tl = b.stile_local[st];
+  const long long i0 = b.row_beg[prob] + (long long)tl * b.tile_pts;
+  const long long i1 = min(b.row_end[prob], i0 + b.tile_pts);
+  const int cb = b.c_off[prob], kp = b.k[prob], nt = b.ntiles[prob];
+  const int* h = pos + b.hoff[prob];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long span = ((i1 - i0 + kScatterWarps - 1) / kScatterWarps + 31) / 32 * 32;
+  const long long s0 = min(i1, i0 + w * span), s1 = min(i1, s0 + span);
+  int* mine = wcnt + (size_t)w * kp;
+  for (int j = threadIdx.x; j < kScatterWarps * kp; j += blockDim.x) wcnt[j] = 0;
+  __syncthreads();
+  constexpr int U = 8;  // labels in flight per lane, in both passes
+  auto load = [&](long long base, int (&lv)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = base + 32 * u + lane;
+      lv[u] = i < s1 ? __ldg(labels + i) - cb : -1;
+      if (lv[u] >= kp) lv[u] = -1;
+    }
+  };
+  for (long long base = s0; base < s1; base += 32 * U) {
+    int lv[U];
+    load(base, lv);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (lv[u] >= 0) atomicAdd(&mine[lv[u]], 1);
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < kp; j += blockDim.x) {
+    int run = __ldg(h + (size_t)j * nt + tl);
+    for (int v = 0; v < kScatterWarps; ++v) {
+      const int c = wcnt[(size_t)v * kp + j];
+      wcnt[(size_t)v * kp + j] = run;
+      run += c;
+    }
+  }
+  __syncthreads();
+  const int nbits = label_bits(kp);
+  for (long long base = s0; base < s1; base += 32 * U) {
+    int lv[U];
+    load(base, lv);
+    if (dirty) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (lv[u] >= 0 && !__ldg(dirty + cb + lv[u])) lv[u] = -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int l = lv[u];
+      if (!__any_sync(0xffffffffu, l >= 0)) continue;
+      const unsigned peers = warp_peers(l, nbits);
+      const int leader = __ffs(peers) - 1;
+      const int rank = __popc(peers & lanemask_lt());
+      int at = 0;
+      if (l >= 0 && lane == leader) at = mine[l];
+      at = __shfl_sync(0xffffffffu, at, leader);
+      if (l >= 0) sorted[at + rank] = (int)(base + 32 * u + lane);
+      if (l >= 0 && lane == leader) mine[l] = at + __popc(peers);
+      __syncwarp();
+    }
+  }
+}
+
 // One warp per problem: SSE = sum of its centers' terms; the reference's stop rule per problem
 // (kmeans.cpp:1194-1237). A problem that has stopped keeps its history; its centers are
 // recomputed from unchanged labels, which reproduces them bit for bit.
@@ -1636,7 +1817,11 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
                                   const UpdateWork& w, const BatchUpdate& b, cudaStream_t s) {
   if (b.P <= 0 || b.K <= 0 || b.n_valid <= 0) return cudaSuccess;
   KMGB_CUDA_TRY(cudaMemsetAsync(w.hist, 0, sizeof(int) * b.hist_elems, s));
-  launch(hist_batched_kernel, (unsigned)b.stiles, 256, 0, s)(labels, b, w.hist, w.err);
+  if (b.kmax <= 12288)
+    launch(hist_batched_kernel<true>, (unsigned)b.stiles, 256, sizeof(int) * (size_t)b.kmax, s)(
+        labels, b, w.hist, w.err);
+  else
+    launch(hist_batched_kernel<false>, (unsigned)b.stiles, 256, 0, s)(labels, b, w.hist, w.err);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.hist, b.hist_elems, w.scan_tmp, w.tickets, s, nullptr, nullptr));
@@ -1645,7 +1830,10 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
   KMGB_CUDA_TRY(excl_scan(w.piece_cnt, b.K + 1, w.scan_tmp, w.tickets, s, nullptr, nullptr));
-  if (b.kmax <= 12288)
+  if (b.kmax <= kScatterMultiK)
+    launch(scatter_batched_multi_kernel, (unsigned)b.stiles, 32 * kScatterWarps,
+           sizeof(int) * (size_t)b.kmax * kScatterWarps, s)(labels, b, w.hist, w.sorted, w.dirty);
+  else if (b.kmax <= 12288)
     launch(scatter_batched_kernel<true>, (unsigned)b.stiles, 32, sizeof(int) * (size_t)b.kmax, s)(
         labels, b, w.hist, w.sorted, w.dirty);
   else
@@ -1657,6 +1845,7 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
                                      w.part, w.partq, nullptr, nullptr, w.max_pieces, s));
   const int groups = (d + 31) / 32;
   const long long fin_warps = (long long)b.K * groups;
+  if (w.centers_free) KMGB_CUDA_TRY(cudaStreamWaitEvent(s, w.centers_free, 0));
   launch(finalize_kernel, (unsigned)((fin_warps * 32 + 255) / 256), 256, 0, s)(
       w.part, w.partq, w.label_off, w.piece_cnt, b.K, d, C, ldc, empty_policy, w.sse_k, w.dirty,
       nullptr);

@@ -518,3 +518,13 @@ def test_means_at_ties_zeros_and_subnormals(km, orc, torch_cuda, n, batched):
         res = km.lloyd(X, 2, init=init, max_iters=3)
     assert np.array_equal(res.labels, ref[2])
     assert np.array_equal(res.centers.view(np.uint32), np.asarray(ref[1], np.float32).view(np.uint32))
+
+
+@pytest.mark.parametrize("d", [4, 16, 20, 32, 36, 64])
+@pytest.mark.parametrize("n,k", [(1, 1), (127, 2), (129, 3), (1025, 5), (70_001, 33), (400_003, 17)])
+def test_narrow_sums_at_every_split(km, orc, torch_cuda, n, k, d):
+    """Narrow rows whose sums take a lane per one, two or four dimensions by the number of pieces, with
+    histogram tiles from 512 rows on."""
+    X, _, _ = mixture_numpy(n, d, max(2, k), seed=n + d)
+    init = X[sample_init(n, k, seed=3)]
+    check_same(km.lloyd(X, k, init=init, max_iters=3), orc.lloyd(X, init, 3))
