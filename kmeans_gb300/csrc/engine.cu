@@ -196,6 +196,7 @@ struct kmgb_handle {
   // centers
   float* C = nullptr;
   float* Cop = nullptr;
+  float* Ct = nullptr;      // FP32 tier: Cop's transpose [d][round_up(k, 4)]
   void* Cb = nullptr;
   void* Cl = nullptr;
   float* cn = nullptr;
@@ -535,6 +536,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     }
     a.take(&h->C, (size_t)k * h->ldx);
     a.take(&h->Cop, (size_t)k * h->ldx);
+    if (!tcore) a.take(&h->Ct, (size_t)d * round_up(k, 4));  // (the tiles of assign_fp32t_kernel)
     if (bf16) a.take_bytes(&h->Cb, (size_t)k * h->ldb * 2);
     if (split) a.take_bytes(&h->Cl, (size_t)k * h->ldb * 2);
     if (fp8) {
@@ -940,7 +942,8 @@ int router_maybe_train(kmgb_handle* h, int slot) {
   // the centers' operand copies, norms and planes for the updated centers
   KM_TRY(cudaMemsetAsync(h->cmax, 0, sizeof(float), s), KMEANS_ERROR_RESET);
   KM_TRY(launch_prep_centers(h->C, h->ldx, h->k, h->d, h->Cop, h->Cb, h->ldb, h->cn, h->cmax, s,
-                             nullptr, h->cinit, h->Cl, h->cbias),
+                             nullptr, h->cinit, h->Cl, h->cbias, nullptr, nullptr, 0.0f, h->Ct,
+                             round_up(h->k, 4)),
          KMEANS_ERROR_RESET);
   const RouterIO io = router_io(h);
   if (!h->router) {
@@ -1055,7 +1058,7 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   const bool prune = h->pr.n > 0 && !assign_only;
   KM_TRY(launch_prep_centers(h->C, h->ldx, h->k, h->d, h->Cop, h->Cb, h->ldb, h->cn, h->cmax, s,
                              h->stop, h->cinit, h->Cl, h->cbias, prune ? h->pr.shift : nullptr,
-                             prune ? h->pr.cxn : nullptr),
+                             prune ? h->pr.cxn : nullptr, 0.0f, h->Ct, round_up(h->k, 4)),
          KMEANS_ERROR_RESET);
   if (h->C8)
     KM_TRY(launch_centers_fp8(h->Cop, h->ldx, h->k, h->d, h->cmax, h->C8, h->ld8, h->cscale, s,
@@ -1077,6 +1080,8 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   a.certify = h->opt.certify;
   a.stop = h->stop;
   a.cinit = h->cinit;
+  a.Ct = h->Ct;
+  a.ldt = round_up(h->k, 4);
   a.cbias = h->cbias;  // BF16 tiers: start values by MMA where the launcher can
   test_wait_hook(&a.test_withhold, &a.test_wait_cycles);  // zero unless a test asks
   const bool tc = h->opt.assign_tier != KMGB_ASSIGN_FP32;
@@ -1200,7 +1205,8 @@ int step_stream(kmgb_handle* h, int slot) {
   KM_TRY(h->pmark(0), KMEANS_ERROR_RESET);
   KM_TRY(cudaMemsetAsync(h->cmax, 0, sizeof(float), s), KMEANS_ERROR_RESET);
   KM_TRY(launch_prep_centers(h->C, h->ldx, h->k, h->d, h->Cop, h->Cb, h->ldb, h->cn, h->cmax, s,
-                             h->stop, h->cinit, h->Cl, h->cbias),
+                             h->stop, h->cinit, h->Cl, h->cbias, nullptr, nullptr, 0.0f, h->Ct,
+                             round_up(h->k, 4)),
          KMEANS_ERROR_RESET);
   KM_TRY(cudaMemsetAsync(h->accS, 0, sizeof(double) * (size_t)h->k * h->d, s), KMEANS_ERROR_RESET);
   KM_TRY(cudaMemsetAsync(h->accQ, 0, sizeof(double) * h->k, s), KMEANS_ERROR_RESET);
@@ -1245,6 +1251,8 @@ int step_stream(kmgb_handle* h, int slot) {
     a.certify = h->opt.certify;
     a.stop = h->stop;
     a.cinit = h->cinit;
+    a.Ct = h->Ct;
+    a.ldt = round_up(h->k, 4);
     a.cbias = h->cbias;
     if (tc) {
       a.gamma = assign_bf16_gamma(h->d);

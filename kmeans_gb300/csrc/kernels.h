@@ -93,6 +93,8 @@ struct AssignArgs {
   // test_wait_cycles SM cycles (0: KMGB_WAIT_CYCLES)
   long long test_withhold;
   unsigned long long test_wait_cycles;
+  const float* Ct = nullptr;  // FP32 tier, nullable: the centers' transpose [d][ldt] (prep_centers)
+  long long ldt = 0;
 };
 
 // Many problems of one dimension in one launch (batched Lloyd): problem p owns rows
@@ -240,7 +242,7 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
                                 const int* stop = nullptr, float* cinit = nullptr,
                                 void* Cl = nullptr, void* cbias = nullptr,
                                 float* shift = nullptr, float* cxn = nullptr,
-                                float shift_pert = 0.0f);
+                                float shift_pert = 0.0f, float* Ct = nullptr, long long ldt = 0);
 
 // Distance bounds within one run (prune.cu): which rows an iteration has to scan again.
 struct PruneState {

@@ -55,7 +55,8 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
                                     const int* stop, float* __restrict__ cinit, int kpad,
                                     __nv_bfloat16* __restrict__ Cl,
                                     __nv_bfloat16* __restrict__ cbias, float* __restrict__ shift,
-                                    float* __restrict__ cxn, float shift_pert) {
+                                    float* __restrict__ cxn, float shift_pert,
+                                    float* __restrict__ Ct, long long ldt) {
   if (grid_enter()) return;
   if (stopped(stop)) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -93,6 +94,7 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
         mx = fmaxf(mx, df);
       }
       if (t < (int)ldc) op[t] = v[u];
+      if (Ct && t < d) Ct[(size_t)t * ldt + warp] = v[u];
       if (ob && t < (int)ldcb) {
         const __nv_bfloat16 h = __float2bfloat16_rn(v[u]);
         ob[t] = h;
@@ -104,6 +106,7 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
   if (bad) {  // unusable: zero operands
     for (int t = lane; t < width; t += 32) {
       if (t < (int)ldc) op[t] = 0.0f;
+      if (Ct && t < d) Ct[(size_t)t * ldt + warp] = 0.0f;
       if (ob && t < (int)ldcb) {
         ob[t] = __float2bfloat16_rn(0.0f);
         if (ol) ol[t] = __float2bfloat16_rn(0.0f);
@@ -461,7 +464,8 @@ cudaError_t launch_centers_fp8(const float* Cop, long long ldc, int k, int d, co
 cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, float* Cop, void* Cb,
                                 long long ldcb, float* cn, float* cmax, cudaStream_t s,
                                 const int* stop, float* cinit, void* Cl, void* cbias,
-                                float* shift, float* cxn, float shift_pert) {
+                                float* shift, float* cxn, float shift_pert, float* Ct,
+                                long long ldt) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (k <= 0) return cudaSuccess;
   const int threads = 256;
@@ -472,7 +476,7 @@ cudaError_t launch_prep_centers(const float* C, long long ldc, int k, int d, flo
                                                  cmax, stop, cinit, kpad,
                                                  reinterpret_cast<__nv_bfloat16*>(Cl),
                                                  reinterpret_cast<__nv_bfloat16*>(cbias), shift,
-                                                 cxn, shift_pert);
+                                                 cxn, shift_pert, Ct, ldt);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }

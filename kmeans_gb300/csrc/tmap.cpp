@@ -35,7 +35,8 @@ cudaError_t kmgb_make_tmap_2d_swz(CUtensorMap* map, const void* base, CUtensorMa
   auto fn = encode_fn();
   if (!fn) return cudaErrorNotSupported;
   const uint32_t width = swizzle == CU_TENSOR_MAP_SWIZZLE_32B ? 32
-                       : swizzle == CU_TENSOR_MAP_SWIZZLE_64B ? 64 : 128;
+                       : swizzle == CU_TENSOR_MAP_SWIZZLE_64B ? 64
+                       : swizzle == CU_TENSOR_MAP_SWIZZLE_NONE ? 256u * elem_bytes : 128;
   if (box_cols * (uint32_t)elem_bytes > width || box_rows > 256 || (row_stride_bytes % 16) ||
       (reinterpret_cast<uintptr_t>(base) & 15))
     return cudaErrorInvalidValue;

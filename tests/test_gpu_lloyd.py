@@ -528,3 +528,13 @@ def test_narrow_sums_at_every_split(km, orc, torch_cuda, n, k, d):
     X, _, _ = mixture_numpy(n, d, max(2, k), seed=n + d)
     init = X[sample_init(n, k, seed=3)]
     check_same(km.lloyd(X, k, init=init, max_iters=3), orc.lloyd(X, init, 3))
+
+
+@pytest.mark.parametrize("d", [1, 3, 4, 31, 33, 64, 324])
+@pytest.mark.parametrize("n,k", [(1, 1), (127, 127), (129, 128), (260, 129), (1000, 257)])
+def test_fp32_tiles_of_transposed_centers(km, orc, torch_cuda, n, k, d):
+    """The FP32 tier at the edges of its tiles: 128 points, 128 centers, 32 dimensions."""
+    rng = np.random.default_rng(n * 1000 + d)
+    X = rng.normal(size=(n, d)).astype(np.float32)
+    init = X[sample_init(n, k, seed=2)]
+    check_same(km.lloyd(X, k, init=init, max_iters=2, assign_tier=0), orc.lloyd(X, init, 2))
