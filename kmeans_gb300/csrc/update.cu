@@ -154,49 +154,6 @@ __global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* 
   }
 }
 
-// label_off[j] = start of label j in the sorted order (label_off[k] = n), counts[j] = members, and
-// piece_cnt[j] = first piece of label j, piece_cnt[k] = pieces in all, from the scanned counters. One
-// block of SCAN_T threads. No pieces for a center that keeps its sums (UpdateWork::dirty).
-__device__ void block_label_offsets(const int* hist, long long n, int k, int ntiles, int* label_off,
-                                    int* piece_cnt, long long* counts, const int* dirty) {
-  __shared__ int carry_sh;
-  constexpr int V = 4;
-  int carry = 0;
-  for (int b0 = 0; b0 < k; b0 += SCAN_T * V) {
-    const int base = b0 + threadIdx.x * V;
-    int at[V + 1], pc[V];
-    int s = 0;
-#pragma unroll
-    for (int v = 0; v <= V; ++v)
-      at[v] = base + v < k ? __ldcg(hist + (size_t)(base + v) * ntiles) : (int)n;
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      pc[v] = 0;
-      if (base + v < k) {
-        const int c = at[v + 1] - at[v];
-        label_off[base + v] = at[v];
-        if (counts) counts[base + v] = c;
-        pc[v] = dirty && !dirty[base + v] ? 0 : (c + kSumPiece - 1) / kSumPiece;
-        s += pc[v];
-      }
-    }
-    int pre = block_excl_scan(s) + carry;
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      if (base + v < k) piece_cnt[base + v] = pre;
-      pre += pc[v];
-    }
-    if (threadIdx.x == SCAN_T - 1) carry_sh = pre;
-    __syncthreads();
-    carry = carry_sh;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    label_off[k] = (int)n;
-    piece_cnt[k] = carry;
-  }
-}
-
 // The counters of one label, tile after tile: their exclusive scan in place by one warp, eight loads in
 // flight; returns their sum.
 __device__ __forceinline__ int scan_label_row(int* row, int ntiles, int lane) {
@@ -278,7 +235,7 @@ label_rows_kernel(int* __restrict__ hist, long long n, int k, int ntiles, int* l
 // ints) and writes every count; otherwise global atomics per warp group (hist cleared before).
 // SMALL (SCAN_T threads): the last block scans the counters and derives the labels' offsets, where
 // they are few enough for one block (kSmallHist): one launch instead of three.
-constexpr long long kSmallHist = 2 * SCAN_SEG;
+constexpr int kSmallHist = 8 * SCAN_T;
 
 template <bool SMEM, bool SMALL>
 __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, int tile_pts,
@@ -327,8 +284,50 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
     for (int j = threadIdx.x; j < k; j += blockDim.x) hist[(size_t)j * ntiles + tile] = cnt_s[j];
   }
   if (SMALL && last_block(ticket)) {
-    block_scan_inplace(hist, (long long)k * ntiles);
-    block_label_offsets(hist, n, k, ntiles, label_off, piece_cnt, counts, dirty);
+    // the scan, eight counters a thread, and from its positions in shared memory the labels' offsets,
+    // member counts and first pieces (through global memory: three more round trips)
+    __shared__ int pos_s[SMALL ? kSmallHist : 1];
+    const int total = k * ntiles, t = threadIdx.x;
+    int live = t < k && dirty ? __ldg(dirty + t) : 1;
+    int v[8], s = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = 8 * t + u < total ? __ldcg(hist + 8 * t + u) : 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+    int pre = block_excl_scan(s);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (8 * t + u < total) {
+        hist[8 * t + u] = pre;
+        pos_s[8 * t + u] = pre;
+      }
+      pre += v[u];
+    }
+    __syncthreads();
+    __shared__ int carry_sh;
+    int carry = 0;
+    for (int j0 = 0; j0 < k; j0 += SCAN_T) {
+      const int j = j0 + t;
+      if (j0 > 0) live = j < k && dirty ? __ldg(dirty + j) : 1;
+      int c = 0, a0 = 0;
+      if (j < k) {
+        a0 = pos_s[j * ntiles];
+        c = (j + 1 < k ? pos_s[(j + 1) * ntiles] : (int)n) - a0;
+        label_off[j] = a0;
+        if (counts) counts[j] = c;
+      }
+      const int pc = live ? (c + kSumPiece - 1) / kSumPiece : 0;
+      const int first = block_excl_scan(pc) + carry;
+      if (j < k) piece_cnt[j] = first;
+      if (t == SCAN_T - 1) carry_sh = first + pc;
+      __syncthreads();
+      carry = carry_sh;
+      __syncthreads();
+    }
+    if (t == 0) {
+      label_off[k] = (int)n;
+      piece_cnt[k] = carry;
+    }
   }
 }
 
@@ -1338,7 +1337,7 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
   const int k = w.k;
   const long long hist_elems = (long long)k * w.ntiles;
   const size_t smem = sizeof(int) * (size_t)k;
-  const bool small = hist_elems <= kSmallHist && smem <= 48 * 1024;
+  const bool small = hist_elems <= kSmallHist && smem <= 12 * 1024;  // (next to the scan's 32 KB)
   if (small) {
     launch(hist_kernel<true, true>, w.ntiles, SCAN_T, smem, s)(
         labels, n, k, w.tile_pts, w.ntiles, w.hist, w.err, w.label_off, w.piece_cnt, w.counts, w.dirty,
