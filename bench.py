@@ -9,14 +9,15 @@ points; synthetic, generated on the device). Prints one JSON line.
   python bench.py [--gpus N] [--steps K] [--warmup W] [--tier bf16x3|bf16|fp32] [--impl reference]
 
 `value` is Lloyd iterations/s with the data resident in HBM (CUDA events on the library's
-stream); `e2e` is the same metric through the public C-ABI one-shot call (kmgb_lloyd_f32) from
+stream): runs of the workload's 30 iterations, each from the initial centers (the library keeps
+distance bounds within a run, so a run's later iterations scan fewer rows than its first); `e2e` is the same metric through the public C-ABI one-shot call (kmgb_lloyd_f32) from
 pinned host memory (`pageable_value`: the same from pageable memory), host<->device copies
-included, one call running the workload's 30 iterations; `roofline` covers the assignment kernel
-(2*N*K*D FLOP per launch, per-launch time from CUDA events bracketing it inside the timed
-region; `tensor_*` counts the tensor-core products the tier actually issues, three per element
+included, one call running the workload's 30 iterations; `roofline` covers the assignment kernel on a
+full scan (2*N*K*D FLOP per launch, per-launch time from CUDA events bracketing it in
+one-iteration runs, which scan every row; `tensor_*` counts the tensor-core products the tier actually issues, three per element
 in the split tier; `traffic` is the DRAM bytes of one launch from an ncu capture, scaled to N);
 `update_roofline` puts the update phase (sort, piece sums, finalize, SSE; N*D*4 + N*4 + K*D*8
-bytes per iteration) against the measured HBM copy rate; `cpu_baseline` is the CPU restatement (oracle FP32 port, all host threads) on a sample.
+bytes per iteration, in the same one-iteration runs) against the measured HBM copy rate; `cpu_baseline` is the CPU restatement (oracle FP32 port, all host threads) on a sample.
 The reference arm (--impl reference) times that CPU path: the reference has no CPU
 implementation of its own and its host code is not built (its sources are only in the x86
 development container; its driver also needs a CMake-generated config.h and cuBLAS). Its line also
@@ -359,7 +360,7 @@ def accuracy_and_plain_fp32(km, torch, h, X, n, k):
            "label_mismatch_rate": mism / idx.numel(),
            "center_max_rel_err": float(cerr), "sse_rel_err": abs(sse - sse64) / abs(sse64),
            "reference": "torch float64 on the GPU (direct squared distances, FP64 means and SSE)"}
-    # plain FP32 tier from the same centers
+    # plain FP32 tier from the same centers; timed in one-iteration runs, which scan every row
     h32 = km.Handle(n, d, k, assign_tier=km.ASSIGN_FP32, max_iters=8)
     h32.set_data(X, True)
     h32.set_centers(C.cpu().numpy(), False)
@@ -370,7 +371,8 @@ def accuracy_and_plain_fp32(km, torch, h, X, n, k):
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     h32.set_profiling(True)
     e0.record(stream)
-    h32.run(5)
+    for _ in range(5):
+        h32.run(1)
     e1.record(stream)
     h32.synchronize()
     ms = e0.elapsed_time(e1) / 5
@@ -386,7 +388,9 @@ def accuracy_and_plain_fp32(km, torch, h, X, n, k):
 def time_kmeanspp(km, torch, h, n, k, reps=1):
     """k-means++ initialisation on the handle's resident data (outside the Lloyd timed region):
     one untimed call, then `reps` calls bracketed by CUDA events on the handle's stream. Each
-    draw reads X once (N*D*4 bytes) and D^2 three times and writes it once (4 * N*4 bytes)."""
+    draw that reads every row reads X once (N*D*4 bytes) and D^2 three times and writes it once
+    (4 * N*4 bytes); rows that a new center cannot reach are not read, so the rate against those
+    bytes can exceed the copy rate."""
     stream = torch.cuda.ExternalStream(h.stream)
     h.init_kmeanspp(1000)
     e0 = torch.cuda.Event(enable_timing=True)
@@ -445,7 +449,7 @@ def batched_workload(args):
     _, st = km.lloyd_batched(probs, max_iters=iters, assign_tier=tier_id)
     full = time.perf_counter() - t0
     launches = km.launch_count() - l0
-    per_iter = st.ms_total / 1000.0 / iters  # CUDA events around the iteration loops
+    per_iter = (full - one) / (iters - 1)  # the groups' iterations run side by side
     sample = probs[: min(200, len(probs))]
     km.lloyd(sample[0][0], sample[0][1], max_iters=1)
     t0 = time.perf_counter()
@@ -466,7 +470,7 @@ def batched_workload(args):
                                         enumerate(["prep", "assign", "rerank", "update"])}
                                        if st.reserved[5] == 0 else
                                        "not recorded: iterations replayed as CUDA graphs"),
-            "setup_s": full - st.ms_total / 1000.0,
+            "setup_s": one - per_iter,
             "assign_tflops_per_iteration": flop / per_iter / 1e12,
             "setup_and_one_iteration_s": one, "generation_s": gen_s,
             "reranked_points_total": st.reranked, "gpu_launches": launches,
@@ -930,6 +934,14 @@ def main():
     h.set_centers(init, False)
     h.run(args.warmup)
     h.synchronize()
+    init_dev = X[idx].contiguous()
+    # full scans: one-iteration runs, whose every row is assigned and every cluster updated
+    h.set_profiling(True)
+    for _ in range(5):
+        h.set_centers(init_dev, True)
+        h.run(1)
+        h.synchronize()
+    full_phase, full_iters = h.phase_ms()
 
     stream = torch.cuda.ExternalStream(h.stream)
     ev0 = torch.cuda.Event(enable_timing=True)
@@ -941,7 +953,9 @@ def main():
     torch.cuda.synchronize()
     clocks = Clocks(local)
     ev0.record(stream)
-    h.run(args.steps)
+    for done in range(0, args.steps, E2E_ITERS):  # the workload's runs
+        h.set_centers(init_dev, True)
+        h.run(min(E2E_ITERS, args.steps - done))
     ev1.record(stream)
     h.synchronize()
     torch.cuda.synchronize()
@@ -953,14 +967,14 @@ def main():
     ms, value = replica_rate(ms, args.steps, world, dist)
 
     flop = 2.0 * n * K * D
-    assign_ms = phase[1] / max(piters, 1)
+    assign_ms = full_phase[1] / max(full_iters, 1)
     achieved = flop / (assign_ms / 1000.0) / 1e12
     bf16_peak, hbm_peak, src = peaks()
     traffic = TRAFFIC_BYTES_PER_ROW.get(tier)
     roofline = {"bound": "tensor", "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
                 "frac": achieved / bf16_peak,
                 "traffic": traffic * n if traffic else None, "traffic_unit": "bytes",
-                "kernel": "assign_fp32_kernel" if tier == "fp32" else "assign_bf16_kernel",
+                "kernel": "assign_fp32t_kernel" if tier == "fp32" else "assign_bf16_kernel",
                 "peak_source": f"{src} bf16 dense (MEASURED_PEAKS.json)",
                 "flop_per_launch": flop, "ms_per_launch": assign_ms}
     if tier in TENSOR_PRODUCTS:
@@ -972,13 +986,13 @@ def main():
     # the update phase (counting sort, piece sums, finalize, SSE; event-timed together) against
     # HBM: its algorithmic bytes per iteration are X once, the labels and the FP64 per-cluster
     # sums
-    upd_ms = phase[3] / max(piters, 1)
+    upd_ms = full_phase[3] / max(full_iters, 1)
     upd_bytes = n * D * 4 + n * 4 + K * D * 8
     upd_gbs = upd_bytes / (upd_ms / 1000.0) / 1e9 if upd_ms > 0 else None
     update_roofline = {"bound": "hbm", "achieved": upd_gbs, "peak": hbm_peak, "unit": "GB/s",
                        "frac": upd_gbs / hbm_peak if upd_gbs else None,
                        "bytes_per_iteration": upd_bytes, "ms_per_iteration": upd_ms,
-                       "kernels": "hist, scans, scatter_multi, piece_sums_ring, finalize, sse",
+                       "kernels": "hist, label_rows, scatter_multi, piece_sums_ring, finalize_update",
                        "peak_source": f"{src} HBM copy (MEASURED_PEAKS.json)"}
 
     checks = None
@@ -1067,7 +1081,7 @@ def main():
                                   f"pass)" if n * D * 4 > L2_BYTES else
                                   f"X ({n * D * 4 / 1e6:.0f} MB) fits in L2: profiling size, "
                                   f"not a bench figure"),
-                           "parallelism": "single"},
+                           "run_iterations": E2E_ITERS, "parallelism": "single"},
                 "assign_tflops": achieved,
                 "phase_ms_per_iter": {n: p / max(piters, 1) for n, p in
                                       zip(["prep", "assign", "rerank", "update"], phase)},
