@@ -83,8 +83,8 @@ KMGB_EXPORT kmeansErrorStatus computeKmeansF(const float* data, const int m, con
  * computeKmeansF's arguments and layouts on FP64 data. Labels are the FP64 arg-min of the
  * direct distance (lowest index on ties); centers are canonical FP64 sums over the counts. Full
  * batches with n <= 320 assign on the tensor cores (the split BF16 tier on FP32 roundings of the
- * data and centers, its bound widened by that rounding, the uncertified points rescanned in
- * FP64); mini-batch windows, wider data and KMGB_ASSIGN=fp32 use the FP64 scan for every point. */
+ * data and centers, its bound widened by that rounding, the uncertified points' candidates settled
+ * in FP64); mini-batch windows, wider data and KMGB_ASSIGN=fp32 use the FP64 scan for every point. */
 KMGB_EXPORT kmeansErrorStatus computeKmeansD(const double* data, const int m, const int n, const int k,
                                  const double criterion, const int maxIters,
                                  const int numRetries, const int initAlgorithm,
@@ -363,7 +363,8 @@ typedef struct kmgb_problem {
  * init_algorithm KMGB_INIT_REFERENCE. Problems of one dimension and tier form a group whose
  * iteration is captured once as a CUDA graph and replayed (KMGB_GRAPHS=0: kernel by kernel).
  * stats (nullable): iterations = the largest over the problems, reranked = rows settled by the
- * exact re-rank, ms_total = GPU time of the iterations (CUDA events, summed over the groups),
+ * exact re-rank, ms_total = GPU time of the iterations (CUDA events, summed over the groups, which
+ * run side by side: more than the time that passed),
  * reserved[0] = wall time of the whole call in microseconds (uploads, initialisation and result
  * copies included), reserved[1..4] = microseconds of center preparation, assignment, re-rank and
  * update summed over the iterations (CUDA events; kernel-by-kernel runs only), reserved[5] =

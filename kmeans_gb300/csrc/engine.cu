@@ -344,7 +344,8 @@ int audit_rows_for(const kmgb_options& o, bool streaming, int k, int d) {
 // centers against themselves (k rows), the pass over the bounds (20 bytes a row) and three more
 // launches, ~25 us in all at 900,000 x 128, K=256, where the scan takes 80 us. On GB300, 10
 // iterations of 4M x 128, K=1024 from sampled centers: 25.9 -> 17.8 ms.
-// The FP32 tier's scan takes some 20 times as long: 796,160 x 324, K=256, 10 iterations 49.5 -> 20.0 ms.
+// The FP32 tier's scan takes some 20 times as long: 796,160 x 324, K=256, 10 iterations 49.5 -> 20.0 ms
+// (15.4 with the packed scan).
 constexpr long long kPruneMinWork = 1LL << 33;  // rows x centers (in chunks of 256) x dimensions
 constexpr long long kPruneMinWorkFp32 = 1LL << 30;
 constexpr long long kPruneMaxBytes = 8LL << 30;  // of the compact copy
