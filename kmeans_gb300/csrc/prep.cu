@@ -175,6 +175,8 @@ __global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, 
 // it at a time (L = 32 from 68 dimensions on, fewer below, so that a warp's lanes are all busy and
 // its loads contiguous), and a warp takes two row groups at a time. One pass per kind of output with
 // a warp and 4 bytes a lane per row took 153 + 69 us for 898,790 x 128 (norms, one plane pair);
+// the tree and the row's results one row at a time, and FP64 conversions that the compiler ran with qn
+// null too, 52 us for 224,698 x 128 (now 40).
 // T = double: the FP32 roundings of FP64 rows (row stride ldx doubles, read element by element
 // unless rows are 16-byte aligned).
 template <typename T>
@@ -277,7 +279,7 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
           Xb[(size_t)r * ldb4 + c / 4] = h;
           if (Xl || inexact) {
             const float4 hv = widen4(h);
-            off |= !(v[u].x == hv.x && v[u].y == hv.y && v[u].z == hv.z && v[u].w == hv.w);
+            if (inexact) off |= !(v[u].x == hv.x && v[u].y == hv.y && v[u].z == hv.z && v[u].w == hv.w);
             if (Xl)
               Xl[(size_t)r * ldb4 + c / 4] = bf16x4(make_float4(v[u].x - hv.x, v[u].y - hv.y,
                                                                 v[u].z - hv.z, v[u].w - hv.w));
@@ -286,40 +288,58 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
       }
     }
     if (!norms) continue;
+    // the two rows' trees: the first step leaves the first row's to the lower half of the lanes and the
+    // second's to the upper half (each adding its pair as lane 0 would), the others run on one value
+    static_assert(U == 2, "a row per half");
+    constexpr int H = L / 2;
+    const bool up = sub >= H;
+    const long long r = r0 + (up ? G : 0) + grp;
+    float h1, l1;
+    {
+      const float oh = __shfl_xor_sync(0xffffffffu, up ? hi[0] : hi[1], H);
+      const float ol = __shfl_xor_sync(0xffffffffu, up ? lo[0] : lo[1], H);
+      const float mh = up ? hi[1] : hi[0], ml = up ? lo[1] : lo[0];
+      float err;
+      ff_two_sum(up ? oh : mh, up ? mh : oh, h1, err);
+      l1 = __fadd_rn(up ? ol : ml, __fadd_rn(up ? ml : ol, err));
+    }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const long long r = r0 + u * G + grp;
-#pragma unroll
-      for (int o = L / 2; o > 0; o >>= 1) {
-        const float oh = __shfl_xor_sync(0xffffffffu, hi[u], o);
-        const float ol = __shfl_xor_sync(0xffffffffu, lo[u], o);
-        float s1, err;
-        ff_two_sum(hi[u], oh, s1, err);
-        hi[u] = s1;
-        lo[u] = __fadd_rn(lo[u], __fadd_rn(ol, err));
-      }
-      // overflow (or NaN input): FP64 sum; for the rounded norm also where squares near the
-      // subnormals lose their low parts
-      const bool wide = !(fabsf(hi[u]) < 1.0e37f) || (nf && hi[u] < 1.0e-24f);
-      if (__any_sync(0xffffffffu, wide)) {
+    for (int o = H / 2; o > 0; o >>= 1) {
+      const float oh = __shfl_xor_sync(0xffffffffu, h1, o);
+      const float ol = __shfl_xor_sync(0xffffffffu, l1, o);
+      float s1, err;
+      ff_two_sum(h1, oh, s1, err);
+      h1 = s1;
+      l1 = __fadd_rn(l1, __fadd_rn(ol, err));
+    }
+    // overflow (or NaN input): FP64 sum; for the rounded norm also where squares near the
+    // subnormals lose their low parts
+    const bool wide = !(fabsf(h1) < 1.0e37f) || (nf && h1 < 1.0e-24f);
+    if (__any_sync(0xffffffffu, wide)) {
+#pragma unroll 1
+      for (int u = 0; u < U; ++u) {
+        const long long ru = r0 + u * G + grp;
         double sd = 0.0;
-        if (r < n)
+        if (ru < n)
           for (int t = sub; t < d; t += L) {
-            const double x = (double)(float)__ldg(X + (size_t)source(r) * ldx + t);
+            const double x = (double)(float)__ldg(X + (size_t)source(ru) * ldx + t);
             sd = fma(x, x, sd);
           }
         for (int o = L / 2; o > 0; o >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, o);
-        if (wide && sub == 0 && r < n) {
-          if (qn) qn[r] = sd;
-          if (nf) nf[r] = __double2float_rn(sd);
-          if (xn) xn[r] = __double2float_ru(sqrt(sd) * (1.0 + 1e-12));
+        if (wide && sub == u * H && ru < n) {
+          if (qn) qn[ru] = sd;
+          if (nf) nf[ru] = __double2float_rn(sd);
+          if (xn) xn[ru] = __double2float_ru(sqrt(sd) * (1.0 + 1e-12));
         }
       }
-      if (!wide && sub == 0 && r < n) {
-        if (qn) qn[r] = (double)hi[u] + (double)lo[u];
-        if (nf) nf[r] = __fadd_rn(hi[u], lo[u]);
-        if (xn) xn[r] = __fsqrt_ru(__fmul_ru(__fadd_ru(hi[u], fabsf(lo[u])), 1.0f + 0x1p-20f));
+    }
+    if (!wide && (sub == 0 || sub == H) && r < n) {
+      if (qn) {
+        asm volatile("" : "+f"(h1));  // (keeps the FP64 conversions from running where qn is null)
+        qn[r] = (double)h1 + (double)l1;
       }
+      if (nf) nf[r] = __fadd_rn(h1, l1);
+      if (xn) xn[r] = __fsqrt_ru(__fmul_ru(__fadd_ru(h1, fabsf(l1)), 1.0f + 0x1p-20f));
     }
   }
   if (inexact && __any_sync(0xffffffffu, off) && lane == 0) atomicExch(inexact, 1);
