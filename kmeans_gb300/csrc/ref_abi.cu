@@ -136,7 +136,8 @@ __device__ __forceinline__ double block_sum(double acc) {
 // float-float values -- u = x - c exactly (TwoSum), u^2 = p + e (FMA), TwoSum accumulation -- and a
 // lane widens one pair per segment of kSegSteps rows. A segment whose sum leaves the range in which
 // that keeps 48 bits (overflow, squares near the subnormals, NaN) is evaluated in FP64.
-// L lanes share a row, 16 bytes each at a time where rows are aligned.
+// L lanes share a row, 16 bytes each at a time where rows are aligned; four rows and the next four's
+// labels are in flight without a branch per row (898,790 x 128: 155 -> 129 us, at some two thirds of the issue slots).
 constexpr int kSegSteps = 32;
 
 template <int L>
@@ -162,24 +163,50 @@ compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const 
       lo = __fadd_rn(lo, __fadd_rn(err, r));
       mx = fmaxf(mx, fabsf(uh));
     };
-#pragma unroll 4
-    for (int i = 0; i < kSegSteps; ++i) {
-      const long long r = s0 + i * G + grp;
-      if (r >= m) continue;
-      const float* x = data + (size_t)r * n;
-      const float* c = centers + (size_t)__ldg(idx + r) * n;
+    // U rows at a time, the next ones' labels with this batch's elements; rows past the end and
+    // dimensions past n add zeros, which change neither hi nor lo
+    constexpr int U = 4;
+    int id[U], nx[U];
+    auto load_ids = [&](int i, int (&o)[U]) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long r = s0 + (i + u) * G + grp;
+        o[u] = i < kSegSteps && r < m ? __ldg(idx + r) : -1;
+      }
+    };
+    load_ids(0, id);
+    for (int i = 0; i < kSegSteps; i += U) {
+      load_ids(i + U, nx);
       if (vec) {
-        for (int t = 4 * sub; t < n; t += 4 * L) {
-          const float4 xv = __ldg(reinterpret_cast<const float4*>(x + t));
-          const float4 cv = __ldg(reinterpret_cast<const float4*>(c + t));
-          term(xv.x, cv.x);
-          term(xv.y, cv.y);
-          term(xv.z, cv.z);
-          term(xv.w, cv.w);
+        for (int t0 = 0; t0 < n; t0 += 4 * L) {
+          const int t = t0 + 4 * sub < n ? t0 + 4 * sub : 0;
+          float4 xv[U], cv[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const long long r = s0 + (i + u) * G + grp;
+            xv[u] = __ldg(reinterpret_cast<const float4*>(data + (size_t)(id[u] >= 0 ? r : 0) * n + t));
+            cv[u] = __ldg(reinterpret_cast<const float4*>(centers + (size_t)max(id[u], 0) * n + t));
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (id[u] < 0 || t0 + 4 * sub >= n) xv[u] = cv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            term(xv[u].x, cv[u].x);
+            term(xv[u].y, cv[u].y);
+            term(xv[u].z, cv[u].z);
+            term(xv[u].w, cv[u].w);
+          }
         }
       } else {
-        for (int t = sub; t < n; t += L) term(__ldg(x + t), __ldg(c + t));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (id[u] < 0) continue;
+          const float* x = data + (size_t)(s0 + (i + u) * G + grp) * n;
+          const float* c = centers + (size_t)id[u] * n;
+          for (int t = sub; t < n; t += L) term(__ldg(x + t), __ldg(c + t));
+        }
       }
+#pragma unroll
+      for (int u = 0; u < U; ++u) id[u] = nx[u];
     }
     if (hi < 1e37f && (hi > 1e-24f || mx == 0.0f)) {
       acc += (double)hi + (double)lo;
