@@ -45,9 +45,15 @@ long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 namespace {
 
-__global__ void set_int_kernel(int* p, int v) {
+// The device words a run starts from (kmeans.cpp:40-41): SSE_old = 0, relErr = 1, the run's criterion,
+// and (nullable) the window index of its first iteration.
+__global__ void begin_run_kernel(double* loopf, double criterion, int* win_base, int base) {
   if (grid_enter()) return;
-  *p = v; }
+  loopf[0] = 0.0;
+  loopf[1] = 1.0;
+  loopf[2] = criterion;
+  if (win_base) *win_base = base;
+}
 
 thread_local std::string g_last_error;
 
@@ -257,7 +263,7 @@ struct kmgb_handle {
   int* kpp_picks = nullptr;
   // device-side loop state: stop flag, previous SSE, last relErr, iterations done
   int* stop = nullptr;
-  double* loopf = nullptr;  // [0] SSE_old, [1] relErr
+  double* loopf = nullptr;  // [0] SSE_old, [1] relErr, [2] the run's criterion
   int* iters_done = nullptr;
   int run_base = 0;         // iter_base when the current run started
   // update
@@ -575,7 +581,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     if (h->audit_rows > 0) a.take(&h->audit, kAuditWords);
     a.take(&h->err, 1);
     a.take(&h->stop, 1);
-    a.take(&h->loopf, 2);
+    a.take(&h->loopf, 3);
     a.take(&h->iters_done, 1);
     a.take(&h->xinexact, 1);
     a.take(&w.hist, hist_elems);
@@ -616,6 +622,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   w.stop = h->stop;
   w.sse_prev = h->loopf;
   w.rel_out = h->loopf + 1;
+  w.criterion = h->loopf + 2;
   w.iters_done = h->iters_done;
   w.sse_indexed = h->streaming ? 0 : 1;  // host-streamed iterations write their own slot
   h->sse_cap = std::max(1, h->opt.max_iters);
@@ -1330,9 +1337,9 @@ int step_stream(kmgb_handle* h, int slot) {
 }
 
 // Enqueues `iters` iterations as launches of one captured CUDA graph holding a whole iteration
-// (resident data): every iteration issues the same kernels with the same parameters -- the SSE slot, the
-// stop rule and a mini-batch window are indexed on the device -- so the graph is captured once and
-// replayed until a buffer it uses is replaced. Returns 0 when launched, -1 when the iteration cannot be
+// (resident data): every iteration issues the same kernels with the same parameters -- the SSE slot and a
+// mini-batch window are indexed on the device, and the stop rule's criterion is a device word of the run
+// -- so the graph is captured once and replayed until a buffer it uses is replaced. Returns 0 when launched, -1 when the iteration cannot be
 // captured (it is then launched kernel by kernel), else an error code.
 int run_graph(kmgb_handle* h, int iters) {
   if (!(h->gexec && h->g_sse == h->sse_dev)) {
@@ -1402,20 +1409,13 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
   }
   h->sse_host.assign(iters, 0.0);
   h->run_base = h->iter_base;
-  h->uw.criterion = criterion;
   h->criterion = criterion;
-  // loop state (kmeans.cpp:40-41): SSE_old = 0, relErr = 1, not stopped
-  static const double kLoopInit[2] = {0.0, 1.0};  // a constant source: nothing to keep alive
+  // loop state: not stopped, nothing done
   KM_TRY(cudaMemsetAsync(h->stop, 0, sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
   KM_TRY(cudaMemsetAsync(h->iters_done, 0, sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
-  KM_TRY(cudaMemcpyAsync(h->loopf, kLoopInit, 2 * sizeof(double), cudaMemcpyHostToDevice,
-                         h->stream),
-         KMEANS_ERROR_COMPUTE);
-  if (h->mini) {
-    launch(set_int_kernel, 1, 1, 0, h->stream)(h->win_base, h->run_base);
-    count_launches(1);
-    KM_TRY(cudaGetLastError(), KMEANS_ERROR_CONSTRUCT_MINIBATCH);
-  }
+  launch(begin_run_kernel, 1, 1, 0, h->stream)(h->loopf, criterion, h->win_base, h->run_base);
+  count_launches(1);
+  KM_TRY(cudaGetLastError(), KMEANS_ERROR_COMPUTE);
   if (h->pr.n > 0)  // no bounds yet: the first iteration scans every row
     KM_TRY(cudaMemsetAsync(h->pr.flags, 0, 8 * sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
   KM_TRY(cudaEventRecord(h->ev0, h->stream), KMEANS_ERROR_COMPUTE);

@@ -375,7 +375,8 @@ struct UpdateWork {
                         // update: its sums, center and SSE terms stay as they are
   // stop rule (kmeans.cpp:1194-1237), evaluated on the device by the SSE reduction
   int* stop;            // nullable
-  double criterion;
+  const double* criterion;  // device word, written per run (a captured iteration outlives the run);
+                            // null with sse_prev
   double* sse_prev;     // previous SSE (0 before the first iteration)
   double* rel_out;      // last relErr
   int* iters_done;      // iterations completed

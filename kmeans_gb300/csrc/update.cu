@@ -1160,17 +1160,21 @@ __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
 // stores they cost three round trips.
 struct LoopIn {
   int it = 0;
-  double prev = 0.0;
+  double prev = 0.0, criterion = 0.0;
 };
-__device__ __forceinline__ LoopIn load_loop(const int* iters_done, const double* sse_prev) {
+__device__ __forceinline__ LoopIn load_loop(const int* iters_done, const double* sse_prev,
+                                            const double* criterion) {
   LoopIn l;
   if (iters_done) l.it = *iters_done;
-  if (sse_prev) l.prev = *sse_prev;
+  if (sse_prev) {
+    l.prev = *sse_prev;
+    l.criterion = *criterion;
+  }
   return l;
 }
 __device__ __forceinline__ void store_sse(double sse, const LoopIn& l, double* out, int* stop,
-                                          double criterion, double* sse_prev, double* rel_out,
-                                          int* iters_done, int indexed) {
+                                          double* sse_prev, double* rel_out, int* iters_done,
+                                          int indexed) {
   if (indexed && iters_done) out[l.it] = sse;
   else *out = sse;
   if (sse_prev) {
@@ -1178,7 +1182,7 @@ __device__ __forceinline__ void store_sse(double sse, const LoopIn& l, double* o
     *sse_prev = sse;
     *rel_out = rel;
     *iters_done = l.it + 1;
-    if (stop && !(rel > criterion)) *stop = 1;
+    if (stop && !(rel > l.criterion)) *stop = 1;
   }
 }
 
@@ -1201,7 +1205,7 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
   const int d = w.d;
   const int groups = (d + 31) / 32;
   LoopIn loop;  // (written by the last block only, at its end)
-  if (threadIdx.x == 0) loop = load_loop(w.iters_done, w.sse_prev);
+  if (threadIdx.x == 0) loop = load_loop(w.iters_done, w.sse_prev, w.criterion);
   for (int j = blockIdx.x; j < w.k; j += gridDim.x) {
     const int live = w.dirty ? pinned(w.dirty + j) : 1;  // uniform over the block
     const int m0 = pinned(w.label_off + j), m1 = pinned(w.label_off + j + 1);
@@ -1268,19 +1272,19 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
   if (threadIdx.x == 0) {
     double sse = 0.0;
     for (int i = 0; i < warps; ++i) sse += red[i];
-    store_sse(sse, loop, sse_out, w.stop, w.criterion, w.sse_prev, w.rel_out, w.iters_done, w.sse_indexed);
+    store_sse(sse, loop, sse_out, w.stop, w.sse_prev, w.rel_out, w.iters_done, w.sse_indexed);
   }
 }
 
 // Second level of the SSE reduction plus the loop's stop rule (host-streamed tiles, shards).
 __global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, double* __restrict__ out,
-                                  int* stop, double criterion, double* sse_prev, double* rel_out,
-                                  int* iters_done, int indexed) {
+                                  int* stop, const double* criterion, double* sse_prev,
+                                  double* rel_out, int* iters_done, int indexed) {
   if (grid_enter()) return;
   if (stopped(stop)) return;
   __shared__ double red[1024];
   LoopIn loop;
-  if (threadIdx.x == 0) loop = load_loop(iters_done, sse_prev);
+  if (threadIdx.x == 0) loop = load_loop(iters_done, sse_prev, criterion);
   const int per = (k + blockDim.x - 1) / blockDim.x;
   double s = 0.0;
   for (int j = threadIdx.x * per; j < min(k, (int)(threadIdx.x + 1) * per); ++j) s += sse_k[j];
@@ -1291,7 +1295,7 @@ __global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, doubl
     __syncthreads();
   }
   if (threadIdx.x == 0)
-    store_sse(red[0], loop, out, stop, criterion, sse_prev, rel_out, iters_done, indexed);
+    store_sse(red[0], loop, out, stop, sse_prev, rel_out, iters_done, indexed);
 }
 
 cudaError_t excl_scan(int* data, long long n, int* tmp, int* ticket, cudaStream_t s,
