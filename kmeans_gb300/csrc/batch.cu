@@ -916,6 +916,17 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
   }
   int dev = 0;
   cudaGetDevice(&dev);
+  // Rows and centers in device memory may still be on their way: as with a handle's, the groups'
+  // streams take their place after the work queued on the default stream.
+  struct Ordered {
+    cudaEvent_t e = nullptr;
+    ~Ordered() {
+      if (e) cudaEventDestroy(e);
+    }
+  } ready;
+  if (!f.code && !f.set(cudaEventCreateWithFlags(&ready.e, cudaEventDisableTiming), KMEANS_ERROR_BUILDDATA,
+                        "default stream"))
+    f.set(cudaEventRecord(ready.e, cudaStreamLegacy), KMEANS_ERROR_BUILDDATA, "default stream");
   auto run_one = [&](Group& g) {
     cudaSetDevice(dev);  // worker threads use the caller's device
     cudaStream_t s = nullptr;
@@ -924,8 +935,9 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
     kmgb_options og = o;
     og.assign_tier = g.tier;
     try {
-      run_group(problems, g.ids, g.d, og, s, &g.reranked, &g.loop_ms, g.phase_ms, g.f, &g.graph_launches,
-                g.audit);
+      if (!g.f.set(cudaStreamWaitEvent(s, ready.e, 0), KMEANS_ERROR_BUILDDATA, "default stream"))
+        run_group(problems, g.ids, g.d, og, s, &g.reranked, &g.loop_ms, g.phase_ms, g.f, &g.graph_launches,
+                  g.audit);
     } catch (const std::exception&) {  // host memory or threads: an exception must not leave a thread
       g.f.code = KMEANS_ERROR_BUILDDATA;
       g.f.msg = "kmgb_lloyd_batched_f32: out of host memory or threads";

@@ -183,3 +183,29 @@ def test_bounds_in_large_batches(km, orc, torch_cuda, tier, policy, criterion):
     for (X, k, init), r in zip(probs, res):
         check(r, orc.lloyd(X, init, 9, criterion=criterion, empty_policy=policy))
     assert st.reserved[7] & 0xFFFFFF == 0
+
+
+@pytest.mark.parametrize("tier", [0, 2])
+def test_rows_still_being_written_on_the_default_stream(km, orc, torch_cuda, tier):
+    """Device rows that work queued on the default stream has yet to write: the call takes its place
+    behind that work, given initial centers in host memory (nothing else would wait for it)."""
+    torch = torch_cuda
+    probs = []
+    for i, (n, d, k) in enumerate([(6000, 32, 20), (9000, 16, 30), (4000, 64, 10)]):
+        X, _, _ = mixture_numpy(n, d, k, seed=300 + i)
+        probs.append((X, k, X[sample_init(n, k, seed=i)].copy()))
+    src = [torch.from_numpy(X).cuda() for X, _, _ in probs]
+    dst = [torch.zeros_like(t) for t in src]
+    a = torch.randn((8192, 8192), device="cuda", dtype=torch.bfloat16)
+    b = torch.empty_like(a)
+    km.lloyd_batched([(t, k, init) for t, (_, k, init) in zip(src, probs)], max_iters=2,
+                     assign_tier=tier)  # the pool holds the call's memory
+    torch.cuda.synchronize()
+    for _ in range(60):  # some 30 ms of work ahead of the rows
+        torch.matmul(a, a, out=b)
+    for t, s in zip(dst, src):
+        t.copy_(s)
+    res, _ = km.lloyd_batched([(t, k, init) for t, (_, k, init) in zip(dst, probs)], max_iters=4,
+                              assign_tier=tier)
+    for (X, k, init), r in zip(probs, res):
+        check(r, orc.lloyd(X, init, 4))
