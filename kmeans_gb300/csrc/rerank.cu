@@ -111,7 +111,7 @@ __global__ void rerank_kernel(RerankArgs a) {
       float lo;
       if (a.mode == 0) lo = v * (1.0f - gam) - 1e-30f;
       else lo = v - e1 - u * 1.01f * fabsf(nbj) - 1e-30f;
-      if (!(lo <= best_hi)) continue;
+      if (!(lo <= best_hi) && !(a.mode == 1 && lo != lo)) continue;  // (NaN: as in exact_pass)
       ++ncand;
       const double ex = exact_value(a.mode, xs, c, a.d, nbj);
       if (ex < best) {  // lanes visit their centers in increasing j: first wins ties
@@ -242,7 +242,9 @@ __device__ __forceinline__ void exact_pass(const RerankArgs& a, const float4* xs
         if (MODE == 0 ? cflag[cl] != 0.0f : j >= a.k) continue;
         const float lo = MODE == 0 ? acc[i][jj] * (1.0f - gam) - 1e-30f
                                    : fmaf(-2.0f, acc[i][jj], cflag[cl]) - es[pl];
-        if (!(lo <= hs[pl])) continue;
+        // MODE 1: a value that overflowed FP32 under an infinite bound says nothing (inf - inf), so
+        // the pair is evaluated; a settled point's NaN end still leaves it alone
+        if (!(lo <= hs[pl]) && !(MODE == 1 && lo != lo && hs[pl] == hs[pl])) continue;
         if (RECORD) {
           const int at = atomicAdd(&ncand[pl], 1);
           if (at < kMaxCand) cand[(g0 + pl) * kMaxCand + at] = j;

@@ -111,3 +111,16 @@ def test_compactness_and_norms(km, torch_cuda, dtype, m, d, k, scale):
         assert (km.colNormalizeF if F else km.colNormalizeD)(m, d, x, q) == 0
         np.testing.assert_allclose(r.cpu().numpy()[2:], rows.astype(dtype), **tol)
         np.testing.assert_allclose(q.cpu().numpy(), cols.astype(dtype), **tol)
+
+
+@pytest.mark.parametrize("n,d,k", [(300, 8, 40), (33, 33, 70), (20_000, 64, 256), (200, 700, 9)])
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_closest_centers_beyond_fp32_range(km, torch_cuda, n, d, k, sign):
+    """Products that overflow FP32 with centers whose norms do not: every center's FP32 value is
+    infinite, the FP64 values decide."""
+    rng = np.random.default_rng(n + k)
+    A = (1e20 * rng.uniform(0.5, 2.0, (n, d))).astype(np.float32)
+    B = (sign * min(1.0, (64 / d) ** 0.5) * rng.uniform(1e18, 2e18, (d, k))).astype(np.float32)
+    nb = (B.astype(np.float64) ** 2).sum(0).astype(np.float32)
+    assert np.isfinite(nb).all()
+    assert np.array_equal(closest(km, torch_cuda, A, B, nb), exact_labels(A, B, nb))
