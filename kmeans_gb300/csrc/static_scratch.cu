@@ -101,16 +101,16 @@ extern "C" kmeansCudaErrorStatus ClusterCentersF_noalloc(const int m0, const int
   plan_update_tiles(m, k, &w.tile_pts, &w.ntiles);
   w.max_pieces = m / kSumPiece + k + 1;
   const long long hist_elems = (long long)k * w.ntiles;
-  // carve the working memory out of the fixed array
+  // carve the working memory out of the fixed array. The block ticket lies where the counters' scan
+  // kept a word per segment: its room stays as it was, so that the same sizes fit the array
   const size_t o_hist = 0;
-  const size_t o_scan = o_hist + align256(sizeof(int) * (size_t)hist_elems);
-  const size_t o_off = o_scan + align256(sizeof(int) * update_scan_tmp_elems(
+  const size_t o_tick = o_hist + align256(sizeof(int) * (size_t)hist_elems);
+  const size_t o_off = o_tick + align256(sizeof(int) * update_scan_tmp_elems(
                                                            hist_elems > k + 1 ? hist_elems : k + 1));
   const size_t o_pcnt = o_off + align256(sizeof(int) * (size_t)(k + 1));
   const size_t o_sorted = o_pcnt + align256(sizeof(int) * (size_t)(k + 1));
   const size_t o_part = o_sorted + align256(sizeof(int) * (size_t)(m > 0 ? m : 1));
-  const size_t o_tick = o_part + align256(sizeof(double) * (size_t)w.max_pieces * n);
-  const size_t total = o_tick + align256(sizeof(int));
+  const size_t total = o_part + align256(sizeof(double) * (size_t)w.max_pieces * n);
   const cudaStream_t stream = 0;  // the reference's per-kernel entries run on the default stream
   cudaError_t e = cudaSuccess;
   // only a call with rows uses the working memory: a finalize-only call (m == 0, lastTile) is
@@ -128,7 +128,6 @@ extern "C" kmeansCudaErrorStatus ClusterCentersF_noalloc(const int m0, const int
     }
     unsigned char* s = static_cast<unsigned char*>(base);
     w.hist = reinterpret_cast<int*>(s + o_hist);
-    w.scan_tmp = reinterpret_cast<int*>(s + o_scan);
     w.label_off = reinterpret_cast<int*>(s + o_off);
     w.piece_cnt = reinterpret_cast<int*>(s + o_pcnt);
     w.sorted = reinterpret_cast<int*>(s + o_sorted);

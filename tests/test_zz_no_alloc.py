@@ -80,3 +80,20 @@ def test_noalloc_finalize_only_call_at_any_size(km, torch_cuda):
         outs.append((cen.cpu().numpy(), cnt.cpu().numpy()))
     assert np.array_equal(outs[0][0], outs[1][0], equal_nan=True)
     assert np.array_equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("m,d,k", [(1_848_512, 8, 37), (1_266_303, 40, 100), (802_752, 100, 100)])
+def test_noalloc_takes_sizes_that_fill_its_array(km, torch_cuda, m, d, k):
+    """These sizes need 8 MiB to the last 256 bytes; 4,096 rows more do not fit."""
+    rng = np.random.default_rng(m)
+    X = rng.standard_normal((m, d), dtype=np.float32)
+    lab = rng.integers(0, k, size=m).astype(np.int32)
+    want_c, want_n = run(km, torch_cuda, km.ClusterCentersF, X, lab, k, 1)
+    got_c, got_n = run(km, torch_cuda, km.ClusterCentersF_noalloc, X, lab, k, 1)
+    assert np.array_equal(got_c, want_c) and np.array_equal(got_n, want_n)
+    t = torch_cuda
+    X = t.zeros((m + 4096, d), device="cuda")
+    lab = t.zeros(m + 4096, dtype=t.int32, device="cuda")
+    big, cen = t.zeros(k * d * 2, device="cuda"), t.zeros((k, d), device="cuda")
+    cnt_big, cnt = (t.zeros(k, dtype=t.int32, device="cuda") for _ in range(2))
+    assert km.ClusterCentersF_noalloc(0, m + 4096, d, k, True, X, lab, big, cnt_big, cen, cnt) == 4
