@@ -412,18 +412,19 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   const long long ld = (d + 3) / 4 * 4, ldb = (d + 7) / 8 * 8;
   const bool direct = ld == d && !(reinterpret_cast<uintptr_t>(A) & 15);  // FP32 kernels' layout
   const long long kp = (k + 127) / 128 * 128;
-  const bool tc = bf16_tc_supported(d, 2) && n >= 256 && n * kp >= (1LL << (kF32 ? 28 : 24)) / d;
+  bool tc = bf16_tc_supported(d, 2) && n >= 256 && n * kp >= (1LL << (kF32 ? 28 : 24)) / d;
   const bool tiled = rerank_tiled_supported(d);
   const int threads = 256;
   const size_t smem = sizeof(double) * (size_t)d * (threads / 32);  // closest_fp64_kernel's
-  if (!kF32 && !tc) {
+  auto scan_fp64 = [&]() -> cudaError_t {
     launch(closest_fp64_kernel, kmgb::num_sms() * 8, threads, smem, kDefault)(
         m0, (int)n, d, reinterpret_cast<const double*>(A), k, reinterpret_cast<const double*>(B),
         reinterpret_cast<const double*>(nb), out, nullptr, nullptr);
     count_launches(1);
     return cudaGetLastError();
-  }
-  const bool copy = !tc && !direct;  // the FP32 scan reads 16-byte aligned rows
+  };
+  if (!kF32 && !tc) return scan_fp64();
+  bool copy = !tc && !direct;  // the FP32 scan reads 16-byte aligned rows
   const long long wave = 256LL * (num_sms() / 2);
   const long long chunk = std::min(n, wave * std::max(1LL, (96LL << 20) / (wave * ldb * 4)));
   const long long cap = std::min(n, std::max(1024LL, n / 8));
@@ -459,12 +460,23 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   Carver size;
   carve(size);
   void* mem = nullptr;
-  KMGB_CUDA_TRY(dev_alloc_async(&mem, size.off, kDefault));
+  cudaError_t e = dev_alloc_async(&mem, size.off, kDefault);
+  if (e == cudaErrorMemoryAllocation && tc) {
+    // no room for the planes and candidates: the scans without them (FP64: without any memory)
+    cudaGetLastError();
+    if (!kF32) return scan_fp64();
+    tc = false;
+    copy = !direct;
+    size = Carver{};
+    carve(size);
+    e = dev_alloc_async(&mem, size.off, kDefault);
+  }
+  if (e) return e;
   Carver cut;
   cut.base = static_cast<char*>(mem);
   carve(cut);
   cmax = reinterpret_cast<float*>(sc);
-  cudaError_t e = cudaMemsetAsync(sc, 0, 8 * sizeof(int), kDefault);
+  e = cudaMemsetAsync(sc, 0, 8 * sizeof(int), kDefault);
   const T* Xa = A;
   if (!e && copy) {
     launch(copy_pad_kernel, num_sms() * 8, 256, 0, kDefault)(reinterpret_cast<const float*>(A), n, d, Ap,

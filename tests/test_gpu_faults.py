@@ -125,3 +125,26 @@ def test_failure_inside_graph_capture_falls_back(km, orc, torch_cuda):
     assert rc == 0
     st, c, lab, sse, it = orc.lloyd(X, init, ITERS)
     assert np.array_equal(res.labels, lab) and np.array_equal(res.centers, c)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_closest_centers_without_room_for_its_planes(km, torch_cuda, dtype):
+    """Sizes that take the tensor-core filter: where its workspace does not fit, the scans that
+    need less memory (FP64: none) give the same labels."""
+    torch = torch_cuda
+    rng = np.random.default_rng(8)
+    n, d, k = 60_000, 64, 128
+    A = (rng.integers(-40, 41, (n, d)) / 8).astype(dtype)
+    B = (rng.integers(-40, 41, (d, k)) / 8).astype(dtype)
+    nb = (B.astype(np.float64) ** 2).sum(0).astype(dtype)
+    want = (nb.astype(np.float64)[None] - 2.0 * (A.astype(np.float64) @ B.astype(np.float64))).argmin(1)
+    a, b, c = (torch.from_numpy(v).cuda() for v in (A, B, nb))
+    fn = km.ClosestCentersF if dtype == np.float32 else km.ClosestCentersD
+    for nth in (0, 1):
+        out = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+        km.debug_fail_nth(km.FAULT_ALLOC, nth)
+        try:
+            assert fn(0, n, d, a, k, b, None, None, c, 0, None, None, out) == 0
+        finally:
+            km.debug_fail_nth(km.FAULT_ALLOC, 0)
+        assert np.array_equal(out.cpu().numpy(), want)
