@@ -193,6 +193,15 @@ struct DevBufs {
     if (e == cudaSuccess) ptrs.push_back(v);
     return e;
   }
+  // Buffers a call can do without: all that `take` allocates, or none of it.
+  template <typename F>
+  bool optional(F take) {
+    const size_t had = ptrs.size();
+    if (take()) return true;
+    cudaGetLastError();
+    for (; ptrs.size() > had; ptrs.pop_back()) dev_free(ptrs.back(), 0);
+    return false;
+  }
 };
 
 #define KD_TRY(expr, code)                \
@@ -214,29 +223,16 @@ void alloc_prune_d(DevBufs& B, PruneState* out, int** crr, long long m, int k, l
   p.k = k;
   p.cap = (int)std::min(m * 13 / 20, (8LL << 30) / (ldb * 4));
   if (p.cap < 256) return;
-  bool ok = true;
-  auto take = [&](auto** q, size_t count) { ok = ok && B.alloc(q, count) == cudaSuccess; };
   uint16_t *xc = nullptr, *xlc = nullptr;
-  take(&p.ub, m);
-  take(&p.lb, m);
-  take(&p.shift, k);
-  take(&p.cxn, k);
-  take(&p.cub, k);
-  take(&p.clb, k);
-  take(&p.clab, k);
-  take(crr, k);
-  take(&p.list, p.cap);
-  take(&p.lab_old, m);
-  take(&p.dirty, k);
-  take(&p.flags, 8);
-  take(&p.top, 2);
-  take(&xc, (size_t)p.cap * ldb);
-  take(&xlc, (size_t)p.cap * ldb);
-  ok = ok && cudaMemsetAsync(p.flags, 0, 8 * sizeof(int), 0) == cudaSuccess;
-  if (!ok) {
-    cudaGetLastError();
+  auto got = [&](auto** q, size_t count) { return B.alloc(q, count) == cudaSuccess; };
+  if (!B.optional([&] {
+        return got(&p.ub, m) && got(&p.lb, m) && got(&p.shift, k) && got(&p.cxn, k) && got(&p.cub, k) &&
+               got(&p.clb, k) && got(&p.clab, k) && got(crr, k) && got(&p.list, p.cap) &&
+               got(&p.lab_old, m) && got(&p.dirty, k) && got(&p.flags, 8) && got(&p.top, 2) &&
+               got(&xc, (size_t)p.cap * ldb) && got(&xlc, (size_t)p.cap * ldb) &&
+               cudaMemsetAsync(p.flags, 0, 8 * sizeof(int), 0) == cudaSuccess;
+      }))
     return;
-  }
   p.Xc = xc;
   p.Xlc = xlc;
   *out = p;
@@ -316,8 +312,10 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
     KD_TRY(B.alloc(&kw.d2, kmeanspp_d2_elems(m)), EI);
     KD_TRY(B.alloc(&kw.blocksum, kmeanspp_blocks(m)), EI);
     KD_TRY(B.alloc(&kw.scalars, kKppScalars), EI);
-    KD_TRY(B.alloc(&kw.near, m), EI);
-    KD_TRY(B.alloc(&kw.cc, k), EI);
+    if (!B.optional([&] {
+          return B.alloc(&kw.near, m) == cudaSuccess && B.alloc(&kw.cc, k) == cudaSuccess;
+        }))
+      kw.near = nullptr, kw.cc = nullptr;  // every draw reads every row
     KD_TRY(B.alloc(&kp, k), EI);
     KD_TRY(B.alloc(&err, 1), EI);
     KD_TRY(cudaMemset(err, 0, sizeof(int)), EI);
@@ -365,7 +363,7 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   int *rr_list = nullptr, *rr_count = nullptr, *derr = nullptr, *over = nullptr, *cand = nullptr,
       *cand_cnt = nullptr;
   // rows of the candidate pass's compact copies; flagged rows past it take the FP64 scan
-  const long long cap = std::min<long long>(m, std::max<long long>(1024, m / 8));
+  long long cap = std::min<long long>(m, std::max<long long>(1024, m / 8));
   PruneState pr;
   int* crr_list = nullptr;
   if (tc) {
@@ -382,17 +380,22 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
     KD_TRY(B.alloc(&cinit, (size_t)((k + kCenterPad - 1) / kCenterPad * kCenterPad)), E);
     KD_TRY(B.alloc(&cbias, (size_t)((k + kCenterPad - 1) / kCenterPad * kCenterPad) * kBiasCols), E);
     KD_TRY(B.alloc(&thr, m), E);
-    KD_TRY(B.alloc(&thrC, cap), E);
-    KD_TRY(B.alloc(&XbC, (size_t)cap * ldb), E);
-    KD_TRY(B.alloc(&XlC, (size_t)cap * ldb), E);
-    KD_TRY(B.alloc(&cand, (size_t)cap * kMaxCand), E);
-    KD_TRY(B.alloc(&cand_cnt, cap), E);
     KD_TRY(B.alloc(&over, m), E);
-    if (maxIters > 1 && prune_worthwhile(m, k, n)) alloc_prune_d(B, &pr, &crr_list, m, k, ldb);
     KD_TRY(B.alloc(&rr_list, m), E);
     KD_TRY(B.alloc(&rr_count, 3), E);
     KD_TRY(B.alloc(&derr, 1), E);
     KD_TRY(cudaMemsetAsync(derr, 0, sizeof(int), s), E);
+    // what can be smaller or missing comes last
+    while (!B.optional([&] {
+      return B.alloc(&thrC, cap) == cudaSuccess && B.alloc(&XbC, (size_t)cap * ldb) == cudaSuccess &&
+             B.alloc(&XlC, (size_t)cap * ldb) == cudaSuccess &&
+             B.alloc(&cand, (size_t)cap * kMaxCand) == cudaSuccess &&
+             B.alloc(&cand_cnt, cap) == cudaSuccess;
+    })) {
+      if (cap <= 1024) return E;
+      cap = std::max<long long>(1024, cap / 4);
+    }
+    if (maxIters > 1 && prune_worthwhile(m, k, n)) alloc_prune_d(B, &pr, &crr_list, m, k, ldb);
     KD_TRY(launch_prep_rows(X, n, m, n, nullptr, xn, Xb, Xl, ldb, nullptr, s), EA);
   }
 

@@ -148,3 +148,37 @@ def test_closest_centers_without_room_for_its_planes(km, torch_cuda, dtype):
         finally:
             km.debug_fail_nth(km.FAULT_ALLOC, 0)
         assert np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("kpp", [False, True])
+def test_double_precision_driver_without_its_optional_memory(km, torch_cuda, kpp):
+    """The candidates' buffers may be smaller, the bounds' and the draws' row-skipping arrays missing:
+    an allocation that fails among them leaves the result as it is; among the others the call fails
+    and gives everything back."""
+    rng = np.random.default_rng(4)
+    n, d, k = 140_000, 64, 200
+    means = rng.uniform(-4, 4, (k, d))
+    X = means[rng.integers(0, k, n)] + rng.standard_normal((n, d))
+
+    def go():
+        out = np.empty(k * d)
+        return km.computeKmeansD(X, n, d, k, -1.0, 4, 1, km.INIT_KMEANSPP if kpp else 0, 0, 0, out, 1.0), out
+
+    rc, want = go()
+    assert rc == km.KMEANS_NONCONVERGENCE
+    base = km.debug_pool_used_bytes()
+    failed = 0
+    for nth in range(1, 61):  # the call makes some fifty allocations
+        km.debug_fail_nth(km.FAULT_ALLOC, nth)
+        rc, got = go()
+        km.debug_fail_nth(km.FAULT_ALLOC, 0)
+        torch_cuda.cuda.synchronize()
+        assert km.debug_pool_used_bytes() == base
+        if rc == km.KMEANS_NONCONVERGENCE:
+            assert np.array_equal(got, want, equal_nan=True)  # (an empty cluster is NaN)
+        else:
+            assert rc in range(1, 13)
+            failed += 1
+    # the required buffers alone: not the five of the candidates, the fifteen of the bounds and the
+    # draws' two
+    assert 0 < failed <= (37 if kpp else 32)
