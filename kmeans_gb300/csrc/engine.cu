@@ -505,8 +505,9 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   }
   // FP32 tier: where thousands of rows can miss its FP32 bounds, the band's centers are recorded as
   // candidates; on smaller data sets the two more launches cost more than the few FP64 rows
-  const bool fp32_band = !tcore && !h->streaming && h->opt.certify && na >= (1 << 16);
+  bool fp32_band = !tcore && !h->streaming && h->opt.certify && na >= (1 << 16);
   if (fp32_band) h->cand_cap = std::max<long long>(1024, na / 32);
+  bool fp32_t = !tcore;  // the centers' transpose, for assign_fp32t_kernel
   h->audit_rows = audit_rows_for(h->opt, h->streaming, k, d);
   UpdateWork& w = h->uw;
   w.n = na;
@@ -543,7 +544,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     }
     a.take(&h->C, (size_t)k * h->ldx);
     a.take(&h->Cop, (size_t)k * h->ldx);
-    if (!tcore) a.take(&h->Ct, (size_t)d * round_up(k, 4));  // (the tiles of assign_fp32t_kernel)
+    if (fp32_t) a.take(&h->Ct, (size_t)d * round_up(k, 4));
     if (bf16) a.take_bytes(&h->Cb, (size_t)k * h->ldb * 2);
     if (split) a.take_bytes(&h->Cl, (size_t)k * h->ldb * 2);
     if (fp8) {
@@ -597,7 +598,17 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   };
   Arena sizing;
   carve(sizing);
-  KM_TRY(dev_alloc(&h->arena, sizing.off, h->stream), (delete h, code));
+  cudaError_t got = dev_alloc(&h->arena, sizing.off, h->stream);
+  if (got == cudaErrorMemoryAllocation && fp32_band) {
+    // no room for all: the FP32 tier also runs without the transpose and the band's candidates
+    cudaGetLastError();
+    fp32_t = fp32_band = false;
+    h->cand_cap = 0;
+    sizing = Arena{};
+    carve(sizing);
+    got = dev_alloc(&h->arena, sizing.off, h->stream);
+  }
+  KM_TRY(got, (delete h, code));
   Arena cut;
   cut.base = static_cast<char*>(h->arena);
   carve(cut);

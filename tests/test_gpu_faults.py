@@ -182,3 +182,22 @@ def test_double_precision_driver_without_its_optional_memory(km, torch_cuda, kpp
     # the required buffers alone: not the five of the candidates, the fifteen of the bounds and the
     # draws' two
     assert 0 < failed <= (37 if kpp else 32)
+
+
+@pytest.mark.parametrize("d", [24, 64])
+def test_fp32_handle_without_room_for_its_extras(km, orc, torch_cuda, d):
+    """The FP32 tier's transposed centers and band candidates are left out where they do not fit:
+    same labels and centers (d = 64: with distance bounds)."""
+    from kmeans_gb300.synthetic import mixture_numpy, sample_init
+    n, k = 70_000, 40
+    X, _, _ = mixture_numpy(n, d, k, seed=31)
+    X[50:60] = X[50]
+    init = X[sample_init(n, k, seed=32)].copy()
+    init[3] = init[9] = X[50]
+    want = orc.lloyd(X, init, 5, empty_policy=1)
+    km.debug_fail_nth(km.FAULT_ALLOC, 1)
+    try:
+        res = km.lloyd(X, k, init=init, max_iters=5, assign_tier=km.ASSIGN_FP32, empty_policy=1)
+    finally:
+        km.debug_fail_nth(km.FAULT_ALLOC, 0)
+    assert np.array_equal(res.labels, want[2]) and np.array_equal(res.centers, want[1])
