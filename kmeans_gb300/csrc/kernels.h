@@ -149,6 +149,9 @@ struct RerankArgs {
   // assignment), stats[1] += counts[full_idx] (points that needed a full rescan of the centers)
   const int* counts;
   int full_idx;
+  // launch_rerank, launch_rerank_settle, mode 1 (nullable): nonzero, every one of the n rows is settled
+  // instead of the list (a wait of the scans gave up, so their list says nothing)
+  const int* redo = nullptr;
 };
 // Any dimension; one warp per point, both modes.
 cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t s);

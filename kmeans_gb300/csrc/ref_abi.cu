@@ -39,12 +39,13 @@ __global__ void copy_pad_kernel(const float* __restrict__ A, long long m, int d,
 }
 
 // FP64 arg-min of nb_j - 2 A_i.B_j (B is d x k, K fastest); one warp per row, lanes over j. list
-// (nullable): only the rows list[0 .. *count).
+// (nullable): only the rows list[0 .. *count), or every row where *redo is set.
 __global__ void closest_fp64_kernel(int m0, int m, int d, const double* __restrict__ A, int k,
                                     const double* __restrict__ B, const double* __restrict__ nb,
                                     int* __restrict__ out, const int* __restrict__ list,
-                                    const int* __restrict__ count) {
+                                    const int* __restrict__ count, const int* redo) {
   if (grid_enter()) return;
+  if (list && pinned(redo) != 0) list = nullptr;
   extern __shared__ double xs_all[];
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* xs = xs_all + (size_t)w * d;
@@ -403,7 +404,8 @@ struct Carver {
 // whose scan runs at 0.6 TFMA/s, from 2^24 on. The rows go through in chunks whose planes stay in L2
 // (and bound the workspace), whole waves of the pair kernel each. What the certificate leaves open
 // is settled from recorded candidates (float-float; FP64 data: FP64), the rest by the tiled stages
-// (FP64 data: a scan of the listed rows). FP32 scan: 898,790 x 128, K=256 took 1.52 ms, its re-rank
+// (FP64 data: a scan of the listed rows). The call returns before its kernels have run, so a scan whose
+// bounded wait gave up is not reported but made up for: the last kernel then takes every row. FP32 scan: 898,790 x 128, K=256 took 1.52 ms, its re-rank
 // 0.28 ms; FP64 scan: 100,000 x 64, K=256 took 2.80 ms.
 template <typename T>
 cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const T* B, const T* nb,
@@ -419,7 +421,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   auto scan_fp64 = [&]() -> cudaError_t {
     launch(closest_fp64_kernel, kmgb::num_sms() * 8, threads, smem, kDefault)(
         m0, (int)n, d, reinterpret_cast<const double*>(A), k, reinterpret_cast<const double*>(B),
-        reinterpret_cast<const double*>(nb), out, nullptr, nullptr);
+        reinterpret_cast<const double*>(nb), out, nullptr, nullptr, nullptr);
     count_launches(1);
     return cudaGetLastError();
   };
@@ -501,6 +503,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   a.k = k;
   a.d = d;
   a.certify = 1;
+  test_wait_hook(&a.test_withhold, &a.test_wait_cycles);  // zero unless a test asks
   if (tc) {
     a.gamma = assign_bf16_gamma(d);
     a.cinit = cinit;
@@ -531,6 +534,10 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
     c2.cand = cand;
     c2.cand_cnt = cand_cnt;
     if (!e) e = launch_assign_bf16(XbC, XlC, ldb, Cb, Cl, ldb, c2, kDefault);
+    if (!e && a.test_withhold) {  // (as a wait of the pair kernel that gave up would leave things)
+      e = cudaMemsetAsync(sc + 4, 1, sizeof(int), kDefault);
+      if (!e) e = cudaMemsetAsync(out + m0, 0xff, sizeof(int) * (size_t)n, kDefault);
+    }
   } else {
     a.gamma = assign_fp32_gamma(d);
     if (!e)
@@ -554,6 +561,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
     r.d = d;
     r.mode = 1;
     r.max_list = tc ? cap : n;
+    r.redo = sc + 4;
     if (!e && tc) e = launch_resolve_expansion(r, cand, cand_cnt, over, sc + 2, kDefault);
     if (tc) {
       r.list = over;
@@ -587,7 +595,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
     if (!e) e = launch_resolve_fp64(r, kDefault);
     if (!e) {
       launch(closest_fp64_kernel, num_sms() * 8, threads, smem, kDefault)(
-          m0, (int)n, d, r.X, k, r.C, r.nb, out, over, sc + 2);
+          m0, (int)n, d, r.X, k, r.C, r.nb, out, over, sc + 2, sc + 4);
       count_launches(1);
       e = cudaGetLastError();
     }

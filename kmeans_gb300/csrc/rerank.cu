@@ -63,12 +63,13 @@ __global__ void rerank_kernel(RerankArgs a) {
   const int warps = blockDim.x >> 5;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* xs = xs_all + (size_t)w * a.d;
-  const long long cnt = min((long long)pinned(a.count), a.max_list);
+  const bool all = a.redo && pinned(a.redo) != 0;
+  const long long cnt = all ? a.n : min((long long)pinned(a.count), a.max_list);
   const float u = 5.9604645e-8f;
   const float gam = (float)(a.d + 4) * 2.0f * u * 1.01f;  // mode 0 relative bound (doubled)
   for (long long slot = (long long)blockIdx.x * warps + w; slot < cnt;
        slot += (long long)gridDim.x * warps) {
-    const int pt = a.list[slot];
+    const int pt = all ? (int)slot : a.list[slot];
     const float* x = a.X + (size_t)pt * a.ldx;
     for (int t = lane; t < a.d; t += 32) xs[t] = x[t];
     __syncwarp();
@@ -183,12 +184,12 @@ __device__ __forceinline__ float expansion_bound(const RerankArgs& a, int pt) {
 
 // The exact pass over the points g0 .. of a.list whose rows lie in xs (see rerank_exact_kernel): every
 // (point, center) pair whose lower end is within the point's best upper end hs (NaN: a settled point,
-// left alone).
+// left alone). all: point g is row g (RerankArgs::redo).
 template <int MODE, bool RECORD>
 __device__ __forceinline__ void exact_pass(const RerankArgs& a, const float4* xs, float4* cs,
                                            float* cflag, int rs, int dq, long long g0, long long cnt,
                                            const float* hs, const float* es, int* __restrict__ cand,
-                                           int* __restrict__ cand_cnt) {
+                                           int* __restrict__ cand_cnt, bool all = false) {
   __shared__ double mb[8][TP];
   __shared__ int mi[8][TP];
   __shared__ int ncand[TP];
@@ -306,7 +307,7 @@ __device__ __forceinline__ void exact_pass(const RerankArgs& a, const float4* xs
       fb = take ? mb[ww][tid] : fb;
       fi = take ? mi[ww][tid] : fi;
     }
-    a.labels[a.list[g0 + tid]] = fi < 0 ? 0 : fi;
+    a.labels[all ? g0 + tid : a.list[g0 + tid]] = fi < 0 ? 0 : fi;
   }
 }
 
@@ -316,7 +317,8 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
                     float* __restrict__ hi2) {
   if (grid_enter()) return;
   const int halt = a.stop ? pinned(a.stop) : 0;
-  const long long cnt = min((long long)pinned(a.count), a.max_list);
+  const bool all = MODE == 1 && SETTLE && a.redo && pinned(a.redo) != 0;
+  const long long cnt = all ? a.n : min((long long)pinned(a.count), a.max_list);
   if (halt) return;
   extern __shared__ float4 sm4[];
   const int dq = (a.d + 3) >> 2;          // float4 per row
@@ -345,7 +347,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
       const int r = e / dq, q = e % dq;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (g0 + r < cnt) {
-        const float* x = a.X + (size_t)a.list[g0 + r] * a.ldx;
+        const float* x = a.X + (size_t)(all ? g0 + r : a.list[g0 + r]) * a.ldx;
         const int c0 = q * 4;
         v.x = c0 < a.d ? x[c0] : 0.f;
         v.y = c0 + 1 < a.d ? x[c0 + 1] : 0.f;
@@ -441,7 +443,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
         fi = take ? oi1 : fi;
         f2 = nb2;
       }
-      const int pt = a.list[g0 + tid];
+      const int pt = all ? (int)(g0 + tid) : a.list[g0 + tid];
       // certified when every other center's lower end exceeds the best's upper end
       float lo2, hi1;
       if (MODE == 0) {
@@ -468,7 +470,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
       es[tid] = 0.0f;
     }
     if (SETTLE && __syncthreads_or(tid < TP && hs[tid] == hs[tid]))
-      exact_pass<MODE, false>(a, xs, cs, cflag, rs, dq, g0, cnt, hs, es, nullptr, nullptr);
+      exact_pass<MODE, false>(a, xs, cs, cflag, rs, dq, g0, cnt, hs, es, nullptr, nullptr, all);
   }
 }
 

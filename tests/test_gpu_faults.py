@@ -201,3 +201,27 @@ def test_fp32_handle_without_room_for_its_extras(km, orc, torch_cuda, d):
     finally:
         km.debug_fail_nth(km.FAULT_ALLOC, 0)
     assert np.array_equal(res.labels, want[2]) and np.array_equal(res.centers, want[1])
+
+
+@pytest.mark.parametrize("dtype,n", [(np.float32, 5_000), (np.float32, 60_000), (np.float64, 60_000)])
+def test_closest_centers_after_a_wait_that_gave_up(km, torch_cuda, dtype, n):
+    """The entry returns before its kernels have run: where a bounded wait of the scan gives up, its
+    last kernel settles every row. (60,000 rows take the tensor-core filter, whose given-up wait is
+    stood in for by its error word and labels of -1.)"""
+    torch = torch_cuda
+    rng = np.random.default_rng(9)
+    d, k = 100, 128
+    A = (rng.integers(-40, 41, (n, d)) / 8).astype(dtype)
+    B = (rng.integers(-40, 41, (d, k)) / 8).astype(dtype)
+    nb = (B.astype(np.float64) ** 2).sum(0).astype(dtype)
+    want = (nb.astype(np.float64)[None] - 2.0 * (A.astype(np.float64) @ B.astype(np.float64))).argmin(1)
+    a, b, c = (torch.from_numpy(v).cuda() for v in (A, B, nb))
+    fn = km.ClosestCentersF if dtype == np.float32 else km.ClosestCentersD
+    out = torch.full((n + 2,), -7, dtype=torch.int32, device="cuda")
+    km.debug_withhold_stage(2, 2_000_000)
+    try:
+        assert fn(2, n, d, a, k, b, None, None, c, 0, None, None, out) == 0
+        torch.cuda.synchronize()
+    finally:
+        km.debug_withhold_stage(0, 0)
+    assert np.array_equal(out.cpu().numpy()[2:], want)
