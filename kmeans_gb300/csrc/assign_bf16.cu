@@ -383,7 +383,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   // where unit u's rows lie: their first row, and whether in the compact copy
   auto unit_rows = [&](long long u, bool& comp) -> long long {
     if (kSel && p.u_src) {
-      const int src = __ldg(p.u_src + u);
+      const int src = ld(p.u_src + u);
       comp = src < 0;
       return src & 0x7fffffff;
     }
@@ -413,7 +413,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       if (p.g_done && p.g_done[pr]) return false;
       ui.nch = (p.g_k[pr] + BN - 1) / BN;
       ui.cbase = p.g_coff[pr];
-      ui.rend = kSel && p.u_cnt ? u * UNIT + __ldg(p.u_cnt + u) : p.g_rend[pr];
+      ui.rend = kSel && p.u_cnt ? u * UNIT + ld(p.u_cnt + u) : p.g_rend[pr];
       ui.cend = ui.cbase + p.g_k[pr];
     }
     ui.rot = (int)(pair % ui.nch);
@@ -616,7 +616,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const int q = warp & 3;       // TMEM lane quadrant this warp may access
     const int h = e >> 2;         // column slice of the chunk (0 .. EPI_PER_QUAD-1)
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-    const float cm = (p.certify || XMAX) ? __ldg(p.cmax) : 0.0f;
+    const float cm = (p.certify || XMAX) ? ld(p.cmax) : 0.0f;
     const uint32_t acc_empty_leader0 = map_to_rank(smem_u32(&bars.acc_empty[0]), 0);
     const uint32_t acc_empty_leader1 = map_to_rank(smem_u32(&bars.acc_empty[1]), 0);
 
@@ -624,7 +624,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     auto row_of = [&](long long u, long long prow) -> long long {
       bool comp;
       const long long r = unit_rows(u, comp) + (prow - u * UNIT);
-      return comp ? (long long)__ldg(p.row_map + r) : p.out0 + r;
+      return comp ? (long long)ld(p.row_map + r) : p.out0 + r;
     };
     bool alive = true;
     for (long long g0 = 0; g0 < 2 && g0 < total_chunks; ++g0)  // both buffers start free
@@ -640,18 +640,18 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       const long long prow = u * UNIT + rank * BM + q * 32 + lane;  // row within the launch
       float floor_key = INFINITY;  // candidate mode: record keys >= floor_key
       int ncand = 0;
-      if (cand_mode && prow < n_rows) floor_key = __ldg(p.thr_in + p.row0 + prow);
+      if (cand_mode && prow < n_rows) floor_key = ld(p.thr_in + p.row0 + prow);
       // the point's norm bound is needed only after the last chunk: load it now so that its
       // HBM latency hides behind the unit's chunks
       const float xn_pt = ((p.certify || XMAX) && !cand_mode && h == 0 && prow < n_rows)
-                              ? __ldg(p.xnorm + row_of(u, prow)) : 0.0f;
+                              ? ld(p.xnorm + row_of(u, prow)) : 0.0f;
       // separation mode: the unit's rows (one group: groups fill whole 256-row units) skip the
       // chunks of their own group
-      const int unit_group = XMAX ? __ldg(p.slot_group + u * UNIT) : 0;
+      const int unit_group = XMAX ? ld(p.slot_group + u * UNIT) : 0;
       // FP8 tier: the row's scale and the accumulator multiplier sx * sc (a power of two)
       const float sx_pt = (fp8 && prow < n_rows)
-                              ? __ldg(p.xscale + (cand_mode ? p.row0 : p.out0) + prow) : 0.0f;
-      const float sc_all = fp8 ? __ldg(p.cscale) : 0.0f;
+                              ? ld(p.xscale + (cand_mode ? p.row0 : p.out0) + prow) : 0.0f;
+      const float sc_all = fp8 ? ld(p.cscale) : 0.0f;
       const float mrow = sx_pt * sc_all;
       for (int c = 0; c < ui.nch; ++c, ++g) {
         const int b = (int)(g & 1);
@@ -677,7 +677,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(b ? acc_empty_leader1 : acc_empty_leader0);
-        if (XMAX && __ldg(p.slot_group + chunk0) == unit_group) continue;
+        if (XMAX && ld(p.slot_group + chunk0) == unit_group) continue;
 #pragma unroll
         for (int cb = 0; cb < COLS_PER_WARP / 32; ++cb) {
           // a 32-column block wholly past the problem's centers holds padding only (unusable
@@ -692,7 +692,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             if (fp8) {
 #pragma unroll
               for (int j4 = 0; j4 < 8; ++j4) {
-                const float4 hv = __ldg(hs + j4);
+                const float4 hv = hs[j4];
                 cur[4 * j4 + 0] = __float_as_uint(__fmaf_rn(__uint_as_float(cur[4 * j4 + 0]), mrow, hv.x));
                 cur[4 * j4 + 1] = __float_as_uint(__fmaf_rn(__uint_as_float(cur[4 * j4 + 1]), mrow, hv.y));
                 cur[4 * j4 + 2] = __float_as_uint(__fmaf_rn(__uint_as_float(cur[4 * j4 + 2]), mrow, hv.z));
@@ -701,7 +701,7 @@ assign_bf16_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             } else if (!bias) {
 #pragma unroll
               for (int j4 = 0; j4 < 8; ++j4) {
-                const float4 hv = __ldg(hs + j4);
+                const float4 hv = hs[j4];
                 cur[4 * j4 + 0] = __float_as_uint(__fadd_rn(__uint_as_float(cur[4 * j4 + 0]), hv.x));
                 cur[4 * j4 + 1] = __float_as_uint(__fadd_rn(__uint_as_float(cur[4 * j4 + 1]), hv.y));
                 cur[4 * j4 + 2] = __float_as_uint(__fadd_rn(__uint_as_float(cur[4 * j4 + 2]), hv.z));

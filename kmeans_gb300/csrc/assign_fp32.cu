@@ -106,15 +106,15 @@ __device__ __forceinline__ void settle_tile(const AssignArgs& p, bool compact, l
   }
 
   if (tx == 0) {
-    const float cm = p.certify ? __ldg(p.cmax) : 0.0f;
+    const float cm = p.certify ? ld(p.cmax) : 0.0f;
 #pragma unroll
     for (int i = 0; i < P; ++i) {
       const long long row = row0 + ty + (BM / P) * i;
       if (row < n_rows) {
-        const long long pt = compact ? (long long)__ldg(p.row_map + row) : row;
+        const long long pt = compact ? (long long)ld(p.row_map + row) : row;
         p.labels[pt] = i1[i] < 0 ? 0 : i1[i];
         if (p.certify) {
-          const float xn = __ldg(p.xnorm + pt);
+          const float xn = ld(p.xnorm + pt);
           const float e = bound_e(xn, cm, p.gamma, p.d);
           const float margin = b2[i] - b1[i];
           const bool flagged = !(margin > 2.0f * e);
@@ -256,7 +256,7 @@ assign_fp32_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int c = chunk * BN + tx + 16 * j;
-      cnv[j] = (c < p.k) ? __ldg(p.cn + c) : INFINITY;
+      cnv[j] = (c < p.k) ? ld(p.cn + c) : INFINITY;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -436,7 +436,7 @@ assign_fp32t_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const int c = c0 + (j & 3) + 32 * (j >> 2);
-      const float cnv = (c < p.k) ? __ldg(p.cn + c) : INFINITY;
+      const float cnv = (c < p.k) ? ld(p.cn + c) : INFINITY;
 #pragma unroll
       for (int i = 0; i < P; ++i) {
         float lo, hi;
@@ -532,7 +532,7 @@ assign_fp32_grouped_kernel(const __grid_constant__ CUtensorMap tmX,
   const int lane = tid & 31;
   const int tx = tid & 15;
   const int ty = tid >> 4;
-  const float cm = p.certify ? __ldg(p.cmax) : 0.0f;
+  const float cm = p.certify ? ld(p.cmax) : 0.0f;
   long long s = 0;  // steps consumed
   bool alive = true;
   for (long long t = first_tile(blockIdx.x); t < ntiles && alive; t = first_tile(t + gridDim.x)) {
@@ -588,7 +588,7 @@ assign_fp32_grouped_kernel(const __grid_constant__ CUtensorMap tmX,
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int c = chunk * BN + tx + 16 * j;
-        cnv[j] = (c < kp) ? __ldg(p.cn + cbeg + c) : INFINITY;
+        cnv[j] = (c < kp) ? ld(p.cn + cbeg + c) : INFINITY;
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -625,7 +625,7 @@ assign_fp32_grouped_kernel(const __grid_constant__ CUtensorMap tmX,
         if (pt < rend) {
           p.labels[pt] = cbeg + (i1[i] < 0 ? 0 : i1[i]);
           if (p.certify) {
-            const float e = bound_e(__ldg(p.xnorm + pt), cm, p.gamma, p.d);
+            const float e = bound_e(ld(p.xnorm + pt), cm, p.gamma, p.d);
             const float margin = b2[i] - b1[i];
             if (!(margin > 2.0f * e)) {
               const int slot = atomicAdd(p.rerank_count, 1);

@@ -121,6 +121,89 @@ __device__ __forceinline__ bool grid_enter() {
   return z != 0;
 }
 
+// Kernels load global memory through coherent loads: one that launch() starts may begin while the grid
+// before it still writes, so what that grid writes is not read-only for the kernel's lifetime, as __ldg and
+// const __restrict__ kernel parameters (which the compiler turns into the same instruction) require.
+// grid_enter() orders the loads after the grid's end and, for coherent loads, makes its writes visible.
+// ld: one that stays in its place among the others, ahead of what is written after it (free to move, loads
+// for the next step of a loop ended up behind the work they were to overlap).
+__device__ __forceinline__ void ld_to(const int* p, int& v) {
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+}
+__device__ __forceinline__ void ld_to(const float* p, float& v) {
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+}
+__device__ __forceinline__ void ld_to(const double* p, double& v) {
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+}
+__device__ __forceinline__ void ld_to(const float4* p, float4& v) {
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+}
+__device__ __forceinline__ void ld_to(const uint4* p, uint4& v) {
+  asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+}
+__device__ __forceinline__ void ld_to(const double2* p, double2& v) {
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+}
+template <typename T>
+__device__ __forceinline__ T ld(const T* p) {
+  T v;
+  ld_to(p, v);
+  return v;
+}
+
+// Rows list[slot], slot < cnt, of one or two planes of row_vec 16-byte vectors a row, into rows `slot` of
+// their compact copies, by the warps w0, w0 + nw, ... (16 bytes a lane). Four loads a lane stand ahead of
+// their stores, which a coherent load does not pass: 86 us an iteration (mean of the first four) of
+// 4M x 128, K=1024; 151 with a load and a store at a time, 123 with the non-coherent loads that the
+// compiler moved ahead itself.
+__device__ __forceinline__ void copy_listed_rows(const int* list, long long cnt, const uint4* Xb,
+                                                 const uint4* Xl, int row_vec, uint4* XbC, uint4* XlC,
+                                                 long long w0, long long nw, int lane) {
+  const int per = Xl ? 2 * row_vec : row_vec;
+  if (per <= 32) {  // 32 / per rows a step, four steps together
+    constexpr int U = 4;
+    const int rows = 32 / per, rr = lane / per, v = lane - rr * per;
+    const uint4* src = v < row_vec ? Xb + v : Xl + (v - row_vec);
+    uint4* dst = v < row_vec ? XbC + v : XlC + (v - row_vec);
+    for (long long s0 = w0 * rows * U; s0 < cnt; s0 += nw * rows * U) {
+      int pt[U];
+      uint4 x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long slot = s0 + u * rows + rr;
+        pt[u] = ld(list + (slot < cnt ? slot : cnt - 1));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = ld(src + (size_t)pt[u] * row_vec);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long slot = s0 + u * rows + rr;
+        if (rr < rows && slot < cnt) dst[(size_t)slot * row_vec] = x[u];
+      }
+    }
+    return;
+  }
+  for (long long s0 = 2 * w0; s0 < cnt; s0 += 2 * nw) {  // two rows, two vectors of each
+    const bool two = s0 + 1 < cnt;
+    const size_t p0 = (size_t)ld(list + s0) * row_vec, p1 = (size_t)ld(list + s0 + two) * row_vec;
+    const size_t d0 = (size_t)s0 * row_vec, d1 = d0 + row_vec;
+    for (int v0 = lane; v0 < per; v0 += 64) {
+      const bool more = v0 + 32 < per;
+      const int v1 = more ? v0 + 32 : v0;
+      const uint4* a = v0 < row_vec ? Xb + v0 : Xl + (v0 - row_vec);
+      const uint4* b = v1 < row_vec ? Xb + v1 : Xl + (v1 - row_vec);
+      uint4* ao = v0 < row_vec ? XbC + v0 : XlC + (v0 - row_vec);
+      uint4* bo = v1 < row_vec ? XbC + v1 : XlC + (v1 - row_vec);
+      const uint4 x0 = ld(a + p0), x1 = ld(a + p1), y0 = ld(b + p0), y1 = ld(b + p1);
+      ao[d0] = x0;
+      if (two) ao[d1] = x1;
+      if (more) bo[d0] = y0;
+      if (more && two) bo[d1] = y1;
+    }
+  }
+}
+
 // A load that stays where it is written, ahead of the test of a flag loaded with it: one after the
 // other, the flags and counts at a kernel's start cost a round trip to L2 (900 cycles) each. It goes
 // through L1 (a volatile load of one word by every warp of a large grid does not: 6.8 -> 13.3 us for two

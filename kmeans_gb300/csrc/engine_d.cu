@@ -27,7 +27,7 @@ using namespace kmgb;
 namespace {
 
 // CT[t][j] = C[j][t]
-__global__ void transpose_d_kernel(const double* __restrict__ C, int k, int d, double* __restrict__ CT) {
+__global__ void transpose_d_kernel(const double* C, int k, int d, double* __restrict__ CT) {
   if (grid_enter()) return;
   const long long total = (long long)k * d;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
@@ -39,10 +39,10 @@ __global__ void transpose_d_kernel(const double* __restrict__ C, int k, int d, d
 
 // One warp per point, lanes over centers (coalesced reads of CT); exact FP64 direct distance.
 // list (nullable): only the points list[0 .. *count) (the tensor pass's uncertified points).
-__global__ void assign_d_kernel(const double* __restrict__ X, long long n, int d,
-                                const double* __restrict__ CT, int k, int* __restrict__ labels,
-                                const int* __restrict__ list,
-                                const int* __restrict__ count) {
+__global__ void assign_d_kernel(const double* X, long long n, int d,
+                                const double* CT, int k, int* __restrict__ labels,
+                                const int* list,
+                                const int* count) {
   if (grid_enter()) return;
   extern __shared__ double xs_all[];
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -79,7 +79,7 @@ __global__ void assign_d_kernel(const double* __restrict__ X, long long n, int d
 }
 
 // out[r][c] = (float)in[r][c] (round to nearest) for c < d, 0 for d <= c < ldo.
-__global__ void d2f_kernel(const double* __restrict__ in, long long rows, int d,
+__global__ void d2f_kernel(const double* in, long long rows, int d,
                            float* __restrict__ out, long long ldo) {
   if (grid_enter()) return;
   const long long total = rows * ldo;
@@ -94,9 +94,9 @@ __global__ void d2f_kernel(const double* __restrict__ in, long long rows, int d,
 // each, as the canonical sums): one warp per piece, lanes over the dimensions, four rows in flight;
 // the lanes meet once per piece.
 __global__ void __launch_bounds__(128)
-sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ sorted,
-                  const int* __restrict__ label_off, const int* __restrict__ pstart, int k,
-                  const double* __restrict__ C, double* __restrict__ piece) {
+sse_pieces_kernel(const double* X, int d, const int* sorted,
+                  const int* label_off, const int* pstart, int k,
+                  const double* C, double* __restrict__ piece) {
   if (grid_enter()) return;
   const int total = pstart[k];
   const int lane = threadIdx.x & 31;
@@ -106,7 +106,7 @@ sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ s
     int lo = 0, hi = k - 1;  // the cluster of piece p
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(pstart + mid) <= p) lo = mid;
+      if (ld(pstart + mid) <= p) lo = mid;
       else hi = mid - 1;
     }
     const int b = label_off[lo] + (p - pstart[lo]) * kSumPiece;
@@ -114,7 +114,7 @@ sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ s
     const double* c = C + (size_t)lo * d;
     double acc = 0.0;
     for (int t0 = b; t0 < e; t0 += 32) {
-      const int ids = t0 + lane < e ? __ldg(sorted + t0 + lane) : 0;
+      const int ids = t0 + lane < e ? ld(sorted + t0 + lane) : 0;
       const int cnt = min(32, e - t0);
       for (int h = 0; h < cnt; h += U) {
         const double* x[U];
@@ -122,10 +122,10 @@ sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ s
         for (int u = 0; u < U; ++u)
           x[u] = X + (size_t)__shfl_sync(0xffffffffu, ids, min(h + u, cnt - 1)) * d;
         for (int t = lane; t < d; t += 32) {
-          const double cv = __ldg(c + t);
+          const double cv = ld(c + t);
           double v[U];
 #pragma unroll
-          for (int u = 0; u < U; ++u) v[u] = __ldg(x[u] + t) - cv;
+          for (int u = 0; u < U; ++u) v[u] = ld(x[u] + t) - cv;
 #pragma unroll
           for (int u = 0; u < U; ++u)
             if (h + u < cnt) acc = fma(v[u], v[u], acc);
@@ -140,8 +140,8 @@ sse_pieces_kernel(const double* __restrict__ X, int d, const int* __restrict__ s
 // One block: every cluster's SSE from its pieces (in order; a cluster without pieces in this
 // iteration keeps its value), and their sum.
 __global__ void __launch_bounds__(1024)
-sse_d_final_kernel(const double* __restrict__ piece, const int* __restrict__ pstart, int k,
-                   const int* __restrict__ dirty, double* __restrict__ sse_k, double* out) {
+sse_d_final_kernel(const double* piece, const int* pstart, int k,
+                   const int* dirty, double* __restrict__ sse_k, double* out) {
   if (grid_enter()) return;
   __shared__ double red[1024];
   double t = 0.0;
@@ -164,7 +164,7 @@ sse_d_final_kernel(const double* __restrict__ piece, const int* __restrict__ pst
   if (threadIdx.x == 0) *out = red[0];
 }
 
-__global__ void gather_d_kernel(const double* __restrict__ X, int d, const int* __restrict__ perm,
+__global__ void gather_d_kernel(const double* X, int d, const int* perm,
                                 long long m, long long start, long long m_mb, double* __restrict__ Xw) {
   if (grid_enter()) return;
   const long long total = m_mb * d;

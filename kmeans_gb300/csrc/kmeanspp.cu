@@ -106,8 +106,8 @@ constexpr int KPP_ROWS = 4;
 
 template <typename T>
 __global__ void __launch_bounds__(KPP_THREADS)
-kpp_update_kernel(const T* __restrict__ X, long long ldx, long long n, int d,
-                  const int* __restrict__ pick, T* __restrict__ d2, int first,
+kpp_update_kernel(const T* X, long long ldx, long long n, int d,
+                  const int* pick, T* __restrict__ d2, int first,
                   unsigned long long* __restrict__ max_key) {
   if (grid_enter()) return;
   __shared__ unsigned long long wmax[KPP_THREADS / 32];
@@ -128,10 +128,10 @@ kpp_update_kernel(const T* __restrict__ X, long long ldx, long long n, int d,
     }
 #pragma unroll 4
     for (int t = lane; t < d; t += 32) {
-      const T cv = __ldg(c + t);
+      const T cv = ld(c + t);
 #pragma unroll
       for (int r = 0; r < KPP_ROWS; ++r) {
-        const T u = __ldg(x[r] + t) - cv;
+        const T u = ld(x[r] + t) - cv;
         s[r] = kpp_fma(u, u, s[r]);
       }
     }
@@ -260,7 +260,7 @@ __device__ __forceinline__ T kpp_gather_rows(const T* __restrict__ X, long long 
       a = nr.near[i + step];
     }
     const bool skip = !in || cur == T(0) ||
-                      (kpp_in_range(cur) && __ldg(cc + cura) >= slack * cur);
+                      (kpp_in_range(cur) && ld(cc + cura) >= slack * cur);
     unsigned todo = __ballot_sync(0xffffffffu, !skip);
     read += __popc(todo);
     if (in && skip) mx = fmax(mx, cur);
@@ -287,7 +287,7 @@ __device__ __forceinline__ T kpp_gather_rows(const T* __restrict__ X, long long 
 #pragma unroll
         for (int q = 0; q < kSteps; ++q)
 #pragma unroll
-          for (int r = 0; r < 8; ++r) xv[q][r] = t0 + 32 * q < d ? __ldg(x[r] + t0 + 32 * q) : T(0);
+          for (int r = 0; r < 8; ++r) xv[q][r] = t0 + 32 * q < d ? ld(x[r] + t0 + 32 * q) : T(0);
 #pragma unroll
         for (int q = 0; q < kSteps; ++q) {
           if (t0 + 32 * q >= d) break;
@@ -320,8 +320,8 @@ __device__ __forceinline__ T kpp_gather_rows(const T* __restrict__ X, long long 
 
 template <typename T>
 __global__ void __launch_bounds__(KPP_BULK_THREADS)
-kpp_update_bulk_kernel(const T* __restrict__ X, long long ldx, long long n, int d,
-                       const int* __restrict__ pick, T* __restrict__ d2, int first,
+kpp_update_bulk_kernel(const T* X, long long ldx, long long n, int d,
+                       const int* pick, T* __restrict__ d2, int first,
                        unsigned long long* __restrict__ max_key, int rows_per_stage, int stages,
                        int* __restrict__ err, KppNear nr) {
   if (grid_enter()) return;
@@ -444,8 +444,8 @@ kpp_update_bulk_kernel(const T* __restrict__ X, long long ldx, long long n, int 
 // Lower bounds of the squared distances from the newest center (row *pick) to the centers of draws
 // 0 .. draw-1 (rows picks[q]), one warp each; block 0 closes the last gathering draw's count.
 template <typename T>
-__global__ void kpp_center_dist_kernel(const T* __restrict__ X, long long ldx, int d,
-                                       const int* __restrict__ picks, int draw, T* __restrict__ cc,
+__global__ void kpp_center_dist_kernel(const T* X, long long ldx, int d,
+                                       const int* picks, int draw, T* __restrict__ cc,
                                        unsigned int* __restrict__ active) {
   if (grid_enter()) return;
   const int q = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -459,7 +459,7 @@ __global__ void kpp_center_dist_kernel(const T* __restrict__ X, long long ldx, i
   const T* o = X + (size_t)picks[q] * ldx;
   T s = T(0);
   for (int t = lane; t < d; t += 32) {
-    const T u = __ldg(c + t) - __ldg(o + t);
+    const T u = ld(c + t) - ld(o + t);
     s = kpp_fma(u, u, s);
   }
   for (int m = 16; m > 0; m >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, m);
@@ -472,8 +472,8 @@ __global__ void kpp_center_dist_kernel(const T* __restrict__ X, long long ldx, i
 // (round 0) the sums are zero and the draw uniform.
 template <typename T>
 __global__ void __launch_bounds__(KPP_BLOCK)
-kpp_draw_kernel(long long n, const T* __restrict__ d2, unsigned long long* blocksum, long long nblocks,
-                bool weights, const unsigned long long* __restrict__ max_key,
+kpp_draw_kernel(long long n, const T* d2, unsigned long long* blocksum, long long nblocks,
+                bool weights, const unsigned long long* max_key,
                 unsigned long long* __restrict__ next_max_key, unsigned int* ticket,
                 unsigned long long seed, int round, int* __restrict__ pick, int* __restrict__ picks) {
   if (grid_enter()) return;
@@ -488,7 +488,7 @@ kpp_draw_kernel(long long n, const T* __restrict__ d2, unsigned long long* block
       const long long p0 = b * (long long)KPP_BLOCK + lane;
       T v[KPP_BLOCK / 32];
 #pragma unroll
-      for (int i = 0; i < KPP_BLOCK / 32; ++i) v[i] = p0 + 32 * i < n ? __ldg(d2 + p0 + 32 * i) : T(0);
+      for (int i = 0; i < KPP_BLOCK / 32; ++i) v[i] = p0 + 32 * i < n ? ld(d2 + p0 + 32 * i) : T(0);
       unsigned long long q = 0;
 #pragma unroll
       for (int i = 0; i < KPP_BLOCK / 32; ++i) q += kpp_weight(v[i], scale);
@@ -551,8 +551,8 @@ kpp_draw_kernel(long long n, const T* __restrict__ d2, unsigned long long* block
 }
 
 template <typename T>
-__global__ void kpp_gather_kernel(const T* __restrict__ X, long long ldx, int d,
-                                  const int* __restrict__ picks, int k, T* __restrict__ C,
+__global__ void kpp_gather_kernel(const T* X, long long ldx, int d,
+                                  const int* picks, int k, T* __restrict__ C,
                                   long long ldc) {
   if (grid_enter()) return;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < (long long)k * d;

@@ -49,7 +49,7 @@ __device__ __forceinline__ void ff_square_add(float v, float& hi, float& lo) {
 // flight. The norm is an error-free float-float sum on the FP32 pipe as a row's (prep_rows_kernel): an
 // FP64 chain per lane, its tree and two FP64 square roots in passes of their own took 36.5 us for
 // 16,384 x 256 (now 16.9) and 6.6 us for 256 x 128 (4.0).
-__global__ void prep_centers_kernel(const float* __restrict__ C, long long ldc, int k, int d,
+__global__ void prep_centers_kernel(const float* C, long long ldc, int k, int d,
                                     float* __restrict__ Cop, __nv_bfloat16* __restrict__ Cb,
                                     long long ldcb, float* __restrict__ cn, float* cmax,
                                     const int* stop, float* __restrict__ cinit, int kpad,
@@ -183,17 +183,17 @@ template <typename T>
 __device__ __forceinline__ float4 load_row4(const T* __restrict__ x, int c, int d, bool vec) {
   float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
   if (sizeof(T) == 4) {
-    if (vec && c + 4 <= d) return __ldg(reinterpret_cast<const float4*>(x + c));
+    if (vec && c + 4 <= d) return ld(reinterpret_cast<const float4*>(x + c));
   } else if (vec && c + 4 <= d) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(x + c));
-    const double2 b = __ldg(reinterpret_cast<const double2*>(x + c + 2));
+    const double2 a = ld(reinterpret_cast<const double2*>(x + c));
+    const double2 b = ld(reinterpret_cast<const double2*>(x + c + 2));
     return make_float4(__double2float_rn(a.x), __double2float_rn(a.y), __double2float_rn(b.x),
                        __double2float_rn(b.y));
   }
-  if (c < d) v.x = (float)__ldg(x + c);
-  if (c + 1 < d) v.y = (float)__ldg(x + c + 1);
-  if (c + 2 < d) v.z = (float)__ldg(x + c + 2);
-  if (c + 3 < d) v.w = (float)__ldg(x + c + 3);
+  if (c < d) v.x = (float)ld(x + c);
+  if (c + 1 < d) v.y = (float)ld(x + c + 1);
+  if (c + 2 < d) v.z = (float)ld(x + c + 2);
+  if (c + 3 < d) v.w = (float)ld(x + c + 3);
   return v;
 }
 
@@ -213,7 +213,7 @@ __device__ __forceinline__ float4 widen4(uint2 b) {
 // rows, their norms and their planes were three launches: 32 + 6 + 19 us for 89,879 x 128).
 template <typename T, int L, int IDX>
 __global__ void __launch_bounds__(256)
-prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, bool vec,
+prep_rows_kernel(const T* X, long long ldx, long long n, int d, bool vec,
                  double* __restrict__ qn, float* __restrict__ xn, uint2* __restrict__ Xb,
                  uint2* __restrict__ Xl, int ldb, int* inexact, float* __restrict__ nf, RowList rl,
                  RowWindow rw, const int* stop) {
@@ -235,10 +235,10 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
   long long start = 0;
   if (IDX == 2) start = (((long long)*rw.base + *rw.done) * n) % rw.m;
   auto source = [&](long long r) -> long long {
-    if (IDX == 1) return __ldg(rl.list + r);
+    if (IDX == 1) return ld(rl.list + r);
     if (IDX == 2) {
       const long long pos = start + r;
-      return __ldg(rw.perm + (pos >= rw.m ? pos - rw.m : pos));
+      return ld(rw.perm + (pos >= rw.m ? pos - rw.m : pos));
     }
     return r;
   };
@@ -322,7 +322,7 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
         double sd = 0.0;
         if (ru < n)
           for (int t = sub; t < d; t += L) {
-            const double x = (double)(float)__ldg(X + (size_t)source(ru) * ldx + t);
+            const double x = (double)(float)ld(X + (size_t)source(ru) * ldx + t);
             sd = fma(x, x, sd);
           }
         for (int o = L / 2; o > 0; o >>= 1) sd += __shfl_xor_sync(0xffffffffu, sd, o);
@@ -352,7 +352,7 @@ prep_rows_kernel(const T* __restrict__ X, long long ldx, long long n, int d, boo
 // (infinite elements, a norm of -inf, magnitudes beyond 1e18) raises it to 3e38: every row then
 // misses its certificate and is settled exactly.
 template <typename T>
-__global__ void prep_expansion_kernel(const T* __restrict__ B, int d, int k, const T* __restrict__ nb,
+__global__ void prep_expansion_kernel(const T* B, int d, int k, const T* nb,
                                       float* __restrict__ Bt, long long ld, float* __restrict__ nbx,
                                       __nv_bfloat16* __restrict__ Cb, __nv_bfloat16* __restrict__ Cl,
                                       long long ldb, float* __restrict__ cinit,
@@ -414,7 +414,7 @@ __device__ __forceinline__ float pow2_scale_for(float mx) {
 }
 
 // One warp per row: the row's scale (sx[row]) and its E4M3 copy, zero padded to ld8 bytes.
-__global__ void to_fp8_kernel(const float* __restrict__ X, long long ldx, long long n, int d,
+__global__ void to_fp8_kernel(const float* X, long long ldx, long long n, int d,
                               uint8_t* __restrict__ X8, long long ld8, float* __restrict__ sx,
                               const int* stop) {
   if (grid_enter()) return;
@@ -438,8 +438,8 @@ __global__ void to_fp8_kernel(const float* __restrict__ X, long long ldx, long l
 
 // The centers' E4M3 copy with one scale for all of them, from the operand copy (unusable centers
 // are zero rows) and the bound of the largest center norm: cscale = 2^(e - 8), cmax < 2^e.
-__global__ void centers_fp8_kernel(const float* __restrict__ Cop, long long ldc, int k, int d,
-                                   const float* __restrict__ cmax, uint8_t* __restrict__ C8,
+__global__ void centers_fp8_kernel(const float* Cop, long long ldc, int k, int d,
+                                   const float* cmax, uint8_t* __restrict__ C8,
                                    long long ld8, float* __restrict__ cscale, const int* stop) {
   if (grid_enter()) return;
   if (stopped(stop)) return;

@@ -88,7 +88,7 @@ prune_top_kernel(PruneState ps, const int* stop) {
 // `cap` rows are listed every row will be scanned (and its bounds written anew): the blocks still
 // to come return.
 __global__ void __launch_bounds__(PF_THREADS)
-prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
+prune_filter_kernel(PruneState ps, const int* labels, const int* stop) {
   if (grid_enter()) return;
   if (stopped(stop)) return;
   __shared__ int wsum[PF_THREADS / 32];
@@ -125,8 +125,8 @@ prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* st
     for (int r = 0; r < 4; ++r) {
       if (i0 + r >= ps.n) continue;
       const bool lab_ok = a[r] >= 0 && a[r] < ps.k;  // always, but for an error upstream
-      const float sh = lab_ok ? __ldg(ps.shift + a[r]) : -1.0f;
-      const float near = lab_ok ? __ldg(ps.clb + a[r]) : 0.0f;
+      const float sh = lab_ok ? ld(ps.shift + a[r]) : -1.0f;
+      const float near = lab_ok ? ld(ps.clb + a[r]) : 0.0f;
       u[r] = sh < 0.0f ? INFINITY : __fadd_ru(u[r], sh);
       l[r] = __fsub_rd(l[r], a[r] == topi ? top2 : top1);
       // the nearest other center is at least `near` from this one, hence near - ub from the row;
@@ -177,44 +177,17 @@ prune_filter_kernel(PruneState ps, const int* __restrict__ labels, const int* st
   }
 }
 
-// One warp per listed row, 16-byte moves, both planes' loads of a row in flight together.
-__global__ void prune_gather_kernel(PruneState ps, const uint4* __restrict__ Xb,
-                                    const uint4* __restrict__ Xl, int row_vec, const int* stop) {
+__global__ void __launch_bounds__(256, 4)
+prune_gather_kernel(PruneState ps, const uint4* Xb, const uint4* Xl, int row_vec,
+                                    const int* stop) {
   if (grid_enter()) return;
   const int halt = stop ? pinned(stop) : 0;
   const int cnt = pinned(ps.flags + 1);
   if (halt) return;
   if (cnt > ps.cap) return;
-  const int lane = threadIdx.x & 31;
-  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  uint4* Xc = static_cast<uint4*>(ps.Xc);
-  uint4* Xlc = static_cast<uint4*>(ps.Xlc);
-  const int planes = Xl ? 2 : 1;
-  const int per = row_vec * planes;
-  // rows of both planes as one run of `per` vectors; 32 / per2 rows per warp step when they are short
-  if (per <= 32) {
-    const int rows = 32 / per;
-    const int rr = lane / per, v = lane % per;
-    const bool on = rr < rows;
-    for (long long s0 = w0 * rows; s0 < cnt; s0 += nw * rows) {
-      const long long slot = s0 + rr;
-      if (!on || slot >= cnt) continue;
-      const long long pt = __ldg(ps.list + slot);
-      if (v < row_vec) Xc[slot * row_vec + v] = __ldg(Xb + pt * row_vec + v);
-      else Xlc[slot * row_vec + v - row_vec] = __ldg(Xl + pt * row_vec + v - row_vec);
-    }
-    return;
-  }
-  for (long long slot = w0; slot < cnt; slot += nw) {
-    const long long pt = __ldg(ps.list + slot);
-    for (int v = lane; v < row_vec; v += 32) {
-      const uint4 hi = __ldg(Xb + pt * row_vec + v);
-      const uint4 lo = Xl ? __ldg(Xl + pt * row_vec + v) : make_uint4(0, 0, 0, 0);
-      Xc[slot * row_vec + v] = hi;
-      if (Xl) Xlc[slot * row_vec + v] = lo;
-    }
-  }
+  copy_listed_rows(ps.list, cnt, Xb, Xl, row_vec, static_cast<uint4*>(ps.Xc), static_cast<uint4*>(ps.Xlc),
+                   ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                   ((long long)gridDim.x * blockDim.x) >> 5, threadIdx.x & 31);
 }
 
 // Marks the old and the new center of every scanned row whose label changed since the last update
@@ -225,7 +198,7 @@ __global__ void prune_gather_kernel(PruneState ps, const uint4* __restrict__ Xb,
 constexpr int kDirtyShared = 32768;
 
 __global__ void __launch_bounds__(1024)
-prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* stop) {
+prune_dirty_kernel(PruneState ps, const int* labels, const int* stop) {
   if (grid_enter()) return;
   const int halt = stop ? pinned(stop) : 0;
   const int cnt = pinned(ps.flags + 1);
@@ -248,7 +221,7 @@ prune_dirty_kernel(PruneState ps, const int* __restrict__ labels, const int* sto
 #pragma unroll 4
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long pt = all ? i : (long long)__ldg(ps.list + i);
+    const long long pt = all ? i : (long long)ld(ps.list + i);
     const int a = ps.lab_old[pt], b = labels[pt];
     if (a == b) continue;
     ps.lab_old[pt] = b;
@@ -311,8 +284,8 @@ prune_top_batched_kernel(PruneBatch pb) {
 // order; a window's last one may be part full, which at 4,096 rows a window costs less than a scan
 // over all windows' counts would.
 __global__ void __launch_bounds__(PF_THREADS)
-prune_window_kernel(PruneBatch pb, const int* __restrict__ labels, const uint4* __restrict__ Xb,
-                    const uint4* __restrict__ Xl, int row_vec) {
+prune_window_kernel(PruneBatch pb, const int* labels, const uint4* Xb,
+                    const uint4* Xl, int row_vec) {
   if (grid_enter()) return;
   constexpr int kPer = kPruneWindow / PF_THREADS;
   __shared__ int rows_sh[kPruneWindow];
@@ -336,10 +309,10 @@ prune_window_kernel(PruneBatch pb, const int* __restrict__ labels, const uint4* 
       const int r = i * PF_THREADS + threadIdx.x;
       if (r >= n) continue;
       const long long pt = (long long)r0 + r;
-      const int a = __ldg(labels + pt);
+      const int a = ld(labels + pt);
       const bool lab_ok = a >= c0 && a < c1;
-      const float sh = lab_ok ? __ldg(ps.shift + a) : -1.0f;
-      const float near = lab_ok ? __ldg(ps.clb + a) : 0.0f;
+      const float sh = lab_ok ? ld(ps.shift + a) : -1.0f;
+      const float near = lab_ok ? ld(ps.clb + a) : 0.0f;
       const float u = sh < 0.0f ? INFINITY : __fadd_ru(ps.ub[pt], sh);
       float l = __fsub_rd(ps.lb[pt], a == topi ? top2 : top1);
       const float l2 = __fsub_rd(near, u);
@@ -407,19 +380,31 @@ prune_window_kernel(PruneBatch pb, const int* __restrict__ labels, const uint4* 
   const int per = row_vec * (Xl ? 2 : 1);
   uint4* Xc = static_cast<uint4*>(ps.Xc);
   uint4* Xlc = static_cast<uint4*>(ps.Xlc);
-#pragma unroll 4
-  for (int e = threadIdx.x; e < total * per; e += PF_THREADS) {
-    const int i = e / per, v = e - i * per;
-    const size_t src = (size_t)rows_sh[i] * row_vec, dst = (size_t)(crow + i) * row_vec;
-    if (v < row_vec) Xc[dst + v] = __ldg(Xb + src + v);
-    else Xlc[dst + v - row_vec] = __ldg(Xl + src + v - row_vec);
+  constexpr int U = 4;  // loads ahead of their stores
+  const int end = total * per;
+  for (int e0 = threadIdx.x; e0 < end; e0 += U * PF_THREADS) {
+    uint4 x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = min(e0 + u * PF_THREADS, end - 1), i = e / per, v = e - i * per;
+      const size_t src = (size_t)rows_sh[i] * row_vec;
+      x[u] = ld(v < row_vec ? Xb + src + v : Xl + src + (v - row_vec));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * PF_THREADS;
+      if (e >= end) break;
+      const int i = e / per, v = e - i * per;
+      const size_t dst = (size_t)(crow + i) * row_vec;
+      *(v < row_vec ? Xc + dst + v : Xlc + dst + (v - row_vec)) = x[u];
+    }
   }
 }
 
 // The centers that lost or won a row since the last update; one block per window. The scans of this
 // iteration are done: block 0 starts the next one's unit table.
 __global__ void __launch_bounds__(PF_THREADS)
-prune_dirty_batched_kernel(PruneBatch pb, const int* __restrict__ labels) {
+prune_dirty_batched_kernel(PruneBatch pb, const int* labels) {
   if (grid_enter()) return;
   const PruneState& ps = pb.ps;
   const int win = blockIdx.x;
@@ -485,7 +470,7 @@ cudaError_t launch_prune_gather(const PruneState& ps, const void* Xb, const void
                                 long long row_bytes, const int* stop, cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (row_bytes % 16 || (Xl && !ps.Xlc)) return cudaErrorInvalidValue;
-  launch(prune_gather_kernel, kmgb::num_sms() * 8, 256, 0, s)(
+  launch(prune_gather_kernel, kmgb::num_sms() * 4, 256, 0, s)(
       ps, static_cast<const uint4*>(Xb), static_cast<const uint4*>(Xl), (int)(row_bytes / 16), stop);
   count_launches(1);
   return cudaGetLastError();

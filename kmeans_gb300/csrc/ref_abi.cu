@@ -26,7 +26,7 @@ void tmp_free(void* p) {
   if (p) cudaFreeAsync(p, kDefault);
 }
 
-__global__ void copy_pad_kernel(const float* __restrict__ A, long long m, int d, float* __restrict__ Ap,
+__global__ void copy_pad_kernel(const float* A, long long m, int d, float* __restrict__ Ap,
                                 long long ld) {
   if (grid_enter()) return;
   const long long total = m * ld;
@@ -40,10 +40,10 @@ __global__ void copy_pad_kernel(const float* __restrict__ A, long long m, int d,
 
 // FP64 arg-min of nb_j - 2 A_i.B_j (B is d x k, K fastest); one warp per row, lanes over j. list
 // (nullable): only the rows list[0 .. *count), or every row where *redo is set.
-__global__ void closest_fp64_kernel(int m0, int m, int d, const double* __restrict__ A, int k,
-                                    const double* __restrict__ B, const double* __restrict__ nb,
-                                    int* __restrict__ out, const int* __restrict__ list,
-                                    const int* __restrict__ count, const int* redo) {
+__global__ void closest_fp64_kernel(int m0, int m, int d, const double* A, int k,
+                                    const double* B, const double* nb,
+                                    int* __restrict__ out, const int* list,
+                                    const int* count, const int* redo) {
   if (grid_enter()) return;
   if (list && pinned(redo) != 0) list = nullptr;
   extern __shared__ double xs_all[];
@@ -80,8 +80,8 @@ __global__ void closest_fp64_kernel(int m0, int m, int d, const double* __restri
 
 // rowTransformMinimum with the reference's expression (RowTransformMinimum.cu:27-50).
 template <typename T>
-__global__ void row_transform_min_kernel(int m0, int m, int n, const T* __restrict__ na,
-                                         const T* __restrict__ nbv, const T* __restrict__ in,
+__global__ void row_transform_min_kernel(int m0, int m, int n, const T* na,
+                                         const T* nbv, const T* in,
                                          int* __restrict__ out) {
   if (grid_enter()) return;
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -143,8 +143,8 @@ constexpr int kSegSteps = 32;
 
 template <int L>
 __global__ void __launch_bounds__(256)
-compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const int* __restrict__ idx,
-                      const float* __restrict__ centers, bool vec, double* __restrict__ partial) {
+compactness_ff_kernel(long long m, int n, const float* data, const int* idx,
+                      const float* centers, bool vec, double* __restrict__ partial) {
   if (grid_enter()) return;
   constexpr int G = 32 / L;
   const int lane = threadIdx.x & 31, grp = lane / L, sub = lane % L;
@@ -172,7 +172,7 @@ compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const 
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const long long r = s0 + (i + u) * G + grp;
-        o[u] = i < kSegSteps && r < m ? __ldg(idx + r) : -1;
+        o[u] = i < kSegSteps && r < m ? ld(idx + r) : -1;
       }
     };
     load_ids(0, id);
@@ -185,8 +185,8 @@ compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const 
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             const long long r = s0 + (i + u) * G + grp;
-            xv[u] = __ldg(reinterpret_cast<const float4*>(data + (size_t)(id[u] >= 0 ? r : 0) * n + t));
-            cv[u] = __ldg(reinterpret_cast<const float4*>(centers + (size_t)max(id[u], 0) * n + t));
+            xv[u] = ld(reinterpret_cast<const float4*>(data + (size_t)(id[u] >= 0 ? r : 0) * n + t));
+            cv[u] = ld(reinterpret_cast<const float4*>(centers + (size_t)max(id[u], 0) * n + t));
           }
 #pragma unroll
           for (int u = 0; u < U; ++u) {
@@ -203,7 +203,7 @@ compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const 
           if (id[u] < 0) continue;
           const float* x = data + (size_t)(s0 + (i + u) * G + grp) * n;
           const float* c = centers + (size_t)id[u] * n;
-          for (int t = sub; t < n; t += L) term(__ldg(x + t), __ldg(c + t));
+          for (int t = sub; t < n; t += L) term(ld(x + t), ld(c + t));
         }
       }
 #pragma unroll
@@ -217,7 +217,7 @@ compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const 
       const long long r = s0 + i * G + grp;
       if (r >= m) continue;
       const float* x = data + (size_t)r * n;
-      const float* c = centers + (size_t)__ldg(idx + r) * n;
+      const float* c = centers + (size_t)ld(idx + r) * n;
       for (int t0 = vec ? 4 * sub : sub; t0 < n; t0 += vec ? 4 * L : L)
         for (int t = t0; t < t0 + (vec ? 4 : 1); ++t) {
           const double u = (double)x[t] - (double)c[t];
@@ -231,8 +231,8 @@ compactness_ff_kernel(long long m, int n, const float* __restrict__ data, const 
 
 // FP64 data: two FP64 operations per element (the lanes' sums meet once, at the end).
 __global__ void __launch_bounds__(256)
-compactness_d_kernel(long long m, int n, const double* __restrict__ data, const int* __restrict__ idx,
-                     const double* __restrict__ centers, double* __restrict__ partial) {
+compactness_d_kernel(long long m, int n, const double* data, const int* idx,
+                     const double* centers, double* __restrict__ partial) {
   if (grid_enter()) return;
   const int lane = threadIdx.x & 31;
   const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -246,12 +246,12 @@ compactness_d_kernel(long long m, int n, const double* __restrict__ data, const 
     for (int u = 0; u < U; ++u) {
       const long long r = r0 + u < m ? r0 + u : m - 1;
       x[u] = data + (size_t)r * n;
-      c[u] = centers + (size_t)__ldg(idx + r) * n;
+      c[u] = centers + (size_t)ld(idx + r) * n;
     }
     for (int t = lane; t < n; t += 32) {
       double v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = __ldg(x[u] + t) - __ldg(c[u] + t);
+      for (int u = 0; u < U; ++u) v[u] = ld(x[u] + t) - ld(c[u] + t);
 #pragma unroll
       for (int u = 0; u < U; ++u)
         if (r0 + u < m) acc = fma(v[u], v[u], acc);
@@ -264,7 +264,7 @@ compactness_d_kernel(long long m, int n, const double* __restrict__ data, const 
 // One block: the partial sums, a strided chain per thread and a tree.
 template <typename T>
 __global__ void __launch_bounds__(256)
-compactness_final_kernel(const double* __restrict__ partial, int nb, double* acc, T* out, bool last) {
+compactness_final_kernel(const double* partial, int nb, double* acc, T* out, bool last) {
   if (grid_enter()) return;
   double t = 0.0;
   for (int i = threadIdx.x; i < nb; i += 256) t += partial[i];
@@ -276,7 +276,7 @@ compactness_final_kernel(const double* __restrict__ partial, int nb, double* acc
 }
 
 template <typename T>
-__global__ void row_norm_kernel(int m0, int m, int n, const T* __restrict__ in, T* __restrict__ out) {
+__global__ void row_norm_kernel(int m0, int m, int n, const T* in, T* __restrict__ out) {
   if (grid_enter()) return;
   const int warps = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (long long i = (long long)blockIdx.x * warps + w; i < m; i += (long long)gridDim.x * warps) {
@@ -291,7 +291,7 @@ __global__ void row_norm_kernel(int m0, int m, int n, const T* __restrict__ in, 
 // sums are added in order. (One thread per column walked the rows alone: 128 x 256 took 23 us.)
 template <typename T>
 __global__ void __launch_bounds__(1024)
-col_norm_kernel(int m, int n, const T* __restrict__ in, T* __restrict__ out) {
+col_norm_kernel(int m, int n, const T* in, T* __restrict__ out) {
   if (grid_enter()) return;
   __shared__ double red[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -300,7 +300,7 @@ col_norm_kernel(int m, int n, const T* __restrict__ in, T* __restrict__ out) {
   if (j < n) {
 #pragma unroll 4
     for (long long i = ty; i < m; i += 32) {
-      const double v = (double)__ldg(in + (size_t)i * n + j);
+      const double v = (double)ld(in + (size_t)i * n + j);
       s = fma(v, v, s);
     }
   }
@@ -318,8 +318,8 @@ col_norm_kernel(int m, int n, const T* __restrict__ in, T* __restrict__ out) {
 // 256 threads (4 x 4 per thread), k in steps of 16 through shared memory; each output is one FMA
 // chain over k in ascending order. Row tiles beyond the grid's y extent are taken in turn.
 template <typename T>
-__global__ void matmul_kernel(int ra, int ca, int cb, const T* __restrict__ A,
-                              const T* __restrict__ B, T* __restrict__ C) {
+__global__ void matmul_kernel(int ra, int ca, int cb, const T* A,
+                              const T* B, T* __restrict__ C) {
   if (grid_enter()) return;
   constexpr int TM = 64, TN = 64, TK = 16;
   __shared__ T As[TK][TM + 1];

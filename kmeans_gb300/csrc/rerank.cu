@@ -33,12 +33,12 @@ __device__ __forceinline__ float approx_value(int mode, const float* __restrict_
   float a = 0.0f;
   if (mode == 0) {
     for (int t = 0; t < d; ++t) {
-      const float u = xs[t] - __ldg(c + t);
+      const float u = xs[t] - ld(c + t);
       a = fmaf(u, u, a);
     }
     return a;
   }
-  for (int t = 0; t < d; ++t) a = fmaf(xs[t], __ldg(c + t), a);
+  for (int t = 0; t < d; ++t) a = fmaf(xs[t], ld(c + t), a);
   return fmaf(-2.0f, a, nbj);
 }
 
@@ -47,12 +47,12 @@ __device__ __forceinline__ double exact_value(int mode, const float* __restrict_
   double s = 0.0;
   if (mode == 0) {
     for (int t = 0; t < d; ++t) {
-      const double u = (double)xs[t] - (double)__ldg(c + t);
+      const double u = (double)xs[t] - (double)ld(c + t);
       s = fma(u, u, s);
     }
     return s;
   }
-  for (int t = 0; t < d; ++t) s = fma((double)xs[t], (double)__ldg(c + t), s);
+  for (int t = 0; t < d; ++t) s = fma((double)xs[t], (double)ld(c + t), s);
   return fma(-2.0, s, (double)nbj);
 }
 
@@ -487,7 +487,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
 // K=256, FP32 tier, 1.05 ms per iteration before. Slots from cand_cap on go to over / over_hi.
 template <int MODE, bool RECORD>
 __global__ void __launch_bounds__(256)
-rerank_exact_kernel(RerankArgs a, const float* __restrict__ hi2, int* __restrict__ cand,
+rerank_exact_kernel(RerankArgs a, const float* hi2, int* __restrict__ cand,
                     int* __restrict__ cand_cnt, long long cand_cap, int* __restrict__ over,
                     int* __restrict__ over_count, float* __restrict__ over_hi) {
   if (grid_enter()) return;
@@ -587,7 +587,7 @@ rerank_grouped_kernel(RerankArgs a, GroupArgs g, int* __restrict__ cand, int* __
       for (int t = 4 * sub; t < ds; t += 4 * L) {
         const float4 xt = *reinterpret_cast<const float4*>(xs + t);
 #pragma unroll
-        for (int r = 0; r < U; ++r) tile_acc<0>(xt, __ldg(reinterpret_cast<const float4*>(cr[r] + t)), sv[r]);
+        for (int r = 0; r < U; ++r) tile_acc<0>(xt, ld(reinterpret_cast<const float4*>(cr[r] + t)), sv[r]);
       }
 #pragma unroll
       for (int o = L / 2; o > 0; o >>= 1) {
@@ -662,41 +662,35 @@ rerank_grouped_kernel(RerankArgs a, GroupArgs g, int* __restrict__ cand, int* __
 
 namespace {
 // Copies the BF16 rows (and residual rows) of the flagged points into a compact buffer, row
-// `slot` for list[slot], with the point's candidate floor. One warp per row, 16-byte moves. The
-// compact buffer holds `cap` rows; flagged points beyond it go straight to `over` (the full
-// rescan), so any number of flagged points is settled exactly.
-__global__ void gather_flagged_kernel(const int* __restrict__ list, const int* __restrict__ count,
-                                      long long cap, const uint4* __restrict__ Xb,
-                                      const uint4* __restrict__ Xl, long long row_vec,
-                                      const float* __restrict__ thr, uint4* __restrict__ XbC,
+// `slot` for list[slot], with the point's candidate floor. The compact buffer holds `cap` rows;
+// flagged points beyond it go straight to `over` (the full rescan), so any number of flagged points
+// is settled exactly.
+__global__ void __launch_bounds__(256, 4)
+gather_flagged_kernel(const int* list, const int* count,
+                                      long long cap, const uint4* Xb,
+                                      const uint4* Xl, long long row_vec,
+                                      const float* thr, uint4* __restrict__ XbC,
                                       uint4* __restrict__ XlC, float* __restrict__ thrC,
                                       int* __restrict__ over, int* __restrict__ over_count,
-                                      const int* stop, const float* __restrict__ xs,
+                                      const int* stop, const float* xs,
                                       float* __restrict__ xsC) {
   if (grid_enter()) return;
   const int halt = stop ? pinned(stop) : 0;
   const long long total = pinned(count);
   if (halt) return;
   const long long cnt = min(total, cap);
-  const int lane = threadIdx.x & 31;
-  const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long slot = cap + w0 * 32 + lane; slot < total; slot += nw * 32)
-    over[atomicAdd(over_count, 1)] = list[slot];
-  for (long long slot = w0; slot < cnt; slot += nw) {
+  const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long nt = (long long)gridDim.x * blockDim.x;
+  for (long long slot = cap + t0; slot < total; slot += nt) over[atomicAdd(over_count, 1)] = list[slot];
+  for (long long slot = nt - 1 - t0; slot < cnt; slot += nt) {  // (the grid's end, while its first warps copy)
     const long long pt = list[slot];
-    for (long long v = lane; v < row_vec; v += 32) {
-      XbC[slot * row_vec + v] = Xb[pt * row_vec + v];
-      if (Xl) XlC[slot * row_vec + v] = Xl[pt * row_vec + v];
-    }
-    if (lane == 0) {
-      // without a finite floor (no usable center, an infinite bound) the keys say nothing: no
-      // candidates, hence the full rescan
-      const float fl = thr[pt];
-      thrC[slot] = fl > -3.0e38f ? fl : INFINITY;
-      if (xs) xsC[slot] = xs[pt];
-    }
+    // without a finite floor (no usable center, an infinite bound) the keys say nothing: no
+    // candidates, hence the full rescan
+    const float fl = thr[pt];
+    thrC[slot] = fl > -3.0e38f ? fl : INFINITY;
+    if (xs) xsC[slot] = xs[pt];
   }
+  copy_listed_rows(list, cnt, Xb, Xl, (int)row_vec, XbC, XlC, t0 >> 5, nt >> 5, threadIdx.x & 31);
 }
 
 // Error-free float-float helpers (FP32 pipe). two_sum: s + e == a + b exactly.
@@ -736,15 +730,15 @@ __device__ __forceinline__ void ff_dist8(const float* __restrict__ x, const floa
   lo = 0.0f;
   if (VEC) {
     for (int t = 4 * r; t < d; t += 4 * kGroupLanes) {
-      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + t));
-      const float4 cv = __ldg(reinterpret_cast<const float4*>(c + t));
+      const float4 xv = ld(reinterpret_cast<const float4*>(x + t));
+      const float4 cv = ld(reinterpret_cast<const float4*>(c + t));
       ff_term(xv.x, cv.x, hi, lo);
       ff_term(xv.y, cv.y, hi, lo);
       ff_term(xv.z, cv.z, hi, lo);
       ff_term(xv.w, cv.w, hi, lo);
     }
   } else {
-    for (int t = r; t < d; t += kGroupLanes) ff_term(__ldg(x + t), __ldg(c + t), hi, lo);
+    for (int t = r; t < d; t += kGroupLanes) ff_term(ld(x + t), ld(c + t), hi, lo);
   }
   for (int o = kGroupLanes / 2; o > 0; o >>= 1) {
     const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
@@ -768,8 +762,8 @@ __device__ __forceinline__ float f32_dist8(const float* __restrict__ x, const fl
   if (VEC) {
     float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
     for (int t = 4 * r; t < d; t += 4 * kGroupLanes) {
-      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + t));
-      const float4 cv = __ldg(reinterpret_cast<const float4*>(c + t));
+      const float4 xv = ld(reinterpret_cast<const float4*>(x + t));
+      const float4 cv = ld(reinterpret_cast<const float4*>(c + t));
       const float u0 = __fsub_rn(xv.x, cv.x), u1 = __fsub_rn(xv.y, cv.y);
       const float u2 = __fsub_rn(xv.z, cv.z), u3 = __fsub_rn(xv.w, cv.w);
       a0 = __fmaf_rn(u0, u0, a0);
@@ -781,7 +775,7 @@ __device__ __forceinline__ float f32_dist8(const float* __restrict__ x, const fl
   } else {
     s = 0.0f;
     for (int t = r; t < d; t += kGroupLanes) {
-      const float u = __fsub_rn(__ldg(x + t), __ldg(c + t));
+      const float u = __fsub_rn(ld(x + t), ld(c + t));
       s = __fmaf_rn(u, u, s);
     }
   }
@@ -833,16 +827,16 @@ ResolveTol resolve_tolerances(int d) {
 }
 
 template <bool VEC>
-__global__ void resolve_candidates_kernel(const int* __restrict__ list, const int* __restrict__ count,
-                                          long long max_list, const int* __restrict__ cand,
-                                          const int* __restrict__ cand_cnt,
-                                          const float* __restrict__ X, long long ldx,
-                                          const float* __restrict__ C, long long ldc,
-                                          const float* __restrict__ cn, int d,
+__global__ void resolve_candidates_kernel(const int* list, const int* count,
+                                          long long max_list, const int* cand,
+                                          const int* cand_cnt,
+                                          const float* X, long long ldx,
+                                          const float* C, long long ldc,
+                                          const float* cn, int d,
                                           int* __restrict__ labels, int* __restrict__ over,
                                           int* __restrict__ over_count, const int* stop,
-                                          const int* __restrict__ row_map,
-                                          const float* __restrict__ hi_in,
+                                          const int* row_map,
+                                          const float* hi_in,
                                           float* __restrict__ over_hi, ResolveTol tol) {
   if (grid_enter()) return;
   const int halt = stop ? pinned(stop) : 0;
@@ -946,7 +940,7 @@ __global__ void resolve_candidates_kernel(const int* __restrict__ list, const in
         const float* c = C + (size_t)j * ldc;
         double s = 0.0;
         for (int t = 0; t < d; ++t) {
-          const double u = (double)__ldg(x + t) - (double)__ldg(c + t);
+          const double u = (double)ld(x + t) - (double)ld(c + t);
           s = fma(u, u, s);
         }
         if (s < INFINITY && (s < best || (s == best && (unsigned)j < (unsigned)bidx))) {
@@ -986,15 +980,15 @@ __device__ __forceinline__ void ff_dot8(const float* __restrict__ x, const float
   lo = 0.0f;
   if (VEC) {
     for (int t = 4 * r; t < d; t += 4 * kGroupLanes) {
-      const float4 xv = __ldg(reinterpret_cast<const float4*>(x + t));
-      const float4 cv = __ldg(reinterpret_cast<const float4*>(c + t));
+      const float4 xv = ld(reinterpret_cast<const float4*>(x + t));
+      const float4 cv = ld(reinterpret_cast<const float4*>(c + t));
       ff_product(xv.x, cv.x, hi, lo);
       ff_product(xv.y, cv.y, hi, lo);
       ff_product(xv.z, cv.z, hi, lo);
       ff_product(xv.w, cv.w, hi, lo);
     }
   } else {
-    for (int t = r; t < d; t += kGroupLanes) ff_product(__ldg(x + t), __ldg(c + t), hi, lo);
+    for (int t = r; t < d; t += kGroupLanes) ff_product(ld(x + t), ld(c + t), hi, lo);
   }
   for (int o = kGroupLanes / 2; o > 0; o >>= 1) {
     const float oh = __shfl_xor_sync(0xffffffffu, hi, o);
@@ -1013,8 +1007,8 @@ __device__ __forceinline__ void ff_dot8(const float* __restrict__ x, const float
 // more than both, twice, is the arg-min. Other points (ties, non-finite values) take the sequential
 // FP64 evaluation, one lane per candidate, lowest index on ties.
 template <bool VEC>
-__global__ void resolve_expansion_kernel(RerankArgs a, const int* __restrict__ cand,
-                                         const int* __restrict__ cand_cnt, int* __restrict__ over,
+__global__ void resolve_expansion_kernel(RerankArgs a, const int* cand,
+                                         const int* cand_cnt, int* __restrict__ over,
                                          int* __restrict__ over_count) {
   if (grid_enter()) return;
   const long long cnt = min((long long)pinned(a.count), a.max_list);
@@ -1121,12 +1115,12 @@ __global__ void resolve_fp64_kernel(ResolveD a) {
         if (a.mode == 0) {
 #pragma unroll 8
           for (int t = 0; t < a.d; ++t) {
-            const double u = __ldg(x + t) - __ldg(c + (size_t)t * a.c_dim);
+            const double u = ld(x + t) - ld(c + (size_t)t * a.c_dim);
             v = fma(u, u, v);
           }
         } else {
 #pragma unroll 8
-          for (int t = 0; t < a.d; ++t) v = fma(__ldg(x + t), __ldg(c + (size_t)t * a.c_dim), v);
+          for (int t = 0; t < a.d; ++t) v = fma(ld(x + t), ld(c + (size_t)t * a.c_dim), v);
           v = fma(-2.0, v, a.nb[j]);
         }
         // (a lane's candidates do not come in index order)
@@ -1178,7 +1172,7 @@ __device__ __forceinline__ float audit_dist32(const float* ax, const float* __re
                                               int lane) {
   float a = 0.0f;
   for (int t = lane; t < d; t += 32) {
-    const float u = ax[t] - __ldg(c + t);
+    const float u = ax[t] - ld(c + t);
     a = fmaf(u, u, a);
   }
   for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -1200,7 +1194,7 @@ __device__ __forceinline__ void audit_dist32x4(const float* ax, const float* __r
     const float xt = ax[t];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const float v = xt - __ldg(c[u] + t);
+      const float v = xt - ld(c[u] + t);
       out[u] = fmaf(v, v, out[u]);
     }
   }
@@ -1247,9 +1241,9 @@ __device__ void audit_close(unsigned long long* ws, int rows) {
 }
 
 __global__ void __launch_bounds__(256)
-audit_scan_kernel(const float* __restrict__ X, long long ldx, long long n, int d,
-                  const float* __restrict__ C, long long ldc, int k,
-                  const int* __restrict__ labels, unsigned long long* ws, int rows, int parts,
+audit_scan_kernel(const float* X, long long ldx, long long n, int d,
+                  const float* C, long long ldc, int k,
+                  const int* labels, unsigned long long* ws, int rows, int parts,
                   GroupArgs g, const int* stop) {
   if (grid_enter()) return;
   if (stopped(stop)) return;
@@ -1331,7 +1325,7 @@ cudaError_t launch_gather_flagged(const int* list, const int* count, long long c
                                   const float* xs, float* xsC) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (row_bytes % 16) return cudaErrorInvalidValue;
-  launch(gather_flagged_kernel, kmgb::num_sms() * 8, 256, 0, s)(
+  launch(gather_flagged_kernel, kmgb::num_sms() * 4, 256, 0, s)(
       list, count, cap, reinterpret_cast<const uint4*>(Xb), reinterpret_cast<const uint4*>(Xl),
       row_bytes / 16, thr, reinterpret_cast<uint4*>(XbC), reinterpret_cast<uint4*>(XlC), thrC, over,
       over_count, stop, xs, xsC);

@@ -111,7 +111,7 @@ __device__ void block_scan_inplace(int* data, long long n) {
 }
 
 // Sums of the segments; the last block turns them into their exclusive scan.
-__global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int* __restrict__ sums,
+__global__ void scan_reduce_kernel(const int* in, long long n, int* __restrict__ sums,
                                    int* ticket, const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   if (skip(stop, any_dirty)) return;
@@ -133,7 +133,7 @@ __global__ void scan_reduce_kernel(const int* __restrict__ in, long long n, int*
 }
 
 // In-place exclusive scan of segment blockIdx.x, plus offset (*offsets)[blockIdx.x] if given.
-__global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* __restrict__ offsets,
+__global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* offsets,
                                 const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   if (skip(stop, any_dirty)) return;
@@ -179,7 +179,7 @@ __device__ __forceinline__ int scan_label_row(int* row, int ntiles, int lane) {
 // passes and two launches before the offsets' own (256 labels x 220 tiles: 18.8 -> 7.6 us in all).
 __global__ void __launch_bounds__(SCAN_T)
 label_rows_kernel(int* __restrict__ hist, long long n, int k, int ntiles, int* label_off, int* piece_cnt,
-                  long long* __restrict__ counts, const int* __restrict__ dirty, int* ticket,
+                  long long* __restrict__ counts, const int* dirty, int* ticket,
                   const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   if (skip(stop, any_dirty)) return;
@@ -238,7 +238,7 @@ label_rows_kernel(int* __restrict__ hist, long long n, int k, int ntiles, int* l
 constexpr int kSmallHist = 8 * SCAN_T;
 
 template <bool SMEM, bool SMALL>
-__global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, int tile_pts,
+__global__ void hist_kernel(const int* labels, long long n, int k, int tile_pts,
                             int ntiles, int* __restrict__ hist, int* err, int* label_off,
                             int* piece_cnt, long long* counts, const int* dirty, int* ticket,
                             const int* any_dirty, const int* stop) {
@@ -260,7 +260,7 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = b + (long long)u * blockDim.x + threadIdx.x;
-      lv[u] = i < i1 ? __ldg(labels + i) : -1;
+      lv[u] = i < i1 ? ld(labels + i) : -1;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -288,7 +288,7 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
     // member counts and first pieces (through global memory: three more round trips)
     __shared__ int pos_s[SMALL ? kSmallHist : 1];
     const int total = k * ntiles, t = threadIdx.x;
-    int live = t < k && dirty ? __ldg(dirty + t) : 1;
+    int live = t < k && dirty ? ld(dirty + t) : 1;
     int v[8], s = 0;
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = 8 * t + u < total ? __ldcg(hist + 8 * t + u) : 0;
@@ -308,7 +308,7 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
     int carry = 0;
     for (int j0 = 0; j0 < k; j0 += SCAN_T) {
       const int j = j0 + t;
-      if (j0 > 0) live = j < k && dirty ? __ldg(dirty + j) : 1;
+      if (j0 > 0) live = j < k && dirty ? ld(dirty + j) : 1;
       int c = 0, a0 = 0;
       if (j < k) {
         a0 = pos_s[j * ntiles];
@@ -337,9 +337,9 @@ __global__ void hist_kernel(const int* __restrict__ labels, long long n, int k, 
 constexpr int kScatterLoad = 512;
 
 template <bool SMEM>
-__global__ void scatter_kernel(const int* __restrict__ labels, long long n, int k, int tile_pts,
-                               int ntiles, int* pos, const int* __restrict__ start,
-                               int* __restrict__ sorted, const int* __restrict__ dirty,
+__global__ void scatter_kernel(const int* labels, long long n, int k, int tile_pts,
+                               int ntiles, int* pos, const int* start,
+                               int* __restrict__ sorted, const int* dirty,
                                const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   if (skip(stop, any_dirty)) return;
@@ -349,7 +349,7 @@ __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int 
   if (tile >= ntiles) return;
   if (SMEM) {
     for (int j = threadIdx.x; j < k; j += blockDim.x)
-      cnt_s[j] = pos[(size_t)j * ntiles + tile] + (start ? __ldg(start + j) : 0);
+      cnt_s[j] = pos[(size_t)j * ntiles + tile] + (start ? ld(start + j) : 0);
     __syncthreads();
     if (threadIdx.x >= 32) return;
   }
@@ -363,13 +363,13 @@ __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = b + 32 * u + lane;
-      lv[u] = i < i1 ? __ldg(labels + i) : -1;
+      lv[u] = i < i1 ? ld(labels + i) : -1;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = b + 32 * u + lane;
       int l = lv[u];
-      if (l < 0 || l >= k || (dirty && !__ldg(dirty + l))) l = -1;
+      if (l < 0 || l >= k || (dirty && !ld(dirty + l))) l = -1;
       const unsigned peers = warp_peers(l, nbits);
       const int leader = __ffs(peers) - 1;
       const int rank = __popc(peers & lanemask_lt());
@@ -377,7 +377,7 @@ __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int 
       if (l >= 0 && lane == leader)
         base = SMEM ? cnt_s[l] : vpos[(size_t)l * ntiles + tile];
       base = __shfl_sync(0xffffffffu, base, leader);
-      if (l >= 0) sorted[base + rank + (!SMEM && start ? __ldg(start + l) : 0)] = (int)i;
+      if (l >= 0) sorted[base + rank + (!SMEM && start ? ld(start + l) : 0)] = (int)i;
       if (l >= 0 && lane == leader) {
         const int nv = base + __popc(peers);
         if (SMEM) cnt_s[l] = nv;
@@ -394,10 +394,10 @@ __global__ void scatter_kernel(const int* __restrict__ labels, long long n, int 
 // place their rows in parallel. Same positions as one warp walking the tile in order.
 constexpr int kScatterWarps = 8;
 
-__global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n, int k,
-                                     int tile_pts, int ntiles, const int* __restrict__ pos,
-                                     const int* __restrict__ start, int* __restrict__ sorted,
-                                     const int* __restrict__ dirty,
+__global__ void scatter_multi_kernel(const int* labels, long long n, int k,
+                                     int tile_pts, int ntiles, const int* pos,
+                                     const int* start, int* __restrict__ sorted,
+                                     const int* dirty,
                                      const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   if (skip(stop, any_dirty)) return;
@@ -416,14 +416,14 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
   for (long long b = s0; b < s1; b += 32 * U) {
     int lv[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) lv[u] = b + 32 * u + lane < s1 ? __ldg(labels + b + 32 * u + lane) : -1;
+    for (int u = 0; u < U; ++u) lv[u] = b + 32 * u + lane < s1 ? ld(labels + b + 32 * u + lane) : -1;
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (lv[u] >= 0 && lv[u] < k) atomicAdd(&mine[lv[u]], 1);
   }
   __syncthreads();
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
-    int run = pos[(size_t)j * ntiles + tile] + (start ? __ldg(start + j) : 0);
+    int run = pos[(size_t)j * ntiles + tile] + (start ? ld(start + j) : 0);
     for (int v = 0; v < kScatterWarps; ++v) {
       const int c = wcnt[(size_t)v * k + j];
       wcnt[(size_t)v * k + j] = run;
@@ -435,11 +435,11 @@ __global__ void scatter_multi_kernel(const int* __restrict__ labels, long long n
   for (long long b0 = s0; b0 < s1; b0 += 32 * U) {
     int lv[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) lv[u] = b0 + 32 * u + lane < s1 ? __ldg(labels + b0 + 32 * u + lane) : -1;
+    for (int u = 0; u < U; ++u) lv[u] = b0 + 32 * u + lane < s1 ? ld(labels + b0 + 32 * u + lane) : -1;
     if (dirty) {
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (lv[u] >= 0 && lv[u] < k && !__ldg(dirty + lv[u])) lv[u] = -1;
+        if (lv[u] >= 0 && lv[u] < k && !ld(dirty + lv[u])) lv[u] = -1;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -485,7 +485,7 @@ __device__ __forceinline__ int find_label_group(const int* __restrict__ pstart, 
   while (__any_sync(0xffffffffu, n > 1)) {
     const int step = (n + L - 1) / L;
     const int at = lo + sub * step;
-    const bool in = n > 1 && sub * step < n && __ldg(pstart + at) <= p;
+    const bool in = n > 1 && sub * step < n && ld(pstart + at) <= p;
     const unsigned bal = (__ballot_sync(0xffffffffu, in) >> shift) & (L == 32 ? 0xffffffffu : (1u << L) - 1u);
     if (n > 1) {
       const int hit = 31 - __clz(bal | 1u);  // place 0 always holds
@@ -500,16 +500,16 @@ __device__ __forceinline__ int find_label(const int* __restrict__ pstart, int k,
   int lo = 0, hi = k - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(pstart + mid) <= p) lo = mid;
+    if (ld(pstart + mid) <= p) lo = mid;
     else hi = mid - 1;
   }
   return lo;
 }
 
 // One warp per piece; dims lane + 32 r in chunks of 256.
-__global__ void piece_sums_kernel(const float* __restrict__ X, long long ldx,
-                                  const double* __restrict__ qn, const int* __restrict__ sorted,
-                                  const int* __restrict__ label_off, const int* __restrict__ pstart,
+__global__ void piece_sums_kernel(const float* X, long long ldx,
+                                  const double* qn, const int* sorted,
+                                  const int* label_off, const int* pstart,
                                   int k, int d, double* __restrict__ part,
                                   double* __restrict__ partq, const int* any_dirty,
                                   const int* stop) {
@@ -529,14 +529,14 @@ __global__ void piece_sums_kernel(const float* __restrict__ X, long long ldx,
       double qs = 0.0;
 #pragma unroll 4
       for (int t = b; t < e; ++t) {
-        const int i = __ldg(sorted + t);
+        const int i = ld(sorted + t);
         const float* x = X + (size_t)i * ldx + d0;
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
           const int c = lane + 32 * r;
-          if (d0 + c < d) acc[r].add(__ldg(x + c));
+          if (d0 + c < d) acc[r].add(ld(x + c));
         }
-        if (qn && d0 == 0) qs += __ldg(qn + i);
+        if (qn && d0 == 0) qs += ld(qn + i);
       }
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
@@ -592,7 +592,7 @@ struct RingCursor {
 
 __device__ __forceinline__ int ring_window_id(const int* __restrict__ sorted, int t0, int e,
                                               int lane) {
-  return t0 + lane < e ? __ldg(sorted + t0 + lane) : 0;
+  return t0 + lane < e ? ld(sorted + t0 + lane) : 0;
 }
 
 __device__ __forceinline__ void ring_start_piece(RingCursor& q, long long ptot,
@@ -632,7 +632,7 @@ __device__ __forceinline__ void ring_issue(RingCursor& q, long long ptot, long l
     q.wt = q.t;
     q.id = q.id_nx;
     q.id_nx = ring_window_id(sorted, q.t + 32, q.e, lane);
-    if (qn && q.d0 == 0 && q.t + lane < q.e) qv = __ldg(qn + q.id);
+    if (qn && q.d0 == 0 && q.t + lane < q.e) qv = ld(qn + q.id);
   }
   const int nr = min(kRingRows, q.e - q.t);
   const int c = q.d0 + 4 * lane;
@@ -667,9 +667,9 @@ __device__ __forceinline__ void ring_issue(RingCursor& q, long long ptot, long l
 }
 
 __global__ void __launch_bounds__(kRingWarps * 32, 4)
-piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double* __restrict__ qn,
-                       const int* __restrict__ sorted, const int* __restrict__ label_off,
-                       const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
+piece_sums_ring_kernel(const float* X, long long ldx, const double* qn,
+                       const int* sorted, const int* label_off,
+                       const int* pstart, int k, int d, double* __restrict__ part,
                        double* __restrict__ partq, const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   const long long ptot = pinned(pstart + k);
@@ -737,9 +737,9 @@ piece_sums_ring_kernel(const float* __restrict__ X, long long ldx, const double*
 // round trip before every 8 rows, the norms piece after piece).
 template <int L>
 __global__ void __launch_bounds__(128)
-piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double* __restrict__ qn,
-                        const int* __restrict__ sorted, const int* __restrict__ label_off,
-                        const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
+piece_sums_small_kernel(const float* X, long long ldx, const double* qn,
+                        const int* sorted, const int* label_off,
+                        const int* pstart, int k, int d, double* __restrict__ part,
                         double* __restrict__ partq, const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   const int ptot = pinned(pstart + k);
@@ -754,14 +754,14 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
     const long long p = p0 + grp;
     const bool live = p < ptot;
     const int j = find_label_group<L>(pstart, k, live ? (int)p : 0);
-    const int b = live ? __ldg(label_off + j) + ((int)p - __ldg(pstart + j)) * kSumPiece : 0;
-    const int n = live ? min(kSumPiece, __ldg(label_off + j + 1) - b) : 0;
+    const int b = live ? ld(label_off + j) + ((int)p - ld(pstart + j)) * kSumPiece : 0;
+    const int n = live ? min(kSumPiece, ld(label_off + j + 1) - b) : 0;
     const bool on = live && c < d;
     const float* xc = X + (on ? c : 0);
     auto load_ids = [&](int t, int (&id)[G]) {
 #pragma unroll
       for (int i = 0; i < G; ++i)
-        id[i] = t + i * L + sub < n ? __ldg(sorted + b + t + i * L + sub) : -1;
+        id[i] = t + i * L + sub < n ? ld(sorted + b + t + i * L + sub) : -1;
     };
     // rows h .. h + R - 1 of the window whose ids are id (zeros past the piece: adding them changes
     // no float-float sum)
@@ -769,7 +769,7 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int row = __shfl_sync(0xffffffffu, id[(h + r) / L], grp * L + (h + r) % L);
-        v[r] = __ldg(reinterpret_cast<const float4*>(xc + (size_t)max(row, 0) * ldx));  // (no branch)
+        v[r] = ld(reinterpret_cast<const float4*>(xc + (size_t)max(row, 0) * ldx));  // (no branch)
         if (row < 0) v[r] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     };
@@ -795,7 +795,7 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
       load_rows(id, R, vb);
       if (qn) {
 #pragma unroll
-        for (int i = 0; i < G; ++i) q[i] = id[i] >= 0 ? __ldg(qn + id[i]) : 0.0;
+        for (int i = 0; i < G; ++i) q[i] = id[i] >= 0 ? ld(qn + id[i]) : 0.0;
       }
       add_rows(va);
       load_rows(nx, 0, va);
@@ -828,9 +828,9 @@ piece_sums_small_kernel(const float* __restrict__ X, long long ldx, const double
 // of the piece, then every row in flight at once. A piece is a serial chain of 128 additions, but its
 // loads need not be one: with 16 rows ahead a warp waits eight times for L2 (900 cycles each).
 __global__ void __launch_bounds__(128)
-piece_sums_few_kernel(const float* __restrict__ X, long long ldx, const double* __restrict__ qn,
-                      const int* __restrict__ sorted, const int* __restrict__ label_off,
-                      const int* __restrict__ pstart, int k, int d, double* __restrict__ part,
+piece_sums_few_kernel(const float* X, long long ldx, const double* qn,
+                      const int* sorted, const int* label_off,
+                      const int* pstart, int k, int d, double* __restrict__ part,
                       double* __restrict__ partq, const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
   const int ptot = pinned(pstart + k);
@@ -844,23 +844,23 @@ piece_sums_few_kernel(const float* __restrict__ X, long long ldx, const double* 
   for (long long it = gw; it < total; it += nw) {
     const int p = (int)(it / groups), g = (int)(it - (long long)p * groups);
     const int j = find_label_group<32>(pstart, k, p);
-    const int b = __ldg(label_off + j) + (p - __ldg(pstart + j)) * kSumPiece;
-    const int n = min(kSumPiece, __ldg(label_off + j + 1) - b);
+    const int b = ld(label_off + j) + (p - ld(pstart + j)) * kSumPiece;
+    const int n = min(kSumPiece, ld(label_off + j + 1) - b);
     const int c = g * 32 + lane;
     const bool on = c < d;
     const float* xc = X + (on ? c : 0);
     int id[W];
     double q[W];
 #pragma unroll
-    for (int w = 0; w < W; ++w) id[w] = 32 * w + lane < n ? __ldg(sorted + b + 32 * w + lane) : -1;
+    for (int w = 0; w < W; ++w) id[w] = 32 * w + lane < n ? ld(sorted + b + 32 * w + lane) : -1;
     float v[kSumPiece];
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-      q[w] = qn && g == 0 && id[w] >= 0 ? __ldg(qn + id[w]) : 0.0;
+      q[w] = qn && g == 0 && id[w] >= 0 ? ld(qn + id[w]) : 0.0;
 #pragma unroll
       for (int r = 0; r < 32; ++r) {
         const int row = __shfl_sync(0xffffffffu, id[w], r);
-        v[32 * w + r] = __ldg(xc + (size_t)max(row, 0) * ldx);  // (no branch per load)
+        v[32 * w + r] = ld(xc + (size_t)max(row, 0) * ldx);  // (no branch per load)
       }
     }
     PieceAcc a;
@@ -935,8 +935,8 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
 // rows are aligned), 16 rows' loads in flight; the additions per (piece, dimension) are in row order.
 // (A warp per piece with 4 rows in flight took 258 us for 400,000 x 64, K=256.)
 __global__ void __launch_bounds__(128)
-piece_sums_d_kernel(const double* __restrict__ X, long long ldx, const int* __restrict__ sorted,
-                    const int* __restrict__ label_off, const int* __restrict__ pstart, int k, int d,
+piece_sums_d_kernel(const double* X, long long ldx, const int* sorted,
+                    const int* label_off, const int* pstart, int k, int d,
                     bool vec, double* __restrict__ part, const int* stop) {
   if (grid_enter()) return;
   if (stopped(stop)) return;
@@ -955,7 +955,7 @@ piece_sums_d_kernel(const double* __restrict__ X, long long ldx, const int* __re
     const bool on0 = c < d, on1 = c + 1 < d;
     double s0 = 0.0, s1 = 0.0;
     for (int t0 = b; t0 < e; t0 += 32) {
-      const int ids = t0 + lane < e ? __ldg(sorted + t0 + lane) : 0;
+      const int ids = t0 + lane < e ? ld(sorted + t0 + lane) : 0;
 #pragma unroll
       for (int h = 0; h < 32; h += U) {
         double2 v[U];
@@ -966,10 +966,10 @@ piece_sums_d_kernel(const double* __restrict__ X, long long ldx, const int* __re
           if (t0 + h + r < e) {
             const double* x = X + (size_t)i * ldx + c;
             if (vec && on1) {
-              v[r] = __ldg(reinterpret_cast<const double2*>(x));
+              v[r] = ld(reinterpret_cast<const double2*>(x));
             } else {
-              if (on0) v[r].x = __ldg(x);
-              if (on1) v[r].y = __ldg(x + 1);
+              if (on0) v[r].x = ld(x);
+              if (on1) v[r].y = ld(x + 1);
             }
           }
         }
@@ -1048,7 +1048,7 @@ __device__ __forceinline__ double sum_pieces_by(const double* __restrict__ part,
     double v[U];
 #pragma unroll
     for (int i = 0; i < U; ++i)
-      if (p + i < p1) v[i] = __ldg(part + (size_t)(p + i) * d);
+      if (p + i < p1) v[i] = ld(part + (size_t)(p + i) * d);
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       if (p + i >= p1) break;
@@ -1067,11 +1067,11 @@ __device__ __forceinline__ double sum_pieces(const double* __restrict__ part, in
 // g*32 + c, adds the center's piece sums in piece order (the canonical order: centers are
 // unchanged by the split), divides in FP64 and rounds once. The group's SSE term
 // sum_c (n mu^2 - 2 mu s) lands in sse_k[j * G + g]; group 0 adds the members' sum of ||x||^2.
-__global__ void finalize_kernel(const double* __restrict__ part, const double* __restrict__ partq,
-                                const int* __restrict__ label_off, const int* __restrict__ pstart,
+__global__ void finalize_kernel(const double* part, const double* partq,
+                                const int* label_off, const int* pstart,
                                 int k, int d, float* __restrict__ C, long long ldc,
                                 int empty_policy, double* __restrict__ sse_k,
-                                const int* __restrict__ dirty, const int* stop) {
+                                const int* dirty, const int* stop) {
   if (grid_enter()) return;
   if (stopped(stop)) return;
   const int groups = (d + 31) / 32;
@@ -1105,7 +1105,7 @@ __global__ void finalize_kernel(const double* __restrict__ part, const double* _
   if (g == 0 && partq && n > 0 && sse_k) {
     for (int b = p0; b < p1; b += 32) {
       const int cnt = min(32, p1 - b);
-      const double v = lane < cnt ? __ldg(partq + b + lane) : 0.0;
+      const double v = lane < cnt ? ld(partq + b + lane) : 0.0;
       for (int i = 0; i < cnt; ++i) q += __shfl_sync(0xffffffffu, v, i);
     }
   }
@@ -1119,11 +1119,11 @@ __global__ void finalize_kernel(const double* __restrict__ part, const double* _
 // Compactness.cu:3-59, gives); the identity's cancellation error is of the order of 1e-15 Q.
 // One warp per center; the direct sum only runs for flagged clusters.
 __global__ void sse_fixup_kernel(double* __restrict__ sse_k, int groups,
-                                 const double* __restrict__ partq, const int* __restrict__ label_off,
-                                 const int* __restrict__ pstart, int k, int d,
-                                 const float* __restrict__ X, long long ldx,
-                                 const int* __restrict__ sorted, const float* __restrict__ C,
-                                 long long ldc, const int* __restrict__ dirty, const int* stop) {
+                                 const double* partq, const int* label_off,
+                                 const int* pstart, int k, int d,
+                                 const float* X, long long ldx,
+                                 const int* sorted, const float* C,
+                                 long long ldc, const int* dirty, const int* stop) {
   if (grid_enter()) return;
   if (stopped(stop)) return;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1196,7 +1196,7 @@ __device__ __forceinline__ void store_sse(double sse, const LoopIn& l, double* o
 // norms, quotients avoid the division and a block takes several centers before its fence and ticket
 // (16,384 x 256: 268 -> 192 us).
 __global__ void __launch_bounds__(256)
-finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long long ldc,
+finalize_update_kernel(const float* X, float* __restrict__ C, long long ldc,
                        int empty_policy, UpdateWork w, double* __restrict__ sse_out) {
   if (grid_enter()) return;
   const int halt = w.stop ? pinned(w.stop) : 0;
@@ -1214,7 +1214,7 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
     if (!live) continue;
     // the members' sum of ||x||^2: the last warp's lanes over the pieces, the first ones ahead
     double q = 0.0;
-    if (wp == warps - 1 && p0 + lane < p1) q = __ldg(w.partq + p0 + lane);
+    if (wp == warps - 1 && p0 + lane < p1) q = ld(w.partq + p0 + lane);
     const int n = m1 - m0;
     const double nd = (double)n, rn = reciprocal_of_count(n > 0 ? n : 1, nd);
     double half = 0.0;  // of the lane's share of n mu^2 - 2 mu s
@@ -1235,7 +1235,7 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
     }
     red[threadIdx.x] = half;
     if (wp == warps - 1)
-      for (int p = p0 + 32 + lane; p < p1; p += 32) q += __ldg(w.partq + p);
+      for (int p = p0 + 32 + lane; p < p1; p += 32) q += ld(w.partq + p);
     __syncthreads();  // and the center's dimensions are written
     if (wp == warps - 1) {
       double t = 0.0;
@@ -1277,7 +1277,7 @@ finalize_update_kernel(const float* __restrict__ X, float* __restrict__ C, long 
 }
 
 // Second level of the SSE reduction plus the loop's stop rule (host-streamed tiles, shards).
-__global__ void sse_reduce_kernel(const double* __restrict__ sse_k, int k, double* __restrict__ out,
+__global__ void sse_reduce_kernel(const double* sse_k, int k, double* __restrict__ out,
                                   int* stop, const double* criterion, double* sse_prev,
                                   double* rel_out, int* iters_done, int indexed) {
   if (grid_enter()) return;
@@ -1415,8 +1415,8 @@ namespace {
 
 // Per-kernel ABI: add this tile's canonical per-center sums to FP64 accumulators. One warp per
 // (center, group of 32 dimensions), eight loads in flight, additions in piece order.
-__global__ void accumulate_kernel(const double* __restrict__ part, const int* __restrict__ label_off,
-                                  const int* __restrict__ pstart, int k, int d,
+__global__ void accumulate_kernel(const double* part, const int* label_off,
+                                  const int* pstart, int k, int d,
                                   double* __restrict__ acc, int* __restrict__ acc_counts) {
   if (grid_enter()) return;
   const int groups = (d + 31) / 32;
@@ -1432,11 +1432,11 @@ __global__ void accumulate_kernel(const double* __restrict__ part, const int* __
     for (; p + 8 <= p1; p += 8) {
       double v[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = __ldg(part + (size_t)(p + i) * d + c);
+      for (int i = 0; i < 8; ++i) v[i] = ld(part + (size_t)(p + i) * d + c);
 #pragma unroll
       for (int i = 0; i < 8; ++i) s += v[i];
     }
-    for (; p < p1; ++p) s += __ldg(part + (size_t)p * d + c);
+    for (; p < p1; ++p) s += ld(part + (size_t)p * d + c);
     acc[(size_t)j * d + c] += s;
   }
   if (g == 0 && lane == 0) acc_counts[j] += label_off[j + 1] - label_off[j];
@@ -1445,10 +1445,10 @@ __global__ void accumulate_kernel(const double* __restrict__ part, const int* __
 // Host-streamed tiles: add this tile's canonical per-center sums, member counts and sum of
 // ||x||^2 to the run's FP64 accumulators (the tile's pieces in piece order, then one addition per
 // tile, tiles in order).
-__global__ void accumulate_stream_kernel(const double* __restrict__ part,
-                                         const double* __restrict__ partq,
-                                         const int* __restrict__ label_off,
-                                         const int* __restrict__ pstart, int k, int d,
+__global__ void accumulate_stream_kernel(const double* part,
+                                         const double* partq,
+                                         const int* label_off,
+                                         const int* pstart, int k, int d,
                                          double* __restrict__ accS, int* __restrict__ accN,
                                          double* __restrict__ accQ, const int* stop) {
   if (grid_enter()) return;
@@ -1472,8 +1472,8 @@ __global__ void accumulate_stream_kernel(const double* __restrict__ part,
 
 // Host-streamed tiles: centers and SSE terms from the run's accumulators, one warp per (center,
 // group of 32 dimensions) as finalize_kernel.
-__global__ void finalize_stream_kernel(const double* __restrict__ accS, const int* __restrict__ accN,
-                                       const double* __restrict__ accQ, int k, int d,
+__global__ void finalize_stream_kernel(const double* accS, const int* accN,
+                                       const double* accQ, int k, int d,
                                        float* __restrict__ C, long long ldc, int empty_policy,
                                        double* __restrict__ sse_k, const int* stop) {
   if (grid_enter()) return;
@@ -1505,9 +1505,9 @@ __global__ void finalize_stream_kernel(const double* __restrict__ accS, const in
 }
 
 template <typename T>
-__global__ void finalize_acc_kernel(const double* __restrict__ acc, const int* __restrict__ acc_counts,
+__global__ void finalize_acc_kernel(const double* acc, const int* acc_counts,
                                     int k, int d, T* __restrict__ centers, int* __restrict__ counts,
-                                    const int* __restrict__ dirty) {
+                                    const int* dirty) {
   if (grid_enter()) return;
   const long long total = (long long)k * d;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
@@ -1600,7 +1600,7 @@ namespace {
 // SMEM: the tile's counters in shared memory (one global atomic per peer group, label by label, took
 // 14.7 us for 1.5M rows in 775 tiles).
 template <bool SMEM>
-__global__ void hist_batched_kernel(const int* __restrict__ labels, BatchUpdate b,
+__global__ void hist_batched_kernel(const int* labels, BatchUpdate b,
                                     int* __restrict__ hist, int* err) {
   if (grid_enter()) return;
   extern __shared__ int cnt_s[];
@@ -1623,7 +1623,7 @@ __global__ void hist_batched_kernel(const int* __restrict__ labels, BatchUpdate 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = base + (long long)u * blockDim.x + threadIdx.x;
-      lv[u] = i < i1 ? __ldg(labels + i) - cb : -1;
+      lv[u] = i < i1 ? ld(labels + i) - cb : -1;
       if (i < i1 && (lv[u] < 0 || lv[u] >= kp)) {
         set_error(err, KMGB_DEV_BAD_LABEL);
         lv[u] = -1;
@@ -1648,10 +1648,10 @@ __global__ void hist_batched_kernel(const int* __restrict__ labels, BatchUpdate 
 
 // label_off[g] = first sorted position of global center g (label_off[K] = rows), piece counts
 // and member counts, from the scanned counters.
-__global__ void label_offsets_batched_kernel(const int* __restrict__ hist, BatchUpdate b,
+__global__ void label_offsets_batched_kernel(const int* hist, BatchUpdate b,
                                              int* __restrict__ label_off, int* __restrict__ piece_cnt,
                                              long long* __restrict__ counts,
-                                             const int* __restrict__ dirty) {
+                                             const int* dirty) {
   if (grid_enter()) return;
   const int gc = blockIdx.x * blockDim.x + threadIdx.x;
   if (gc > b.K) return;
@@ -1673,8 +1673,8 @@ __global__ void label_offsets_batched_kernel(const int* __restrict__ hist, Batch
 
 // One warp per sort tile. SMEM: the tile's k counters live in shared memory (k <= smem_k).
 template <bool SMEM>
-__global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpdate b, int* pos,
-                                       int* __restrict__ sorted, const int* __restrict__ dirty) {
+__global__ void scatter_batched_kernel(const int* labels, BatchUpdate b, int* pos,
+                                       int* __restrict__ sorted, const int* dirty) {
   if (grid_enter()) return;
   extern __shared__ int cnt_s[];
   const long long st = blockIdx.x;
@@ -1696,7 +1696,7 @@ __global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpda
     int l = -1;
     if (i < i1) {
       l = lnext - cb;
-      if (l < 0 || l >= kp || (dirty && !__ldg(dirty + cb + l))) l = -1;
+      if (l < 0 || l >= kp || (dirty && !ld(dirty + cb + l))) l = -1;
     }
     if (base + 32 + lane < i1) lnext = labels[base + 32 + lane];  // next batch in flight
     if (!__any_sync(0xffffffffu, l >= 0)) continue;
@@ -1719,9 +1719,9 @@ __global__ void scatter_batched_kernel(const int* __restrict__ labels, BatchUpda
 // kScatterMultiK): one warp's chain of steps took 29.5 us for 775 tiles of 2048 rows.
 constexpr int kScatterMultiK = 48 * 1024 / 4 / kScatterWarps;
 
-__global__ void scatter_batched_multi_kernel(const int* __restrict__ labels, BatchUpdate b,
-                                             const int* __restrict__ pos, int* __restrict__ sorted,
-                                             const int* __restrict__ dirty) {
+__global__ void scatter_batched_multi_kernel(const int* labels, BatchUpdate b,
+                                             const int* pos, int* __restrict__ sorted,
+                                             const int* dirty) {
   if (grid_enter()) return;
   extern __shared__ int wcnt[];  // [kScatterWarps][kp]
   const long long st = blockIdx.x;
@@ -1742,7 +1742,7 @@ __global__ void scatter_batched_multi_kernel(const int* __restrict__ labels, Bat
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = base + 32 * u + lane;
-      lv[u] = i < s1 ? __ldg(labels + i) - cb : -1;
+      lv[u] = i < s1 ? ld(labels + i) - cb : -1;
       if (lv[u] >= kp) lv[u] = -1;
     }
   };
@@ -1755,7 +1755,7 @@ __global__ void scatter_batched_multi_kernel(const int* __restrict__ labels, Bat
   }
   __syncthreads();
   for (int j = threadIdx.x; j < kp; j += blockDim.x) {
-    int run = __ldg(h + (size_t)j * nt + tl);
+    int run = ld(h + (size_t)j * nt + tl);
     for (int v = 0; v < kScatterWarps; ++v) {
       const int c = wcnt[(size_t)v * kp + j];
       wcnt[(size_t)v * kp + j] = run;
@@ -1770,7 +1770,7 @@ __global__ void scatter_batched_multi_kernel(const int* __restrict__ labels, Bat
     if (dirty) {
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (lv[u] >= 0 && !__ldg(dirty + cb + lv[u])) lv[u] = -1;
+        if (lv[u] >= 0 && !ld(dirty + cb + lv[u])) lv[u] = -1;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -1794,7 +1794,7 @@ __global__ void scatter_batched_multi_kernel(const int* __restrict__ labels, Bat
 // recomputed from unchanged labels, which reproduces them bit for bit.
 // The problem's SSE history slot is its own count of recorded iterations (a stopped problem
 // records nothing more), so every iteration issues the same launch: a CUDA graph replays it.
-__global__ void sse_batched_kernel(const double* __restrict__ sse_k, int groups, BatchUpdate b) {
+__global__ void sse_batched_kernel(const double* sse_k, int groups, BatchUpdate b) {
   if (grid_enter()) return;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
