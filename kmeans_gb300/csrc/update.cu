@@ -866,13 +866,11 @@ piece_sums_few_kernel(const float* X, long long ldx, const double* qn,
     PieceAcc a;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
-      if (32 * w + 32 <= n) {
-#pragma unroll
-        for (int r = 0; r < 32; ++r) a.add(v[32 * w + r]);
-      } else {  // zeros past the piece: adding them changes no float-float sum
+      // zeros past the piece: adding them changes no float-float sum (no window ends the loop, or v
+      // would be indexed at run time and lie in local memory)
+      if (32 * w < n) {
 #pragma unroll
         for (int r = 0; r < 32; ++r) a.add(32 * w + r < n ? v[32 * w + r] : 0.0f);
-        break;
       }
     }
     if (on) part[(size_t)p * d + c] = a.value();
@@ -901,8 +899,8 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
   const bool vec = ldx % 4 == 0 && d % 4 == 0 && d < (1 << 23) &&
                    (reinterpret_cast<uintptr_t>(X) & 15) == 0;
   // up to 8 warps of work an SM, what it holds of the kernel: the latency of a piece's loads is what
-  // counts (846 pieces of 32 dimensions 16.7 -> 11.2 us, 63 pieces 16.2 -> 8.9; 958 of 128 dimensions,
-  // 25 warps an SM, 20.9 -> 25.2)
+  // counts (846 pieces of 32 dimensions 16.7 -> 9.1 us, 63 pieces 16.2 -> 7.2; 958 of 128 dimensions,
+  // 25 warps an SM, 14.4 with the ring and 20.7 with this kernel)
   const long long few = max_pieces * ((d + 31) / 32);
   if (few <= kmgb::num_sms() * 8LL) {
     launch(piece_sums_few_kernel, (unsigned)((few + 3) / 4), 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k,
