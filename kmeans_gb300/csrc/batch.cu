@@ -542,7 +542,7 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
   long long* d_crend = nullptr;
   double work = 0.0;
   for (int i = 0; i < P; ++i) work += (double)(rend[i] - rbeg[i]) * (double)rup(kk[i], 256) * d;
-  if (tc && o.certify && max_iters > 1 && work >= kPruneMinWork) {
+  if (tc && o.certify && max_iters > 1 && work >= kPruneMinWork && prune_enabled()) {
     std::vector<int> wprob, wrow, cuprob(K / 256);
     std::vector<long long> crend(P);
     for (int i = 0; i < P; ++i) {

@@ -137,6 +137,21 @@ void dev_trim(size_t keep) {
   if (pool_of_current_device(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, keep);
 }
 
+size_t dev_available() {
+  size_t mem_free = 0, mem_total = 0;
+  cudaMemPool_t pool = nullptr;
+  uint64_t held = 0, used = 0;
+  if (cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (pool_of_current_device(&pool) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
+    mem_free += held - used;
+  return mem_free;
+}
+
 cudaError_t dev_release_cached() {
   cudaError_t r = cudaDeviceSynchronize();
   std::lock_guard<std::mutex> g(g_mu);

@@ -256,6 +256,7 @@ struct kmgb_handle {
   void* XlF = nullptr;
   // distance bounds between the iterations of a run (n 0: off), their buffers in one allocation
   PruneState pr;
+  bool bounds_wanted = false;  // worth their memory, and not tried yet
   void* prune_arena = nullptr;
   int* crr_list = nullptr;  // scratch of the centers' own scan
   // k-means++ work space (allocated on first use): D^2, block weight sums, max/pick, picks
@@ -363,16 +364,19 @@ constexpr int kPruneLong = 8;  // iterations
 
 bool prune_wanted(const kmgb_options& o, bool mini, bool streaming, long long n, int d, int k) {
   if (o.assign_tier == KMGB_ASSIGN_FP8) return false;
-  if (!o.certify || mini || streaming || o.router || k < 2) return false;
+  if (!o.certify || mini || streaming || o.router || k < 2 || !prune_enabled()) return false;
   const long long least = o.assign_tier == KMGB_ASSIGN_FP32 ? kPruneMinWorkFp32 : kPruneMinWork;
   return n * round_up(k, kCenterPad) >= least / d &&
          k * (o.max_iters >= kPruneLong ? kPruneRowsLong : kPruneRows) <= n;
 }
 
-// The bounds' buffers, from the pool. They are an optimisation: where they do not fit, the handle
-// scans every row in every iteration.
-void alloc_prune(kmgb_handle* h, bool split) {
+// The bounds' buffers, from the pool: an optimisation, so a handle that stays takes them only where three
+// times as much is left for others, and gives them up where it cannot use them (drop_bounds); without
+// them it scans every row in every iteration.
+void alloc_prune(kmgb_handle* h, bool one_shot) {
+  h->bounds_wanted = false;
   const bool tc = h->opt.assign_tier != KMGB_ASSIGN_FP32;
+  const bool split = h->opt.assign_tier == KMGB_ASSIGN_BF16X3;
   const long long row = tc ? h->ldb * 2 * (split ? 2 : 1) : h->ldx * 4;
   PruneState p;
   p.n = h->n;
@@ -400,6 +404,7 @@ void alloc_prune(kmgb_handle* h, bool split) {
   };
   Arena sizing;
   carve(sizing);
+  if (!one_shot && dev_available() / 4 < sizing.off) return;
   if (dev_alloc(&h->prune_arena, sizing.off, h->stream) != cudaSuccess) {
     cudaGetLastError();
     h->prune_arena = nullptr;
@@ -411,7 +416,34 @@ void alloc_prune(kmgb_handle* h, bool split) {
   h->pr = p;
 }
 
-int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_options* opt) {
+// Gives the bounds' memory back; the captured iteration, which uses it, goes with it. False: none held.
+bool drop_bounds(kmgb_handle* h) {
+  h->bounds_wanted = false;
+  if (!h->prune_arena) return false;
+  cudaStreamSynchronize(h->stream);
+  if (h->gexec) cudaGraphExecDestroy(h->gexec);
+  h->gexec = nullptr;
+  dev_free(h->prune_arena, h->stream);
+  h->prune_arena = nullptr;
+  h->pr = PruneState{};
+  h->crr_list = nullptr;
+  return true;
+}
+
+// Memory a call of the handle needs goes before the bounds.
+template <typename F>
+cudaError_t needed(kmgb_handle* h, F alloc) {
+  cudaError_t r = alloc();
+  if (r == cudaErrorMemoryAllocation && drop_bounds(h)) {
+    cudaGetLastError();
+    r = alloc();
+  }
+  return r;
+}
+
+// one_shot: the handle of a single call, gone when it returns.
+int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_options* opt,
+                  bool one_shot = false) {
   *out = nullptr;
   if (n <= 0 || d <= 0 || k <= 0) {
     set_err("kmgb_create: n, d and k must be positive");
@@ -638,7 +670,8 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   w.sse_indexed = h->streaming ? 0 : 1;  // host-streamed iterations write their own slot
   h->sse_cap = std::max(1, h->opt.max_iters);
   KM_TRY(dalloc(&h->sse_dev, h->sse_cap, h->stream), (delete h, code));
-  if (prune_wanted(h->opt, h->mini, h->streaming, n, d, k)) alloc_prune(h, split);
+  h->bounds_wanted = prune_wanted(h->opt, h->mini, h->streaming, n, d, k);
+  if (h->bounds_wanted && h->opt.max_iters > 1) alloc_prune(h, one_shot);
   *out = h;
   return 0;
 }
@@ -1413,10 +1446,17 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
   iters = std::max(iters, 0);
   if (iters > h->sse_cap) {
     double* nd = nullptr;
-    KM_TRY(dalloc(&nd, iters, h->stream), KMEANS_ERROR_COMPUTE);
+    KM_TRY(needed(h, [&] { return dalloc(&nd, iters, h->stream); }), KMEANS_ERROR_COMPUTE);
     dev_free(h->sse_dev, h->stream);
     h->sse_dev = nd;
     h->sse_cap = iters;
+  }
+  if (h->bounds_wanted && iters > 1) {  // created for single iterations
+    alloc_prune(h, false);
+    if (h->pr.n > 0 && h->gexec) {
+      cudaGraphExecDestroy(h->gexec);
+      h->gexec = nullptr;
+    }
   }
   h->sse_host.assign(iters, 0.0);
   h->run_base = h->iter_base;
@@ -1590,8 +1630,8 @@ int init_kmeanspp(kmgb_handle* h, unsigned long long seed, int* picks_out) {
     return code;
   }
   if (!h->kpp_picks) {
-    KM_TRY(alloc_kpp(&h->kpp, h->n, h->k, h->stream), code);
-    KM_TRY(dalloc(&h->kpp_picks, (size_t)h->k, h->stream), code);
+    KM_TRY(needed(h, [&] { return alloc_kpp(&h->kpp, h->n, h->k, h->stream); }), code);
+    KM_TRY(needed(h, [&] { return dalloc(&h->kpp_picks, (size_t)h->k, h->stream); }), code);
   }
   KM_TRY(cudaMemsetAsync(h->C, 0, sizeof(float) * h->ldx * h->k, h->stream), code);
   KM_TRY(launch_kmeanspp(h->X, h->ldx, h->n, h->d, h->k, seed, h->C, h->ldx, h->kpp_picks,
@@ -1936,6 +1976,7 @@ static int shard_prepare(kmgb_handle* h) {
     };
     Arena sizing;
     carve(sizing);
+    drop_bounds(h);  // a shard's labels come from full scans
     KM_TRY(dev_alloc(&h->shard_arena, sizing.off, h->stream), KMEANS_ERROR_COMPUTE);
     Arena cut;
     cut.base = static_cast<char*>(h->shard_arena);
@@ -2076,7 +2117,7 @@ int kmgb_tc_accumulators(const float* X, long long n, int d, const float* C, int
   o.certify = 0;
   o.max_iters = 1;
   kmgb_handle* h = nullptr;
-  int rc = create_handle(&h, n, d, k, &o);
+  int rc = create_handle(&h, n, d, k, &o, true);
   if (rc) return rc;
   const int kpad = (int)round_up(k, kCenterPad);
   float* dump = nullptr;
@@ -2147,7 +2188,7 @@ int kmgb_lloyd_f32(const float* X, long long n, int d, int k, const float* init,
   else kmgb_default_options(&o);
   if (!X) return KMEANS_ERROR_BUILDDATA;
   kmgb_handle* h = nullptr;
-  int rc = create_handle(&h, n, d, k, &o);
+  int rc = create_handle(&h, n, d, k, &o, true);
   if (rc) return rc;
   const bool x_dev = is_device_ptr(X);
   const bool kpp = !init && o.init_algorithm == KMGB_INIT_KMEANSPP;
@@ -2234,7 +2275,7 @@ kmeansErrorStatus computeKmeansF(const float* data, const int m, const int n, co
   o.criterion = criterion;
   o.mini_batch_fraction = miniBatchFraction;
   kmgb_handle* h = nullptr;
-  int rc = create_handle(&h, m, n, k, &o);
+  int rc = create_handle(&h, m, n, k, &o, true);
   if (rc) return (kmeansErrorStatus)rc;
   const bool kpp = initAlgorithm == KMGB_INIT_KMEANSPP;  // the reference ignores numRetries
   std::shared_future<RefInit> ref;

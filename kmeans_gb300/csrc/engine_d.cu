@@ -213,7 +213,7 @@ struct DevBufs {
 // sums and SSE of the unchanged clusters are saved as well (400,000 x 64, K=256).
 bool prune_worthwhile(long long m, int k, int d) {
   const long long kp = (k + kCenterPad - 1) / kCenterPad * kCenterPad;
-  return k >= 2 && (long long)k * 32 <= m && m * kp >= (1LL << 31) / d;
+  return prune_enabled() && k >= 2 && (long long)k * 32 <= m && m * kp >= (1LL << 31) / d;
 }
 
 // The bounds' buffers; where they do not fit, every iteration scans every row.

@@ -269,6 +269,8 @@ struct PruneState {
   void* Xc = nullptr;      // [cap][ldb] compact rows (BF16), and their residual plane
   void* Xlc = nullptr;
 };
+// False with KMGB_BOUNDS=0 in the environment: every row is scanned, no memory is taken for bounds.
+bool prune_enabled();
 // Resets / reads the flags and the two largest moves; then every row's bounds are moved with the
 // centers and the rows whose label they no longer prove are listed (flags[1] > cap: all rows).
 cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
@@ -502,6 +504,8 @@ cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
 // Unused memory beyond `keep` bytes goes back to the device.
 void dev_trim(size_t keep);
+// Bytes that could be allocated now: the device's free memory and the pool's unused.
+size_t dev_available();
 cudaError_t dev_release_cached();
 
 }  // namespace kmgb

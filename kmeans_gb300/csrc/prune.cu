@@ -13,6 +13,9 @@
 // (kmeans.cpp:910-1014). Nothing survives a run: its first iteration scans every row.
 //
 // prune_filter_kernel is bound by HBM: 12 bytes read and 8 written per row.
+#include <cstdlib>
+#include <cstring>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -428,6 +431,11 @@ prune_dirty_batched_kernel(PruneBatch pb, const int* labels) {
 }
 
 }  // namespace
+
+bool prune_enabled() {
+  const char* v = std::getenv("KMGB_BOUNDS");
+  return !(v && std::strcmp(v, "0") == 0);
+}
 
 cudaError_t launch_prune_batched(const PruneBatch& pb, const int* labels, const void* Xb,
                                  const void* Xl, long long row_bytes, cudaStream_t s) {

@@ -94,3 +94,103 @@ def test_fp64_driver(km, orc, torch_cuda, n, d, k, span):
     assert km.computeKmeansD(X, n, d, k, -1.0, 6, 1, 0, 0, 0, result, 1.0) == 13
     _, c, _, _, _ = orc.lloyd_d(X, init, 6)
     assert np.array_equal(result.reshape(d, k).T, c, equal_nan=True)
+
+
+def large():
+    n, d, k = 70_001, 128, 1000
+    X, _, _ = mixture_numpy(n, d, k, seed=31, mean_lo=-20, mean_hi=20, std=(0.3, 3.0))
+    return n, d, k, X, X[sample_init(n, k, seed=5)].copy()
+
+
+def test_bounds_memory_only_where_it_is_used(km, orc, torch_cuda, monkeypatch):
+    """A handle for single iterations and a sharded one hold what a handle without bounds holds; a
+    longer run takes the memory when it comes."""
+    n, d, k, X, init = large()
+    torch_cuda.cuda.synchronize()
+    base = km.debug_pool_used_bytes()
+
+    def held(h):
+        h.synchronize()
+        torch_cuda.cuda.synchronize()
+        return km.debug_pool_used_bytes() - base
+
+    def make(max_iters):
+        h = km.Handle(n, d, k, assign_tier=km.ASSIGN_BF16X3, empty_policy=1, max_iters=max_iters)
+        h.set_data(X, on_device=False)
+        h.set_centers(init)
+        return h
+
+    monkeypatch.setenv("KMGB_BOUNDS", "0")
+    plain = make(6)
+    least = held(plain)
+    S0, c0, Q0 = plain.shard_partials()
+    least_shard = held(plain)
+    plain.close()
+    monkeypatch.delenv("KMGB_BOUNDS")
+
+    h = make(6)
+    assert held(h) > least + n * 20
+    S, c, Q = h.shard_partials()
+    assert held(h) == least_shard
+    assert np.array_equal(S, S0) and np.array_equal(c, c0) and np.array_equal(Q, Q0)
+    h.shard_update(S, c, Q)
+    one = orc.lloyd_tiled(X, init, 1, tile_rows=n, empty_policy=1)
+    assert np.array_equal(h.centers(), one[1])
+    h.close()
+
+    h = make(1)
+    h.run(1)
+    assert held(h) <= least
+    h.set_centers(init)
+    h.run(5)  # after a captured iteration without bounds
+    h.synchronize()
+    want = orc.lloyd(X, init, 5, empty_policy=1)
+    assert np.array_equal(h.centers(), want[1]) and np.array_equal(h.labels(), want[2])
+    assert held(h) > least + n * 20
+    h.close()
+    assert km.debug_pool_used_bytes() == base
+
+
+def test_bounds_give_way_to_memory_a_call_needs(km, orc, torch_cuda):
+    n, d, k, X, init = large()
+    h = km.Handle(n, d, k, assign_tier=km.ASSIGN_BF16X3, empty_policy=1, max_iters=4)
+    h.set_data(X, on_device=False)
+    h.set_centers(init)
+    h.run(2)
+    h.synchronize()
+    km.debug_fail_nth(km.FAULT_ALLOC, 1)
+    try:
+        picks = h.init_kmeanspp(3)
+    finally:
+        km.debug_fail_nth(km.FAULT_ALLOC, 0)
+    assert len(set(picks.tolist())) == k
+    h.set_centers(init)
+    h.run(4)
+    h.synchronize()
+    want = orc.lloyd(X, init, 4, empty_policy=1)
+    assert np.array_equal(h.centers(), want[1]) and np.array_equal(h.labels(), want[2])
+    h.close()
+
+
+def test_bounds_without_room(km, orc, torch_cuda):
+    """The bounds' own allocation (the third of a call) does not fit: every row is scanned."""
+    n, d, k, X, init = large()
+    km.debug_fail_nth(km.FAULT_ALLOC, 3)
+    try:
+        res = km.lloyd(X, k, init=init, max_iters=5, assign_tier=km.ASSIGN_BF16X3, empty_policy=1)
+    finally:
+        km.debug_fail_nth(km.FAULT_ALLOC, 0)
+    check(res, orc.lloyd(X, init, 5, empty_policy=1))
+
+
+@pytest.mark.parametrize("tier", ["BF16X3", "FP32"])
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e30])
+def test_bounds_with_rows_that_spoil_a_center(km, torch_cuda, monkeypatch, tier, value):
+    n, d, k, X, init = large()
+    X[5, 3] = X[60_000, 100] = value
+    t = getattr(km, "ASSIGN_" + tier)
+    got = km.lloyd(X, k, init=init, max_iters=5, assign_tier=t, empty_policy=1)
+    monkeypatch.setenv("KMGB_BOUNDS", "0")
+    want = km.lloyd(X, k, init=init, max_iters=5, assign_tier=t, empty_policy=1)
+    assert np.array_equal(got.labels, want.labels)
+    assert np.array_equal(got.centers, want.centers, equal_nan=True)
