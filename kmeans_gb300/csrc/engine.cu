@@ -257,6 +257,7 @@ struct kmgb_handle {
   // distance bounds between the iterations of a run (n 0: off), their buffers in one allocation
   PruneState pr;
   bool bounds_wanted = false;  // worth their memory, and not tried yet
+  bool bounds_on = false;      // in the current run
   void* prune_arena = nullptr;
   int* crr_list = nullptr;  // scratch of the centers' own scan
   // k-means++ work space (allocated on first use): D^2, block weight sums, max/pick, picks
@@ -356,18 +357,21 @@ int audit_rows_for(const kmgb_options& o, bool streaming, int k, int d) {
 constexpr long long kPruneMinWork = 1LL << 33;  // rows x centers (in chunks of 256) x dimensions
 constexpr long long kPruneMinWorkFp32 = 1LL << 30;
 constexpr long long kPruneMaxBytes = 8LL << 30;  // of the compact copy
-// The centers' scan is k / n of the rows' scan, and what it saves comes after the first moves have died
-// down: 3 iterations of 1M x 256, K=16,384 took 43.17 ms with the bounds and 43.04 without. From 64
-// rows a center on it is small next to one iteration; down to 32 the run has to be long enough.
-constexpr long long kPruneRows = 64, kPruneRowsLong = 32;
-constexpr int kPruneLong = 8;  // iterations
+// What the bounds save comes after the first moves have died down, so it is the length of the run that
+// decides: time with them over time without, for 24 shapes from 30,000 x 256, K=900 to 4M x 128, K=1024 (32
+// to 7,800 rows a center, both tiers) in clusters that lie apart: 3 iterations 0.98 - 1.15, 4 iterations
+// 0.89 - 1.14, 5 iterations 0.78 - 1.09, 8 iterations 0.57 - 0.92; in overlapping and Zipf-sized ones 0.93 -
+// 1.16 whatever the length up to 8. Within each of them the rows a center made no difference (at K=16,384,
+// 8 iterations: 0.62 at 32, 0.57 at 40, 0.59 at 48, 0.61 at 61, 0.59 at 79); 32 keeps the scan of the
+// centers, k / n of the rows', small.
+constexpr long long kPruneRows = 32;
+constexpr int kPruneIters = 4;  // of a run
 
 bool prune_wanted(const kmgb_options& o, bool mini, bool streaming, long long n, int d, int k) {
   if (o.assign_tier == KMGB_ASSIGN_FP8) return false;
   if (!o.certify || mini || streaming || o.router || k < 2 || !prune_enabled()) return false;
   const long long least = o.assign_tier == KMGB_ASSIGN_FP32 ? kPruneMinWorkFp32 : kPruneMinWork;
-  return n * round_up(k, kCenterPad) >= least / d &&
-         k * (o.max_iters >= kPruneLong ? kPruneRowsLong : kPruneRows) <= n;
+  return n * round_up(k, kCenterPad) >= least / d && k * kPruneRows <= n;
 }
 
 // The bounds' buffers, from the pool: an optimisation, so a handle that stays takes them only where three
@@ -426,6 +430,7 @@ bool drop_bounds(kmgb_handle* h) {
   dev_free(h->prune_arena, h->stream);
   h->prune_arena = nullptr;
   h->pr = PruneState{};
+  h->bounds_on = false;
   h->crr_list = nullptr;
   return true;
 }
@@ -671,7 +676,7 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
   h->sse_cap = std::max(1, h->opt.max_iters);
   KM_TRY(dalloc(&h->sse_dev, h->sse_cap, h->stream), (delete h, code));
   h->bounds_wanted = prune_wanted(h->opt, h->mini, h->streaming, n, d, k);
-  if (h->bounds_wanted && h->opt.max_iters > 1) alloc_prune(h, one_shot);
+  if (h->bounds_wanted && h->opt.max_iters >= kPruneIters) alloc_prune(h, one_shot);
   *out = h;
   return 0;
 }
@@ -1107,7 +1112,7 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
   KM_TRY(h->pmark(0), KMEANS_ERROR_RESET);
   // reset (kmeans.cpp:1142-1170): norms of the current centers, cleared counters
   KM_TRY(cudaMemsetAsync(h->cmax, 0, sizeof(float) + 4 * sizeof(int), s), KMEANS_ERROR_RESET);
-  const bool prune = h->pr.n > 0 && !assign_only;
+  const bool prune = h->bounds_on && !assign_only;
   KM_TRY(launch_prep_centers(h->C, h->ldx, h->k, h->d, h->Cop, h->Cb, h->ldb, h->cn, h->cmax, s,
                              h->stop, h->cinit, h->Cl, h->cbias, prune ? h->pr.shift : nullptr,
                              prune ? h->pr.cxn : nullptr, 0.0f, h->Ct, round_up(h->k, 4)),
@@ -1451,13 +1456,13 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
     h->sse_dev = nd;
     h->sse_cap = iters;
   }
-  if (h->bounds_wanted && iters > 1) {  // created for single iterations
-    alloc_prune(h, false);
-    if (h->pr.n > 0 && h->gexec) {
-      cudaGraphExecDestroy(h->gexec);
-      h->gexec = nullptr;
-    }
+  if (h->bounds_wanted && iters >= kPruneIters) alloc_prune(h, false);  // created for shorter runs
+  const bool bounds = h->pr.n > 0 && iters >= kPruneIters;
+  if (bounds != h->bounds_on && h->gexec) {  // captured the other way
+    cudaGraphExecDestroy(h->gexec);
+    h->gexec = nullptr;
   }
+  h->bounds_on = bounds;
   h->sse_host.assign(iters, 0.0);
   h->run_base = h->iter_base;
   h->criterion = criterion;
@@ -1467,7 +1472,7 @@ int run(kmgb_handle* h, int iters, double criterion, const float* upload = nullp
   launch(begin_run_kernel, 1, 1, 0, h->stream)(h->loopf, criterion, h->win_base, h->run_base);
   count_launches(1);
   KM_TRY(cudaGetLastError(), KMEANS_ERROR_COMPUTE);
-  if (h->pr.n > 0)  // no bounds yet: the first iteration scans every row
+  if (h->bounds_on)  // no bounds yet: the first iteration scans every row
     KM_TRY(cudaMemsetAsync(h->pr.flags, 0, 8 * sizeof(int), h->stream), KMEANS_ERROR_COMPUTE);
   KM_TRY(cudaEventRecord(h->ev0, h->stream), KMEANS_ERROR_COMPUTE);
   int first = 0;

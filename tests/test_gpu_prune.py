@@ -194,3 +194,21 @@ def test_bounds_with_rows_that_spoil_a_center(km, torch_cuda, monkeypatch, tier,
     want = km.lloyd(X, k, init=init, max_iters=5, assign_tier=t, empty_policy=1)
     assert np.array_equal(got.labels, want.labels)
     assert np.array_equal(got.centers, want.centers, equal_nan=True)
+
+
+@pytest.mark.parametrize("graphs", ["1", "0"])
+def test_run_length_decides(km, orc, torch_cuda, monkeypatch, graphs):
+    """Short and long runs of one handle in turn (without and with bounds, each its own capture), and a
+    handle created for short runs that gets a long one."""
+    monkeypatch.setenv("KMGB_GRAPHS", graphs)
+    n, d, k, X, init = large()
+    want = {it: orc.lloyd(X, init, it, empty_policy=1) for it in (1, 3, 4, 6)}
+    for max_iters, runs in ((8, (3, 6, 1, 4)), (2, (1, 3, 6, 3))):
+        h = km.Handle(n, d, k, assign_tier=km.ASSIGN_BF16X3, empty_policy=1, max_iters=max_iters)
+        h.set_data(X, on_device=False)
+        for it in runs:
+            h.set_centers(init)
+            h.run(it)
+            h.synchronize()
+            assert np.array_equal(h.centers(), want[it][1]) and np.array_equal(h.labels(), want[it][2])
+        h.close()
