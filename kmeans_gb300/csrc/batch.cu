@@ -194,24 +194,45 @@ bool initial_centers(const kmgb_problem* pr, const std::vector<int>& ids, int d,
   return true;
 }
 
+// Page-locked memory of the uploads' buffers; a group takes no more than its rows need, and groups
+// side by side share it.
+constexpr size_t kStagingBytes = 512ull << 20;
+
+cudaError_t pinned_alloc(float** p, size_t bytes) {
+  *p = nullptr;
+  if (inject_fault(kFaultAlloc)) return cudaErrorMemoryAllocation;
+  return cudaHostAlloc(reinterpret_cast<void**>(p), bytes, cudaHostAllocDefault);
+}
+
 // Host problems' rows into X (rows x ldx): chunks of rows are packed into two alternating
 // pinned buffers by host threads (zeros for padding rows and columns) and copied with
-// cudaMemcpyAsync while the next chunk is packed.
+// cudaMemcpyAsync while the next chunk is packed. `staging` bytes of pinned memory at most, less where
+// less can be had.
 bool upload_host_rows(const kmgb_problem* pr, const std::vector<int>& ids, int d, long long ldx,
                       long long rows, long long row_pad, const std::vector<long long>& rbeg,
                       const std::vector<long long>& rend, const std::vector<char>& is_dev,
-                      float* X, cudaStream_t s, Fail& f) {
+                      float* X, cudaStream_t s, Fail& f, size_t staging) {
   const int E = KMEANS_ERROR_BUILDDATA;
-  const long long chunk_rows = std::max<long long>(1, (256LL << 20) / (ldx * 4));
+  long long chunk_rows = std::max<long long>(1, (long long)(staging / 2) / (ldx * 4));
+  chunk_rows = std::min(chunk_rows, (rows + 1) / 2);
   float* buf[2] = {nullptr, nullptr};
   cudaEvent_t freed[2] = {nullptr, nullptr};
   bool ok = true;
-  for (int b = 0; b < 2 && ok; ++b) {
-    ok = !f.set(cudaHostAlloc(reinterpret_cast<void**>(&buf[b]),
-                              sizeof(float) * chunk_rows * ldx, cudaHostAllocDefault),
-                E, "pinned staging") &&
-         !f.set(cudaEventCreateWithFlags(&freed[b], cudaEventDisableTiming), E, "staging event");
+  for (;;) {
+    cudaError_t e = pinned_alloc(&buf[0], sizeof(float) * chunk_rows * ldx);
+    if (e == cudaSuccess) e = pinned_alloc(&buf[1], sizeof(float) * chunk_rows * ldx);
+    if (e == cudaSuccess) break;
+    cudaGetLastError();
+    if (buf[0]) cudaFreeHost(buf[0]);
+    buf[0] = buf[1] = nullptr;
+    if (chunk_rows * ldx <= 1 << 16) {  // 256 KB
+      f.set(e, E, "pinned staging");
+      return false;
+    }
+    chunk_rows = (chunk_rows + 3) / 4;
   }
+  for (int b = 0; b < 2 && ok; ++b)
+    ok = !f.set(cudaEventCreateWithFlags(&freed[b], cudaEventDisableTiming), E, "staging event");
   const int P = (int)ids.size();
   // problem i's padded region is rows [rbeg[i], pend(i)); the regions tile [0, rows)
   auto pend = [&](int i) { return rbeg[i] + rup(rend[i] - rbeg[i], row_pad); };
@@ -273,7 +294,7 @@ bool upload_host_rows(const kmgb_problem* pr, const std::vector<int>& ids, int d
 // One group: problems `ids` (all of dimension d).
 int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_options& o,
               cudaStream_t s, unsigned long long* reranked, double* loop_ms, double* phase_ms,
-              Fail& f, long long* graph_launches, unsigned long long* audit) {
+              Fail& f, long long* graph_launches, unsigned long long* audit, size_t staging) {
   const int P = (int)ids.size();
   const long long ldx = rup(d, 4);
   const long long ldb = rup(d, 8);
@@ -389,7 +410,8 @@ int run_group(kmgb_problem* pr, const std::vector<int>& ids, int d, const kmgb_o
     is_dev[i] = on_device(pr[ids[i]].X) ? 1 : 0;
     any_host |= !is_dev[i];
   }
-  if (any_host && !upload_host_rows(pr, ids, d, ldx, rows, row_pad, rbeg, rend, is_dev, X, s, f))
+  if (any_host &&
+      !upload_host_rows(pr, ids, d, ldx, rows, row_pad, rbeg, rend, is_dev, X, s, f, staging))
     return f.code;
   for (int i = 0; i < P; ++i) {
     const kmgb_problem& q = pr[ids[i]];
@@ -927,6 +949,7 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
   if (!f.code && !f.set(cudaEventCreateWithFlags(&ready.e, cudaEventDisableTiming), KMEANS_ERROR_BUILDDATA,
                         "default stream"))
     f.set(cudaEventRecord(ready.e, cudaStreamLegacy), KMEANS_ERROR_BUILDDATA, "default stream");
+  size_t staging = kStagingBytes;
   auto run_one = [&](Group& g) {
     cudaSetDevice(dev);  // worker threads use the caller's device
     cudaStream_t s = nullptr;
@@ -937,7 +960,7 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
     try {
       if (!g.f.set(cudaStreamWaitEvent(s, ready.e, 0), KMEANS_ERROR_BUILDDATA, "default stream"))
         run_group(problems, g.ids, g.d, og, s, &g.reranked, &g.loop_ms, g.phase_ms, g.f, &g.graph_launches,
-                  g.audit);
+                  g.audit, staging);
     } catch (const std::exception&) {  // host memory or threads: an exception must not leave a thread
       g.f.code = KMEANS_ERROR_BUILDDATA;
       g.f.msg = "kmgb_lloyd_batched_f32: out of host memory or threads";
@@ -958,6 +981,7 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
   size_t next = 0;
   if (side_by_side) {
     std::atomic<size_t> at{0};
+    staging /= std::min<size_t>(groups.size(), kGroupThreads);
     auto work = [&] {
       for (size_t g; (g = at.fetch_add(1)) < groups.size();) run_one(groups[g]);
     };
@@ -969,6 +993,7 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
     for (std::thread& t : workers) t.join();
     next = groups.size();
   }
+  staging = kStagingBytes;
   for (; next < groups.size() && !f.code; ++next) {
     run_one(groups[next]);
     f = groups[next].f;

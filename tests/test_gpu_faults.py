@@ -225,3 +225,30 @@ def test_closest_centers_after_a_wait_that_gave_up(km, torch_cuda, dtype, n):
     finally:
         km.debug_withhold_stage(0, 0)
     assert np.array_equal(out.cpu().numpy()[2:], want)
+
+
+def test_batched_upload_with_less_pinned_memory(km, orc, torch_cuda, no_graphs):
+    """Page-locked staging that cannot be had at its size is taken smaller: among the allocations of a
+    call made to fail in turn, its two leave the result as it is; the ones before and after fail the
+    call."""
+    from kmeans_gb300.synthetic import mixture_numpy, sample_init
+    probs = []
+    for i, (n, d, k) in enumerate([(9000, 24, 8), (7001, 24, 5), (20_000, 24, 12)]):
+        X, _, _ = mixture_numpy(n, d, k, seed=80 + i)
+        probs.append((X, k, X[sample_init(n, k, seed=i)].copy()))
+    want = [orc.lloyd(X, init, 3) for X, _, init in probs]
+    ran = []
+    for nth in range(1, 81):
+        km.debug_fail_nth(km.FAULT_ALLOC, nth)
+        try:
+            res, _ = km.lloyd_batched(probs, max_iters=3, assign_tier=km.ASSIGN_FP32)
+            ran.append(True)
+            for r, w in zip(res, want):
+                assert np.array_equal(r.labels, w[2]) and np.array_equal(r.centers, w[1])
+        except km.KmeansError:
+            ran.append(False)
+        finally:
+            km.debug_fail_nth(km.FAULT_ALLOC, 0)
+    first = ran.index(True)
+    assert first > 0 and ran[first:first + 3] == [True, True, False]
+    assert ran[-1]  # past the call's last allocation
