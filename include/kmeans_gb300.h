@@ -445,7 +445,9 @@ KMGB_EXPORT long long kmgb_launch_count(void);
  * memory for the next handle (no reference counterpart: the reference allocates and frees with
  * cudaMalloc/cudaFree in kmeans.cpp:577-683 and its destructor, kmeans.cpp:145-244). This call waits for the current
  * device and returns every pool's unused memory to the device; 0 on success. Setting
- * KMGB_POOL=0 in the environment makes every free return its memory at once. */
+ * KMGB_POOL=0 in the environment makes every free return its memory at once. computeKmeansD, the
+ * batched call, kmgb_kmeanspp_* and ClosestCentersF/D take their workspaces from a pool of their own,
+ * which keeps at most 8 GB from one call for the next (KMGB_POOL=0: nothing). */
 KMGB_EXPORT int kmgb_release_cached_memory(void);
 
 /* Test hooks for failure paths (no reference counterpart; the reference reports failures only

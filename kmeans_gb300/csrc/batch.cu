@@ -78,7 +78,6 @@ constexpr long long kMaxHist = 60LL << 20;  // scan capacity of the counting sor
 constexpr long long kMaxXBytes = 32LL << 30;
 
 constexpr size_t kGroupThreads = 4;     // groups side by side
-constexpr size_t kPoolKeep = 8ull << 30;  // of the groups' memory, for the next call
 constexpr double kPruneMinWork = 2147483648.0;  // rows x centers (chunks of 256) x dimensions
 
 long long rup(long long v, long long m) { return (v + m - 1) / m * m; }
@@ -100,12 +99,12 @@ struct DevPool {
   cudaStream_t s;
   explicit DevPool(cudaStream_t st) : s(st) {}
   ~DevPool() {
-    for (void* p : ptrs) dev_free(p, s);
+    for (void* p : ptrs) call_free(p, s);
   }
   template <typename T>
   cudaError_t alloc(T** p, size_t count) {
     void* v = nullptr;
-    const cudaError_t e = dev_alloc_async(&v, sizeof(T) * (count ? count : 1), s);
+    const cudaError_t e = call_alloc(&v, sizeof(T) * (count ? count : 1), s);
     *p = static_cast<T*>(v);
     if (e == cudaSuccess) ptrs.push_back(v);
     return e;
@@ -1011,7 +1010,6 @@ extern "C" int kmgb_lloyd_batched_f32(kmgb_problem* problems, int count, const k
     for (int ph = 0; ph < 4; ++ph) phase_ms[ph] += g.phase_ms[ph];
     graph_launches += g.graph_launches;
   }
-  dev_trim(kPoolKeep);
   if (stats) {
     std::memset(stats, 0, sizeof(*stats));
     int it = 0;

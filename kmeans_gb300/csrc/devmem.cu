@@ -1,12 +1,17 @@
-// Device memory of handles: one stream-ordered memory pool per device, owned by the library.
+// Device memory: two stream-ordered memory pools per device, owned by the library.
 //
-// A handle's fixed buffers are one arena (engine.cu). With cudaMalloc/cudaFree a one-shot call
+// Handles. A handle's fixed buffers are one arena (engine.cu). With cudaMalloc/cudaFree a one-shot call
 // on the 4M x 128, K=1024 workload spent ~1 ms allocating and ~3.3 ms freeing its ~7 GB (the
 // free synchronizes the device and unmaps). Here the arena comes from a pool whose release
 // threshold is unbounded: cudaFreeAsync hands the memory back to the pool, and the next handle
 // of the same or a smaller size takes it again without mapping anything. The pool keeps what it
-// holds until kmgb_release_cached_memory() (or a failed allocation, which trims it and retries
+// holds until kmgb_release_cached_memory() (or a failed allocation, which trims both pools and retries
 // once); KMGB_POOL=0 trims after every free, which gives back cudaMalloc/cudaFree behaviour.
+//
+// Calls (computeKmeansD, batched problems, kmgb_kmeanspp_*, ClosestCenters). Their workspaces come from
+// a pool of their own that keeps at most kCallPoolKeep between them: what it holds beyond goes back to
+// the device with the next synchronization after the call (KMGB_POOL=0: all of it). So a call neither
+// leaves a large workspace behind nor unmaps what handles have cached.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -23,7 +28,9 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
-cudaMemPool_t g_pools[kMaxDevices] = {};
+constexpr int kHandles = 0, kCalls = 1;
+constexpr uint64_t kCallPoolKeep = 8ull << 30;
+cudaMemPool_t g_pools[2][kMaxDevices] = {};
 
 bool keep_freed_memory() {
   static const bool keep = [] {
@@ -33,13 +40,13 @@ bool keep_freed_memory() {
   return keep;
 }
 
-cudaError_t pool_of_current_device(cudaMemPool_t* out) {
+cudaError_t pool_of_current_device(int kind, cudaMemPool_t* out) {
   int dev = 0;
   cudaError_t r = cudaGetDevice(&dev);
   if (r != cudaSuccess) return r;
   if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> g(g_mu);
-  if (!g_pools[dev]) {
+  if (!g_pools[kind][dev]) {
     cudaMemPoolProps props;
     std::memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -49,15 +56,15 @@ cudaError_t pool_of_current_device(cudaMemPool_t* out) {
     cudaMemPool_t p = nullptr;
     r = cudaMemPoolCreate(&p, &props);
     if (r != cudaSuccess) return r;
-    uint64_t threshold = UINT64_MAX;
+    uint64_t threshold = kind == kHandles ? UINT64_MAX : keep_freed_memory() ? kCallPoolKeep : 0;
     r = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &threshold);
     if (r != cudaSuccess) {
       cudaMemPoolDestroy(p);
       return r;
     }
-    g_pools[dev] = p;
+    g_pools[kind][dev] = p;
   }
-  *out = g_pools[dev];
+  *out = g_pools[kind][dev];
   return cudaSuccess;
 }
 
@@ -96,27 +103,29 @@ int num_sms() {
   return v;
 }
 
-cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s) {
+static cudaError_t alloc_from(int kind, void** p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
   if (inject_fault(kFaultAlloc)) return cudaErrorMemoryAllocation;
   if (bytes == 0) bytes = 1;
-  cudaMemPool_t pool = nullptr;
-  cudaError_t r = pool_of_current_device(&pool);
-  if (r != cudaSuccess) return r;
-  r = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  cudaMemPool_t pool[2] = {nullptr, nullptr};
+  for (int i = 0; i < 2; ++i) {
+    const cudaError_t r = pool_of_current_device(i, &pool[i]);
+    if (r != cudaSuccess) return r;
+  }
+  cudaError_t r = cudaMallocFromPoolAsync(p, bytes, pool[kind], s);
   if (r == cudaErrorMemoryAllocation) {
-    // memory the pool holds but nobody uses goes back to the device, then one more try
+    // memory the pools hold but nobody uses goes back to the device, then one more try
     cudaGetLastError();
     cudaDeviceSynchronize();
-    cudaMemPoolTrimTo(pool, 0);
-    r = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    for (cudaMemPool_t q : pool) cudaMemPoolTrimTo(q, 0);
+    r = cudaMallocFromPoolAsync(p, bytes, pool[kind], s);
   }
   if (r != cudaSuccess) *p = nullptr;
   return r;
 }
 
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s) {
-  const cudaError_t r = dev_alloc_async(p, bytes, s);
+  const cudaError_t r = alloc_from(kHandles, p, bytes, s);
   if (r != cudaSuccess) return r;
   // usable from every stream (copies on the legacy stream, a handle's copy stream) at once
   return cudaStreamSynchronize(s);
@@ -128,38 +137,42 @@ void dev_free(void* p, cudaStream_t s) {
   if (!keep_freed_memory()) {
     cudaStreamSynchronize(s);
     cudaMemPool_t pool = nullptr;
-    if (pool_of_current_device(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+    if (pool_of_current_device(kHandles, &pool) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
   }
 }
 
-void dev_trim(size_t keep) {
-  cudaMemPool_t pool = nullptr;
-  if (pool_of_current_device(&pool) == cudaSuccess) cudaMemPoolTrimTo(pool, keep);
+cudaError_t call_alloc(void** p, size_t bytes, cudaStream_t s) { return alloc_from(kCalls, p, bytes, s); }
+
+void call_free(void* p, cudaStream_t s) {
+  if (p) cudaFreeAsync(p, s);
 }
 
 size_t dev_available() {
   size_t mem_free = 0, mem_total = 0;
-  cudaMemPool_t pool = nullptr;
-  uint64_t held = 0, used = 0;
   if (cudaMemGetInfo(&mem_free, &mem_total) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  if (pool_of_current_device(&pool) == cudaSuccess &&
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
-    mem_free += held - used;
+  for (int kind = 0; kind < 2; ++kind) {
+    cudaMemPool_t pool = nullptr;
+    uint64_t held = 0, used = 0;
+    if (pool_of_current_device(kind, &pool) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && held > used)
+      mem_free += held - used;
+  }
   return mem_free;
 }
 
 cudaError_t dev_release_cached() {
   cudaError_t r = cudaDeviceSynchronize();
   std::lock_guard<std::mutex> g(g_mu);
-  for (int d = 0; d < kMaxDevices; ++d)
-    if (g_pools[d]) {
-      const cudaError_t t = cudaMemPoolTrimTo(g_pools[d], 0);
-      if (r == cudaSuccess) r = t;
-    }
+  for (auto& pools : g_pools)
+    for (cudaMemPool_t p : pools)
+      if (p) {
+        const cudaError_t t = cudaMemPoolTrimTo(p, 0);
+        if (r == cudaSuccess) r = t;
+      }
   return r;
 }
 
@@ -178,11 +191,16 @@ void kmgb_debug_withhold_stage(long long stage, unsigned long long wait_cycles) 
 }
 
 long long kmgb_debug_pool_used_bytes(void) {
-  cudaMemPool_t pool = nullptr;
-  if (kmgb::pool_of_current_device(&pool) != cudaSuccess) return -1;
-  uint64_t used = 0;
-  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) return -1;
-  return (long long)used;
+  long long sum = 0;
+  for (int kind = 0; kind < 2; ++kind) {
+    cudaMemPool_t pool = nullptr;
+    uint64_t used = 0;
+    if (kmgb::pool_of_current_device(kind, &pool) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+      return -1;
+    sum += (long long)used;
+  }
+  return sum;
 }
 
 int kmgb_release_cached_memory(void) {

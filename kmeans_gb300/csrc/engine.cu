@@ -89,6 +89,15 @@ cudaError_t dalloc(T** p, size_t count, cudaStream_t s) {
   return r;
 }
 
+// a call's buffer, for work on s
+template <typename T>
+cudaError_t call_dalloc(T** p, size_t count, cudaStream_t s) {
+  void* v = nullptr;
+  const cudaError_t r = call_alloc(&v, sizeof(T) * (count ? count : 1), s);
+  *p = static_cast<T*>(v);
+  return r;
+}
+
 bool is_device_ptr(const void* p) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -1605,18 +1614,20 @@ int set_centers(kmgb_handle* h, const float* C, bool on_device) {
   return 0;
 }
 
-// k-means++ work space (what is there already stays); without room for the row-skipping test's
-// arrays every draw reads every row.
+// k-means++ work space (what is there already stays), a handle's or (call) a call's; without room for
+// the row-skipping test's arrays every draw reads every row.
 template <typename T>
-cudaError_t alloc_kpp(KppWork<T>* w, long long n, int k, cudaStream_t s) {
-  cudaError_t r = w->d2 ? cudaSuccess : dalloc(&w->d2, (size_t)kmeanspp_d2_elems(n), s);
-  if (r == cudaSuccess && !w->blocksum) r = dalloc(&w->blocksum, (size_t)kmeanspp_blocks(n), s);
-  if (r == cudaSuccess && !w->scalars) r = dalloc(&w->scalars, kKppScalars, s);
+cudaError_t alloc_kpp(KppWork<T>* w, long long n, int k, cudaStream_t s, bool call = false) {
+  auto take = [&](auto** p, size_t count) {
+    return *p ? cudaSuccess : call ? call_dalloc(p, count, s) : dalloc(p, count, s);
+  };
+  cudaError_t r = take(&w->d2, (size_t)kmeanspp_d2_elems(n));
+  if (r == cudaSuccess) r = take(&w->blocksum, (size_t)kmeanspp_blocks(n));
+  if (r == cudaSuccess) r = take(&w->scalars, kKppScalars);
   if (r != cudaSuccess) return r;
-  if (!w->cc && (dalloc(&w->near, (size_t)n, s) != cudaSuccess ||
-                 dalloc(&w->cc, (size_t)k, s) != cudaSuccess)) {
+  if (take(&w->near, (size_t)n) != cudaSuccess || take(&w->cc, (size_t)k) != cudaSuccess) {
     cudaGetLastError();
-    dev_free(w->near, s);
+    call ? call_free(w->near, s) : dev_free(w->near, s);
     w->near = nullptr;
   }
   return cudaSuccess;
@@ -1828,16 +1839,16 @@ int kmeanspp_oneshot(const T* X, long long n, int d, int k, unsigned long long s
   if (x_dev) {
     fail(cudaStreamSynchronize(nullptr), "k-means++ (legacy stream)");
   } else {
-    fail(dalloc(&Xd, (size_t)n * ldx, s), "k-means++ (data)");
+    fail(call_dalloc(&Xd, (size_t)n * ldx, s), "k-means++ (data)");
     if (!rc)
       fail(cudaMemcpy2DAsync(Xd, sizeof(T) * ldx, X, sizeof(T) * d, sizeof(T) * d, n,
                              cudaMemcpyHostToDevice, s),
            "k-means++ (upload)");
   }
-  if (!rc) fail(dalloc(&Cd, (size_t)k * d, s), "k-means++ (centers)");
-  if (!rc) fail(alloc_kpp(&w, n, k, s), "k-means++ (work space)");
-  if (!rc) fail(dalloc(&kp, (size_t)k, s), "k-means++ (picks)");
-  if (!rc) fail(dalloc(&err, 1, s), "k-means++ (error word)");
+  if (!rc) fail(call_dalloc(&Cd, (size_t)k * d, s), "k-means++ (centers)");
+  if (!rc) fail(alloc_kpp(&w, n, k, s, true), "k-means++ (work space)");
+  if (!rc) fail(call_dalloc(&kp, (size_t)k, s), "k-means++ (picks)");
+  if (!rc) fail(call_dalloc(&err, 1, s), "k-means++ (error word)");
   if (!rc) fail(cudaMemsetAsync(err, 0, sizeof(int), s), "k-means++ (error word)");
   if (!rc)
     fail(launch_kmeanspp(x_dev ? X : Xd, ldx, n, d, k, seed, Cd, d, kp, w, err, s),
@@ -1859,7 +1870,7 @@ int kmeanspp_oneshot(const T* X, long long n, int d, int k, unsigned long long s
   }
   for (void* p : {(void*)Xd, (void*)Cd, (void*)w.d2, (void*)w.blocksum, (void*)w.scalars,
                   (void*)w.near, (void*)w.cc, (void*)kp, (void*)err})
-    dev_free(p, s);
+    call_free(p, s);
   cudaStreamSynchronize(s);
   cudaStreamDestroy(s);
   return rc;

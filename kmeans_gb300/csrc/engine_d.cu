@@ -183,12 +183,12 @@ struct DevBufs {
   std::vector<void*> ptrs;
   ~DevBufs() {
     cudaStreamSynchronize(0);
-    for (void* p : ptrs) dev_free(p, 0);
+    for (void* p : ptrs) call_free(p, 0);
   }
   template <typename T>
   cudaError_t alloc(T** p, size_t count) {
     void* v = nullptr;
-    const cudaError_t e = dev_alloc_async(&v, sizeof(T) * (count ? count : 1), 0);
+    const cudaError_t e = call_alloc(&v, sizeof(T) * (count ? count : 1), 0);
     *p = static_cast<T*>(v);
     if (e == cudaSuccess) ptrs.push_back(v);
     return e;
@@ -199,7 +199,7 @@ struct DevBufs {
     const size_t had = ptrs.size();
     if (take()) return true;
     cudaGetLastError();
-    for (; ptrs.size() > had; ptrs.pop_back()) dev_free(ptrs.back(), 0);
+    for (; ptrs.size() > had; ptrs.pop_back()) call_free(ptrs.back(), 0);
     return false;
   }
 };

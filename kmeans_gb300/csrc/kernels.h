@@ -496,14 +496,13 @@ bool inject_fault(int kind);
 // and bound every wait by *wait_cycles SM cycles (0: the default limit).
 void test_wait_hook(long long* withhold, unsigned long long* wait_cycles);
 
-// Device memory from the library's stream-ordered pool of the current device (devmem.cu):
+// Device memory from the library's stream-ordered pools of the current device (devmem.cu), for handles:
 // dev_alloc returns memory usable from every stream; dev_free gives it back in the order of s.
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t s);
-// The same without waiting for s: memory for work queued on s after the call.
-cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t s);
 void dev_free(void* p, cudaStream_t s);
-// Unused memory beyond `keep` bytes goes back to the device.
-void dev_trim(size_t keep);
+// For a call's workspace, in the order of s and without waiting for it: memory for work queued on s.
+cudaError_t call_alloc(void** p, size_t bytes, cudaStream_t s);
+void call_free(void* p, cudaStream_t s);
 // Bytes that could be allocated now: the device's free memory and the pool's unused.
 size_t dev_available();
 cudaError_t dev_release_cached();

@@ -3,7 +3,7 @@
 // default stream like the reference; the reference's scratch arguments (Bpadded, C, Cindices,
 // normRowsOfA_squared in ClosestCenters) are accepted and not needed. Temporary buffers are
 // stream-ordered on the default stream: cudaMallocAsync, and for ClosestCenters one allocation from
-// the library's pool (devmem.cu), bounded by working through the rows in chunks.
+// the library's pool for calls (devmem.cu).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -462,7 +462,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
   Carver size;
   carve(size);
   void* mem = nullptr;
-  cudaError_t e = dev_alloc_async(&mem, size.off, kDefault);
+  cudaError_t e = call_alloc(&mem, size.off, kDefault);
   if (e == cudaErrorMemoryAllocation && tc) {
     // no room for the planes and candidates: the scans without them (FP64: without any memory)
     cudaGetLastError();
@@ -471,7 +471,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
     copy = !direct;
     size = Carver{};
     carve(size);
-    e = dev_alloc_async(&mem, size.off, kDefault);
+    e = call_alloc(&mem, size.off, kDefault);
   }
   if (e) return e;
   Carver cut;
@@ -600,7 +600,7 @@ cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const
       e = cudaGetLastError();
     }
   }
-  dev_free(mem, kDefault);
+  call_free(mem, kDefault);
   return e;
 }
 

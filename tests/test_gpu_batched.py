@@ -209,3 +209,32 @@ def test_rows_still_being_written_on_the_default_stream(km, orc, torch_cuda, tie
                               assign_tier=tier)
     for (X, k, init), r in zip(probs, res):
         check(r, orc.lloyd(X, init, 4))
+
+
+def test_batched_call_leaves_handles_cached_memory(km, torch_cuda):
+    """What handles have cached for the next handle (here some 12 GB) is not unmapped by a batched
+    call, whose own workspace comes from another pool; k-means++ and ClosestCenters likewise."""
+    torch = torch_cuda
+    km.release_cached_memory()
+    probs = [(p[0], p[1], None) for p in make_batch(6, 77, dims=(16,), nmax=3000, kmax=20)]
+    X = torch.randn((4000, 16), device="cuda")
+    lab = torch.empty(4000, dtype=torch.int32, device="cuda")
+    c = X[:8].t().contiguous()
+
+    def calls():
+        km.lloyd_batched(probs, max_iters=2)
+        km.kmeanspp(X, 8, seed=1)
+        assert km.ClosestCentersF(0, 4000, 16, X, 8, c, None, None, (c * c).sum(0), 0, None, None, lab) == 0
+        torch.cuda.synchronize()
+
+    calls()
+    h = km.Handle(45_000_000, 32, 8, assign_tier=km.ASSIGN_FP32)
+    h.close()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    calls()
+    after = torch.cuda.mem_get_info()[0]
+    km.release_cached_memory()
+    freed = torch.cuda.mem_get_info()[0] - before
+    assert freed > 9e9  # the handle's memory was there to be lost
+    assert after <= before + (1 << 26)
