@@ -126,7 +126,10 @@ __global__ void prep_centers_kernel(const float* C, long long ldc, int k, int d,
       mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
   }
-  // the squared norm, and an upper bound of the norm
+  // the squared norm, and an upper bound of the norm. The lanes' lo parts may differ in their last bits
+  // (the butterfly adds them in another order on either side): one lane's serve all, since the lanes
+  // write parts of one number below
+  lo = __shfl_sync(0xffffffffu, lo, 0);
   float nn = __fadd_rn(hi, lo);
   float nrm = __fsqrt_ru(__fmul_ru(__fadd_ru(hi, fabsf(lo)), 1.0f + 0x1p-22f));
   if (!bad && !(hi < 1.0e37f && hi >= 1.0e-24f)) {  // squares out of FP32's normal range (uniform)

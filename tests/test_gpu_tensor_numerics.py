@@ -91,3 +91,34 @@ def test_fp8_keys_within_model_and_certificate_bound(km, torch_cuda):
         worst = np.max(np.abs(keys - exact) / eb)
         print(f"{name} fp8: key error {worst:.3f} of the certificate bound")
         assert worst <= 1.0
+
+
+# Centers whose squared norm lies halfway between two FP32 numbers, one of them halfway between two BF16
+# numbers: the lanes of a warp that adds it up may round it either way, and the start value -|c|^2/2, which
+# three of them write as three BF16 numbers, must still be one number's.
+MIDWAY = [
+    ["-0x1.2c2d9ap-1", "-0x1.168d3cp-3", "0x1.f627fp-1", "-0x1.a0c12cp-3", "0x1.0c6bc2p-1", "0x1.dcd99cp-1"],
+    ["-0x1.38ec4p-2", "-0x1.2ffabap-3", "-0x1.80610ap-2", "-0x1.ba09b4p-1", "0x1.5acf58p-1", "0x1.3b189cp-1",
+     "0x1.de053cp-1"],
+    ["-0x1.245e2p-1", "0x1.8522bep-1", "-0x1.444acp-1", "-0x1.312248p-1", "-0x1.a0ffe4p-1", "0x1.b2c18ep-3",
+     "0x1.cd657cp-2", "0x1.16d4bep+0"],
+    ["0x1.28d73ap-1", "-0x1.ba7958p-1", "-0x1.bb6c82p-1", "0x1.283d3cp-1", "0x1.bffd74p-2", "-0x1.9e533p-1",
+     "0x1.95ca86p-1", "0x1.1315b4p+0"],
+]
+
+
+@pytest.mark.parametrize("tier", ["BF16X3", "BF16", "FP32"])
+@pytest.mark.parametrize("center", MIDWAY)
+def test_norms_halfway_between_fp32_numbers(km, torch_cuda, tier, center):
+    import oracle
+    a = np.array([float.fromhex(v) for v in center], np.float32)
+    d = a.size
+    init = np.stack([a, a, a])
+    init[1, 0] += 0.0625  # |a - b|^2 / 2 = 0.002, a quarter of a BF16 step of the start value
+    init[2] += 3.0
+    rng = np.random.default_rng(d)
+    X = init[rng.integers(0, 2, 600)] + rng.uniform(-1e-3, 1e-3, (600, d)).astype(np.float32)
+    X[:2] = init[:2]
+    got = km.lloyd(X, 3, init=init, max_iters=1, assign_tier=getattr(km, "ASSIGN_" + tier), empty_policy=1)
+    want = oracle.lloyd(X, init, 1, empty_policy=1)
+    assert np.array_equal(got.labels, want[2]) and np.array_equal(got.centers, want[1])
