@@ -45,6 +45,14 @@ __device__ __forceinline__ void ff_square_add(float v, float& hi, float& lo) {
   lo = __fadd_rn(lo, __fadd_rn(err, e));
 }
 
+// Whether float-float (hi, lo), a sum of d squares, lies within its error bound of the middle between two
+// FP32 numbers. The bound: (d + 256) 2^-51 of the sum (d / 32 + 8 additions a lane and its tree, each
+// 2^-46), taken twice. There the FP64 sum decides, so that every rounded norm is that of the FP64 sum.
+__device__ __forceinline__ bool nearly_midway(float hi, float lo, int d) {
+  const float e = __fmul_rn(hi, (float)(d + 256) * 0x1p-50f);
+  return __fadd_rn(hi, __fadd_rn(lo, e)) != __fadd_rn(hi, __fsub_rn(lo, e));
+}
+
 // One warp per center, one pass over its old operand copy and its new values, four dimensions a lane in
 // flight. The norm is an error-free float-float sum on the FP32 pipe as a row's (prep_rows_kernel): an
 // FP64 chain per lane, its tree and two FP64 square roots in passes of their own took 36.5 us for
@@ -132,7 +140,8 @@ __global__ void prep_centers_kernel(const float* C, long long ldc, int k, int d,
   lo = __shfl_sync(0xffffffffu, lo, 0);
   float nn = __fadd_rn(hi, lo);
   float nrm = __fsqrt_ru(__fmul_ru(__fadd_ru(hi, fabsf(lo)), 1.0f + 0x1p-22f));
-  if (!bad && !(hi < 1.0e37f && hi >= 1.0e-24f)) {  // squares out of FP32's normal range (uniform)
+  // squares out of FP32's normal range, or a norm halfway between two FP32 numbers (uniform)
+  if (!bad && (!(hi < 1.0e37f && hi >= 1.0e-24f) || nearly_midway(hi, lo, d))) {
     double s = 0.0;
     for (int t = lane; t < d; t += 32) s = fma((double)c[t], (double)c[t], s);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -316,8 +325,8 @@ prep_rows_kernel(const T* X, long long ldx, long long n, int d, bool vec,
       l1 = __fadd_rn(l1, __fadd_rn(ol, err));
     }
     // overflow (or NaN input): FP64 sum; for the rounded norm also where squares near the
-    // subnormals lose their low parts
-    const bool wide = !(fabsf(h1) < 1.0e37f) || (nf && h1 < 1.0e-24f);
+    // subnormals lose their low parts, and where its rounding could differ from the FP64 sum's
+    const bool wide = !(fabsf(h1) < 1.0e37f) || (nf && (h1 < 1.0e-24f || nearly_midway(h1, l1, d)));
     if (__any_sync(0xffffffffu, wide)) {
 #pragma unroll 1
       for (int u = 0; u < U; ++u) {

@@ -124,3 +124,33 @@ def test_closest_centers_beyond_fp32_range(km, torch_cuda, n, d, k, sign):
     nb = (B.astype(np.float64) ** 2).sum(0).astype(np.float32)
     assert np.isfinite(nb).all()
     assert np.array_equal(closest(km, torch_cuda, A, B, nb), exact_labels(A, B, nb))
+
+
+# Rows whose squared norm lies within 2^-46 of the middle between two FP32 numbers.
+NEARLY_MIDWAY = [
+    "0x1.bd8ff8p-4 0x1.ba67f4p-1 -0x1.b7f980p-4 -0x1.888288p-2 0x1.6cec4cp-10 0x1.2c0592p-1 0x1.b69d1ap-3 0x1.ad9c86p-1",
+    "-0x1.3c572ap-1 0x1.5c5984p-1 0x1.578ce2p-5 0x1.e65b9cp-3 -0x1.3e26a4p-3 0x1.7a3870p-1 0x1.f23a48p-2 0x1.2ecfd0p-1",
+    "0x1.96e9a4p-1 -0x1.2a8184p-1 -0x1.c481b8p-1 0x1.743e32p-3 0x1.ba0478p-4 0x1.670c88p-2 0x1.6dc126p-2 0x1.e6b306p-1",
+    "0x1.b85822p-1 -0x1.fa089ap-1 -0x1.099144p-3 -0x1.6c51ecp-1 0x1.c4a526p-1 0x1.ede244p-3 0x1.1f59cap-2 0x1.0ccc0ep+0",
+    "0x1.2d6fdap-1 -0x1.8dcd54p-1 -0x1.c2f75ap-2 -0x1.428910p-1 -0x1.8a8634p-1 -0x1.055c46p-2 0x1.567434p-2 0x1.7f29aap-1",
+    "-0x1.6c7afcp-1 0x1.00789ap-4 0x1.2265c2p-1 -0x1.c585fcp-1 0x1.1db252p-4 -0x1.abedd8p-1 0x1.e670f6p-2 0x1.3eff7cp-1",
+]
+
+
+def test_row_norms_are_the_fp64_sums_rounded(km, torch_cuda):
+    from fractions import Fraction
+    rows = np.array([[float.fromhex(v) for v in r.split()] for r in NEARLY_MIDWAY], np.float32)
+    want = []
+    for r in rows:
+        s = sum(Fraction(float(v)) ** 2 for v in r)
+        near = np.float32(float(s))
+        want.append(min((near, np.nextafter(near, np.float32(0)), np.nextafter(near, np.float32(9))),
+                        key=lambda c: abs(Fraction(float(c)) - s)))
+    X = np.tile(rows, (50, 1))  # whole warps of them, and beside ordinary rows
+    X[7::11] = np.random.default_rng(1).standard_normal(X[7::11].shape)
+    out = torch_cuda.zeros(len(X), device="cuda")
+    assert km.rowNormalizeF(0, len(X), 8, torch_cuda.from_numpy(X).cuda(), out) == 0
+    got = out.cpu().numpy()
+    for i, w in enumerate(np.tile(np.array(want, np.float32), 50)):
+        if i % 11 != 7:
+            assert got[i] == w, i
