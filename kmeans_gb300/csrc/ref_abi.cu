@@ -135,11 +135,13 @@ __device__ __forceinline__ double block_sum(double acc) {
 // the centers come from L1/L2), with FP32 data also by GB300's narrow FP64 pipe as long as every
 // element is widened (898,790 x 128: 1.21 ms): there the terms run on the FP32 pipe as error-free
 // float-float values -- u = x - c exactly (TwoSum), u^2 = p + e (FMA), TwoSum accumulation -- and a
-// lane widens one pair per segment of kSegSteps rows. A segment whose sum leaves the range in which
-// that keeps 48 bits (overflow, squares near the subnormals, NaN) is evaluated in FP64.
+// lane widens a pair at every kSegTerms terms: the low part is a plain sum, so its rounding errors, 2^-24
+// of it each, stay within 2^-35 of the pair (some 2^-44 as they fall), however wide the rows. A segment of
+// kSegSteps rows in which a pair leaves the range where that holds (overflow, squares near the subnormals,
+// NaN) is evaluated in FP64.
 // L lanes share a row, 16 bytes each at a time where rows are aligned; four rows and the next four's
 // labels are in flight without a branch per row (898,790 x 128: 155 -> 129 us, at some two thirds of the issue slots).
-constexpr int kSegSteps = 32;
+constexpr int kSegSteps = 32, kSegTerms = 128;
 
 template <int L>
 __global__ void __launch_bounds__(256)
@@ -153,6 +155,15 @@ compactness_ff_kernel(long long m, int n, const float* data, const int* idx,
   double acc = 0.0;
   for (long long s0 = w0 * G * kSegSteps; s0 < m; s0 += nw * G * kSegSteps) {
     float hi = 0.0f, lo = 0.0f, mx = 0.0f;
+    double seg = 0.0;
+    bool off = false;
+    int terms = 0;
+    auto widen = [&] {
+      off |= !(hi < 1e37f && (hi > 1e-24f || mx == 0.0f));
+      seg += (double)hi + (double)lo;
+      hi = lo = mx = 0.0f;
+      terms = 0;
+    };
     auto term = [&](float x, float c) {
       float uh, ul, t, err;
       ff_two_sum(x, -c, uh, ul);
@@ -196,6 +207,7 @@ compactness_ff_kernel(long long m, int n, const float* data, const int* idx,
             term(xv[u].z, cv[u].z);
             term(xv[u].w, cv[u].w);
           }
+          if (L == 32 && (terms += 4 * U) >= kSegTerms) widen();  // (fewer lanes: at most kSegTerms a segment)
         }
       } else {
 #pragma unroll
@@ -203,13 +215,22 @@ compactness_ff_kernel(long long m, int n, const float* data, const int* idx,
           if (id[u] < 0) continue;
           const float* x = data + (size_t)(s0 + (i + u) * G + grp) * n;
           const float* c = centers + (size_t)id[u] * n;
-          for (int t = sub; t < n; t += L) term(ld(x + t), ld(c + t));
+          for (int t = sub; t < n; t += L) {
+            term(ld(x + t), ld(c + t));
+            if (L == 32 && ++terms >= kSegTerms) widen();
+          }
         }
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) id[u] = nx[u];
     }
-    if (hi < 1e37f && (hi > 1e-24f || mx == 0.0f)) {
+    if (L == 32) {
+      if (terms > 0) widen();
+      if (!off) {
+        acc += seg;
+        continue;
+      }
+    } else if (hi < 1e37f && (hi > 1e-24f || mx == 0.0f)) {
       acc += (double)hi + (double)lo;
       continue;
     }

@@ -154,3 +154,21 @@ def test_row_norms_are_the_fp64_sums_rounded(km, torch_cuda):
     for i, w in enumerate(np.tile(np.array(want, np.float32), 50)):
         if i % 11 != 7:
             assert got[i] == w, i
+
+
+@pytest.mark.parametrize("n", [8192, 1000, 8190])  # 16 bytes a lane, and one element a lane
+@pytest.mark.parametrize("big,small", [(4096.0, 0.9), (4096.0, 0.47), (1000.0, 0.1)])
+def test_compactness_of_wide_rows(km, torch_cuda, n, big, small):
+    """The running FP64 sum (the value behind out[0]) of rows whose squares all round the same way below
+    one large square: within the 2^-35 of a lane's 128 terms, however wide the rows."""
+    torch = torch_cuda
+    X = np.full((64, n), small, np.float32)
+    X[::32, :128] = big
+    out = torch.zeros(6, device="cuda")
+    lab = torch.zeros(64, dtype=torch.int32, device="cuda")
+    c = torch.zeros((1, n), device="cuda")
+    assert km.CompactnessF(0, 64, True, n, 1, torch.from_numpy(X).cuda(), lab, c, out) == 0
+    acc = float(out.cpu().numpy()[2:4].copy().view(np.float64)[0])
+    x = X.astype(np.float64)
+    want = float(np.sum(np.sort((x * x).ravel())))
+    assert abs(acc - want) <= 2.0 ** -35 * want
