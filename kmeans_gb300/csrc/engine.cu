@@ -632,7 +632,6 @@ int create_handle(kmgb_handle** out, long long n, int d, int k, const kmgb_optio
     a.take(&h->iters_done, 1);
     a.take(&h->xinexact, 1);
     a.take(&w.hist, hist_elems);
-    a.take(&w.scan_tmp, update_scan_tmp_elems(std::max<long long>(hist_elems, k + 1)));
     a.take(&w.label_off, k + 1);
     a.take(&w.piece_cnt, k + 1);
     a.take(&w.sorted, na);

@@ -337,7 +337,6 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   w.max_pieces = m_mb / kSumPiece + k + 1;
   const long long hist_elems = (long long)k * w.ntiles;
   KD_TRY(B.alloc(&w.hist, hist_elems), E);
-  KD_TRY(B.alloc(&w.scan_tmp, update_scan_tmp_elems(std::max<long long>(hist_elems, k + 1))), E);
   KD_TRY(B.alloc(&w.label_off, k + 1), E);
   KD_TRY(B.alloc(&w.piece_cnt, k + 1), E);
   KD_TRY(B.alloc(&w.sorted, m_mb), E);

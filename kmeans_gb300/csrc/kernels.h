@@ -157,7 +157,7 @@ struct RerankArgs {
 cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t s);
 // Whether the tiled stages below take this dimension (their tiles stay in shared memory).
 bool rerank_tiled_supported(int d);
-// FP32 stage of the re-rank, both modes: certifies what FP32 can, passes the rest to list2.
+// FP32 stage of the re-rank, mode 0: certifies what FP32 can, passes the rest to list2.
 // hi2[slot] receives the FP32 upper end of the best center of every point passed on.
 cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, float* hi2,
                                 cudaStream_t s);
@@ -363,7 +363,7 @@ struct UpdateWork {
   long long max_pieces;
   // buffers (device)
   int* hist;            // [k * ntiles]
-  int* scan_tmp;        // [scan_blocks]
+  int* scan_tmp;        // [update_scan_tmp_elems], launch_update_batched only
   int* label_off;       // [k + 1]
   int* piece_cnt;       // [k + 1] -> exclusive scan = piece start
   int* sorted;          // [n]

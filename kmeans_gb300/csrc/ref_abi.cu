@@ -643,7 +643,6 @@ kmeansCudaErrorStatus cluster_centers(int m0, int m, int n, int k, bool lastTile
   cudaError_t e = cudaSuccess;
   if (m > 0) {
     e = tmp_alloc(&w.hist, hist_elems);
-    if (!e) e = tmp_alloc(&w.scan_tmp, update_scan_tmp_elems(hist_elems > k + 1 ? hist_elems : k + 1));
     if (!e) e = tmp_alloc(&w.label_off, k + 1);
     if (!e) e = tmp_alloc(&w.piece_cnt, k + 1);
     if (!e) e = tmp_alloc(&w.sorted, m);
@@ -654,7 +653,6 @@ kmeansCudaErrorStatus cluster_centers(int m0, int m, int n, int k, bool lastTile
   }
   if (!e && lastTile) e = launch_finalize_acc<T>(acc, counts_large, k, n, centers, counts, kDefault);
   tmp_free(w.hist);
-  tmp_free(w.scan_tmp);
   tmp_free(w.label_off);
   tmp_free(w.piece_cnt);
   tmp_free(w.sorted);

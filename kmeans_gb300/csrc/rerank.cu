@@ -485,7 +485,7 @@ rerank_tiled_kernel(RerankArgs a, int* __restrict__ list2, int* __restrict__ cou
 // holds its whole warp on the narrow FP64 pipe), the band's centers become the candidates of
 // resolve_candidates_kernel, whose float-float tier settles nearly all of them: 796,160 x 324,
 // K=256, FP32 tier, 1.05 ms per iteration before. Slots from cand_cap on go to over / over_hi.
-template <int MODE, bool RECORD>
+template <bool RECORD>
 __global__ void __launch_bounds__(256)
 rerank_exact_kernel(RerankArgs a, const float* hi2, int* __restrict__ cand,
                     int* __restrict__ cand_cnt, long long cand_cap, int* __restrict__ over,
@@ -499,7 +499,6 @@ rerank_exact_kernel(RerankArgs a, const float* hi2, int* __restrict__ cand,
   float4* cs = xs + TP * rs;              // [TC][rs]
   float* cflag = reinterpret_cast<float*>(cs + TC * rs);  // [TC] value offset (tile_offset)
   __shared__ float hs[TP];
-  __shared__ float es[TP];  // MODE 1: the point's bound
   const int tid = threadIdx.x;
   long long cnt = min((long long)pinned(a.count), a.max_list);
   if (RECORD && cnt > cand_cap) {
@@ -526,12 +525,9 @@ rerank_exact_kernel(RerankArgs a, const float* hi2, int* __restrict__ cand,
       }
       xs[r * rs + q] = v;
     }
-    if (tid < TP) {
-      hs[tid] = (g0 + tid < cnt) ? hi2[g0 + tid] : -INFINITY;
-      es[tid] = MODE == 1 && g0 + tid < cnt ? expansion_bound(a, a.list[g0 + tid]) : 0.0f;
-    }
+    if (tid < TP) hs[tid] = (g0 + tid < cnt) ? hi2[g0 + tid] : -INFINITY;
     __syncthreads();
-    exact_pass<MODE, RECORD>(a, xs, cs, cflag, rs, dq, g0, cnt, hs, es, cand, cand_cnt);
+    exact_pass<0, RECORD>(a, xs, cs, cflag, rs, dq, g0, cnt, hs, nullptr, cand, cand_cnt);
   }
 }
 
@@ -1388,8 +1384,8 @@ cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStrea
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
-  if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
-  auto kern = a.mode == 0 ? rerank_exact_kernel<0, false> : rerank_exact_kernel<1, false>;
+  if (smem > (size_t)kMaxTileSmem || a.mode != 0) return cudaErrorInvalidValue;
+  auto kern = rerank_exact_kernel<false>;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, hi2, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
@@ -1405,9 +1401,9 @@ cudaError_t launch_rerank_band(const RerankArgs& a, const float* hi2, int* cand,
   const size_t smem = tiled_smem(a.d);
   if (smem > (size_t)kMaxTileSmem || a.mode != 0) return cudaErrorInvalidValue;
   if (smem > 48 * 1024)
-    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<0, true>,
+    KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
-  launch(rerank_exact_kernel<0, true>, kmgb::num_sms() * 2, 256, smem, s)(
+  launch(rerank_exact_kernel<true>, kmgb::num_sms() * 2, 256, smem, s)(
       a, hi2, cand, cand_cnt, cand_cap, over, over_count, over_hi);
   count_launches(1);
   return cudaGetLastError();
@@ -1418,8 +1414,8 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
-  if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
-  auto kern = a.mode == 0 ? rerank_tiled_kernel<0, false> : rerank_tiled_kernel<1, false>;
+  if (smem > (size_t)kMaxTileSmem || a.mode != 0) return cudaErrorInvalidValue;
+  auto kern = rerank_tiled_kernel<0, false>;
   if (smem > 48 * 1024)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, list2, count2, hi2);

@@ -112,9 +112,8 @@ __device__ void block_scan_inplace(int* data, long long n) {
 
 // Sums of the segments; the last block turns them into their exclusive scan.
 __global__ void scan_reduce_kernel(const int* in, long long n, int* __restrict__ sums,
-                                   int* ticket, const int* any_dirty, const int* stop) {
+                                   int* ticket) {
   if (grid_enter()) return;
-  if (skip(stop, any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int s = 0;
 #pragma unroll
@@ -133,10 +132,8 @@ __global__ void scan_reduce_kernel(const int* in, long long n, int* __restrict__
 }
 
 // In-place exclusive scan of segment blockIdx.x, plus offset (*offsets)[blockIdx.x] if given.
-__global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* offsets,
-                                const int* any_dirty, const int* stop) {
+__global__ void scan_seg_kernel(int* __restrict__ data, long long n, const int* offsets) {
   if (grid_enter()) return;
-  if (skip(stop, any_dirty)) return;
   const long long base = (long long)blockIdx.x * SCAN_SEG + (long long)threadIdx.x * SCAN_V;
   int vals[SCAN_V];
   int s = 0;
@@ -1296,16 +1293,15 @@ __global__ void sse_reduce_kernel(const double* sse_k, int k, double* __restrict
     store_sse(red[0], loop, out, stop, sse_prev, rel_out, iters_done, indexed);
 }
 
-cudaError_t excl_scan(int* data, long long n, int* tmp, int* ticket, cudaStream_t s,
-                      const int* any_dirty, const int* stop) {
+cudaError_t excl_scan(int* data, long long n, int* tmp, int* ticket, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const long long nb = (n + SCAN_SEG - 1) / SCAN_SEG;
   if (nb > SCAN_SEG) return cudaErrorInvalidValue;
   if (nb > 1) {
-    launch(scan_reduce_kernel, (unsigned)nb, SCAN_T, 0, s)(data, n, tmp, ticket, any_dirty, stop);
+    launch(scan_reduce_kernel, (unsigned)nb, SCAN_T, 0, s)(data, n, tmp, ticket);
     kmgb::count_launches(1);
   }
-  launch(scan_seg_kernel, (unsigned)nb, SCAN_T, 0, s)(data, n, nb > 1 ? tmp : nullptr, any_dirty, stop);
+  launch(scan_seg_kernel, (unsigned)nb, SCAN_T, 0, s)(data, n, nb > 1 ? tmp : nullptr);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
@@ -1829,12 +1825,12 @@ cudaError_t launch_update_batched(const float* X, long long ldx, int d, const do
     launch(hist_batched_kernel<false>, (unsigned)b.stiles, 256, 0, s)(labels, b, w.hist, w.err);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  KMGB_CUDA_TRY(excl_scan(w.hist, b.hist_elems, w.scan_tmp, w.tickets, s, nullptr, nullptr));
+  KMGB_CUDA_TRY(excl_scan(w.hist, b.hist_elems, w.scan_tmp, w.tickets, s));
   launch(label_offsets_batched_kernel, (b.K + 1 + 255) / 256, 256, 0, s)(w.hist, b, w.label_off,
                                                                     w.piece_cnt, w.counts, w.dirty);
   count_launches(1);
   KMGB_CUDA_TRY(cudaGetLastError());
-  KMGB_CUDA_TRY(excl_scan(w.piece_cnt, b.K + 1, w.scan_tmp, w.tickets, s, nullptr, nullptr));
+  KMGB_CUDA_TRY(excl_scan(w.piece_cnt, b.K + 1, w.scan_tmp, w.tickets, s));
   if (b.kmax <= kScatterMultiK)
     launch(scatter_batched_multi_kernel, (unsigned)b.stiles, 32 * kScatterWarps,
            sizeof(int) * (size_t)b.kmax * kScatterWarps, s)(labels, b, w.hist, w.sorted, w.dirty);
