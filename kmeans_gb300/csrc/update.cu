@@ -175,7 +175,7 @@ __device__ __forceinline__ int scan_label_row(int* row, int ntiles, int lane) {
 // the labels' totals. One launch and one pass over the counters where a scan over all of them took two
 // passes and two launches before the offsets' own (256 labels x 220 tiles: 18.8 -> 7.6 us in all).
 __global__ void __launch_bounds__(SCAN_T)
-label_rows_kernel(int* __restrict__ hist, long long n, int k, int ntiles, int* label_off, int* piece_cnt,
+label_rows_kernel(int* __restrict__ hist, int k, int ntiles, int* label_off, int* piece_cnt,
                   long long* __restrict__ counts, const int* dirty, int* ticket,
                   const int* any_dirty, const int* stop) {
   if (grid_enter()) return;
@@ -223,7 +223,7 @@ label_rows_kernel(int* __restrict__ hist, long long n, int k, int ntiles, int* l
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    label_off[k] = (int)n;
+    label_off[k] = carry;  // (n, but for labels out of range, whose rows are left out)
     piece_cnt[k] = pcarry;
   }
 }
@@ -300,8 +300,9 @@ __global__ void hist_kernel(const int* labels, long long n, int k, int tile_pts,
       }
       pre += v[u];
     }
+    __shared__ int carry_sh, all_sh;  // all_sh: the rows with a label (all but labels out of range)
+    if (t == SCAN_T - 1) all_sh = pre;
     __syncthreads();
-    __shared__ int carry_sh;
     int carry = 0;
     for (int j0 = 0; j0 < k; j0 += SCAN_T) {
       const int j = j0 + t;
@@ -309,7 +310,7 @@ __global__ void hist_kernel(const int* labels, long long n, int k, int tile_pts,
       int c = 0, a0 = 0;
       if (j < k) {
         a0 = pos_s[j * ntiles];
-        c = (j + 1 < k ? pos_s[(j + 1) * ntiles] : (int)n) - a0;
+        c = (j + 1 < k ? pos_s[(j + 1) * ntiles] : all_sh) - a0;
         label_off[j] = a0;
         if (counts) counts[j] = c;
       }
@@ -322,7 +323,7 @@ __global__ void hist_kernel(const int* labels, long long n, int k, int tile_pts,
       __syncthreads();
     }
     if (t == 0) {
-      label_off[k] = (int)n;
+      label_off[k] = all_sh;
       piece_cnt[k] = carry;
     }
   }
@@ -1361,7 +1362,7 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
   KMGB_CUDA_TRY(cudaGetLastError());
   if (!small) {
     launch(label_rows_kernel, (unsigned)((k + SCAN_T / 32 - 1) / (SCAN_T / 32)), SCAN_T, 0, s)(
-        w.hist, n, k, w.ntiles, w.label_off, w.piece_cnt, w.counts, w.dirty, w.tickets, w.any_dirty,
+        w.hist, k, w.ntiles, w.label_off, w.piece_cnt, w.counts, w.dirty, w.tickets, w.any_dirty,
         w.stop);
     kmgb::count_launches(1);
     KMGB_CUDA_TRY(cudaGetLastError());

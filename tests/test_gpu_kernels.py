@@ -221,3 +221,28 @@ def test_mat_mat_mult_rejects_negative_sizes(km, torch_cuda):
     out = torch_cuda.zeros(4, device="cuda")
     assert km.MatMatMultF(-1, 2, None, 2, None, out) == 1  # ERROR_MATMATMULT
     assert km.MatMatMultD(2, 2, None, -3, None, out) == 1
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k", [(3000, 8, 10), (3000, 40, 1), (200_000, 36, 300), (60_000, 5, 30_000)])
+def test_cluster_centers_leaves_out_rows_with_labels_out_of_range(km, torch_cuda, dtype, n, d, k):
+    """Such rows are in no center: the last center's members end where the valid labels do."""
+    torch = torch_cuda
+    rng = np.random.default_rng(n + k)
+    X = rng.integers(-50, 50, (n, d)).astype(dtype)
+    lab = rng.integers(0, k, n).astype(np.int32)
+    lab[::7], lab[1::13], lab[2::17] = -1, k, 2 ** 30
+    ok = (lab >= 0) & (lab < k)
+    want_n = np.bincount(lab[ok], minlength=k)
+    want = np.zeros((k, d))
+    np.add.at(want, lab[ok], X[ok].astype(np.float64))
+    x, l = torch.from_numpy(X).cuda(), torch.from_numpy(lab).cuda()
+    big = torch.zeros(k * d, dtype=torch.float64, device="cuda")
+    cnt_big, cnt = (torch.zeros(k, dtype=torch.int32, device="cuda") for _ in range(2))
+    cen = torch.zeros((k, d), dtype=x.dtype, device="cuda")
+    fn = km.ClusterCentersF if dtype == np.float32 else km.ClusterCentersD
+    assert fn(0, n, d, k, True, x, l, big, cnt_big, cen, cnt) == 0
+    assert np.array_equal(cnt.cpu().numpy(), want_n)
+    assert np.array_equal(big.cpu().numpy().reshape(k, d), want)
+    with np.errstate(all="ignore"):
+        assert np.array_equal(cen.cpu().numpy(), (want / want_n[:, None]).astype(dtype), equal_nan=True)
