@@ -294,11 +294,13 @@ __device__ __forceinline__ void halves(unsigned long long p, float& lo, float& h
 // assign_fp32_kernel over the centers' transpose (tmT: dimension by dimension, 128 centers x 32
 // dimensions per stage, unswizzled), so that a dimension's values of neighbouring centers are a register
 // pair: a thread's 4 points x 16 centers (4 tx .. 4 tx + 3 of each quarter of the chunk) take 32 packed
-// FMAs per dimension instead of 64, and 4 points' values have to be doubled into pairs for them. Every (point, center) sum is the same chain in the same order, so
-// the values are bit for bit assign_fp32_kernel's. That kernel issues 84% FMAs at 61% of the issue slots
-// (dispatch stalls of three-operand FMAs, one CTA of 255 registers a thread per SM) and takes 3.17 ms for
-// 796,160 x 324, K=256; this one takes 2.26 ms: 128 registers, so two CTAs hide each other's waits (one
-// CTA: 2.7 ms), and 4 points x 16 centers instead of 8 x 8, which doubles half as many values (2.8).
+// FMAs per dimension instead of 64, and 4 points' values have to be doubled into pairs for them. Every
+// (point, center) sum is the same chain in the same order, so the values are bit for bit
+// assign_fp32_kernel's. That kernel issues 84% FMAs at 61% of the issue slots (dispatch stalls of
+// three-operand FMAs, one CTA of 255 registers a thread per SM) and takes 3.17 ms for 796,160 x 324, K=256;
+// this one takes 2.26 ms: 128 registers (64 bytes a thread are spilled), so
+// two CTAs hide each other's waits (one CTA: 2.7 ms), and 4 points x 16 centers instead of 8 x 8, which
+// doubles half as many values (2.8).
 // assign_fp32_kernel stays for centers without a transposed copy (the per-kernel interface).
 __global__ void __launch_bounds__(NTHREADS, 2)
 assign_fp32t_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmT,

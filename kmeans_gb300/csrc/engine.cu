@@ -322,8 +322,8 @@ struct kmgb_handle {
     if (stream) {
       cudaStreamSynchronize(stream);
       // the fixed buffers live in the arena; these are allocated on their own
-      void* ptrs[] = {arena, sse_dev, kpp.d2, kpp.blocksum, kpp.scalars, kpp.near, kpp.cc, kpp_picks, fb_arena, shard_arena,
-                      prune_arena};
+      void* ptrs[] = {arena,  sse_dev,   kpp.d2,   kpp.blocksum, kpp.scalars, kpp.near,
+                      kpp.cc, kpp_picks, fb_arena, shard_arena,  prune_arena};
       for (void* p : ptrs) dev_free(p, stream);
       router_destroy(router, stream);
       cudaStreamSynchronize(stream);
@@ -1396,8 +1396,9 @@ int step_stream(kmgb_handle* h, int slot) {
 // Enqueues `iters` iterations as launches of one captured CUDA graph holding a whole iteration
 // (resident data): every iteration issues the same kernels with the same parameters -- the SSE slot and a
 // mini-batch window are indexed on the device, and the stop rule's criterion is a device word of the run
-// -- so the graph is captured once and replayed until a buffer it uses is replaced. Returns 0 when launched, -1 when the iteration cannot be
-// captured (it is then launched kernel by kernel), else an error code.
+// -- so the graph is captured once and replayed until a buffer it uses is replaced or a run's length turns
+// the distance bounds on or off. Returns 0 when launched, -1 when the iteration cannot be captured (it is
+// then launched kernel by kernel), else an error code.
 int run_graph(kmgb_handle* h, int iters) {
   if (!(h->gexec && h->g_sse == h->sse_dev)) {
     if (h->gexec) {

@@ -411,7 +411,8 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
   while (it < maxIters && rel > criterion) {
     const double* Xa = X;
     if (mini) {
-      launch(gather_d_kernel, kmgb::num_sms() * 8, 256, 0, s)(X, n, permd, m, start, m_mb, Xw); kmgb::count_launches(1);
+      launch(gather_d_kernel, kmgb::num_sms() * 8, 256, 0, s)(X, n, permd, m, start, m_mb, Xw);
+      kmgb::count_launches(1);
       Xa = Xw;
     }
     launch(transpose_d_kernel, kmgb::num_sms() * 4, 256, 0, s)(Cd, k, n, CT); kmgb::count_launches(1);

@@ -9,8 +9,9 @@
 // second threshold. While ub stays below the larger of the two, every other center is strictly
 // farther, so the label is still the FP64 arg-min and the row is not scanned; the other rows are
 // copied to a compact matrix and scanned as ever. A center none of whose rows changed keeps its
-// sums, its place and its SSE terms: the update is deterministic, so they would come out the same. The reference scans every row in every iteration
-// (kmeans.cpp:910-1014). Nothing survives a run: its first iteration scans every row.
+// sums, its place and its SSE terms: the update is deterministic, so they would come out the same. The
+// reference scans every row in every iteration (kmeans.cpp:910-1014). Nothing survives a run: its first
+// iteration scans every row.
 //
 // prune_filter_kernel is bound by HBM: 12 bytes read and 8 written per row.
 #include <cstdlib>
@@ -457,7 +458,8 @@ cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const in
                                cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   const long long blocks = (ps.n + 1023) / 1024, most = 2LL * kmgb::num_sms();
-  launch(prune_dirty_kernel, (unsigned)(blocks < most ? blocks : most), 1024, ps.k <= kDirtyShared ? ps.k : 0, s)(ps, labels, stop);
+  launch(prune_dirty_kernel, (unsigned)(blocks < most ? blocks : most), 1024,
+         ps.k <= kDirtyShared ? ps.k : 0, s)(ps, labels, stop);
   count_launches(1);
   return cudaGetLastError();
 }

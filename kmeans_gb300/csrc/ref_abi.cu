@@ -140,7 +140,8 @@ __device__ __forceinline__ double block_sum(double acc) {
 // kSegSteps rows in which a pair leaves the range where that holds (overflow, squares near the subnormals,
 // NaN) is evaluated in FP64.
 // L lanes share a row, 16 bytes each at a time where rows are aligned; four rows and the next four's
-// labels are in flight without a branch per row (898,790 x 128: 155 -> 129 us, at some two thirds of the issue slots).
+// labels are in flight without a branch per row (898,790 x 128: 155 -> 129 us, at some two thirds of the
+// issue slots).
 constexpr int kSegSteps = 32, kSegTerms = 128;
 
 template <int L>
@@ -426,8 +427,8 @@ struct Carver {
 // (and bound the workspace), whole waves of the pair kernel each. What the certificate leaves open
 // is settled from recorded candidates (float-float; FP64 data: FP64), the rest by the tiled stages
 // (FP64 data: a scan of the listed rows). The call returns before its kernels have run, so a scan whose
-// bounded wait gave up is not reported but made up for: the last kernel then takes every row. FP32 scan: 898,790 x 128, K=256 took 1.52 ms, its re-rank
-// 0.28 ms; FP64 scan: 100,000 x 64, K=256 took 2.80 ms.
+// bounded wait gave up is not reported but made up for: the last kernel then takes every row. FP32 scan:
+// 898,790 x 128, K=256 took 1.52 ms, its re-rank 0.28 ms; FP64 scan: 100,000 x 64, K=256 took 2.80 ms.
 template <typename T>
 cudaError_t closest_centers(int m0, long long n, int d, const T* A, int k, const T* B, const T* nb,
                             int* out) {
@@ -666,10 +667,10 @@ void launch_compactness(long long m, int n, const float* data, const int* idx, c
   const bool vec = n % 4 == 0 && !(reinterpret_cast<uintptr_t>(data) & 15) &&
                    !(reinterpret_cast<uintptr_t>(centers) & 15);
   const int per = vec ? (n + 3) / 4 : n;  // lanes' worth of a row
-  if (per <= 4) launch(compactness_ff_kernel<4>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
-  else if (per <= 8) launch(compactness_ff_kernel<8>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
-  else if (per <= 16) launch(compactness_ff_kernel<16>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
-  else launch(compactness_ff_kernel<32>, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
+  auto kern = per <= 4 ? compactness_ff_kernel<4>
+                       : (per <= 8 ? compactness_ff_kernel<8>
+                                   : (per <= 16 ? compactness_ff_kernel<16> : compactness_ff_kernel<32>));
+  launch(kern, blocks, 256, 0, kDefault)(m, n, data, idx, centers, vec, part);
   count_launches(1);
 }
 void launch_compactness(long long m, int n, const double* data, const int* idx, const double* centers,
@@ -693,7 +694,8 @@ kmeansCudaErrorStatus compactness(int m0, int m, bool lastTile, int n, int k, co
     e = cudaGetLastError();
   }
   if (!e) {
-    launch(compactness_final_kernel<T>, 1, 256, 0, kDefault)(part, blocks, acc, out, lastTile); kmgb::count_launches(1);
+    launch(compactness_final_kernel<T>, 1, 256, 0, kDefault)(part, blocks, acc, out, lastTile);
+    kmgb::count_launches(1);
     e = cudaGetLastError();
   }
   tmp_free(part);
@@ -821,20 +823,25 @@ kmeansCudaErrorStatus rowNormalizeD(const int m0, const int m, const int n, cons
                                     double* output) {
   if (m < 0 || n <= 0) return ERROR_ROWNORMALIZE;
   if (m == 0) return NO_ERROR;
-  launch(row_norm_kernel<double>, kmgb::num_sms() * 8, 256, 0, kDefault)(m0, m, n, input, output); kmgb::count_launches(1);
+  launch(row_norm_kernel<double>, kmgb::num_sms() * 8, 256, 0, kDefault)(m0, m, n, input, output);
+  kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_ROWNORMALIZE : NO_ERROR;
 }
 
 kmeansCudaErrorStatus colNormalizeF(const int m, const int n, const float* input, float* output) {
   if (m < 0 || n <= 0) return ERROR_COLNORMALIZE;
-  launch(col_norm_kernel<float>, (unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault)(m, n, input, output); kmgb::count_launches(1);
+  launch(col_norm_kernel<float>, (unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault)(m, n, input,
+                                                                                         output);
+  kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_COLNORMALIZE : NO_ERROR;
 }
 
 kmeansCudaErrorStatus colNormalizeD(const int m, const int n, const double* input,
                                     double* output) {
   if (m < 0 || n <= 0) return ERROR_COLNORMALIZE;
-  launch(col_norm_kernel<double>, (unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault)(m, n, input, output); kmgb::count_launches(1);
+  launch(col_norm_kernel<double>, (unsigned)(((long long)n + 31) / 32), 1024, 0, kDefault)(m, n, input,
+                                                                                          output);
+  kmgb::count_launches(1);
   return cudaGetLastError() ? ERROR_COLNORMALIZE : NO_ERROR;
 }
 

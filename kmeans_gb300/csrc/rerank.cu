@@ -536,8 +536,8 @@ rerank_exact_kernel(RerankArgs a, const float* hi2, int* __restrict__ cand,
 // center's dimensions, 16 bytes each at a time, 32 / L centers side by side and four in turn (a tree
 // sum per center -- like any order it stays within the (d+4) 2u relative bound of a sum of
 // non-negative terms); the values of up to RG_VCAP centers stay in shared memory. (A whole warp per
-// center left 16 of 32 lanes idle at D = 16 and took four centers a step.) Pass 2: every usable center whose FP32
-// lower end is within the smallest upper end is evaluated in FP64 in the oracle's order
+// center left 16 of 32 lanes idle at D = 16 and took four centers a step.) Pass 2: every usable center
+// whose FP32 lower end is within the smallest upper end is evaluated in FP64 in the oracle's order
 // (sequential fma over the dimensions), the smallest value winning, lowest index on ties.
 // Labels are global center indices.
 constexpr int RG_VCAP = 512;
@@ -1338,16 +1338,10 @@ cudaError_t launch_resolve_candidates(const int* list, const int* count, long lo
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
   const bool vec = d % 4 == 0 && ldx % 4 == 0 && ldc % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(X) % 16 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0;
-  if (vec)
-    launch(resolve_candidates_kernel<true>, kmgb::num_sms() * 8, 256, 0, s)(list, count, max_list, cand, cand_cnt,
-                                                            X, ldx, C, ldc, cn, d, labels, over,
-                                                            over_count, stop, row_map, hi_in, over_hi,
-                                                            resolve_tolerances(d));
-  else
-    launch(resolve_candidates_kernel<false>, kmgb::num_sms() * 8, 256, 0, s)(list, count, max_list, cand, cand_cnt,
-                                                             X, ldx, C, ldc, cn, d, labels, over,
-                                                             over_count, stop, row_map, hi_in, over_hi,
-                                                            resolve_tolerances(d));
+  auto kern = vec ? resolve_candidates_kernel<true> : resolve_candidates_kernel<false>;
+  launch(kern, kmgb::num_sms() * 8, 256, 0, s)(list, count, max_list, cand, cand_cnt, X, ldx, C, ldc, cn, d,
+                                               labels, over, over_count, stop, row_map, hi_in, over_hi,
+                                               resolve_tolerances(d));
   count_launches(1);
   return cudaGetLastError();
 }

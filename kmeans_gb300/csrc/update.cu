@@ -3,10 +3,11 @@
 // Replaces the reference's privatised accumulation (main/cuda/ClusterCenters.cu:3-23, one
 // G x K x D partial buffer), its per-center reduce and divide (ClusterCenters.cu:47-87), and the
 // compactness reduction (main/cuda/Compactness.cu:3-59). Instead of G*K*D partials:
-//   1. hist     per-tile label histogram (tile = `tile_pts` >= 4096 consecutive points),
-//               K x T int32, counted in shared memory (global atomics per peer group when K
-//               does not fit);
-//   2. scan     exclusive scan of the K-major histogram = start of every (label, tile) run;
+//   1. hist     per-tile label histogram (tile = `tile_pts` consecutive points: 4096 or more, down to
+//               512 on small data sets), K x T int32, counted in shared memory (global atomics per
+//               peer group when K does not fit);
+//   2. scan     exclusive scan of the K-major histogram = start of every (label, tile) run (few
+//               counters: by the histogram's last block);
 //   3. scatter  eight warps share a tile: each counts its slice, a scan across the warps gives
 //               each its first positions, and each walks its points in order writing every
 //               point id to start + rank (rank among equal labels of a 32-point step, from
@@ -15,11 +16,11 @@
 //               piece (a warp, or 32/L pieces per warp when D <= 64) sums its rows in point
 //               order (FP32 data: error-free float-float sum turned into FP64 once per piece;
 //               FP64 data: FP64) and the warp the rows' FP64 ||x||^2;
-//   5. finalize one warp per center adds its pieces in order, divides by the count in FP64,
+//   5. finalize one block per center adds its pieces in order, divides by the count in FP64,
 //               rounds once to FP32 (empty cluster: NaN as in ClusterCenters.cu:81, or keep the
 //               previous center), and evaluates the cluster's SSE against the new center with
-//               Q - 2 mu.S + n ||mu||^2 in FP64;
-//   6. sse      one block adds the K cluster SSEs in a fixed order.
+//               Q - 2 mu.S + n ||mu||^2 in FP64; the last block adds the K cluster SSEs in a fixed
+//               order (batched problems and host-streamed tiles: kernels of their own).
 // No floating-point atomics: the result is bit-identical run to run and equals the oracle's
 // canonical FP64 order.
 #include <algorithm>
@@ -459,8 +460,8 @@ __global__ void scatter_multi_kernel(const int* labels, long long n, int k,
 
 // Piece accumulator. FP32 data: an error-free float-float sum (Knuth's TwoSum on the FP32
 // pipe: hi + lo carries ~48 significant bits), turned into one FP64 value per piece; FP64 data:
-// a plain FP64 sum (piece_sums_d_kernel). GB300 issues FP64 (and FP32->FP64 conversions) at a small fraction of the
-// FP32 rate, so converting every element would bound the update.
+// a plain FP64 sum (piece_sums_d_kernel). GB300 issues FP64 (and FP32->FP64 conversions) at a small
+// fraction of the FP32 rate, so converting every element would bound the update.
 struct PieceAcc {
   float hi = 0.0f, lo = 0.0f;
   __device__ __forceinline__ void add(float x) {
@@ -901,8 +902,8 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
   // 25 warps an SM, 14.4 with the ring and 20.7 with this kernel)
   const long long few = max_pieces * ((d + 31) / 32);
   if (few <= kmgb::num_sms() * 8LL) {
-    launch(piece_sums_few_kernel, (unsigned)((few + 3) / 4), 128, 0, s)(X, ldx, qn, sorted, label_off, pstart, k,
-                                                                   d, part, partq, any, stop);
+    launch(piece_sums_few_kernel, (unsigned)((few + 3) / 4), 128, 0, s)(
+        X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, any, stop);
     kmgb::count_launches(1);
     return cudaGetLastError();
   }
@@ -919,7 +920,8 @@ cudaError_t launch_piece_sums_f32(const float* X, long long ldx, const double* q
     // four blocks (48 KB of ring each) per SM
     const long long cap = kmgb::num_sms() * 4LL * kRingWarps;
     const long long rw = max_pieces < cap ? max_pieces : cap;
-    launch(piece_sums_ring_kernel, (unsigned)((rw + kRingWarps - 1) / kRingWarps), kRingWarps * 32, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, any, stop);
+    launch(piece_sums_ring_kernel, (unsigned)((rw + kRingWarps - 1) / kRingWarps), kRingWarps * 32, 0, s)(
+        X, ldx, qn, sorted, label_off, pstart, k, d, part, partq, any, stop);
   } else
     launch(piece_sums_kernel, blocks, 256, 0, s)(X, ldx, qn, sorted, label_off, pstart, k, d,
                                                     part, partq, any, stop);
@@ -1380,11 +1382,13 @@ static cudaError_t sort_by_label(const int* labels, const UpdateWork& w, cudaStr
     if (smem > 48 * 1024)
       KMGB_CUDA_TRY(cudaFuncSetAttribute(scatter_kernel<true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    launch(scatter_kernel<true>, w.ntiles, kScatterLoad, smem, s)(labels, n, k, w.tile_pts, w.ntiles, w.hist, start,
-                                                    w.sorted, w.dirty, w.any_dirty, w.stop); kmgb::count_launches(1);
+    launch(scatter_kernel<true>, w.ntiles, kScatterLoad, smem, s)(
+        labels, n, k, w.tile_pts, w.ntiles, w.hist, start, w.sorted, w.dirty, w.any_dirty, w.stop);
+    kmgb::count_launches(1);
   } else {
-    launch(scatter_kernel<false>, w.ntiles, 32, 0, s)(labels, n, k, w.tile_pts, w.ntiles, w.hist, start,
-                                                  w.sorted, w.dirty, w.any_dirty, w.stop); kmgb::count_launches(1);
+    launch(scatter_kernel<false>, w.ntiles, 32, 0, s)(
+        labels, n, k, w.tile_pts, w.ntiles, w.hist, start, w.sorted, w.dirty, w.any_dirty, w.stop);
+    kmgb::count_launches(1);
   }
   return cudaGetLastError();
 }
@@ -1401,7 +1405,8 @@ cudaError_t launch_update(const float* X, const double* qn, const int* labels, f
   const int warps = std::min(8, (w.d + 31) / 32);
   if (w.centers_free) KMGB_CUDA_TRY(cudaStreamWaitEvent(s, w.centers_free, 0));
   const int most = kmgb::num_sms() * (64 / warps);  // blocks the SMs hold at a time
-  launch(finalize_update_kernel, (unsigned)std::min(k, most), 32 * warps, 0, s)(X, C, ldc, empty_policy, w, sse_out);
+  launch(finalize_update_kernel, (unsigned)std::min(k, most), 32 * warps, 0, s)(X, C, ldc, empty_policy, w,
+                                                                                sse_out);
   kmgb::count_launches(1);
   return cudaGetLastError();
 }
