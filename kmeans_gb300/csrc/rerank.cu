@@ -147,6 +147,9 @@ __global__ void rerank_kernel(RerankArgs a) {
 // The dynamic shared memory that launches here may ask for. Always this limit is set, not a launch's
 // own size: another thread's smaller one could arrive between the call and the launch.
 constexpr int kMaxTileSmem = 200 * 1024;
+// From here on a launch sets it: the 48 KB that need no setting are for dynamic and static shared memory
+// together, and the tiled kernels have up to 7 KB of static arrays.
+constexpr size_t kPlainSmem = 40 * 1024;
 constexpr int TP = 32;   // points per CTA iteration
 constexpr int TC = 64;   // centers per block
 
@@ -1380,7 +1383,7 @@ cudaError_t launch_rerank_exact(const RerankArgs& a, const float* hi2, cudaStrea
   const size_t smem = tiled_smem(a.d);
   if (smem > (size_t)kMaxTileSmem || a.mode != 0) return cudaErrorInvalidValue;
   auto kern = rerank_exact_kernel<false>;
-  if (smem > 48 * 1024)
+  if (smem > kPlainSmem)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, hi2, nullptr, nullptr, 0, nullptr, nullptr, nullptr);
   count_launches(1);
@@ -1394,7 +1397,7 @@ cudaError_t launch_rerank_band(const RerankArgs& a, const float* hi2, int* cand,
   if (a.n <= 0 || a.k <= 0) return cudaSuccess;
   const size_t smem = tiled_smem(a.d);
   if (smem > (size_t)kMaxTileSmem || a.mode != 0) return cudaErrorInvalidValue;
-  if (smem > 48 * 1024)
+  if (smem > kPlainSmem)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_exact_kernel<true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   launch(rerank_exact_kernel<true>, kmgb::num_sms() * 2, 256, smem, s)(
@@ -1410,7 +1413,7 @@ cudaError_t launch_rerank_tiled(const RerankArgs& a, int* list2, int* count2, fl
   const size_t smem = tiled_smem(a.d);
   if (smem > (size_t)kMaxTileSmem || a.mode != 0) return cudaErrorInvalidValue;
   auto kern = rerank_tiled_kernel<0, false>;
-  if (smem > 48 * 1024)
+  if (smem > kPlainSmem)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, list2, count2, hi2);
   count_launches(1);
@@ -1423,7 +1426,7 @@ cudaError_t launch_rerank_settle(const RerankArgs& a, cudaStream_t s) {
   const size_t smem = tiled_smem(a.d);
   if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
   auto kern = a.mode == 0 ? rerank_tiled_kernel<0, true> : rerank_tiled_kernel<1, true>;
-  if (smem > 48 * 1024)
+  if (smem > kPlainSmem)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   launch(kern, kmgb::num_sms() * 2, 256, smem, s)(a, nullptr, nullptr, nullptr);
   count_launches(1);
@@ -1440,7 +1443,7 @@ cudaError_t launch_rerank_grouped(const RerankArgs& a, const GroupArgs& g, cudaS
   auto kern = a.d <= 16 ? rerank_grouped_kernel<4>
                         : (a.d <= 32 ? rerank_grouped_kernel<8>
                                      : (a.d <= 64 ? rerank_grouped_kernel<16> : rerank_grouped_kernel<32>));
-  if (smem > 48 * 1024)
+  if (smem > kPlainSmem)
     KMGB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem));
   launch(kern, kmgb::num_sms() * 4, RG_WARPS * 32, smem, s)(a, g, cand, cand_cnt, cand_cap);
   count_launches(1);
@@ -1452,7 +1455,7 @@ cudaError_t launch_rerank(const RerankArgs& a, cudaStream_t s) {
   const int threads = 256;
   const size_t smem = sizeof(float) * (size_t)a.d * (threads / 32);
   if (smem > (size_t)kMaxTileSmem) return cudaErrorInvalidValue;
-  if (smem > 48 * 1024) {
+  if (smem > kPlainSmem) {
     KMGB_CUDA_TRY(cudaFuncSetAttribute(rerank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        kMaxTileSmem));
   }
