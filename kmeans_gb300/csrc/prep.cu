@@ -259,8 +259,8 @@ prep_rows_kernel(const T* X, long long ldx, long long n, int d, bool vec,
       rl.over[atomicAdd(rl.over_count, 1)] = rl.list[i];
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
-      const float fl = rl.thr[rl.list[i]];  // without a finite floor: no candidates
-      rl.thr_out[i] = fl > -3.0e38f ? fl : INFINITY;
+      const float fl = rl.thr[rl.list[i]];  // without a finite floor: no candidates (gather_flagged_kernel)
+      rl.thr_out[i] = fl > -3.0e38f ? fl : __int_as_float(0x7fc00000);
     }
   }
   long long start = 0;

@@ -683,10 +683,10 @@ gather_flagged_kernel(const int* list, const int* count,
   for (long long slot = cap + t0; slot < total; slot += nt) over[atomicAdd(over_count, 1)] = list[slot];
   for (long long slot = nt - 1 - t0; slot < cnt; slot += nt) {  // (the grid's end, while its first warps copy)
     const long long pt = list[slot];
-    // without a finite floor (no usable center, an infinite bound) the keys say nothing: no
-    // candidates, hence the full rescan
+    // without a finite floor (no usable center, an infinite bound) the keys say nothing: no key
+    // reaches NaN (an infinite one would reach infinity), so no candidates, hence the full rescan
     const float fl = thr[pt];
-    thrC[slot] = fl > -3.0e38f ? fl : INFINITY;
+    thrC[slot] = fl > -3.0e38f ? fl : __int_as_float(0x7fc00000);
     if (xs) xsC[slot] = xs[pt];
   }
   copy_listed_rows(list, cnt, Xb, Xl, (int)row_vec, XbC, XlC, t0 >> 5, nt >> 5, threadIdx.x & 31);

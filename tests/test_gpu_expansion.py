@@ -172,3 +172,32 @@ def test_compactness_of_wide_rows(km, torch_cuda, n, big, small):
     x = X.astype(np.float64)
     want = float(np.sum(np.sort((x * x).ravel())))
     assert abs(acc - want) <= 2.0 ** -35 * want
+
+
+def spoiled_rows(rng, n, d, k):
+    """Rows with one element near FP32's largest number: every bound is infinite and every tensor-core
+    key infinite or NaN; a key that stays infinite is one of a multiple of 32."""
+    C = rng.uniform(-1000, 1000, (k, d)).astype(np.float32)
+    X = C[rng.integers(0, k, n)] + rng.standard_normal((n, d)).astype(np.float32)
+    rows = rng.choice(n, 60, replace=False)
+    X[rows, rng.integers(0, d, 60)] = rng.choice([3e38, -3e38, 1e38], 60)
+    return X, C, rows
+
+
+@pytest.mark.parametrize("n,d,k", [(20_000, 64, 256), (30_000, 161, 115), (300, 40, 70)])
+def test_closest_centers_of_rows_near_the_largest_number(km, torch_cuda, n, d, k):
+    X, C, _ = spoiled_rows(np.random.default_rng(n), n, d, k)
+    B = np.ascontiguousarray(C.T)
+    nb = (B.astype(np.float64) ** 2).sum(0).astype(np.float32)
+    assert np.array_equal(closest(km, torch_cuda, X, B, nb), exact_labels(X, B, nb))
+
+
+@pytest.mark.parametrize("tier", ["BF16X3", "BF16", "FP32"])
+@pytest.mark.parametrize("n,d,k", [(20_000, 64, 256), (70_000, 100, 115)])
+def test_lloyd_with_rows_near_the_largest_number(km, orc, torch_cuda, tier, n, d, k):
+    X, C, rows = spoiled_rows(np.random.default_rng(n), n, d, k)
+    for flip in (1, -1):  # the sign decides which centers' keys are +inf
+        Y = X * np.float32(flip)
+        want = orc.lloyd(Y, C, 1, empty_policy=1)
+        got = km.lloyd(Y, k, init=C, max_iters=1, assign_tier=getattr(km, "ASSIGN_" + tier), empty_policy=1)
+        assert np.array_equal(got.labels, want[2])
