@@ -309,8 +309,9 @@ __global__ void row_norm_kernel(int m0, int m, int n, const T* in, T* __restrict
   }
 }
 
-// 32 columns per block (coalesced rows), 32 threads of a column taking every 32nd row; their FP64
-// sums are added in order. (One thread per column walked the rows alone: 128 x 256 took 23 us.)
+// 32 columns per block (coalesced rows), up to 32 threads a column, 16 rows or more each (strided); their
+// FP64 chains are added in order. (One thread per column walked the rows alone: 128 x 256 took 23 us.
+// Fewer rows a thread would round every square on its own: up to 16 rows stay one chain.)
 template <typename T>
 __global__ void __launch_bounds__(1024)
 col_norm_kernel(int m, int n, const T* in, T* __restrict__ out) {
@@ -319,9 +320,10 @@ col_norm_kernel(int m, int n, const T* in, T* __restrict__ out) {
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long long j = (long long)blockIdx.x * 32 + tx;
   double s = 0.0;
-  if (j < n) {
-#pragma unroll 4
-    for (long long i = ty; i < m; i += 32) {
+  const int slices = min(32, (m + 15) / 16);
+  if (j < n && ty < slices) {
+#pragma unroll 8
+    for (long long i = ty; i < m; i += slices) {
       const double v = (double)ld(in + (size_t)i * n + j);
       s = fma(v, v, s);
     }
@@ -330,8 +332,7 @@ col_norm_kernel(int m, int n, const T* in, T* __restrict__ out) {
   __syncthreads();
   if (ty == 0 && j < n) {
     double t = 0.0;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) t += red[i][tx];
+    for (int i = 0; i < slices; ++i) t += red[i][tx];
     out[j] = (T)t;
   }
 }

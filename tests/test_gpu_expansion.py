@@ -201,3 +201,30 @@ def test_lloyd_with_rows_near_the_largest_number(km, orc, torch_cuda, tier, n, d
         want = orc.lloyd(Y, C, 1, empty_policy=1)
         got = km.lloyd(Y, k, init=C, max_iters=1, assign_tier=getattr(km, "ASSIGN_" + tier), empty_policy=1)
         assert np.array_equal(got.labels, want[2])
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 9, 16, 17, 40, 128, 700])
+def test_column_norms_no_further_off_than_one_chain(km, torch_cuda, m):
+    """colNormalizeD against exact sums: up to 16 rows the FP64 FMA chain over the rows itself, beyond
+    no larger an error (root mean square over the columns) than that chain's."""
+    from fractions import Fraction
+    n = 600
+    X = np.random.default_rng(m).standard_normal((m, n))
+    out = torch_cuda.zeros(n, dtype=torch_cuda.float64, device="cuda")
+    assert km.colNormalizeD(m, n, torch_cuda.from_numpy(X).cuda(), out) == 0
+    got = out.cpu().numpy()
+    chain, exact = np.empty(n), []
+    for j in range(n):
+        c, e = 0.0, Fraction(0)
+        for v in X[:, j]:
+            q = Fraction(float(v)) ** 2
+            c = float(q + Fraction(c))
+            e += q
+        chain[j] = c
+        exact.append(e)
+    if m <= 16:
+        assert np.array_equal(got, chain)
+    else:
+        def rms(v):
+            return np.sqrt(np.mean([float((Fraction(float(a)) - e) / e) ** 2 for a, e in zip(v, exact)]))
+        assert rms(got) <= rms(chain)
