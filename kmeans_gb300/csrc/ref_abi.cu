@@ -211,14 +211,28 @@ compactness_ff_kernel(long long m, int n, const float* data, const int* idx,
           if (L == 32 && (terms += 4 * U) >= kSegTerms) widen();  // (fewer lanes: at most kSegTerms a segment)
         }
       } else {
+        // a test per term keeps the loads apart (200,000 x 210: 116 -> 230 us), one per row still some
+        // (122): one per U rows where their terms fit, else per piece of a row
+        const int cnt = (n + L - 1) / L;
+        const bool fit = L < 32 || U * cnt <= kSegTerms;
+        if (L == 32 && fit) {
+          if (terms + U * cnt > kSegTerms) widen();
+          terms += U * cnt;
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           if (id[u] < 0) continue;
           const float* x = data + (size_t)(s0 + (i + u) * G + grp) * n;
           const float* c = centers + (size_t)id[u] * n;
-          for (int t = sub; t < n; t += L) {
-            term(ld(x + t), ld(c + t));
-            if (L == 32 && ++terms >= kSegTerms) widen();
+          if (fit) {
+            for (int t = sub; t < n; t += L) term(ld(x + t), ld(c + t));
+          } else {
+            for (int b0 = 0; b0 < n; b0 += kSegTerms * L) {
+              const int e = min(n, b0 + kSegTerms * L);
+              if (terms > 0) widen();
+              for (int t = b0 + sub; t < e; t += L) term(ld(x + t), ld(c + t));
+              terms = kSegTerms;
+            }
           }
         }
       }

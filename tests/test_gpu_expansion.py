@@ -174,6 +174,24 @@ def test_compactness_of_wide_rows(km, torch_cuda, n, big, small):
     assert abs(acc - want) <= 2.0 ** -35 * want
 
 
+@pytest.mark.parametrize("n", [129, 2047, 4095, 4097, 8193])  # around 32 lanes of 128 terms, unaligned rows
+@pytest.mark.parametrize("m", [1, 70])
+def test_compactness_of_unaligned_wide_rows(km, torch_cuda, n, m):
+    """The running FP64 sum where a row ends within, at and past the terms a lane adds up before it
+    widens them: within the 2^-35 of these terms."""
+    torch = torch_cuda
+    rng = np.random.default_rng(n)
+    X = rng.uniform(0.5, 900.0, (m, n)).astype(np.float32)
+    C = rng.uniform(0.5, 900.0, (3, n)).astype(np.float32)
+    lab = rng.integers(0, 3, m).astype(np.int32)
+    out = torch.zeros(6, device="cuda")
+    x, c, l = (torch.from_numpy(v).cuda() for v in (X, C, lab))
+    assert km.CompactnessF(0, m, True, n, 3, x, l, c, out) == 0
+    acc = float(out.cpu().numpy()[2:4].copy().view(np.float64)[0])
+    want = float(((X.astype(np.float64) - C.astype(np.float64)[lab]) ** 2).sum())
+    assert abs(acc - want) <= 2.0 ** -35 * want
+
+
 def spoiled_rows(rng, n, d, k):
     """Rows with one element near FP32's largest number: every bound is infinite and every tensor-core
     key infinite or NaN; a key that stays infinite is one of a multiple of 32."""
