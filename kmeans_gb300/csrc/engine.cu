@@ -368,10 +368,10 @@ constexpr long long kPruneMinWorkFp32 = 1LL << 30;
 constexpr long long kPruneMaxBytes = 8LL << 30;  // of the compact copy
 // What the bounds save comes after the first moves have died down, so it is the length of the run that
 // decides: time with them over time without, for 24 shapes from 30,000 x 256, K=900 to 4M x 128, K=1024 (32
-// to 7,800 rows a center, both tiers) in clusters that lie apart: 3 iterations 0.98 - 1.15, 4 iterations
-// 0.89 - 1.14, 5 iterations 0.78 - 1.09, 8 iterations 0.57 - 0.92; in overlapping and Zipf-sized ones 0.93 -
-// 1.16 whatever the length up to 8. Within each of them the rows a center made no difference (at K=16,384,
-// 8 iterations: 0.62 at 32, 0.57 at 40, 0.59 at 48, 0.61 at 61, 0.59 at 79); 32 keeps the scan of the
+// to 7,800 rows a center, both tiers) in clusters that lie apart: 3 iterations 1.00 - 1.09, 4 iterations
+// 0.91 - 1.07, 5 iterations 0.80 - 1.04, 8 iterations 0.59 - 0.90; in overlapping and Zipf-sized ones 0.94 -
+// 1.12 whatever the length up to 8. Within each of them the rows a center made no difference (at K=16,384,
+// 8 iterations: 0.64 at 32, 0.59 at 40, 0.59 at 48, 0.62 at 61, 0.60 at 79); 32 keeps the scan of the
 // centers, k / n of the rows', small.
 constexpr long long kPruneRows = 32;
 constexpr int kPruneIters = 4;  // of a run
@@ -397,6 +397,7 @@ void alloc_prune(kmgb_handle* h, bool one_shot) {
   // at about 0.65 of the rows the copy and the scan of the listed rows take as long as the scan of
   // all rows
   p.cap = (int)std::min(h->n * 13 / 20, kPruneMaxBytes / row);
+  p.wait = kPruneWait;
   if (p.cap < 256) return;
   auto carve = [&](Arena& a) {
     a.take(&p.ub, p.n);
@@ -1065,9 +1066,10 @@ int router_step(kmgb_handle* h, AssignArgs a) {
 int prune_rows(kmgb_handle* h, AssignArgs& a, const void* Xba, const void* Xla, bool tc) {
   cudaStream_t s = h->stream;
   PruneState& p = h->pr;
+  KM_TRY(launch_prune_top(p, h->stop, s), KMEANS_ERROR_CLOSEST_CENTERS);
   AssignArgs c = a;
   c.n = h->k;
-  c.n_dev = p.flags;  // no rows while there are no bounds to check
+  c.n_dev = p.flags + 6;  // none where the rows are not tested
   c.xnorm = p.cxn;
   c.labels = p.clab;
   c.rerank_list = h->crr_list;
@@ -1160,10 +1162,11 @@ int step(kmgb_handle* h, int slot, const float* upload = nullptr, bool assign_on
     if (prune) {  // this iteration scans every row and leaves valid bounds
       a.ub = h->pr.ub;
       a.lb = h->pr.lb;
-      KM_TRY(cudaMemsetAsync(h->pr.flags, 1, 8 * sizeof(int), s), KMEANS_ERROR_COPY_TILE);
-      KM_TRY(cudaMemsetAsync(h->pr.flags + 2, 0, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
-      KM_TRY(cudaMemsetAsync(h->pr.flags + 5, 0, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      // (the flags are zero) as prune_top_kernel leaves them for such an iteration
+      KM_TRY(cudaMemsetAsync(h->pr.flags, 1, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
       KM_TRY(cudaMemsetAsync(h->pr.flags + 1, 0x7f, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      KM_TRY(cudaMemsetAsync(h->pr.flags + 4, 1, sizeof(int), s), KMEANS_ERROR_COPY_TILE);
+      KM_TRY(cudaMemsetAsync(h->pr.flags + 7, kPruneFull, 1, s), KMEANS_ERROR_COPY_TILE);
       KM_TRY(cudaMemsetAsync(h->pr.dirty, 1, sizeof(int) * h->k, s), KMEANS_ERROR_COPY_TILE);
     }
     if (h->Xb) KM_TRY(cudaMemsetAsync(h->xinexact, 0, sizeof(int), s), KMEANS_ERROR_COPY_TILE);

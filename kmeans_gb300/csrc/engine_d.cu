@@ -443,9 +443,10 @@ kmeansErrorStatus run_d(const double* data, int m, int n, int k, double criterio
       a.pert = 0x1p-22f;
       AssignArgs af = a;
       if (pr.n > 0) {  // distance bounds (prune.cu)
+        KD_TRY(launch_prune_top(pr, nullptr, s), EA);
         AssignArgs c = a;
         c.n = k;
-        c.n_dev = pr.flags;
+        c.n_dev = pr.flags + 6;
         c.xnorm = pr.cxn;
         c.labels = pr.clab;
         c.rerank_list = crr_list;

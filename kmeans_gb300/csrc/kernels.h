@@ -262,16 +262,28 @@ struct PruneState {
   int* list = nullptr;     // [cap] rows to scan
   int* lab_old = nullptr;  // [n] labels of the last update
   int* dirty = nullptr;    // [k] nonzero: the center's members may differ from the last update's
-  int* flags = nullptr;    // [0] 0: no bounds yet, else >= k, [1] rows to scan, [2] scratch count,
-                           // [3] index of the center that moved most, [4] nonzero: some center is
-                           // dirty, [5] nonzero: no center moved
+  int* flags = nullptr;    // [0] 0: no bounds yet, [1] rows to scan, [2] scratch count, [3] index of the
+                           // center that moved most, [4] nonzero: some center is dirty, [5] nonzero: no
+                           // center moved, [6] centers to scan against themselves (k or 0), [7] state
+                           // (prune_top_kernel; kPruneFull: an iteration that scans every row untested)
+  int wait = 0;            // most iterations in a row to go untested after tests that failed (kPruneWait)
   float* top = nullptr;    // [2] the two largest moves
   void* Xc = nullptr;      // [cap][ldb] compact rows (BF16), and their residual plane
   void* Xlc = nullptr;
 };
 // False with KMGB_BOUNDS=0 in the environment: every row is scanned, no memory is taken for bounds.
 bool prune_enabled();
-// Resets / reads the flags and the two largest moves; then every row's bounds are moved with the
+constexpr int kPruneFull = 3;
+// After a test that listed more rows than the compact copy holds, the next iterations scan every row
+// untested: 1, then 3, then 7 of them while tests go on failing. In overlapping clusters no test holds for
+// long, and each costs the centers' scan and two passes over the rows (2M x 64, K=256: 53 of 618 us an
+// iteration); in clusters that lie apart the first tests fail only while the centers still move far. Not in
+// double precision: an untested iteration counts every center as changed, and its sums cost more than the
+// tests (400,000 x 64, K=256: 7.9 -> 8.4 ms).
+constexpr int kPruneWait = 7;
+// Resets / reads the flags and the two largest moves, and decides whether this iteration tests its rows.
+cudaError_t launch_prune_top(const PruneState& ps, const int* stop, cudaStream_t s);
+// Then (after the centers' scan, flags[6] rows) every row's bounds are moved with the
 // centers and the rows whose label they no longer prove are listed (flags[1] > cap: all rows).
 cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
                                 cudaStream_t s);

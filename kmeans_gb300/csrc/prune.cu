@@ -27,8 +27,10 @@ constexpr int PF_THREADS = 256;
 constexpr int PF_ROWS = 4 * PF_THREADS;  // rows per block step, four consecutive ones per thread
 
 // The two largest moves and the center of the largest (unusable centers, -1, never count); starts
-// the list of rows to scan: empty when the bounds are valid, else past every capacity (and every
+// the list of rows to scan: empty when the rows are tested, else past every capacity (and every
 // center's members count as changed). One block.
+// State (flags[7]): bit 0, this iteration scans every row untested; bit 1, lab_old is not that of the last
+// update; bits 8 up, iterations yet to go untested; bits 16 up, how many the last failed test asked for.
 __global__ void __launch_bounds__(1024)
 prune_top_kernel(PruneState ps, const int* stop) {
   if (grid_enter()) return;
@@ -36,7 +38,22 @@ prune_top_kernel(PruneState ps, const int* stop) {
   __shared__ float s1[32], s2[32];
   __shared__ int si[32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int first = ps.flags[0] == 0;
+  const bool first = ps.flags[0] == 0;
+  const bool still = !first && ps.flags[4] == 0;  // the last update found no center's members changed
+  const int state = ps.flags[7];
+  bool stale = ps.wait > 0;  // else prune_dirty_kernel keeps the labels of an untested iteration
+  int wait = 0, back = 0;
+  if (!first) {
+    wait = (state >> 8) & 0xff;
+    back = (state >> 16) & 0xff;
+    if (!(state & 1)) {  // the last iteration was tested
+      stale = ps.flags[1] > ps.cap && (state & 2);
+      if (ps.flags[1] <= ps.cap) back = 0;
+      else wait = back = min(2 * back + 1, ps.wait);
+    }
+  }
+  const bool full = first || (wait > 0 && !still);
+  if (full && !first) --wait;
   float b1 = 0.0f, b2 = 0.0f;
   int i1 = -1;
   for (int j = threadIdx.x; j < ps.k; j += blockDim.x) {
@@ -48,7 +65,7 @@ prune_top_kernel(PruneState ps, const int* stop) {
     } else {
       b2 = fmaxf(b2, v);
     }
-    ps.dirty[j] = first;
+    ps.dirty[j] = full;
   }
   auto merge = [&](float o1, float o2, int oi) {
     b2 = fmaxf(fminf(b1, o1), fmaxf(b2, o2));
@@ -76,21 +93,21 @@ prune_top_kernel(PruneState ps, const int* stop) {
     if (lane == 0) {
       ps.top[0] = b1;
       ps.top[1] = b2;
+      ps.flags[0] = 1;
+      ps.flags[1] = full ? 0x7fffffff : 0;
+      ps.flags[2] = 0;  // the scan of the centers counts from zero
       ps.flags[3] = i1;
-      ps.flags[1] = first ? 0x7fffffff : 0;
-      // the last update found every center's members unchanged, so no center has moved: every label
-      // and bound stands and nothing is scanned
-      ps.flags[5] = !first && ps.flags[4] == 0;
-      ps.flags[4] = first;
-      ps.flags[0] = ps.k;
-      ps.flags[2] = 0;  // the next iteration's scan of the centers counts from zero
+      ps.flags[4] = full;
+      ps.flags[5] = still;  // no center has moved: every label and bound stands and nothing is scanned
+      ps.flags[6] = full || still ? 0 : ps.k;
+      ps.flags[7] = (full ? 1 : 0) | (stale ? 2 : 0) | wait << 8 | back << 16;
     }
   }
 }
 
 // Moves every row's bounds with the centers and lists the rows they no longer prove. Once more than
 // `cap` rows are listed every row will be scanned (and its bounds written anew): the blocks still
-// to come return.
+// to come return. Where lab_old is stale it takes the labels of the last update on the way.
 __global__ void __launch_bounds__(PF_THREADS)
 prune_filter_kernel(PruneState ps, const int* labels, const int* stop) {
   if (grid_enter()) return;
@@ -101,6 +118,7 @@ prune_filter_kernel(PruneState ps, const int* labels, const int* stop) {
   if (ps.flags[5]) return;
   const float top1 = ps.top[0], top2 = ps.top[1];
   const int topi = ps.flags[3];
+  const bool stale = ps.flags[7] & 2;
   for (long long b0 = (long long)blockIdx.x * PF_ROWS; b0 < ps.n; b0 += (long long)gridDim.x * PF_ROWS) {
     if (threadIdx.x == 0) base_sh = *(volatile int*)(ps.flags + 1);
     __syncthreads();
@@ -143,11 +161,13 @@ prune_filter_kernel(PruneState ps, const int* labels, const int* stop) {
     if (i0 + 4 <= ps.n) {
       *reinterpret_cast<float4*>(ps.ub + i0) = make_float4(u[0], u[1], u[2], u[3]);
       *reinterpret_cast<float4*>(ps.lb + i0) = make_float4(l[0], l[1], l[2], l[3]);
+      if (stale) *reinterpret_cast<int4*>(ps.lab_old + i0) = make_int4(a[0], a[1], a[2], a[3]);
     } else {
       for (int r = 0; r < 4; ++r)
         if (i0 + r < ps.n) {
           ps.ub[i0 + r] = u[r];
           ps.lb[i0 + r] = l[r];
+          if (stale) ps.lab_old[i0 + r] = a[r];
         }
     }
     // one block-wide scan and one atomic per block step
@@ -195,7 +215,8 @@ prune_gather_kernel(PruneState ps, const uint4* Xb, const uint4* Xl, int row_vec
 }
 
 // Marks the old and the new center of every scanned row whose label changed since the last update
-// (after a first iteration every center is marked already and lab_old takes all labels). A block
+// (every center, where the rows were not tested or lab_old is not known for all of them; it is kept after an
+// untested iteration where none of these may follow another, else by the next filter). A block
 // collects its marks in shared memory where the centers fit: in early iterations hundreds of
 // thousands of rows mark the same few hundred centers (898,790 rows, K=256: 300 us through global
 // memory).
@@ -205,9 +226,23 @@ __global__ void __launch_bounds__(1024)
 prune_dirty_kernel(PruneState ps, const int* labels, const int* stop) {
   if (grid_enter()) return;
   const int halt = stop ? pinned(stop) : 0;
-  const int cnt = pinned(ps.flags + 1);
+  const int cnt = pinned(ps.flags + 1), state = pinned(ps.flags + 7);
   if (halt) return;
   if (cnt == 0) return;
+  if (state & 1) {  // untested: prune_top_kernel marked every center
+    if (state & 2) return;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ps.n;
+         i += (long long)gridDim.x * blockDim.x)
+      ps.lab_old[i] = labels[i];
+    return;
+  }
+  if (cnt > ps.cap && (state & 2)) {  // the filter stopped before lab_old was known for all rows
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < ps.k; j += gridDim.x * blockDim.x) {
+      ps.dirty[j] = 1;
+      ps.flags[4] = 1;
+    }
+    return;
+  }
   extern __shared__ unsigned char mark[];
   const bool sh = ps.k <= kDirtyShared;
   if (sh) {
@@ -464,15 +499,21 @@ cudaError_t launch_prune_dirty(const PruneState& ps, const int* labels, const in
   return cudaGetLastError();
 }
 
+cudaError_t launch_prune_top(const PruneState& ps, const int* stop, cudaStream_t s) {
+  if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
+  launch(prune_top_kernel, 1, 1024, 0, s)(ps, stop);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_prune_filter(const PruneState& ps, const int* labels, const int* stop,
                                 cudaStream_t s) {
   if (inject_fault(kFaultLaunch)) return cudaErrorLaunchOutOfResources;
-  launch(prune_top_kernel, 1, 1024, 0, s)(ps, stop);
   const long long steps = (ps.n + PF_ROWS - 1) / PF_ROWS;
   const long long most = kmgb::num_sms() * 8LL;
   launch(prune_filter_kernel, (unsigned)(steps < most ? steps : most), PF_THREADS, 0, s)(ps, labels,
                                                                                      stop);
-  count_launches(2);
+  count_launches(1);
   return cudaGetLastError();
 }
 

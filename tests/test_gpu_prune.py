@@ -212,3 +212,20 @@ def test_run_length_decides(km, orc, torch_cuda, monkeypatch, graphs):
             h.synchronize()
             assert np.array_equal(h.centers(), want[it][1]) and np.array_equal(h.labels(), want[it][2])
         h.close()
+
+
+@pytest.mark.parametrize("tier", ["BF16X3", "FP32"])
+@pytest.mark.parametrize("device", [False, True])
+def test_bounds_after_tests_that_listed_too_many_rows(km, orc, torch_cuda, tier, device):
+    """Byte-valued rows whose first tests fail (so that the next iterations go untested) and whose later
+    ones hold: every iteration's state is that of the oracle's loop."""
+    n, d, k = 70_000, 128, 256
+    rng = np.random.default_rng(17)
+    means = rng.uniform(-60, 60, (k, d)) + 20
+    X = np.clip(np.round(means[rng.integers(0, k, n)] + 30 * rng.standard_normal((n, d))), 0, 255)
+    X = X.astype(np.float32)
+    init = X[sample_init(n, k, seed=18)].copy()
+    src = torch_cuda.from_numpy(X).cuda() if device else X
+    for iters in (5, 9, 24):
+        check(km.lloyd(src, k, init=init, max_iters=iters, assign_tier=getattr(km, "ASSIGN_" + tier),
+                       empty_policy=1), orc.lloyd(X, init, iters, empty_policy=1), iters)
